@@ -5,6 +5,7 @@
 // Hugging Face `apply_rotary_pos_emb` and `act_fn(gate) * up`); the arithmetic below reproduces the
 // eager torch results bit for bit: every product and sum is rounded to fp32 separately, the same
 // `expf` and IEEE division, bf16 rounding after SiLU and after the product.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -25,6 +26,14 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   uint32_t r;
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
   return r;
+}
+
+__device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
+  asm("max.bf16x2 %0, %0, %1;" : "+r"(a) : "r"(b));
+  return a;
+}
+__device__ __forceinline__ uint32_t gt_mask_bf16x2(uint32_t a, uint32_t b) {   // 0xffff per half where a > b
+  return __hgt2_mask(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
 }
 
 // x: [tokens, row_elems] bf16; the first `heads` heads of `dim` elements of each row are rotated:
@@ -546,68 +555,118 @@ __global__ void arcq_ep_rows_kernel(const uint4* __restrict__ src, const int* __
 
 // Calibration statistics in one pass over the activations (utilize.py:108 and :546-547 of ARCQuant):
 // per-channel running max|x| and the number of elements larger than an eighth of their row's (signed)
-// maximum.  A CTA of 256 threads walks rows b, b + grid, ...; thread t owns the 16-byte chunks t, t + 256,
-// ... of every row, so its channels' maxima stay in registers and leave with one atomic each at the end.
-template <int CPT>
-__global__ void __launch_bounds__(256) arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K,
-                                                               unsigned int* chan_absmax, unsigned long long* above) {
-  __shared__ float s_max[2][8];
+// maximum.  Thread t of a CTA owns the 16-byte chunks t, t + 512, ... of every row it meets, so its channels'
+// maxima stay in registers; RB rows are in flight together, so that one barrier serves their RB row maxima.
+// Bound: HBM in principle (2 bytes per element); what set the time was the channel maxima's way out.  One
+// atomic per channel and CTA, 4.85 million on 4096 addresses at [2000, 4096], took 184 us of which the data
+// needs 3.  Here the CTAs of a cluster of eight reduce their maxima through distributed shared memory, and an
+// eighth of the CTAs' worth of results meets the running maxima, with an atomic only where a larger value was
+// found.
+constexpr int CALIB_THREADS = 512, CALIB_CLUSTER = 8;
+template <int CPT, int RB>
+__global__ void __launch_bounds__(CALIB_THREADS, CPT * RB > 8 ? 1 : 2)
+arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, unsigned int* chan_absmax,
+                        unsigned long long* above) {
+  constexpr int WARPS = CALIB_THREADS / 32;
+  extern __shared__ __align__(16) uint32_t s_col[];           // [K/2]: this CTA's channel maxima, two per word
+  __shared__ uint32_t s_max[2][WARPS][RB / 2];
+  namespace cg = cooperative_groups;
+  const cg::cluster_group cluster = cg::this_cluster();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nchunks = K >> 3;
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   uint32_t cmax[CPT][4];
 #pragma unroll
   for (int j = 0; j < CPT; ++j) cmax[j][0] = cmax[j][1] = cmax[j][2] = cmax[j][3] = 0;
   unsigned long long count = 0;
   int buf = 0;
-  for (long long r = blockIdx.x; r < rows; r += gridDim.x, buf ^= 1) {
-    const uint4* row = reinterpret_cast<const uint4*>(x + r * (long long)K);
-    uint4 v[CPT];
-    float m = -INFINITY;
+  for (long long r0 = (long long)blockIdx.x * RB; r0 < rows; r0 += (long long)gridDim.x * RB, buf ^= 1) {
+    uint4 v[RB][CPT];
 #pragma unroll
-    for (int j = 0; j < CPT; ++j) {
-      const int c = tid + j * 256;
-      v[j] = c < nchunks ? __ldg(row + c) : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);   // -inf
-      const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+    for (int i = 0; i < RB; ++i) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        m = fmaxf(m, fmaxf(lo_f(w[k]), hi_f(w[k])));
-        if (c < nchunks) asm("max.u16x2 %0, %0, %1;" : "+r"(cmax[j][k]) : "r"(w[k] & 0x7fff7fffu));
+      for (int j = 0; j < CPT; ++j) {
+        const int c = tid + j * CALIB_THREADS;
+        v[i][j] = make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);   // -inf: never above, never a maximum
+        if (c < nchunks && r0 + i < rows) v[i][j] = __ldcs(reinterpret_cast<const uint4*>(x + (r0 + i) * (long long)K) + c);
       }
     }
+    uint32_t m[RB / 2];                                        // (row 2i, row 2i + 1): signed maxima
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, d));
-    if (lane == 0) s_max[buf][warp] = m;
+    for (int i = 0; i < RB; i += 2) {
+      uint32_t a = 0xff80ff80u, b = 0xff80ff80u;
+#pragma unroll
+      for (int j = 0; j < CPT; ++j) {
+        const uint32_t wa[4] = {v[i][j].x, v[i][j].y, v[i][j].z, v[i][j].w};
+        const uint32_t wb[4] = {v[i + 1][j].x, v[i + 1][j].y, v[i + 1][j].z, v[i + 1][j].w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          a = max_bf16x2(a, wa[k]);
+          b = max_bf16x2(b, wb[k]);
+          if (r0 + i < rows) asm("max.u16x2 %0, %0, %1;" : "+r"(cmax[j][k]) : "r"(wa[k] & 0x7fff7fffu));
+          if (r0 + i + 1 < rows) asm("max.u16x2 %0, %0, %1;" : "+r"(cmax[j][k]) : "r"(wb[k] & 0x7fff7fffu));
+        }
+      }
+      m[i / 2] = max_bf16x2(__byte_perm(a, b, 0x5410), __byte_perm(a, b, 0x7632));
+    }
+#pragma unroll
+    for (int i = 0; i < RB / 2; ++i) {
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) m[i] = max_bf16x2(m[i], __shfl_xor_sync(0xffffffffu, m[i], d));
+      if (lane == 0) s_max[buf][warp][i] = m[i];
+    }
     __syncthreads();
-    float rm = s_max[buf][0];
+    int above16 = 0;                                           // sixteen per element above
 #pragma unroll
-    for (int k = 1; k < 8; ++k) rm = fmaxf(rm, s_max[buf][k]);
-    // the threshold in the tensor's own type, as torch computes `max * 0.125` on a bf16 tensor
-    const float thr = __uint_as_float(pack2(__fmul_rn(rm, 0.125f), 0.f) << 16);
+    for (int i = 0; i < RB; i += 2) {
+      uint32_t rm = s_max[buf][0][i / 2];
 #pragma unroll
-    for (int j = 0; j < CPT; ++j) {
-      if (tid + j * 256 < nchunks) {
-        const uint32_t w[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+      for (int k = 1; k < WARPS; ++k) rm = max_bf16x2(rm, s_max[buf][k][i / 2]);
+      // the threshold in the tensor's own type, as torch computes `max * 0.125` on a bf16 tensor
+      const uint32_t t = pack2(__fmul_rn(lo_f(rm), 0.125f), __fmul_rn(hi_f(rm), 0.125f));
+      const uint32_t ta = __byte_perm(t, t, 0x1010), tb = __byte_perm(t, t, 0x3232);
 #pragma unroll
-        for (int k = 0; k < 4; ++k) count += (lo_f(w[k]) > thr ? 1 : 0) + (hi_f(w[k]) > thr ? 1 : 0);
+      for (int j = 0; j < CPT; ++j) {
+        const uint32_t wa[4] = {v[i][j].x, v[i][j].y, v[i][j].z, v[i][j].w};
+        const uint32_t wb[4] = {v[i + 1][j].x, v[i + 1][j].y, v[i + 1][j].z, v[i + 1][j].w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) above16 += __popc(gt_mask_bf16x2(wa[k], ta)) + __popc(gt_mask_bf16x2(wb[k], tb));
       }
     }
+    count += (unsigned long long)(above16 >> 4);
   }
 #pragma unroll
   for (int j = 0; j < CPT; ++j) {
-    const int c = tid + j * 256;
-    if (c < nchunks) {
+    const int c = tid + j * CALIB_THREADS;
+    if (c < nchunks) *reinterpret_cast<uint4*>(s_col + 4 * c) = make_uint4(cmax[j][0], cmax[j][1], cmax[j][2], cmax[j][3]);
+  }
+  cluster.sync();
+  const int rank = (int)cluster.block_rank();
+  const uint32_t* peers[CALIB_CLUSTER];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        atomicMax(chan_absmax + 8 * c + 2 * k, (cmax[j][k] & 0xffffu) << 16);
-        atomicMax(chan_absmax + 8 * c + 2 * k + 1, cmax[j][k] & 0xffff0000u);
-      }
-    }
+  for (int q = 0; q < CALIB_CLUSTER; ++q) peers[q] = cluster.map_shared_rank(s_col, q);
+  for (int w = rank * CALIB_THREADS + tid; w < (K >> 1); w += CALIB_CLUSTER * CALIB_THREADS) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int q = 0; q < CALIB_CLUSTER; ++q) asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(peers[q][w]));
+    // (non-negative floats order like their bit patterns; a stale value read here only costs an atomic)
+    if ((m << 16) > __ldcg(chan_absmax + 2 * w)) atomicMax(chan_absmax + 2 * w, m << 16);
+    if ((m & 0xffff0000u) > __ldcg(chan_absmax + 2 * w + 1)) atomicMax(chan_absmax + 2 * w + 1, m & 0xffff0000u);
   }
   if (above != nullptr) {
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) count += __shfl_xor_sync(0xffffffffu, count, d);
-    if (lane == 0 && count) atomicAdd(above, count);
+    __shared__ unsigned long long s_count[WARPS];
+    if (lane == 0) s_count[warp] = count;
+    __syncthreads();
+    if (tid == 0) {
+      unsigned long long t = 0;
+      for (int k = 0; k < WARPS; ++k) t += s_count[k];
+      if (t) atomicAdd(above, t);
+    }
   }
+  cluster.sync();                                              // nobody leaves while its maxima are being read
 }
 
 }  // namespace
@@ -618,21 +677,37 @@ int launch_calib_stats(const void* x, int64_t rows, int K, float* chan_absmax, u
   DeviceInfo di;
   int rc = get_device_info(&di);
   if (rc != ARCQ_OK) return rc;
-  long long grid = (long long)di.num_sms * 8;
-  if (grid > rows) grid = rows;
-  const int cpt = (K / 8 + 255) / 256;
+  const int cpt = (K / 8 + CALIB_THREADS - 1) / CALIB_THREADS;
   auto xs = static_cast<const uint16_t*>(x);
   auto cm = reinterpret_cast<unsigned int*>(chan_absmax);
-#define ARCQ_CALIB(CPT_) arcq_calib_stats_kernel<CPT_><<<(unsigned)grid, 256, 0, stream>>>(xs, rows, K, cm, above)
-  if (cpt <= 1) ARCQ_CALIB(1);
-  else if (cpt <= 2) ARCQ_CALIB(2);
-  else if (cpt <= 4) ARCQ_CALIB(4);
-  else if (cpt <= 8) ARCQ_CALIB(8);
-  else if (cpt <= 16) ARCQ_CALIB(16);
-  else return ARCQ_ERR_UNSUPPORTED_K;
-#undef ARCQ_CALIB
-  ARCQ_CUDA_TRY(cudaGetLastError());
-  return ARCQ_OK;
+  auto launch = [&](auto kern, int rb) -> int {
+    const size_t smem = (size_t)K * 2;
+    if (smem > 48 * 1024) ARCQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    long long grid = (rows + rb - 1) / rb;
+    if (grid > 2LL * di.num_sms) grid = 2LL * di.num_sms;
+    grid = (grid + CALIB_CLUSTER - 1) / CALIB_CLUSTER * CALIB_CLUSTER;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(CALIB_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = CALIB_CLUSTER;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, xs, (long long)rows, K, cm, above));
+    return ARCQ_OK;
+  };
+  // (rows in flight per CTA: eight 16-byte loads per thread, two rows at least)
+  if (cpt <= 1) return launch(arcq_calib_stats_kernel<1, 8>, 8);
+  if (cpt <= 2) return launch(arcq_calib_stats_kernel<2, 4>, 4);
+  if (cpt <= 4) return launch(arcq_calib_stats_kernel<4, 2>, 2);
+  if (cpt <= 8) return launch(arcq_calib_stats_kernel<8, 2>, 2);
+  return ARCQ_ERR_UNSUPPORTED_K;
 }
 
 int launch_ep_send_layout(const long long* ids, int n, int e_local, int ep, int cap, int rank, int* slot,

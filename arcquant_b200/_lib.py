@@ -20,8 +20,10 @@ ERR_ALIGNMENT = 5
 ERR_TIMEOUT = 6
 ERR_SCRATCH_LIMIT = 7
 STATIC_SCRATCH_BYTES = 2 << 20
+SCALE_SCRATCH = 512
 
-GEMM_KIND_SINGLE, GEMM_KIND_SPLIT_K, GEMM_KIND_PAIR = 0, 1, 2
+GEMM_KIND_SINGLE, GEMM_KIND_SPLIT_K, GEMM_KIND_PAIR, GEMM_KIND_SKINNY = 0, 1, 2, 3
+SKINNY_ROWS = 64
 
 MODE_16 = 16
 MODE_32 = 32
@@ -37,6 +39,8 @@ SIGNATURES = {
     "arcq_reference_mode": (_i32, [_i32]),
     "arcq_reorder_quantize_x": (_i32, [_vp, _vp, _i64, _i32, _i32, _i32, _vp, _vp, _vp]),
     "arcq_reorder_quantize_x_scaled": (_i32, [_vp, _vp, _vp, _i64, _i32, _i32, _i32, _vp, _vp, _vp]),
+    "arcq_quantize_tensor_scale": (_i32, [_vp, _vp, _i32, _vp, _i64, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp]),
+    "arcq_quantize_x_grouped_amax": (_i32, [_vp, _vp, _vp, _vp, _vp, _i32, _i64, _i32, _i32, _i32, _vp, _vp, _vp, _vp]),
     "arcq_rmsnorm_quantize_x": (_i32, [_vp, _vp, _f32, _vp, _i64, _i32, _i32, _vp, _vp, _vp]),
     "arcq_reorder_quantize_w": (_i32, [_vp, _vp, _i64, _i32, _i32, _i32, _vp, _vp, _vp]),
     "arcq_matmul_nvfp4": (_i32, [_vp, _vp, _vp, _vp, _i64, _i64, _i64, _f32, _vp, _vp]),

@@ -14,6 +14,8 @@ import math
 
 import torch
 
+from . import ops
+
 
 class ChannelAbsMax:
     """Running per-channel max |x| over any number of batches [..., channels], and with it the running
@@ -26,24 +28,29 @@ class ChannelAbsMax:
         self._above: torch.Tensor | None = None      # elements larger than an eighth of their row's maximum
         self._seen = 0                               # elements seen
 
-    @torch.no_grad()
     def update(self, x: torch.Tensor) -> None:
-        x2 = x.detach().reshape(-1, x.shape[-1])
-        k = x2.shape[1]
-        if x2.is_cuda and x2.dtype == torch.bfloat16 and k % 8 == 0 and k <= 32768 and x2.is_contiguous():
-            from . import ops
-
+        k = x.shape[-1]
+        native = x.is_cuda and x.dtype == torch.bfloat16 and k % 8 == 0 and k <= 32768
+        if native and not x.is_contiguous():
+            x = x.detach().reshape(-1, k)
+            native = x.is_contiguous()
+        if native:
             if self.value is None:
-                self.value = torch.zeros(k, dtype=torch.float32, device=x2.device)
+                self.value = torch.zeros(k, dtype=torch.float32, device=x.device)
             if self._above is None:
-                self._above = torch.zeros((), dtype=torch.int64, device=x2.device)
-            ops.calib_stats(x2, self.value, self._above)
+                self._above = torch.zeros((), dtype=torch.int64, device=x.device)
+            ops.calib_stats(x, self.value, self._above)
+            self._seen += x.numel()
         else:
-            cur = x2.abs().amax(dim=0).float()
-            self.value = cur if self.value is None else torch.maximum(self.value, cur.to(self.value.device))
-            thr = x2.max(dim=-1, keepdim=True)[0] * 0.125
-            n = (x2 > thr).sum().to(torch.int64)
-            self._above = n if self._above is None else self._above + n.to(self._above.device)
+            self._update_eager(x.detach().reshape(-1, k))
+
+    @torch.no_grad()
+    def _update_eager(self, x2: torch.Tensor) -> None:
+        cur = x2.abs().amax(dim=0).float()
+        self.value = cur if self.value is None else torch.maximum(self.value, cur.to(self.value.device))
+        thr = x2.max(dim=-1, keepdim=True)[0] * 0.125
+        n = (x2 > thr).sum().to(torch.int64)
+        self._above = n if self._above is None else self._above + n.to(self._above.device)
         self._seen += x2.numel()
 
     def reorder_index(self) -> torch.Tensor:

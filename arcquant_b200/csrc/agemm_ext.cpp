@@ -99,8 +99,8 @@ torch::Tensor matmul(const torch::Tensor& A, const torch::Tensor& B, const torch
   std::tie(M, N, K) = check_gemm_operands(A, B, SFA, SFB);
   c10::cuda::CUDAGuard guard(A.device());
   auto C = torch::empty({M, N}, torch::dtype(torch::kBFloat16).device(A.device()));
-  // skinny problems split K over idle SMs; the fp32 partial sums need scratch
-  const int64_t ws_bytes = static_cast<int64_t>(arcq_matmul_workspace_bytes(M, N, K));
+  // problems with few tiles split K over idle SMs; above ARCQ_SKINNY_ROWS rows the fp32 partial sums need scratch
+  const int64_t ws_bytes = M <= ARCQ_SKINNY_ROWS ? 0 : static_cast<int64_t>(arcq_matmul_workspace_bytes(M, N, K));
   torch::Tensor ws;
   if (ws_bytes > 0) ws = torch::empty({ws_bytes}, torch::dtype(torch::kUInt8).device(A.device()));
   int status = arcq_matmul_nvfp4_ws(A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(),
@@ -121,8 +121,8 @@ torch::Tensor matmul_dev_alpha(const torch::Tensor& A, const torch::Tensor& B, c
   if (alpha_b.has_value()) require_scalar_f32(*alpha_b, A, "alpha_b");
   c10::cuda::CUDAGuard guard(A.device());
   auto C = torch::empty({M, N}, torch::dtype(torch::kBFloat16).device(A.device()));
-  // skinny problems split K over idle SMs; the fp32 partial sums need scratch
-  const int64_t ws_bytes = static_cast<int64_t>(arcq_matmul_workspace_bytes(M, N, K));
+  // problems with few tiles split K over idle SMs; above ARCQ_SKINNY_ROWS rows the fp32 partial sums need scratch
+  const int64_t ws_bytes = M <= ARCQ_SKINNY_ROWS ? 0 : static_cast<int64_t>(arcq_matmul_workspace_bytes(M, N, K));
   torch::Tensor ws;
   if (ws_bytes > 0) ws = torch::empty({ws_bytes}, torch::dtype(torch::kUInt8).device(A.device()));
   int status = arcq_matmul_nvfp4_ws(
@@ -184,6 +184,53 @@ std::tuple<torch::Tensor, torch::Tensor> reorder_quantize_x_scaled(const torch::
   return std::make_tuple(Q, SF);
 }
 
+// (codes, scales, per-tensor scale): x or w divided by max / (448 * 6), then reordered and quantized; see
+// arcq_quantize_tensor_scale.  amax: max|x| as a 0-dim fp32 CUDA tensor if the caller has it.
+std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> quantize_tensor_scale(const torch::Tensor& X,
+                                                                              const torch::Tensor& reorder_index, const int KE,
+                                                                              int mode, bool is_weight,
+                                                                              const c10::optional<torch::Tensor>& amax) {
+  require_cuda(X, "input");
+  TORCH_CHECK(X.scalar_type() == at::kBFloat16, "input: expected bfloat16");
+  require_on(reorder_index, X, at::kShort, "reorder_index");
+  if (amax.has_value()) require_scalar_f32(*amax, X, "amax");
+  TORCH_CHECK(X.dim() == 2, "input must be 2-D");
+  const int64_t rows = X.size(0);
+  const int KQ = static_cast<int>(X.size(1));
+  const int K = KQ + KE;
+  TORCH_CHECK(KE >= 0 && KE <= KQ, "KE must lie in [0, KQ]");
+  TORCH_CHECK(reorder_index.numel() == KQ, "reorder_index must have KQ entries");
+  if (mode < 0) mode = arcq_reference_mode(KQ);
+  c10::cuda::CUDAGuard guard(X.device());
+  const auto u8 = X.options().dtype(torch::kUInt8), f32 = X.options().dtype(torch::kFloat32);
+  auto Q = torch::empty({rows, K / 2}, u8);
+  auto SF = torch::empty({static_cast<int64_t>(arcq_sf_bytes(rows, K))}, u8);
+  auto scale = torch::empty({}, f32);
+  torch::Tensor scratch;
+  if (!amax.has_value()) scratch = torch::empty({ARCQ_SCALE_SCRATCH}, f32);
+  check_status(arcq_quantize_tensor_scale(X.data_ptr(), amax.has_value() ? amax->data_ptr<float>() : nullptr, is_weight ? 1 : 0,
+                                          reorder_index.data_ptr<int16_t>(), rows, KQ, KE, mode, Q.data_ptr<uint8_t>(),
+                                          SF.data_ptr<uint8_t>(), scale.data_ptr<float>(),
+                                          amax.has_value() ? nullptr : scratch.data_ptr<float>(), current_stream(X)),
+               is_weight ? "run_reorder_w_bf16_nvfp4" : "run_reorder_x_bf16_nvfp4");
+  return std::make_tuple(Q, SF, scale);
+}
+
+// One batch of calibration statistics, accumulated in place; see arcq_calib_stats_bf16.
+void calib_stats(const torch::Tensor& X, const torch::Tensor& chan_absmax, const c10::optional<torch::Tensor>& above) {
+  require_cuda(X, "input");
+  TORCH_CHECK(X.scalar_type() == at::kBFloat16, "input: expected bfloat16");
+  require_on(chan_absmax, X, at::kFloat, "chan_absmax");
+  const int64_t K = X.size(-1);
+  TORCH_CHECK(chan_absmax.numel() == K, "chan_absmax must have one entry per channel");
+  if (above.has_value()) require_on(*above, X, at::kLong, "above");
+  c10::cuda::CUDAGuard guard(X.device());
+  check_status(arcq_calib_stats_bf16(X.data_ptr(), K ? X.numel() / K : 0, static_cast<int>(K), chan_absmax.data_ptr<float>(),
+                                     above.has_value() ? reinterpret_cast<unsigned long long*>(above->data_ptr<int64_t>()) : nullptr,
+                                     current_stream(X)),
+               "calib_stats");
+}
+
 std::tuple<torch::Tensor, torch::Tensor> silu_mul(const torch::Tensor& GU) {
   require_cuda(GU, "gate_up");
   TORCH_CHECK(GU.dim() == 2 && GU.size(1) % 16 == 0, "gate_up must be [tokens, 2F] with F a multiple of 8");
@@ -237,6 +284,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("B"), py::arg("SFA"), py::arg("SFB"), py::arg("alpha_a"), py::arg("alpha_b") = py::none());
   m.def("reorder_quantize_x_scaled", &reorder_quantize_x_scaled, "reorder_quantize_x of X / scale (device scalar)",
         py::arg("X"), py::arg("scale"), py::arg("reorder_index"), py::arg("KE"), py::arg("mode") = -1);
+  m.def("quantize_tensor_scale", &quantize_tensor_scale, "(Q, SF, scale) of x or w over its per-tensor scale", py::arg("X"),
+        py::arg("reorder_index"), py::arg("KE"), py::arg("mode") = -1, py::arg("is_weight") = false,
+        py::arg("amax") = py::none());
+  m.def("calib_stats", &calib_stats, "accumulate the calibration statistics of one batch", py::arg("X"),
+        py::arg("chan_absmax"), py::arg("above") = py::none());
   m.def("silu_mul", &silu_mul, "(silu(gate) * up, max|.|) of [gate | up]", py::arg("gate_up"));
   m.def("rope_inplace", &rope_inplace, "rotate-half rotary embedding in place on the first heads of each row",
         py::arg("X"), py::arg("cos"), py::arg("sin"), py::arg("heads"), py::arg("head_dim"));

@@ -33,6 +33,7 @@ int get_device_info(DeviceInfo* out) {
     DeviceInfo d;
     d.device = dev;
     ARCQ_CUDA_TRY(cudaDeviceGetAttribute(&d.num_sms, cudaDevAttrMultiProcessorCount, dev));
+    d.all_sms = d.num_sms;
     ARCQ_CUDA_TRY(cudaDeviceGetAttribute(&d.max_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     cache[dev] = d;
     have[dev] = true;
@@ -115,6 +116,35 @@ int arcq_reorder_quantize_x_scaled(const void* x, const float* scale, const int1
   if (!x || !scale || !qx || !sfx) return ARCQ_ERR_NULL_POINTER;
   if (!aligned16(x) || !aligned16(qx)) return ARCQ_ERR_ALIGNMENT;
   return launch_quantize(x, nullptr, 0.f, reorder_index, M, KQ, KE, mode, 0, qx, sfx, (cudaStream_t)stream, scale);
+}
+
+int arcq_quantize_tensor_scale(const void* x, const float* amax, int is_weight, const int16_t* reorder_index, int64_t rows,
+                               int KQ, int KE, int mode, uint8_t* q, uint8_t* sf, float* scale_out, float* scratch,
+                               void* stream) {
+  int rc = check_quant_shape(rows, KQ, KE, mode);
+  if (rc != ARCQ_OK) return rc;
+  if (!scale_out) return ARCQ_ERR_NULL_POINTER;
+  if (rows == 0) {
+    ARCQ_CUDA_TRY(cudaMemsetAsync(scale_out, 0, sizeof(float), (cudaStream_t)stream));
+    return ARCQ_OK;
+  }
+  if (!x || !q || !sf || (!amax && !scratch)) return ARCQ_ERR_NULL_POINTER;
+  if (!aligned16(x) || !aligned16(q)) return ARCQ_ERR_ALIGNMENT;
+  return launch_quantize_tensor_scale(x, amax, is_weight ? 1 : 0, reorder_index, rows, KQ, KE, mode, q, sf, scale_out, scratch,
+                                      (cudaStream_t)stream);
+}
+
+int arcq_quantize_x_grouped_amax(const void* x, const int32_t* row_map, const float* amax, const int16_t* reorder_indices,
+                                 const int32_t* groups, int ngroups, int64_t rows_bound, int KQ, int KE, int mode,
+                                 uint8_t* qx, uint8_t* sfx, float* scale_out, void* stream) {
+  int rc = check_quant_shape(rows_bound, KQ, KE, mode);
+  if (rc != ARCQ_OK) return rc;
+  if (ngroups < 1 || ngroups > 64) return ARCQ_ERR_BAD_SHAPE;
+  if (rows_bound == 0) return ARCQ_OK;
+  if (!x || !amax || !groups || !qx || !sfx || !scale_out) return ARCQ_ERR_NULL_POINTER;
+  if (!aligned16(x) || !aligned16(qx)) return ARCQ_ERR_ALIGNMENT;
+  return launch_quantize_tensor_scale(x, amax, 0, reorder_indices, rows_bound, KQ, KE, mode, qx, sfx, scale_out, nullptr,
+                                      (cudaStream_t)stream, groups, ngroups, row_map);
 }
 
 int arcq_rmsnorm_quantize_x(const void* x, const void* gamma, float eps, const int16_t* reorder_index,

@@ -18,11 +18,20 @@ int cuda_fail(cudaError_t e);
 
 struct DeviceInfo {
   int device;
-  int num_sms;
+  int num_sms;        // SMs that launches may use (arcq_set_sm_limit)
+  int all_sms;
   int max_smem_optin;
 };
 // Cached properties of the current device (queried once per device).
 int get_device_info(DeviceInfo* out);
+
+// How the divisor of a scaled quantization comes about: `scale` times the factor, or - npartials > 0 - the maximum of
+// that many values at `scale` times the factor; out (device, or null) receives it, per run of grouped rows.
+struct ScaleOptions {
+  float factor = 1.0f;
+  float* out = nullptr;
+  int npartials = 0;
+};
 
 // Launchers (defined in arcq_quant.cu / arcq_gemm.cu); arguments are validated by the callers
 // in arcq_api.cu.
@@ -32,7 +41,12 @@ int launch_quantize(const void* x, const void* gamma, float eps, const int16_t* 
                     const int* groups = nullptr, int ngroups = 0,   // runs of rows with their own order and scale
                     const int* row_map = nullptr,                   // input row of every output row
                     // further copies of the output (e.g. the peers' gathered buffers), see QuantParams
-                    uint8_t* const* q_extra = nullptr, uint8_t* const* sf_extra = nullptr, int nextra = 0);
+                    uint8_t* const* q_extra = nullptr, uint8_t* const* sf_extra = nullptr, int nextra = 0,
+                    const ScaleOptions& so = ScaleOptions());
+int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight, const int16_t* idx, int64_t rows, int KQ,
+                                 int KE, int mode, uint8_t* q, uint8_t* sf, float* scale_out, float* scratch,
+                                 cudaStream_t stream, const int* groups = nullptr, int ngroups = 0,
+                                 const int* row_map = nullptr);
 int launch_absmax(const void* x, int64_t n, float* out, int accumulate, cudaStream_t stream);
 // workspace (may be null): scratch for split-K partial sums, see gemm_workspace_bytes().
 int launch_gemm(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,
@@ -89,6 +103,12 @@ int launch_sum_partials(const void* const* srcs, int n, int64_t elems, const voi
 // Device address of the 65536-entry table bf16(silu(g)) on the current device; the first call per device
 // builds it on `stream`, later calls on other streams wait for that (arcq_layer.cu).
 int silu_table_ptr(cudaStream_t stream, const uint16_t** out);
+// Few rows: weight streaming (arcq_skinny.cu).
+int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, const uint8_t* SFW, int64_t M, int64_t N,
+                       int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, const void* residual, void* C,
+                       float* swiglu_amax, const int* groups, int ngroups, cudaStream_t stream);
+int skinny_plan_splits(int64_t N, int64_t K_eff);
+int skinny_poll_error();
 int gemm_poll_error();
 // Same for the bounded waits of the warp-specialised quantizer.
 int quant_poll_error();

@@ -132,6 +132,36 @@ def reorder_quantize_w(w, reorder_index, ke: int, mode=None):
     return _quantize("w", w, None, 0.0, reorder_index, ke, mode)
 
 
+def quantize_tensor_scale(x, reorder_index, ke: int, mode=None, is_weight: bool = False, amax=None):
+    """(codes, scales, scale) of x over its own per-tensor scale max / (448 * 6) - |x| for activations, the signed
+    maximum for weights - in two launches (one if `amax`, max|x| on the device, is given), or None where that
+    path does not apply: an empty or non-contiguous tensor, another type, no channel order, KQ > 16384."""
+    if (reorder_index is None or not x.is_cuda or x.dtype != torch.bfloat16 or x.dim() != 2 or not x.is_contiguous()
+            or x.shape[0] == 0 or x.shape[1] > 16384):
+        return None
+    ext = _ext()
+    if ext:
+        return ext.quantize_tensor_scale(x, reorder_index, ke, -1 if mode is None else mode, is_weight, amax)
+    lib = _lib.load()
+    _require(reorder_index, torch.int16, "reorder_index")
+    rows, kq = x.shape
+    if reorder_index.numel() != kq:
+        raise RuntimeError("reorder_index must have KQ entries")
+    q = torch.empty((rows, (kq + ke) // 2), dtype=torch.uint8, device=x.device)
+    sf = torch.empty((sf_bytes(rows, kq + ke),), dtype=torch.uint8, device=x.device)
+    scale = torch.empty((), dtype=torch.float32, device=x.device)
+    if amax is not None:
+        _require(amax, torch.float32, "amax")
+    scratch = torch.empty((_lib.SCALE_SCRATCH,), dtype=torch.float32, device=x.device)
+    with torch.cuda.device(x.device):
+        rc = lib.arcq_quantize_tensor_scale(x.data_ptr(), None if amax is None else amax.data_ptr(), int(is_weight),
+                                            reorder_index.data_ptr(), rows, kq, ke,
+                                            reference_mode(kq) if mode is None else mode, q.data_ptr(), sf.data_ptr(),
+                                            scale.data_ptr(), scratch.data_ptr(), _stream())
+    _lib.check(rc, f"quantize with tensor scale KQ={kq} KE={ke}")
+    return q, sf, scale
+
+
 def rmsnorm_quantize_x(x, weight, eps: float, reorder_index, ke: int, out=None):
     """RMSNorm(x)*weight fused in front of reorder_quantize_x."""
     ext = _ext()
@@ -150,8 +180,8 @@ def _matmul(a, b, sfa, sfb, alpha: float, alpha_a, alpha_b) -> torch.Tensor:
         raise RuntimeError("A and B disagree on K")
     c = torch.empty((m, n), dtype=torch.bfloat16, device=a.device)
     with torch.cuda.device(a.device):
-        # skinny problems split K over idle SMs; the fp32 partial sums need scratch
-        ws_bytes = int(lib.arcq_matmul_workspace_bytes(m, n, kb * 2))
+        # problems with few tiles split K over idle SMs; above SKINNY_ROWS rows the fp32 partial sums need scratch
+        ws_bytes = 0 if m <= _lib.SKINNY_ROWS else int(lib.arcq_matmul_workspace_bytes(m, n, kb * 2))
         ws = torch.empty((ws_bytes,), dtype=torch.uint8, device=a.device) if ws_bytes else None
         rc = lib.arcq_matmul_nvfp4_ws(a.data_ptr(), b.data_ptr(), sfa.data_ptr(), sfb.data_ptr(), m, n, kb * 2,
                                       float(alpha), None if alpha_a is None else alpha_a.data_ptr(),
@@ -236,6 +266,9 @@ def calib_stats(x: torch.Tensor, chan_absmax: torch.Tensor, above: torch.Tensor 
     """Accumulates the calibration statistics of x [..., K] (bf16, CUDA) in one pass: per-channel running
     max|x| into chan_absmax (fp32 [K]) and, if given, the count of elements above an eighth of their row's
     maximum into `above` (int64 scalar tensor)."""
+    ext = _ext()
+    if ext and x.is_contiguous():
+        return ext.calib_stats(x, chan_absmax, above)
     lib = _lib.load()
     x2 = x.reshape(-1, x.shape[-1])
     _require(x2, torch.bfloat16, "input")

@@ -17,8 +17,12 @@ FP8_MAX = 448.0
 def NVFP4_reorder_quantize_x(x: torch.Tensor, reorder_index: torch.Tensor, select_num: int, mode=None, amax=None):
     """(qx, scale_x, scale): per-tensor scale = max|x| / (448*6) as a 0-dim fp32 CUDA tensor,
     ``x / scale`` in bf16 as the reference forms it, then the fused reorder + NVFP4 + ARC kernel.
-    One pass for the amax (``arcq_absmax_bf16``) instead of ``torch.max(x.abs())``; a caller that
-    already has max|x| on the device (``ops.silu_mul``) passes it as ``amax``."""
+    One pass for partial maxima, the rest of the scale and the division inside the quantizer
+    (``arcq_quantize_tensor_scale``); a caller that already has max|x| on the device (``ops.silu_mul``)
+    passes it as ``amax``."""
+    fused = ops.quantize_tensor_scale(x, reorder_index, select_num, mode, False, amax)
+    if fused is not None:
+        return fused
     scale = (ops.absmax(x) if amax is None else amax) / (FP8_MAX * FP4_MAX)
     qx, scale_x = ops.reorder_quantize_x(x, reorder_index, select_num, mode=mode, scale=scale)   # x / scale, fused
     return qx, scale_x, scale
@@ -27,6 +31,9 @@ def NVFP4_reorder_quantize_x(x: torch.Tensor, reorder_index: torch.Tensor, selec
 def NVFP4_reorder_quantize_w(w: torch.Tensor, reorder_index: torch.Tensor, select_num: int, mode=None):
     """(qw, scale_w, scale).  The reference takes the SIGNED maximum of the weight here
     (model/qLinearLayer.py:26); kept for drop-in parity."""
+    fused = ops.quantize_tensor_scale(w, reorder_index, select_num, mode, True)
+    if fused is not None:
+        return fused
     scale = torch.max(w).float() / (FP8_MAX * FP4_MAX)
     qw, scale_w = ops.reorder_quantize_w(w / scale, reorder_index, select_num, mode=mode)
     return qw, scale_w, scale

@@ -91,6 +91,22 @@ int arcq_reference_mode(int kq);
 int arcq_reorder_quantize_x(const void* x, const int16_t* reorder_index, int64_t M, int KQ, int KE,
                             int mode, uint8_t* qx, uint8_t* sfx, void* stream);
 
+/* The two steps a caller of the reference takes around the operator, in one call: the per-tensor scale
+ * max / (448 * 6) (`scale = max|x| / (448.0 * 6.0)` in NVFP4_reorder_quantize_x, model/qLlamaLayer.py:73-77; the SIGNED
+ * maximum of a weight, model/qLinearLayer.py:25-28), then arcq_reorder_quantize_x_scaled - or its weight flavour - by it.
+ * amax: max|x| in device memory if the caller has it already, or NULL: a first pass leaves partial maxima in
+ * `scratch` (ARCQ_SCALE_SCRATCH floats of device memory).  scale_out (device) receives the scale: the fp32 product of
+ * the maximum with the fp32 reciprocal of 2688, as torch's division of a tensor by a host scalar computes it.
+ * ARCQ_ERR_UNSUPPORTED_K for KQ > 16384. */
+#define ARCQ_SCALE_SCRATCH 512
+int arcq_quantize_tensor_scale(const void* x, const float* amax, int is_weight, const int16_t* reorder_index, int64_t rows,
+                               int KQ, int KE, int mode, uint8_t* q, uint8_t* sf, float* scale_out, float* scratch,
+                               void* stream);
+/* arcq_reorder_quantize_x_grouped (below) from the runs' maxima amax[e]: divisor and scale_out[e] as above. */
+int arcq_quantize_x_grouped_amax(const void* x, const int32_t* row_map, const float* amax, const int16_t* reorder_indices,
+                                 const int32_t* groups, int ngroups, int64_t rows_bound, int KQ, int KE, int mode,
+                                 uint8_t* qx, uint8_t* sfx, float* scale_out, void* stream);
+
 /* arcq_reorder_quantize_x on x / *scale: the division by the per-tensor scale that the reference's
  * callers do in torch before the operator (`x / scale` in NVFP4_reorder_quantize_x,
  * model/qLlamaLayer.py:73-77) is done while the rows are staged.  No counterpart in the reference's
@@ -134,10 +150,10 @@ int arcq_matmul_nvfp4_dev_alpha(const uint8_t* A, const uint8_t* B, const uint8_
                                 int64_t M, int64_t N, int64_t K_eff, const float* alpha_a,
                                 const float* alpha_b, void* C, void* stream);
 
-/* Skinny problems (M <= 128 with a long K leave most SMs without an output tile) run faster when K
- * is split over the idle SMs; that needs scratch for the fp32 partial sums.
- * arcq_matmul_workspace_bytes: how much scratch the split-K path would use for this shape on the
- * current device (0 = the shape is not split).  arcq_matmul_nvfp4_ws: arcq_matmul_nvfp4 /
+/* Problems with few output tiles and a long K run faster when K is split over the idle SMs.  Up to ARCQ_SKINNY_ROWS
+ * rows the partial sums are exchanged on chip; above, the split needs scratch for them.
+ * arcq_matmul_workspace_bytes: how much scratch a split over global memory takes for this shape on the
+ * current device (0 = the shape is not split); up to ARCQ_SKINNY_ROWS rows it is not touched.  arcq_matmul_nvfp4_ws: arcq_matmul_nvfp4 /
  * _dev_alpha (alpha = alpha * *alpha_a * *alpha_b, the pointers may be NULL) with caller-provided
  * scratch; with workspace == NULL or too small it behaves exactly like arcq_matmul_nvfp4.  The
  * partials are summed in a fixed order, so results are reproducible.  Same reference interface
@@ -150,11 +166,14 @@ int arcq_matmul_nvfp4_ws(const uint8_t* A, const uint8_t* B, const uint8_t* SFA,
 /* Which kernel arcq_matmul_nvfp4* would run for this shape on the current device (no counterpart in the
  * reference, whose CUTLASS template picks nothing at run time): *kind = ARCQ_GEMM_KIND_PAIR (persistent
  * CTA pairs, 256 x 256 tiles), ARCQ_GEMM_KIND_SINGLE (one CTA per 128 x tile_n tile) or
- * ARCQ_GEMM_KIND_SPLIT_K (single-CTA tiles over *splits ranges of K; needs scratch).  *tile_n: tile
- * width; *splits: 1 unless split.  Any output pointer may be NULL. */
+ * ARCQ_GEMM_KIND_SPLIT_K (single-CTA tiles over *splits ranges of K; needs scratch) or
+ * ARCQ_GEMM_KIND_SKINNY (up to ARCQ_SKINNY_ROWS rows: weight streaming, K split over *splits CTAs of a cluster that add
+ * their partial sums on chip; no scratch).  *tile_n: tile width; *splits: 1 unless split.  Any output pointer may be NULL. */
 #define ARCQ_GEMM_KIND_SINGLE 0
 #define ARCQ_GEMM_KIND_SPLIT_K 1
 #define ARCQ_GEMM_KIND_PAIR 2
+#define ARCQ_GEMM_KIND_SKINNY 3
+#define ARCQ_SKINNY_ROWS 64
 int arcq_matmul_plan(int64_t M, int64_t N, int64_t K_eff, int* kind, int* tile_n, int* splits);
 
 /* No counterpart in the reference.  The split-K GEMM for callers that must not allocate device

@@ -1,0 +1,94 @@
+"""The row kernel of the quantizer and the per-tensor scale taken inside it: against the oracle, and against the scale
+formed in torch followed by the scaled operator.  Codes, scale bytes and the scale itself are exact."""
+import numpy as np
+import pytest
+import torch
+
+from arcquant_b200 import synth
+from tests.helpers import sf_take_rows, valid_sf
+
+pytestmark = pytest.mark.gpu
+
+
+# narrow rows, one group in the last warp, both sides of 512 groups, odd row counts, and both sides of the row count
+# up to which the row kernel runs (444 pairs of rows at 4096 channels, 148 at 14336 on 148 SMs)
+@pytest.mark.parametrize("rows,kq,ke", [(1, 16, 16), (3, 64, 0), (5, 528, 16), (33, 1040, 64), (1, 4096, 128), (887, 4096, 128),
+                                        (889, 4096, 128), (2, 8192, 256), (3, 8208, 16), (295, 14336, 128), (298, 14336, 64),
+                                        (7, 16384, 128), (300, 128, 32)])
+@pytest.mark.parametrize("weight", [False, True])
+def test_tensor_scale_inside_the_quantizer(rows, kq, ke, weight):
+    from arcquant_b200 import ops
+    from arcquant_b200.qlinear import NVFP4_reorder_quantize_w, NVFP4_reorder_quantize_x
+    from oracle import oracle as O
+
+    x = synth.activations(rows, kq, rows + kq, synth.outlier_channels(kq, max(1, kq // 100), 1), device="cuda")
+    x[rows // 2, kq // 3] = -x.abs().max() * 3            # the largest magnitude is negative: not a weight's maximum
+    idx = torch.randperm(kq, generator=torch.Generator().manual_seed(kq)).to(torch.int16).cuda()
+    scale = (x.max() if weight else x.abs().max()).float() / 2688.0
+    xs = (x / scale).cpu()
+    q, sf, s = (NVFP4_reorder_quantize_w if weight else NVFP4_reorder_quantize_x)(x, idx, ke, mode=16)
+    torch.cuda.synchronize()
+    assert s.shape == () and torch.equal(s, scale)
+    qo, so = (O.quantize_w if weight else O.quantize_x)(xs, idx.cpu().numpy(), ke, mode=16)
+    assert np.array_equal(q.cpu().numpy(), qo)
+    assert np.array_equal(valid_sf(sf, rows, kq + ke), valid_sf(so, rows, kq + ke))
+    if not weight:      # the maximum known beforehand
+        q2, sf2, s2 = NVFP4_reorder_quantize_x(x, idx, ke, mode=16, amax=x.abs().max().float())
+        assert torch.equal(q2, q) and torch.equal(s2, s)
+        assert np.array_equal(valid_sf(sf2, rows, kq + ke), valid_sf(sf, rows, kq + ke))
+    assert ops.gemm_poll_error() == 0
+
+
+@pytest.mark.parametrize("rows,kq", [(1, 1024), (7, 1536), (593, 4096), (590, 4096), (149, 8192), (297, 5120)])
+def test_fused_rmsnorm_of_few_rows(rows, kq):
+    from arcquant_b200 import ops
+    from oracle import oracle as O
+
+    x = synth.activations(rows, kq, rows, synth.outlier_channels(kq, kq // 100, 2), device="cuda")
+    gain = synth.rms_gain(kq, 3)
+    idx = synth.reorder_index_from_stats(x.abs().amax(0))
+    q, sf = ops.rmsnorm_quantize_x(x, gain.cuda(), 1e-5, idx.cuda(), 64)
+    qo, so = O.quantize_x(x.cpu(), idx.numpy(), 64, mode=16, gamma=gain, eps=1e-5)
+    assert np.array_equal(q.cpu().numpy(), qo)
+    assert np.array_equal(valid_sf(sf, rows, kq + 64), valid_sf(so, rows, kq + 64))
+
+
+@pytest.mark.parametrize("counts,kq", [((1, 0, 5, 2), 4096), ((0, 0, 3, 255), 14336), ((300, 257, 1, 0), 1024)])
+def test_grouped_rows_from_the_runs_maxima(counts, kq):
+    """Runs with their own maximum, order and divisor equal the per-run calls; an odd run length and an empty run."""
+    from arcquant_b200 import _lib, ops
+    from arcquant_b200.qlinear import NVFP4_reorder_quantize_x
+
+    e, ke = len(counts), 64
+    starts, at = [], 0
+    for c in counts:
+        starts.append(at)
+        at += (c + 255) // 256 * 256
+    bound = at + 256
+    x = synth.activations(sum(counts), kq, 5, synth.outlier_channels(kq, kq // 100, 2), device="cuda")
+    row_map = torch.zeros(bound, dtype=torch.int32)
+    src, k = {}, 0
+    for i, (s, c) in enumerate(zip(starts, counts)):
+        src[i] = torch.arange(k, k + c).flip(0)            # (not the identity)
+        row_map[s:s + c] = src[i].int()
+        k += c
+    groups = torch.tensor(starts + list(counts), dtype=torch.int32, device="cuda")
+    idx = torch.stack([torch.randperm(kq, generator=torch.Generator().manual_seed(i)) for i in range(e)]).to(torch.int16).cuda()
+    row_map = row_map.cuda()
+    amax = ops.absmax_grouped(x, row_map, groups, e)
+    q = torch.zeros((bound, (kq + ke) // 2), dtype=torch.uint8, device="cuda")
+    sf = torch.zeros((ops.sf_bytes(bound, kq + ke),), dtype=torch.uint8, device="cuda")
+    scale = torch.full((e,), -1.0, device="cuda")
+    rc = _lib.load().arcq_quantize_x_grouped_amax(x.data_ptr(), row_map.data_ptr(), amax.data_ptr(), idx.data_ptr(), groups.data_ptr(),
+                                                  e, bound, kq, ke, 16, q.data_ptr(), sf.data_ptr(), scale.data_ptr(),
+                                                  torch.cuda.current_stream().cuda_stream)
+    assert rc == 0
+    assert torch.equal(scale, amax / 2688.0)
+    for i, (s, c) in enumerate(zip(starts, counts)):
+        if c == 0:
+            continue
+        qi, sfi, si = NVFP4_reorder_quantize_x(x[src[i].cuda()].contiguous(), idx[i], ke, mode=16)
+        assert torch.equal(si, scale[i])
+        assert torch.equal(q[s:s + c], qi)
+        run = sf_take_rows(sf, np.arange(s, s + c), kq + ke)
+        assert np.array_equal(valid_sf(run, c, kq + ke), valid_sf(sfi, c, kq + ke))

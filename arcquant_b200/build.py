@@ -19,7 +19,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(ROOT, "include")
 LIB = os.path.join(HERE, "libarcq.so")
-CUDA_SOURCES = ["arcq_api.cu", "arcq_quant.cu", "arcq_gemm.cu", "arcq_layer.cu"]
+CUDA_SOURCES = ["arcq_api.cu", "arcq_quant.cu", "arcq_gemm.cu", "arcq_skinny.cu", "arcq_layer.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-I" + INCLUDE, "-I" + CSRC]
 
@@ -44,7 +44,7 @@ def _cuda_sources():
 
 def build_lib(force: bool = False, ptxas: bool = False) -> str:
     srcs = _cuda_sources()
-    deps = srcs + [os.path.join(CSRC, "arcq_internal.h"), os.path.join(INCLUDE, "arcq.h")]
+    deps = srcs + [os.path.join(CSRC, "arcq_internal.h"), os.path.join(CSRC, "arcq_tc.cuh"), os.path.join(INCLUDE, "arcq.h")]
     if not force and _newer(LIB, deps):
         return LIB
     objs = []

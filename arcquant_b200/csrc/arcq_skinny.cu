@@ -1,0 +1,530 @@
+// Block-scaled NVFP4 GEMM for few rows of A (decoding, experts with a handful of tokens): weight streaming.
+//
+// Bound: HBM, by the packed weight (N * K_eff * 9/16 bytes); the products are a rounding error.  So the operands
+// change sides: 128 rows of the WEIGHT are the M side of the MMA and the tokens its N side (16 to 64 columns), so
+// that a stage of the ring is weight (16 KB of codes + 2 KB of scales for K = 256) and little else, and the whole
+// chip's shared memory is a window of weight bytes in flight: two CTAs per SM, three to five stages each.
+//  * K is split over the CTAs of a cluster (up to eight) where N alone gives too few CTAs.  Every CTA pushes its fp32
+//    partial sums into the shared memory of the cluster's CTA that owns the token, one cluster barrier later they are
+//    added there in rank order (the same bits on every run): no scratch, no second launch.
+//  * SwiGLU (gate and up rows interleaved in blocks of 128): half of a cluster's CTAs compute the gate block, half the up
+//    block, and the owner of a token forms bf16(bf16(silu(g)) * u) from their sums, and its maximum.  (Grouped: one CTA
+//    computes both, one after the other, into two accumulators.)
+//  * Grouped problems (the experts of a MoE block): persistent CTAs walk over (expert, weight tile); the rows of each
+//    expert are read from the device, experts without rows cost nothing, and more than NT rows are taken NT at a time.
+//  * Programmatic dependent launch: while the kernel before is still running, every CTA pulls its first weight tiles
+//    into L2 (a prefetch reads nothing into the CTA, so a weight still being written is not read early).
+//
+// Roles: warp 0 producer (TMA), warp 1 MMA issuer, warps 2-5 epilogue, warps 6-9 scale warps (shared memory -> tensor
+// memory with tcgen05.st, as in arcq_gemm.cu; with tcgen05.cp in the issuing thread a stage took 1190 cycles, more than
+// its bytes need at HBM rate).
+#include "arcq_tc.cuh"
+
+namespace arcq {
+namespace {
+
+constexpr int SK_THREADS = 320;
+constexpr int SK_W_BYTES = 128 * BK_BYTES;      // 16 KB: 128 weight rows of one stage
+constexpr int SK_SF_BYTES = KSTEPS * ATOM;      // 2 KB: the scale atoms of 128 rows of one stage
+constexpr int SK_SF_COLS = 2 * KSTEPS * 4;      // tensor-memory columns of one stage's scales (both sides)
+
+// NT token columns, NA accumulators; SPLIT: room for the cluster's partial sums.  Two CTAs per SM (half of 228 KB, less
+// 1 KB per CTA for the system, 1 KB for alignment and the barriers).
+template <int NT, int NA, bool SPLIT>
+struct SkCfg {
+  static constexpr int X_BYTES = NT * BK_BYTES;
+  static constexpr int STAGE_BYTES = SK_W_BYTES + X_BYTES + 2 * SK_SF_BYTES;
+  static constexpr int BAR_BYTES = 256;
+  static constexpr int PART_BYTES = SPLIT ? NA * (NT + 7) * 512 : 0;   // (tokens rounded up to the cluster, at most eight)
+  static constexpr int FIT = (113 * 1024 - 1024 - BAR_BYTES - PART_BYTES) / STAGE_BYTES;
+  static constexpr int STAGES = FIT < 5 ? FIT : 5;
+  static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + PART_BYTES + BAR_BYTES;
+  static constexpr int TMEM_NEED = NA * NT + STAGES * SK_SF_COLS;
+  static constexpr int TMEM_COLS = TMEM_NEED <= 128 ? 128 : 256;
+  static_assert(STAGES >= 2 && TMEM_NEED <= 256, "two CTAs share 512 columns of tensor memory");
+};
+
+struct SkinnyParams {
+  const uint8_t* sfx;
+  const uint8_t* sfw;
+  __nv_bfloat16* c;                  // [M, N], or [M, N/2] with SwiGLU
+  const __nv_bfloat16* residual;     // [M, N] or nullptr
+  const float* alpha_a;
+  const float* alpha_b;
+  float alpha;
+  int M, N;
+  int ksteps_total;                  // K_eff / 64
+  int natoms;                        // scale atoms per 128-row tile
+  int tiles;                         // work items per matrix: ceil(N / 128), halved with SwiGLU
+  int sfw_tiles;                     // 128-row scale tiles of all matrices
+  int splits;                        // K ranges = CTAs per cluster
+  const int* groups;                 // run table of a grouped problem (device) or nullptr
+  int ngroups;
+  unsigned int* amax;                // SwiGLU: max|C| per matrix (bit pattern of a non-negative float)
+};
+
+__device__ __forceinline__ void sk_prefetch_tile(const CUtensorMap* map, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(map), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {   // the same place in another CTA's shared memory
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void st_cluster_f32(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ float bf16_round(float v) {
+  return __uint_as_float((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v)) << 16);
+}
+__device__ __forceinline__ float swiglu_bf16(float g, float u) {   // both already bf16 values
+  const float s = bf16_round(__fdiv_rn(g, __fadd_rn(1.0f, expf(-g))));
+  return bf16_round(__fmul_rn(s, u));
+}
+
+// NT: token columns per pass.  GATED: SwiGLU.  SPLIT: more than one CTA per cluster.
+template <int NT, bool GATED, bool SPLIT>
+__global__ void __launch_bounds__(SK_THREADS, 2)
+arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const SkinnyParams p) {
+  constexpr int NA = GATED && !SPLIT ? 2 : 1;          // accumulators of a CTA
+  constexpr int NB = GATED ? 2 : 1;                    // 128-row blocks of weight per work item
+  using C = SkCfg<NT, NA, SPLIT>;
+  constexpr int TMEM_COLS = C::TMEM_COLS;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* base_ptr = smem_raw + (base - smem_u32(smem_raw));
+  constexpr int BAR_AT = C::STAGES * C::STAGE_BYTES + C::PART_BYTES;
+  const uint32_t part_base = base + C::STAGES * C::STAGE_BYTES, bar_base = base + BAR_AT;
+  volatile uint32_t* misc = reinterpret_cast<volatile uint32_t*>(base_ptr + BAR_AT + 192);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(misc + 1);
+  auto full_bar = [&](int s) { return bar_base + 8u * s; };
+  auto empty_bar = [&](int s) { return bar_base + 8u * (C::STAGES + s); };
+  auto sf_bar = [&](int s) { return bar_base + 8u * (2 * C::STAGES + s); };       // scale atoms landed
+  const uint32_t acc_full_bar = bar_base + 8u * (3 * C::STAGES), acc_empty_bar = acc_full_bar + 8u;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  const int kstages = (p.ksteps_total + KSTEPS - 1) / KSTEPS;
+  const int csize = SPLIT ? p.splits * NB : 1;                         // CTAs per cluster
+  const int rank = SPLIT ? (int)(blockIdx.x % csize) : 0;
+  const int splits = SPLIT ? p.splits : 1, split = SPLIT ? rank % splits : 0;
+  const int block = SPLIT ? rank / splits : 0;                         // SwiGLU: 0 = gate, 1 = up
+  const int ks_begin = kstages * split / splits, ks_end = kstages * (split + 1) / splits;
+  const int first_item = (int)(blockIdx.x / csize), item_step = (int)(gridDim.x / csize);
+  const int num_items = p.tiles * p.ngroups;
+  // first weight row of accumulator a of work item `item`, in the stacked matrices
+  auto weight_row = [&](int item, int a) {
+    const int g = item / p.tiles, t = item - g * p.tiles;
+    return g * p.N + t * (128 * NB) + 128 * (block + a);
+  };
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < C::STAGES; ++s) {
+      mbar_init(full_bar(s), 1 + 4);       // the codes' bytes, and the four scale warps
+      mbar_init(empty_bar(s), 1);
+      mbar_init(sf_bar(s), 1);
+    }
+    mbar_init(acc_full_bar, 1);
+    mbar_init(acc_empty_bar, 4);
+    misc[1] = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    // the first ring of weight tiles on its way into L2
+    int n = 0;
+    for (int item = first_item; item < num_items && n < C::STAGES; item += item_step)
+      for (int a = 0; a < NA; ++a)
+        for (int ks = ks_begin; ks < ks_end && n < C::STAGES; ++ks, ++n) sk_prefetch_tile(&map_w, ks * BK_BYTES, weight_row(item, a));
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)misc)),
+                 "r"((uint32_t)TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");   // (every thread: everything below reads or writes global memory)
+  const uint32_t tmem_base = misc[0];
+  const uint32_t tmem_sf = tmem_base + NA * NT;
+
+  // rows of matrix g: first row in A / C, number
+  auto run_of = [&](int g, int& row0, int& cnt) {
+    if (p.groups == nullptr) { row0 = 0; cnt = p.M; return; }
+    row0 = __ldg(p.groups + g);
+    cnt = __ldg(p.groups + p.ngroups + g);
+  };
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ producer
+    if (lane == 0) {
+      uint32_t it = 0;
+      bool ok = true;
+      for (int item = first_item; item < num_items && ok; item += item_step) {
+        int row0, cnt;
+        run_of(item / p.tiles, row0, cnt);
+        for (int c0 = 0; c0 < cnt && ok; c0 += NT) {
+          const int boxes = (min(NT, cnt - c0) + 15) >> 4;               // 16 rows of A each
+          const int xt = (row0 + c0) >> 7;                               // 128-row scale tile of these rows
+          for (int ai = 0; ai < NA && ok; ++ai) {
+            const int wrow = weight_row(item, ai), wt = wrow >> 7;
+            for (int ks = ks_begin; ks < ks_end; ++ks, ++it) {
+              const int s = it % C::STAGES;
+              if (!mbar_wait(empty_bar(s), ((it / C::STAGES) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+              const uint32_t sf_bytes = (uint32_t)min(KSTEPS, p.ksteps_total - ks * KSTEPS) * ATOM;
+              const uint32_t st = base + s * C::STAGE_BYTES, x_s = st + SK_W_BYTES, sfw_s = x_s + C::X_BYTES, sfx_s = sfw_s + SK_SF_BYTES;
+              mbar_expect_tx(sf_bar(s), 2u * sf_bytes);
+              mbar_expect_tx(full_bar(s), SK_W_BYTES + (uint32_t)boxes * 2048u);
+              bulk_load(sfw_s, p.sfw + ((size_t)wt * p.natoms + (size_t)ks * KSTEPS) * ATOM, sf_bytes, sf_bar(s));
+              bulk_load(sfx_s, p.sfx + ((size_t)xt * p.natoms + (size_t)ks * KSTEPS) * ATOM, sf_bytes, sf_bar(s));
+              tma_load_2d(st, &map_w, full_bar(s), ks * BK_BYTES, wrow);
+              for (int b = 0; b < boxes; ++b) tma_load_2d(x_s + b * 2048, &map_x, full_bar(s), ks * BK_BYTES, row0 + c0 + 16 * b);
+            }
+          }
+        }
+      }
+      if (!ok) {
+        // giving up with copies possibly in flight: wait (bounded) for those started here, so that none lands in
+        // shared memory after the CTA has gone
+        const unsigned long long t0 = globaltimer_ns();
+        for (uint32_t j = it > (uint32_t)C::STAGES ? it - C::STAGES : 0; j < it; ++j)
+          while (!(mbar_try_wait(full_bar(j % C::STAGES), (j / C::STAGES) & 1u) && mbar_try_wait(sf_bar(j % C::STAGES), (j / C::STAGES) & 1u)) &&
+                 globaltimer_ns() - t0 < WAIT_LIMIT_NS) {}
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (lane == 0) {
+      uint32_t it = 0, acc_it = 0;
+      bool ok = true;
+      for (int item = first_item; item < num_items && ok; item += item_step) {
+        int row0, cnt;
+        run_of(item / p.tiles, row0, cnt);
+        for (int c0 = 0; c0 < cnt && ok; c0 += NT, ++acc_it) {
+          const uint32_t ncols = (uint32_t)((min(NT, cnt - c0) + 15) & ~15);
+          // e2m1 x e2m1, ue4m3 scales, K-major operands (see arcq_gemm.cu), N = ncols, M = 128
+          const uint32_t idesc = (1u << 7) | (1u << 10) | ((ncols >> 3) << 17) | (8u << 24);
+          if (!mbar_wait(acc_empty_bar, (acc_it & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+          tc_fence_after();
+          for (int ai = 0; ai < NA && ok; ++ai) {
+            for (int ks = ks_begin; ks < ks_end; ++ks, ++it) {
+              const int s = it % C::STAGES;
+              if (!mbar_wait(full_bar(s), (it / C::STAGES) & 1u, abort_flag)) { ok = false; break; }
+              tc_fence_after();
+              const int nk = min(KSTEPS, p.ksteps_total - ks * KSTEPS);
+              const uint32_t st = base + s * C::STAGE_BYTES;
+              const uint32_t t_sfw = tmem_sf + s * SK_SF_COLS, t_sfx = t_sfw + KSTEPS * 4;
+              const uint64_t wd = smem_desc(st, 1024, LAYOUT_SW128), xd = smem_desc(st + SK_W_BYTES, 1024, LAYOUT_SW128);
+              if (nk == KSTEPS) {
+#pragma unroll
+                for (int k = 0; k < KSTEPS; ++k)
+                  tc_mma_nvf4(tmem_base + ai * NT, wd + 2 * k, xd + 2 * k, idesc, t_sfw + k * 4, t_sfx + k * 4,
+                              (ks > ks_begin || k > 0) ? 1u : 0u);
+              } else {
+                for (int k = 0; k < nk; ++k)
+                  tc_mma_nvf4(tmem_base + ai * NT, wd + 2 * k, xd + 2 * k, idesc, t_sfw + k * 4, t_sfx + k * 4,
+                              (ks > ks_begin || k > 0) ? 1u : 0u);
+              }
+              tc_commit(empty_bar(s));
+            }
+          }
+          if (ok) tc_commit(acc_full_bar);
+        }
+      }
+    }
+  } else if (warp < 6) {
+    // ------------------------------------------------------------------ epilogue (warps 2..5)
+    const int quad = warp & 3;       // TMEM lanes 32*quad .. 32*quad+31 belong to this warp: weight rows of the tile
+    const uint32_t t_row = tmem_base + ((uint32_t)(quad * 32) << 16);
+    const int nl = quad * 32 + lane;                       // weight row within the tile
+    uint32_t acc_it = 0;
+    bool ok = true;
+    for (int item = first_item; item < num_items && ok; item += item_step) {
+      const int g = item / p.tiles, t = item - g * p.tiles;
+      int row0, cnt;
+      run_of(g, row0, cnt);
+      float alpha = p.alpha;
+      if (p.alpha_a) alpha *= __ldg(p.alpha_a + g);
+      if (p.alpha_b) alpha *= __ldg(p.alpha_b + g);
+      for (int c0 = 0; c0 < cnt; c0 += NT, ++acc_it) {
+        ok = mbar_wait(acc_full_bar, acc_it & 1u, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        tc_fence_after();
+        const int here = min(NT, cnt - c0);
+        if (SPLIT) {
+          // fp32 partial sums to the CTAs that own the tokens: token j belongs to rank j % csize, where it is
+          // number j / csize; layout there: [token number][source rank][128]
+          uint32_t dst[8];
+#pragma unroll
+          for (int r = 0; r < 8; ++r) dst[r] = cluster_addr(part_base, (uint32_t)min(r, csize - 1));
+          int r = 0;                                       // (rank of token j without a division per token)
+          uint32_t at = (uint32_t)(rank * 512 + nl * 4);
+          for (int j0 = 0; j0 < here; j0 += 16) {
+            uint32_t v[16];
+            tc_ld16(t_row + j0, v);
+            tc_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              if (j0 + j < here) {
+                uint32_t d = dst[0];
+#pragma unroll
+                for (int q = 1; q < 8; ++q) d = r == q ? dst[q] : d;
+                st_cluster_f32(d + at, v[j]);
+                if (++r == csize) { r = 0; at += (uint32_t)(csize * 512); }
+              }
+            }
+          }
+        } else {
+          const int n = t * 128 + nl;                      // output column
+          const int ncols = GATED ? p.N >> 1 : p.N;
+          float m = 0.f;
+          bool nan = false;
+          for (int j0 = 0; j0 < here; j0 += 16) {
+            uint32_t r[16], u[16];
+            tc_ld16(t_row + j0, r);
+            if (GATED) tc_ld16(t_row + (NA - 1) * NT + j0, u);
+            tc_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+              if (j0 + j < here && n < ncols) {
+                const size_t at = (size_t)(row0 + c0 + j0 + j) * ncols + n;
+                float v = bf16_round(__uint_as_float(r[j]) * alpha);
+                if (GATED) {
+                  v = swiglu_bf16(v, bf16_round(__uint_as_float(u[j]) * alpha));
+                  m = fmaxf(m, fabsf(v));
+                  nan |= v != v;
+                } else if (p.residual != nullptr) {
+                  v = bf16_round(__fadd_rn(__bfloat162float(p.residual[at]), v));
+                }
+                p.c[at] = __float2bfloat16_rn(v);
+              }
+            }
+          }
+          if (GATED) {
+            if (nan) m = __uint_as_float(0x7fff0000u);     // (a NaN counts as larger than everything, as in the other epilogues)
+            uint32_t mi = __float_as_uint(m);
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) mi = max(mi, __shfl_xor_sync(0xffffffffu, mi, d));
+            if (lane == 0 && mi) atomicMax(p.amax + g, mi);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty_bar);
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ scale warps (6..9)
+    // Warp q writes TMEM lanes 32q..32q+31: lane l's 16 bytes of an atom are its four columns (see arcq_gemm.cu).
+    const int quad = warp & 3;
+    uint32_t it = 0;
+    bool ok = true;
+    for (int item = first_item; item < num_items && ok; item += item_step) {
+      int row0, cnt;
+      run_of(item / p.tiles, row0, cnt);
+      for (int c0 = 0; c0 < cnt && ok; c0 += NT) {
+        const bool upper = ((row0 + c0) & 64) != 0;        // rows 64.. of a 128-row scale tile: words 2 and 3 of the atoms
+        for (int n = NA * (ks_end - ks_begin); n > 0; --n, ++it) {
+          const int s = it % C::STAGES;
+          ok = mbar_wait(sf_bar(s), (it / C::STAGES) & 1u, abort_flag);
+          ok = __all_sync(0xffffffffu, ok);
+          if (!ok) break;
+          // (the MMAs that read the stage's old scale columns are complete: its producer waited for them)
+          const uint4* sf = reinterpret_cast<const uint4*>(base_ptr + s * C::STAGE_BYTES + SK_W_BYTES + C::X_BYTES);
+          const uint32_t taddr = tmem_sf + s * SK_SF_COLS + ((uint32_t)(quad * 32) << 16);
+#pragma unroll
+          for (int side = 0; side < 2; ++side) {
+            uint32_t r[16];
+#pragma unroll
+            for (int k = 0; k < KSTEPS; ++k) {
+              uint4 v = sf[(side * KSTEPS + k) * 32 + lane];
+              if (side == 1 && upper) { v.x = v.z; v.y = v.w; }
+              r[4 * k] = v.x; r[4 * k + 1] = v.y; r[4 * k + 2] = v.z; r[4 * k + 3] = v.w;
+            }
+            tc_st16(taddr + side * (KSTEPS * 4), r);
+          }
+          tc_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(full_bar(s));
+        }
+      }
+    }
+  }
+
+  __syncwarp();
+  tc_fence_before();
+  if (SPLIT) {
+    // ------------------------------------------------------------------ the cluster's partial sums
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (*abort_flag == 0) {
+      const int t = first_item;
+      const int ncols = GATED ? p.N >> 1 : p.N;
+      float alpha = p.alpha;
+      if (p.alpha_a) alpha *= __ldg(p.alpha_a);
+      if (p.alpha_b) alpha *= __ldg(p.alpha_b);
+      uint32_t mi = 0;
+      const float4* part = reinterpret_cast<const float4*>(base_ptr + C::STAGES * C::STAGE_BYTES);
+      // four neighbouring columns of one of this CTA's tokens per thread and step
+      for (int i = threadIdx.x;; i += SK_THREADS) {
+        const int num = i >> 5, tok = num * csize + rank, n4 = (i & 31) * 4;
+        if (tok >= p.M) break;
+        float v[NB][4];
+#pragma unroll
+        for (int a = 0; a < NB; ++a) {
+          float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int r = 0; r < splits; ++r) {
+            const float4 q = part[(num * csize + a * splits + r) * 32 + (i & 31)];
+            sum.x += q.x; sum.y += q.y; sum.z += q.z; sum.w += q.w;
+          }
+          v[a][0] = sum.x; v[a][1] = sum.y; v[a][2] = sum.z; v[a][3] = sum.w;
+        }
+        const int n = t * 128 + n4;
+        if (n < ncols) {                                   // (a multiple of four columns is in or out: N % 8 == 0)
+          float o[4];
+          const size_t at = (size_t)tok * ncols + n;
+          uint2 res = make_uint2(0, 0);
+          if (!GATED && p.residual != nullptr) res = *reinterpret_cast<const uint2*>(p.residual + at);
+          const uint32_t rw[2] = {res.x, res.y};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            o[e] = bf16_round(v[0][e] * alpha);
+            if (GATED) {
+              o[e] = swiglu_bf16(o[e], bf16_round(v[NB - 1][e] * alpha));
+              mi = max(mi, __float_as_uint(o[e]) & 0x7fffffffu);
+            } else if (p.residual != nullptr) {
+              const float rv = __uint_as_float((e & 1) ? rw[e >> 1] & 0xffff0000u : rw[e >> 1] << 16);
+              o[e] = __fadd_rn(rv, o[e]);
+            }
+          }
+          *reinterpret_cast<uint2*>(p.c + at) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+        }
+      }
+      if (GATED) {
+        __syncwarp();
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) mi = max(mi, __shfl_xor_sync(0xffffffffu, mi, d));
+        if (lane == 0 && mi) atomicMax(p.amax, mi);
+      }
+    }
+  } else {
+    __syncthreads();
+  }
+  if (warp == 1) {
+    __syncwarp();
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"((uint32_t)TMEM_COLS) : "memory");
+  }
+}
+
+template <int NT, bool GATED, bool SPLIT>
+int launch_one(const CUtensorMap& mx, const CUtensorMap& mw, const SkinnyParams& p, int grid, cudaStream_t stream) {
+  using C = SkCfg<NT, GATED && !SPLIT ? 2 : 1, SPLIT>;
+  auto kern = arcq_skinny_kernel<NT, GATED, SPLIT>;
+  static thread_local int c_dev = -1;
+  int dev = 0;
+  ARCQ_CUDA_TRY(cudaGetDevice(&dev));
+  if (c_dev != dev) {
+    ARCQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
+    c_dev = dev;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(SK_THREADS);
+  cfg.dynamicSmemBytes = C::SMEM_BYTES;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)(p.splits * (GATED ? 2 : 1));
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = SPLIT ? 2 : 1;
+  ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, mx, mw, p));
+  return ARCQ_OK;
+}
+template <int NT>
+int launch_nt(const CUtensorMap& mx, const CUtensorMap& mw, const SkinnyParams& p, bool gated, int grid, cudaStream_t stream) {
+  if (gated) return launch_one<NT, true, true>(mx, mw, p, grid, stream);
+  return p.splits > 1 ? launch_one<NT, false, true>(mx, mw, p, grid, stream) : launch_one<NT, false, false>(mx, mw, p, grid, stream);
+}
+
+}  // namespace
+
+// K ranges of a plain problem.  More CTAs shorten each one's chain of stages until the clusters no longer fit the chip
+// at once; measured over 1..8 ranges (16 rows, us): [6144, 4224] 10.5 unsplit, 6.6 with 192 CTAs, 6.8 with 240, 10.4 with
+// 288; [4096, 4224] 10.5, 5.7 with 192, 6.4 with 256; [4096, 14464] 26.1, 9.8 with 192, 9.7 with 256.  So one and a half
+// CTAs per SM (one under an SM limit), at most eight ranges (the portable cluster
+// size), each at least two stages long.
+static int skinny_splits(int tiles, int kstages, const DeviceInfo& di) {
+  const int ctas = di.num_sms == di.all_sms ? di.num_sms * 3 / 2 : di.num_sms;
+  int s = ctas / tiles;
+  if (s > 8) s = 8;
+  if (s > kstages / 2) s = kstages / 2;
+  return s < 1 ? 1 : s;
+}
+// See SkinnyParams; `residual` and `swiglu_amax` exclude each other; groups (device) with ngroups matrices stacked in W.
+int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, const uint8_t* SFW, int64_t M, int64_t N,
+                       int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, const void* residual, void* C,
+                       float* swiglu_amax, const int* groups, int ngroups, cudaStream_t stream) {
+  DeviceInfo di;
+  int rc = get_device_info(&di);
+  if (rc != ARCQ_OK) return rc;
+  const bool gated = swiglu_amax != nullptr;
+  SkinnyParams p = {};
+  p.sfx = SFX;
+  p.sfw = SFW;
+  p.c = static_cast<__nv_bfloat16*>(C);
+  p.residual = static_cast<const __nv_bfloat16*>(residual);
+  p.alpha_a = alpha_a;
+  p.alpha_b = alpha_b;
+  p.alpha = alpha;
+  p.M = (int)M;
+  p.N = (int)N;
+  p.ksteps_total = (int)(K_eff / 64);
+  p.natoms = (int)((K_eff / 16 + 3) / 4);
+  p.tiles = gated ? (int)(N / 256) : (int)((N + 127) / 128);
+  p.groups = groups;
+  p.ngroups = groups != nullptr ? ngroups : 1;
+  p.amax = reinterpret_cast<unsigned int*>(swiglu_amax);
+  const int kstages = (p.ksteps_total + KSTEPS - 1) / KSTEPS;
+  // (runs of a grouped problem may start in the middle of a scale tile only in steps of 64 rows)
+  const int nt = groups != nullptr || M > 32 ? 64 : (M <= 16 ? 16 : 32);
+  p.splits = groups != nullptr ? 1 : skinny_splits(gated ? 2 * p.tiles : p.tiles, kstages, di);
+  if (gated && p.splits > 4) p.splits = 4;
+  const int csize = groups != nullptr ? 1 : p.splits * (gated ? 2 : 1);
+  long long grid = (long long)p.tiles * p.ngroups * csize;
+  // one CTA per item where several form a cluster; else persistent CTAs, two per SM
+  const long long slots = di.num_sms == di.all_sms ? 2LL * di.num_sms : di.num_sms;
+  if (csize == 1 && grid > slots) grid = slots;
+  if (gated) ARCQ_CUDA_TRY(cudaMemsetAsync(swiglu_amax, 0, sizeof(float) * p.ngroups, stream));
+  CUtensorMap mx, mw;
+  rc = make_operand_map(&mx, X, M, K_eff / 2, 16);
+  if (rc != ARCQ_OK) return rc;
+  rc = make_operand_map(&mw, W, N * p.ngroups, K_eff / 2, 128);
+  if (rc != ARCQ_OK) return rc;
+  if (groups != nullptr)
+    return gated ? launch_one<64, true, false>(mx, mw, p, (int)grid, stream) : launch_one<64, false, false>(mx, mw, p, (int)grid, stream);
+  if (nt == 16) return launch_nt<16>(mx, mw, p, gated, (int)grid, stream);
+  if (nt == 32) return launch_nt<32>(mx, mw, p, gated, (int)grid, stream);
+  return launch_nt<64>(mx, mw, p, gated, (int)grid, stream);
+}
+
+int skinny_plan_splits(int64_t N, int64_t K_eff) {
+  DeviceInfo di;
+  if (get_device_info(&di) != ARCQ_OK) return 1;
+  return skinny_splits((int)((N + 127) / 128), (int)((K_eff / 64 + KSTEPS - 1) / KSTEPS), di);
+}
+
+int skinny_poll_error() { return poll_tc_error(); }
+
+}  // namespace arcq

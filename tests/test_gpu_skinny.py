@@ -1,0 +1,130 @@
+"""The weight-streaming GEMM for few rows (arcq_skinny.cu): against the oracle's fp32 product rounded to the output
+type, at the edges of its token columns (16, 32, 64), of the 128-row weight tiles and of the K stages, split over a
+cluster or not; its residual and SwiGLU epilogues; grouped runs, more rows than one pass takes included."""
+import numpy as np
+import pytest
+import torch
+
+from arcquant_b200 import synth
+
+pytestmark = pytest.mark.gpu
+
+
+def _operands(m, n, kq, ke, seed):
+    from arcquant_b200.qlinear import NVFP4_reorder_quantize_w, NVFP4_reorder_quantize_x
+
+    x = synth.activations(m, kq, seed, synth.outlier_channels(kq, max(1, kq // 100), seed), device="cuda")
+    w = synth.weights(n, kq, seed + 1, device="cuda")
+    idx = torch.randperm(kq, generator=torch.Generator().manual_seed(seed)).to(torch.int16).cuda()
+    a, sfa, sx = NVFP4_reorder_quantize_x(x, idx, ke, mode=16)
+    b, sfb, sw = NVFP4_reorder_quantize_w(w, idx, ke, mode=16)
+    return a, sfa, sx, b, sfb, sw, x, w, idx
+
+
+def _oracle(a, sfa, b, sfb, alpha):
+    from oracle import oracle as O
+
+    ref = O.gemm_fast(a.cpu().numpy(), sfa.cpu().numpy(), b.cpu().numpy(), sfb.cpu().numpy(), alpha)
+    return torch.from_numpy(ref).to(torch.bfloat16).float()
+
+
+def _close(got, ref):
+    """An fp32 sum in another order moves an element by at most one bf16 step (2^-8) now and then."""
+    got = got.float().cpu()
+    assert torch.isfinite(got).all()
+    assert float((got - ref).norm() / ref.norm()) <= 1e-3
+    assert float((got == ref).float().mean()) >= 0.99
+
+
+@pytest.mark.parametrize("m,n,kq,ke", [(1, 8, 64, 0), (15, 136, 256, 64), (16, 4096, 4096, 128), (17, 1000, 1984, 64),
+                                        (32, 512, 2048, 64), (33, 2048, 1024, 128), (64, 6144, 4096, 128), (64, 24, 512, 512)])
+def test_few_rows_against_the_oracle(m, n, kq, ke):
+    from arcquant_b200 import _lib, ops
+
+    a, sfa, sx, b, sfb, sw, *_ = _operands(m, n, kq, ke, m + n)
+    guard = torch.full((m + 8, n), 7.0, dtype=torch.bfloat16, device="cuda")
+    L = _lib.load()
+    for _ in range(2):          # (reproducible: the split's partial sums are added in rank order)
+        rc = L.arcq_matmul_nvfp4_dev_alpha(a.data_ptr(), b.data_ptr(), sfa.data_ptr(), sfb.data_ptr(), m, n, kq + ke,
+                                           sx.data_ptr(), sw.data_ptr(), guard.data_ptr(),
+                                           torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        first = guard[:m].clone() if _ == 0 else first
+    torch.cuda.synchronize()
+    assert ops.gemm_poll_error() == 0
+    assert torch.equal(guard[:m], first) and bool((guard[m:] == 7.0).all())
+    _close(guard[:m], _oracle(a, sfa, b, sfb, float(sx * sw)))
+    res = (0.05 * torch.randn((m, n), generator=torch.Generator().manual_seed(9))).to(torch.bfloat16).cuda()
+    out = ops.matmul_residual(a, b, sfa, sfb, sx, sw, res)
+    assert torch.equal(out, res + first)
+    assert torch.equal(ops.matmul(a, b, sfa, sfb, float(sx * sw)), first) or m * n < 64
+
+
+@pytest.mark.parametrize("m,f,kq", [(1, 128, 256), (16, 2048, 1024), (20, 14336, 4096), (37, 384, 512), (64, 2048, 4096)])
+def test_few_rows_swiglu_equals_gemm_then_silu(m, f, kq):
+    from arcquant_b200 import ops
+
+    a, sfa, sx, _, _, _, x, _, idx = _operands(m, 16, kq, 64, m)
+    wg, wu = synth.weights(f, kq, 5, device="cuda"), synth.weights(f, kq, 6, device="cuda")
+    wcat = torch.cat([wg, wu], 0)
+    sw = torch.max(wcat).float() / 2688.0
+    b1, sfb1 = ops.reorder_quantize_w((wcat / sw).contiguous(), idx, 64)
+    b2, sfb2 = ops.reorder_quantize_w((ops.interleave_gate_up(wg, wu) / sw).contiguous(), idx, 64)
+    for factor in (1.0, 1e-30, 1e8):
+        sx2 = sx * factor
+        want, amax_w = ops.silu_mul(ops.matmul_dev_alpha(a, b1, sfa, sfb1, sx2, sw))
+        got, amax_g = ops.matmul_swiglu(a, b2, sfa, sfb2, sx2, sw)
+        if factor == 1.0:
+            _close(got, want.float().cpu())
+            assert abs(float(amax_g) - float(amax_w)) <= float(amax_w) * 2.0 ** -7
+        assert float(amax_g) == float(got.abs().max()) or bool(got.isnan().any())
+    assert ops.gemm_poll_error() == 0
+
+
+@pytest.mark.parametrize("counts", [(5, 0, 17, 1), (0, 0, 0, 3), (64, 65, 0, 1), (130, 0, 2, 1)])
+def test_grouped_few_rows_equal_the_per_run_calls(counts):
+    """(130 rows: three passes of 64 columns, the second of them starting in the middle of a scale tile)"""
+    from arcquant_b200 import ops
+    from arcquant_b200.qlinear import NVFP4_reorder_quantize_w
+
+    e, kq, ke, n = len(counts), 1024, 64, 512
+    k_eff = kq + ke
+    idx = torch.stack([torch.randperm(kq, generator=torch.Generator().manual_seed(i)) for i in range(e)]).to(torch.int16).cuda()
+    ws = [NVFP4_reorder_quantize_w(synth.weights(n, kq, 40 + i, device="cuda"), idx[i], ke, mode=16) for i in range(e)]
+    B, sw = torch.cat([w[0] for w in ws]), torch.stack([w[2] for w in ws])
+    span = (n // 128) * ((k_eff // 16 + 3) // 4) * 512
+    SFB = torch.cat([w[1][:span] for w in ws])
+    starts, at = [], 0
+    for c in counts:
+        starts.append(at)
+        at += (c + 255) // 256 * 256
+    total = sum(counts)
+    bound = (total + 255) // 256 * 256 + e * 256
+    groups = torch.tensor(starts + list(counts), dtype=torch.int32, device="cuda")
+    tile_group = torch.full((bound // 256,), -1, dtype=torch.int32)
+    row_map = torch.zeros(bound, dtype=torch.int32)
+    k = 0
+    for i, (s, c) in enumerate(zip(starts, counts)):
+        tile_group[s // 256:(s + c + 255) // 256] = i
+        row_map[s:s + c] = torch.arange(k, k + c).int()
+        k += c
+    tile_group, row_map = tile_group.cuda(), row_map.cuda()
+    x = synth.activations(total, kq, 5, synth.outlier_channels(kq, 10, 2), device="cuda")
+    sx = ops.absmax_grouped(x, row_map, groups, e) / 2688.0
+    a, sfa = ops.reorder_quantize_x_grouped(x, row_map, sx, idx, groups, bound, ke)
+    y, amax = ops.matmul_grouped_swiglu(a, B, sfa, SFB, tile_group, groups, e, n, sx, sw)
+    z = ops.matmul_grouped(a, B, sfa, SFB, tile_group, e, n, sx, sw)
+    torch.cuda.synchronize()
+    assert ops.gemm_poll_error() == 0
+    tile = ((k_eff // 16 + 3) // 4) * 512
+    for i, (s, c) in enumerate(zip(starts, counts)):
+        if c == 0:
+            assert float(amax[i]) == 0.0
+            continue
+        ai, sfi = a[s:s + c].contiguous(), sfa[(s // 128) * tile:].contiguous()
+        ref = _oracle(ai, sfi, ws[i][0], ws[i][1], float(sx[i] * sw[i]))
+        _close(z[s:s + c], ref)
+        g, u = ref.to(torch.bfloat16).reshape(c, n // 256, 2, 128).unbind(2)
+        want = torch.nn.functional.silu(g) * u
+        _close(y[s:s + c], want.reshape(c, n // 2).float())
+        assert float(amax[i]) == float(y[s:s + c].abs().max())

@@ -99,14 +99,9 @@ torch::Tensor matmul(const torch::Tensor& A, const torch::Tensor& B, const torch
   std::tie(M, N, K) = check_gemm_operands(A, B, SFA, SFB);
   c10::cuda::CUDAGuard guard(A.device());
   auto C = torch::empty({M, N}, torch::dtype(torch::kBFloat16).device(A.device()));
-  // problems with few tiles split K over idle SMs; above ARCQ_SKINNY_ROWS rows the fp32 partial sums need scratch
-  const int64_t ws_bytes = M <= ARCQ_SKINNY_ROWS ? 0 : static_cast<int64_t>(arcq_matmul_workspace_bytes(M, N, K));
-  torch::Tensor ws;
-  if (ws_bytes > 0) ws = torch::empty({ws_bytes}, torch::dtype(torch::kUInt8).device(A.device()));
   int status = arcq_matmul_nvfp4_ws(A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(),
                                     SFB.data_ptr<uint8_t>(), M, N, K, scale, nullptr, nullptr,
-                                    C.data_ptr<at::BFloat16>(), ws_bytes > 0 ? ws.data_ptr() : nullptr,
-                                    static_cast<size_t>(ws_bytes), current_stream(A));
+                                    C.data_ptr<at::BFloat16>(), nullptr, 0, current_stream(A));
   check_status(status, "matmul_host_nvfp4_bf16");
   return C;
 }
@@ -121,15 +116,10 @@ torch::Tensor matmul_dev_alpha(const torch::Tensor& A, const torch::Tensor& B, c
   if (alpha_b.has_value()) require_scalar_f32(*alpha_b, A, "alpha_b");
   c10::cuda::CUDAGuard guard(A.device());
   auto C = torch::empty({M, N}, torch::dtype(torch::kBFloat16).device(A.device()));
-  // problems with few tiles split K over idle SMs; above ARCQ_SKINNY_ROWS rows the fp32 partial sums need scratch
-  const int64_t ws_bytes = M <= ARCQ_SKINNY_ROWS ? 0 : static_cast<int64_t>(arcq_matmul_workspace_bytes(M, N, K));
-  torch::Tensor ws;
-  if (ws_bytes > 0) ws = torch::empty({ws_bytes}, torch::dtype(torch::kUInt8).device(A.device()));
   int status = arcq_matmul_nvfp4_ws(
       A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(), SFB.data_ptr<uint8_t>(), M, N, K, 1.0f,
       alpha_a.data_ptr<float>(), alpha_b.has_value() ? alpha_b->data_ptr<float>() : nullptr,
-      C.data_ptr<at::BFloat16>(), ws_bytes > 0 ? ws.data_ptr() : nullptr, static_cast<size_t>(ws_bytes),
-      current_stream(A));
+      C.data_ptr<at::BFloat16>(), nullptr, 0, current_stream(A));
   check_status(status, "matmul_host_nvfp4_bf16");
   return C;
 }

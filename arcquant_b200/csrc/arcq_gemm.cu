@@ -57,8 +57,6 @@ struct GemmParams {
   int natoms;         // ceil((K_eff/16)/4): scale atoms per 128-row tile
   int tiles_m, tiles_n;
   int sfb_tiles;      // ceil(N/128): 128-row scale tiles of B that exist
-  float* ws;          // split-K: fp32 partial sums [splits][M][N] (scratch), else nullptr
-  int splits;         // K is cut into this many ranges of whole stages (1 = no split)
 };
 
 // Instruction descriptor of kind::mxf4nvf4 block-scaled MMA: e2m1 x e2m1 (format id 1), ue4m3
@@ -107,22 +105,18 @@ arcq_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   const uint32_t tmem_base = misc[0];
   const uint32_t tmem_sf = tmem_base + BN;   // two stage-parity buffers of SF_COLS columns each
 
-  // A work item is (output tile, K range).  Without split-K there is one range per tile.
-  const int num_tiles = p.tiles_m * p.tiles_n * p.splits;
-  const int kstages_all = (p.ksteps_total + KSTEPS - 1) / KSTEPS;
-  const int kstages_per = (kstages_all + p.splits - 1) / p.splits;
+  const int num_tiles = p.tiles_m * p.tiles_n;
+  const int kstages = (p.ksteps_total + KSTEPS - 1) / KSTEPS;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
     if (lane == 0) {
       uint32_t it = 0;
       bool ok = true;
-      for (int item = blockIdx.x; item < num_tiles && ok; item += gridDim.x) {
-        const int tile = item / p.splits, split = item - tile * p.splits;
+      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;
         const int rtb = (tn * BN) / 128;   // first 128-row scale tile of B this output tile touches
-        const int ks_end = min(kstages_all, (split + 1) * kstages_per);
-        for (int ks = split * kstages_per; ks < ks_end; ++ks, ++it) {
+        for (int ks = 0; ks < kstages; ++ks, ++it) {
           const int s = it % C::STAGES;
           const uint32_t ph = (it / C::STAGES) & 1u;
           if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag)) { ok = false; break; }
@@ -154,17 +148,15 @@ arcq_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       constexpr uint32_t idesc = instr_desc<BN>();
       uint32_t it = 0, tile_it = 0;
       bool ok = true;
-      for (int item = blockIdx.x; item < num_tiles && ok; item += gridDim.x, ++tile_it) {
-        const int tile = item / p.splits, split = item - tile * p.splits;
+      for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++tile_it) {
         const int tn = tile / p.tiles_m;
-        const int ks_begin = split * kstages_per, ks_end = min(kstages_all, (split + 1) * kstages_per);
         // sub-atom column offset when BN = 64: rows 32j..32j+31 of an atom live in TMEM column j, so
         // the upper half of a 128-row scale atom starts two columns in.  (Tiles narrower than 64
         // would need an odd column offset, which the block-scaled MMA rejects as misaligned.)
         const uint32_t sfb_sub = (BN < 128) ? (uint32_t)(((tn * BN) % 128) / 32) : 0u;
         if (!mbar_wait(tmem_empty_bar, (tile_it & 1u) ^ 1u, abort_flag)) { ok = false; break; }
         tc_fence_after();
-        for (int ks = ks_begin; ks < ks_end; ++ks, ++it) {
+        for (int ks = 0; ks < kstages; ++ks, ++it) {
           const int s = it % C::STAGES;
           const uint32_t ph = (it / C::STAGES) & 1u;
           if (!mbar_wait(full_bar(s), ph, abort_flag)) { ok = false; break; }
@@ -186,7 +178,7 @@ arcq_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
             const uint64_t adesc = smem_desc(a_s + k * 32, 1024, LAYOUT_SW128);
             const uint64_t bdesc = smem_desc(b_s + k * 32, 1024, LAYOUT_SW128);
             tc_mma_nvf4(tmem_base, adesc, bdesc, idesc, t_sfa + k * 4, t_sfb + k * 4 * C::NB + sfb_sub,
-                        ((ks - ks_begin) | k) ? 1u : 0u);
+                        (ks | k) ? 1u : 0u);
           }
           tc_commit(empty_bar(s));   // stage reusable once these MMAs have read it
         }
@@ -201,8 +193,7 @@ arcq_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     if (p.alpha_b) alpha *= __ldg(p.alpha_b);
     uint32_t tile_it = 0;
     bool ok = true;
-    for (int item = blockIdx.x; item < num_tiles && ok; item += gridDim.x, ++tile_it) {
-      const int tile = item / p.splits, split = item - tile * p.splits;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x, ++tile_it) {
       const int tm = tile % p.tiles_m, tn = tile / p.tiles_m;
       ok = mbar_wait(tmem_full_bar, tile_it & 1u, abort_flag);
       ok = __all_sync(0xffffffffu, ok);   // keep the warp converged for the .sync.aligned loads
@@ -216,16 +207,7 @@ arcq_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         tc_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, r);
         tc_wait_ld();
         const int col = tn * BN + c0;
-        if (p.ws != nullptr) {
-          // split-K: raw fp32 partial sums of this K range; the reduction kernel applies alpha
-          if (row < p.M && col < p.N) {
-            float* wrow = p.ws + ((size_t)split * p.M + row) * p.N + col;
-#pragma unroll
-            for (int v = 0; v < 8; ++v)
-              if (col + v * 4 < p.N)   // N is a multiple of 8, so groups of four are in or out
-                *reinterpret_cast<uint4*>(wrow + v * 4) = make_uint4(r[v * 4], r[v * 4 + 1], r[v * 4 + 2], r[v * 4 + 3]);
-          }
-        } else if (row < p.M && col < p.N) {
+        if (row < p.M && col < p.N) {
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
             if (col + v * 8 < p.N) {   // N is a multiple of 8: whole 16-byte pieces are in or out
@@ -737,29 +719,6 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   }
 }
 
-// Sum of the split-K partials in a fixed order, times alpha, to bf16.  Eight outputs per thread.
-__global__ void arcq_splitk_reduce_kernel(const float* __restrict__ ws, int splits, long long mn, float alpha,
-                                          const float* alpha_a, const float* alpha_b, __nv_bfloat16* __restrict__ c) {
-  if (alpha_a) alpha *= __ldg(alpha_a);
-  if (alpha_b) alpha *= __ldg(alpha_b);
-  const long long nvec = mn / 8;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (int s = 0; s < splits; ++s) {
-      const float4* src = reinterpret_cast<const float4*>(ws + (size_t)s * mn + i * 8);
-      const float4 a = src[0], b = src[1];
-      acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
-      acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
-    }
-    uint4 o;
-    o.x = pack_bf16x2(acc[0] * alpha, acc[1] * alpha);
-    o.y = pack_bf16x2(acc[2] * alpha, acc[3] * alpha);
-    o.z = pack_bf16x2(acc[4] * alpha, acc[5] * alpha);
-    o.w = pack_bf16x2(acc[6] * alpha, acc[7] * alpha);
-    reinterpret_cast<uint4*>(c)[i] = o;
-  }
-}
-
 // ----------------------------------------------------------------------------- host side
 
 // Scale-factor buffer as a 2-D tensor of 32-bit words: one row per 512-byte atom; box = four atoms
@@ -878,7 +837,7 @@ int launch_bn(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int nu
   auto kern = arcq_gemm_kernel<BN>;
   ARCQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES));
   p.tiles_n = (p.N + BN - 1) / BN;
-  long long tiles = (long long)p.tiles_m * p.tiles_n * p.splits;
+  long long tiles = (long long)p.tiles_m * p.tiles_n;
   int grid = (int)(tiles < num_sms ? tiles : num_sms);
   kern<<<grid, NUM_THREADS, C::SMEM_BYTES, stream>>>(ma, mb, p);
   ARCQ_CUDA_TRY(cudaGetLastError());
@@ -887,7 +846,9 @@ int launch_bn(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int nu
 
 }  // namespace
 
-// Narrowest tile width and K split the launcher would use for a skinny problem.
+// Scratch for partial sums (see gemm_workspace_bytes) and tile width of the single-CTA kernel, by the cost model of a
+// single row of tiles (microseconds: ~5 fixed, 0.35 + 0.65 * bn/256 per stage, 2 + 0.35 per MB of partial sums), among
+// the choices that fit one wave of CTAs and 8 MB.
 static void plan_splitk(int64_t M, int64_t N, int64_t K_eff, int num_sms, int* bn_out, int* splits_out,
                         bool allow_split = true) {
   const int tiles_m = (int)((M + BM - 1) / BM);
@@ -897,12 +858,6 @@ static void plan_splitk(int64_t M, int64_t N, int64_t K_eff, int num_sms, int* b
   const int kstages = (int)((K_eff / 64 + KSTEPS - 1) / KSTEPS);
   int splits = 1;
   if (tiles_m == 1) {
-    // One row of tiles (M <= 128: weight streaming).  The K loop is a serial chain of stages whose
-    // latency, not bandwidth, sets the time; splitting K shortens the chain at the price of a second
-    // kernel that adds the fp32 partial sums.  Pick tile width and split count by a small cost model
-    // fitted to measurements on B200 (microseconds: ~5 fixed, 0.35 + 0.65 * bn/256 per stage of the
-    // chain, 2 + 0.35 per MB of partial sums when split), among the choices that fit one wave of CTAs
-    // and 8 MB of scratch.  Measured: N 6144, M 16: 15.4 -> 9.6 us; N 4096 / K 14464, M 16: 24.7 -> 13.4 us.
     double best = 1e30;
     int best_bn = 64, best_splits = 1;
     for (int cand = 64; cand <= 256; cand <<= 1) {
@@ -933,6 +888,20 @@ static void plan_splitk(int64_t M, int64_t N, int64_t K_eff, int num_sms, int* b
   *splits_out = splits;
 }
 
+// Weight streaming (arcq_skinny.cu): up to 64 rows, and as long as 128 x 128 tiles leave an SM for each, so that a cluster
+// of two or four can share a tile's K and the whole problem is one wave.  Measured, us (this kernel / the single-CTA
+// kernel with its partial sums in global memory, or CTA pairs where there are enough 256 x 256 tiles for them):
+//   [4096, 4224]   65 rows 8.1 / 11.7   200 rows 10.9 / 15.7   333 rows 12.1 / 27.7   512 rows 12.8 / 27.8
+//   [6144, 4224]  128 rows 11.0 / 16.3  200 rows 12.2 / 28.4   333 rows 13.1 / 14.3
+//   [4096, 14464] 128 rows 15.8 / 20.7  333 rows 22.7 / 81.8   512 rows 23.4 / 81.9
+// and beyond that line 777 rows of [4096, 4224] 21.1 / 14.3, [28672, 4224] 128 rows 24.5 / 22.4.
+static bool use_skinny_kernel(int64_t M, int64_t N, int num_sms) {
+  return M <= ARCQ_SKINNY_ROWS || ((M + 127) / 128) * ((N + 127) / 128) <= num_sms;
+}
+// With the SwiGLU epilogue (gate and up blocks in different CTAs of a cluster): [28672, 4224] 65 rows 24.8 / 30.9 us,
+// 128 rows 26.9 / 31.4, 200 rows 43.1 / 31.6.
+constexpr int64_t SKINNY_GATED_ROWS = 128;
+
 int launch_gemm_grouped(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,
                         int64_t N, int64_t K_eff, const int* tile_group, int ngroups, const float* alpha_a,
                         const float* alpha_b, void* Cout, cudaStream_t stream, float* swiglu_amax, const int* groups) {
@@ -948,10 +917,9 @@ int launch_gemm_grouped(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, 
   p.N = (int)N;
   p.ksteps_total = (int)(K_eff / 64);
   p.natoms = (int)((K_eff / 16 + 3) / 4);
-  p.splits = 1;
   // Few rows per matrix: the weight bytes are the time, and a 256-row tile holds mostly padding (see arcq_skinny.cu).
   // Of a grouped problem the host knows a bound, M = routed rows rounded up to a tile + a tile per matrix.
-  if (tile_group == nullptr && ngroups == 1 && swiglu_amax != nullptr && M <= ARCQ_SKINNY_ROWS)
+  if (tile_group == nullptr && ngroups == 1 && swiglu_amax != nullptr && M <= SKINNY_GATED_ROWS)
     return launch_gemm_skinny(A, B, SFA, SFB, M, N, K_eff, 1.0f, alpha_a, alpha_b, nullptr, Cout, swiglu_amax, nullptr, 1, stream);
   if (groups != nullptr && M - 256LL * ngroups <= 32LL * ngroups)
     return launch_gemm_skinny(A, B, SFA, SFB, M, N, K_eff, 1.0f, alpha_a, alpha_b, nullptr, Cout, swiglu_amax, groups, ngroups,
@@ -977,7 +945,6 @@ int launch_gemm_scatter(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, 
   p.N = (int)N;
   p.ksteps_total = (int)(K_eff / 64);
   p.natoms = (int)((K_eff / 16 + 3) / 4);
-  p.splits = 1;
   return launch_pair(A, B, SFA, SFB, M, N, K_eff, p, di.num_sms, stream, nullptr, 1, nullptr, nullptr, dests, ndests);
 }
 
@@ -986,11 +953,11 @@ int launch_gemm_scatter(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, 
 int launch_gemm_residual(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,
                          int64_t N, int64_t K_eff, const float* alpha_a, const float* alpha_b, const void* residual,
                          void* Cout, cudaStream_t stream) {
-  if (M <= ARCQ_SKINNY_ROWS)
-    return launch_gemm_skinny(A, B, SFA, SFB, M, N, K_eff, 1.0f, alpha_a, alpha_b, residual, Cout, nullptr, nullptr, 1, stream);
   DeviceInfo di;
   int rc = get_device_info(&di);
   if (rc != ARCQ_OK) return rc;
+  if (use_skinny_kernel(M, N, di.num_sms))
+    return launch_gemm_skinny(A, B, SFA, SFB, M, N, K_eff, 1.0f, alpha_a, alpha_b, residual, Cout, nullptr, nullptr, 1, stream);
   GemmParams p = {};
   p.c = static_cast<__nv_bfloat16*>(Cout);
   p.alpha_a = alpha_a;
@@ -1000,11 +967,11 @@ int launch_gemm_residual(const uint8_t* A, const uint8_t* B, const uint8_t* SFA,
   p.N = (int)N;
   p.ksteps_total = (int)(K_eff / 64);
   p.natoms = (int)((K_eff / 16 + 3) / 4);
-  p.splits = 1;
   return launch_pair(A, B, SFA, SFB, M, N, K_eff, p, di.num_sms, stream, nullptr, 1, nullptr, nullptr, nullptr, 0,
                      residual);
 }
 
+// What earlier versions put their partial sums in; no kernel touches it any more.
 size_t gemm_workspace_bytes(int64_t M, int64_t N, int64_t K_eff) {
   DeviceInfo di;
   if (get_device_info(&di) != ARCQ_OK) return 0;
@@ -1024,15 +991,14 @@ int gemm_plan(int64_t M, int64_t N, int64_t K_eff, int* kind, int* tile_n, int* 
   int rc = get_device_info(&di);
   if (rc != ARCQ_OK) return rc;
   int k = ARCQ_GEMM_KIND_SINGLE, bn = 256, sp = 1;
-  if (M <= ARCQ_SKINNY_ROWS) {
+  if (use_skinny_kernel(M, N, di.num_sms)) {
     k = ARCQ_GEMM_KIND_SKINNY;
     bn = 128;
-    sp = skinny_plan_splits(N, K_eff);
+    sp = skinny_plan_splits(M, N, K_eff);
   } else if (use_pair_kernel(M, N, di.num_sms)) {
     k = ARCQ_GEMM_KIND_PAIR;
   } else {
-    plan_splitk(M, N, K_eff, di.num_sms, &bn, &sp);
-    if (sp > 1) k = ARCQ_GEMM_KIND_SPLIT_K;
+    plan_splitk(M, N, K_eff, di.num_sms, &bn, &sp, false);
   }
   if (kind) *kind = k;
   if (tile_n) *tile_n = bn;
@@ -1041,13 +1007,12 @@ int gemm_plan(int64_t M, int64_t N, int64_t K_eff, int* kind, int* tile_n, int* 
 }
 
 int launch_gemm(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M, int64_t N,
-                int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, void* Cout,
-                void* workspace, size_t workspace_bytes, cudaStream_t stream) {
-  if (M <= ARCQ_SKINNY_ROWS)
-    return launch_gemm_skinny(A, B, SFA, SFB, M, N, K_eff, alpha, alpha_a, alpha_b, nullptr, Cout, nullptr, nullptr, 1, stream);
+                int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, void* Cout, cudaStream_t stream) {
   DeviceInfo di;
   int rc = get_device_info(&di);
   if (rc != ARCQ_OK) return rc;
+  if (use_skinny_kernel(M, N, di.num_sms))
+    return launch_gemm_skinny(A, B, SFA, SFB, M, N, K_eff, alpha, alpha_a, alpha_b, nullptr, Cout, nullptr, nullptr, 1, stream);
 
   GemmParams p;
   p.sfa = SFA;
@@ -1063,88 +1028,30 @@ int launch_gemm(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const ui
   p.tiles_m = (int)((M + BM - 1) / BM);
   p.tiles_n = 0;
   p.sfb_tiles = (int)((N + 127) / 128);
-  p.ws = nullptr;
-  p.splits = 1;
-
-  // Widest tile that still gives every SM work; narrow tiles for skinny problems.  Partial tiles
-  // are clipped by the TMA box (zero fill) and by the store guards.
-  int bn = 256;
-  while (bn > 64 && (long long)p.tiles_m * ((N + bn - 1) / bn) < di.num_sms) bn >>= 1;
-
   if (use_pair_kernel(M, N, di.num_sms)) return launch_pair(A, B, SFA, SFB, M, N, K_eff, p, di.num_sms, stream);
 
-  // Skinny problems (few output tiles, long K): split K over otherwise idle SMs when the caller
-  // provided scratch for the fp32 partial sums.
-  {
-    int bn2, splits;
-    plan_splitk(M, N, K_eff, di.num_sms, &bn2, &splits, workspace != nullptr);
-    if (splits > 1 && workspace_bytes < (size_t)splits * (size_t)M * (size_t)N * sizeof(float))
-      plan_splitk(M, N, K_eff, di.num_sms, &bn2, &splits, false);   // scratch too small: do not split
-    if (splits > 1 && workspace == nullptr) splits = 1;             // (never split without scratch)
-    if (splits > 1) {
-      bn = bn2;
-      p.ws = static_cast<float*>(workspace);
-      p.splits = splits;
-    } else if (p.tiles_m == 1) {
-      bn = bn2;   // single row of tiles: the cost model also picks the width of an unsplit launch
-    }
-  }
-
+  int bn, splits;
+  plan_splitk(M, N, K_eff, di.num_sms, &bn, &splits, false);
   CUtensorMap ma, mb;
   rc = make_operand_map(&ma, A, M, K_eff / 2, BM);
   if (rc != ARCQ_OK) return rc;
   rc = make_operand_map(&mb, B, N, K_eff / 2, bn);
   if (rc != ARCQ_OK) return rc;
-
   switch (bn) {
-    case 256: rc = launch_bn<256>(ma, mb, p, di.num_sms, stream); break;
-    case 128: rc = launch_bn<128>(ma, mb, p, di.num_sms, stream); break;
-    default: rc = launch_bn<64>(ma, mb, p, di.num_sms, stream); break;
+    case 256: return launch_bn<256>(ma, mb, p, di.num_sms, stream);
+    case 128: return launch_bn<128>(ma, mb, p, di.num_sms, stream);
+    default: return launch_bn<64>(ma, mb, p, di.num_sms, stream);
   }
-  if (rc != ARCQ_OK || p.splits == 1) return rc;
-  const long long mn = (long long)M * N;
-  long long blocks = (mn / 8 + 255) / 256;
-  if (blocks > (long long)di.num_sms * 8) blocks = (long long)di.num_sms * 8;
-  arcq_splitk_reduce_kernel<<<(unsigned)blocks, 256, 0, stream>>>(p.ws, p.splits, mn, alpha, alpha_a, alpha_b, p.c);
-  ARCQ_CUDA_TRY(cudaGetLastError());
-  return ARCQ_OK;
 }
 
 // ----------------------------------------------------------------------------- no-allocation entry point
 //
-// Scratch for arcq_matmul_nvfp4_static: a fixed block of device memory that is part of the loaded
-// library image (every GPU that loads libarcq.so carries these 2 MiB until the process exits).
-// In host code the name below is only a handle; the device address is looked up once per device
-// with cudaGetSymbolAddress and that address is what the kernels receive.
-constexpr size_t STATIC_SCRATCH_BYTES = (size_t)ARCQ_STATIC_SCRATCH_BYTES;
-static __device__ __align__(256) unsigned char g_static_scratch[STATIC_SCRATCH_BYTES];
-
-static int static_scratch_address(void** out) {
-  static std::mutex mu;
-  static void* addr[64] = {};
-  int dev = 0;
-  ARCQ_CUDA_TRY(cudaGetDevice(&dev));
-  if (dev < 0 || dev >= 64) return ARCQ_ERR_CUDA;
-  std::lock_guard<std::mutex> lock(mu);
-  if (addr[dev] == nullptr) {
-    void* ptr = nullptr;
-    ARCQ_CUDA_TRY(cudaGetSymbolAddress(&ptr, g_static_scratch));   // with device `dev` current
-    if (ptr == nullptr) return cuda_fail(cudaErrorInvalidSymbol);
-    addr[dev] = ptr;
-  }
-  *out = addr[dev];
-  return ARCQ_OK;
-}
-
+// No kernel needs scratch; the shapes that once needed more than the block inside the library are refused as before.
 int launch_gemm_static(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,
                        int64_t N, int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, void* Cout,
                        cudaStream_t stream) {
-  const size_t need = gemm_workspace_bytes(M, N, K_eff);
-  if (need > STATIC_SCRATCH_BYTES) return ARCQ_ERR_SCRATCH_LIMIT;
-  void* scratch = nullptr;
-  int rc = static_scratch_address(&scratch);
-  if (rc != ARCQ_OK) return rc;
-  return launch_gemm(A, B, SFA, SFB, M, N, K_eff, alpha, alpha_a, alpha_b, Cout, scratch, STATIC_SCRATCH_BYTES, stream);
+  if (gemm_workspace_bytes(M, N, K_eff) > (size_t)ARCQ_STATIC_SCRATCH_BYTES) return ARCQ_ERR_SCRATCH_LIMIT;
+  return launch_gemm(A, B, SFA, SFB, M, N, K_eff, alpha, alpha_a, alpha_b, Cout, stream);
 }
 
 int gemm_poll_error() {

@@ -48,14 +48,13 @@ int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight
                                  cudaStream_t stream, const int* groups = nullptr, int ngroups = 0,
                                  const int* row_map = nullptr);
 int launch_absmax(const void* x, int64_t n, float* out, int accumulate, cudaStream_t stream);
-// workspace (may be null): scratch for split-K partial sums, see gemm_workspace_bytes().
 int launch_gemm(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,
                 int64_t N, int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, void* C,
-                void* workspace, size_t workspace_bytes, cudaStream_t stream);
+                cudaStream_t stream);
 size_t gemm_workspace_bytes(int64_t M, int64_t N, int64_t K_eff);
 // Kernel choice for a shape (see arcq_matmul_plan).
 int gemm_plan(int64_t M, int64_t N, int64_t K_eff, int* kind, int* tile_n, int* splits);
-// Split-K GEMM whose scratch is the library's own static device array (no allocation anywhere).
+// launch_gemm for callers that must not allocate; refuses what gemm_workspace_bytes() puts above the documented limit.
 int launch_gemm_static(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,
                        int64_t N, int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, void* C,
                        cudaStream_t stream);
@@ -107,7 +106,7 @@ int silu_table_ptr(cudaStream_t stream, const uint16_t** out);
 int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, const uint8_t* SFW, int64_t M, int64_t N,
                        int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, const void* residual, void* C,
                        float* swiglu_amax, const int* groups, int ngroups, cudaStream_t stream);
-int skinny_plan_splits(int64_t N, int64_t K_eff);
+int skinny_plan_splits(int64_t M, int64_t N, int64_t K_eff);
 int skinny_poll_error();
 int gemm_poll_error();
 // Same for the bounded waits of the warp-specialised quantizer.

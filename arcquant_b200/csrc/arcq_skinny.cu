@@ -1,7 +1,7 @@
-// Block-scaled NVFP4 GEMM for few rows of A (decoding, experts with a handful of tokens): weight streaming.
+// Block-scaled NVFP4 GEMM for few rows of A (decoding, short prompts, experts with a handful of tokens): weight streaming.
 //
 // Bound: HBM, by the packed weight (N * K_eff * 9/16 bytes); the products are a rounding error.  So the operands
-// change sides: 128 rows of the WEIGHT are the M side of the MMA and the tokens its N side (16 to 64 columns), so
+// change sides: 128 rows of the WEIGHT are the M side of the MMA and the tokens its N side (16 to 128 columns), so
 // that a stage of the ring is weight (16 KB of codes + 2 KB of scales for K = 256) and little else, and the whole
 // chip's shared memory is a window of weight bytes in flight: two CTAs per SM, three to five stages each.
 //  * K is split over the CTAs of a cluster (up to eight) where N alone gives too few CTAs.  Every CTA pushes its fp32
@@ -33,15 +33,20 @@ constexpr int SK_SF_COLS = 2 * KSTEPS * 4;      // tensor-memory columns of one 
 template <int NT, int NA, bool SPLIT>
 struct SkCfg {
   static constexpr int X_BYTES = NT * BK_BYTES;
+  static constexpr int XBOX = NT > 64 ? 32 : 16;                       // rows of A per TMA box
+  // Up to 64 columns the partial sums have memory of their own and are pushed there; 128 columns (64 KB) take the ring's
+  // place once the CTA's products are complete, and their owners pull them.
+  static constexpr bool PULL = SPLIT && NT > 64;
   static constexpr int STAGE_BYTES = SK_W_BYTES + X_BYTES + 2 * SK_SF_BYTES;
   static constexpr int BAR_BYTES = 256;
-  static constexpr int PART_BYTES = SPLIT ? NA * (NT + 7) * 512 : 0;   // (tokens rounded up to the cluster, at most eight)
+  static constexpr int PART_BYTES = SPLIT && !PULL ? NA * (NT + 7) * 512 : 0;   // (tokens rounded up to the cluster, at most eight)
   static constexpr int FIT = (113 * 1024 - 1024 - BAR_BYTES - PART_BYTES) / STAGE_BYTES;
   static constexpr int STAGES = FIT < 5 ? FIT : 5;
   static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + PART_BYTES + BAR_BYTES;
   static constexpr int TMEM_NEED = NA * NT + STAGES * SK_SF_COLS;
   static constexpr int TMEM_COLS = TMEM_NEED <= 128 ? 128 : 256;
   static_assert(STAGES >= 2 && TMEM_NEED <= 256, "two CTAs share 512 columns of tensor memory");
+  static_assert(!PULL || (NA == 1 && STAGES * STAGE_BYTES >= NT * 512), "the partial sums fit the ring");
 };
 
 struct SkinnyParams {
@@ -55,7 +60,8 @@ struct SkinnyParams {
   int M, N;
   int ksteps_total;                  // K_eff / 64
   int natoms;                        // scale atoms per 128-row tile
-  int tiles;                         // work items per matrix: ceil(N / 128), halved with SwiGLU
+  int tiles;                         // weight tiles per matrix: ceil(N / 128), halved with SwiGLU
+  int ttiles;                        // token tiles of NT rows (1 for grouped problems, which take their rows NT at a time)
   int sfw_tiles;                     // 128-row scale tiles of all matrices
   int splits;                        // K ranges = CTAs per cluster
   const int* groups;                 // run table of a grouped problem (device) or nullptr
@@ -81,6 +87,11 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
 }
 __device__ __forceinline__ void st_cluster_f32(uint32_t addr, uint32_t v) {
   asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
 }
 __device__ __forceinline__ float bf16_round(float v) {
   return __uint_as_float((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v)) << 16);
@@ -111,6 +122,7 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   const uint32_t acc_full_bar = bar_base + 8u * (3 * C::STAGES), acc_empty_bar = acc_full_bar + 8u;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
+  const int ttiles = NT > 64 ? p.ttiles : 1;           // (a constant up to 64 rows: four divisions less before the first load)
   const int kstages = (p.ksteps_total + KSTEPS - 1) / KSTEPS;
   const int csize = SPLIT ? p.splits * NB : 1;                         // CTAs per cluster
   const int rank = SPLIT ? (int)(blockIdx.x % csize) : 0;
@@ -118,10 +130,10 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   const int block = SPLIT ? rank / splits : 0;                         // SwiGLU: 0 = gate, 1 = up
   const int ks_begin = kstages * split / splits, ks_end = kstages * (split + 1) / splits;
   const int first_item = (int)(blockIdx.x / csize), item_step = (int)(gridDim.x / csize);
-  const int num_items = p.tiles * p.ngroups;
+  const int num_items = p.tiles * p.ngroups * ttiles;                // token tiles of one weight tile are neighbours
   // first weight row of accumulator a of work item `item`, in the stacked matrices
   auto weight_row = [&](int item, int a) {
-    const int g = item / p.tiles, t = item - g * p.tiles;
+    const int wt = item / ttiles, g = wt / p.tiles, t = wt - g * p.tiles;
     return g * p.N + t * (128 * NB) + 128 * (block + a);
   };
 
@@ -150,14 +162,23 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  // A CTA's shared memory may be written by its cluster only once it has started: the other half of this barrier is in
+  // front of the first such store (waiting here cost 0.6 us a call at 1 to 16 rows).
+  if (SPLIT) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+  bool met = false;
+  auto meet = [&]() {
+    if (SPLIT && !met) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    met = true;
+  };
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");   // (every thread: everything below reads or writes global memory)
   const uint32_t tmem_base = misc[0];
   const uint32_t tmem_sf = tmem_base + NA * NT;
 
-  // rows of matrix g: first row in A / C, number
-  auto run_of = [&](int g, int& row0, int& cnt) {
-    if (p.groups == nullptr) { row0 = 0; cnt = p.M; return; }
+  // rows of a work item: first row in A / C, number
+  auto run_of = [&](int item, int& row0, int& cnt) {
+    if (p.groups == nullptr) { row0 = (item % ttiles) * NT; cnt = min(NT, p.M - row0); return; }
+    const int g = item / p.tiles;
     row0 = __ldg(p.groups + g);
     cnt = __ldg(p.groups + p.ngroups + g);
   };
@@ -169,9 +190,9 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       bool ok = true;
       for (int item = first_item; item < num_items && ok; item += item_step) {
         int row0, cnt;
-        run_of(item / p.tiles, row0, cnt);
+        run_of(item, row0, cnt);
         for (int c0 = 0; c0 < cnt && ok; c0 += NT) {
-          const int boxes = (min(NT, cnt - c0) + 15) >> 4;               // 16 rows of A each
+          const int boxes = (min(NT, cnt - c0) + C::XBOX - 1) / C::XBOX;
           const int xt = (row0 + c0) >> 7;                               // 128-row scale tile of these rows
           for (int ai = 0; ai < NA && ok; ++ai) {
             const int wrow = weight_row(item, ai), wt = wrow >> 7;
@@ -181,11 +202,11 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
               const uint32_t sf_bytes = (uint32_t)min(KSTEPS, p.ksteps_total - ks * KSTEPS) * ATOM;
               const uint32_t st = base + s * C::STAGE_BYTES, x_s = st + SK_W_BYTES, sfw_s = x_s + C::X_BYTES, sfx_s = sfw_s + SK_SF_BYTES;
               mbar_expect_tx(sf_bar(s), 2u * sf_bytes);
-              mbar_expect_tx(full_bar(s), SK_W_BYTES + (uint32_t)boxes * 2048u);
+              mbar_expect_tx(full_bar(s), SK_W_BYTES + (uint32_t)(boxes * C::XBOX * BK_BYTES));
               bulk_load(sfw_s, p.sfw + ((size_t)wt * p.natoms + (size_t)ks * KSTEPS) * ATOM, sf_bytes, sf_bar(s));
               bulk_load(sfx_s, p.sfx + ((size_t)xt * p.natoms + (size_t)ks * KSTEPS) * ATOM, sf_bytes, sf_bar(s));
               tma_load_2d(st, &map_w, full_bar(s), ks * BK_BYTES, wrow);
-              for (int b = 0; b < boxes; ++b) tma_load_2d(x_s + b * 2048, &map_x, full_bar(s), ks * BK_BYTES, row0 + c0 + 16 * b);
+              for (int b = 0; b < boxes; ++b) tma_load_2d(x_s + b * (C::XBOX * BK_BYTES), &map_x, full_bar(s), ks * BK_BYTES, row0 + c0 + C::XBOX * b);
             }
           }
         }
@@ -206,7 +227,7 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       bool ok = true;
       for (int item = first_item; item < num_items && ok; item += item_step) {
         int row0, cnt;
-        run_of(item / p.tiles, row0, cnt);
+        run_of(item, row0, cnt);
         for (int c0 = 0; c0 < cnt && ok; c0 += NT, ++acc_it) {
           const uint32_t ncols = (uint32_t)((min(NT, cnt - c0) + 15) & ~15);
           // e2m1 x e2m1, ue4m3 scales, K-major operands (see arcq_gemm.cu), N = ncols, M = 128
@@ -247,9 +268,9 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     uint32_t acc_it = 0;
     bool ok = true;
     for (int item = first_item; item < num_items && ok; item += item_step) {
-      const int g = item / p.tiles, t = item - g * p.tiles;
+      const int wt = item / ttiles, g = wt / p.tiles, t = wt - g * p.tiles;
       int row0, cnt;
-      run_of(g, row0, cnt);
+      run_of(item, row0, cnt);
       float alpha = p.alpha;
       if (p.alpha_a) alpha *= __ldg(p.alpha_a + g);
       if (p.alpha_b) alpha *= __ldg(p.alpha_b + g);
@@ -259,9 +280,20 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         if (!ok) break;
         tc_fence_after();
         const int here = min(NT, cnt - c0);
-        if (SPLIT) {
+        if (C::PULL) {
+          // fp32 partial sums in place of the ring (every product that reads it is complete): [token][128]
+          for (int j0 = 0; j0 < here; j0 += 16) {
+            uint32_t v[16];
+            tc_ld16(t_row + j0, v);
+            tc_wait_ld();
+            float* dst = reinterpret_cast<float*>(base_ptr) + j0 * 128 + nl;
+#pragma unroll
+            for (int j = 0; j < 16; ++j) dst[j * 128] = __uint_as_float(v[j]);
+          }
+        } else if (SPLIT) {
           // fp32 partial sums to the CTAs that own the tokens: token j belongs to rank j % csize, where it is
           // number j / csize; layout there: [token number][source rank][128]
+          meet();
           uint32_t dst[8];
 #pragma unroll
           for (int r = 0; r < 8; ++r) dst[r] = cluster_addr(part_base, (uint32_t)min(r, csize - 1));
@@ -329,7 +361,7 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     bool ok = true;
     for (int item = first_item; item < num_items && ok; item += item_step) {
       int row0, cnt;
-      run_of(item / p.tiles, row0, cnt);
+      run_of(item, row0, cnt);
       for (int c0 = 0; c0 < cnt && ok; c0 += NT) {
         const bool upper = ((row0 + c0) & 64) != 0;        // rows 64.. of a 128-row scale tile: words 2 and 3 of the atoms
         for (int n = NA * (ks_end - ks_begin); n > 0; --n, ++it) {
@@ -364,9 +396,12 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   tc_fence_before();
   if (SPLIT) {
     // ------------------------------------------------------------------ the cluster's partial sums
+    meet();
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (*abort_flag == 0) {
-      const int t = first_item;
+      const int t = first_item / ttiles;
+      int row0, cnt;
+      run_of(first_item, row0, cnt);
       const int ncols = GATED ? p.N >> 1 : p.N;
       float alpha = p.alpha;
       if (p.alpha_a) alpha *= __ldg(p.alpha_a);
@@ -376,13 +411,15 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       // four neighbouring columns of one of this CTA's tokens per thread and step
       for (int i = threadIdx.x;; i += SK_THREADS) {
         const int num = i >> 5, tok = num * csize + rank, n4 = (i & 31) * 4;
-        if (tok >= p.M) break;
+        if (tok >= cnt) break;
         float v[NB][4];
 #pragma unroll
         for (int a = 0; a < NB; ++a) {
           float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
           for (int r = 0; r < splits; ++r) {
-            const float4 q = part[(num * csize + a * splits + r) * 32 + (i & 31)];
+            float4 q;
+            if (C::PULL) q = ld_cluster_f4(cluster_addr(base + (uint32_t)(tok * 512 + n4 * 4), (uint32_t)(a * splits + r)));
+            else q = part[(num * csize + a * splits + r) * 32 + (i & 31)];
             sum.x += q.x; sum.y += q.y; sum.z += q.z; sum.w += q.w;
           }
           v[a][0] = sum.x; v[a][1] = sum.y; v[a][2] = sum.z; v[a][3] = sum.w;
@@ -390,7 +427,7 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         const int n = t * 128 + n4;
         if (n < ncols) {                                   // (a multiple of four columns is in or out: N % 8 == 0)
           float o[4];
-          const size_t at = (size_t)tok * ncols + n;
+          const size_t at = (size_t)(row0 + tok) * ncols + n;
           uint2 res = make_uint2(0, 0);
           if (!GATED && p.residual != nullptr) res = *reinterpret_cast<const uint2*>(p.residual + at);
           const uint32_t rw[2] = {res.x, res.y};
@@ -414,6 +451,10 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         for (int d = 16; d > 0; d >>= 1) mi = max(mi, __shfl_xor_sync(0xffffffffu, mi, d));
         if (lane == 0 && mi) atomicMax(p.amax, mi);
       }
+    }
+    if (C::PULL) {       // nobody's partial sums go away while another CTA reads them
+      __syncwarp();
+      asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     }
   } else {
     __syncthreads();
@@ -472,6 +513,17 @@ static int skinny_splits(int tiles, int kstages, const DeviceInfo& di) {
   if (s > kstages / 2) s = kstages / 2;
   return s < 1 ? 1 : s;
 }
+// The same for tiles of 128 token columns, whose stages take two to three times as long.  Clusters of two and four only: of
+// three or six, CTAs that would fit one by one do not fit the chip at once ([4096, 4224], 333 rows, us: unsplit 20.4, two
+// ranges = 192 CTAs 12.2, three = 288 CTAs 19.1; 200 rows: two 11.6, three 11.3, four = 256 CTAs 10.9, six 19.5).
+static int skinny_splits_wide(int tiles, int kstages, const DeviceInfo& di) {
+  const bool all = di.num_sms == di.all_sms;
+  int s = 1;
+  if (2LL * tiles <= (all ? 2 * di.num_sms : di.num_sms)) s = 2;
+  if (4LL * tiles <= (all ? di.num_sms * 7 / 4 : di.num_sms)) s = 4;
+  while (s > 1 && s > kstages / 2) s >>= 1;
+  return s;
+}
 // See SkinnyParams; `residual` and `swiglu_amax` exclude each other; groups (device) with ngroups matrices stacked in W.
 int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, const uint8_t* SFW, int64_t M, int64_t N,
                        int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, const void* residual, void* C,
@@ -498,17 +550,19 @@ int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, c
   p.amax = reinterpret_cast<unsigned int*>(swiglu_amax);
   const int kstages = (p.ksteps_total + KSTEPS - 1) / KSTEPS;
   // (runs of a grouped problem may start in the middle of a scale tile only in steps of 64 rows)
-  const int nt = groups != nullptr || M > 32 ? 64 : (M <= 16 ? 16 : 32);
-  p.splits = groups != nullptr ? 1 : skinny_splits(gated ? 2 * p.tiles : p.tiles, kstages, di);
+  const int nt = groups != nullptr ? 64 : (M > 64 ? 128 : (M > 32 ? 64 : (M <= 16 ? 16 : 32)));
+  p.ttiles = groups != nullptr ? 1 : (int)((M + nt - 1) / nt);
+  const int blocks = (gated ? 2 * p.tiles : p.tiles) * p.ttiles;
+  p.splits = groups != nullptr ? 1 : (nt > 64 ? skinny_splits_wide(blocks, kstages, di) : skinny_splits(blocks, kstages, di));
   if (gated && p.splits > 4) p.splits = 4;
   const int csize = groups != nullptr ? 1 : p.splits * (gated ? 2 : 1);
-  long long grid = (long long)p.tiles * p.ngroups * csize;
+  long long grid = (long long)p.tiles * p.ngroups * p.ttiles * csize;
   // one CTA per item where several form a cluster; else persistent CTAs, two per SM
   const long long slots = di.num_sms == di.all_sms ? 2LL * di.num_sms : di.num_sms;
   if (csize == 1 && grid > slots) grid = slots;
   if (gated) ARCQ_CUDA_TRY(cudaMemsetAsync(swiglu_amax, 0, sizeof(float) * p.ngroups, stream));
   CUtensorMap mx, mw;
-  rc = make_operand_map(&mx, X, M, K_eff / 2, 16);
+  rc = make_operand_map(&mx, X, M, K_eff / 2, nt > 64 ? 32 : 16);
   if (rc != ARCQ_OK) return rc;
   rc = make_operand_map(&mw, W, N * p.ngroups, K_eff / 2, 128);
   if (rc != ARCQ_OK) return rc;
@@ -516,13 +570,15 @@ int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, c
     return gated ? launch_one<64, true, false>(mx, mw, p, (int)grid, stream) : launch_one<64, false, false>(mx, mw, p, (int)grid, stream);
   if (nt == 16) return launch_nt<16>(mx, mw, p, gated, (int)grid, stream);
   if (nt == 32) return launch_nt<32>(mx, mw, p, gated, (int)grid, stream);
-  return launch_nt<64>(mx, mw, p, gated, (int)grid, stream);
+  if (nt == 64) return launch_nt<64>(mx, mw, p, gated, (int)grid, stream);
+  return launch_nt<128>(mx, mw, p, gated, (int)grid, stream);
 }
 
-int skinny_plan_splits(int64_t N, int64_t K_eff) {
+int skinny_plan_splits(int64_t M, int64_t N, int64_t K_eff) {
   DeviceInfo di;
   if (get_device_info(&di) != ARCQ_OK) return 1;
-  return skinny_splits((int)((N + 127) / 128), (int)((K_eff / 64 + KSTEPS - 1) / KSTEPS), di);
+  const int tiles = (int)((N + 127) / 128), kstages = (int)((K_eff / 64 + KSTEPS - 1) / KSTEPS);
+  return M > 64 ? skinny_splits_wide(tiles * (int)((M + 127) / 128), kstages, di) : skinny_splits(tiles, kstages, di);
 }
 
 int skinny_poll_error() { return poll_tc_error(); }

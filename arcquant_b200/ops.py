@@ -180,13 +180,10 @@ def _matmul(a, b, sfa, sfb, alpha: float, alpha_a, alpha_b) -> torch.Tensor:
         raise RuntimeError("A and B disagree on K")
     c = torch.empty((m, n), dtype=torch.bfloat16, device=a.device)
     with torch.cuda.device(a.device):
-        # problems with few tiles split K over idle SMs; above SKINNY_ROWS rows the fp32 partial sums need scratch
-        ws_bytes = 0 if m <= _lib.SKINNY_ROWS else int(lib.arcq_matmul_workspace_bytes(m, n, kb * 2))
-        ws = torch.empty((ws_bytes,), dtype=torch.uint8, device=a.device) if ws_bytes else None
         rc = lib.arcq_matmul_nvfp4_ws(a.data_ptr(), b.data_ptr(), sfa.data_ptr(), sfb.data_ptr(), m, n, kb * 2,
                                       float(alpha), None if alpha_a is None else alpha_a.data_ptr(),
-                                      None if alpha_b is None else alpha_b.data_ptr(), c.data_ptr(),
-                                      None if ws is None else ws.data_ptr(), ws_bytes, _stream())
+                                      None if alpha_b is None else alpha_b.data_ptr(), c.data_ptr(), None, 0,
+                                      _stream())
     _lib.check(rc, f"matmul M={m} N={n} K={kb * 2}")
     return c
 

@@ -150,13 +150,12 @@ int arcq_matmul_nvfp4_dev_alpha(const uint8_t* A, const uint8_t* B, const uint8_
                                 int64_t M, int64_t N, int64_t K_eff, const float* alpha_a,
                                 const float* alpha_b, void* C, void* stream);
 
-/* Problems with few output tiles and a long K run faster when K is split over the idle SMs.  Up to ARCQ_SKINNY_ROWS
- * rows the partial sums are exchanged on chip; above, the split needs scratch for them.
- * arcq_matmul_workspace_bytes: how much scratch a split over global memory takes for this shape on the
- * current device (0 = the shape is not split); up to ARCQ_SKINNY_ROWS rows it is not touched.  arcq_matmul_nvfp4_ws: arcq_matmul_nvfp4 /
- * _dev_alpha (alpha = alpha * *alpha_a * *alpha_b, the pointers may be NULL) with caller-provided
- * scratch; with workspace == NULL or too small it behaves exactly like arcq_matmul_nvfp4.  The
- * partials are summed in a fixed order, so results are reproducible.  Same reference interface
+/* Problems with few output tiles run faster when K is split over the idle SMs.  The partial sums are exchanged on chip
+ * and added in a fixed order, so results are reproducible; no call needs scratch.
+ * arcq_matmul_workspace_bytes: the scratch that a split over global memory would take for this shape on the current
+ * device (0 = none); callers that provide it may go on doing so.  arcq_matmul_nvfp4_ws: arcq_matmul_nvfp4 /
+ * _dev_alpha (alpha = alpha * *alpha_a * *alpha_b, the pointers may be NULL); the workspace may be NULL and is not
+ * touched.  Same reference interface
  * as arcq_matmul_nvfp4 (kernels/src/bindings.cpp:99-120). */
 size_t arcq_matmul_workspace_bytes(int64_t M, int64_t N, int64_t K_eff);
 int arcq_matmul_nvfp4_ws(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB,
@@ -166,9 +165,9 @@ int arcq_matmul_nvfp4_ws(const uint8_t* A, const uint8_t* B, const uint8_t* SFA,
 /* Which kernel arcq_matmul_nvfp4* would run for this shape on the current device (no counterpart in the
  * reference, whose CUTLASS template picks nothing at run time): *kind = ARCQ_GEMM_KIND_PAIR (persistent
  * CTA pairs, 256 x 256 tiles), ARCQ_GEMM_KIND_SINGLE (one CTA per 128 x tile_n tile) or
- * ARCQ_GEMM_KIND_SPLIT_K (single-CTA tiles over *splits ranges of K; needs scratch) or
- * ARCQ_GEMM_KIND_SKINNY (up to ARCQ_SKINNY_ROWS rows: weight streaming, K split over *splits CTAs of a cluster that add
- * their partial sums on chip; no scratch).  *tile_n: tile width; *splits: 1 unless split.  Any output pointer may be NULL. */
+ * ARCQ_GEMM_KIND_SKINNY (up to ARCQ_SKINNY_ROWS rows, or 128 x 128 tiles that leave an SM for each: weight streaming, K
+ * split over *splits CTAs of a cluster that add their partial sums on chip); ARCQ_GEMM_KIND_SPLIT_K (partial sums in
+ * scratch) is no longer chosen.  *tile_n: tile width; *splits: 1 unless split.  Any output pointer may be NULL. */
 #define ARCQ_GEMM_KIND_SINGLE 0
 #define ARCQ_GEMM_KIND_SPLIT_K 1
 #define ARCQ_GEMM_KIND_PAIR 2
@@ -180,20 +179,11 @@ int arcq_matmul_plan(int64_t M, int64_t N, int64_t K_eff, int* kind, int* tile_n
  * memory: code that runs where an allocation would fail or stall - an inference-server plugin
  * whose enqueue hook is forbidden to call the allocator, a process whose whole device memory has
  * been handed to another framework's pool, a latency-critical loop where a cudaMalloc would
- * serialise the device.  Same arithmetic and same split as arcq_matmul_nvfp4_ws, but the fp32
- * partial sums live in a block of ARCQ_STATIC_SCRATCH_BYTES (2 MiB) that is part of the library
- * image itself; every GPU that loads the library holds that block until the process exits.  Inputs
- * and the output are still the caller's.  The call allocates nothing: no cudaMalloc / cudaFree, no
- * allocating library routine.
- *   - Shapes whose partial sums exceed the block (arcq_matmul_workspace_bytes(M,N,K_eff) >
- *     ARCQ_STATIC_SCRATCH_BYTES, e.g. M 128 x N 4096 x K_eff 14464) are refused with
- *     ARCQ_ERR_SCRATCH_LIMIT; shapes that are not split at all run without touching the block.
- *   - The first call on each device looks up the block's device address (one cudaGetSymbolAddress,
- *     with that device current); make that first call outside any stream capture.
- *   - All calls share the one block and it keeps whatever the previous call left.  Nothing in it
- *     needs clearing: every partial sum that is read was written earlier in the same call.  For the
- *     same reason two calls that overlap on the GPU (different streams, or different host threads
- *     on one device) race on it - serialise them on one stream. */
+ * serialise the device.  Same arithmetic and same split as arcq_matmul_nvfp4_ws.  Inputs and the output are the
+ * caller's.  The call allocates nothing: no cudaMalloc / cudaFree, no allocating library routine.
+ *   - Shapes with arcq_matmul_workspace_bytes(M,N,K_eff) > ARCQ_STATIC_SCRATCH_BYTES (e.g. M 128 x N 4096 x
+ *     K_eff 14464) are refused with ARCQ_ERR_SCRATCH_LIMIT.
+ *   - Calls share nothing: they may overlap on several streams. */
 #define ARCQ_STATIC_SCRATCH_BYTES (2u << 20)
 int arcq_matmul_nvfp4_static(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB,
                              int64_t M, int64_t N, int64_t K_eff, float alpha, const float* alpha_a,

@@ -1,5 +1,5 @@
 """The weight-streaming GEMM for few rows (arcq_skinny.cu): against the oracle's fp32 product rounded to the output
-type, at the edges of its token columns (16, 32, 64), of the 128-row weight tiles and of the K stages, split over a
+type, at the edges of its token columns (16, 32, 64, 128), of the 128-row weight tiles and of the K stages, split over a
 cluster or not; its residual and SwiGLU epilogues; grouped runs, more rows than one pass takes included."""
 import numpy as np
 import pytest
@@ -37,7 +37,11 @@ def _close(got, ref):
 
 
 @pytest.mark.parametrize("m,n,kq,ke", [(1, 8, 64, 0), (15, 136, 256, 64), (16, 4096, 4096, 128), (17, 1000, 1984, 64),
-                                        (32, 512, 2048, 64), (33, 2048, 1024, 128), (64, 6144, 4096, 128), (64, 24, 512, 512)])
+                                        (32, 512, 2048, 64), (33, 2048, 1024, 128), (64, 6144, 4096, 128), (64, 24, 512, 512),
+                                        # tiles of 128 tokens: one and several, last ones of 1, 16, 127 and 128 rows, one
+                                        # to four ranges of K, a last stage of one K step, a ragged last weight tile
+                                        (65, 4096, 4096, 128), (127, 136, 256, 64), (128, 1000, 1984, 64), (129, 2048, 2048, 64),
+                                        (144, 4104, 1024, 128), (333, 6144, 4096, 128), (512, 4096, 512, 64), (1000, 24, 64, 0)])
 def test_few_rows_against_the_oracle(m, n, kq, ke):
     from arcquant_b200 import _lib, ops
 
@@ -60,7 +64,8 @@ def test_few_rows_against_the_oracle(m, n, kq, ke):
     assert torch.equal(ops.matmul(a, b, sfa, sfb, float(sx * sw)), first) or m * n < 64
 
 
-@pytest.mark.parametrize("m,f,kq", [(1, 128, 256), (16, 2048, 1024), (20, 14336, 4096), (37, 384, 512), (64, 2048, 4096)])
+@pytest.mark.parametrize("m,f,kq", [(1, 128, 256), (16, 2048, 1024), (20, 14336, 4096), (37, 384, 512), (64, 2048, 4096),
+                                    (65, 128, 256), (128, 2048, 4096), (100, 14336, 1024)])
 def test_few_rows_swiglu_equals_gemm_then_silu(m, f, kq):
     from arcquant_b200 import ops
 

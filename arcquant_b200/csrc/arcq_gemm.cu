@@ -261,7 +261,7 @@ arcq_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // leader's "accumulator free" barrier.  No load uses cluster multicast.
 
 constexpr int C2_STAGES = 5;
-constexpr int C2_THREADS = 320;                     // producer, MMA, 4 epilogue, 4 scale warps
+constexpr int C2_THREADS = 512;                     // producer, MMA, 2 idle; 4 scale; 8 epilogue warps
 constexpr int C2_A_BYTES = 128 * BK_BYTES;          // 16 KB
 constexpr int C2_B_BYTES = 128 * BK_BYTES;          // 16 KB: this CTA's half of the 256 B rows
 constexpr int C2_SFA_BYTES = KSTEPS * ATOM;         // 2 KB
@@ -269,7 +269,7 @@ constexpr int C2_SFB_BYTES = 2 * KSTEPS * ATOM;     // 4 KB: both 128-row scale 
 constexpr int C2_STAGE_BYTES = C2_A_BYTES + C2_B_BYTES + C2_SFA_BYTES + C2_SFB_BYTES;   // 38 KB
 constexpr int C2_SF_COLS = KSTEPS * 4 + KSTEPS * 8;  // 48 TMEM columns of scales per stage
 constexpr int C2_TMEM_COLS = 512;                    // 256 accumulator + 5 x 48 scale columns
-constexpr int C2_CSTAGE_BYTES = 4 * 8192;             // output staging: 32 rows x 128 columns of bf16 per epilogue warp
+constexpr int C2_CSTAGE_BYTES = 8 * 4096;             // output staging: 32 rows x 64 columns of bf16 per epilogue warp
 constexpr int C2_SMEM_BYTES = 1024 + C2_STAGES * C2_STAGE_BYTES + C2_CSTAGE_BYTES + 256 + 64;   // + residual barriers
 constexpr uint32_t PEER_BIT_MASK = 0xFEFFFFFFu;      // clears the pair-rank bit of a shared address
 
@@ -330,7 +330,6 @@ struct Gemm2Params {
   unsigned int* amax;
   const int* groups;
   int ngroups;
-  const uint16_t* silu_table;   // bf16(silu(g)) for all 65536 bf16 patterns g (device memory, see silu_table_ptr)
   // Scattered output (0 = off): rows [d * rows_per_dest, (d + 1) * rows_per_dest) of the result go to output
   // map d, a [rows_per_dest, N] buffer of its own - in a tensor-parallel group, this rank's slot in the memory
   // of the rank that owns those rows (a peer's memory over NVLink, or local memory).  A multiple of 32: one
@@ -381,7 +380,7 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   auto sf_ready_bar = [&](int s) { return bar_base + 8u * (3 * C2_STAGES + s); }; // scales in TMEM (leader's is used)
   const uint32_t tmem_full_bar = bar_base + 8u * (4 * C2_STAGES);
   const uint32_t tmem_empty_bar = tmem_full_bar + 8u;
-  auto resid_bar = [&](int q, int b) { return bar_base + 256u + 8u * (2 * q + b); };   // residual box landed in slot b of epilogue warp q
+  auto resid_bar = [&](int w) { return bar_base + 256u + 8u * w; };              // residual box of epilogue warp w landed
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();        // 0 = leader (issues the MMAs), 1 = peer
@@ -395,8 +394,8 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       mbar_init(sf_ready_bar(s), 8);              // four scale warps in each of the two CTAs
     }
     mbar_init(tmem_full_bar, 1);
-    mbar_init(tmem_empty_bar, 8);                 // four epilogue warps in each of the two CTAs
-    for (int q = 0; q < 8; ++q) mbar_init(resid_bar(q >> 1, q & 1), 1);
+    mbar_init(tmem_empty_bar, 16);                // eight epilogue warps in each of the two CTAs
+    for (int w = 0; w < 8; ++w) mbar_init(resid_bar(w), 1);
     misc[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -488,9 +487,14 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         ++tile_it;
       }
     }
-  } else if (warp < 6) {
+  } else if (warp >= 8) {
     // ------------------------------------------------------------------ epilogue (both CTAs)
-    const int quad = warp & 3;
+    // Two warps per tensor-memory quadrant, each with half of the columns: [128 half, 128 half + 128), with SwiGLU gate
+    // columns [64 half, 64 half + 64) and the up columns that belong to them.
+    // (One warp per quadrant, with all 256 columns and SiLU from a table in L2, was busy for longer than a tile's MMAs:
+    // SwiGLU [28672, 4224], us, before / eight warps and the table / eight warps and silu_for_bf16: 333 rows 55 / 52 / 49,
+    // 2048 rows 147 / 142 / 137, 16384 rows 1057 / 1035 / 978.  The other epilogues are hidden either way.)
+    const int quad = warp & 3, ew = warp - 8, half = ew >> 2;
     float alpha = p.alpha;
     if (p.tile_group == nullptr) {
       if (p.alpha_a) alpha *= __ldg(p.alpha_a);
@@ -512,10 +516,10 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       if (RESID) {
         // the first residual box of this tile is fetched while the tile's MMAs are still running
         const int row0r = tm * 256 + (int)rank * 128 + quad * 32;
-        if (lane == 0 && row0r < p.M) {
-          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");     // slot 0 is free again
-          mbar_expect_tx(resid_bar(quad, 0), 4096u);
-          tma_load_2d_once(cstage_base + (uint32_t)quad * 8192u, &map_r, resid_bar(quad, 0), tn * 256, row0r);
+        if (lane == 0 && row0r < p.M && tn * 256 + 128 * half < p.N) {
+          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");     // the slot is free again
+          mbar_expect_tx(resid_bar(ew), 4096u);
+          tma_load_2d_once(cstage_base + (uint32_t)ew * 4096u, &map_r, resid_bar(ew), tn * 256 + 128 * half, row0r);
         }
       }
       ok = mbar_wait(tmem_full_bar, tile_it & 1u, abort_flag);
@@ -523,19 +527,20 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       if (!ok) break;
       tc_fence_after();
       const int row = tm * 256 + (int)rank * 128 + quad * 32 + lane;
-      // Drain the accumulator into registers as packed bf16 (128 registers for this thread's 256
-      // columns) and hand tensor memory back at once: the stores below then overlap the next tile's MMAs.
-      uint32_t o[128];
+      // Drain the accumulator into registers as packed bf16 (64 registers for this thread's 128 columns) and hand tensor
+      // memory back at once: the stores below then overlap the next tile's MMAs.
+      uint32_t o[64];
 #pragma unroll
-      for (int c0 = 0; c0 < 256; c0 += 64) {
+      for (int c = 0; c < 2; ++c) {
+        const uint32_t col = SWIGLU ? (uint32_t)(128 * c + 64 * half) : (uint32_t)(128 * half + 64 * c);
         uint32_t r0[32], r1[32];
-        tc_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)c0, r0);
-        tc_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c0 + 32), r1);
+        tc_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + col, r0);
+        tc_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + col + 32u, r1);
         tc_wait_ld();
 #pragma unroll
         for (int v = 0; v < 16; ++v) {
-          o[c0 / 2 + v] = pack_bf16x2(__uint_as_float(r0[2 * v]) * alpha, __uint_as_float(r0[2 * v + 1]) * alpha);
-          o[c0 / 2 + 16 + v] = pack_bf16x2(__uint_as_float(r1[2 * v]) * alpha, __uint_as_float(r1[2 * v + 1]) * alpha);
+          o[32 * c + v] = pack_bf16x2(__uint_as_float(r0[2 * v]) * alpha, __uint_as_float(r0[2 * v + 1]) * alpha);
+          o[32 * c + 16 + v] = pack_bf16x2(__uint_as_float(r1[2 * v]) * alpha, __uint_as_float(r1[2 * v + 1]) * alpha);
         }
       }
       tc_fence_before();
@@ -548,12 +553,10 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         if (p.groups != nullptr) row_end = __ldg(p.groups + grp) + __ldg(p.groups + p.ngroups + grp);
         uint32_t m = 0;
 #pragma unroll
-        for (int j = 0; j < 64; ++j) {
-          // SiLU of a bf16 value is one of 65536 results: looked up (the table stays in L2; evaluating
-          // expf and a division 128 times per row made the epilogue slower than the tile's MMAs)
-          const uint32_t g = o[j], u = o[64 + j];
-          const float sa = __uint_as_float((uint32_t)__ldg(p.silu_table + (g & 0xffffu)) << 16);
-          const float sb = __uint_as_float((uint32_t)__ldg(p.silu_table + (g >> 16)) << 16);
+        for (int j = 0; j < 32; ++j) {
+          const uint32_t g = o[j], u = o[32 + j];
+          const uint32_t s2 = pack_bf16x2(silu_for_bf16(__uint_as_float(g << 16)), silu_for_bf16(__uint_as_float(g & 0xffff0000u)));
+          const float sa = __uint_as_float(s2 << 16), sb = __uint_as_float(s2 & 0xffff0000u);
           o[j] = pack_bf16x2(sa * __uint_as_float(u << 16), sb * __uint_as_float(u & 0xffff0000u));
           asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(o[j] & 0x7fff7fffu));
         }
@@ -562,16 +565,16 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         for (int d = 16; d > 0; d >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, d));
         if (lane == 0 && v) atomicMax(p.amax + grp, v << 16);
       }
-      const int col0 = SWIGLU ? tn * 128 : tn * 256;
+      const int col0 = SWIGLU ? tn * 128 + 64 * half : tn * 256 + 128 * half;
       const int ncols = SWIGLU ? (p.N >> 1) : p.N;
       {
-        // Through shared memory: the warp's 32 rows x 256 columns leave as four boxes of 64 columns
+        // Through shared memory: the warp's 32 rows x 128 columns (SwiGLU: 64) leave as boxes of 64 columns
         // (32 rows x 128 bytes, 128-byte swizzle: lane = row, 16-byte chunk c of row r sits at chunk
-        // c ^ (r & 7), so a warp's 128-bit stores are conflict free), two boxes per round in the
-        // warp's 8 KB of staging.  The bulk stores write whole 128-byte lines, clip rows >= M and
+        // c ^ (r & 7), so a warp's 128-bit stores are conflict free), one after the other from the
+        // warp's 4 KB of staging.  The bulk stores write whole 128-byte lines, clip rows >= M and
         // columns >= N themselves, and keep the load/store pipe free for the scale warps.
         const int row0 = tm * 256 + (int)rank * 128 + quad * 32;
-        const uint32_t cst = cstage_base + (uint32_t)quad * 8192u;
+        const uint32_t slot = cstage_base + (uint32_t)ew * 4096u;
         const CUtensorMap* map_c = &maps_c.m[0];
         int row_st = row0;
         if (p.rows_per_dest) {       // these 32 rows belong to one destination
@@ -579,35 +582,39 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           map_c = &maps_c.m[d];
           row_st = row0 - d * p.rows_per_dest;
         }
-        if (RESID && row0 < p.M) {
-          // Four boxes of 64 columns, two slots: box k is added and stored from slot k & 1 while box k + 1 is
-          // on its way into the other slot (box 0 was requested before the accumulator was ready).
+        if (row0 < p.M) {
 #pragma unroll
-          for (int k = 0; k < 4; ++k) {
+          for (int k = 0; k < (SWIGLU ? 1 : 2); ++k) {
             const int col = col0 + 64 * k;
             if (col >= ncols) break;
-            const uint32_t slot = cst + (uint32_t)(k & 1) * 4096u;
-            if (lane == 0 && k + 1 < 4 && col + 64 < ncols) {
-              if (k >= 1) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // box k - 1 has left its slot
-              mbar_expect_tx(resid_bar(quad, (k + 1) & 1), 4096u);
-              tma_load_2d_once(cst + (uint32_t)((k + 1) & 1) * 4096u, &map_r, resid_bar(quad, (k + 1) & 1), col + 64, row0);
+            if (RESID) {
+              // (box 0 was requested before the accumulator was ready)
+              if (k > 0 && lane == 0) {
+                asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // box 0 has left the slot
+                mbar_expect_tx(resid_bar(ew), 4096u);
+                tma_load_2d_once(slot, &map_r, resid_bar(ew), col, row0);
+              }
+              ok = mbar_wait(resid_bar(ew), resid_it & 1u, abort_flag);
+              ok = __all_sync(0xffffffffu, ok);
+              if (!ok) break;
+              ++resid_it;
+            } else {
+              if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the slot is free again
+              __syncwarp();
             }
-            ok = mbar_wait(resid_bar(quad, k & 1), (resid_it >> (k & 1)) & 1u, abort_flag);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            resid_it ^= 1u << (k & 1);      // (bit b: parity of slot b's next box)
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
               const int j = 32 * k + 4 * c;
               const uint32_t addr = slot + (uint32_t)lane * 128u + (uint32_t)((c ^ (lane & 7)) << 4);
-              uint32_t r0, r1, r2, r3;
-              asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3) : "r"(addr) : "memory");
-              const uint32_t rr[4] = {r0, r1, r2, r3};
-              uint32_t out4[4];
+              uint32_t out4[4] = {o[j], o[j + 1], o[j + 2], o[j + 3]};
+              if (RESID) {
+                uint32_t rr[4];
+                asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(rr[0]), "=r"(rr[1]), "=r"(rr[2]), "=r"(rr[3]) : "r"(addr) : "memory");
 #pragma unroll
-              for (int e = 0; e < 4; ++e)
-                out4[e] = pack_bf16x2(__uint_as_float(rr[e] << 16) + __uint_as_float(o[j + e] << 16),
-                                      __uint_as_float(rr[e] & 0xffff0000u) + __uint_as_float(o[j + e] & 0xffff0000u));
+                for (int e = 0; e < 4; ++e)
+                  out4[e] = pack_bf16x2(__uint_as_float(rr[e] << 16) + __uint_as_float(o[j + e] << 16),
+                                        __uint_as_float(rr[e] & 0xffff0000u) + __uint_as_float(o[j + e] & 0xffff0000u));
+              }
               asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(out4[0]), "r"(out4[1]), "r"(out4[2]),
                            "r"(out4[3])
                            : "memory");
@@ -621,36 +628,6 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
               asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             }
           }
-        } else if (row0 < p.M) {
-#pragma unroll
-          for (int h = 0; h < (SWIGLU ? 1 : 2); ++h) {
-            if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // staging is free again
-            __syncwarp();
-#pragma unroll
-            for (int bs = 0; bs < 2; ++bs) {
-#pragma unroll
-              for (int c = 0; c < 8; ++c) {
-                const int j = 32 * (2 * h + bs) + 4 * c;
-                const uint32_t addr = cst + (uint32_t)bs * 4096u + (uint32_t)lane * 128u + (uint32_t)((c ^ (lane & 7)) << 4);
-                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(o[j]), "r"(o[j + 1]),
-                             "r"(o[j + 2]), "r"(o[j + 3])
-                             : "memory");
-              }
-            }
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) {
-#pragma unroll
-              for (int bs = 0; bs < 2; ++bs) {
-                const int col = col0 + 64 * (2 * h + bs);
-                if (col < ncols)
-                  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];" ::"l"(map_c),
-                               "r"(cst + (uint32_t)bs * 4096u), "r"(col), "r"(row_st)
-                               : "memory");
-              }
-              asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-            }
-          }
         }
       }
       ++tile_it;
@@ -658,7 +635,7 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     // the last boxes must have left shared memory (and reached global memory) before the CTA goes
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     __syncwarp();
-  } else {
+  } else if (warp >= 4) {
     // ------------------------------------------------------------------ scale warps (both CTAs)
     // Warp q writes TMEM lanes 32q..32q+31.  An atom is 32 rows x 16 bytes: lane l's 16 bytes are
     // its four TMEM columns (rows l, l+32, l+64, l+96 of the 128-row tile, four K blocks each);
@@ -792,12 +769,7 @@ int launch_pair(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const ui
   p.tile_group = tile_group;
   CUtensorMap ma, mb, msa, msb;
   OutputMaps mc;
-  p.silu_table = nullptr;
-  if (swiglu_amax != nullptr) {
-    ARCQ_CUDA_TRY(cudaMemsetAsync(swiglu_amax, 0, sizeof(float) * ngroups, stream));
-    int rc_t = silu_table_ptr(stream, &p.silu_table);
-    if (rc_t != ARCQ_OK) return rc_t;
-  }
+  if (swiglu_amax != nullptr) ARCQ_CUDA_TRY(cudaMemsetAsync(swiglu_amax, 0, sizeof(float) * ngroups, stream));
   int rc = ARCQ_OK;
   if (ndests > 0) {
     for (int d = 0; d < ndests && rc == ARCQ_OK; ++d) rc = make_c_map(&mc.m[d], dests[d], M / ndests, N);

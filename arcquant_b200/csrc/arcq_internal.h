@@ -99,9 +99,6 @@ int peer_poll_error();
 int peer_set_wait_limit_ms(int ms);
 int launch_sum_partials(const void* const* srcs, int n, int64_t elems, const void* residual, void* out,
                         cudaStream_t stream);
-// Device address of the 65536-entry table bf16(silu(g)) on the current device; the first call per device
-// builds it on `stream`, later calls on other streams wait for that (arcq_layer.cu).
-int silu_table_ptr(cudaStream_t stream, const uint16_t** out);
 // Few rows: weight streaming (arcq_skinny.cu).
 int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, const uint8_t* SFW, int64_t M, int64_t N,
                        int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, const void* residual, void* C,

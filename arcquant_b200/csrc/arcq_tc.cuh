@@ -67,6 +67,16 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
   }
 }
+// SiLU for a gate that is a bf16 value and a result that is rounded to bf16: after that rounding, the bits of the eager
+// chain g / (1 + expf(-g)) for every one of the 65 536 gates (tests/test_gpu_silu.py), from two special-function
+// instructions and four on the FMA pipe.  The factor 1/4 keeps the reciprocal's argument below 2^126 - where it would be
+// flushed - exactly as long as expf(-g) is finite.
+__device__ __forceinline__ float silu_for_bf16(float g) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(__fmaf_rn(g, -1.44269504f, -2.0f)));      // exp(-g) / 4
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(__fadd_rn(e, 0.25f)));
+  return __fmul_rn(g, __fmul_rn(r, 0.25f));
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"

@@ -54,6 +54,7 @@ SIGNATURES = {
     "arcq_rope_bf16": (_i32, [_vp, _vp, _vp, _i64, _i32, _i32, _i32, _i32, _vp]),
     "arcq_silu_mul_bf16": (_i32, [_vp, _vp, _i64, _i32, _vp, _vp]),
     "arcq_calib_stats_bf16": (_i32, [_vp, _i64, _i32, _vp, _vp, _vp]),
+    "arcq_route_topk_bf16": (_i32, [_vp, _i64, _i32, _i32, _vp, _vp, _vp]),
     "arcq_moe_layout": (_i32, [_vp, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp]),
     "arcq_silu_mul_grouped_bf16": (_i32, [_vp, _vp, _i64, _i32, _vp, _vp, _i32, _vp, _vp]),
     "arcq_absmax_grouped_bf16": (_i32, [_vp, _vp, _vp, _i32, _i32, _vp, _vp]),

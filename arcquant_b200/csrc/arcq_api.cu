@@ -331,6 +331,13 @@ int arcq_calib_stats_bf16(const void* x, int64_t rows, int K, float* chan_absmax
   return launch_calib_stats(x, rows, K, chan_absmax, above, (cudaStream_t)stream);
 }
 
+int arcq_route_topk_bf16(const void* logits, int64_t tokens, int experts, int top_k, int64_t* ids, void* weights, void* stream) {
+  if (tokens < 0 || experts < 1 || experts > 32 || top_k < 1 || top_k > experts) return ARCQ_ERR_BAD_SHAPE;
+  if (tokens == 0) return ARCQ_OK;
+  if (!logits || !ids || !weights) return ARCQ_ERR_NULL_POINTER;
+  return launch_route_topk(logits, tokens, experts, top_k, reinterpret_cast<long long*>(ids), weights, (cudaStream_t)stream);
+}
+
 int arcq_moe_layout(const int64_t* slot_group, int n, int ngroups, int tile, int rows_bound, int div, int32_t* dest,
                     int32_t* row_map, int32_t* groups, int32_t* tile_group, void* stream) {
   if (n < 0 || n > (1 << 20) || ngroups < 1 || ngroups > 64 || tile < 1 || div < 1 || rows_bound % tile ||

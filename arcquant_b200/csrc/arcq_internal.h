@@ -76,6 +76,8 @@ int launch_absmax_grouped(const void* x, const int* row_map, const int* groups, 
                           cudaStream_t stream);
 int launch_moe_layout(const long long* slot_group, int n, int ngroups, int tile, int rows_bound, int div, int* dest,
                       int* row_map, int* groups, int* tile_group, cudaStream_t stream);
+int launch_route_topk(const void* logits, int64_t tokens, int experts, int top_k, long long* ids, void* weights,
+                      cudaStream_t stream);
 int launch_calib_stats(const void* x, int64_t rows, int K, float* chan_absmax, unsigned long long* above,
                        cudaStream_t stream);
 int launch_silu_mul_grouped(const void* gu, void* out, int64_t rows, int F, const int* tile_group, const int* groups,

@@ -398,74 +398,134 @@ __global__ void arcq_absmax_grouped_kernel(const uint16_t* __restrict__ x, const
 // their original order.  dest[i] = padded row of slot i (rows_bound for nobody), row_map[r] = i / div for
 // the padded row r that holds slot i (0 for padding), groups = [first row of every run | rows of every
 // run], tile_group[m] = run of tile m or -1.
+// Bound: latency.  Every warp owns a run of slots and counts its runs 32 slots at a time (lanes of one run find each other
+// by match, their first adds the count), the 32 warps' counts are scanned per run, and the same walk places the slots:
+// 2 n / 1024 steps whatever the number of runs, coalesced.  One scan over all slots per run took 13 us for 74 slots of 8
+// runs and 71 us for 8192.
 __global__ void __launch_bounds__(1024, 1)
 arcq_moe_layout_kernel(const long long* __restrict__ slot_group, int n, int ngroups, int tile, int rows_bound, int div,
                        int* __restrict__ dest, int* __restrict__ row_map, int* __restrict__ groups,
                        int* __restrict__ tile_group) {
-  __shared__ int s_cnt[64], s_off[64], s_warp[32];
+  constexpr int BATCH = 8;
+  __shared__ int s_hist[32][65], s_cnt[64], s_off[64];     // (65: a column is read by 32 lanes)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int per = (n + 1023) >> 10;
-  const int lo = min(n, tid * per), hi = min(n, lo + per);
-  for (int r = tid; r < rows_bound; r += 1024) row_map[r] = 0;
-  // this thread's matches of run e, and the number of matches in all earlier threads (exclusive scan)
-  auto scan = [&](int e, int& mine, int& before, int& total) {
-    mine = 0;
-    for (int i = lo; i < hi; ++i) mine += (slot_group[i] == (long long)e) ? 1 : 0;
-    int inc = mine;
+  const int chunk = ((n + 1023) >> 10) * 32;               // slots per warp
+  const int lo = min(n, warp * chunk), hi = min(n, lo + chunk);
+  int e[BATCH];                                            // runs of this lane's slots, -1: nobody
+  auto load = [&](int at) {
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int v = __shfl_up_sync(0xffffffffu, inc, d);
-      if (lane >= d) inc += v;
+    for (int b = 0; b < BATCH; ++b) {
+      const int i = at + 32 * b + lane;
+      const long long g = i < hi ? slot_group[i] : -1;
+      e[b] = g >= 0 && g < ngroups ? (int)g : -1;
     }
-    if (lane == 31) s_warp[warp] = inc;
-    __syncthreads();
-    if (warp == 0) {
-      int w = s_warp[lane], winc = w;
-#pragma unroll
-      for (int d = 1; d < 32; d <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, winc, d);
-        if (lane >= d) winc += v;
-      }
-      s_warp[lane] = winc - w;                         // matches in earlier warps
-      if (lane == 31) s_cnt[e] = winc;
-    }
-    __syncthreads();
-    before = s_warp[warp] + inc - mine;
-    total = s_cnt[e];
-    __syncthreads();                                   // s_warp is reused by the next scan
   };
-  int mine, before, total;
-  for (int e = 0; e < ngroups; ++e) scan(e, mine, before, total);   // fills s_cnt
-  if (tid == 0) {
-    int off = 0;
-    for (int e = 0; e < ngroups; ++e) {
-      s_off[e] = off;
-      groups[e] = off;
-      groups[ngroups + e] = s_cnt[e];
-      off += (s_cnt[e] + tile - 1) / tile * tile;
+  load(lo);
+  for (int r = tid; r < rows_bound; r += 1024) row_map[r] = 0;
+  for (int g = lane; g < 64; g += 32) s_hist[warp][g] = 0;
+  __syncwarp();
+  for (int at = lo; at < hi; at += 32 * BATCH) {
+    if (at != lo) load(at);
+#pragma unroll
+    for (int b = 0; b < BATCH; ++b) {
+      if (at + 32 * b >= hi) break;
+      const uint32_t same = __match_any_sync(0xffffffffu, e[b]);
+      if (e[b] >= 0 && lane == __ffs(same) - 1) s_hist[warp][e[b]] += __popc(same);
+      __syncwarp();
     }
   }
   __syncthreads();
-  for (int e = 0; e < ngroups; ++e) {
-    const int off = s_off[e];
-    scan(e, mine, before, total);
-    int r = off + before;
-    for (int i = lo; i < hi; ++i) {
-      if (slot_group[i] == (long long)e) {
-        dest[i] = r;
-        row_map[r] = i / div;
-        ++r;
-      }
+  for (int g = warp; g < ngroups; g += 32) {               // exclusive scan over the warps
+    const int v = s_hist[lane][g];
+    int inc = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, inc, d);
+      if (lane >= d) inc += u;
+    }
+    s_hist[lane][g] = inc - v;
+    if (lane == 31) s_cnt[g] = inc;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    int off = 0;
+    for (int g = 0; g < ngroups; ++g) {
+      s_off[g] = off;
+      groups[g] = off;
+      groups[ngroups + g] = s_cnt[g];
+      off += (s_cnt[g] + tile - 1) / tile * tile;
     }
   }
-  for (int i = lo; i < hi; ++i)
-    if (slot_group[i] < 0 || slot_group[i] >= (long long)ngroups) dest[i] = rows_bound;
+  __syncthreads();
+  const bool again = hi - lo > 32 * BATCH;                 // (else the first batch is still in registers)
+  for (int at = lo; at < hi; at += 32 * BATCH) {
+    if (again) load(at);
+#pragma unroll
+    for (int b = 0; b < BATCH; ++b) {
+      if (at + 32 * b >= hi) break;
+      const int i = at + 32 * b + lane;
+      const uint32_t same = __match_any_sync(0xffffffffu, e[b]);
+      const int first = e[b] >= 0 ? s_hist[warp][e[b]] : 0;
+      __syncwarp();
+      if (e[b] >= 0) {
+        const int r = s_off[e[b]] + first + __popc(same & ((1u << lane) - 1u));
+        dest[i] = r;
+        row_map[r] = i / div;
+        if (lane == __ffs(same) - 1) s_hist[warp][e[b]] = first + __popc(same);
+      } else if (i < hi) {
+        dest[i] = rows_bound;
+      }
+      __syncwarp();
+    }
+  }
   for (int m = tid; m < rows_bound / tile; m += 1024) {
     const int start = m * tile;
-    int g = -1;
-    for (int e = 0; e < ngroups; ++e)
-      if (start >= s_off[e] && start < s_off[e] + s_cnt[e]) g = e;
-    tile_group[m] = g;
+    int run = -1;
+    for (int g = 0; g < ngroups; ++g)
+      if (start >= s_off[g] && start < s_off[g] + s_cnt[g]) run = g;
+    tile_group[m] = run;
+  }
+}
+
+// Routing of a MoE block: softmax over a token's logits in fp32, the top_k largest probabilities (of equal ones the
+// earliest), their shares of the selected sum rounded to bf16.  width (a power of two >= experts, at most 32) lanes per
+// token; sums in the order of a butterfly over them.  Bound: launches - softmax, top-k, its sort, the sum, the division
+// and the cast as torch operations were seven launches, 21 us of kernels for 37 tokens and 29 us for 4096.
+__global__ void arcq_route_topk_kernel(const uint16_t* __restrict__ logits, long long tokens, int experts, int width, int top_k,
+                                       long long* __restrict__ ids, uint16_t* __restrict__ weights) {
+  const int per_warp = 32 / width, lane = threadIdx.x & 31, sub = lane & (width - 1);
+  const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
+  for (long long t0 = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * per_warp; t0 < tokens; t0 += warps * per_warp) {
+    const long long t = t0 + lane / width;
+    const bool in = t < tokens && sub < experts;
+    const float l = in ? __uint_as_float((uint32_t)logits[t * experts + sub] << 16) : -INFINITY;
+    float mx = l;
+    for (int d = width >> 1; d > 0; d >>= 1) {
+      const float o = __shfl_xor_sync(0xffffffffu, mx, d);
+      mx = mx < o ? o : mx;
+    }
+    const float ex = in ? expf(l - mx) : 0.f;
+    float sum = ex;
+    for (int d = width >> 1; d > 0; d >>= 1) sum = __fadd_rn(sum, __shfl_xor_sync(0xffffffffu, sum, d));
+    const float p = __fdiv_rn(ex, sum);
+    int key = in ? (int)(__float_as_uint(p) & 0x7fffffffu) : -1;       // (a NaN orders above everything)
+    float mine = 0.f, total = 0.f;
+    int mine_id = 0;
+    for (int j = 0; j < top_k; ++j) {
+      int bk = key, bi = sub;
+      for (int d = width >> 1; d > 0; d >>= 1) {
+        const int ok = __shfl_xor_sync(0xffffffffu, bk, d), oi = __shfl_xor_sync(0xffffffffu, bi, d);
+        if (ok > bk || (ok == bk && oi < bi)) { bk = ok; bi = oi; }
+      }
+      const float pv = __shfl_sync(0xffffffffu, p, (lane & ~(width - 1)) | bi);
+      total = j == 0 ? pv : __fadd_rn(total, pv);
+      if (sub == j) { mine = pv; mine_id = bi; }
+      if (sub == bi) key = -1;
+    }
+    if (t < tokens && sub < top_k) {
+      ids[t * top_k + sub] = mine_id;
+      weights[t * top_k + sub] = (uint16_t)pack2(__fdiv_rn(mine, total), 0.f);
+    }
   }
 }
 
@@ -740,6 +800,23 @@ int launch_moe_layout(const long long* slot_group, int n, int ngroups, int tile,
                       int* row_map, int* groups, int* tile_group, cudaStream_t stream) {
   arcq_moe_layout_kernel<<<1, 1024, 0, stream>>>(slot_group, n, ngroups, tile, rows_bound, div, dest, row_map, groups,
                                                  tile_group);
+  ARCQ_CUDA_TRY(cudaGetLastError());
+  return ARCQ_OK;
+}
+
+int launch_route_topk(const void* logits, int64_t tokens, int experts, int top_k, long long* ids, void* weights,
+                      cudaStream_t stream) {
+  if (tokens == 0) return ARCQ_OK;
+  DeviceInfo di;
+  int rc = get_device_info(&di);
+  if (rc != ARCQ_OK) return rc;
+  int width = 1;
+  while (width < experts) width <<= 1;
+  const long long per_block = 4 * (32 / width);            // four warps
+  long long blocks = (tokens + per_block - 1) / per_block;
+  if (blocks > (long long)di.num_sms * 16) blocks = (long long)di.num_sms * 16;
+  arcq_route_topk_kernel<<<(unsigned)blocks, 128, 0, stream>>>(static_cast<const uint16_t*>(logits), tokens, experts, width, top_k,
+                                                               ids, static_cast<uint16_t*>(weights));
   ARCQ_CUDA_TRY(cudaGetLastError());
   return ARCQ_OK;
 }

@@ -60,12 +60,12 @@ def _counts(ids: torch.Tensor, n: int) -> torch.Tensor:
     return (ids.unsqueeze(1) == torch.arange(n, device=ids.device).unsqueeze(0)).sum(0)
 
 
-def padded_layout(slot_expert: torch.Tensor, n_groups: int, tile: int = TILE):
+def padded_layout(slot_expert: torch.Tensor, n_groups: int, tile: int = TILE, div: int = 1):
     """Places `n` slots (slot i belongs to expert slot_expert[i], or to nobody if that is >= n_groups) into
     a padded buffer: expert after expert, every run starting at a multiple of `tile` rows, slots of one
     expert in their original order.  Returns
       dest       int64 [n]: padded row of every slot (`rows_bound` for slots of nobody),
-      row_slot   int64 [rows_bound]: slot held by every padded row (0 for padding rows),
+      row_slot   int [rows_bound]: slot held by every padded row, divided by `div` (0 for padding rows),
       groups     int32 [2 * n_groups]: first row and number of rows of every run,
       tile_group int32 [rows_bound / tile]: run of every tile, -1 for tiles without rows,
       rows_bound int: size of the padded buffer - the only number the host knows, a worst-case bound."""
@@ -73,7 +73,7 @@ def padded_layout(slot_expert: torch.Tensor, n_groups: int, tile: int = TILE):
     rows_bound = (n + tile - 1) // tile * tile + n_groups * tile
     if slot_expert.is_cuda and n_groups <= 64 and n <= (1 << 20):       # one small launch does all of it
         dest, row_slot, groups, tile_group = ops.moe_layout(slot_expert.to(torch.int64).contiguous(), n_groups, tile,
-                                                            rows_bound)
+                                                            rows_bound, div)
         return dest, row_slot, groups, tile_group, rows_bound
     order = torch.argsort(slot_expert, stable=True)
     sorted_e = slot_expert[order]
@@ -87,7 +87,7 @@ def padded_layout(slot_expert: torch.Tensor, n_groups: int, tile: int = TILE):
     dest = torch.empty_like(dest_sorted)
     dest[order] = dest_sorted
     row_slot = torch.zeros(rows_bound + 1, dtype=torch.int64, device=dev)
-    row_slot[dest] = ar
+    row_slot[dest] = torch.div(ar, div, rounding_mode="floor")
     groups = torch.cat([offs, counts]).to(torch.int32)
     tile_start = torch.arange(rows_bound // tile, device=dev) * tile
     e_of = (torch.searchsorted(offs, tile_start, right=True) - 1).clamp(min=0)
@@ -168,9 +168,8 @@ class ExpertParallelDispatcher:
         T, k = ids.shape
         flat = ids.reshape(-1)
         if self.ep == 1:
-            dest, row_slot, groups, tile_group, rows_bound = padded_layout(flat, self.e_local)
-            row_map = torch.div(row_slot, k, rounding_mode="floor").to(torch.int32)
-            return RoutedBatch(x, row_map, groups, tile_group, rows_bound, self.e_local,
+            dest, row_map, groups, tile_group, rows_bound = padded_layout(flat, self.e_local, div=k)
+            return RoutedBatch(x, row_map.to(torch.int32), groups, tile_group, rows_bound, self.e_local,
                                dict(T=T, k=k, copy_row=dest))
         n = flat.numel()
         cap = self._agree_capacity(n, x.device)
@@ -489,7 +488,12 @@ class QMixtralMoEBlockEP(torch.nn.Module):
     def forward(self, x: torch.Tensor, routing=None) -> torch.Tensor:
         """x: this rank's tokens [T, hidden] (bf16).  routing: optional precomputed
         (expert ids [T,k], weights [T,k]) - otherwise the block's own router decides."""
-        ids, w = routing if routing is not None else route_top_k(x, self.router, self.cfg.top_k)
+        if routing is not None:
+            ids, w = routing
+        elif x.is_cuda and x.dim() == 2 and x.dtype == torch.bfloat16 and self.cfg.top_k <= self.cfg.n_experts <= 32:
+            ids, w = ops.route_topk(F.linear(x, self.router), self.cfg.top_k)     # `route_top_k` in one launch
+        else:
+            ids, w = route_top_k(x, self.router, self.cfg.top_k)
         batch = self.dispatcher.dispatch(x, ids)
         y = self.expert_forward_grouped(batch) if self.grouped else self.expert_forward_padded(batch)
         return self.dispatcher.combine(y, w, batch)

@@ -280,6 +280,22 @@ def calib_stats(x: torch.Tensor, chan_absmax: torch.Tensor, above: torch.Tensor 
     _lib.check(rc, "calib_stats")
 
 
+def route_topk(logits: torch.Tensor, top_k: int):
+    """(ids int64 [T, k], weights bf16 [T, k]) of router logits bf16 [T, E], E <= 32, in one launch: fp32 softmax, top-k
+    in descending order, weights renormalised over the selected experts."""
+    lib = _lib.load()
+    _require(logits, torch.bfloat16, "logits")
+    if logits.dim() != 2:
+        raise RuntimeError("logits must be [tokens, experts]")
+    t, e = logits.shape
+    ids = torch.empty((t, top_k), dtype=torch.int64, device=logits.device)
+    w = torch.empty((t, top_k), dtype=torch.bfloat16, device=logits.device)
+    with torch.cuda.device(logits.device):
+        rc = lib.arcq_route_topk_bf16(logits.data_ptr(), t, e, top_k, ids.data_ptr(), w.data_ptr(), _stream())
+    _lib.check(rc, "route_topk")
+    return ids, w
+
+
 def moe_layout(slot_group: torch.Tensor, ngroups: int, tile: int, rows_bound: int, div: int = 1):
     """Padded layout of routed rows in one launch: (dest int32 [n], row_map int32 [rows_bound], groups int32
     [2*ngroups], tile_group int32 [rows_bound/tile]); see `arcq_moe_layout` in arcq.h."""

@@ -259,6 +259,10 @@ int arcq_calib_stats_bf16(const void* x, int64_t rows, int K, float* chan_absmax
  *   B [ngroups*N, K_eff/2] and SFB hold the experts' packed weights one after another (N % 128 == 0);
  *   tile_group int32 [ceil(M_bound/256)] in device memory: the run that owns each 256-row tile of A, or
  *   a negative number for a tile without rows (skipped).  alpha_b may be NULL. */
+/* Routing (model/qMixtralLayer.py:441-447): fp32 softmax over the router's bf16 logits [tokens, experts], the top_k largest
+ * probabilities of a token in descending order (of equal ones the earliest), each divided by the sum of the selected.
+ * ids int64 and weights bf16 [tokens, top_k]; experts <= 32. */
+int arcq_route_topk_bf16(const void* logits, int64_t tokens, int experts, int top_k, int64_t* ids, void* weights, void* stream);
 /* The padded layout itself, computed on the device in one small launch (no counterpart in the reference,
  * whose Python loop asks torch.where for every expert's rows, model/qMixtralLayer.py:458-466).
  * slot_group int64 [n]: the run (local expert) of every slot - a routed copy (token, j) or a row of the

@@ -109,18 +109,48 @@ torch::Tensor matmul(const torch::Tensor& A, const torch::Tensor& B, const torch
 // Extra: alpha = alpha_a * alpha_b read on the device (0-dim fp32 CUDA tensors), no host sync.
 torch::Tensor matmul_dev_alpha(const torch::Tensor& A, const torch::Tensor& B, const torch::Tensor& SFA,
                                const torch::Tensor& SFB, const torch::Tensor& alpha_a,
-                               const c10::optional<torch::Tensor>& alpha_b) {
+                               const c10::optional<torch::Tensor>& alpha_b, const c10::optional<torch::Tensor>& bias) {
   int64_t M, N, K;
   std::tie(M, N, K) = check_gemm_operands(A, B, SFA, SFB);
   require_scalar_f32(alpha_a, A, "alpha_a");
   if (alpha_b.has_value()) require_scalar_f32(*alpha_b, A, "alpha_b");
   c10::cuda::CUDAGuard guard(A.device());
   auto C = torch::empty({M, N}, torch::dtype(torch::kBFloat16).device(A.device()));
-  int status = arcq_matmul_nvfp4_ws(
-      A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(), SFB.data_ptr<uint8_t>(), M, N, K, 1.0f,
-      alpha_a.data_ptr<float>(), alpha_b.has_value() ? alpha_b->data_ptr<float>() : nullptr,
-      C.data_ptr<at::BFloat16>(), nullptr, 0, current_stream(A));
+  const float* pb = alpha_b.has_value() ? alpha_b->data_ptr<float>() : nullptr;
+  int status;
+  if (bias.has_value()) {
+    TORCH_CHECK(bias->scalar_type() == torch::kBFloat16 && bias->is_contiguous() && bias->numel() == N &&
+                bias->device() == A.device(), "bias must be a contiguous bf16 vector of N elements on A's device");
+    status = arcq_matmul_nvfp4_bias(A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(),
+                                    SFB.data_ptr<uint8_t>(), M, N, K, alpha_a.data_ptr<float>(), pb, bias->data_ptr(),
+                                    C.data_ptr<at::BFloat16>(), current_stream(A));
+  } else {
+    status = arcq_matmul_nvfp4_dev_alpha(A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(),
+                                         SFB.data_ptr<uint8_t>(), M, N, K, alpha_a.data_ptr<float>(), pb,
+                                         C.data_ptr<at::BFloat16>(), current_stream(A));
+  }
   check_status(status, "matmul_host_nvfp4_bf16");
+  return C;
+}
+
+// Extra: residual [M, N] + the product, added in the GEMM's epilogue.
+torch::Tensor matmul_residual(const torch::Tensor& A, const torch::Tensor& B, const torch::Tensor& SFA,
+                              const torch::Tensor& SFB, const torch::Tensor& alpha_a,
+                              const c10::optional<torch::Tensor>& alpha_b, const torch::Tensor& residual) {
+  int64_t M, N, K;
+  std::tie(M, N, K) = check_gemm_operands(A, B, SFA, SFB);
+  require_scalar_f32(alpha_a, A, "alpha_a");
+  if (alpha_b.has_value()) require_scalar_f32(*alpha_b, A, "alpha_b");
+  TORCH_CHECK(residual.scalar_type() == torch::kBFloat16 && residual.is_contiguous() && residual.dim() == 2 &&
+              residual.size(0) == M && residual.size(1) == N && residual.device() == A.device(),
+              "residual must be a contiguous bf16 [M, N] tensor on A's device");
+  c10::cuda::CUDAGuard guard(A.device());
+  auto C = torch::empty({M, N}, torch::dtype(torch::kBFloat16).device(A.device()));
+  int status = arcq_matmul_nvfp4_residual(
+      A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(), SFB.data_ptr<uint8_t>(), M, N, K,
+      alpha_a.data_ptr<float>(), alpha_b.has_value() ? alpha_b->data_ptr<float>() : nullptr, residual.data_ptr(),
+      C.data_ptr<at::BFloat16>(), current_stream(A));
+  check_status(status, "matmul_residual");
   return C;
 }
 
@@ -271,7 +301,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rmsnorm_quantize_x", &rmsnorm_quantize_x, "RMSNorm, reorder and quantize activation.", py::arg("X"),
         py::arg("W"), py::arg("eps"), py::arg("reorder_index"), py::arg("KE"));
   m.def("matmul_dev_alpha", &matmul_dev_alpha, "gemm with device-resident global scales", py::arg("A"),
-        py::arg("B"), py::arg("SFA"), py::arg("SFB"), py::arg("alpha_a"), py::arg("alpha_b") = py::none());
+        py::arg("B"), py::arg("SFA"), py::arg("SFB"), py::arg("alpha_a"), py::arg("alpha_b") = py::none(),
+        py::arg("bias") = py::none());
+  m.def("matmul_residual", &matmul_residual, "residual + gemm with device-resident global scales", py::arg("A"), py::arg("B"),
+        py::arg("SFA"), py::arg("SFB"), py::arg("alpha_a"), py::arg("alpha_b"), py::arg("residual"));
   m.def("reorder_quantize_x_scaled", &reorder_quantize_x_scaled, "reorder_quantize_x of X / scale (device scalar)",
         py::arg("X"), py::arg("scale"), py::arg("reorder_index"), py::arg("KE"), py::arg("mode") = -1);
   m.def("quantize_tensor_scale", &quantize_tensor_scale, "(Q, SF, scale) of x or w over its per-tensor scale", py::arg("X"),

@@ -259,6 +259,15 @@ int arcq_matmul_nvfp4_dev_alpha(const uint8_t* A, const uint8_t* B, const uint8_
   return launch_gemm(A, B, SFA, SFB, M, N, K_eff, 1.0f, alpha_a, alpha_b, C, (cudaStream_t)stream);
 }
 
+int arcq_matmul_nvfp4_bias(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M, int64_t N,
+                           int64_t K_eff, const float* alpha_a, const float* alpha_b, const void* bias, void* C, void* stream) {
+  int rc = check_gemm(A, B, SFA, SFB, M, N, K_eff, C);
+  if (rc != ARCQ_OK || M == 0) return rc;
+  if (!alpha_a || !bias) return ARCQ_ERR_NULL_POINTER;
+  if (!aligned16(bias)) return ARCQ_ERR_ALIGNMENT;
+  return launch_gemm(A, B, SFA, SFB, M, N, K_eff, 1.0f, alpha_a, alpha_b, C, (cudaStream_t)stream, bias);
+}
+
 size_t arcq_matmul_workspace_bytes(int64_t M, int64_t N, int64_t K_eff) {
   if (M <= 0 || N <= 0 || K_eff <= 0) return 0;
   return gemm_workspace_bytes(M, N, K_eff);

@@ -49,6 +49,7 @@ struct GemmParams {
   const uint8_t* sfa;
   const uint8_t* sfb;
   __nv_bfloat16* c;
+  const __nv_bfloat16* bias;   // [N], added to the bf16-rounded result, or nullptr
   const float* alpha_a;
   const float* alpha_b;
   float alpha;
@@ -64,6 +65,16 @@ struct GemmParams {
 template <int BN>
 __device__ __forceinline__ constexpr uint32_t instr_desc() {
   return (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+}
+
+// Eight bf16 results plus eight bias values, as a bf16 addition behind the GEMM gives them.
+__device__ __forceinline__ void add_bias8(uint4& o, const __nv_bfloat16* bias) {
+  const uint4 b = __ldg(reinterpret_cast<const uint4*>(bias));
+  auto add = [](uint32_t x, uint32_t y) {
+    return pack_bf16x2(__fadd_rn(__uint_as_float(x << 16), __uint_as_float(y << 16)),
+                       __fadd_rn(__uint_as_float(x & 0xffff0000u), __uint_as_float(y & 0xffff0000u)));
+  };
+  o = make_uint4(add(o.x, b.x), add(o.y, b.y), add(o.z, b.z), add(o.w, b.w));
 }
 
 // ----------------------------------------------------------------------------- kernel
@@ -216,6 +227,7 @@ arcq_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
               o.y = pack_bf16x2(__uint_as_float(r[v * 8 + 2]) * alpha, __uint_as_float(r[v * 8 + 3]) * alpha);
               o.z = pack_bf16x2(__uint_as_float(r[v * 8 + 4]) * alpha, __uint_as_float(r[v * 8 + 5]) * alpha);
               o.w = pack_bf16x2(__uint_as_float(r[v * 8 + 6]) * alpha, __uint_as_float(r[v * 8 + 7]) * alpha);
+              if (p.bias != nullptr) add_bias8(o, p.bias + col + v * 8);
               *reinterpret_cast<uint4*>(crow + col + v * 8) = o;
             }
           }
@@ -309,6 +321,7 @@ __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {   // remote a
 }
 struct Gemm2Params {
   __nv_bfloat16* c;
+  const __nv_bfloat16* bias;   // see GemmParams (plain epilogue only)
   const float* alpha_a;
   const float* alpha_b;
   float alpha;
@@ -607,6 +620,11 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
               const int j = 32 * k + 4 * c;
               const uint32_t addr = slot + (uint32_t)lane * 128u + (uint32_t)((c ^ (lane & 7)) << 4);
               uint32_t out4[4] = {o[j], o[j + 1], o[j + 2], o[j + 3]};
+              if (!RESID && !SWIGLU && p.bias != nullptr && col + 8 * c < ncols) {
+                uint4 b4 = make_uint4(out4[0], out4[1], out4[2], out4[3]);
+                add_bias8(b4, p.bias + col + 8 * c);
+                out4[0] = b4.x; out4[1] = b4.y; out4[2] = b4.z; out4[3] = b4.w;
+              }
               if (RESID) {
                 uint32_t rr[4];
                 asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(rr[0]), "=r"(rr[1]), "=r"(rr[2]), "=r"(rr[3]) : "r"(addr) : "memory");
@@ -746,6 +764,7 @@ int launch_pair(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const ui
   p.groups = groups;
   p.ngroups = ngroups;
   p.c = gp.c;
+  p.bias = gp.bias;
   p.alpha_a = gp.alpha_a;
   p.alpha_b = gp.alpha_b;
   p.alpha = gp.alpha;
@@ -979,17 +998,20 @@ int gemm_plan(int64_t M, int64_t N, int64_t K_eff, int* kind, int* tile_n, int* 
 }
 
 int launch_gemm(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M, int64_t N,
-                int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, void* Cout, cudaStream_t stream) {
+                int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, void* Cout, cudaStream_t stream,
+                const void* bias) {
   DeviceInfo di;
   int rc = get_device_info(&di);
   if (rc != ARCQ_OK) return rc;
   if (use_skinny_kernel(M, N, di.num_sms))
-    return launch_gemm_skinny(A, B, SFA, SFB, M, N, K_eff, alpha, alpha_a, alpha_b, nullptr, Cout, nullptr, nullptr, 1, stream);
+    return launch_gemm_skinny(A, B, SFA, SFB, M, N, K_eff, alpha, alpha_a, alpha_b, bias, Cout, nullptr, nullptr, 1, stream,
+                              bias != nullptr);
 
   GemmParams p;
   p.sfa = SFA;
   p.sfb = SFB;
   p.c = static_cast<__nv_bfloat16*>(Cout);
+  p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.alpha_a = alpha_a;
   p.alpha_b = alpha_b;
   p.alpha = alpha;

@@ -50,7 +50,7 @@ int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight
 int launch_absmax(const void* x, int64_t n, float* out, int accumulate, cudaStream_t stream);
 int launch_gemm(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,
                 int64_t N, int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, void* C,
-                cudaStream_t stream);
+                cudaStream_t stream, const void* bias = nullptr);   // bias: bf16 [N], added to the bf16-rounded result
 size_t gemm_workspace_bytes(int64_t M, int64_t N, int64_t K_eff);
 // Kernel choice for a shape (see arcq_matmul_plan).
 int gemm_plan(int64_t M, int64_t N, int64_t K_eff, int* kind, int* tile_n, int* splits);
@@ -104,7 +104,7 @@ int launch_sum_partials(const void* const* srcs, int n, int64_t elems, const voi
 // Few rows: weight streaming (arcq_skinny.cu).
 int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, const uint8_t* SFW, int64_t M, int64_t N,
                        int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, const void* residual, void* C,
-                       float* swiglu_amax, const int* groups, int ngroups, cudaStream_t stream);
+                       float* swiglu_amax, const int* groups, int ngroups, cudaStream_t stream, bool residual_is_bias = false);
 int skinny_plan_splits(int64_t M, int64_t N, int64_t K_eff);
 int skinny_poll_error();
 int gemm_poll_error();

@@ -53,7 +53,8 @@ struct SkinnyParams {
   const uint8_t* sfx;
   const uint8_t* sfw;
   __nv_bfloat16* c;                  // [M, N], or [M, N/2] with SwiGLU
-  const __nv_bfloat16* residual;     // [M, N] or nullptr
+  const __nv_bfloat16* residual;     // [M, N] (a bias: [N], residual_ld 0) or nullptr
+  int residual_ld;                   // elements between its rows
   const float* alpha_a;
   const float* alpha_b;
   float alpha;
@@ -334,7 +335,7 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                   m = fmaxf(m, fabsf(v));
                   nan |= v != v;
                 } else if (p.residual != nullptr) {
-                  v = bf16_round(__fadd_rn(__bfloat162float(p.residual[at]), v));
+                  v = bf16_round(__fadd_rn(__bfloat162float(p.residual[(size_t)(row0 + c0 + j0 + j) * p.residual_ld + n]), v));
                 }
                 p.c[at] = __float2bfloat16_rn(v);
               }
@@ -429,7 +430,7 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
           float o[4];
           const size_t at = (size_t)(row0 + tok) * ncols + n;
           uint2 res = make_uint2(0, 0);
-          if (!GATED && p.residual != nullptr) res = *reinterpret_cast<const uint2*>(p.residual + at);
+          if (!GATED && p.residual != nullptr) res = *reinterpret_cast<const uint2*>(p.residual + (size_t)(row0 + tok) * p.residual_ld + n);
           const uint32_t rw[2] = {res.x, res.y};
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
@@ -527,7 +528,7 @@ static int skinny_splits_wide(int tiles, int kstages, const DeviceInfo& di) {
 // See SkinnyParams; `residual` and `swiglu_amax` exclude each other; groups (device) with ngroups matrices stacked in W.
 int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, const uint8_t* SFW, int64_t M, int64_t N,
                        int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, const void* residual, void* C,
-                       float* swiglu_amax, const int* groups, int ngroups, cudaStream_t stream) {
+                       float* swiglu_amax, const int* groups, int ngroups, cudaStream_t stream, bool residual_is_bias) {
   DeviceInfo di;
   int rc = get_device_info(&di);
   if (rc != ARCQ_OK) return rc;
@@ -537,6 +538,7 @@ int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, c
   p.sfw = SFW;
   p.c = static_cast<__nv_bfloat16*>(C);
   p.residual = static_cast<const __nv_bfloat16*>(residual);
+  p.residual_ld = residual_is_bias ? 0 : (int)N;
   p.alpha_a = alpha_a;
   p.alpha_b = alpha_b;
   p.alpha = alpha;

@@ -143,7 +143,7 @@ class PackedLinear(torch.nn.Module):
         return self
 
     def gemm(self, qx, sfx, scale_x=None, residual=None):
-        """x W^T (+ residual, added in the GEMM's epilogue: for prefill-sized batches)."""
+        """x W^T (+ residual, added in the GEMM's epilogue)."""
         if residual is not None:
             return ops.matmul_residual(qx, self.W, sfx, self.SFW, self.scale if scale_x is None else scale_x,
                                        None if scale_x is None else self.scale, residual)
@@ -299,8 +299,8 @@ class QLlamaDecoderLayerTP(torch.nn.Module):
         x2d = x.reshape(bsz * seq, hidden).contiguous()
         if self.tp > 1 and x2d.shape[0] >= 2 * self.overlap_rows and self._dist_ready():
             return self._forward_overlapped(x2d, bsz, seq, positions).reshape(bsz, seq, hidden)
-        if self.tp == 1 and self.fuse_residual and x2d.shape[0] >= 1024:
-            # one rank, a prefill-sized batch: both residual additions happen in the epilogues of the o and down GEMMs
+        if self.tp == 1 and self.fuse_residual:
+            # one rank: both residual additions happen in the epilogues of the o and down GEMMs
             h = self.attn_partial(x2d, bsz, seq, positions, residual=x2d)
             return self.mlp_partial(h, residual=h).reshape(bsz, seq, hidden)
         y = self.attn_partial(x2d, bsz, seq, positions)

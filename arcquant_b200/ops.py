@@ -197,11 +197,18 @@ def matmul(a, b, sfa, sfb, scale) -> torch.Tensor:
     return _matmul(a, b, sfa, sfb, float(scale), None, None)
 
 
-def matmul_dev_alpha(a, b, sfa, sfb, alpha_a: torch.Tensor, alpha_b: torch.Tensor | None = None) -> torch.Tensor:
-    """matmul with alpha = alpha_a * alpha_b, both fp32 scalars in device memory."""
+def matmul_dev_alpha(a, b, sfa, sfb, alpha_a: torch.Tensor, alpha_b: torch.Tensor | None = None,
+                     bias: torch.Tensor | None = None) -> torch.Tensor:
+    """matmul with alpha = alpha_a * alpha_b, both fp32 scalars in device memory; plus a bias, in the GEMM's epilogue
+    where it is an aligned bf16 vector on the same device (the same bits either way)."""
+    if bias is not None and (bias.dtype != torch.bfloat16 or bias.device != a.device or bias.dim() != 1 or not bias.is_contiguous()
+                             or bias.numel() != b.shape[0] or bias.data_ptr() % 16):
+        return matmul_dev_alpha(a, b, sfa, sfb, alpha_a, alpha_b) + bias
     ext = _ext()
     if ext:
-        return ext.matmul_dev_alpha(a, b, sfa, sfb, alpha_a, alpha_b)
+        return ext.matmul_dev_alpha(a, b, sfa, sfb, alpha_a, alpha_b, bias)
+    if bias is not None:
+        return _matmul(a, b, sfa, sfb, 1.0, alpha_a, alpha_b) + bias
     return _matmul(a, b, sfa, sfb, 1.0, alpha_a, alpha_b)
 
 
@@ -574,6 +581,9 @@ def matmul_residual(a, b, sfa, sfb, alpha_a: torch.Tensor, alpha_b: torch.Tensor
                     out: torch.Tensor | None = None) -> torch.Tensor:
     """bf16 [M, N] = residual + bf16(alpha_a * alpha_b * (A.SFA)(B.SFB)^T), the addition done in the GEMM's epilogue
     (same bits as `matmul_dev_alpha` followed by a bf16 addition)."""
+    ext = _ext()
+    if ext and out is None:
+        return ext.matmul_residual(a, b, sfa, sfb, alpha_a, alpha_b, residual)
     lib = _lib.load()
     for t, name in ((a, "A"), (b, "B"), (sfa, "SFA"), (sfb, "SFB")):
         _require(t, torch.uint8, name)

@@ -72,11 +72,11 @@ class QLinearLayer(nn.Module):
     def forward(self, x):
         qx, scale_x, scale, bsz, q_len = x
         if isinstance(scale, torch.Tensor) and scale.is_cuda:
-            y = ops.matmul_dev_alpha(qx, self.W, scale_x, self.scale_w, scale, self.scale)
+            y = ops.matmul_dev_alpha(qx, self.W, scale_x, self.scale_w, scale, self.scale, self.bias)
         else:
             y = ops.matmul(qx, self.W, scale_x, self.scale_w, float(scale) * float(self.scale))
-        if self.bias is not None:
-            y = y + self.bias
+            if self.bias is not None:
+                y = y + self.bias
         if bsz is not None:
             return y.reshape(bsz, q_len, -1)
         return y.reshape(q_len, -1)

@@ -150,6 +150,11 @@ int arcq_matmul_nvfp4_dev_alpha(const uint8_t* A, const uint8_t* B, const uint8_
                                 int64_t M, int64_t N, int64_t K_eff, const float* alpha_a,
                                 const float* alpha_b, void* C, void* stream);
 
+/* The same with a bias bf16 [N] (16-byte aligned) added to the bf16-rounded product, C = bf16(bf16(alpha A B^T) + bias):
+ * what `y + self.bias` computes behind the GEMM (model/qLinearLayer.py:70-72). */
+int arcq_matmul_nvfp4_bias(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M, int64_t N,
+                           int64_t K_eff, const float* alpha_a, const float* alpha_b, const void* bias, void* C, void* stream);
+
 /* Problems with few output tiles run faster when K is split over the idle SMs.  The partial sums are exchanged on chip
  * and added in a fixed order, so results are reproducible; no call needs scratch.
  * arcq_matmul_workspace_bytes: the scratch that a split over global memory would take for this shape on the current
@@ -313,7 +318,7 @@ int arcq_matmul_nvfp4_grouped_swiglu(const uint8_t* A, const uint8_t* B, const u
  * The reference adds the residual stream in torch after o_proj and down_proj (`residual + hidden_states`,
  * model/qLlamaLayer.py:162, 168).  arcq_matmul_nvfp4_residual writes C = bf16(R + bf16(alpha_a * alpha_b *
  * A B^T)) - the bits of that addition - with R (bf16 [M, N], may be C itself) fetched tile by tile in the
- * epilogue instead of a pass of its own over [M, N].  Always the CTA-pair kernel (meant for prefill-sized M). */
+ * epilogue instead of a pass of its own over [M, N]. */
 int arcq_matmul_nvfp4_residual(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,
                                int64_t N, int64_t K_eff, const float* alpha_a, const float* alpha_b,
                                const void* residual, void* C, void* stream);

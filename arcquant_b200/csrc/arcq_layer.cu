@@ -744,7 +744,9 @@ int launch_calib_stats(const void* x, int64_t rows, int K, float* chan_absmax, u
   auto cm = reinterpret_cast<unsigned int*>(chan_absmax);
   auto launch = [&](auto kern, int rb) -> int {
     const size_t smem = (size_t)K * 2;
-    if (smem > 48 * 1024) ARCQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // Unasked, a launch gets 48 KB, its static part (below 1 KB here) included.  The limit is the kernel's, not this call's:
+    // always the same value, so that calls of several threads and widths cannot lower one another's.
+    if (smem > 47 * 1024) ARCQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 32768));
     long long grid = (rows + rb - 1) / rb;
     if (grid > 2LL * di.num_sms) grid = 2LL * di.num_sms;
     grid = (grid + CALIB_CLUSTER - 1) / CALIB_CLUSTER * CALIB_CLUSTER;

@@ -487,6 +487,25 @@ def test_calibration_statistics_in_one_pass(k, rows):
     assert torch.equal(eager.value, want) and eager.select_num() == stat.select_num()
 
 
+def test_calibration_of_any_width_as_the_first_call_of_a_process():
+    """Widths at which the kernel's dynamic shared memory alone, or only together with its static part, exceeds the 48 KB
+    that a launch gets unasked; each of them first, since a wider call raises the limit for those that follow."""
+    import os
+    import subprocess
+    import sys
+
+    code = ("import torch\n"
+            "from arcquant_b200.calibrate import ChannelAbsMax\n"
+            "for k in (24576, 24456, 24584, 32768):\n"
+            "    x = torch.randn((9, k), generator=torch.Generator().manual_seed(k)).to(torch.bfloat16).cuda()\n"
+            "    stats = ChannelAbsMax()\n"
+            "    stats.update(x)\n"
+            "    assert torch.equal(stats.value, x.abs().amax(0).float())\n")
+    run = subprocess.run([sys.executable, "-c", code], cwd=os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                         capture_output=True, text=True, timeout=300)
+    assert run.returncode == 0, run.stderr[-2000:]
+
+
 @pytest.mark.parametrize("m,f,kq", [(300, 256, 512), (1000, 2048, 1024), (4100, 7168, 4096), (257, 14336, 4096)])
 def test_swiglu_epilogue_equals_gemm_then_silu(m, f, kq):
     """`matmul_swiglu` over the interleaved gate/up weight against `matmul` over [gate; up] followed by

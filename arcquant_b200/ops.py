@@ -135,9 +135,10 @@ def reorder_quantize_w(w, reorder_index, ke: int, mode=None):
 def quantize_tensor_scale(x, reorder_index, ke: int, mode=None, is_weight: bool = False, amax=None):
     """(codes, scales, scale) of x over its own per-tensor scale max / (448 * 6) - |x| for activations, the signed
     maximum for weights - in two launches (one if `amax`, max|x| on the device, is given), or None where that
-    path does not apply: an empty or non-contiguous tensor, another type, no channel order, KQ > 16384."""
+    path does not apply: an empty or non-contiguous tensor, one off a 16-byte boundary, another type, no channel order,
+    KQ > 16384."""
     if (reorder_index is None or not x.is_cuda or x.dtype != torch.bfloat16 or x.dim() != 2 or not x.is_contiguous()
-            or x.shape[0] == 0 or x.shape[1] > 16384):
+            or x.shape[0] == 0 or x.shape[1] > 16384 or x.data_ptr() % 16):
         return None
     ext = _ext()
     if ext:

@@ -92,3 +92,18 @@ def test_grouped_rows_from_the_runs_maxima(counts, kq):
         assert torch.equal(q[s:s + c], qi)
         run = sf_take_rows(sf, np.arange(s, s + c), kq + ke)
         assert np.array_equal(valid_sf(run, c, kq + ke), valid_sf(sfi, c, kq + ke))
+
+
+def test_a_weight_off_its_alignment_packs_like_its_copy():
+    """A contiguous view at an odd offset of a flat parameter buffer."""
+    from arcquant_b200.qlinear import NVFP4_reorder_quantize_w
+
+    n, kq = 130, 1024
+    flat = synth.weights(1, n * kq + 8, 3, device="cuda").reshape(-1)
+    idx = torch.randperm(kq, generator=torch.Generator().manual_seed(1)).to(torch.int16).cuda()
+    for at in (1, 4):
+        w = flat[at:at + n * kq].view(n, kq)
+        q, sf, s = NVFP4_reorder_quantize_w(w, idx, 64)
+        q2, sf2, s2 = NVFP4_reorder_quantize_w(w.clone(), idx, 64)
+        assert torch.equal(q, q2) and torch.equal(s, s2)
+        assert np.array_equal(valid_sf(sf, n, kq + 64), valid_sf(sf2, n, kq + 64))

@@ -134,15 +134,16 @@ def reorder_quantize_w(w, reorder_index, ke: int, mode=None):
 
 def quantize_tensor_scale(x, reorder_index, ke: int, mode=None, is_weight: bool = False, amax=None):
     """(codes, scales, scale) of x over its own per-tensor scale max / (448 * 6) - |x| for activations, the signed
-    maximum for weights - in two launches (one if `amax`, max|x| on the device, is given), or None where that
-    path does not apply: an empty or non-contiguous tensor, one off a 16-byte boundary, another type, no channel order,
-    KQ > 16384."""
+    maximum for weights - in two launches (one if `amax`, max|x| on the device, is given: the scale then has its
+    shape), or None where that path does not apply: an empty or non-contiguous tensor, one off a 16-byte boundary,
+    another type, no channel order, KQ > 16384."""
     if (reorder_index is None or not x.is_cuda or x.dtype != torch.bfloat16 or x.dim() != 2 or not x.is_contiguous()
             or x.shape[0] == 0 or x.shape[1] > 16384 or x.data_ptr() % 16):
         return None
     ext = _ext()
     if ext:
-        return ext.quantize_tensor_scale(x, reorder_index, ke, -1 if mode is None else mode, is_weight, amax)
+        q, sf, scale = ext.quantize_tensor_scale(x, reorder_index, ke, -1 if mode is None else mode, is_weight, amax)
+        return q, sf, scale if amax is None or amax.dim() == 0 else scale.reshape(amax.shape)
     lib = _lib.load()
     _require(reorder_index, torch.int16, "reorder_index")
     rows, kq = x.shape
@@ -150,9 +151,11 @@ def quantize_tensor_scale(x, reorder_index, ke: int, mode=None, is_weight: bool 
         raise RuntimeError("reorder_index must have KQ entries")
     q = torch.empty((rows, (kq + ke) // 2), dtype=torch.uint8, device=x.device)
     sf = torch.empty((sf_bytes(rows, kq + ke),), dtype=torch.uint8, device=x.device)
-    scale = torch.empty((), dtype=torch.float32, device=x.device)
     if amax is not None:
         _require(amax, torch.float32, "amax")
+        if amax.numel() != 1:
+            raise RuntimeError("amax must be one value")
+    scale = torch.empty(() if amax is None else amax.shape, dtype=torch.float32, device=x.device)
     scratch = torch.empty((_lib.SCALE_SCRATCH,), dtype=torch.float32, device=x.device)
     with torch.cuda.device(x.device):
         rc = lib.arcq_quantize_tensor_scale(x.data_ptr(), None if amax is None else amax.data_ptr(), int(is_weight),

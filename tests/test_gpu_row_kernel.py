@@ -107,3 +107,13 @@ def test_a_weight_off_its_alignment_packs_like_its_copy():
         q2, sf2, s2 = NVFP4_reorder_quantize_w(w.clone(), idx, 64)
         assert torch.equal(q, q2) and torch.equal(s, s2)
         assert np.array_equal(valid_sf(sf, n, kq + 64), valid_sf(sf2, n, kq + 64))
+
+
+@pytest.mark.parametrize("shape", [(), (1,), (1, 1)])
+def test_the_scale_has_the_shape_of_the_given_maximum(shape):
+    from arcquant_b200.qlinear import NVFP4_reorder_quantize_x
+
+    x = synth.activations(5, 1024, 1, synth.outlier_channels(1024, 10, 1), device="cuda")
+    amax = x.abs().max().float().reshape(shape)
+    scale = NVFP4_reorder_quantize_x(x, torch.arange(1024, dtype=torch.int16, device="cuda"), 64, amax=amax)[2]
+    assert scale.shape == amax.shape and torch.equal(scale, amax / 2688.0)

@@ -1683,6 +1683,14 @@ __global__ void __launch_bounds__(512) arcq_max_partials_kernel(const uint4* __r
   }
 }
 
+// The limit of a launch's dynamic shared memory belongs to the kernel on its device, not to the thread that sets it.  So it
+// is always set to what the device has: set to the need of one call, a narrower call of another thread would lower it, and
+// the next wide call of the thread that remembers having set it would be refused.
+template <typename Kernel>
+cudaError_t allow_shared_memory(Kernel kern, const DeviceInfo& di) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem_optin);
+}
+
 template <int R, int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB>
 int launch_rows(const QuantParams& p, int T, const DeviceInfo& di, cudaStream_t stream) {
   auto kern = arcq_quantize_rows_kernel<R, GPT, RMS, SCALED, GROUPED, PF, MAXT, MINB>;
@@ -1692,7 +1700,7 @@ int launch_rows(const QuantParams& p, int T, const DeviceInfo& di, cudaStream_t 
   static thread_local size_t c_smem = 0;
   if (c_dev != di.device || c_threads != T || c_smem != smem) {
     int occ = 0;
-    ARCQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ARCQ_CUDA_TRY(allow_shared_memory(kern, di));
     ARCQ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, T, smem));
     c_dev = di.device; c_threads = T; c_smem = smem; c_occ = occ;
   }
@@ -1728,7 +1736,7 @@ int launch_ws(const QuantParams& p, int nct, int npt, int nteams, int npteams, s
   if (c_dev == di.device && c_threads == threads && c_smem == smem) {
     occ = c_occ;
   } else {
-    ARCQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ARCQ_CUDA_TRY(allow_shared_memory(kern, di));
     ARCQ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem));
     c_dev = di.device; c_threads = threads; c_smem = smem; c_occ = occ;
   }
@@ -1756,7 +1764,7 @@ int launch_ws(const QuantParams& p, int nct, int npt, int nteams, int npteams, s
 template <int CPT, int NBUF, int PAIRS, bool RMS, bool RAWIDX, int MAXT, int MINB>
 int launch_variant(const QuantParams& p, int nt, size_t smem, const DeviceInfo& di, cudaStream_t stream) {
   auto kern = arcq_quantize_kernel<CPT, NBUF, PAIRS, RMS, RAWIDX, MAXT, MINB>;
-  ARCQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  ARCQ_CUDA_TRY(allow_shared_memory(kern, di));
   int occ = 0;
   ARCQ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, nt, smem));
   if (occ < 1) return ARCQ_ERR_UNSUPPORTED_K;

@@ -117,3 +117,23 @@ def test_the_scale_has_the_shape_of_the_given_maximum(shape):
     amax = x.abs().max().float().reshape(shape)
     scale = NVFP4_reorder_quantize_x(x, torch.arange(1024, dtype=torch.int16, device="cuda"), 64, amax=amax)[2]
     assert scale.shape == amax.shape and torch.equal(scale, amax / 2688.0)
+
+
+@pytest.mark.parametrize("rows,widths", [(2, (16384, 14336)), (3000, (2048, 1024)), (3000, (16384, 14336))])
+def test_widths_of_one_kernel_from_two_threads(rows, widths):
+    """The shared-memory limit belongs to the kernel, not to the thread that raised it: a narrower call of another thread
+    must not take it away."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    from arcquant_b200 import ops
+
+    def call(kq):
+        x = synth.activations(rows, kq, 1, synth.outlier_channels(kq, 10, 1), device="cuda")
+        q, _ = ops.reorder_quantize_x(x, torch.arange(kq, dtype=torch.int16, device="cuda"), 64)
+        torch.cuda.synchronize()
+        return q
+
+    with ThreadPoolExecutor(1) as a, ThreadPoolExecutor(1) as b:
+        first = a.submit(call, widths[0]).result()
+        b.submit(call, widths[1]).result()
+        assert torch.equal(a.submit(call, widths[0]).result(), first)

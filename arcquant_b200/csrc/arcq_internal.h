@@ -21,6 +21,9 @@ struct DeviceInfo {
   int num_sms;        // SMs that launches may use (arcq_set_sm_limit)
   int all_sms;
   int max_smem_optin;
+  // CTAs of a launch of which `per_sm` fit an SM at once.  Under a limit one per SM that may be used: the scheduler fills
+  // idle SMs first, so n CTAs may spread over n SMs whatever fits beside them.
+  long long resident(int per_sm) const { return num_sms < all_sms ? num_sms : (long long)num_sms * per_sm; }
 };
 // Cached properties of the current device (queried once per device).
 int get_device_info(DeviceInfo* out);

@@ -1705,7 +1705,7 @@ int launch_rows(const QuantParams& p, int T, const DeviceInfo& di, cudaStream_t 
     c_dev = di.device; c_threads = T; c_smem = smem; c_occ = occ;
   }
   if (c_occ < 1) return ARCQ_ERR_UNSUPPORTED_K;
-  long long grid = (long long)di.num_sms * c_occ;
+  long long grid = di.resident(c_occ);
   const long long units = (p.rows + R - 1) / R;
   if (grid > units) grid = units;
   // Programmatic dependent launch: the grid may be set up while the previous kernel of the stream is
@@ -1741,9 +1741,12 @@ int launch_ws(const QuantParams& p, int nct, int npt, int nteams, int npteams, s
     c_dev = di.device; c_threads = threads; c_smem = smem; c_occ = occ;
   }
   if (occ < 1) return ARCQ_ERR_UNSUPPORTED_K;
-  long long grid = (long long)di.num_sms * occ;
+  long long grid = di.resident(occ);
   if (p.groups == nullptr && grid > p.npairs) grid = p.npairs;
-  if (p.groups != nullptr && grid < p.ngroups) return ARCQ_ERR_BAD_SHAPE;   // every run needs a CTA
+  if (p.groups != nullptr && grid < p.ngroups) {                            // every run needs a CTA
+    if ((long long)di.num_sms * occ < p.ngroups) return ARCQ_ERR_BAD_SHAPE;
+    grid = p.ngroups;
+  }
   // Programmatic dependent launch: the grid may be set up while the previous kernel of the stream is
   // still draining; the kernel itself waits (griddepcontrol.wait) before it touches global memory.
   cudaLaunchConfig_t cfg = {};
@@ -1769,7 +1772,7 @@ int launch_variant(const QuantParams& p, int nt, size_t smem, const DeviceInfo& 
   ARCQ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, nt, smem));
   if (occ < 1) return ARCQ_ERR_UNSUPPORTED_K;
   const long long nunits = (p.npairs + PAIRS - 1) / PAIRS;
-  long long grid = (long long)di.num_sms * occ;
+  long long grid = di.resident(occ);
   if (grid > nunits) grid = nunits;
   kern<<<(unsigned)grid, nt, smem, stream>>>(p);
   ARCQ_CUDA_TRY(cudaGetLastError());
@@ -2018,7 +2021,7 @@ int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight
     const long long nvec = rows * (long long)KQ / 8;
     // four 16-byte loads per thread, at most two CTAs per SM
     long long grid = (nvec + 4 * 512 - 1) / (4 * 512);
-    if (grid > 2LL * di.num_sms) grid = 2LL * di.num_sms;
+    if (grid > di.resident(2)) grid = di.resident(2);
     if (grid > ARCQ_SCALE_SCRATCH) grid = ARCQ_SCALE_SCRATCH;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);

@@ -66,9 +66,12 @@ int arcq_version(void);
 /* The quantizer and GEMM kernels are persistent: by default every launch spreads over all SMs of the
  * device, with one CTA that fills its SM.  A collective that should run at the same time on another
  * stream (an NCCL all-gather or reduce-scatter under the next GEMM) then finds no SM to start on.
- * arcq_set_sm_limit(n) makes every later launch of this process use at most n SMs (0 = all), leaving the
- * rest to whatever else runs; it returns the previous limit.  Process-wide, not per stream; a CUDA graph
- * keeps the grid sizes it was captured with.  No counterpart in the reference (it has no collectives). */
+ * arcq_set_sm_limit(n) makes every later quantizer and GEMM launch of this process use at most n SMs (0 = all): at most
+ * n CTAs.  The rest is left to whatever else runs.  (The small kernels around them - maxima of a tensor, rotary
+ * embedding, routing, sums - end within microseconds and are not limited.)  Returns the previous limit.  Process-wide,
+ * not per stream; a CUDA graph keeps the grid sizes it was captured with.  (A grouped quantizer of many rows needs a CTA
+ * per run: with a limit below the number of runs it takes that many, or - where they do not fit the n SMs together -
+ * refuses with ARCQ_ERR_BAD_SHAPE.)  No counterpart in the reference (it has no collectives). */
 int arcq_set_sm_limit(int sms);
 
 /* Bytes to allocate for the scale-factor buffer of `rows` rows and K_eff =

@@ -109,3 +109,39 @@ def sf_take_rows(sf, rows, k_eff: int) -> np.ndarray:
     out = np.zeros(O.sf_alloc_bytes(len(rows), k_eff), np.uint8)
     out[offsets(np.arange(len(rows)))] = src[offsets(rows)]
     return out
+
+
+def launched_kernels(fn):
+    """[(mangled name, CTAs, bytes of local memory per thread)] of the kernels that fn() launches, in order, read from a
+    stream capture of it.  fn runs once beforehand, so that nothing is loaded for the first time inside the capture."""
+    import ctypes as C
+
+    class Params(C.Structure):      # CUDA_KERNEL_NODE_PARAMS
+        _fields_ = [("func", C.c_void_p)] + [(n, C.c_uint) for n in ("gx", "gy", "gz", "bx", "by", "bz", "smem")] + \
+                   [("args", C.c_void_p), ("extra", C.c_void_p), ("kern", C.c_void_p), ("ctx", C.c_void_p)]
+
+    cu = C.CDLL("libcuda.so.1")
+    fn()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        fn()
+    handle = C.c_void_p(int(graph.raw_cuda_graph()))
+    n = C.c_size_t(0)
+    assert cu.cuGraphGetNodes(handle, None, C.byref(n)) == 0
+    nodes = (C.c_void_p * n.value)()
+    assert cu.cuGraphGetNodes(handle, nodes, C.byref(n)) == 0
+    out = []
+    for node in nodes:
+        kind, local, p, name = C.c_int(-1), C.c_int(-1), Params(), C.c_char_p()
+        assert cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0
+        if kind.value != 0:          # (a memset, a copy)
+            continue
+        assert cu.cuGraphKernelNodeGetParams_v2(C.c_void_p(node), C.byref(p)) == 0
+        func = C.c_void_p(p.func)
+        if not p.func:
+            assert cu.cuKernelGetFunction(C.byref(func), C.c_void_p(p.kern)) == 0
+        assert cu.cuFuncGetName(C.byref(name), func) == 0
+        assert cu.cuFuncGetAttribute(C.byref(local), 3, func) == 0      # CU_FUNC_ATTRIBUTE_LOCAL_SIZE_BYTES
+        out.append((name.value.decode(), p.gx * p.gy * p.gz, local.value))
+    return out

@@ -1,0 +1,57 @@
+"""Under `set_sm_limit(n)` the quantizer and GEMM launches have at most n CTAs - so they occupy at most n SMs, wherever the
+scheduler puts them - and give the same results."""
+import pytest
+import torch
+
+from arcquant_b200 import synth
+from tests.helpers import launched_kernels
+
+pytestmark = pytest.mark.gpu
+
+
+def _x(rows, k):
+    return synth.activations(rows, k, rows + k, synth.outlier_channels(k, max(1, k // 100), 1), device="cuda")
+
+
+def _order(k):
+    return torch.randperm(k, generator=torch.Generator().manual_seed(k)).to(torch.int16).cuda()
+
+
+def _quantizers():
+    from arcquant_b200 import ops
+    from arcquant_b200.qlinear import NVFP4_reorder_quantize_w, NVFP4_reorder_quantize_x
+
+    def rms(rows, k):
+        x, idx, gain = _x(rows, k), _order(k), synth.rms_gain(k, 3).cuda()
+        return lambda: ops.rmsnorm_quantize_x(x, gain, 1e-5, idx, 64)
+
+    def plain(rows, k):
+        x, idx = _x(rows, k), _order(k)
+        return lambda: ops.reorder_quantize_x(x, idx, 32)
+
+    def scaled(rows, k, weight=False):
+        x, idx = _x(rows, k), _order(k)
+        return lambda: (NVFP4_reorder_quantize_w if weight else NVFP4_reorder_quantize_x)(x, idx, 64)
+
+    # the row kernel, the warp-specialised kernel with one and two CTAs per SM, and the kernel of the remaining widths
+    return [rms(16, 4096), rms(500, 4096), rms(5000, 4096), rms(3000, 1024), plain(3000, 256), plain(5000, 512), plain(600, 1024),
+            plain(5000, 1024), plain(16, 14336), plain(300, 18944), scaled(777, 4096), scaled(16, 14336), scaled(400, 4096, True)]
+
+
+@pytest.mark.parametrize("limit", [20, 100])
+@pytest.mark.parametrize("case", range(13))
+def test_quantizers(case, limit):
+    from arcquant_b200 import ops
+
+    call = _quantizers()[case]
+    want = call()
+    before = ops.set_sm_limit(limit)
+    try:
+        kernels = launched_kernels(call)
+        got = call()
+    finally:
+        ops.set_sm_limit(before)
+    torch.cuda.synchronize()
+    assert kernels and all("arcq" in name and ctas <= limit for name, ctas, _ in kernels), kernels
+    assert torch.equal(got[0], want[0])
+    assert all(torch.equal(a, b) for a, b in zip(got[2:], want[2:]))

@@ -892,6 +892,11 @@ static bool use_skinny_kernel(int64_t M, int64_t N, int num_sms) {
 // With the SwiGLU epilogue (gate and up blocks in different CTAs of a cluster): [28672, 4224] 65 rows 24.8 / 30.9 us,
 // 128 rows 26.9 / 31.4, 200 rows 43.1 / 31.6 (CTA pairs with four epilogue warps; eight take about 5 % off).
 constexpr int64_t SKINNY_GATED_ROWS = 128;
+// (At least two CTAs per 256 columns and 128 rows: under an SM limit only where that many may run, see arcq_set_sm_limit.)
+static bool use_skinny_gated(int64_t M, int64_t N, const DeviceInfo& di) {
+  const int64_t ctas = 2 * (N / 256) * ((M + 127) / 128);
+  return M <= SKINNY_GATED_ROWS && (di.num_sms == di.all_sms || ctas <= di.num_sms);
+}
 
 int launch_gemm_grouped(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,
                         int64_t N, int64_t K_eff, const int* tile_group, int ngroups, const float* alpha_a,
@@ -910,7 +915,7 @@ int launch_gemm_grouped(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, 
   p.natoms = (int)((K_eff / 16 + 3) / 4);
   // Few rows per matrix: the weight bytes are the time, and a 256-row tile holds mostly padding (see arcq_skinny.cu).
   // Of a grouped problem the host knows a bound, M = routed rows rounded up to a tile + a tile per matrix.
-  if (tile_group == nullptr && ngroups == 1 && swiglu_amax != nullptr && M <= SKINNY_GATED_ROWS)
+  if (tile_group == nullptr && ngroups == 1 && swiglu_amax != nullptr && use_skinny_gated(M, N, di))
     return launch_gemm_skinny(A, B, SFA, SFB, M, N, K_eff, 1.0f, alpha_a, alpha_b, nullptr, Cout, swiglu_amax, nullptr, 1, stream);
   if (groups != nullptr && M - 256LL * ngroups <= 32LL * ngroups)
     return launch_gemm_skinny(A, B, SFA, SFB, M, N, K_eff, 1.0f, alpha_a, alpha_b, nullptr, Cout, swiglu_amax, groups, ngroups,

@@ -55,3 +55,36 @@ def test_quantizers(case, limit):
     assert kernels and all("arcq" in name and ctas <= limit for name, ctas, _ in kernels), kernels
     assert torch.equal(got[0], want[0])
     assert all(torch.equal(a, b) for a, b in zip(got[2:], want[2:]))
+
+
+def _packed(rows, k):
+    from arcquant_b200 import ops
+
+    return ops.reorder_quantize_x(_x(rows, k), None, 0)
+
+
+@pytest.mark.parametrize("limit", [20, 100])
+@pytest.mark.parametrize("kind,m,n", [("plain", 16, 4096), ("plain", 200, 4096), ("plain", 100, 19200), ("plain", 700, 4096),
+                                      ("residual", 333, 1024), ("swiglu", 1, 512), ("swiglu", 16, 28672), ("swiglu", 64, 3584),
+                                      ("swiglu", 100, 28672), ("swiglu", 128, 512), ("swiglu", 300, 28672)])
+def test_gemms(kind, m, n, limit):
+    from arcquant_b200 import ops
+
+    k = 1088
+    (a, sfa), (b, sfb) = _packed(m, k), _packed(n, k)
+    alpha = torch.tensor(1e-3, device="cuda")
+    res = torch.randn((m, n), generator=torch.Generator().manual_seed(1)).to(torch.bfloat16).cuda()
+    call = {"plain": lambda: ops.matmul_dev_alpha(a, b, sfa, sfb, alpha),
+            "residual": lambda: ops.matmul_residual(a, b, sfa, sfb, alpha, None, res),
+            "swiglu": lambda: ops.matmul_swiglu(a, b, sfa, sfb, alpha, None)[0]}[kind]
+    want = call().double()
+    before = ops.set_sm_limit(limit)
+    try:
+        kernels = launched_kernels(call)
+        got = call().double()
+    finally:
+        ops.set_sm_limit(before)
+    assert ops.gemm_poll_error() == 0
+    assert kernels and all("arcq" in name and ctas <= limit for name, ctas, _ in kernels), kernels
+    # (K may be split differently: an fp32 sum in another order moves an element by one bf16 step now and then)
+    assert float((got - want).norm() / want.norm()) <= 1e-3

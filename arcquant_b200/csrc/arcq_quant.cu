@@ -58,12 +58,10 @@ struct QuantParams {
   const int* groups;
   int ngroups;
   const int* row_map;
-  // Row kernel: the divisor is scale[e] * scale_factor, or - npartials > 0 - the maximum of the `npartials` values
-  // at `scale` times the factor; scale_out (or nullptr) receives it, per run.
-  float scale_factor;
-  float* scale_out;
-  int npartials;
 };
+// (ScaleOptions travels behind it as a kernel parameter of its own.  As three more members of this struct it made ptxas
+// spill in the warp-specialised kernel, whose 64 registers are all in use: fused RMSNorm of 32 768 x 4096 94.4 -> 94.9 us,
+// 16 384 x 8192 divided by their scale 75.4 -> 80.5.)
 
 __device__ __forceinline__ float bf16lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
@@ -770,7 +768,7 @@ __device__ __forceinline__ void div_pair_words(uint32_t wa, uint32_t wb, float s
 // thread's two groups side by side instead of one after the other costs time with 88 and with 104 registers.
 template <bool RMS, bool WIDE, bool SCALED, int S, int R, bool XR = false>
 __global__ void __launch_bounds__(1024, 1) arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const int nteams,
-                                                                        const int npteams) {
+                                                                        const int npteams, const ScaleOptions so) {
   extern __shared__ __align__(16) uint8_t smem[];
   const int tid = threadIdx.x;
   const int KQ = p.KQ, G = p.G;
@@ -793,8 +791,8 @@ __global__ void __launch_bounds__(1024, 1) arcq_quantize_ws_kernel(const QuantPa
     if (scale_g) scale_g += e;
   }
   if (cta >= npairs) {   // (whole CTA: nothing was set up yet)
-    if (SCALED && p.groups != nullptr && p.scale_out != nullptr && blockIdx.x == 0)
-      for (int e = tid; e < p.ngroups; e += blockDim.x) p.scale_out[e] = __ldg(p.scale + e) * p.scale_factor;
+    if (SCALED && p.groups != nullptr && so.out != nullptr && blockIdx.x == 0)
+      for (int e = tid; e < p.ngroups; e += blockDim.x) so.out[e] = __ldg(p.scale + e) * so.factor;
     return;
   }
   const int* row_map = p.row_map;
@@ -990,16 +988,16 @@ __global__ void __launch_bounds__(1024, 1) arcq_quantize_ws_kernel(const QuantPa
     }
 
     auto divisor = [&]() {
-      const float v = p.npartials > 0 ? partials_max(p.scale, p.npartials, lane) : __ldg(scale_g);
-      return v * p.scale_factor;
+      const float v = so.npartials > 0 ? partials_max(p.scale, so.npartials, lane) : __ldg(scale_g);
+      return v * so.factor;
     };
     // (SCALED: the producer team of CTA 0 reports the divisors)
-    if (SCALED && p.scale_out != nullptr && blockIdx.x == 0 && ptid < 32) {
-      if (p.npartials > 0) {
+    if (SCALED && so.out != nullptr && blockIdx.x == 0 && ptid < 32) {
+      if (so.npartials > 0) {
         const float v = divisor();
-        if (lane == 0) p.scale_out[0] = v;
+        if (lane == 0) so.out[0] = v;
       } else {
-        for (int e = lane; e < (p.groups != nullptr ? p.ngroups : 1); e += 32) p.scale_out[e] = __ldg(p.scale + e) * p.scale_factor;
+        for (int e = lane; e < (p.groups != nullptr ? p.ngroups : 1); e += 32) so.out[e] = __ldg(p.scale + e) * so.factor;
       }
     }
     const uint4 zero = make_uint4(0, 0, 0, 0);
@@ -1301,7 +1299,7 @@ __device__ __forceinline__ uint32_t row_pos(uint32_t ch) {      // byte offset o
 }
 
 template <int R, int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB>
-__global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const QuantParams p) {
+__global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const QuantParams p, const ScaleOptions so) {
   constexpr int NW = R / 2, CPT = 2 * GPT;
   static_assert(!RMS || GPT == 1, "RMSNorm: one group per thread");
   extern __shared__ __align__(16) uint8_t smem[];
@@ -1359,14 +1357,14 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
     fast = div_by_reciprocal_ok(sc);
   };
   if (SCALED) {
-    if (p.npartials > 0) {
-      const float m = partials_max(p.scale, p.npartials, lane) * p.scale_factor;
-      if (blockIdx.x == 0 && tid == 0 && p.scale_out != nullptr) p.scale_out[0] = m;
+    if (so.npartials > 0) {
+      const float m = partials_max(p.scale, so.npartials, lane) * so.factor;
+      if (blockIdx.x == 0 && tid == 0 && so.out != nullptr) so.out[0] = m;
       set_scale(m);
     } else {
-      if (p.scale_out != nullptr && blockIdx.x == 0)
-        for (int e = tid; e < ng; e += T) p.scale_out[e] = __ldg(p.scale + e) * p.scale_factor;
-      if (!GROUPED) set_scale(__ldg(p.scale) * p.scale_factor);
+      if (so.out != nullptr && blockIdx.x == 0)
+        for (int e = tid; e < ng; e += T) so.out[e] = __ldg(p.scale + e) * so.factor;
+      if (!GROUPED) set_scale(__ldg(p.scale) * so.factor);
     }
   }
 
@@ -1424,7 +1422,7 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
   seek(unit);
   auto new_run = [&]() {
     load_order(p.idx == nullptr ? nullptr : p.idx + (size_t)e_cur * (size_t)KQ);
-    if (SCALED && GROUPED) set_scale(__ldg(p.scale + e_cur) * p.scale_factor);
+    if (SCALED && GROUPED) set_scale(__ldg(p.scale + e_cur) * so.factor);
   };
   if (PF) load_unit(e_row0 + (unit - e_first) * R, rows_of(unit));
   new_run();
@@ -1692,7 +1690,7 @@ cudaError_t allow_shared_memory(Kernel kern, const DeviceInfo& di) {
 }
 
 template <int R, int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB>
-int launch_rows(const QuantParams& p, int T, const DeviceInfo& di, cudaStream_t stream) {
+int launch_rows(const QuantParams& p, const ScaleOptions& so, int T, const DeviceInfo& di, cudaStream_t stream) {
   auto kern = arcq_quantize_rows_kernel<R, GPT, RMS, SCALED, GROUPED, PF, MAXT, MINB>;
   const size_t smem = (size_t)p.KQ * 2 * R + (RMS ? (size_t)(R * T + R) * sizeof(float) : 64);
   // the attribute and the occupancy query cost host time: once per (device, block size, shared memory)
@@ -1720,13 +1718,13 @@ int launch_rows(const QuantParams& p, int T, const DeviceInfo& di, cudaStream_t 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p));
+  ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p, so));
   return ARCQ_OK;
 }
 
 template <bool RMS, bool WIDE, bool SCALED, int S, int R, bool XR = false>
-int launch_ws(const QuantParams& p, int nct, int npt, int nteams, int npteams, size_t smem, const DeviceInfo& di,
-              cudaStream_t stream) {
+int launch_ws(const QuantParams& p, const ScaleOptions& so, int nct, int npt, int nteams, int npteams, size_t smem,
+              const DeviceInfo& di, cudaStream_t stream) {
   auto kern = arcq_quantize_ws_kernel<RMS, WIDE, SCALED, S, R, XR>;
   const int threads = XR ? 1024 : nteams * nct + npteams * (npt + (RMS ? 96 : 0));
   // the attribute and the occupancy query cost host time: once per (device, block size, shared memory)
@@ -1759,7 +1757,7 @@ int launch_ws(const QuantParams& p, int nct, int npt, int nteams, int npteams, s
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p, nct, npt, nteams, npteams));
+  ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p, nct, npt, nteams, npteams, so));
   ARCQ_CUDA_TRY(cudaGetLastError());
   return ARCQ_OK;
 }
@@ -1843,9 +1841,6 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
   p.groups = groups;
   p.ngroups = ngroups;
   p.row_map = row_map;
-  p.scale_factor = so.factor;
-  p.scale_out = so.out;
-  p.npartials = so.npartials;
 
   const bool rms = gamma != nullptr;
   int nt, cpt;
@@ -1875,16 +1870,16 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
       ((real_rows + 1) / 2 <= per_sm * di.num_sms || (p.G < 32 && !rms))) {
 #define ARCQ_ROWS(RMS_, SC_, GR_)                                                                                   \
   {                                                                                                                 \
-    if (wide) return launch_rows<2, 2, false, SC_, GR_, false, 512, 1>(p, T, di, stream);                           \
-    return T <= 256 ? launch_rows<2, 1, RMS_, SC_, GR_, true, 256, 3>(p, T, di, stream)                             \
-                    : launch_rows<2, 1, RMS_, SC_, GR_, true, 512, 1>(p, T, di, stream);                            \
+    if (wide) return launch_rows<2, 2, false, SC_, GR_, false, 512, 1>(p, so, T, di, stream);                           \
+    return T <= 256 ? launch_rows<2, 1, RMS_, SC_, GR_, true, 256, 3>(p, so, T, di, stream)                             \
+                    : launch_rows<2, 1, RMS_, SC_, GR_, true, 512, 1>(p, so, T, di, stream);                            \
   }
     if (groups != nullptr && scale != nullptr) ARCQ_ROWS(false, true, true)
     if (groups != nullptr) ARCQ_ROWS(false, false, true)
     if (scale != nullptr) ARCQ_ROWS(false, true, false)
     if (!rms) ARCQ_ROWS(false, false, false)
-    return T <= 256 ? launch_rows<2, 1, true, false, false, true, 256, 3>(p, T, di, stream)
-                    : launch_rows<2, 1, true, false, false, true, 512, 1>(p, T, di, stream);
+    return T <= 256 ? launch_rows<2, 1, true, false, false, true, 256, 3>(p, so, T, di, stream)
+                    : launch_rows<2, 1, true, false, false, true, 512, 1>(p, so, T, di, stream);
 #undef ARCQ_ROWS
   }
 
@@ -1907,13 +1902,13 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
       const size_t smem = fixed + 2 * stage + (size_t)R * (stage / 2);
       if (R >= 2) {
         if (p.scale) {
-          if (R == 4) return launch_ws<false, true, true, 2, 4>(p, nct, npt, nteams, 1, smem, di, stream);
-          if (R == 3) return launch_ws<false, true, true, 2, 3>(p, nct, npt, nteams, 1, smem, di, stream);
-          return launch_ws<false, true, true, 2, 2>(p, nct, npt, nteams, 1, smem, di, stream);
+          if (R == 4) return launch_ws<false, true, true, 2, 4>(p, so, nct, npt, nteams, 1, smem, di, stream);
+          if (R == 3) return launch_ws<false, true, true, 2, 3>(p, so, nct, npt, nteams, 1, smem, di, stream);
+          return launch_ws<false, true, true, 2, 2>(p, so, nct, npt, nteams, 1, smem, di, stream);
         }
-        if (R == 4) return launch_ws<false, true, false, 2, 4>(p, nct, npt, nteams, 1, smem, di, stream);
-        if (R == 3) return launch_ws<false, true, false, 2, 3>(p, nct, npt, nteams, 1, smem, di, stream);
-        return launch_ws<false, true, false, 2, 2>(p, nct, npt, nteams, 1, smem, di, stream);
+        if (R == 4) return launch_ws<false, true, false, 2, 4>(p, so, nct, npt, nteams, 1, smem, di, stream);
+        if (R == 3) return launch_ws<false, true, false, 2, 3>(p, so, nct, npt, nteams, 1, smem, di, stream);
+        return launch_ws<false, true, false, 2, 2>(p, so, nct, npt, nteams, 1, smem, di, stream);
       }
     } else {
       // Consumer teams of 128 threads (two groups per thread at hidden 4096) were measured faster than
@@ -1958,14 +1953,14 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
         const int ncons = nteams * nct;
         if (kind == 0 && (ncons == 128 || ncons == 256) && ncons + npteams * ptt > 512) {
 #define ARCQ_WS_XR(S_, R_) \
-  if (S == S_ && R == R_) return launch_ws<true, false, false, S_, R_, true>(p, nct, npt, nteams, npteams, smem, di, stream);
+  if (S == S_ && R == R_) return launch_ws<true, false, false, S_, R_, true>(p, so, nct, npt, nteams, npteams, smem, di, stream);
           ARCQ_WS_XR(2, 2) ARCQ_WS_XR(2, 4) ARCQ_WS_XR(2, 6) ARCQ_WS_XR(2, 8)
           ARCQ_WS_XR(4, 2) ARCQ_WS_XR(4, 4) ARCQ_WS_XR(4, 6) ARCQ_WS_XR(4, 8)
 #undef ARCQ_WS_XR
         }
 #define ARCQ_WS_CASE(KIND_, RMS_, SCALED_, S_, R_) \
   if (kind == KIND_ && S == S_ && R == R_) \
-    return launch_ws<RMS_, false, SCALED_, S_, R_>(p, nct, npt, nteams, npteams, smem, di, stream);
+    return launch_ws<RMS_, false, SCALED_, S_, R_>(p, so, nct, npt, nteams, npteams, smem, di, stream);
 #define ARCQ_WS_ROW(KIND_, RMS_, SCALED_, S_)                                                          \
   ARCQ_WS_CASE(KIND_, RMS_, SCALED_, S_, 2) ARCQ_WS_CASE(KIND_, RMS_, SCALED_, S_, 4)                  \
   ARCQ_WS_CASE(KIND_, RMS_, SCALED_, S_, 6) ARCQ_WS_CASE(KIND_, RMS_, SCALED_, S_, 8)

@@ -53,7 +53,7 @@ def test_fused_rmsnorm_of_few_rows(rows, kq):
     assert np.array_equal(valid_sf(sf, rows, kq + 64), valid_sf(so, rows, kq + 64))
 
 
-@pytest.mark.parametrize("counts,kq", [((1, 0, 5, 2), 4096), ((0, 0, 3, 255), 14336), ((300, 257, 1, 0), 1024)])
+@pytest.mark.parametrize("counts,kq", [((1, 0, 5, 2), 4096), ((0, 0, 3, 255), 14336), ((300, 257, 1, 0), 1024), ((3, 0, 0, 2) * 10, 2048)])
 def test_grouped_rows_from_the_runs_maxima(counts, kq):
     """Runs with their own maximum, order and divisor equal the per-run calls; an odd run length and an empty run."""
     from arcquant_b200 import _lib, ops

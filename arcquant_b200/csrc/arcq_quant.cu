@@ -751,6 +751,10 @@ __device__ __forceinline__ void div_pair_words(uint32_t wa, uint32_t wb, float s
   }
 }
 
+// How the plain operator's divisor comes about: none; *scale, as it is; or by ScaleOptions.  (One instance for the last two
+// made the plain division 1 - 2 % slower: 16 384 x 14 336 145.4 -> 147.1 us, 880 rows 12.4 -> 12.7.)
+enum { DIV_NONE = 0, DIV_GIVEN = 1, DIV_MAXIMA = 2 };
+
 // S: stages of the gather ring (interleaved row pairs).  R: stages of the raw ring (row pairs as they
 // lie in global memory, filled by bulk copies - this is what keeps enough bytes in flight to cover
 // the HBM latency).  RMS: fused RMSNorm.  WIDE (plain only): rows of more than 8192 channels - the offset
@@ -766,9 +770,10 @@ __device__ __forceinline__ void div_pair_words(uint32_t wa, uint32_t wb, float s
 // slower: 48 / 104 (0.105 ms) and 40 / 128 (0.152 ms) starve the producers; helper warps cut to 32 or 48
 // registers in warpgroups of their own double the time (the reducers sit on the critical path); quantizing a
 // thread's two groups side by side instead of one after the other costs time with 88 and with 104 registers.
-template <bool RMS, bool WIDE, bool SCALED, int S, int R, bool XR = false>
-__global__ void __launch_bounds__(1024, 1) arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const int nteams,
-                                                                        const int npteams, const ScaleOptions so) {
+template <bool RMS, bool WIDE, int DIV, int S, int R, bool XR = false>
+__global__ void __launch_bounds__(1024, 1)
+arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const int nteams, const int npteams, const ScaleOptions so) {
+  constexpr bool SCALED = DIV != DIV_NONE;
   extern __shared__ __align__(16) uint8_t smem[];
   const int tid = threadIdx.x;
   const int KQ = p.KQ, G = p.G;
@@ -791,7 +796,7 @@ __global__ void __launch_bounds__(1024, 1) arcq_quantize_ws_kernel(const QuantPa
     if (scale_g) scale_g += e;
   }
   if (cta >= npairs) {   // (whole CTA: nothing was set up yet)
-    if (SCALED && p.groups != nullptr && so.out != nullptr && blockIdx.x == 0)
+    if (DIV == DIV_MAXIMA && p.groups != nullptr && so.out != nullptr && blockIdx.x == 0)
       for (int e = tid; e < p.ngroups; e += blockDim.x) so.out[e] = __ldg(p.scale + e) * so.factor;
     return;
   }
@@ -988,11 +993,12 @@ __global__ void __launch_bounds__(1024, 1) arcq_quantize_ws_kernel(const QuantPa
     }
 
     auto divisor = [&]() {
+      if (DIV == DIV_GIVEN) return __ldg(scale_g);
       const float v = so.npartials > 0 ? partials_max(p.scale, so.npartials, lane) : __ldg(scale_g);
       return v * so.factor;
     };
-    // (SCALED: the producer team of CTA 0 reports the divisors)
-    if (SCALED && so.out != nullptr && blockIdx.x == 0 && ptid < 32) {
+    // (the producer team of CTA 0 reports the divisors)
+    if (DIV == DIV_MAXIMA && so.out != nullptr && blockIdx.x == 0 && ptid < 32) {
       if (so.npartials > 0) {
         const float v = divisor();
         if (lane == 0) so.out[0] = v;
@@ -1739,10 +1745,10 @@ int launch_rows(const QuantParams& p, const ScaleOptions& so, int T, const Devic
   return ARCQ_OK;
 }
 
-template <bool RMS, bool WIDE, bool SCALED, int S, int R, bool XR = false>
+template <bool RMS, bool WIDE, int DIV, int S, int R, bool XR = false>
 int launch_ws(const QuantParams& p, const ScaleOptions& so, int nct, int npt, int nteams, int npteams, size_t smem,
               const DeviceInfo& di, cudaStream_t stream) {
-  auto kern = arcq_quantize_ws_kernel<RMS, WIDE, SCALED, S, R, XR>;
+  auto kern = arcq_quantize_ws_kernel<RMS, WIDE, DIV, S, R, XR>;
   const int threads = XR ? 1024 : nteams * nct + npteams * (npt + (RMS ? 96 : 0));
   // the attribute and the occupancy query cost host time: once per (device, block size, shared memory)
   static thread_local int c_dev = -1, c_threads = 0, c_occ = 0;
@@ -1906,6 +1912,7 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
   if (gamma_ok && p.G >= 32 && (!rms || (p.G % 32 == 0 && p.G >= 64)) && rows < (1LL << 30) &&
       (wide ? (!rms && p.G <= 1024) : true)) {
     const size_t stage = (size_t)KQ * 4;
+    const int div = p.scale == nullptr ? DIV_NONE : (so.npartials > 0 || so.out != nullptr ? DIV_MAXIMA : DIV_GIVEN);
     if (wide) {
       // 256 producers, two consumer teams of 256, two gather stages, 16-bit offset table; one raw
       // stage (two if they fit)
@@ -1918,14 +1925,14 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
       if (R > 4) R = 4;
       const size_t smem = fixed + 2 * stage + (size_t)R * (stage / 2);
       if (R >= 2) {
-        if (p.scale) {
-          if (R == 4) return launch_ws<false, true, true, 2, 4>(p, so, nct, npt, nteams, 1, smem, di, stream);
-          if (R == 3) return launch_ws<false, true, true, 2, 3>(p, so, nct, npt, nteams, 1, smem, di, stream);
-          return launch_ws<false, true, true, 2, 2>(p, so, nct, npt, nteams, 1, smem, di, stream);
-        }
-        if (R == 4) return launch_ws<false, true, false, 2, 4>(p, so, nct, npt, nteams, 1, smem, di, stream);
-        if (R == 3) return launch_ws<false, true, false, 2, 3>(p, so, nct, npt, nteams, 1, smem, di, stream);
-        return launch_ws<false, true, false, 2, 2>(p, so, nct, npt, nteams, 1, smem, di, stream);
+#define ARCQ_WS_WIDE(DIV_)                                                                                     \
+  if (div == DIV_) {                                                                                            \
+    if (R == 4) return launch_ws<false, true, DIV_, 2, 4>(p, so, nct, npt, nteams, 1, smem, di, stream);        \
+    if (R == 3) return launch_ws<false, true, DIV_, 2, 3>(p, so, nct, npt, nteams, 1, smem, di, stream);        \
+    return launch_ws<false, true, DIV_, 2, 2>(p, so, nct, npt, nteams, 1, smem, di, stream);                    \
+  }
+        ARCQ_WS_WIDE(DIV_NONE) ARCQ_WS_WIDE(DIV_GIVEN) ARCQ_WS_WIDE(DIV_MAXIMA)
+#undef ARCQ_WS_WIDE
       }
     } else {
       // Consumer teams of 128 threads (two groups per thread at hidden 4096) were measured faster than
@@ -1962,28 +1969,28 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
       while (R > r_floor && fixed + (S + R) * stage > (size_t)di.max_smem_optin) R -= 2;
       const size_t smem = fixed + (S + R) * stage;
       if (nteams >= 1 && smem <= (size_t)di.max_smem_optin) {
-        const int kind = rms ? 0 : (p.scale ? 2 : 1);   // RMSNorm / plain / plain with the division
         // Fused RMSNorm with one or two whole warpgroups of consumers: registers move from the other warps to them
         // (1024 - ncons warps' worth at 56 leave at least 88 for the consumers).
         // (Only where one CTA per SM is the rule anyway: narrow rows, whose CTAs are small enough for two per
         // SM, keep their own thread count.)
         const int ncons = nteams * nct;
-        if (kind == 0 && (ncons == 128 || ncons == 256) && ncons + npteams * ptt > 512) {
+        if (rms && (ncons == 128 || ncons == 256) && ncons + npteams * ptt > 512) {
 #define ARCQ_WS_XR(S_, R_) \
-  if (S == S_ && R == R_) return launch_ws<true, false, false, S_, R_, true>(p, so, nct, npt, nteams, npteams, smem, di, stream);
+  if (S == S_ && R == R_) return launch_ws<true, false, DIV_NONE, S_, R_, true>(p, so, nct, npt, nteams, npteams, smem, di, stream);
           ARCQ_WS_XR(2, 2) ARCQ_WS_XR(2, 4) ARCQ_WS_XR(2, 6) ARCQ_WS_XR(2, 8)
           ARCQ_WS_XR(4, 2) ARCQ_WS_XR(4, 4) ARCQ_WS_XR(4, 6) ARCQ_WS_XR(4, 8)
 #undef ARCQ_WS_XR
         }
-#define ARCQ_WS_CASE(KIND_, RMS_, SCALED_, S_, R_) \
-  if (kind == KIND_ && S == S_ && R == R_) \
-    return launch_ws<RMS_, false, SCALED_, S_, R_>(p, so, nct, npt, nteams, npteams, smem, di, stream);
-#define ARCQ_WS_ROW(KIND_, RMS_, SCALED_, S_)                                                          \
-  ARCQ_WS_CASE(KIND_, RMS_, SCALED_, S_, 2) ARCQ_WS_CASE(KIND_, RMS_, SCALED_, S_, 4)                  \
-  ARCQ_WS_CASE(KIND_, RMS_, SCALED_, S_, 6) ARCQ_WS_CASE(KIND_, RMS_, SCALED_, S_, 8)
-        ARCQ_WS_ROW(0, true, false, 2) ARCQ_WS_ROW(0, true, false, 4)
-        ARCQ_WS_ROW(1, false, false, 2) ARCQ_WS_ROW(1, false, false, 4)
-        ARCQ_WS_ROW(2, false, true, 2) ARCQ_WS_ROW(2, false, true, 4)
+#define ARCQ_WS_CASE(RMS_, DIV_, S_, R_)                 \
+  if (rms == RMS_ && div == DIV_ && S == S_ && R == R_) \
+    return launch_ws<RMS_, false, DIV_, S_, R_>(p, so, nct, npt, nteams, npteams, smem, di, stream);
+#define ARCQ_WS_ROW(RMS_, DIV_, S_)                                              \
+  ARCQ_WS_CASE(RMS_, DIV_, S_, 2) ARCQ_WS_CASE(RMS_, DIV_, S_, 4)                \
+  ARCQ_WS_CASE(RMS_, DIV_, S_, 6) ARCQ_WS_CASE(RMS_, DIV_, S_, 8)
+        ARCQ_WS_ROW(true, DIV_NONE, 2) ARCQ_WS_ROW(true, DIV_NONE, 4)
+        ARCQ_WS_ROW(false, DIV_NONE, 2) ARCQ_WS_ROW(false, DIV_NONE, 4)
+        ARCQ_WS_ROW(false, DIV_GIVEN, 2) ARCQ_WS_ROW(false, DIV_GIVEN, 4)
+        ARCQ_WS_ROW(false, DIV_MAXIMA, 2) ARCQ_WS_ROW(false, DIV_MAXIMA, 4)
 #undef ARCQ_WS_ROW
 #undef ARCQ_WS_CASE
       }

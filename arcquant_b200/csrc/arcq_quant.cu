@@ -770,8 +770,10 @@ enum { DIV_NONE = 0, DIV_GIVEN = 1, DIV_MAXIMA = 2 };
 // slower: 48 / 104 (0.105 ms) and 40 / 128 (0.152 ms) starve the producers; helper warps cut to 32 or 48
 // registers in warpgroups of their own double the time (the reducers sit on the critical path); quantizing a
 // thread's two groups side by side instead of one after the other costs time with 88 and with 104 registers.
+// (The wide plain operator has 256 producers and 512 consumers: 80 registers each instead of 64 and a spill, 16 384 x 14 336
+// 135.1 -> 127.5 us, 880 x 14 336 11.6 -> 11.1.)
 template <bool RMS, bool WIDE, int DIV, int S, int R, bool XR = false>
-__global__ void __launch_bounds__(1024, 1)
+__global__ void __launch_bounds__(WIDE && DIV == DIV_NONE ? 768 : 1024, 1)
 arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const int nteams, const int npteams, const ScaleOptions so) {
   constexpr bool SCALED = DIV != DIV_NONE;
   extern __shared__ __align__(16) uint8_t smem[];

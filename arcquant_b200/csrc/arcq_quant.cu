@@ -1715,7 +1715,7 @@ cudaError_t allow_shared_memory(Kernel kern, const DeviceInfo& di) {
 }
 
 template <int R, int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB>
-int launch_rows(const QuantParams& p, const ScaleOptions& so, int T, const DeviceInfo& di, cudaStream_t stream) {
+int launch_rows(const QuantParams& p, const ScaleOptions& so, long long units, int T, const DeviceInfo& di, cudaStream_t stream) {
   auto kern = arcq_quantize_rows_kernel<R, GPT, RMS, SCALED, GROUPED, PF, MAXT, MINB>;
   const size_t smem = (size_t)p.KQ * 2 * R + (RMS ? (size_t)(R * T + R) * sizeof(float) : 64);
   // the attribute and the occupancy query cost host time: once per (device, block size, shared memory)
@@ -1728,15 +1728,20 @@ int launch_rows(const QuantParams& p, const ScaleOptions& so, int T, const Devic
     c_dev = di.device; c_threads = T; c_smem = smem; c_occ = occ;
   }
   if (c_occ < 1) return ARCQ_ERR_UNSUPPORTED_K;
-  long long grid = di.resident(c_occ);
-  const long long units = (p.rows + R - 1) / R;
-  if (grid > units) grid = units;
+  // No more CTAs per SM than the units need, by shared memory asked for: set up early, while the kernel before still holds
+  // most SMs, several of them would crowd on the first SMs that come free
+  // (290 rows of 4096 channels, call after call 3.8 -> 2.7 us; with RMSNorm and the GEMM [6144, 4224] 17.3 -> 15.3).
+  const long long need = (units + di.num_sms - 1) / di.num_sms;
+  const int per_sm = need < c_occ ? (int)need : c_occ;
+  const size_t share = per_sm < c_occ ? ((size_t)di.max_smem_optin + 1024) / (per_sm + 1) : 0;
+  long long grid = di.resident(per_sm);
+  if (grid > (p.rows + R - 1) / R) grid = (p.rows + R - 1) / R;
   // Programmatic dependent launch: the grid may be set up while the previous kernel of the stream is
   // still draining; the kernel itself waits (griddepcontrol.wait) before it touches global memory.
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3((unsigned)T);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = std::max(smem, share);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1889,22 +1894,23 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
   // 5.3, 16 rows of 14336 channels 6.8 -> 5.5.  Beyond it the warp-specialised kernel below streams better (fused
   // RMSNorm, 16 384 rows: 50.6 against 60.7 us).  With grouped rows the host knows a bound only.
   const long long real_rows = groups != nullptr ? std::max<long long>(rows - 256LL * ngroups, 1) : rows;
+  const long long units = (real_rows + 1) / 2;
   const int T = wide ? ((p.G + 1) / 2 + 31) / 32 * 32 : (p.G + 31) / 32 * 32;
   const long long per_sm = T <= 256 ? (rms ? 2 : 3) : 1;
   if (gamma_ok && p.G <= 1024 && !(rms && wide) && (row_map == nullptr || groups != nullptr) && rows < (1LL << 30) &&
-      ((real_rows + 1) / 2 <= per_sm * di.num_sms || (p.G < 32 && !rms))) {
+      (units <= per_sm * di.num_sms || (p.G < 32 && !rms))) {
 #define ARCQ_ROWS(RMS_, SC_, GR_)                                                                                   \
   {                                                                                                                 \
-    if (wide) return launch_rows<2, 2, false, SC_, GR_, false, 512, 1>(p, so, T, di, stream);                           \
-    return T <= 256 ? launch_rows<2, 1, RMS_, SC_, GR_, true, 256, 3>(p, so, T, di, stream)                             \
-                    : launch_rows<2, 1, RMS_, SC_, GR_, true, 512, 1>(p, so, T, di, stream);                            \
+    if (wide) return launch_rows<2, 2, false, SC_, GR_, false, 512, 1>(p, so, units, T, di, stream);                           \
+    return T <= 256 ? launch_rows<2, 1, RMS_, SC_, GR_, true, 256, 3>(p, so, units, T, di, stream)                             \
+                    : launch_rows<2, 1, RMS_, SC_, GR_, true, 512, 1>(p, so, units, T, di, stream);                            \
   }
     if (groups != nullptr && scale != nullptr) ARCQ_ROWS(false, true, true)
     if (groups != nullptr) ARCQ_ROWS(false, false, true)
     if (scale != nullptr) ARCQ_ROWS(false, true, false)
     if (!rms) ARCQ_ROWS(false, false, false)
-    return T <= 256 ? launch_rows<2, 1, true, false, false, true, 256, 3>(p, so, T, di, stream)
-                    : launch_rows<2, 1, true, false, false, true, 512, 1>(p, so, T, di, stream);
+    return T <= 256 ? launch_rows<2, 1, true, false, false, true, 256, 3>(p, so, units, T, di, stream)
+                    : launch_rows<2, 1, true, false, false, true, 512, 1>(p, so, units, T, di, stream);
 #undef ARCQ_ROWS
   }
 

@@ -94,12 +94,13 @@ __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
   return v;
 }
-__device__ __forceinline__ float bf16_round(float v) {
-  return __uint_as_float((uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v)) << 16);
+__device__ __forceinline__ uint32_t swiglu_bf16x2(uint32_t g, uint32_t u) {
+  const uint32_t s = pack_bf16x2(silu_for_bf16(__uint_as_float(g << 16)), silu_for_bf16(__uint_as_float(g & 0xffff0000u)));
+  return pack_bf16x2(__uint_as_float(s << 16) * __uint_as_float(u << 16), __uint_as_float(s & 0xffff0000u) * __uint_as_float(u & 0xffff0000u));
 }
-__device__ __forceinline__ float swiglu_bf16(float g, float u) {   // both already bf16 values
-  const float s = bf16_round(__fdiv_rn(g, __fadd_rn(1.0f, expf(-g))));
-  return bf16_round(__fmul_rn(s, u));
+__device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {   // in fp32, rounded once
+  return pack_bf16x2(__fadd_rn(__uint_as_float(a << 16), __uint_as_float(b << 16)),
+                     __fadd_rn(__uint_as_float(a & 0xffff0000u), __uint_as_float(b & 0xffff0000u)));
 }
 
 // NT: token columns per pass.  GATED: SwiGLU.  SPLIT: more than one CTA per cluster.
@@ -268,14 +269,30 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     const int nl = quad * 32 + lane;                       // weight row within the tile
     uint32_t acc_it = 0;
     bool ok = true;
+    const int ncols = GATED ? p.N >> 1 : p.N;
+    // (unsplit) the residual of the next AHEAD tokens of this lane's four columns
+    constexpr int AHEAD = NT < 64 ? NT : 64;
+    uint2 res[AHEAD / 4];
+    auto fetch_residual = [&](int row, int rows_here, int col) {
+      if constexpr (!GATED) {
+        if (p.residual == nullptr) return;
+#pragma unroll
+        for (int k = 0; k < AHEAD / 4; ++k) {
+          const int tok = 4 * k + (lane & 3);
+          if (tok < rows_here && col < ncols) res[k] = *reinterpret_cast<const uint2*>(p.residual + (size_t)(row + tok) * p.residual_ld + col);
+        }
+      }
+    };
     for (int item = first_item; item < num_items && ok; item += item_step) {
       const int wt = item / ttiles, g = wt / p.tiles, t = wt - g * p.tiles;
+      const int n4 = t * 128 + quad * 32 + (lane & ~3);    // (unsplit) first of this lane's four output columns
       int row0, cnt;
       run_of(item, row0, cnt);
       float alpha = p.alpha;
       if (p.alpha_a) alpha *= __ldg(p.alpha_a + g);
       if (p.alpha_b) alpha *= __ldg(p.alpha_b + g);
       for (int c0 = 0; c0 < cnt; c0 += NT, ++acc_it) {
+        if (!SPLIT) fetch_residual(row0 + c0, min(NT, cnt - c0), n4);     // (while the products are still being formed)
         ok = mbar_wait(acc_full_bar, acc_it & 1u, abort_flag);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
@@ -316,34 +333,51 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             }
           }
         } else {
-          const int n = t * 128 + nl;                      // output column
-          const int ncols = GATED ? p.N >> 1 : p.N;
-          float m = 0.f;
-          bool nan = false;
-          for (int j0 = 0; j0 < here; j0 += 16) {
-            uint32_t r[16], u[16];
-            tc_ld16(t_row + j0, r);
-            if (GATED) tc_ld16(t_row + (NA - 1) * NT + j0, u);
-            tc_wait_ld();
+          // A lane holds one column of 16 tokens; two exchanges between neighbouring lanes leave it four columns of the
+          // tokens 4 k + lane % 4, which go out as 8-byte stores.  (Element by element - 16 stores, 16 dependent loads of
+          // the residual - a pass of 64 tokens cost more than its weight stream, us: [256, 576] 128 rows 14.5 -> 6.5, with
+          // a residual 33.9 -> 8.9; grouped SwiGLU [7168, 2176], 256 rows of one run out of eight 80.0 -> 51.3.)
+          uint32_t m = 0;                                  // max|C| of two tokens
+#pragma unroll 1
+          for (int h0 = 0; h0 < here; h0 += AHEAD) {
+            if (h0 > 0) fetch_residual(row0 + c0 + h0, here - h0, n4);
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              if (j0 + j < here && n < ncols) {
-                const size_t at = (size_t)(row0 + c0 + j0 + j) * ncols + n;
-                float v = bf16_round(__uint_as_float(r[j]) * alpha);
-                if (GATED) {
-                  v = swiglu_bf16(v, bf16_round(__uint_as_float(u[j]) * alpha));
-                  m = fmaxf(m, fabsf(v));
-                  nan |= v != v;
-                } else if (p.residual != nullptr) {
-                  v = bf16_round(__fadd_rn(__bfloat162float(p.residual[(size_t)(row0 + c0 + j0 + j) * p.residual_ld + n]), v));
+            for (int b = 0; b < AHEAD / 16; ++b) {
+              const int j0 = h0 + 16 * b;
+              if (j0 >= here) break;
+              uint32_t r[16], u[16], o[8];
+              tc_ld16(t_row + j0, r);
+              if (GATED) tc_ld16(t_row + (NA - 1) * NT + j0, u);
+              tc_wait_ld();
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {                // tokens 2 i, 2 i + 1
+                o[i] = pack_bf16x2(__uint_as_float(r[2 * i]) * alpha, __uint_as_float(r[2 * i + 1]) * alpha);
+                if (GATED) o[i] = swiglu_bf16x2(o[i], pack_bf16x2(__uint_as_float(u[2 * i]) * alpha, __uint_as_float(u[2 * i + 1]) * alpha));
+              }
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {                // token 2 i + lane % 2, two columns
+                const uint32_t x = __shfl_xor_sync(0xffffffffu, o[i], 1);
+                o[i] = (lane & 1) ? __byte_perm(x, o[i], 0x7632) : __byte_perm(o[i], x, 0x5410);
+              }
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {                // token 4 k + lane % 4, four columns
+                const uint32_t x = __shfl_xor_sync(0xffffffffu, (lane & 2) ? o[2 * k] : o[2 * k + 1], 2);
+                uint2 v = (lane & 2) ? make_uint2(x, o[2 * k + 1]) : make_uint2(o[2 * k], x);
+                const int tok = j0 + 4 * k + (lane & 3);
+                if (tok < here && n4 < ncols) {
+                  if (GATED) {
+                    asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(v.x & 0x7fff7fffu));
+                    asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(v.y & 0x7fff7fffu));
+                  } else if (p.residual != nullptr) {
+                    v = make_uint2(add_bf16x2(res[4 * b + k].x, v.x), add_bf16x2(res[4 * b + k].y, v.y));
+                  }
+                  *reinterpret_cast<uint2*>(p.c + (size_t)(row0 + c0 + tok) * ncols + n4) = v;
                 }
-                p.c[at] = __float2bfloat16_rn(v);
               }
             }
           }
-          if (GATED) {
-            if (nan) m = __uint_as_float(0x7fff0000u);     // (a NaN counts as larger than everything, as in the other epilogues)
-            uint32_t mi = __float_as_uint(m);
+          if (GATED) {       // (a NaN counts as larger than everything, as in the other epilogues)
+            uint32_t mi = max(m & 0xffffu, m >> 16) << 16;
 #pragma unroll
             for (int d = 16; d > 0; d >>= 1) mi = max(mi, __shfl_xor_sync(0xffffffffu, mi, d));
             if (lane == 0 && mi) atomicMax(p.amax + g, mi);
@@ -407,7 +441,7 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       float alpha = p.alpha;
       if (p.alpha_a) alpha *= __ldg(p.alpha_a);
       if (p.alpha_b) alpha *= __ldg(p.alpha_b);
-      uint32_t mi = 0;
+      uint32_t m = 0;                                      // max|C|, two columns
       const float4* part = reinterpret_cast<const float4*>(base_ptr + C::STAGES * C::STAGE_BYTES);
       // four neighbouring columns of one of this CTA's tokens per thread and step
       for (int i = threadIdx.x;; i += SK_THREADS) {
@@ -427,27 +461,23 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         }
         const int n = t * 128 + n4;
         if (n < ncols) {                                   // (a multiple of four columns is in or out: N % 8 == 0)
-          float o[4];
           const size_t at = (size_t)(row0 + tok) * ncols + n;
-          uint2 res = make_uint2(0, 0);
-          if (!GATED && p.residual != nullptr) res = *reinterpret_cast<const uint2*>(p.residual + (size_t)(row0 + tok) * p.residual_ld + n);
-          const uint32_t rw[2] = {res.x, res.y};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            o[e] = bf16_round(v[0][e] * alpha);
-            if (GATED) {
-              o[e] = swiglu_bf16(o[e], bf16_round(v[NB - 1][e] * alpha));
-              mi = max(mi, __float_as_uint(o[e]) & 0x7fffffffu);
-            } else if (p.residual != nullptr) {
-              const float rv = __uint_as_float((e & 1) ? rw[e >> 1] & 0xffff0000u : rw[e >> 1] << 16);
-              o[e] = __fadd_rn(rv, o[e]);
-            }
+          uint2 o = make_uint2(pack_bf16x2(v[0][0] * alpha, v[0][1] * alpha), pack_bf16x2(v[0][2] * alpha, v[0][3] * alpha));
+          if (GATED) {
+            o.x = swiglu_bf16x2(o.x, pack_bf16x2(v[NB - 1][0] * alpha, v[NB - 1][1] * alpha));
+            o.y = swiglu_bf16x2(o.y, pack_bf16x2(v[NB - 1][2] * alpha, v[NB - 1][3] * alpha));
+            asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(o.x & 0x7fff7fffu));
+            asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(o.y & 0x7fff7fffu));
+          } else if (p.residual != nullptr) {
+            const uint2 r2 = *reinterpret_cast<const uint2*>(p.residual + (size_t)(row0 + tok) * p.residual_ld + n);
+            o = make_uint2(add_bf16x2(r2.x, o.x), add_bf16x2(r2.y, o.y));
           }
-          *reinterpret_cast<uint2*>(p.c + at) = make_uint2(pack_bf16x2(o[0], o[1]), pack_bf16x2(o[2], o[3]));
+          *reinterpret_cast<uint2*>(p.c + at) = o;
         }
       }
       if (GATED) {
         __syncwarp();
+        uint32_t mi = max(m & 0xffffu, m >> 16) << 16;
 #pragma unroll
         for (int d = 16; d > 0; d >>= 1) mi = max(mi, __shfl_xor_sync(0xffffffffu, mi, d));
         if (lane == 0 && mi) atomicMax(p.amax, mi);

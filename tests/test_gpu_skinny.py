@@ -6,6 +6,7 @@ import pytest
 import torch
 
 from arcquant_b200 import synth
+from tests.helpers import launched_kernels
 
 pytestmark = pytest.mark.gpu
 
@@ -41,7 +42,9 @@ def _close(got, ref):
                                         # tiles of 128 tokens: one and several, last ones of 1, 16, 127 and 128 rows, one
                                         # to four ranges of K, a last stage of one K step, a ragged last weight tile
                                         (65, 4096, 4096, 128), (127, 136, 256, 64), (128, 1000, 1984, 64), (129, 2048, 2048, 64),
-                                        (144, 4104, 1024, 128), (333, 6144, 4096, 128), (512, 4096, 512, 64), (1000, 24, 64, 0)])
+                                        (144, 4104, 1024, 128), (333, 6144, 4096, 128), (512, 4096, 512, 64), (1000, 24, 64, 0),
+                                        # more weight tiles than CTAs
+                                        (7, 38024, 128, 0), (30, 38024, 128, 0), (61, 38024, 128, 64)])
 def test_few_rows_against_the_oracle(m, n, kq, ke):
     from arcquant_b200 import _lib, ops
 
@@ -79,16 +82,21 @@ def test_few_rows_swiglu_equals_gemm_then_silu(m, f, kq):
         sx2 = sx * factor
         want, amax_w = ops.silu_mul(ops.matmul_dev_alpha(a, b1, sfa, sfb1, sx2, sw))
         got, amax_g = ops.matmul_swiglu(a, b2, sfa, sfb2, sx2, sw)
-        if factor == 1.0:
-            _close(got, want.float().cpu())
-            assert abs(float(amax_g) - float(amax_w)) <= float(amax_w) * 2.0 ** -7
+        # (1e-30: every product underflows; 1e8: silu is the identity or zero)
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+        g64, w64 = got.double(), want.double()
+        assert float((g64 - w64).norm()) <= 1e-3 * float(w64.norm()) and float((got == want).float().mean()) >= 0.99
+        assert abs(float(amax_g) - float(amax_w)) <= float(amax_w) * 2.0 ** -7
         assert float(amax_g) == float(got.abs().max()) or bool(got.isnan().any())
     assert ops.gemm_poll_error() == 0
 
 
-@pytest.mark.parametrize("counts", [(5, 0, 17, 1), (0, 0, 0, 3), (64, 65, 0, 1), (130, 0, 2, 1)])
+# fewer than eight runs: 256-row tiles; eight and more with few rows in all: weight streaming (SwiGLU), where 65 and 130
+# rows of a run are two and three passes of 64 columns, the second of them starting in the middle of a scale tile
+@pytest.mark.parametrize("counts", [(5, 0, 17, 1), (0, 0, 0, 3), (64, 65, 0, 1), (130, 0, 2, 1), (5, 0, 17, 1, 0, 0, 2, 12),
+                                    (0, 0, 0, 0, 0, 0, 0, 1), (130, 64, 0, 1, 0, 0, 58, 2), (65, 0, 63, 1, 0, 127, 0, 0),
+                                    (1, 0, 33, 16, 0, 64, 65, 0, 7, 3), (2, 0, 66, 1) * 10])
 def test_grouped_few_rows_equal_the_per_run_calls(counts):
-    """(130 rows: three passes of 64 columns, the second of them starting in the middle of a scale tile)"""
     from arcquant_b200 import ops
     from arcquant_b200.qlinear import NVFP4_reorder_quantize_w
 
@@ -117,7 +125,12 @@ def test_grouped_few_rows_equal_the_per_run_calls(counts):
     x = synth.activations(total, kq, 5, synth.outlier_channels(kq, 10, 2), device="cuda")
     sx = ops.absmax_grouped(x, row_map, groups, e) / 2688.0
     a, sfa = ops.reorder_quantize_x_grouped(x, row_map, sx, idx, groups, bound, ke)
-    y, amax = ops.matmul_grouped_swiglu(a, B, sfa, SFB, tile_group, groups, e, n, sx, sw)
+    def swiglu():
+        return ops.matmul_grouped_swiglu(a, B, sfa, SFB, tile_group, groups, e, n, sx, sw)
+
+    kernels = [name for name, _, _ in launched_kernels(swiglu)]
+    assert len(kernels) == 1 and ("arcq_skinny_kernel" if e >= 8 else "arcq_gemm2_kernel") in kernels[0]
+    y, amax = swiglu()
     z = ops.matmul_grouped(a, B, sfa, SFB, tile_group, e, n, sx, sw)
     torch.cuda.synchronize()
     assert ops.gemm_poll_error() == 0

@@ -34,9 +34,10 @@ template <int NT, int NA, bool SPLIT>
 struct SkCfg {
   static constexpr int X_BYTES = NT * BK_BYTES;
   static constexpr int XBOX = NT > 64 ? 32 : 16;                       // rows of A per TMA box
-  // Up to 64 columns the partial sums have memory of their own and are pushed there; 128 columns (64 KB) take the ring's
-  // place once the CTA's products are complete, and their owners pull them.
-  static constexpr bool PULL = SPLIT && NT > 64;
+  // Up to 32 columns the partial sums have memory of their own and are pushed there; more take the ring's place once the
+  // CTA's products are complete, and their owners pull them.  (64 columns pushed left room for two stages only; 64 rows, us:
+  // [6144, 4224] 11.2 -> 9.2, [10240, 8320] 19.8 -> 15.3, SwiGLU [14336, 4224] 22.7 -> 18.6.)
+  static constexpr bool PULL = SPLIT && NT > 32;
   static constexpr int STAGE_BYTES = SK_W_BYTES + X_BYTES + 2 * SK_SF_BYTES;
   static constexpr int BAR_BYTES = 256;
   static constexpr int PART_BYTES = SPLIT && !PULL ? NA * (NT + 7) * 512 : 0;   // (tokens rounded up to the cluster, at most eight)

@@ -10,8 +10,8 @@
 //  * SwiGLU (gate and up rows interleaved in blocks of 128): half of a cluster's CTAs compute the gate block, half the up
 //    block, and the owner of a token forms bf16(bf16(silu(g)) * u) from their sums, and its maximum.  (Grouped: one CTA
 //    computes both, one after the other, into two accumulators.)
-//  * Grouped problems (the experts of a MoE block): persistent CTAs walk over (expert, weight tile); the rows of each
-//    expert are read from the device, experts without rows cost nothing, and more than NT rows are taken NT at a time.
+//  * Grouped problems (the experts of a MoE block): persistent CTAs walk over (expert, weight tile, pass of up to NT of
+//    its rows); the rows of each expert are read from the device, and experts without rows cost nothing.
 //  * Programmatic dependent launch: while the kernel before is still running, every CTA pulls its first weight tiles
 //    into L2 (a prefetch reads nothing into the CTA, so a weight still being written is not read early).
 //
@@ -41,9 +41,10 @@ struct SkCfg {
   static constexpr int STAGE_BYTES = SK_W_BYTES + X_BYTES + 2 * SK_SF_BYTES;
   static constexpr int BAR_BYTES = 256;
   static constexpr int PART_BYTES = SPLIT && !PULL ? NA * (NT + 7) * 512 : 0;   // (tokens rounded up to the cluster, at most eight)
-  static constexpr int FIT = (113 * 1024 - 1024 - BAR_BYTES - PART_BYTES) / STAGE_BYTES;
+  static constexpr int TABLE_BYTES = NA == 2 ? 3 * 64 * 4 : 0;         // grouped: the run table
+  static constexpr int FIT = (113 * 1024 - 1024 - BAR_BYTES - TABLE_BYTES - PART_BYTES) / STAGE_BYTES;
   static constexpr int STAGES = FIT < 5 ? FIT : 5;
-  static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + PART_BYTES + BAR_BYTES;
+  static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + PART_BYTES + BAR_BYTES + TABLE_BYTES;
   static constexpr int TMEM_NEED = NA * NT + STAGES * SK_SF_COLS;
   static constexpr int TMEM_COLS = TMEM_NEED <= 128 ? 128 : 256;
   static_assert(STAGES >= 2 && TMEM_NEED <= 256, "two CTAs share 512 columns of tensor memory");
@@ -63,8 +64,7 @@ struct SkinnyParams {
   int ksteps_total;                  // K_eff / 64
   int natoms;                        // scale atoms per 128-row tile
   int tiles;                         // weight tiles per matrix: ceil(N / 128), halved with SwiGLU
-  int ttiles;                        // token tiles of NT rows (1 for grouped problems, which take their rows NT at a time)
-  int sfw_tiles;                     // 128-row scale tiles of all matrices
+  int ttiles;                        // token tiles of NT rows (grouped problems: counted on the device)
   int splits;                        // K ranges = CTAs per cluster
   const int* groups;                 // run table of a grouped problem (device) or nullptr
   int ngroups;
@@ -110,6 +110,7 @@ __global__ void __launch_bounds__(SK_THREADS, 2)
 arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const SkinnyParams p) {
   constexpr int NA = GATED && !SPLIT ? 2 : 1;          // accumulators of a CTA
   constexpr int NB = GATED ? 2 : 1;                    // 128-row blocks of weight per work item
+  constexpr bool GROUPED = GATED && !SPLIT;            // runs of rows, each with its own matrix (SwiGLU of one matrix is always split)
   using C = SkCfg<NT, NA, SPLIT>;
   constexpr int TMEM_COLS = C::TMEM_COLS;
   extern __shared__ uint8_t smem_raw[];
@@ -133,12 +134,9 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   const int block = SPLIT ? rank / splits : 0;                         // SwiGLU: 0 = gate, 1 = up
   const int ks_begin = kstages * split / splits, ks_end = kstages * (split + 1) / splits;
   const int first_item = (int)(blockIdx.x / csize), item_step = (int)(gridDim.x / csize);
-  const int num_items = p.tiles * p.ngroups * ttiles;                // token tiles of one weight tile are neighbours
-  // first weight row of accumulator a of work item `item`, in the stacked matrices
-  auto weight_row = [&](int item, int a) {
-    const int wt = item / ttiles, g = wt / p.tiles, t = wt - g * p.tiles;
-    return g * p.N + t * (128 * NB) + 128 * (block + a);
-  };
+  int num_items = p.tiles * ttiles;                                  // token tiles of one weight tile are neighbours
+  // first weight row of accumulator a of weight tile t of matrix g, in the stacked matrices
+  auto weight_row = [&](int g, int t, int a) { return g * p.N + t * (128 * NB) + 128 * (block + a); };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
@@ -150,11 +148,13 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     mbar_init(acc_empty_bar, 4);
     misc[1] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    // the first ring of weight tiles on its way into L2
+    // the first ring of weight tiles on its way into L2 (grouped: as if every run had rows for one pass)
     int n = 0;
-    for (int item = first_item; item < num_items && n < C::STAGES; item += item_step)
+    for (int item = first_item; item < (GROUPED ? p.tiles * p.ngroups : num_items) && n < C::STAGES; item += item_step) {
+      const int g = GROUPED ? item / p.tiles : 0, t = GROUPED ? item - g * p.tiles : item / ttiles;
       for (int a = 0; a < NA; ++a)
-        for (int ks = ks_begin; ks < ks_end && n < C::STAGES; ++ks, ++n) sk_prefetch_tile(&map_w, ks * BK_BYTES, weight_row(item, a));
+        for (int ks = ks_begin; ks < ks_end && n < C::STAGES; ++ks, ++n) sk_prefetch_tile(&map_w, ks * BK_BYTES, weight_row(g, t, a));
+    }
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32((const void*)misc)),
@@ -178,12 +178,50 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   const uint32_t tmem_base = misc[0];
   const uint32_t tmem_sf = tmem_base + NA * NT;
 
-  // rows of a work item: first row in A / C, number
-  auto run_of = [&](int item, int& row0, int& cnt) {
-    if (p.groups == nullptr) { row0 = (item % ttiles) * NT; cnt = min(NT, p.M - row0); return; }
-    const int g = item / p.tiles;
-    row0 = __ldg(p.groups + g);
-    cnt = __ldg(p.groups + p.ngroups + g);
+  // Grouped: per run (up to 64) the items up to and including it, its rows and its first row.  The passes of a long run
+  // are items of their own: one CTA after the other taking them in turn made a batch that routes to few experts wait for
+  // a few CTAs (256 rows of one run out of eight, [7168, 2176]: 51.3 -> 18.5 us).
+  int* const run_end = reinterpret_cast<int*>(base_ptr + BAR_AT + C::BAR_BYTES);
+  if (GROUPED) {
+    if (warp == 0) {
+      int before = 0;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int e = lane + 32 * h;
+        const int row0 = e < p.ngroups ? __ldg(p.groups + e) : 0, cnt = e < p.ngroups ? __ldg(p.groups + p.ngroups + e) : 0;
+        int inc = p.tiles * ((cnt + NT - 1) / NT);
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, inc, d);
+          if (lane >= d) inc += v;
+        }
+        run_end[e] = before + inc;
+        run_end[64 + e] = cnt;
+        run_end[128 + e] = row0;
+        before += __shfl_sync(0xffffffffu, inc, 31);
+      }
+    }
+    __syncthreads();
+    num_items = run_end[63];
+  }
+  // a work item: matrix, weight tile, first row in A / C, rows (at most NT)
+  auto locate = [&](int item, int& g, int& t, int& row0, int& cnt) {
+    if (GROUPED) {
+      g = 0;                                              // the first run that ends beyond the item
+#pragma unroll
+      for (int d = 32; d > 0; d >>= 1)
+        if (run_end[g + d - 1] <= item) g += d;
+      const int i = item - (g > 0 ? run_end[g - 1] : 0), passes = (run_end[64 + g] + NT - 1) / NT;
+      t = passes > 1 ? i / passes : i;                    // (the passes of one weight tile are neighbours)
+      const int at = (i - t * passes) * NT;
+      row0 = run_end[128 + g] + at;
+      cnt = min(NT, run_end[64 + g] - at);
+    } else {
+      g = 0;
+      t = item / ttiles;
+      row0 = (item - t * ttiles) * NT;
+      cnt = min(NT, p.M - row0);
+    }
   };
 
   if (warp == 0) {
@@ -192,25 +230,23 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       uint32_t it = 0;
       bool ok = true;
       for (int item = first_item; item < num_items && ok; item += item_step) {
-        int row0, cnt;
-        run_of(item, row0, cnt);
-        for (int c0 = 0; c0 < cnt && ok; c0 += NT) {
-          const int boxes = (min(NT, cnt - c0) + C::XBOX - 1) / C::XBOX;
-          const int xt = (row0 + c0) >> 7;                               // 128-row scale tile of these rows
-          for (int ai = 0; ai < NA && ok; ++ai) {
-            const int wrow = weight_row(item, ai), wt = wrow >> 7;
-            for (int ks = ks_begin; ks < ks_end; ++ks, ++it) {
-              const int s = it % C::STAGES;
-              if (!mbar_wait(empty_bar(s), ((it / C::STAGES) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
-              const uint32_t sf_bytes = (uint32_t)min(KSTEPS, p.ksteps_total - ks * KSTEPS) * ATOM;
-              const uint32_t st = base + s * C::STAGE_BYTES, x_s = st + SK_W_BYTES, sfw_s = x_s + C::X_BYTES, sfx_s = sfw_s + SK_SF_BYTES;
-              mbar_expect_tx(sf_bar(s), 2u * sf_bytes);
-              mbar_expect_tx(full_bar(s), SK_W_BYTES + (uint32_t)(boxes * C::XBOX * BK_BYTES));
-              bulk_load(sfw_s, p.sfw + ((size_t)wt * p.natoms + (size_t)ks * KSTEPS) * ATOM, sf_bytes, sf_bar(s));
-              bulk_load(sfx_s, p.sfx + ((size_t)xt * p.natoms + (size_t)ks * KSTEPS) * ATOM, sf_bytes, sf_bar(s));
-              tma_load_2d(st, &map_w, full_bar(s), ks * BK_BYTES, wrow);
-              for (int b = 0; b < boxes; ++b) tma_load_2d(x_s + b * (C::XBOX * BK_BYTES), &map_x, full_bar(s), ks * BK_BYTES, row0 + c0 + C::XBOX * b);
-            }
+        int g, t, row0, cnt;
+        locate(item, g, t, row0, cnt);
+        const int boxes = (cnt + C::XBOX - 1) / C::XBOX;
+        const int xt = row0 >> 7;                                        // 128-row scale tile of these rows
+        for (int ai = 0; ai < NA && ok; ++ai) {
+          const int wrow = weight_row(g, t, ai), wt = wrow >> 7;
+          for (int ks = ks_begin; ks < ks_end; ++ks, ++it) {
+            const int s = it % C::STAGES;
+            if (!mbar_wait(empty_bar(s), ((it / C::STAGES) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+            const uint32_t sf_bytes = (uint32_t)min(KSTEPS, p.ksteps_total - ks * KSTEPS) * ATOM;
+            const uint32_t st = base + s * C::STAGE_BYTES, x_s = st + SK_W_BYTES, sfw_s = x_s + C::X_BYTES, sfx_s = sfw_s + SK_SF_BYTES;
+            mbar_expect_tx(sf_bar(s), 2u * sf_bytes);
+            mbar_expect_tx(full_bar(s), SK_W_BYTES + (uint32_t)(boxes * C::XBOX * BK_BYTES));
+            bulk_load(sfw_s, p.sfw + ((size_t)wt * p.natoms + (size_t)ks * KSTEPS) * ATOM, sf_bytes, sf_bar(s));
+            bulk_load(sfx_s, p.sfx + ((size_t)xt * p.natoms + (size_t)ks * KSTEPS) * ATOM, sf_bytes, sf_bar(s));
+            tma_load_2d(st, &map_w, full_bar(s), ks * BK_BYTES, wrow);
+            for (int b = 0; b < boxes; ++b) tma_load_2d(x_s + b * (C::XBOX * BK_BYTES), &map_x, full_bar(s), ks * BK_BYTES, row0 + C::XBOX * b);
           }
         }
       }
@@ -228,39 +264,37 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     if (lane == 0) {
       uint32_t it = 0, acc_it = 0;
       bool ok = true;
-      for (int item = first_item; item < num_items && ok; item += item_step) {
-        int row0, cnt;
-        run_of(item, row0, cnt);
-        for (int c0 = 0; c0 < cnt && ok; c0 += NT, ++acc_it) {
-          const uint32_t ncols = (uint32_t)((min(NT, cnt - c0) + 15) & ~15);
-          // e2m1 x e2m1, ue4m3 scales, K-major operands (see arcq_gemm.cu), N = ncols, M = 128
-          const uint32_t idesc = (1u << 7) | (1u << 10) | ((ncols >> 3) << 17) | (8u << 24);
-          if (!mbar_wait(acc_empty_bar, (acc_it & 1u) ^ 1u, abort_flag)) { ok = false; break; }
-          tc_fence_after();
-          for (int ai = 0; ai < NA && ok; ++ai) {
-            for (int ks = ks_begin; ks < ks_end; ++ks, ++it) {
-              const int s = it % C::STAGES;
-              if (!mbar_wait(full_bar(s), (it / C::STAGES) & 1u, abort_flag)) { ok = false; break; }
-              tc_fence_after();
-              const int nk = min(KSTEPS, p.ksteps_total - ks * KSTEPS);
-              const uint32_t st = base + s * C::STAGE_BYTES;
-              const uint32_t t_sfw = tmem_sf + s * SK_SF_COLS, t_sfx = t_sfw + KSTEPS * 4;
-              const uint64_t wd = smem_desc(st, 1024, LAYOUT_SW128), xd = smem_desc(st + SK_W_BYTES, 1024, LAYOUT_SW128);
-              if (nk == KSTEPS) {
+      for (int item = first_item; item < num_items && ok; item += item_step, ++acc_it) {
+        int g, t, row0, cnt;
+        locate(item, g, t, row0, cnt);
+        const uint32_t ncols = (uint32_t)((cnt + 15) & ~15);
+        // e2m1 x e2m1, ue4m3 scales, K-major operands (see arcq_gemm.cu), N = ncols, M = 128
+        const uint32_t idesc = (1u << 7) | (1u << 10) | ((ncols >> 3) << 17) | (8u << 24);
+        if (!mbar_wait(acc_empty_bar, (acc_it & 1u) ^ 1u, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        for (int ai = 0; ai < NA && ok; ++ai) {
+          for (int ks = ks_begin; ks < ks_end; ++ks, ++it) {
+            const int s = it % C::STAGES;
+            if (!mbar_wait(full_bar(s), (it / C::STAGES) & 1u, abort_flag)) { ok = false; break; }
+            tc_fence_after();
+            const int nk = min(KSTEPS, p.ksteps_total - ks * KSTEPS);
+            const uint32_t st = base + s * C::STAGE_BYTES;
+            const uint32_t t_sfw = tmem_sf + s * SK_SF_COLS, t_sfx = t_sfw + KSTEPS * 4;
+            const uint64_t wd = smem_desc(st, 1024, LAYOUT_SW128), xd = smem_desc(st + SK_W_BYTES, 1024, LAYOUT_SW128);
+            if (nk == KSTEPS) {
 #pragma unroll
-                for (int k = 0; k < KSTEPS; ++k)
-                  tc_mma_nvf4(tmem_base + ai * NT, wd + 2 * k, xd + 2 * k, idesc, t_sfw + k * 4, t_sfx + k * 4,
-                              (ks > ks_begin || k > 0) ? 1u : 0u);
-              } else {
-                for (int k = 0; k < nk; ++k)
-                  tc_mma_nvf4(tmem_base + ai * NT, wd + 2 * k, xd + 2 * k, idesc, t_sfw + k * 4, t_sfx + k * 4,
-                              (ks > ks_begin || k > 0) ? 1u : 0u);
-              }
-              tc_commit(empty_bar(s));
+              for (int k = 0; k < KSTEPS; ++k)
+                tc_mma_nvf4(tmem_base + ai * NT, wd + 2 * k, xd + 2 * k, idesc, t_sfw + k * 4, t_sfx + k * 4,
+                            (ks > ks_begin || k > 0) ? 1u : 0u);
+            } else {
+              for (int k = 0; k < nk; ++k)
+                tc_mma_nvf4(tmem_base + ai * NT, wd + 2 * k, xd + 2 * k, idesc, t_sfw + k * 4, t_sfx + k * 4,
+                            (ks > ks_begin || k > 0) ? 1u : 0u);
             }
+            tc_commit(empty_bar(s));
           }
-          if (ok) tc_commit(acc_full_bar);
         }
+        if (ok) tc_commit(acc_full_bar);
       }
     }
   } else if (warp < 6) {
@@ -284,110 +318,106 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         }
       }
     };
-    for (int item = first_item; item < num_items && ok; item += item_step) {
-      const int wt = item / ttiles, g = wt / p.tiles, t = wt - g * p.tiles;
+    for (int item = first_item; item < num_items; item += item_step, ++acc_it) {
+      int g, t, row0, here;
+      locate(item, g, t, row0, here);
       const int n4 = t * 128 + quad * 32 + (lane & ~3);    // (unsplit) first of this lane's four output columns
-      int row0, cnt;
-      run_of(item, row0, cnt);
       float alpha = p.alpha;
       if (p.alpha_a) alpha *= __ldg(p.alpha_a + g);
       if (p.alpha_b) alpha *= __ldg(p.alpha_b + g);
-      for (int c0 = 0; c0 < cnt; c0 += NT, ++acc_it) {
-        if (!SPLIT) fetch_residual(row0 + c0, min(NT, cnt - c0), n4);     // (while the products are still being formed)
-        ok = mbar_wait(acc_full_bar, acc_it & 1u, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        tc_fence_after();
-        const int here = min(NT, cnt - c0);
-        if (C::PULL) {
-          // fp32 partial sums in place of the ring (every product that reads it is complete): [token][128]
-          for (int j0 = 0; j0 < here; j0 += 16) {
-            uint32_t v[16];
-            tc_ld16(t_row + j0, v);
-            tc_wait_ld();
-            float* dst = reinterpret_cast<float*>(base_ptr) + j0 * 128 + nl;
+      if (!SPLIT) fetch_residual(row0, here, n4);        // (while the products are still being formed)
+      ok = mbar_wait(acc_full_bar, acc_it & 1u, abort_flag);
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) break;
+      tc_fence_after();
+      if (C::PULL) {
+        // fp32 partial sums in place of the ring (every product that reads it is complete): [token][128]
+        for (int j0 = 0; j0 < here; j0 += 16) {
+          uint32_t v[16];
+          tc_ld16(t_row + j0, v);
+          tc_wait_ld();
+          float* dst = reinterpret_cast<float*>(base_ptr) + j0 * 128 + nl;
 #pragma unroll
-            for (int j = 0; j < 16; ++j) dst[j * 128] = __uint_as_float(v[j]);
-          }
-        } else if (SPLIT) {
-          // fp32 partial sums to the CTAs that own the tokens: token j belongs to rank j % csize, where it is
-          // number j / csize; layout there: [token number][source rank][128]
-          meet();
-          uint32_t dst[8];
+          for (int j = 0; j < 16; ++j) dst[j * 128] = __uint_as_float(v[j]);
+        }
+      } else if (SPLIT) {
+        // fp32 partial sums to the CTAs that own the tokens: token j belongs to rank j % csize, where it is
+        // number j / csize; layout there: [token number][source rank][128]
+        meet();
+        uint32_t dst[8];
 #pragma unroll
-          for (int r = 0; r < 8; ++r) dst[r] = cluster_addr(part_base, (uint32_t)min(r, csize - 1));
-          int r = 0;                                       // (rank of token j without a division per token)
-          uint32_t at = (uint32_t)(rank * 512 + nl * 4);
-          for (int j0 = 0; j0 < here; j0 += 16) {
-            uint32_t v[16];
-            tc_ld16(t_row + j0, v);
-            tc_wait_ld();
+        for (int r = 0; r < 8; ++r) dst[r] = cluster_addr(part_base, (uint32_t)min(r, csize - 1));
+        int r = 0;                                       // (rank of token j without a division per token)
+        uint32_t at = (uint32_t)(rank * 512 + nl * 4);
+        for (int j0 = 0; j0 < here; j0 += 16) {
+          uint32_t v[16];
+          tc_ld16(t_row + j0, v);
+          tc_wait_ld();
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-              if (j0 + j < here) {
-                uint32_t d = dst[0];
+          for (int j = 0; j < 16; ++j) {
+            if (j0 + j < here) {
+              uint32_t d = dst[0];
 #pragma unroll
-                for (int q = 1; q < 8; ++q) d = r == q ? dst[q] : d;
-                st_cluster_f32(d + at, v[j]);
-                if (++r == csize) { r = 0; at += (uint32_t)(csize * 512); }
-              }
+              for (int q = 1; q < 8; ++q) d = r == q ? dst[q] : d;
+              st_cluster_f32(d + at, v[j]);
+              if (++r == csize) { r = 0; at += (uint32_t)(csize * 512); }
             }
-          }
-        } else {
-          // A lane holds one column of 16 tokens; two exchanges between neighbouring lanes leave it four columns of the
-          // tokens 4 k + lane % 4, which go out as 8-byte stores.  (Element by element - 16 stores, 16 dependent loads of
-          // the residual - a pass of 64 tokens cost more than its weight stream, us: [256, 576] 128 rows 14.5 -> 6.5, with
-          // a residual 33.9 -> 8.9; grouped SwiGLU [7168, 2176], 256 rows of one run out of eight 80.0 -> 51.3.)
-          uint32_t m = 0;                                  // max|C| of two tokens
-#pragma unroll 1
-          for (int h0 = 0; h0 < here; h0 += AHEAD) {
-            if (h0 > 0) fetch_residual(row0 + c0 + h0, here - h0, n4);
-#pragma unroll
-            for (int b = 0; b < AHEAD / 16; ++b) {
-              const int j0 = h0 + 16 * b;
-              if (j0 >= here) break;
-              uint32_t r[16], u[16], o[8];
-              tc_ld16(t_row + j0, r);
-              if (GATED) tc_ld16(t_row + (NA - 1) * NT + j0, u);
-              tc_wait_ld();
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {                // tokens 2 i, 2 i + 1
-                o[i] = pack_bf16x2(__uint_as_float(r[2 * i]) * alpha, __uint_as_float(r[2 * i + 1]) * alpha);
-                if (GATED) o[i] = swiglu_bf16x2(o[i], pack_bf16x2(__uint_as_float(u[2 * i]) * alpha, __uint_as_float(u[2 * i + 1]) * alpha));
-              }
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {                // token 2 i + lane % 2, two columns
-                const uint32_t x = __shfl_xor_sync(0xffffffffu, o[i], 1);
-                o[i] = (lane & 1) ? __byte_perm(x, o[i], 0x7632) : __byte_perm(o[i], x, 0x5410);
-              }
-#pragma unroll
-              for (int k = 0; k < 4; ++k) {                // token 4 k + lane % 4, four columns
-                const uint32_t x = __shfl_xor_sync(0xffffffffu, (lane & 2) ? o[2 * k] : o[2 * k + 1], 2);
-                uint2 v = (lane & 2) ? make_uint2(x, o[2 * k + 1]) : make_uint2(o[2 * k], x);
-                const int tok = j0 + 4 * k + (lane & 3);
-                if (tok < here && n4 < ncols) {
-                  if (GATED) {
-                    asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(v.x & 0x7fff7fffu));
-                    asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(v.y & 0x7fff7fffu));
-                  } else if (p.residual != nullptr) {
-                    v = make_uint2(add_bf16x2(res[4 * b + k].x, v.x), add_bf16x2(res[4 * b + k].y, v.y));
-                  }
-                  *reinterpret_cast<uint2*>(p.c + (size_t)(row0 + c0 + tok) * ncols + n4) = v;
-                }
-              }
-            }
-          }
-          if (GATED) {       // (a NaN counts as larger than everything, as in the other epilogues)
-            uint32_t mi = max(m & 0xffffu, m >> 16) << 16;
-#pragma unroll
-            for (int d = 16; d > 0; d >>= 1) mi = max(mi, __shfl_xor_sync(0xffffffffu, mi, d));
-            if (lane == 0 && mi) atomicMax(p.amax + g, mi);
           }
         }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(acc_empty_bar);
+      } else {
+        // A lane holds one column of 16 tokens; two exchanges between neighbouring lanes leave it four columns of the
+        // tokens 4 k + lane % 4, which go out as 8-byte stores.  (Element by element - 16 stores, 16 dependent loads of
+        // the residual - a pass of 64 tokens cost more than its weight stream, us: [256, 576] 128 rows 14.5 -> 6.5, with
+        // a residual 33.9 -> 8.9; grouped SwiGLU [7168, 2176], 256 rows of one run out of eight 80.0 -> 51.3.)
+        uint32_t m = 0;                                  // max|C| of two tokens
+#pragma unroll 1
+        for (int h0 = 0; h0 < here; h0 += AHEAD) {
+          if (h0 > 0) fetch_residual(row0 + h0, here - h0, n4);
+#pragma unroll
+          for (int b = 0; b < AHEAD / 16; ++b) {
+            const int j0 = h0 + 16 * b;
+            if (j0 >= here) break;
+            uint32_t r[16], u[16], o[8];
+            tc_ld16(t_row + j0, r);
+            if (GATED) tc_ld16(t_row + (NA - 1) * NT + j0, u);
+            tc_wait_ld();
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {                // tokens 2 i, 2 i + 1
+              o[i] = pack_bf16x2(__uint_as_float(r[2 * i]) * alpha, __uint_as_float(r[2 * i + 1]) * alpha);
+              if (GATED) o[i] = swiglu_bf16x2(o[i], pack_bf16x2(__uint_as_float(u[2 * i]) * alpha, __uint_as_float(u[2 * i + 1]) * alpha));
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {                // token 2 i + lane % 2, two columns
+              const uint32_t x = __shfl_xor_sync(0xffffffffu, o[i], 1);
+              o[i] = (lane & 1) ? __byte_perm(x, o[i], 0x7632) : __byte_perm(o[i], x, 0x5410);
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {                // token 4 k + lane % 4, four columns
+              const uint32_t x = __shfl_xor_sync(0xffffffffu, (lane & 2) ? o[2 * k] : o[2 * k + 1], 2);
+              uint2 v = (lane & 2) ? make_uint2(x, o[2 * k + 1]) : make_uint2(o[2 * k], x);
+              const int tok = j0 + 4 * k + (lane & 3);
+              if (tok < here && n4 < ncols) {
+                if (GATED) {
+                  asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(v.x & 0x7fff7fffu));
+                  asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(v.y & 0x7fff7fffu));
+                } else if (p.residual != nullptr) {
+                  v = make_uint2(add_bf16x2(res[4 * b + k].x, v.x), add_bf16x2(res[4 * b + k].y, v.y));
+                }
+                *reinterpret_cast<uint2*>(p.c + (size_t)(row0 + tok) * ncols + n4) = v;
+              }
+            }
+          }
+        }
+        if (GATED) {       // (a NaN counts as larger than everything, as in the other epilogues)
+          uint32_t mi = max(m & 0xffffu, m >> 16) << 16;
+#pragma unroll
+          for (int d = 16; d > 0; d >>= 1) mi = max(mi, __shfl_xor_sync(0xffffffffu, mi, d));
+          if (lane == 0 && mi) atomicMax(p.amax + g, mi);
+        }
       }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acc_empty_bar);
     }
   } else {
     // ------------------------------------------------------------------ scale warps (6..9)
@@ -396,34 +426,32 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     uint32_t it = 0;
     bool ok = true;
     for (int item = first_item; item < num_items && ok; item += item_step) {
-      int row0, cnt;
-      run_of(item, row0, cnt);
-      for (int c0 = 0; c0 < cnt && ok; c0 += NT) {
-        const bool upper = ((row0 + c0) & 64) != 0;        // rows 64.. of a 128-row scale tile: words 2 and 3 of the atoms
-        for (int n = NA * (ks_end - ks_begin); n > 0; --n, ++it) {
-          const int s = it % C::STAGES;
-          ok = mbar_wait(sf_bar(s), (it / C::STAGES) & 1u, abort_flag);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-          // (the MMAs that read the stage's old scale columns are complete: its producer waited for them)
-          const uint4* sf = reinterpret_cast<const uint4*>(base_ptr + s * C::STAGE_BYTES + SK_W_BYTES + C::X_BYTES);
-          const uint32_t taddr = tmem_sf + s * SK_SF_COLS + ((uint32_t)(quad * 32) << 16);
+      int g, t, row0, cnt;
+      locate(item, g, t, row0, cnt);
+      const bool upper = (row0 & 64) != 0;                 // rows 64.. of a 128-row scale tile: words 2 and 3 of the atoms
+      for (int n = NA * (ks_end - ks_begin); n > 0; --n, ++it) {
+        const int s = it % C::STAGES;
+        ok = mbar_wait(sf_bar(s), (it / C::STAGES) & 1u, abort_flag);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        // (the MMAs that read the stage's old scale columns are complete: its producer waited for them)
+        const uint4* sf = reinterpret_cast<const uint4*>(base_ptr + s * C::STAGE_BYTES + SK_W_BYTES + C::X_BYTES);
+        const uint32_t taddr = tmem_sf + s * SK_SF_COLS + ((uint32_t)(quad * 32) << 16);
 #pragma unroll
-          for (int side = 0; side < 2; ++side) {
-            uint32_t r[16];
+        for (int side = 0; side < 2; ++side) {
+          uint32_t r[16];
 #pragma unroll
-            for (int k = 0; k < KSTEPS; ++k) {
-              uint4 v = sf[(side * KSTEPS + k) * 32 + lane];
-              if (side == 1 && upper) { v.x = v.z; v.y = v.w; }
-              r[4 * k] = v.x; r[4 * k + 1] = v.y; r[4 * k + 2] = v.z; r[4 * k + 3] = v.w;
-            }
-            tc_st16(taddr + side * (KSTEPS * 4), r);
+          for (int k = 0; k < KSTEPS; ++k) {
+            uint4 v = sf[(side * KSTEPS + k) * 32 + lane];
+            if (side == 1 && upper) { v.x = v.z; v.y = v.w; }
+            r[4 * k] = v.x; r[4 * k + 1] = v.y; r[4 * k + 2] = v.z; r[4 * k + 3] = v.w;
           }
-          tc_wait_st();
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(full_bar(s));
+          tc_st16(taddr + side * (KSTEPS * 4), r);
         }
+        tc_wait_st();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full_bar(s));
       }
     }
   }
@@ -435,9 +463,8 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
     meet();
     asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (*abort_flag == 0) {
-      const int t = first_item / ttiles;
-      int row0, cnt;
-      run_of(first_item, row0, cnt);
+      int g, t, row0, cnt;
+      locate(first_item, g, t, row0, cnt);
       const int ncols = GATED ? p.N >> 1 : p.N;
       float alpha = p.alpha;
       if (p.alpha_a) alpha *= __ldg(p.alpha_a);
@@ -556,7 +583,8 @@ static int skinny_splits_wide(int tiles, int kstages, const DeviceInfo& di) {
   while (s > 1 && s > kstages / 2) s >>= 1;
   return s;
 }
-// See SkinnyParams; `residual` and `swiglu_amax` exclude each other; groups (device) with ngroups matrices stacked in W.
+// See SkinnyParams; `residual` and `swiglu_amax` exclude each other; groups (device, with swiglu_amax): ngroups matrices
+// (at most 64) stacked in W.
 int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, const uint8_t* SFW, int64_t M, int64_t N,
                        int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, const void* residual, void* C,
                        float* swiglu_amax, const int* groups, int ngroups, cudaStream_t stream, bool residual_is_bias) {
@@ -589,7 +617,9 @@ int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, c
   p.splits = groups != nullptr ? 1 : (nt > 64 ? skinny_splits_wide(blocks, kstages, di) : skinny_splits(blocks, kstages, di));
   if (gated && p.splits > 4) p.splits = 4;
   const int csize = groups != nullptr ? 1 : p.splits * (gated ? 2 : 1);
-  long long grid = (long long)p.tiles * p.ngroups * p.ttiles * csize;
+  // (grouped: of the rows the host knows a bound, see launch_gemm_grouped)
+  const long long passes = groups != nullptr ? p.ngroups + (M > 256LL * p.ngroups ? (M - 256LL * p.ngroups) / nt : 0) : p.ttiles;
+  long long grid = p.tiles * passes * csize;
   // one CTA per item where several form a cluster; else persistent CTAs, two per SM
   const long long slots = di.num_sms == di.all_sms ? 2LL * di.num_sms : di.num_sms;
   if (csize == 1 && grid > slots) grid = slots;
@@ -599,8 +629,7 @@ int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, c
   if (rc != ARCQ_OK) return rc;
   rc = make_operand_map(&mw, W, N * p.ngroups, K_eff / 2, 128);
   if (rc != ARCQ_OK) return rc;
-  if (groups != nullptr)
-    return gated ? launch_one<64, true, false>(mx, mw, p, (int)grid, stream) : launch_one<64, false, false>(mx, mw, p, (int)grid, stream);
+  if (groups != nullptr) return launch_one<64, true, false>(mx, mw, p, (int)grid, stream);
   if (nt == 16) return launch_nt<16>(mx, mw, p, gated, (int)grid, stream);
   if (nt == 32) return launch_nt<32>(mx, mw, p, gated, (int)grid, stream);
   if (nt == 64) return launch_nt<64>(mx, mw, p, gated, (int)grid, stream);

@@ -886,8 +886,10 @@ static void plan_splitk(int64_t M, int64_t N, int64_t K_eff, int num_sms, int* b
 //   [6144, 4224]  128 rows 11.0 / 16.3  200 rows 12.2 / 28.4   333 rows 13.1 / 14.3
 //   [4096, 14464] 128 rows 15.8 / 20.7  333 rows 22.7 / 81.8   512 rows 23.4 / 81.9
 // and beyond that line 777 rows of [4096, 4224] 21.1 / 14.3, [28672, 4224] 128 rows 24.5 / 22.4.
-static bool use_skinny_kernel(int64_t M, int64_t N, int num_sms) {
-  return M <= ARCQ_SKINNY_ROWS || ((M + 127) / 128) * ((N + 127) / 128) <= num_sms;
+// Above 64 rows only where K is split: with a K of less than four stages this kernel's stores are the time, [256, 576]
+// 512 rows 5.5 / 5.1, 4096 rows 6.2 / 5.1 (with a residual 8.2 / 11.4 and 8.5 / 10.6: there it is the better one all the same).
+static bool use_skinny_kernel(int64_t M, int64_t N, int64_t K_eff, int num_sms, bool residual = false) {
+  return M <= ARCQ_SKINNY_ROWS || (((M + 127) / 128) * ((N + 127) / 128) <= num_sms && (residual || skinny_plan_splits(M, N, K_eff) > 1));
 }
 // With the SwiGLU epilogue (gate and up blocks in different CTAs of a cluster): [28672, 4224] 65 rows 24.8 / 30.9 us,
 // 128 rows 26.9 / 31.4, 200 rows 43.1 / 31.6 (CTA pairs with four epilogue warps; eight take about 5 % off).
@@ -952,7 +954,7 @@ int launch_gemm_residual(const uint8_t* A, const uint8_t* B, const uint8_t* SFA,
   DeviceInfo di;
   int rc = get_device_info(&di);
   if (rc != ARCQ_OK) return rc;
-  if (use_skinny_kernel(M, N, di.num_sms))
+  if (use_skinny_kernel(M, N, K_eff, di.num_sms, true))
     return launch_gemm_skinny(A, B, SFA, SFB, M, N, K_eff, 1.0f, alpha_a, alpha_b, residual, Cout, nullptr, nullptr, 1, stream);
   GemmParams p = {};
   p.c = static_cast<__nv_bfloat16*>(Cout);
@@ -987,7 +989,7 @@ int gemm_plan(int64_t M, int64_t N, int64_t K_eff, int* kind, int* tile_n, int* 
   int rc = get_device_info(&di);
   if (rc != ARCQ_OK) return rc;
   int k = ARCQ_GEMM_KIND_SINGLE, bn = 256, sp = 1;
-  if (use_skinny_kernel(M, N, di.num_sms)) {
+  if (use_skinny_kernel(M, N, K_eff, di.num_sms)) {
     k = ARCQ_GEMM_KIND_SKINNY;
     bn = 128;
     sp = skinny_plan_splits(M, N, K_eff);
@@ -1008,7 +1010,7 @@ int launch_gemm(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const ui
   DeviceInfo di;
   int rc = get_device_info(&di);
   if (rc != ARCQ_OK) return rc;
-  if (use_skinny_kernel(M, N, di.num_sms))
+  if (use_skinny_kernel(M, N, K_eff, di.num_sms))
     return launch_gemm_skinny(A, B, SFA, SFB, M, N, K_eff, alpha, alpha_a, alpha_b, bias, Cout, nullptr, nullptr, 1, stream,
                               bias != nullptr);
 

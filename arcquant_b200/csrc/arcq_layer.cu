@@ -625,7 +625,7 @@ __global__ void arcq_ep_rows_kernel(const uint4* __restrict__ src, const int* __
 // eighth of the CTAs' worth of results meets the running maxima, with an atomic only where a larger value was
 // found.
 constexpr int CALIB_THREADS = 512, CALIB_CLUSTER = 8;
-template <int CPT, int RB>
+template <int CPT, int RB, bool CLUSTER = true>
 __global__ void __launch_bounds__(CALIB_THREADS, CPT * RB > 8 ? 1 : 2)
 arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, unsigned int* chan_absmax,
                         unsigned long long* above) {
@@ -698,23 +698,38 @@ arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, u
     }
     count += (unsigned long long)(above16 >> 4);
   }
+  if constexpr (!CLUSTER) {
+    // a handful of rows: nothing to reduce on chip first
 #pragma unroll
-  for (int j = 0; j < CPT; ++j) {
-    const int c = tid + j * CALIB_THREADS;
-    if (c < nchunks) *reinterpret_cast<uint4*>(s_col + 4 * c) = make_uint4(cmax[j][0], cmax[j][1], cmax[j][2], cmax[j][3]);
-  }
-  cluster.sync();
-  const int rank = (int)cluster.block_rank();
-  const uint32_t* peers[CALIB_CLUSTER];
+    for (int j = 0; j < CPT; ++j) {
+      const int c = tid + j * CALIB_THREADS;
+      if (c < nchunks) {
 #pragma unroll
-  for (int q = 0; q < CALIB_CLUSTER; ++q) peers[q] = cluster.map_shared_rank(s_col, q);
-  for (int w = rank * CALIB_THREADS + tid; w < (K >> 1); w += CALIB_CLUSTER * CALIB_THREADS) {
-    uint32_t m = 0;
+        for (int k = 0; k < 4; ++k) {
+          atomicMax(chan_absmax + 8 * c + 2 * k, cmax[j][k] << 16);
+          atomicMax(chan_absmax + 8 * c + 2 * k + 1, cmax[j][k] & 0xffff0000u);
+        }
+      }
+    }
+  } else {
 #pragma unroll
-    for (int q = 0; q < CALIB_CLUSTER; ++q) asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(peers[q][w]));
-    // (non-negative floats order like their bit patterns; a stale value read here only costs an atomic)
-    if ((m << 16) > __ldcg(chan_absmax + 2 * w)) atomicMax(chan_absmax + 2 * w, m << 16);
-    if ((m & 0xffff0000u) > __ldcg(chan_absmax + 2 * w + 1)) atomicMax(chan_absmax + 2 * w + 1, m & 0xffff0000u);
+    for (int j = 0; j < CPT; ++j) {
+      const int c = tid + j * CALIB_THREADS;
+      if (c < nchunks) *reinterpret_cast<uint4*>(s_col + 4 * c) = make_uint4(cmax[j][0], cmax[j][1], cmax[j][2], cmax[j][3]);
+    }
+    cluster.sync();
+    const int rank = (int)cluster.block_rank();
+    const uint32_t* peers[CALIB_CLUSTER];
+#pragma unroll
+    for (int q = 0; q < CALIB_CLUSTER; ++q) peers[q] = cluster.map_shared_rank(s_col, q);
+    for (int w = rank * CALIB_THREADS + tid; w < (K >> 1); w += CALIB_CLUSTER * CALIB_THREADS) {
+      uint32_t m = 0;
+#pragma unroll
+      for (int q = 0; q < CALIB_CLUSTER; ++q) asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(peers[q][w]));
+      // (non-negative floats order like their bit patterns; a stale value read here only costs an atomic)
+      if ((m << 16) > __ldcg(chan_absmax + 2 * w)) atomicMax(chan_absmax + 2 * w, m << 16);
+      if ((m & 0xffff0000u) > __ldcg(chan_absmax + 2 * w + 1)) atomicMax(chan_absmax + 2 * w + 1, m & 0xffff0000u);
+    }
   }
   if (above != nullptr) {
 #pragma unroll
@@ -728,7 +743,7 @@ arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, u
       if (t) atomicAdd(above, t);
     }
   }
-  cluster.sync();                                              // nobody leaves while its maxima are being read
+  if constexpr (CLUSTER) cluster.sync();                       // nobody leaves while its maxima are being read
 }
 
 }  // namespace
@@ -742,14 +757,14 @@ int launch_calib_stats(const void* x, int64_t rows, int K, float* chan_absmax, u
   const int cpt = (K / 8 + CALIB_THREADS - 1) / CALIB_THREADS;
   auto xs = static_cast<const uint16_t*>(x);
   auto cm = reinterpret_cast<unsigned int*>(chan_absmax);
-  auto launch = [&](auto kern, int rb) -> int {
+  auto launch = [&](auto kern, int rb, int csize = CALIB_CLUSTER) -> int {
     const size_t smem = (size_t)K * 2;
     // Unasked, a launch gets 48 KB, its static part (below 1 KB here) included.  The limit is the kernel's, not this call's:
     // always the same value, so that calls of several threads and widths cannot lower one another's.
     if (smem > 47 * 1024) ARCQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 32768));
     long long grid = (rows + rb - 1) / rb;
     if (grid > 2LL * di.num_sms) grid = 2LL * di.num_sms;
-    grid = (grid + CALIB_CLUSTER - 1) / CALIB_CLUSTER * CALIB_CLUSTER;
+    grid = (grid + csize - 1) / csize * csize;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(CALIB_THREADS);
@@ -759,13 +774,16 @@ int launch_calib_stats(const void* x, int64_t rows, int K, float* chan_absmax, u
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = CALIB_CLUSTER;
+    attr[1].val.clusterDim.x = (unsigned)csize;
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = csize > 1 ? 2 : 1;
     ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, xs, (long long)rows, K, cm, above));
     return ARCQ_OK;
   };
+  // Up to 64 rows of up to 4096 channels are one step of a few small CTAs, which a cluster's barriers and its look at the
+  // running maxima would only lengthen (2048 channels: 7 rows 5.5 -> 2.5 us, 40 rows 5.3 -> 3.4).
+  if (cpt <= 1 && rows <= 64) return launch(arcq_calib_stats_kernel<1, 2, false>, 2, 1);
   // (rows in flight per CTA: eight 16-byte loads per thread, two rows at least)
   if (cpt <= 1) return launch(arcq_calib_stats_kernel<1, 8>, 8);
   if (cpt <= 2) return launch(arcq_calib_stats_kernel<2, 4>, 4);

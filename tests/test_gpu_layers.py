@@ -487,6 +487,19 @@ def test_calibration_statistics_in_one_pass(k, rows):
     assert torch.equal(eager.value, want) and eager.select_num() == stat.select_num()
 
 
+@pytest.mark.parametrize("k,rows", [(8, 1), (64, 3), (4096, 2), (4096, 64), (4096, 65), (2040, 63), (4104, 5)])
+def test_calibration_of_few_rows(k, rows):
+    """Both sides of the row count and the width up to which the CTAs hand in their maxima one by one."""
+    from arcquant_b200 import calibrate
+
+    batches = [synth.activations(rows, k, i, synth.outlier_channels(k, 1, 3), device="cuda") * (1 + i) for i in range(2)]
+    stat = calibrate.ChannelAbsMax()
+    for b in batches:
+        stat.update(b)
+    assert torch.equal(stat.value, torch.cat(batches).abs().amax(0).float())
+    assert int(stat._above) == sum(int((b > b.max(dim=-1, keepdim=True)[0] * 0.125).sum()) for b in batches)
+
+
 def test_calibration_of_any_width_as_the_first_call_of_a_process():
     """Widths at which the kernel's dynamic shared memory alone, or only together with its static part, exceeds the 48 KB
     that a launch gets unasked; each of them first, since a wider call raises the limit for those that follow."""

@@ -135,15 +135,16 @@ def reorder_quantize_w(w, reorder_index, ke: int, mode=None):
 def quantize_tensor_scale(x, reorder_index, ke: int, mode=None, is_weight: bool = False, amax=None):
     """(codes, scales, scale) of x over its own per-tensor scale max / (448 * 6) - |x| for activations, the signed
     maximum for weights - in two launches (one if `amax`, max|x| on the device, is given: the scale then has its
-    shape), or None where that path does not apply: an empty or non-contiguous tensor, one off a 16-byte boundary,
+    shape), or None where that path does not apply: an empty or non-contiguous tensor, a weight off a 16-byte boundary,
     another type, no channel order, KQ > 16384."""
     if (reorder_index is None or not x.is_cuda or x.dtype != torch.bfloat16 or x.dim() != 2 or not x.is_contiguous()
-            or x.shape[0] == 0 or x.shape[1] > 16384 or x.data_ptr() % 16):
+            or x.shape[0] == 0 or x.shape[1] > 16384
+            or (is_weight and x.data_ptr() % 16)):
         return None
     ext = _ext()
     if ext:
-        q, sf, scale = ext.quantize_tensor_scale(x, reorder_index, ke, -1 if mode is None else mode, is_weight, amax)
-        return q, sf, scale if amax is None or amax.dim() == 0 else scale.reshape(amax.shape)
+        out = ext.quantize_tensor_scale(x, reorder_index, ke, -1 if mode is None else mode, is_weight, amax)
+        return out if amax is None or amax.dim() == 0 else (out[0], out[1], out[2].reshape(amax.shape))
     lib = _lib.load()
     _require(reorder_index, torch.int16, "reorder_index")
     rows, kq = x.shape

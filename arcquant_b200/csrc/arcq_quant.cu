@@ -50,8 +50,8 @@ struct QuantParams {
   int mode;       // 16 or 32 (placement of critical groups, residual flavour)
   int is_weight;  // residual slot = copy of the main codes
   float eps;
-  const float* scale;   // warp-specialised plain kernel only: x is divided by *scale (device) first, or nullptr
-  // Grouped rows (warp-specialised kernel only): the rows form `ngroups` runs, run e starting at output
+  const float* scale;   // plain operator: x is divided by *scale (device) first (see ScaleOptions), or nullptr
+  // Grouped rows: the rows form `ngroups` runs, run e starting at output
   // row groups[e] with groups[ngroups + e] rows (device memory, so the host never learns the sizes);
   // run e uses the channel order idx + e*KQ and the scale scale[e].  row_map (or nullptr): input row of
   // every output row.
@@ -1289,8 +1289,8 @@ arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const
 //
 // Bound: HBM (2*KQ + 9/16*(KQ+KE) bytes per row); what competes with it is shared-memory bandwidth and issue
 // slots, and this organisation is the one that needs the least of both:
-//  * the R rows are interleaved in shared memory (word pair (row0, row1) per channel for R = 2, 8 bytes per
-//    channel for R = 4), so one shared load gathers a channel of all R rows;
+//  * the two rows are interleaved in shared memory (a word (row0, row1) per channel), so one shared load gathers a
+//    channel of both;
 //  * a thread keeps the same GPT groups for all the rows it meets: their 16 GPT (swizzled) positions stay in
 //    registers, two per register, and no offset table is read;
 //  * rows go from global memory through registers straight into the interleaved buffer (no staging copy), with
@@ -1299,16 +1299,9 @@ arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const
 // A warp stores 256 contiguous bytes of codes per row; the scale bytes of four neighbouring groups are brought
 // together with two shuffles and leave as one 32-bit word per row.
 // RMSNorm: thread t holds chunks t and t + KQ/16, the reference's assignment and summation order (T == KQ/16).
-template <int R>
-__device__ __forceinline__ uint32_t row_pos(uint32_t ch) {      // byte offset of channel ch's R values
-  if (R == 2) return word_offset(ch);
-  const uint32_t j = ch >> 1;                                  // 16-byte unit of two channels
-  return ((j ^ ((j >> 3) & 3u)) << 4) | ((ch & 1u) << 3);
-}
-
-template <int R, int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB>
+template <int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const QuantParams p, const ScaleOptions so) {
-  constexpr int NW = R / 2, CPT = 2 * GPT;
+  constexpr int R = 2, CPT = 2 * GPT;                           // rows of a unit, 16-byte chunks per thread and row
   static_assert(!RMS || GPT == 1, "RMSNorm: one group per thread");
   extern __shared__ __align__(16) uint8_t smem[];
   const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5;
@@ -1401,16 +1394,16 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
       const int g = min(tid + j * T, G - 1);
       if (idx == nullptr) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) off[j][k] = row_pos<R>(16 * g + 2 * k) | (row_pos<R>(16 * g + 2 * k + 1) << 16);
+        for (int k = 0; k < 8; ++k) off[j][k] = word_offset(16 * g + 2 * k) | (word_offset(16 * g + 2 * k + 1) << 16);
       } else if ((reinterpret_cast<uintptr_t>(idx) & 15u) == 0) {
         const uint4 lo = __ldg(reinterpret_cast<const uint4*>(idx) + 2 * g), hi = __ldg(reinterpret_cast<const uint4*>(idx) + 2 * g + 1);
         const uint32_t ww[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
-        for (int k = 0; k < 8; ++k) off[j][k] = row_pos<R>(ww[k] & 0xffffu) | (row_pos<R>(ww[k] >> 16) << 16);
+        for (int k = 0; k < 8; ++k) off[j][k] = word_offset(ww[k] & 0xffffu) | (word_offset(ww[k] >> 16) << 16);
       } else {
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-          off[j][k] = row_pos<R>((uint32_t)(uint16_t)idx[16 * g + 2 * k]) | (row_pos<R>((uint32_t)(uint16_t)idx[16 * g + 2 * k + 1]) << 16);
+          off[j][k] = word_offset((uint32_t)(uint16_t)idx[16 * g + 2 * k]) | (word_offset((uint32_t)(uint16_t)idx[16 * g + 2 * k + 1]) << 16);
       }
     }
   };
@@ -1490,41 +1483,31 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
     for (int j = 0; j < CPT; ++j) {
       const int c = tid + j * T;
       if (c < nchunks) {
-        uint32_t o[NW][8];        // [row pair][channel]
+        uint32_t o[8];            // a word (row 0, row 1) per channel
+        const uint4 x0 = a[0][j], x1 = a[1][j];
+        const uint32_t wa[4] = {x0.x, x0.y, x0.z, x0.w}, wb[4] = {x1.x, x1.y, x1.z, x1.w};
 #pragma unroll
-        for (int q = 0; q < NW; ++q) {
-          const uint4 x0 = a[2 * q][j], x1 = a[2 * q + 1][j];
-          const uint32_t wa[4] = {x0.x, x0.y, x0.z, x0.w}, wb[4] = {x1.x, x1.y, x1.z, x1.w};
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            if (RMS) {
-              // bf16 x bf16 is exact in fp32; then one rounding by rstd (both rows in one FMUL2), one to bf16
-              const uint4 g8 = gn[j & 1];
-              const uint32_t gw = k == 0 ? g8.x : (k == 1 ? g8.y : (k == 2 ? g8.z : g8.w));
-              const uint16_t ga = half_lo(gw), gb = half_hi(gw);
-              const float2 r2 = make_float2(rstd[2 * q], rstd[2 * q + 1]);
-              const float2 n0 = __fmul2_rn(make_float2(fma_bf16(half_lo(wa[k]), ga, -0.0f), fma_bf16(half_lo(wb[k]), ga, -0.0f)), r2);
-              const float2 n1 = __fmul2_rn(make_float2(fma_bf16(half_hi(wa[k]), gb, -0.0f), fma_bf16(half_hi(wb[k]), gb, -0.0f)), r2);
-              o[q][2 * k] = pack_bf16x2_rn(n0.x, n0.y);
-              o[q][2 * k + 1] = pack_bf16x2_rn(n1.x, n1.y);
-            } else if (SCALED) {
-              div_pair_words(wa[k], wb[k], sc, rsc, fast, o[q][2 * k], o[q][2 * k + 1]);
-            } else {
-              o[q][2 * k] = __byte_perm(wa[k], wb[k], 0x5410);
-              o[q][2 * k + 1] = __byte_perm(wa[k], wb[k], 0x7632);
-            }
+        for (int k = 0; k < 4; ++k) {
+          if (RMS) {
+            // bf16 x bf16 is exact in fp32; then one rounding by rstd (both rows in one FMUL2), one to bf16
+            const uint4 g8 = gn[j & 1];
+            const uint32_t gw = k == 0 ? g8.x : (k == 1 ? g8.y : (k == 2 ? g8.z : g8.w));
+            const uint16_t ga = half_lo(gw), gb = half_hi(gw);
+            const float2 r2 = make_float2(rstd[0], rstd[1]);
+            const float2 n0 = __fmul2_rn(make_float2(fma_bf16(half_lo(wa[k]), ga, -0.0f), fma_bf16(half_lo(wb[k]), ga, -0.0f)), r2);
+            const float2 n1 = __fmul2_rn(make_float2(fma_bf16(half_hi(wa[k]), gb, -0.0f), fma_bf16(half_hi(wb[k]), gb, -0.0f)), r2);
+            o[2 * k] = pack_bf16x2_rn(n0.x, n0.y);
+            o[2 * k + 1] = pack_bf16x2_rn(n1.x, n1.y);
+          } else if (SCALED) {
+            div_pair_words(wa[k], wb[k], sc, rsc, fast, o[2 * k], o[2 * k + 1]);
+          } else {
+            o[2 * k] = __byte_perm(wa[k], wb[k], 0x5410);
+            o[2 * k + 1] = __byte_perm(wa[k], wb[k], 0x7632);
           }
         }
         uint4* b4 = reinterpret_cast<uint4*>(buf);
-        if (R == 2) {
-          b4[swz16(2u * c)] = make_uint4(o[0][0], o[0][1], o[0][2], o[0][3]);
-          b4[swz16(2u * c + 1u)] = make_uint4(o[0][4], o[0][5], o[0][6], o[0][7]);
-        } else {
-          const uint32_t x = ((uint32_t)c >> 1) & 3u;          // unit 4c + u sits at 4c + (u ^ x): see row_pos
-#pragma unroll
-          for (int u = 0; u < 4; ++u)
-            b4[4u * c + ((uint32_t)u ^ x)] = make_uint4(o[0][2 * u], o[NW - 1][2 * u], o[0][2 * u + 1], o[NW - 1][2 * u + 1]);
-        }
+        b4[swz16(2u * c)] = make_uint4(o[0], o[1], o[2], o[3]);
+        b4[swz16(2u * c + 1u)] = make_uint4(o[4], o[5], o[6], o[7]);
       }
     }
     __syncthreads();
@@ -1546,48 +1529,37 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
       const int g = tid + j * T;
       if (GPT > 1 && (g & ~31) >= G) break;                    // (whole warps)
       const bool live = g < G;
-      auto gather = [&](uint32_t (&w)[NW][16]) {
+      auto gather = [&](uint32_t (&w)[16]) {
 #pragma unroll
-        for (int k = 0; k < 16; ++k) {
-          const uint32_t o = (k & 1) ? off[j][k >> 1] >> 16 : off[j][k >> 1] & 0xffffu;
-          if (R == 2) {
-            w[0][k] = *reinterpret_cast<const uint32_t*>(buf + o);
-          } else {
-            const uint2 v = *reinterpret_cast<const uint2*>(buf + o);
-            w[0][k] = v.x;
-            w[NW - 1][k] = v.y;
-          }
-        }
+        for (int k = 0; k < 16; ++k)
+          w[k] = *reinterpret_cast<const uint32_t*>(buf + ((k & 1) ? off[j][k >> 1] >> 16 : off[j][k >> 1] & 0xffffu));
       };
-      uint32_t w[NW][16];
+      uint32_t w[16];
       gather(w);
       const int jc = g - (int)e_G0;
       const bool critical = jc >= 0;
       uint32_t col = (uint32_t)g;
       if (critical) col = mode32 ? (uint32_t)((int)e_G0 + ((jc >> 1) << 2) + (jc & 1)) : (uint32_t)(g + jc);
-      uint32_t codes = 0;                                      // scale code of row i in byte i
-#pragma unroll
-      for (int q = 0; q < NW; ++q) {
-        uint32_t c2;
+      uint32_t codes;                                          // scale code of row i in byte i
+      {
         float2 dec, rcp;
-        scale_of_pair_fma(amax_pair_h(w[q]), c2, dec, rcp);
+        scale_of_pair_fma(amax_pair_h(w), codes, dec, rcp);
         uint2 c0, c1;
-        encode_pair(w[q], rcp.x, rcp.y, c0, c1);
-        codes |= c2 << (16 * q);
-        uint8_t* q0 = qrow + (size_t)(2 * q) * row_bytes + 8u * col;
-        if (live && (uint32_t)(2 * q) < nrows) *reinterpret_cast<uint2*>(q0) = c0;
-        if (live && (uint32_t)(2 * q + 1) < nrows) *reinterpret_cast<uint2*>(q0 + row_bytes) = c1;
+        encode_pair(w, rcp.x, rcp.y, c0, c1);
+        uint8_t* q0 = qrow + 8u * col;
+        if (live) *reinterpret_cast<uint2*>(q0) = c0;
+        if (live && nrows > 1) *reinterpret_cast<uint2*>(q0 + row_bytes) = c1;
       }
       // scale bytes: four plain groups side by side form a 32-bit word per row
       {
         const uint32_t x = __shfl_xor_sync(0xffffffffu, codes, 1);
-        const uint32_t t = (lane & 1) ? __byte_perm(x, codes, 0x7351) : __byte_perm(codes, x, 0x6240);   // rows 1,3 / 0,2
+        const uint32_t t = (lane & 1) ? __byte_perm(x, codes, 0x7351) : __byte_perm(codes, x, 0x6240);   // row 1 / 0
         const uint32_t y = __shfl_xor_sync(0xffffffffu, t, 2);
         const uint32_t word = (lane & 2) ? __byte_perm(y, t, 0x7632) : __byte_perm(t, y, 0x5410);
         const uint32_t gq = (uint32_t)g & ~3u;
         if (gq + 3 < e_G0) {                                   // (G0 <= G: all four lanes are live)
           const uint32_t i = (uint32_t)lane & 3u;              // this lane's row of the unit
-          if (i < nrows && i < (uint32_t)R) *reinterpret_cast<uint32_t*>(sfrow + 16u * i + ((gq >> 2) << 9)) = word;
+          if (i < nrows) *reinterpret_cast<uint32_t*>(sfrow + 16u * i + ((gq >> 2) << 9)) = word;
         } else if (live) {
           uint8_t* s0 = sfrow + (((col >> 2) << 9) | (col & 3u));
 #pragma unroll
@@ -1598,33 +1570,27 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
       if (critical && live) {
         // the re-quantized residual (or, for weights, a copy of the main codes)
         const uint32_t rcol = col + (mode32 ? 2u : 1u);
-        uint32_t v[NW][16];
+        uint32_t v[16];
         gather(v);
-#pragma unroll
-        for (int q = 0; q < NW; ++q) {
-          const uint32_t m = amax_pair_h(v[q]);
-          uint32_t rc;
-          float2 dec, rcp, raw;
-          scale_of_pair_fma(m, rc, dec, rcp, &raw);
-          uint2 c0, c1;
-          encode_pair(v[q], rcp.x, rcp.y, c0, c1);
-          if (!is_weight) {
-            if (mode32) dec = raw;      // against the un-rounded fp32 scale
-            residual_pair(v[q], c0, c1, dec.x, dec.y);
-            float2 rdec, rrcp;
-            scale_of_pair_fma(amax_pair_h(v[q]), rc, rdec, rrcp);
-            encode_pair(v[q], rrcp.x, rrcp.y, c0, c1);
-          }
-          uint8_t* q0 = qrow + (size_t)(2 * q) * row_bytes + 8u * rcol;
-          uint8_t* s0 = sfrow + 32 * q + (((rcol >> 2) << 9) | (rcol & 3u));
-          if ((uint32_t)(2 * q) < nrows) {
-            *reinterpret_cast<uint2*>(q0) = c0;
-            s0[0] = (uint8_t)rc;
-          }
-          if ((uint32_t)(2 * q + 1) < nrows) {
-            *reinterpret_cast<uint2*>(q0 + row_bytes) = c1;
-            s0[16] = (uint8_t)(rc >> 8);
-          }
+        uint32_t rc;
+        float2 dec, rcp, raw;
+        scale_of_pair_fma(amax_pair_h(v), rc, dec, rcp, &raw);
+        uint2 c0, c1;
+        encode_pair(v, rcp.x, rcp.y, c0, c1);
+        if (!is_weight) {
+          if (mode32) dec = raw;        // against the un-rounded fp32 scale
+          residual_pair(v, c0, c1, dec.x, dec.y);
+          float2 rdec, rrcp;
+          scale_of_pair_fma(amax_pair_h(v), rc, rdec, rrcp);
+          encode_pair(v, rrcp.x, rrcp.y, c0, c1);
+        }
+        uint8_t* q0 = qrow + 8u * rcol;
+        uint8_t* s0 = sfrow + (((rcol >> 2) << 9) | (rcol & 3u));
+        *reinterpret_cast<uint2*>(q0) = c0;
+        s0[0] = (uint8_t)rc;
+        if (nrows > 1) {
+          *reinterpret_cast<uint2*>(q0 + row_bytes) = c1;
+          s0[16] = (uint8_t)(rc >> 8);
         }
       }
     }
@@ -1714,9 +1680,10 @@ cudaError_t allow_shared_memory(Kernel kern, const DeviceInfo& di) {
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem_optin);
 }
 
-template <int R, int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB>
+template <int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB>
 int launch_rows(const QuantParams& p, const ScaleOptions& so, long long units, int T, const DeviceInfo& di, cudaStream_t stream) {
-  auto kern = arcq_quantize_rows_kernel<R, GPT, RMS, SCALED, GROUPED, PF, MAXT, MINB>;
+  constexpr int R = 2;
+  auto kern = arcq_quantize_rows_kernel<GPT, RMS, SCALED, GROUPED, PF, MAXT, MINB>;
   const size_t smem = (size_t)p.KQ * 2 * R + (RMS ? (size_t)(R * T + R) * sizeof(float) : 64);
   // the attribute and the occupancy query cost host time: once per (device, block size, shared memory)
   static thread_local int c_dev = -1, c_threads = 0, c_occ = 0;
@@ -1890,9 +1857,9 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
 
   // Row kernel: little work per SM.  A unit is a pair of rows and the kernel's resident CTAs take one unit each at
   // once (three CTAs of up to 256 threads per SM, one of 512), so up to that many units it is a single pass with no
-  // rings to set up: 16 rows of 4096 channels 4.0 -> 3.3 us (fused RMSNorm), 777 rows divided by their scale 6.2 ->
-  // 5.3, 16 rows of 14336 channels 6.8 -> 5.5.  Beyond it the warp-specialised kernel below streams better (fused
-  // RMSNorm, 16 384 rows: 50.6 against 60.7 us).  With grouped rows the host knows a bound only.
+  // rings to set up.  us, the kernel below / this one: fused RMSNorm of 4096 channels 16 rows 4.1 / 3.3, 592 rows 5.0 /
+  // 4.2; divided by their scale 880 rows 5.5 / 4.9; 14 336 channels 16 rows 6.0 / 4.7, 290 rows 6.3 / 5.0.  Beyond it the
+  // warp-specialised kernel streams better (fused RMSNorm, 16 384 rows: 50.6 / 60.7).  With grouped rows the host knows a bound only.
   const long long real_rows = groups != nullptr ? std::max<long long>(rows - 256LL * ngroups, 1) : rows;
   const long long units = (real_rows + 1) / 2;
   const int T = wide ? ((p.G + 1) / 2 + 31) / 32 * 32 : (p.G + 31) / 32 * 32;
@@ -1901,16 +1868,16 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
       (units <= per_sm * di.num_sms || (p.G < 32 && !rms))) {
 #define ARCQ_ROWS(RMS_, SC_, GR_)                                                                                   \
   {                                                                                                                 \
-    if (wide) return launch_rows<2, 2, false, SC_, GR_, false, 512, 1>(p, so, units, T, di, stream);                           \
-    return T <= 256 ? launch_rows<2, 1, RMS_, SC_, GR_, true, 256, 3>(p, so, units, T, di, stream)                             \
-                    : launch_rows<2, 1, RMS_, SC_, GR_, true, 512, 1>(p, so, units, T, di, stream);                            \
+    if (wide) return launch_rows<2, false, SC_, GR_, false, 512, 1>(p, so, units, T, di, stream);                           \
+    return T <= 256 ? launch_rows<1, RMS_, SC_, GR_, true, 256, 3>(p, so, units, T, di, stream)                             \
+                    : launch_rows<1, RMS_, SC_, GR_, true, 512, 1>(p, so, units, T, di, stream);                            \
   }
     if (groups != nullptr && scale != nullptr) ARCQ_ROWS(false, true, true)
     if (groups != nullptr) ARCQ_ROWS(false, false, true)
     if (scale != nullptr) ARCQ_ROWS(false, true, false)
     if (!rms) ARCQ_ROWS(false, false, false)
-    return T <= 256 ? launch_rows<2, 1, true, false, false, true, 256, 3>(p, so, units, T, di, stream)
-                    : launch_rows<2, 1, true, false, false, true, 512, 1>(p, so, units, T, di, stream);
+    return T <= 256 ? launch_rows<1, true, false, false, true, 256, 3>(p, so, units, T, di, stream)
+                    : launch_rows<1, true, false, false, true, 512, 1>(p, so, units, T, di, stream);
 #undef ARCQ_ROWS
   }
 
@@ -2004,7 +1971,7 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
       }
     }
   }
-  // only the warp-specialised kernel divides by the scale, walks grouped rows or follows a row map
+  // the kernel below neither divides by the scale nor walks grouped rows nor follows a row map
   if (p.scale || p.groups || p.row_map) return ARCQ_ERR_UNSUPPORTED_K;
 
   const size_t table = 160 + (((size_t)KQ * (rawidx ? 2 : 4) + 15) & ~(size_t)15);

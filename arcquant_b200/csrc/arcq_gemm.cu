@@ -891,8 +891,10 @@ static void plan_splitk(int64_t M, int64_t N, int64_t K_eff, int num_sms, int* b
 static bool use_skinny_kernel(int64_t M, int64_t N, int64_t K_eff, int num_sms, bool residual = false) {
   return M <= ARCQ_SKINNY_ROWS || (((M + 127) / 128) * ((N + 127) / 128) <= num_sms && (residual || skinny_plan_splits(M, N, K_eff) > 1));
 }
-// With the SwiGLU epilogue (gate and up blocks in different CTAs of a cluster): [28672, 4224] 65 rows 24.8 / 30.9 us,
-// 128 rows 26.9 / 31.4, 200 rows 43.1 / 31.6 (CTA pairs with four epilogue warps; eight take about 5 % off).
+// With the SwiGLU epilogue (gate and up blocks in different CTAs of a cluster), us, this kernel at 65 and at 128 rows / CTA
+// pairs at 129: [2048, 2176] 10.3 and 12.2 / 14.3, [3584, 4224] 12.2 and 12.4 / 16.5, [7168, 4224] 14.4 and 17.0 / 18.5, [14336,
+// 4224] 16.9 and 19.6 / 18.6, [28672, 4224] 22.6 and 24.6 / 28.7, [57344, 8320] 62.0 and 69.8 / 82.5.  At 200 rows CTA pairs are
+// the better ones ([28672, 4224] 43.1 / 31.6).
 constexpr int64_t SKINNY_GATED_ROWS = 128;
 // (At least two CTAs per 256 columns and 128 rows: under an SM limit only where that many may run, see arcq_set_sm_limit.)
 static bool use_skinny_gated(int64_t M, int64_t N, const DeviceInfo& di) {

@@ -68,8 +68,9 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   }
 }
 // SiLU for a gate that is a bf16 value and a result that is rounded to bf16: after that rounding, the bits of the eager
-// chain g / (1 + expf(-g)) for every one of the 65 536 gates (tests/test_gpu_silu.py), from two special-function
-// instructions and four on the FMA pipe.  The factor 1/4 keeps the reciprocal's argument below 2^126 - where it would be
+// chain g / (1 + expf(-g)) for every finite gate, from two special-function instructions and four on the FMA pipe.
+// (tests/test_gpu_silu.py goes through all of them, times an up value of the gate's size: below |g| ~ 2^-66 that product
+// underflows and does not show SiLU's bits, but there both chains are g / 2 exactly.)  +-inf and NaN as in the eager chain.  The factor 1/4 keeps the reciprocal's argument below 2^126 - where it would be
 // flushed - exactly as long as expf(-g) is finite.
 __device__ __forceinline__ float silu_for_bf16(float g) {
   float e, r;

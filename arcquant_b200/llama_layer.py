@@ -186,8 +186,8 @@ class QLlamaDecoderLayerTP(torch.nn.Module):
                  group=None, device="cuda", fuse_swiglu: bool = True):
         """fuse_swiglu: pack gate and up interleaved in blocks of 128 channels so that SiLU(gate) * up (and its
         max|.|) is computed in the gate_up GEMM's epilogue instead of a pass of its own over [tokens, 2 * ffn];
-        same bits either way.  Needs ffn / tp_size to be a multiple of 128; meant for prefill-sized batches
-        (the fused GEMM always runs the CTA-pair kernel)."""
+        the same bits, except that few tokens may sum K in another order.  Needs ffn / tp_size to be a multiple
+        of 128."""
         super().__init__()
         self.cfg, self.rank, self.tp, self.group = cfg, tp_rank, tp_size, group
         self.fuse_swiglu = bool(fuse_swiglu) and (cfg.ffn // tp_size) % 128 == 0

@@ -173,8 +173,8 @@ int arcq_matmul_nvfp4_ws(const uint8_t* A, const uint8_t* B, const uint8_t* SFA,
 /* Which kernel arcq_matmul_nvfp4* would run for this shape on the current device (no counterpart in the
  * reference, whose CUTLASS template picks nothing at run time): *kind = ARCQ_GEMM_KIND_PAIR (persistent
  * CTA pairs, 256 x 256 tiles), ARCQ_GEMM_KIND_SINGLE (one CTA per 128 x tile_n tile) or
- * ARCQ_GEMM_KIND_SKINNY (up to ARCQ_SKINNY_ROWS rows, or 128 x 128 tiles that leave an SM for each: weight streaming, K
- * split over *splits CTAs of a cluster that add their partial sums on chip); ARCQ_GEMM_KIND_SPLIT_K (partial sums in
+ * ARCQ_GEMM_KIND_SKINNY (up to ARCQ_SKINNY_ROWS rows, or 128 x 128 tiles that leave an SM for each and a K long enough to
+ * be split: weight streaming, K split over *splits CTAs of a cluster that add their partial sums on chip); ARCQ_GEMM_KIND_SPLIT_K (partial sums in
  * scratch) is no longer chosen.  *tile_n: tile width; *splits: 1 unless split.  Any output pointer may be NULL. */
 #define ARCQ_GEMM_KIND_SINGLE 0
 #define ARCQ_GEMM_KIND_SPLIT_K 1
@@ -187,7 +187,7 @@ int arcq_matmul_plan(int64_t M, int64_t N, int64_t K_eff, int* kind, int* tile_n
  * memory: code that runs where an allocation would fail or stall - an inference-server plugin
  * whose enqueue hook is forbidden to call the allocator, a process whose whole device memory has
  * been handed to another framework's pool, a latency-critical loop where a cudaMalloc would
- * serialise the device.  Same arithmetic and same split as arcq_matmul_nvfp4_ws.  Inputs and the output are the
+ * serialise the device.  The same kernels as arcq_matmul_nvfp4_ws, with the same result.  Inputs and the output are the
  * caller's.  The call allocates nothing: no cudaMalloc / cudaFree, no allocating library routine.
  *   - Shapes with arcq_matmul_workspace_bytes(M,N,K_eff) > ARCQ_STATIC_SCRATCH_BYTES (e.g. M 128 x N 4096 x
  *     K_eff 14464) are refused with ARCQ_ERR_SCRATCH_LIMIT.
@@ -303,10 +303,11 @@ int arcq_matmul_nvfp4_grouped(const uint8_t* A, const uint8_t* B, const uint8_t*
  * in blocks of 128 output channels - rows [256 t, 256 t + 128) of B are gate channels [128 t, 128 t + 128),
  * rows [256 t + 128, 256 t + 256) the same up channels - so one output tile holds matching gate and up
  * columns and the epilogue writes C [M, N/2] = bf16(bf16(silu(g)) * u) directly, g and u being the
- * bf16-rounded GEMM results: the same bits as arcq_matmul_nvfp4 followed by arcq_silu_mul_bf16, without the
- * [M, N] round trip through memory.  amax (fp32, device) receives max|C| over the valid rows - the
- * per-tensor maximum the down projection's quantizer needs.  N % 256 == 0.  Always runs the CTA-pair
- * kernel (meant for prefill-sized M).
+ * bf16-rounded GEMM results: arcq_matmul_nvfp4 followed by arcq_silu_mul_bf16 without the [M, N] round trip
+ * through memory.  The same bits where neither call splits K (arcq_matmul_plan); where one does - few rows, or
+ * few output tiles - their fp32 sums are formed in another order and may differ by a bf16 step now and then.
+ * amax (fp32, device) receives max|C| over the valid rows - the per-tensor maximum the down projection's
+ * quantizer needs.  N % 256 == 0.  CTA pairs, or weight streaming for few rows.
  * arcq_matmul_nvfp4_grouped_swiglu: the same over the runs of a grouped problem (see above); amax has one
  * entry per run and `groups` says where each run's valid rows end. */
 int arcq_matmul_nvfp4_swiglu(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB,

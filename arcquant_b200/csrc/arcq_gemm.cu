@@ -259,21 +259,21 @@ arcq_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 // Per SM this is 9.5 KB of operands per K step instead of 13.5 KB, and the smaller stage
 // (38 KB) lets five stages fit.
 //
-// Scale factors do not go through tcgen05.cp here: measured on this kernel, the twelve copies of
-// a stage execute strictly in sequence with its MMAs in the tensor pipe and cost as much as the
-// MMAs themselves.  Instead four "scale" warps per CTA (one per TMEM lane quadrant) read the
-// stage's atoms from shared memory and write them to TMEM with tcgen05.st, off the tensor pipe,
-// one stage ahead of the MMAs; each stage owns its own 48 TMEM columns.
+// Scale factors go shared memory -> tensor memory with tcgen05.cp (cta_group::2: each CTA's own atoms into its own tensor
+// memory), twelve copies in front of a stage's MMAs, issued by the same thread.  Each stage owns 48 TMEM columns, so a copy
+// never meets an MMA that still reads them: the stage's barrier was released by those MMAs.
+// What bounds the main loop: the tensor pipe, 4 x 128 cycles a stage.  Loads alone need 450 cycles a stage, copies alone 325,
+// MMAs alone 512 + what a tile boundary costs (730 a tile); all together 588, of which 76 are the boundary (17 stages
+// a tile, [16384, 27648, 4224]).  While every role sat behind `lane == 0` a stage took 866 (see elect_one), and four warps
+// carried the scales with tcgen05.st because copies looked as expensive as the MMAs.
 //
-// Synchronisation: A/B loads of either CTA complete on the LEADER's "full" barrier
-// (.cta_group::2 form; the barrier address is the CTA-local one with the pair's rank bit cleared);
-// scale loads complete on a CTA-local barrier; the scale warps of both CTAs arrive on the leader's
-// "scales ready" barrier; tcgen05.commit with a two-CTA mask releases the stage in both CTAs and
-// publishes the accumulator to both epilogues; the epilogue warps of both CTAs arrive on the
-// leader's "accumulator free" barrier.  No load uses cluster multicast.
+// Synchronisation: all loads of either CTA complete on the LEADER's "full" barrier (.cta_group::2 form; the barrier address
+// is the CTA-local one with the pair's rank bit cleared); tcgen05.commit with a two-CTA mask releases the stage in both
+// CTAs and publishes the accumulator to both epilogues; the epilogue warps of both CTAs arrive on the leader's
+// "accumulator free" barrier.  No load uses cluster multicast.
 
 constexpr int C2_STAGES = 5;
-constexpr int C2_THREADS = 512;                     // producer, MMA, 2 idle; 4 scale; 8 epilogue warps
+constexpr int C2_THREADS = 320;                     // producer, MMA, 8 epilogue warps
 constexpr int C2_A_BYTES = 128 * BK_BYTES;          // 16 KB
 constexpr int C2_B_BYTES = 128 * BK_BYTES;          // 16 KB: this CTA's half of the 256 B rows
 constexpr int C2_SFA_BYTES = KSTEPS * ATOM;         // 2 KB
@@ -315,6 +315,9 @@ __device__ __forceinline__ void tc_mma_nvf4_pair(uint32_t tmem_d, uint64_t adesc
       "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%4], [%5], p;\n}"
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(tsfa), "r"(tsfb), "r"(accumulate)
       : "memory");
+}
+__device__ __forceinline__ void tc_cp_sf_pair(uint32_t taddr, uint64_t desc) {
+  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {   // remote arrive on the leader's barrier
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar & PEER_BIT_MASK) : "memory");
@@ -371,8 +374,7 @@ __device__ __forceinline__ void pair_tile_coords(int tile, const Gemm2Params& p,
 
 // RESID: the epilogue adds a residual tile (bf16 [M, N], map_r) to the bf16-rounded result before it stores:
 // C = bf16(R + bf16(alpha * A B^T)), what a bf16 addition after the GEMM computes.  The tile arrives by TMA in
-// the same staging memory the output leaves from (per-thread loads of 32 different rows per instruction would
-// hold up the scale warps' shared-memory loads, as per-thread stores did).
+// the same staging memory the output leaves from (per-thread loads would touch 32 different rows per instruction).
 template <bool SWIGLU, bool RESID = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(C2_THREADS, 1)
 arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -387,15 +389,13 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   volatile uint32_t* misc =
       reinterpret_cast<volatile uint32_t*>(base_ptr + C2_STAGES * C2_STAGE_BYTES + C2_CSTAGE_BYTES + 192);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(misc + 1);
-  auto full_bar = [&](int s) { return bar_base + 8u * s; };                       // A/B landed (leader's is used)
+  auto full_bar = [&](int s) { return bar_base + 8u * s; };                       // both CTAs' loads landed (leader's is used)
   auto empty_bar = [&](int s) { return bar_base + 8u * (C2_STAGES + s); };        // stage reusable
-  auto sf_full_bar = [&](int s) { return bar_base + 8u * (2 * C2_STAGES + s); };  // this CTA's scale atoms landed
-  auto sf_ready_bar = [&](int s) { return bar_base + 8u * (3 * C2_STAGES + s); }; // scales in TMEM (leader's is used)
-  const uint32_t tmem_full_bar = bar_base + 8u * (4 * C2_STAGES);
+  const uint32_t tmem_full_bar = bar_base + 8u * (2 * C2_STAGES);
   const uint32_t tmem_empty_bar = tmem_full_bar + 8u;
   auto resid_bar = [&](int w) { return bar_base + 256u + 8u * w; };              // residual box of epilogue warp w landed
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();        // 0 = leader (issues the MMAs), 1 = peer
   const int cluster_id = blockIdx.x >> 1, num_clusters = gridDim.x >> 1;
 
@@ -403,8 +403,6 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     for (int s = 0; s < C2_STAGES; ++s) {
       mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
-      mbar_init(sf_full_bar(s), 1);
-      mbar_init(sf_ready_bar(s), 8);              // four scale warps in each of the two CTAs
     }
     mbar_init(tmem_full_bar, 1);
     mbar_init(tmem_empty_bar, 16);                // eight epilogue warps in each of the two CTAs
@@ -427,12 +425,10 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 
   const int num_tiles = p.tiles_m * p.tiles_n;
   const int kstages = (p.ksteps_total + KSTEPS - 1) / KSTEPS;
-  constexpr uint32_t AB_TX = 2u * (C2_A_BYTES + C2_B_BYTES);   // A/B bytes both CTAs deliver per stage
-  constexpr uint32_t SF_TX = C2_SFA_BYTES + C2_SFB_BYTES;      // scale bytes of one CTA per stage
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer (both CTAs)
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (int tile = cluster_id; tile < num_tiles && ok; tile += num_clusters) {
@@ -450,15 +446,12 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag)) { ok = false; break; }
           const uint32_t st = base + s * C2_STAGE_BYTES;
           const uint32_t lbar = full_bar(s) & PEER_BIT_MASK;
-          if (rank == 0) mbar_expect_tx(full_bar(s), AB_TX);
-          mbar_expect_tx(sf_full_bar(s), SF_TX);
-          // scale atoms first (the scale warps work one hop ahead of the MMAs): rows of the map are
-          // atoms (128 words each); one box = the four K atoms of this stage
-          tma_load_2d(st + C2_A_BYTES + C2_B_BYTES, &map_sfa, sf_full_bar(s), 0, sfa_tile * p.natoms + ks * KSTEPS);
-          tma_load_2d(st + C2_A_BYTES + C2_B_BYTES + C2_SFA_BYTES, &map_sfb, sf_full_bar(s), 0,
-                      sfb_tile * p.natoms + ks * KSTEPS);
-          tma_load_2d(st + C2_A_BYTES + C2_B_BYTES + C2_SFA_BYTES + KSTEPS * ATOM, &map_sfb, sf_full_bar(s), 0,
-                      (sfb_tile + 1) * p.natoms + ks * KSTEPS);
+          if (rank == 0) mbar_expect_tx(full_bar(s), 2u * C2_STAGE_BYTES);   // what both CTAs deliver
+          // scale atoms: rows of the map are atoms (128 words each); one box = the four K atoms of this stage
+          tma_load_2d_pair(st + C2_A_BYTES + C2_B_BYTES, &map_sfa, lbar, 0, sfa_tile * p.natoms + ks * KSTEPS);
+          tma_load_2d_pair(st + C2_A_BYTES + C2_B_BYTES + C2_SFA_BYTES, &map_sfb, lbar, 0, sfb_tile * p.natoms + ks * KSTEPS);
+          tma_load_2d_pair(st + C2_A_BYTES + C2_B_BYTES + C2_SFA_BYTES + KSTEPS * ATOM, &map_sfb, lbar, 0,
+                           (sfb_tile + 1) * p.natoms + ks * KSTEPS);
           tma_load_2d_pair(st, &map_a, lbar, ks * BK_BYTES, row_a);
           tma_load_2d_pair(st + C2_A_BYTES, &map_b, lbar, ks * BK_BYTES, row_b);
         }
@@ -466,7 +459,7 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer (leader CTA only)
-    if (lane == 0 && rank == 0) {
+    if (rank == 0 && elect_one()) {
       constexpr uint32_t idesc = (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
       uint32_t it = 0, tile_it = 0;
       bool ok = true;
@@ -481,7 +474,6 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         for (int ks = 0; ks < kstages; ++ks, ++it) {
           const int s = it % C2_STAGES;
           const uint32_t ph = (it / C2_STAGES) & 1u;
-          if (!mbar_wait(sf_ready_bar(s), ph, abort_flag)) { ok = false; break; }
           if (!mbar_wait(full_bar(s), ph, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const int nk = min(KSTEPS, p.ksteps_total - ks * KSTEPS);
@@ -489,6 +481,12 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           const uint32_t a_s = st, b_s = st + C2_A_BYTES;
           const uint32_t t_sfa = tmem_sf + s * C2_SF_COLS;
           const uint32_t t_sfb = t_sfa + KSTEPS * 4;
+          const uint32_t sfa_s = b_s + C2_B_BYTES, sfb_s = sfa_s + C2_SFA_BYTES;
+          for (int k = 0; k < nk; ++k) {
+            tc_cp_sf_pair(t_sfa + k * 4, smem_desc(sfa_s + k * ATOM, 128, LAYOUT_NONE));
+            tc_cp_sf_pair(t_sfb + k * 8, smem_desc(sfb_s + k * ATOM, 128, LAYOUT_NONE));
+            tc_cp_sf_pair(t_sfb + k * 8 + 4, smem_desc(sfb_s + (KSTEPS + k) * ATOM, 128, LAYOUT_NONE));
+          }
           for (int k = 0; k < nk; ++k) {
             const uint64_t adesc = smem_desc(a_s + k * 32, 1024, LAYOUT_SW128);
             const uint64_t bdesc = smem_desc(b_s + k * 32, 1024, LAYOUT_SW128);
@@ -500,14 +498,14 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         ++tile_it;
       }
     }
-  } else if (warp >= 8) {
+  } else {
     // ------------------------------------------------------------------ epilogue (both CTAs)
     // Two warps per tensor-memory quadrant, each with half of the columns: [128 half, 128 half + 128), with SwiGLU gate
     // columns [64 half, 64 half + 64) and the up columns that belong to them.
     // (One warp per quadrant, with all 256 columns and SiLU from a table in L2, was busy for longer than a tile's MMAs:
     // SwiGLU [28672, 4224], us, before / eight warps and the table / eight warps and silu_for_bf16: 333 rows 55 / 52 / 49,
     // 2048 rows 147 / 142 / 137, 16384 rows 1057 / 1035 / 978.  The other epilogues are hidden either way.)
-    const int quad = warp & 3, ew = warp - 8, half = ew >> 2;
+    const int quad = warp & 3, ew = warp - 2, half = ew >> 2;
     float alpha = p.alpha;
     if (p.tile_group == nullptr) {
       if (p.alpha_a) alpha *= __ldg(p.alpha_a);
@@ -585,7 +583,7 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         // (32 rows x 128 bytes, 128-byte swizzle: lane = row, 16-byte chunk c of row r sits at chunk
         // c ^ (r & 7), so a warp's 128-bit stores are conflict free), one after the other from the
         // warp's 4 KB of staging.  The bulk stores write whole 128-byte lines, clip rows >= M and
-        // columns >= N themselves, and keep the load/store pipe free for the scale warps.
+        // columns >= N themselves.
         const int row0 = tm * 256 + (int)rank * 128 + quad * 32;
         const uint32_t slot = cstage_base + (uint32_t)ew * 4096u;
         const CUtensorMap* map_c = &maps_c.m[0];
@@ -653,52 +651,6 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     // the last boxes must have left shared memory (and reached global memory) before the CTA goes
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     __syncwarp();
-  } else if (warp >= 4) {
-    // ------------------------------------------------------------------ scale warps (both CTAs)
-    // Warp q writes TMEM lanes 32q..32q+31.  An atom is 32 rows x 16 bytes: lane l's 16 bytes are
-    // its four TMEM columns (rows l, l+32, l+64, l+96 of the 128-row tile, four K blocks each);
-    // every quadrant holds the same copy.
-    const int quad = warp & 3;
-    uint32_t it = 0;
-    bool ok = true;
-    for (int tile = cluster_id; tile < num_tiles && ok; tile += num_clusters) {
-      if (p.tile_group != nullptr) {
-        int tm, tn;
-        pair_tile_coords(tile, p, tm, tn);
-        if (__ldg(p.tile_group + tm) < 0) continue;
-      }
-      for (int ks = 0; ks < kstages; ++ks, ++it) {
-        const int s = it % C2_STAGES;
-        const uint32_t ph = (it / C2_STAGES) & 1u;
-        ok = mbar_wait(sf_full_bar(s), ph, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        const uint4* sf = reinterpret_cast<const uint4*>(base_ptr + s * C2_STAGE_BYTES + C2_A_BYTES + C2_B_BYTES);
-        const uint32_t taddr = tmem_sf + s * C2_SF_COLS + ((uint32_t)(quad * 32) << 16);
-        // TMEM columns: [SFA k0..k3 (4 each)] [SFB k0: tile0, tile1][k1: ...] ...
-        // shared:       [SFA k0..k3][SFB tile0 k0..k3][SFB tile1 k0..k3], 512 bytes each
-#pragma unroll
-        for (int part = 0; part < 3; ++part) {
-          uint32_t r[16];
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            int atom;
-            if (part == 0) atom = j;                                        // SFA k = j
-            else {
-              const int k = (part - 1) * 2 + (j >> 1), t = j & 1;           // SFB k, tile t
-              atom = KSTEPS + t * KSTEPS + k;
-            }
-            const uint4 v = sf[atom * 32 + lane];
-            r[4 * j + 0] = v.x; r[4 * j + 1] = v.y; r[4 * j + 2] = v.z; r[4 * j + 3] = v.w;
-          }
-          tc_st16(taddr + part * 16, r);
-        }
-        tc_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive_leader(sf_ready_bar(s));
-      }
-    }
   }
 
   // Neither CTA may leave (or give back tensor memory) while the other can still touch it.

@@ -15,9 +15,8 @@
 //  * Programmatic dependent launch: while the kernel before is still running, every CTA pulls its first weight tiles
 //    into L2 (a prefetch reads nothing into the CTA, so a weight still being written is not read early).
 //
-// Roles: warp 0 producer (TMA), warp 1 MMA issuer, warps 2-5 epilogue, warps 6-9 scale warps (shared memory -> tensor
-// memory with tcgen05.st, as in arcq_gemm.cu; with tcgen05.cp in the issuing thread a stage took 1190 cycles, more than
-// its bytes need at HBM rate).
+// Roles: warp 0 producer (TMA), warp 1 issuer of the scale copies (tcgen05.cp) and MMAs, warps 2-5 epilogue; warps 6-9 help
+// to add the partial sums.
 #include "arcq_tc.cuh"
 
 namespace arcq {
@@ -122,9 +121,8 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   volatile int* abort_flag = reinterpret_cast<volatile int*>(misc + 1);
   auto full_bar = [&](int s) { return bar_base + 8u * s; };
   auto empty_bar = [&](int s) { return bar_base + 8u * (C::STAGES + s); };
-  auto sf_bar = [&](int s) { return bar_base + 8u * (2 * C::STAGES + s); };       // scale atoms landed
-  const uint32_t acc_full_bar = bar_base + 8u * (3 * C::STAGES), acc_empty_bar = acc_full_bar + 8u;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t acc_full_bar = bar_base + 8u * (2 * C::STAGES), acc_empty_bar = acc_full_bar + 8u;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
 
   const int ttiles = NT > 64 ? p.ttiles : 1;           // (a constant up to 64 rows: four divisions less before the first load)
   const int kstages = (p.ksteps_total + KSTEPS - 1) / KSTEPS;
@@ -140,9 +138,8 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) {
-      mbar_init(full_bar(s), 1 + 4);       // the codes' bytes, and the four scale warps
+      mbar_init(full_bar(s), 1);
       mbar_init(empty_bar(s), 1);
-      mbar_init(sf_bar(s), 1);
     }
     mbar_init(acc_full_bar, 1);
     mbar_init(acc_empty_bar, 4);
@@ -226,7 +223,7 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (int item = first_item; item < num_items && ok; item += item_step) {
@@ -241,10 +238,9 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             if (!mbar_wait(empty_bar(s), ((it / C::STAGES) & 1u) ^ 1u, abort_flag)) { ok = false; break; }
             const uint32_t sf_bytes = (uint32_t)min(KSTEPS, p.ksteps_total - ks * KSTEPS) * ATOM;
             const uint32_t st = base + s * C::STAGE_BYTES, x_s = st + SK_W_BYTES, sfw_s = x_s + C::X_BYTES, sfx_s = sfw_s + SK_SF_BYTES;
-            mbar_expect_tx(sf_bar(s), 2u * sf_bytes);
-            mbar_expect_tx(full_bar(s), SK_W_BYTES + (uint32_t)(boxes * C::XBOX * BK_BYTES));
-            bulk_load(sfw_s, p.sfw + ((size_t)wt * p.natoms + (size_t)ks * KSTEPS) * ATOM, sf_bytes, sf_bar(s));
-            bulk_load(sfx_s, p.sfx + ((size_t)xt * p.natoms + (size_t)ks * KSTEPS) * ATOM, sf_bytes, sf_bar(s));
+            mbar_expect_tx(full_bar(s), SK_W_BYTES + (uint32_t)(boxes * C::XBOX * BK_BYTES) + 2u * sf_bytes);
+            bulk_load(sfw_s, p.sfw + ((size_t)wt * p.natoms + (size_t)ks * KSTEPS) * ATOM, sf_bytes, full_bar(s));
+            bulk_load(sfx_s, p.sfx + ((size_t)xt * p.natoms + (size_t)ks * KSTEPS) * ATOM, sf_bytes, full_bar(s));
             tma_load_2d(st, &map_w, full_bar(s), ks * BK_BYTES, wrow);
             for (int b = 0; b < boxes; ++b) tma_load_2d(x_s + b * (C::XBOX * BK_BYTES), &map_x, full_bar(s), ks * BK_BYTES, row0 + C::XBOX * b);
           }
@@ -255,13 +251,12 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
         // shared memory after the CTA has gone
         const unsigned long long t0 = globaltimer_ns();
         for (uint32_t j = it > (uint32_t)C::STAGES ? it - C::STAGES : 0; j < it; ++j)
-          while (!(mbar_try_wait(full_bar(j % C::STAGES), (j / C::STAGES) & 1u) && mbar_try_wait(sf_bar(j % C::STAGES), (j / C::STAGES) & 1u)) &&
-                 globaltimer_ns() - t0 < WAIT_LIMIT_NS) {}
+          while (!mbar_try_wait(full_bar(j % C::STAGES), (j / C::STAGES) & 1u) && globaltimer_ns() - t0 < WAIT_LIMIT_NS) {}
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0, acc_it = 0;
       bool ok = true;
       for (int item = first_item; item < num_items && ok; item += item_step, ++acc_it) {
@@ -279,17 +274,28 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             tc_fence_after();
             const int nk = min(KSTEPS, p.ksteps_total - ks * KSTEPS);
             const uint32_t st = base + s * C::STAGE_BYTES;
-            const uint32_t t_sfw = tmem_sf + s * SK_SF_COLS, t_sfx = t_sfw + KSTEPS * 4;
+            // Scales: shared -> tensor memory, in front of the MMAs (the pipe keeps the order of copies and MMAs that one
+            // thread issues; the MMAs that read the stage's old columns are complete, its producer waited for them).
+            // `upper`: rows 64.. of a 128-row scale tile are words 2 and 3 of its atoms.
+            const uint32_t t_sfw = tmem_sf + s * SK_SF_COLS, t_cpx = t_sfw + KSTEPS * 4, t_sfx = t_cpx + ((row0 & 64) ? 2u : 0u);
             const uint64_t wd = smem_desc(st, 1024, LAYOUT_SW128), xd = smem_desc(st + SK_W_BYTES, 1024, LAYOUT_SW128);
+            const uint64_t sd = smem_desc(st + SK_W_BYTES + C::X_BYTES, 128, LAYOUT_NONE);   // (descriptors count 16-byte units)
+            auto copy_scales = [&](int k) {
+              tc_cp_sf(t_sfw + k * 4, sd + k * (ATOM / 16));
+              tc_cp_sf(t_cpx + k * 4, sd + (KSTEPS + k) * (ATOM / 16));
+            };
+            auto multiply = [&](int k) {
+              tc_mma_nvf4(tmem_base + ai * NT, wd + 2 * k, xd + 2 * k, idesc, t_sfw + k * 4, t_sfx + k * 4,
+                          (ks > ks_begin || k > 0) ? 1u : 0u);
+            };
             if (nk == KSTEPS) {
 #pragma unroll
-              for (int k = 0; k < KSTEPS; ++k)
-                tc_mma_nvf4(tmem_base + ai * NT, wd + 2 * k, xd + 2 * k, idesc, t_sfw + k * 4, t_sfx + k * 4,
-                            (ks > ks_begin || k > 0) ? 1u : 0u);
+              for (int k = 0; k < KSTEPS; ++k) copy_scales(k);
+#pragma unroll
+              for (int k = 0; k < KSTEPS; ++k) multiply(k);
             } else {
-              for (int k = 0; k < nk; ++k)
-                tc_mma_nvf4(tmem_base + ai * NT, wd + 2 * k, xd + 2 * k, idesc, t_sfw + k * 4, t_sfx + k * 4,
-                            (ks > ks_begin || k > 0) ? 1u : 0u);
+              for (int k = 0; k < nk; ++k) copy_scales(k);
+              for (int k = 0; k < nk; ++k) multiply(k);
             }
             tc_commit(empty_bar(s));
           }
@@ -418,41 +424,6 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(acc_empty_bar);
-    }
-  } else {
-    // ------------------------------------------------------------------ scale warps (6..9)
-    // Warp q writes TMEM lanes 32q..32q+31: lane l's 16 bytes of an atom are its four columns (see arcq_gemm.cu).
-    const int quad = warp & 3;
-    uint32_t it = 0;
-    bool ok = true;
-    for (int item = first_item; item < num_items && ok; item += item_step) {
-      int g, t, row0, cnt;
-      locate(item, g, t, row0, cnt);
-      const bool upper = (row0 & 64) != 0;                 // rows 64.. of a 128-row scale tile: words 2 and 3 of the atoms
-      for (int n = NA * (ks_end - ks_begin); n > 0; --n, ++it) {
-        const int s = it % C::STAGES;
-        ok = mbar_wait(sf_bar(s), (it / C::STAGES) & 1u, abort_flag);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-        // (the MMAs that read the stage's old scale columns are complete: its producer waited for them)
-        const uint4* sf = reinterpret_cast<const uint4*>(base_ptr + s * C::STAGE_BYTES + SK_W_BYTES + C::X_BYTES);
-        const uint32_t taddr = tmem_sf + s * SK_SF_COLS + ((uint32_t)(quad * 32) << 16);
-#pragma unroll
-        for (int side = 0; side < 2; ++side) {
-          uint32_t r[16];
-#pragma unroll
-          for (int k = 0; k < KSTEPS; ++k) {
-            uint4 v = sf[(side * KSTEPS + k) * 32 + lane];
-            if (side == 1 && upper) { v.x = v.z; v.y = v.w; }
-            r[4 * k] = v.x; r[4 * k + 1] = v.y; r[4 * k + 2] = v.z; r[4 * k + 3] = v.w;
-          }
-          tc_st16(taddr + side * (KSTEPS * 4), r);
-        }
-        tc_wait_st();
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(full_bar(s));
-      }
     }
   }
 

@@ -26,15 +26,6 @@ __device__ int g_tc_error = 0;     // sticky until polled
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
-// One thread of a converged warp, the same on every call.  A role that starts copies or MMAs is entered through this and
-// not through `lane == 0`: of elect.sync the compiler knows that a single thread is active and issues those instructions
-// directly; behind a comparison it wraps each in a loop over the active threads.  Measured (cycles): a tcgen05.cp 81 -> 27,
-// a TMA load about 65 -> 20.
-__device__ __forceinline__ bool elect_one() {
-  uint32_t p;
-  asm volatile("{\n.reg .pred P;\nelect.sync _|P, 0xffffffff;\nselp.u32 %0, 1, 0, P;\n}" : "=r"(p));
-  return p != 0;
-}
 __device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }   // uniform
 __device__ __forceinline__ unsigned long long globaltimer_ns() {
   unsigned long long t;

@@ -860,7 +860,7 @@ arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const
     bulk_load(dst, in_row(r0) + hoff, hbytes, bar);
     if (has1) bulk_load(dst + hbytes, in_row(r0 + 1) + hoff, hbytes, bar);
   };
-  if (tid == 0) {
+  if (tid < 32 && elect_one()) {
     for (int s = 0; s < S; ++s) {
       mbar_init(full0 + 8 * s, (uint32_t)(npt >> 5));    // one arrival per producer warp
       mbar_init(empty0 + 8 * s, (uint32_t)(nct >> 5));   // one arrival per warp of the consuming team
@@ -942,7 +942,7 @@ arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const
             mbar_arrive(rsr + 8 * (m & 1u));
           }
         }
-      } else if (lane == 0) {
+      } else if (XR ? elect_one() : lane == 0) {
         // -------------------------------------------------------------- loader
         uint32_t next = (uint32_t)pteam;    // first pair of this team whose copies are not started yet
         while (next < n && next < (uint32_t)R) next += NP;   // (the first R pairs were started in the prologue)
@@ -1052,10 +1052,7 @@ arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const
       if (lane == 0) mbar_arrive(full0 + 8 * s);
     };
 
-    // Copies in flight are tracked by pair number (this team's pairs: pteam, pteam + NP, ...):
-    uint32_t issued = (uint32_t)pteam;   // first pair of this team whose copies were NOT started yet
-    while (issued < n && issued < (uint32_t)R) issued += NP;
-    uint32_t landed = (uint32_t)pteam;   // first pair of this team whose copies were not waited for yet
+    uint32_t at = 0, issued = 0;   // plain operator, after a failure: the (half) pair it happened at, the first one not started
     bool failed = false;
     if (!RMS && WIDE) {
       const int hc = KQ >> 4;   // 16-byte chunks of half a row
@@ -1067,14 +1064,11 @@ arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const
         fast = div_by_reciprocal_ok(sc);
       }
       const uint32_t nu = 2 * n;
-      issued = nu < (uint32_t)R ? nu : (uint32_t)R;
-      landed = 0;
       for (uint32_t u = 0; u < nu; ++u) {
         const uint32_t it = u >> 1, h = u & 1u;
         const uint32_t unit = cta + it * stride;
         const bool has1 = (2 * unit + 1) < rows;
         if (!failed && !mbar_wait(raw0 + 8 * (u % R), (u / R) & 1u, abort_flag)) failed = true;
-        if (!failed) landed = u + 1;
         if (h == 0 && !failed && !mbar_wait(empty0 + 8 * (it % S), ((it / S) & 1u) ^ 1u, abort_flag)) failed = true;
         if (!failed) {
           const uint4* rw = reinterpret_cast<const uint4*>(raw + (size_t)(u % R) * row_in_bytes);
@@ -1105,8 +1099,8 @@ arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const
           }
         }
         // every producer is done with this half stage: refill it, or leave together
-        if (named_barrier_or(bar_id, team_threads, failed)) break;
-        if (ptid == 0 && u + R < nu) { issue_half(u + R, u % R); issued = u + R + 1; }
+        if (named_barrier_or(bar_id, team_threads, failed)) { failed = true; at = u; issued = min(nu, u + R); break; }
+        if (ptid == 0 && u + R < nu) issue_half(u + R, u % R);
       }
     } else if (!RMS) {
       const int nchunks = KQ >> 3;
@@ -1122,7 +1116,6 @@ arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const
         const uint32_t unit = cta + it * stride;
         const bool has1 = (2 * unit + 1) < rows;
         if (!failed && !mbar_wait(raw0 + 8 * (it % R), (it / R) & 1u, abort_flag)) failed = true;
-        if (!failed) landed = it + 1;
         if (!failed && !mbar_wait(empty0 + 8 * (it % S), ((it / S) & 1u) ^ 1u, abort_flag)) failed = true;
         if (!failed) {
           // this thread's chunks c = ptid, ptid + npt, ...: interleave the two rows (dividing by the
@@ -1159,8 +1152,8 @@ arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const
         }
         // Producers meet once per pair: every one of them is done with the raw stage, so it is
         // refilled; and all leave together if any wait gave up.
-        if (named_barrier_or(bar_id, team_threads, failed)) break;
-        if (ptid == 0 && it + R < n) { issue(unit + R * stride, it % R); issued = it + R + 1; }
+        if (named_barrier_or(bar_id, team_threads, failed)) { failed = true; at = it; issued = min(n, it + R); break; }
+        if (ptid < 32 && it + R < n && elect_one()) issue(unit + R * stride, it % R);
       }
     } else {
       // Software pipeline, synchronised by mbarriers only: normalise and hand over this team's pair
@@ -1207,7 +1200,7 @@ arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const
     // Giving up with bulk copies possibly in flight: wait (bounded) for those this CTA started, so that
     // none lands in shared memory after the CTA has gone.
     if (!RMS && failed && ptid == 0) {
-      for (uint32_t j = landed; j < issued; j += NP) {
+      for (uint32_t j = at; j < issued; ++j) {
         unsigned long long t0, t1;
         asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
         while (!mbar_try_wait(raw0 + 8 * (j % R), (j / R) & 1u)) {

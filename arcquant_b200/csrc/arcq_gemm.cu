@@ -95,7 +95,7 @@ arcq_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   const uint32_t tmem_full_bar = bar_base + 8u * (2 * C::STAGES);
   const uint32_t tmem_empty_bar = tmem_full_bar + 8u;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < C::STAGES; ++s) { mbar_init(full_bar(s), 1); mbar_init(empty_bar(s), 1); }
@@ -121,7 +121,7 @@ arcq_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
@@ -155,7 +155,7 @@ arcq_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc = instr_desc<BN>();
       uint32_t it = 0, tile_it = 0;
       bool ok = true;
@@ -172,24 +172,27 @@ arcq_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           const uint32_t ph = (it / C::STAGES) & 1u;
           if (!mbar_wait(full_bar(s), ph, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          const int nk = min(KSTEPS, p.ksteps_total - ks * KSTEPS);
+          const uint32_t t_sfa = tmem_sf + (it & 1u) * C::SF_COLS, t_sfb = t_sfa + KSTEPS * 4;
           const uint32_t st = base + s * C::STAGE_BYTES;
-          const uint32_t a_s = st, b_s = st + C::A_BYTES;
-          const uint32_t sfa_s = b_s + C::B_BYTES, sfb_s = sfa_s + C::SFA_BYTES;
-          const uint32_t t_sfa = tmem_sf + (it & 1u) * C::SF_COLS;
-          const uint32_t t_sfb = t_sfa + KSTEPS * 4;
-          for (int k = 0; k < nk; ++k) {
-            tc_cp_sf(t_sfa + k * 4, smem_desc(sfa_s + k * ATOM, 128, LAYOUT_NONE));
+          const uint64_t ad = smem_desc(st, 1024, LAYOUT_SW128), bd = smem_desc(st + C::A_BYTES, 1024, LAYOUT_SW128);
+          const uint64_t sd = smem_desc(st + C::A_BYTES + C::B_BYTES, 128, LAYOUT_NONE);   // (descriptors count 16-byte units)
+          auto copy_scales = [&](int k) {
+            tc_cp_sf(t_sfa + k * 4, sd + k * (ATOM / 16));
 #pragma unroll
-            for (int a = 0; a < C::NB; ++a)
-              tc_cp_sf(t_sfb + k * 4 * C::NB + a * 4,
-                       smem_desc(sfb_s + a * (KSTEPS * ATOM) + k * ATOM, 128, LAYOUT_NONE));
-          }
-          for (int k = 0; k < nk; ++k) {
-            const uint64_t adesc = smem_desc(a_s + k * 32, 1024, LAYOUT_SW128);
-            const uint64_t bdesc = smem_desc(b_s + k * 32, 1024, LAYOUT_SW128);
-            tc_mma_nvf4(tmem_base, adesc, bdesc, idesc, t_sfa + k * 4, t_sfb + k * 4 * C::NB + sfb_sub,
-                        (ks | k) ? 1u : 0u);
+            for (int a = 0; a < C::NB; ++a) tc_cp_sf(t_sfb + k * 4 * C::NB + a * 4, sd + ((1 + a) * KSTEPS + k) * (ATOM / 16));
+          };
+          auto multiply = [&](int k) {
+            tc_mma_nvf4(tmem_base, ad + 2 * k, bd + 2 * k, idesc, t_sfa + k * 4, t_sfb + k * 4 * C::NB + sfb_sub, (ks | k) ? 1u : 0u);
+          };
+          const int nk = p.ksteps_total - ks * KSTEPS;
+          if (nk >= KSTEPS) {
+#pragma unroll
+            for (int k = 0; k < KSTEPS; ++k) copy_scales(k);
+#pragma unroll
+            for (int k = 0; k < KSTEPS; ++k) multiply(k);
+          } else {
+            for (int k = 0; k < nk; ++k) copy_scales(k);
+            for (int k = 0; k < nk; ++k) multiply(k);
           }
           tc_commit(empty_bar(s));   // stage reusable once these MMAs have read it
         }
@@ -476,21 +479,27 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           const uint32_t ph = (it / C2_STAGES) & 1u;
           if (!mbar_wait(full_bar(s), ph, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          const int nk = min(KSTEPS, p.ksteps_total - ks * KSTEPS);
+          const uint32_t t_sfa = tmem_sf + s * C2_SF_COLS, t_sfb = t_sfa + KSTEPS * 4;
           const uint32_t st = base + s * C2_STAGE_BYTES;
-          const uint32_t a_s = st, b_s = st + C2_A_BYTES;
-          const uint32_t t_sfa = tmem_sf + s * C2_SF_COLS;
-          const uint32_t t_sfb = t_sfa + KSTEPS * 4;
-          const uint32_t sfa_s = b_s + C2_B_BYTES, sfb_s = sfa_s + C2_SFA_BYTES;
-          for (int k = 0; k < nk; ++k) {
-            tc_cp_sf_pair(t_sfa + k * 4, smem_desc(sfa_s + k * ATOM, 128, LAYOUT_NONE));
-            tc_cp_sf_pair(t_sfb + k * 8, smem_desc(sfb_s + k * ATOM, 128, LAYOUT_NONE));
-            tc_cp_sf_pair(t_sfb + k * 8 + 4, smem_desc(sfb_s + (KSTEPS + k) * ATOM, 128, LAYOUT_NONE));
-          }
-          for (int k = 0; k < nk; ++k) {
-            const uint64_t adesc = smem_desc(a_s + k * 32, 1024, LAYOUT_SW128);
-            const uint64_t bdesc = smem_desc(b_s + k * 32, 1024, LAYOUT_SW128);
-            tc_mma_nvf4_pair(tmem_base, adesc, bdesc, idesc, t_sfa + k * 4, t_sfb + k * 8, (ks | k) ? 1u : 0u);
+          const uint64_t ad = smem_desc(st, 1024, LAYOUT_SW128), bd = smem_desc(st + C2_A_BYTES, 1024, LAYOUT_SW128);
+          const uint64_t sd = smem_desc(st + C2_A_BYTES + C2_B_BYTES, 128, LAYOUT_NONE);   // (descriptors count 16-byte units)
+          auto copy_scales = [&](int k) {
+            tc_cp_sf_pair(t_sfa + k * 4, sd + k * (ATOM / 16));
+            tc_cp_sf_pair(t_sfb + k * 8, sd + (KSTEPS + k) * (ATOM / 16));
+            tc_cp_sf_pair(t_sfb + k * 8 + 4, sd + (2 * KSTEPS + k) * (ATOM / 16));
+          };
+          auto multiply = [&](int k) {
+            tc_mma_nvf4_pair(tmem_base, ad + 2 * k, bd + 2 * k, idesc, t_sfa + k * 4, t_sfb + k * 8, (ks | k) ? 1u : 0u);
+          };
+          const int nk = p.ksteps_total - ks * KSTEPS;
+          if (nk >= KSTEPS) {        // (unrolled: sixteen instructions have to leave in less than the MMAs' 512 cycles)
+#pragma unroll
+            for (int k = 0; k < KSTEPS; ++k) copy_scales(k);
+#pragma unroll
+            for (int k = 0; k < KSTEPS; ++k) multiply(k);
+          } else {
+            for (int k = 0; k < nk; ++k) copy_scales(k);
+            for (int k = 0; k < nk; ++k) multiply(k);
           }
           tc_commit_pair(empty_bar(s));
         }

@@ -472,8 +472,6 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           pair_tile_coords(tile, p, tm, tn);
           if (__ldg(p.tile_group + tm) < 0) continue;      // a tile without rows: every role skips it
         }
-        if (!mbar_wait(tmem_empty_bar, (tile_it & 1u) ^ 1u, abort_flag)) { ok = false; break; }
-        tc_fence_after();
         for (int ks = 0; ks < kstages; ++ks, ++it) {
           const int s = it % C2_STAGES;
           const uint32_t ph = (it / C2_STAGES) & 1u;
@@ -491,14 +489,23 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
           auto multiply = [&](int k) {
             tc_mma_nvf4_pair(tmem_base, ad + 2 * k, bd + 2 * k, idesc, t_sfa + k * 4, t_sfb + k * 8, (ks | k) ? 1u : 0u);
           };
+          // (the scales do not wait for the accumulator)
+          auto accumulator_free = [&]() {
+            if (ks != 0) return true;
+            if (!mbar_wait(tmem_empty_bar, (tile_it & 1u) ^ 1u, abort_flag)) return false;
+            tc_fence_after();
+            return true;
+          };
           const int nk = p.ksteps_total - ks * KSTEPS;
           if (nk >= KSTEPS) {        // (unrolled: sixteen instructions have to leave in less than the MMAs' 512 cycles)
 #pragma unroll
             for (int k = 0; k < KSTEPS; ++k) copy_scales(k);
+            if (!accumulator_free()) { ok = false; break; }
 #pragma unroll
             for (int k = 0; k < KSTEPS; ++k) multiply(k);
           } else {
             for (int k = 0; k < nk; ++k) copy_scales(k);
+            if (!accumulator_free()) { ok = false; break; }
             for (int k = 0; k < nk; ++k) multiply(k);
           }
           tc_commit_pair(empty_bar(s));
@@ -547,25 +554,26 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       if (!ok) break;
       tc_fence_after();
       const int row = tm * 256 + (int)rank * 128 + quad * 32 + lane;
-      // Drain the accumulator into registers as packed bf16 (64 registers for this thread's 128 columns) and hand tensor
-      // memory back at once: the stores below then overlap the next tile's MMAs.
+      // Drain the accumulator into registers (128 columns per thread) and hand tensor memory back before anything is done
+      // with it: scaling, rounding and the stores then overlap the next tile's MMAs.
       uint32_t o[64];
+      {
+        uint32_t r[4][32];
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const uint32_t col = SWIGLU ? (uint32_t)(128 * c + 64 * half) : (uint32_t)(128 * half + 64 * c);
-        uint32_t r0[32], r1[32];
-        tc_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + col, r0);
-        tc_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + col + 32u, r1);
-        tc_wait_ld();
-#pragma unroll
-        for (int v = 0; v < 16; ++v) {
-          o[32 * c + v] = pack_bf16x2(__uint_as_float(r0[2 * v]) * alpha, __uint_as_float(r0[2 * v + 1]) * alpha);
-          o[32 * c + 16 + v] = pack_bf16x2(__uint_as_float(r1[2 * v]) * alpha, __uint_as_float(r1[2 * v + 1]) * alpha);
+        for (int c = 0; c < 4; ++c) {
+          const uint32_t col = SWIGLU ? (uint32_t)(128 * (c >> 1) + 64 * half + 32 * (c & 1)) : (uint32_t)(128 * half + 32 * c);
+          tc_ld32(tmem_base + ((uint32_t)(quad * 32) << 16) + col, r[c]);
         }
+        tc_wait_ld();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_leader(tmem_empty_bar);
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+          for (int v = 0; v < 16; ++v)
+            o[16 * c + v] = pack_bf16x2(__uint_as_float(r[c][2 * v]) * alpha, __uint_as_float(r[c][2 * v + 1]) * alpha);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_leader(tmem_empty_bar);
       if (SWIGLU) {
         // columns 0..127 of the tile are gate, 128..255 the matching up columns: out = silu(gate) * up in
         // the gate registers, and its maximum over the rows that hold data

@@ -113,6 +113,8 @@ arcq_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");   // (every thread: everything below reads or writes global memory)
   const uint32_t tmem_base = misc[0];
   const uint32_t tmem_sf = tmem_base + BN;   // two stage-parity buffers of SF_COLS columns each
 
@@ -423,6 +425,10 @@ arcq_gemm2_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
   __syncthreads();
   cluster_sync_all();                             // both CTAs' barriers exist before anyone signals them
   tc_fence_after();
+  // Programmatic dependent launch: what is above overlaps the end of the kernel before, everything below reads or writes
+  // global memory.
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const uint32_t tmem_base = misc[0];
   const uint32_t tmem_sf = tmem_base + 256;       // stage s: scale columns [256 + 48 s, 256 + 48 s + 48)
 
@@ -719,6 +725,24 @@ int make_c_map(CUtensorMap* map, const void* ptr, int64_t M, int64_t N) {
   return ARCQ_OK;
 }
 
+// Launch as a programmatic dependent of the kernel before: the grid may be set up while that one drains, and waits itself
+// (griddepcontrol.wait) before it touches global memory.
+template <typename... Params, typename... Args>
+int launch_dependent(void (*kern)(Params...), unsigned grid, unsigned threads, size_t smem, cudaStream_t stream, const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, args...));
+  return ARCQ_OK;
+}
+
 // ngroups > 1: B and SFB hold `ngroups` matrices of N rows each, tile_group says which one every
 // 256-row tile of A multiplies (see Gemm2Params).
 // swiglu_amax != nullptr: SwiGLU epilogue (see Gemm2Params), C is [M, N/2]; groups: the run table of a grouped
@@ -786,9 +810,7 @@ int launch_pair(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const ui
   long long tiles = (long long)p.tiles_m * p.tiles_n;
   long long clusters = num_sms / 2;
   if (clusters > tiles) clusters = tiles;
-  kern<<<(unsigned)(2 * clusters), C2_THREADS, C2_SMEM_BYTES, stream>>>(ma, mb, msa, msb, mc, p, mr);
-  ARCQ_CUDA_TRY(cudaGetLastError());
-  return ARCQ_OK;
+  return launch_dependent(kern, (unsigned)(2 * clusters), C2_THREADS, C2_SMEM_BYTES, stream, ma, mb, msa, msb, mc, p, mr);
 }
 
 template <int BN>
@@ -799,9 +821,7 @@ int launch_bn(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int nu
   p.tiles_n = (p.N + BN - 1) / BN;
   long long tiles = (long long)p.tiles_m * p.tiles_n;
   int grid = (int)(tiles < num_sms ? tiles : num_sms);
-  kern<<<grid, NUM_THREADS, C::SMEM_BYTES, stream>>>(ma, mb, p);
-  ARCQ_CUDA_TRY(cudaGetLastError());
-  return ARCQ_OK;
+  return launch_dependent(kern, (unsigned)grid, NUM_THREADS, C::SMEM_BYTES, stream, ma, mb, p);
 }
 
 }  // namespace

@@ -55,6 +55,7 @@ SIGNATURES = {
     "arcq_rope_bf16": (_i32, [_vp, _vp, _vp, _i64, _i32, _i32, _i32, _i32, _vp]),
     "arcq_silu_mul_bf16": (_i32, [_vp, _vp, _i64, _i32, _vp, _vp]),
     "arcq_calib_stats_bf16": (_i32, [_vp, _i64, _i32, _vp, _vp, _vp]),
+    "arcq_channel_order": (_i32, [_vp, _i32, _vp, _vp]),
     "arcq_route_topk_bf16": (_i32, [_vp, _i64, _i32, _i32, _vp, _vp, _vp]),
     "arcq_moe_layout": (_i32, [_vp, _i32, _i32, _i32, _i32, _i32, _vp, _vp, _vp, _vp, _vp]),
     "arcq_silu_mul_grouped_bf16": (_i32, [_vp, _vp, _i64, _i32, _vp, _vp, _i32, _vp, _vp]),

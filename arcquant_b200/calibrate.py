@@ -59,6 +59,11 @@ class ChannelAbsMax:
             raise RuntimeError("no batch seen")
         if self.value.numel() > 32752:
             raise ValueError("more channels than an int16 order can hold")
+        # (its work grows with the square of the width, us against torch's sort: 4096 8.6 / 45.7, 8192 16 / 63, 14 336 50 / 62,
+        # 28 672 167 / 67)
+        if (self.value.is_cuda and self.value.dtype == torch.float32 and self.value.dim() == 1 and self.value.is_contiguous()
+                and 0 < self.value.numel() <= 14336):
+            return ops.channel_order(self.value)
         return torch.argsort(self.value).to(torch.int16)
 
     def select_num(self, granule: int = 64) -> int:

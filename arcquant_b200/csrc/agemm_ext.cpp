@@ -251,6 +251,17 @@ void calib_stats(const torch::Tensor& X, const torch::Tensor& chan_absmax, const
                "calib_stats");
 }
 
+// Channels by ascending statistic; see arcq_channel_order.
+torch::Tensor channel_order(const torch::Tensor& value) {
+  require_on(value, value, at::kFloat, "value");
+  c10::cuda::CUDAGuard guard(value.device());
+  auto order = torch::empty({value.numel()}, value.options().dtype(torch::kInt16));
+  if (value.numel() == 0) return order;
+  check_status(arcq_channel_order(value.data_ptr<float>(), static_cast<int>(value.numel()), order.data_ptr<int16_t>(), current_stream(value)),
+               "channel_order");
+  return order;
+}
+
 std::tuple<torch::Tensor, torch::Tensor> silu_mul(const torch::Tensor& GU) {
   require_cuda(GU, "gate_up");
   TORCH_CHECK(GU.dim() == 2 && GU.size(1) % 16 == 0, "gate_up must be [tokens, 2F] with F a multiple of 8");
@@ -310,6 +321,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("quantize_tensor_scale", &quantize_tensor_scale, "(Q, SF, scale) of x or w over its per-tensor scale", py::arg("X"),
         py::arg("reorder_index"), py::arg("KE"), py::arg("mode") = -1, py::arg("is_weight") = false,
         py::arg("amax") = py::none());
+  m.def("channel_order", &channel_order, "channels by ascending statistic, int16", py::arg("value"));
   m.def("calib_stats", &calib_stats, "accumulate the calibration statistics of one batch", py::arg("X"),
         py::arg("chan_absmax"), py::arg("above") = py::none());
   m.def("silu_mul", &silu_mul, "(silu(gate) * up, max|.|) of [gate | up]", py::arg("gate_up"));

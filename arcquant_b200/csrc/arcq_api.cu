@@ -340,6 +340,13 @@ int arcq_calib_stats_bf16(const void* x, int64_t rows, int K, float* chan_absmax
   return launch_calib_stats(x, rows, K, chan_absmax, above, (cudaStream_t)stream);
 }
 
+int arcq_channel_order(const float* value, int K, int16_t* order, void* stream) {
+  if (K <= 0) return ARCQ_ERR_BAD_SHAPE;
+  if (K > 32768) return ARCQ_ERR_UNSUPPORTED_K;
+  if (!value || !order) return ARCQ_ERR_NULL_POINTER;
+  return launch_channel_order(value, K, order, (cudaStream_t)stream);
+}
+
 int arcq_route_topk_bf16(const void* logits, int64_t tokens, int experts, int top_k, int64_t* ids, void* weights, void* stream) {
   if (tokens < 0 || experts < 1 || experts > 32 || top_k < 1 || top_k > experts) return ARCQ_ERR_BAD_SHAPE;
   if (tokens == 0) return ARCQ_OK;

@@ -95,6 +95,7 @@ int launch_route_topk(const void* logits, int64_t tokens, int experts, int top_k
                       cudaStream_t stream);
 int launch_calib_stats(const void* x, int64_t rows, int K, float* chan_absmax, unsigned long long* above,
                        cudaStream_t stream);
+int launch_channel_order(const float* value, int K, int16_t* order, cudaStream_t stream);
 int launch_silu_mul_grouped(const void* gu, void* out, int64_t rows, int F, const int* tile_group, const int* groups,
                             int ngroups, float* amax, cudaStream_t stream);
 // GEMM whose result rows go to `ndests` buffers of M / ndests rows each (host array of device addresses; peers'

@@ -746,7 +746,64 @@ arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, u
   if constexpr (CLUSTER) cluster.sync();                       // nobody leaves while its maxima are being read
 }
 
+// Channel order of K statistics: ascending, equal values in order of their channels (a stable sort; NaN last).  A channel's
+// place is the number of channels before it, counted against all others: K^2 comparisons are 17 million at 4096 channels, a
+// microsecond or two of this chip's integer units, where a sort is a chain of dependent passes in a handful of CTAs.
+// A CTA serves 32 channels (lane = channel), its 32 warps a share of the keys each.  Bound: the comparisons; 4096 channels
+// 8.6 us where torch's argsort and its conversion to int16 take 45.7 (with eight warps per CTA: 12.7).
+constexpr int ORDER_THREADS = 1024, ORDER_BLOCK = 8192;
+__device__ __forceinline__ uint32_t order_key(float v) {      // unsigned order = order of the values; below 2^32 - 1
+  if (v != v) return 0xfffffffeu;
+  const uint32_t b = v == 0.f ? 0u : __float_as_uint(v);
+  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+__global__ void __launch_bounds__(ORDER_THREADS) arcq_channel_order_kernel(const float* __restrict__ value, int K, int16_t* __restrict__ order) {
+  __shared__ uint4 s_key[ORDER_BLOCK / 4];
+  __shared__ int s_place[32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int c = blockIdx.x * 32 + lane;
+  const uint32_t key = c < K ? order_key(__ldcg(value + c)) : 0u;
+  if (tid < 32) s_place[tid] = 0;
+  int before = 0;
+  for (int b0 = 0; b0 < K; b0 += ORDER_BLOCK) {
+    __syncthreads();                                          // (the block before is done with)
+    uint32_t* sk = reinterpret_cast<uint32_t*>(s_key);
+    const int here = min(ORDER_BLOCK, K - b0), vecs = (here + 3) >> 2;   // vectors of four keys
+    for (int j = tid; j < 4 * vecs; j += ORDER_THREADS) sk[j] = j < here ? order_key(__ldcg(value + b0 + j)) : 0xffffffffu;
+    __syncthreads();
+    // Keys of channels before c's group of four count where they are equal too: against them the bound is one higher.
+    const int own = (c - b0) >> 2;                            // (negative, or beyond the block: another block's)
+#pragma unroll 4
+    for (int at = warp; at < vecs; at += ORDER_THREADS / 32) {
+      const uint4 k4 = s_key[at];
+      const uint32_t bound = key + (at < own ? 1u : 0u);
+      before += (k4.x < bound) + (k4.y < bound) + (k4.z < bound) + (k4.w < bound);
+    }
+    if (warp == 0 && c >= b0 && c < b0 + here)                // equal keys among the group's own four
+      for (int j = 4 * own; j < c - b0; ++j) before += sk[j] == key;
+  }
+  atomicAdd(&s_place[lane], before);
+  __syncthreads();
+  if (tid < 32 && c < K) order[s_place[tid]] = (int16_t)c;
+}
+
 }  // namespace
+
+int launch_channel_order(const float* value, int K, int16_t* order, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((K + 31) / 32));
+  cfg.blockDim = dim3(ORDER_THREADS);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, arcq_channel_order_kernel, value, K, order));
+  return ARCQ_OK;
+}
 
 int launch_calib_stats(const void* x, int64_t rows, int K, float* chan_absmax, unsigned long long* above,
                        cudaStream_t stream) {

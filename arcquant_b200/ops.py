@@ -292,6 +292,20 @@ def calib_stats(x: torch.Tensor, chan_absmax: torch.Tensor, above: torch.Tensor 
     _lib.check(rc, "calib_stats")
 
 
+def channel_order(value: torch.Tensor) -> torch.Tensor:
+    """int16 [K]: channels by ascending fp32 statistic (CUDA), equal ones in order of their numbers, NaN last."""
+    _require(value, torch.float32, "value")
+    ext = _ext()
+    if ext:
+        return ext.channel_order(value)
+    order = torch.empty(value.numel(), dtype=torch.int16, device=value.device)
+    if value.numel() == 0:
+        return order
+    with torch.cuda.device(value.device):
+        _lib.check(_lib.load().arcq_channel_order(value.data_ptr(), value.numel(), order.data_ptr(), _stream()), "channel_order")
+    return order
+
+
 def route_topk(logits: torch.Tensor, top_k: int):
     """(ids int64 [T, k], weights bf16 [T, k]) of router logits bf16 [T, E], E <= 32, in one launch: fp32 softmax, top-k
     in descending order, weights renormalised over the selected experts."""

@@ -246,6 +246,10 @@ int arcq_moe_combine_bf16(const void* y, const int32_t* pos, const void* weights
 int arcq_calib_stats_bf16(const void* x, int64_t rows, int K, float* chan_absmax, unsigned long long* above,
                           void* stream);
 
+/* Channel order of a statistic: order[i] = channel of the i-th smallest of K values (device memory), equal values in
+ * order of their channels, NaN last - the reference's ascending argsort (utilize.py:42), K <= 32768. */
+int arcq_channel_order(const float* value, int K, int16_t* order, void* stream);
+
 /* ---- Grouped forms: all experts of a sparse MoE block in one launch ---------------------------------
  * The reference runs its experts one after another from Python, each with its own quantize and GEMM
  * calls on that expert's batch of tokens (model/qMixtralLayer.py:458-471, 524-543).  Here the routed

@@ -419,9 +419,9 @@ class QMixtralMoEBlockEP(torch.nn.Module):
         """All local experts in five launches: [rows_bound, hidden] in the padded layout of `batch`."""
         cfg, E = self.cfg, self.dispatcher.e_local
         ke = cfg.select_num
-        s1 = ops.absmax_grouped(batch.src, batch.row_map, batch.groups, E) / (448.0 * 6.0)   # per-expert scales
-        a, sfa = ops.reorder_quantize_x_grouped(batch.src, batch.row_map, s1, self.gu_index, batch.groups,
-                                                batch.rows_bound, ke)
+        amax1 = ops.absmax_grouped(batch.src, batch.row_map, batch.groups, E)
+        a, sfa, s1 = ops.quantize_grouped_amax(batch.src, batch.row_map, amax1, self.gu_index, batch.groups,
+                                               batch.rows_bound, ke)          # (s1: per-expert scales)
         if self.fuse_swiglu:        # SiLU * up and the per-expert maxima in the GEMM's epilogue
             act, amax2 = ops.matmul_grouped_swiglu(a, self.gu_W, sfa, self.gu_SF, batch.tile_group, batch.groups, E,
                                                    2 * cfg.ffn, s1, self.gu_scale)
@@ -432,8 +432,7 @@ class QMixtralMoEBlockEP(torch.nn.Module):
             else:
                 act, _ = ops.silu_mul(h, with_amax=False)
                 amax2 = ops.absmax_grouped(act, None, batch.groups, E)
-        s2 = amax2 / (448.0 * 6.0)
-        b, sfb = ops.reorder_quantize_x_grouped(act, None, s2, self.dn_index, batch.groups, batch.rows_bound, ke)
+        b, sfb, s2 = ops.quantize_grouped_amax(act, None, amax2, self.dn_index, batch.groups, batch.rows_bound, ke)
         return ops.matmul_grouped(b, self.dn_W, sfb, self.dn_SF, batch.tile_group, E, cfg.hidden, s2, self.dn_scale)
 
     n_streams = 4   # per-expert path: a few streams hide the launch gaps of the experts' small kernels

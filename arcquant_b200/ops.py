@@ -404,6 +404,39 @@ def reorder_quantize_x_grouped(x: torch.Tensor, row_map, scales: torch.Tensor, r
     return q, sf
 
 
+def quantize_grouped_amax(x: torch.Tensor, row_map, amax: torch.Tensor, reorder_indices: torch.Tensor, groups: torch.Tensor,
+                          rows_bound: int, ke: int, mode: int = 16):
+    """(codes, scales, scale fp32 [runs]): `reorder_quantize_x_grouped` over scale = amax / (448 * 6) of every run, taken
+    inside the quantizer."""
+    ngroups, kq = reorder_indices.shape
+    if ngroups > 64 or kq > 16384 or amax.numel() != ngroups:
+        scale = amax / (448.0 * 6.0)
+        return (*reorder_quantize_x_grouped(x, row_map, scale, reorder_indices, groups, rows_bound, ke, mode), scale)
+    lib = _lib.load()
+    _require(x, torch.bfloat16, "input")
+    _require(amax, torch.float32, "amax")
+    _require(reorder_indices, torch.int16, "reorder_indices")
+    _require(groups, torch.int32, "groups")
+    if x.shape[-1] != kq or groups.numel() != 2 * ngroups:
+        raise RuntimeError("reorder_indices / groups disagree on the number of runs or on KQ")
+    if row_map is not None:
+        _require(row_map, torch.int32, "row_map")
+        if row_map.numel() < rows_bound:
+            raise RuntimeError("row_map must cover rows_bound rows")
+    elif x.shape[0] < rows_bound:
+        raise RuntimeError("input has fewer rows than rows_bound")
+    k_eff = kq + ke
+    q = torch.empty((rows_bound, k_eff // 2), dtype=torch.uint8, device=x.device)
+    sf = torch.empty((sf_bytes(rows_bound, k_eff),), dtype=torch.uint8, device=x.device)
+    scale = torch.empty((ngroups,), dtype=torch.float32, device=x.device)
+    with torch.cuda.device(x.device):
+        rc = lib.arcq_quantize_x_grouped_amax(x.data_ptr(), None if row_map is None else row_map.data_ptr(), amax.data_ptr(),
+                                              reorder_indices.data_ptr(), groups.data_ptr(), ngroups, rows_bound, kq, ke, mode,
+                                              q.data_ptr(), sf.data_ptr(), scale.data_ptr(), _stream())
+    _lib.check(rc, f"grouped x-quantize KQ={kq} KE={ke}")
+    return q, sf, scale
+
+
 def matmul_grouped(a, b, sfa, sfb, tile_group: torch.Tensor, ngroups: int, n: int, alpha_a: torch.Tensor,
                    alpha_b: torch.Tensor | None = None) -> torch.Tensor:
     """bf16 [rows, n]: every 256-row tile m of A times the weight matrix tile_group[m] of the `ngroups`

@@ -85,7 +85,8 @@ int launch_gemm_grouped(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, 
                         int64_t N, int64_t K_eff, const int* tile_group, int ngroups, const float* alpha_a,
                         const float* alpha_b, void* C, cudaStream_t stream,
                         // SwiGLU epilogue: C is [M, N/2], swiglu_amax[ngroups] takes max|C| per matrix; tile_group
-                        // may be null with ngroups 1 (one matrix); groups: run table of a grouped problem
+                        // may be null with ngroups 1 (one matrix); groups: run table of a grouped problem (where
+                        // it is known, few rows per matrix take the weight-streaming kernel)
                         float* swiglu_amax = nullptr, const int* groups = nullptr);
 int launch_absmax_grouped(const void* x, const int* row_map, const int* groups, int ngroups, int K, float* out,
                           cudaStream_t stream);

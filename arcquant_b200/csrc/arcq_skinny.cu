@@ -10,7 +10,7 @@
 //  * SwiGLU (gate and up rows interleaved in blocks of 128): half of a cluster's CTAs compute the gate block, half the up
 //    block, and the owner of a token forms bf16(bf16(silu(g)) * u) from their sums, and its maximum.  (Grouped: one CTA
 //    computes both, one after the other, into two accumulators.)
-//  * Grouped problems (the experts of a MoE block): persistent CTAs walk over (expert, weight tile, pass of up to NT of
+//  * Grouped problems (the experts of a MoE block; with SwiGLU and plain): persistent CTAs walk over (expert, weight tile, pass of up to NT of
 //    its rows); the rows of each expert are read from the device, and experts without rows cost nothing.
 //  * Programmatic dependent launch: while the kernel before is still running, every CTA pulls its first weight tiles
 //    into L2 (a prefetch reads nothing into the CTA, so a weight still being written is not read early).
@@ -29,7 +29,7 @@ constexpr int SK_SF_COLS = 2 * KSTEPS * 4;      // tensor-memory columns of one 
 
 // NT token columns, NA accumulators; SPLIT: room for the cluster's partial sums.  Two CTAs per SM (half of 228 KB, less
 // 1 KB per CTA for the system, 1 KB for alignment and the barriers).
-template <int NT, int NA, bool SPLIT>
+template <int NT, int NA, bool SPLIT, bool GROUPED>
 struct SkCfg {
   static constexpr int X_BYTES = NT * BK_BYTES;
   static constexpr int XBOX = NT > 64 ? 32 : 16;                       // rows of A per TMA box
@@ -40,7 +40,7 @@ struct SkCfg {
   static constexpr int STAGE_BYTES = SK_W_BYTES + X_BYTES + 2 * SK_SF_BYTES;
   static constexpr int BAR_BYTES = 256;
   static constexpr int PART_BYTES = SPLIT && !PULL ? NA * (NT + 7) * 512 : 0;   // (tokens rounded up to the cluster, at most eight)
-  static constexpr int TABLE_BYTES = NA == 2 ? 3 * 64 * 4 : 0;         // grouped: the run table
+  static constexpr int TABLE_BYTES = GROUPED ? 3 * 64 * 4 : 0;         // the run table
   static constexpr int FIT = (113 * 1024 - 1024 - BAR_BYTES - TABLE_BYTES - PART_BYTES) / STAGE_BYTES;
   static constexpr int STAGES = FIT < 5 ? FIT : 5;
   static constexpr int SMEM_BYTES = 1024 + STAGES * STAGE_BYTES + PART_BYTES + BAR_BYTES + TABLE_BYTES;
@@ -103,14 +103,15 @@ __device__ __forceinline__ uint32_t add_bf16x2(uint32_t a, uint32_t b) {   // in
                      __fadd_rn(__uint_as_float(a & 0xffff0000u), __uint_as_float(b & 0xffff0000u)));
 }
 
-// NT: token columns per pass.  GATED: SwiGLU.  SPLIT: more than one CTA per cluster.
-template <int NT, bool GATED, bool SPLIT>
+// NT: token columns per pass.  GATED: SwiGLU.  SPLIT: more than one CTA per cluster.  GROUPED: runs of rows, each with its
+// own matrix (never split; SwiGLU of one matrix always is).
+template <int NT, bool GATED, bool SPLIT, bool GROUPED>
 __global__ void __launch_bounds__(SK_THREADS, 2)
 arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_w, const SkinnyParams p) {
   constexpr int NA = GATED && !SPLIT ? 2 : 1;          // accumulators of a CTA
   constexpr int NB = GATED ? 2 : 1;                    // 128-row blocks of weight per work item
-  constexpr bool GROUPED = GATED && !SPLIT;            // runs of rows, each with its own matrix (SwiGLU of one matrix is always split)
-  using C = SkCfg<NT, NA, SPLIT>;
+  static_assert(!(GROUPED && SPLIT) && (!GATED || GROUPED || SPLIT), "see above");
+  using C = SkCfg<NT, NA, SPLIT, GROUPED>;
   constexpr int TMEM_COLS = C::TMEM_COLS;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -496,10 +497,10 @@ arcq_skinny_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
   }
 }
 
-template <int NT, bool GATED, bool SPLIT>
+template <int NT, bool GATED, bool SPLIT, bool GROUPED = false>
 int launch_one(const CUtensorMap& mx, const CUtensorMap& mw, const SkinnyParams& p, int grid, cudaStream_t stream) {
-  using C = SkCfg<NT, GATED && !SPLIT ? 2 : 1, SPLIT>;
-  auto kern = arcq_skinny_kernel<NT, GATED, SPLIT>;
+  using C = SkCfg<NT, GATED && !SPLIT ? 2 : 1, SPLIT, GROUPED>;
+  auto kern = arcq_skinny_kernel<NT, GATED, SPLIT, GROUPED>;
   static thread_local int c_dev = -1;
   int dev = 0;
   ARCQ_CUDA_TRY(cudaGetDevice(&dev));
@@ -554,8 +555,7 @@ static int skinny_splits_wide(int tiles, int kstages, const DeviceInfo& di) {
   while (s > 1 && s > kstages / 2) s >>= 1;
   return s;
 }
-// See SkinnyParams; `residual` and `swiglu_amax` exclude each other; groups (device, with swiglu_amax): ngroups matrices
-// (at most 64) stacked in W.
+// See SkinnyParams; `residual` excludes `swiglu_amax` and groups; groups (device): ngroups matrices (at most 64) stacked in W.
 int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, const uint8_t* SFW, int64_t M, int64_t N,
                        int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, const void* residual, void* C,
                        float* swiglu_amax, const int* groups, int ngroups, cudaStream_t stream, bool residual_is_bias) {
@@ -600,7 +600,8 @@ int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, c
   if (rc != ARCQ_OK) return rc;
   rc = make_operand_map(&mw, W, N * p.ngroups, K_eff / 2, 128);
   if (rc != ARCQ_OK) return rc;
-  if (groups != nullptr) return launch_one<64, true, false>(mx, mw, p, (int)grid, stream);
+  if (groups != nullptr)
+    return gated ? launch_one<64, true, false, true>(mx, mw, p, (int)grid, stream) : launch_one<64, false, false, true>(mx, mw, p, (int)grid, stream);
   if (nt == 16) return launch_nt<16>(mx, mw, p, gated, (int)grid, stream);
   if (nt == 32) return launch_nt<32>(mx, mw, p, gated, (int)grid, stream);
   if (nt == 64) return launch_nt<64>(mx, mw, p, gated, (int)grid, stream);

@@ -433,7 +433,7 @@ class QMixtralMoEBlockEP(torch.nn.Module):
                 act, _ = ops.silu_mul(h, with_amax=False)
                 amax2 = ops.absmax_grouped(act, None, batch.groups, E)
         b, sfb, s2 = ops.quantize_grouped_amax(act, None, amax2, self.dn_index, batch.groups, batch.rows_bound, ke)
-        return ops.matmul_grouped(b, self.dn_W, sfb, self.dn_SF, batch.tile_group, E, cfg.hidden, s2, self.dn_scale)
+        return ops.matmul_grouped(b, self.dn_W, sfb, self.dn_SF, batch.tile_group, E, cfg.hidden, s2, self.dn_scale, batch.groups)
 
     n_streams = 4   # per-expert path: a few streams hide the launch gaps of the experts' small kernels
 

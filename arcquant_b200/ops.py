@@ -438,10 +438,11 @@ def quantize_grouped_amax(x: torch.Tensor, row_map, amax: torch.Tensor, reorder_
 
 
 def matmul_grouped(a, b, sfa, sfb, tile_group: torch.Tensor, ngroups: int, n: int, alpha_a: torch.Tensor,
-                   alpha_b: torch.Tensor | None = None) -> torch.Tensor:
+                   alpha_b: torch.Tensor | None = None, groups: torch.Tensor | None = None) -> torch.Tensor:
     """bf16 [rows, n]: every 256-row tile m of A times the weight matrix tile_group[m] of the `ngroups`
     matrices stacked in b [ngroups * n, K_eff/2] (negative = tile skipped), scaled by
-    alpha_a[g] * alpha_b[g]."""
+    alpha_a[g] * alpha_b[g].  groups (optional, at most 64 runs): the run table; with it only the runs' rows are
+    written, and a few rows per run are multiplied as weight streaming."""
     lib = _lib.load()
     for t, name in ((a, "A"), (b, "B"), (sfa, "SFA"), (sfb, "SFB")):
         _require(t, torch.uint8, name)
@@ -456,6 +457,16 @@ def matmul_grouped(a, b, sfa, sfb, tile_group: torch.Tensor, ngroups: int, n: in
     if sfa.numel() < ((m + 127) // 128) * atoms * 512 or sfb.numel() < ((ngroups * n + 127) // 128) * atoms * 512:
         raise RuntimeError("scale buffers are smaller than the scale layout of their operands")
     c = torch.empty((m, n), dtype=torch.bfloat16, device=a.device)
+    if groups is not None and ngroups <= 64:
+        _require(groups, torch.int32, "groups")
+        if groups.numel() != 2 * ngroups:
+            raise RuntimeError("groups must hold 2 * ngroups entries")
+        with torch.cuda.device(a.device):
+            rc = lib.arcq_matmul_nvfp4_grouped_runs(a.data_ptr(), b.data_ptr(), sfa.data_ptr(), sfb.data_ptr(), m, n, kb * 2,
+                                                    tile_group.data_ptr(), groups.data_ptr(), ngroups, alpha_a.data_ptr(),
+                                                    None if alpha_b is None else alpha_b.data_ptr(), c.data_ptr(), _stream())
+        _lib.check(rc, f"grouped matmul M={m} N={n} K={kb * 2} groups={ngroups}")
+        return c
     with torch.cuda.device(a.device):
         rc = lib.arcq_matmul_nvfp4_grouped(a.data_ptr(), b.data_ptr(), sfa.data_ptr(), sfb.data_ptr(), m, n, kb * 2,
                                            tile_group.data_ptr(), ngroups, alpha_a.data_ptr(),

@@ -300,6 +300,13 @@ int arcq_reorder_quantize_x_grouped(const void* x, const int32_t* row_map, const
 int arcq_matmul_nvfp4_grouped(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB,
                               int64_t M_bound, int64_t N, int64_t K_eff, const int32_t* tile_group, int ngroups,
                               const float* alpha_a, const float* alpha_b, void* C, void* stream);
+/* The same with the run table (groups as in arcq_reorder_quantize_x_grouped, at most 64 runs): only the rows of the runs are
+ * written, and where the bound says that a run has a handful of rows the weights are streamed past them instead of filling
+ * 256-row tiles. */
+int arcq_matmul_nvfp4_grouped_runs(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB,
+                                   int64_t M_bound, int64_t N, int64_t K_eff, const int32_t* tile_group,
+                                   const int32_t* groups, int ngroups, const float* alpha_a, const float* alpha_b, void* C,
+                                   void* stream);
 
 /* ---- Gate/up projection with the SwiGLU fused into the GEMM's epilogue -------------------------------
  * The reference runs gate_proj and up_proj as two GEMMs and then `act_fn(gate) * up` in torch

@@ -1,0 +1,58 @@
+"""The plain grouped GEMM with a run table: a few rows per run stream the weights past them.  Reference: the same call
+without the table (256-row tiles), which the oracle tests cover."""
+import pytest
+import torch
+
+from arcquant_b200 import synth
+from tests.helpers import launched_kernels
+
+pytestmark = pytest.mark.gpu
+
+
+# 65 and 130 rows of a run are two and three passes of 64 columns, the second starting in the middle of a scale tile; K of one
+# partial stage, and of several; more than a wave of work items; too many rows per run for streaming
+@pytest.mark.parametrize("counts,kq,n,streams", [
+    ((5, 0, 17, 1, 0, 0, 2, 12), 1024, 512, True), ((0, 0, 0, 0, 0, 0, 0, 1), 128, 128, True),
+    ((130, 0, 2, 1, 0, 64, 58, 1), 1024, 384, True), ((65, 0, 63, 1, 0, 127, 0, 0), 320, 256, True),
+    ((9, 10, 11, 12, 13, 0, 1, 2), 2048, 6144, True), ((1, 0, 33, 16, 0, 64, 65, 0, 7, 3), 512, 256, True),
+    ((2, 0, 66, 1) * 10, 192, 128, True), ((300, 17, 0, 257), 512, 256, False)])
+def test_grouped_plain_gemm_with_the_run_table(counts, kq, n, streams):
+    from arcquant_b200 import ops
+    from arcquant_b200.qlinear import NVFP4_reorder_quantize_w
+
+    e, ke = len(counts), 64
+    k_eff = kq + ke
+    idx = torch.stack([torch.randperm(kq, generator=torch.Generator().manual_seed(i)) for i in range(e)]).to(torch.int16).cuda()
+    ws = [NVFP4_reorder_quantize_w(synth.weights(n, kq, 40 + i, device="cuda"), idx[i], ke, mode=16) for i in range(e)]
+    span = (n // 128) * ((k_eff // 16 + 3) // 4) * 512
+    B, SFB, sw = torch.cat([w[0] for w in ws]), torch.cat([w[1][:span] for w in ws]), torch.stack([w[2] for w in ws])
+    starts, at = [], 0
+    for c in counts:
+        starts.append(at)
+        at += (c + 255) // 256 * 256
+    total = sum(counts)
+    bound = (total + 255) // 256 * 256 + e * 256
+    groups = torch.tensor(starts + list(counts), dtype=torch.int32, device="cuda")
+    tile_group = torch.full((bound // 256,), -1, dtype=torch.int32)
+    row_map = torch.zeros(bound, dtype=torch.int32)
+    k = 0
+    for i, (s, c) in enumerate(zip(starts, counts)):
+        tile_group[s // 256:(s + c + 255) // 256] = i
+        row_map[s:s + c] = torch.arange(k, k + c).int()
+        k += c
+    tile_group, row_map = tile_group.cuda(), row_map.cuda()
+    x = synth.activations(total, kq, 5, synth.outlier_channels(kq, max(1, kq // 100), 2), device="cuda")
+    a, sfa, sx = ops.quantize_grouped_amax(x, row_map, ops.absmax_grouped(x, row_map, groups, e), idx, groups, bound, ke)
+
+    def run():
+        return ops.matmul_grouped(a, B, sfa, SFB, tile_group, e, n, sx, sw, groups)
+
+    kernels = [name for name, _, _ in launched_kernels(run)]
+    assert len(kernels) == 1 and ("arcq_skinny_kernel" if streams else "arcq_gemm2_kernel") in kernels[0]
+    got, want = run(), ops.matmul_grouped(a, B, sfa, SFB, tile_group, e, n, sx, sw)
+    torch.cuda.synchronize()
+    assert ops.gemm_poll_error() == 0
+    for s, c in zip(starts, counts):
+        g, w = got[s:s + c].double(), want[s:s + c].double()
+        # fp32 sums of the same products: at most a bf16 rounding apart here and there
+        assert float((g - w).norm()) <= 1e-3 * float(w.norm()) and (c == 0 or float((g == w).float().mean()) >= 0.99)

@@ -1642,16 +1642,21 @@ __global__ void __launch_bounds__(512) arcq_max_partials_kernel(const uint4* __r
     if (SIGNED) asm("max.NaN.bf16x2 %0, %0, %1;" : "+r"(m) : "r"(w));
     else m = max_u16x2(m, w & 0x7fff7fffu);
   };
+  // IN loads in flight per thread; what is left over at the end goes one by one.
+  constexpr int IN = 4;
   long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  for (; i + 3 * step < nvec; i += 4 * step) {
-    uint4 v[4];
+  const uint4* at = x + (nvec - 1 - i);
+#pragma unroll 1
+  for (; i + (IN - 1) * step < nvec; i += IN * step, at -= IN * step) {
+    uint4 v[IN];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = __ldg(x + (nvec - 1 - i - k * step));
+    for (int k = 0; k < IN; ++k) v[k] = __ldg(at - k * step);
 #pragma unroll
-    for (int k = 0; k < 4; ++k) { take(v[k].x); take(v[k].y); take(v[k].z); take(v[k].w); }
+    for (int k = 0; k < IN; ++k) { take(v[k].x); take(v[k].y); take(v[k].z); take(v[k].w); }
   }
-  for (; i < nvec; i += step) {
-    const uint4 v = __ldg(x + (nvec - 1 - i));
+#pragma unroll 1
+  for (; i < nvec; i += step, at -= step) {
+    const uint4 v = __ldg(at);
     take(v.x); take(v.y); take(v.z); take(v.w);
   }
 #pragma unroll
@@ -2006,9 +2011,9 @@ int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight
     int rc = get_device_info(&di);
     if (rc != ARCQ_OK) return rc;
     const long long nvec = rows * (long long)KQ / 8;
-    // four 16-byte loads per thread, at most two CTAs per SM
+    // four 16-byte loads per thread, at most three CTAs per SM
     long long grid = (nvec + 4 * 512 - 1) / (4 * 512);
-    if (grid > di.resident(2)) grid = di.resident(2);
+    if (grid > di.resident(3)) grid = di.resident(3);
     if (grid > ARCQ_SCALE_SCRATCH) grid = ARCQ_SCALE_SCRATCH;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);

@@ -49,7 +49,8 @@ struct GemmParams {
   const uint8_t* sfa;
   const uint8_t* sfb;
   __nv_bfloat16* c;
-  const __nv_bfloat16* bias;   // [N], added to the bf16-rounded result, or nullptr
+  const __nv_bfloat16* bias;   // added to the bf16-rounded result, or nullptr: [N], or a residual [M, N] (bias_ld = N)
+  int bias_ld;                 // elements between its rows: 0 or N
   const float* alpha_a;
   const float* alpha_b;
   float alpha;
@@ -232,7 +233,7 @@ arcq_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
               o.y = pack_bf16x2(__uint_as_float(r[v * 8 + 2]) * alpha, __uint_as_float(r[v * 8 + 3]) * alpha);
               o.z = pack_bf16x2(__uint_as_float(r[v * 8 + 4]) * alpha, __uint_as_float(r[v * 8 + 5]) * alpha);
               o.w = pack_bf16x2(__uint_as_float(r[v * 8 + 6]) * alpha, __uint_as_float(r[v * 8 + 7]) * alpha);
-              if (p.bias != nullptr) add_bias8(o, p.bias + col + v * 8);
+              if (p.bias != nullptr) add_bias8(o, p.bias + (size_t)row * p.bias_ld + col + v * 8);
               *reinterpret_cast<uint4*>(crow + col + v * 8) = o;
             }
           }
@@ -329,7 +330,7 @@ __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {   // remote a
 }
 struct Gemm2Params {
   __nv_bfloat16* c;
-  const __nv_bfloat16* bias;   // see GemmParams (plain epilogue only)
+  const __nv_bfloat16* bias;   // [N], see GemmParams (plain epilogue only)
   const float* alpha_a;
   const float* alpha_b;
   float alpha;
@@ -824,6 +825,21 @@ int launch_bn(const CUtensorMap& ma, const CUtensorMap& mb, GemmParams p, int nu
   return launch_dependent(kern, (unsigned)grid, NUM_THREADS, C::SMEM_BYTES, stream, ma, mb, p);
 }
 
+// The single-CTA kernel with tiles of bn columns.
+int launch_single(const uint8_t* A, const uint8_t* B, int64_t M, int64_t N, int64_t K_eff, int bn, const GemmParams& p, int num_sms,
+                  cudaStream_t stream) {
+  CUtensorMap ma, mb;
+  int rc = make_operand_map(&ma, A, M, K_eff / 2, BM);
+  if (rc != ARCQ_OK) return rc;
+  rc = make_operand_map(&mb, B, N, K_eff / 2, bn);
+  if (rc != ARCQ_OK) return rc;
+  switch (bn) {
+    case 256: return launch_bn<256>(ma, mb, p, num_sms, stream);
+    case 128: return launch_bn<128>(ma, mb, p, num_sms, stream);
+    default: return launch_bn<64>(ma, mb, p, num_sms, stream);
+  }
+}
+
 }  // namespace
 
 // Scratch for partial sums (see gemm_workspace_bytes) and tile width of the single-CTA kernel, by the cost model of a
@@ -868,15 +884,30 @@ static void plan_splitk(int64_t M, int64_t N, int64_t K_eff, int num_sms, int* b
   *splits_out = splits;
 }
 
-// Weight streaming (arcq_skinny.cu): up to 64 rows, and as long as 128 x 128 tiles leave an SM for each, so that a cluster
-// of two or four can share a tile's K and the whole problem is one wave.  Measured, us (this kernel / the single-CTA
-// kernel with its partial sums in global memory, or CTA pairs where there are enough 256 x 256 tiles for them):
-//   [4096, 4224]   65 rows 8.1 / 11.7   200 rows 10.9 / 15.7   333 rows 12.1 / 27.7   512 rows 12.8 / 27.8
-//   [6144, 4224]  128 rows 11.0 / 16.3  200 rows 12.2 / 28.4   333 rows 13.1 / 14.3
-//   [4096, 14464] 128 rows 15.8 / 20.7  333 rows 22.7 / 81.8   512 rows 23.4 / 81.9
-// and beyond that line 777 rows of [4096, 4224] 21.1 / 14.3, [28672, 4224] 128 rows 24.5 / 22.4.
-// Above 64 rows only where K is split: with a K of less than four stages this kernel's stores are the time, [256, 576]
-// 512 rows 5.5 / 5.1, 4096 rows 6.2 / 5.1 (with a residual 8.2 / 11.4 and 8.5 / 10.6: there it is the better one all the same).
+// Width of the single-CTA kernel's tiles for more than 64 rows where its tiles are one wave (the narrowest that are: a narrow
+// tile's stages are short), or 0 where another kernel is the faster one.  Its K loop is one chain of stages; weight streaming
+// splits a long K over a cluster, which pays while there are one or two tiles of rows.  us, weight streaming (CTA pairs in
+// brackets where they apply, their threshold lowered to 18 tiles) / this kernel, products without a residual:
+//   [1024, 4224]    65 rows 6.5 / 7.5   100 rows 7.7 / 7.2    333 rows 8.3 / 7.5
+//   [2048, 4224]    65 rows 6.7 / 7.1   128 rows 8.1 / 7.3    333 rows 10.8 / 7.8
+//   [4096, 4224]    65 rows 7.6 / 7.4   128 rows 9.5 / 7.6    200 rows 11.0 / 7.9    333 rows 12.1 (10.6) / 8.9
+//   [6144, 4224]    65 rows 8.5 / 7.6   128 rows 11.0 / 8.2   200 rows 11.9 / 8.6    333 rows 12.6 (11.6) / 8.9
+//   [4096, 6272]    65 rows 8.5 / 8.3   128 rows 10.4 / 10.2  200 rows 11.9 / 10.3   333 rows 14.3 / 11.3
+//   [4096, 7296]    65 rows 9.0 / 11.3  128 rows 11.8 / 13.0  256 rows 13.2 / 11.3   333 rows 16.1 (14.7) / 13.1
+//   [4096, 14464]   65 rows 14.0 / 17.3 128 rows 16.1 / 19.2  256 rows 17.3 / 19.8   512 rows 22.6 (24.3) / 17.6
+// With a residual (read 16 bytes per row here): [4096, 4224] 128 rows 9.9 / 9.5, 333 rows 13.0 / 12.1, [4096, 14464] 333 rows
+// 22.6 / 21.8.  Tiles of 256 columns lose to CTA pairs (777 rows of [4096, 4224] 14.3 / 11.4), so 128 is the widest here.
+static int single_tile(int64_t M, int64_t N, int64_t K_eff, int num_sms) {
+  const int64_t rows = (M + BM - 1) / BM, stages = (K_eff / 64 + KSTEPS - 1) / KSTEPS;
+  if (M <= ARCQ_SKINNY_ROWS || rows * ((N + 127) / 128) > num_sms) return 0;
+  const int64_t chain = rows > 2 ? stages : (rows == 2 ? 40 : (M <= 96 && N <= 2048 ? 12 : 24));
+  if (stages > chain && skinny_plan_splits(M, N, K_eff) > 1) return 0;
+  return rows * ((N + 63) / 64) <= num_sms ? 64 : 128;
+}
+
+// Weight streaming (arcq_skinny.cu): up to 64 rows, a long K (see above), and with a residual as long as 128 x 128 tiles leave
+// an SM for each, so that a cluster of two or four can share a tile's K and the whole problem is one wave.  us, this kernel /
+// CTA pairs: [4096, 14464] 128 rows 15.8 / 20.7, 333 rows 22.7 / 24; beyond that line 777 rows of [4096, 4224] 21.1 / 11.
 static bool use_skinny_kernel(int64_t M, int64_t N, int64_t K_eff, int num_sms, bool residual = false) {
   return M <= ARCQ_SKINNY_ROWS || (((M + 127) / 128) * ((N + 127) / 128) <= num_sms && (residual || skinny_plan_splits(M, N, K_eff) > 1));
 }
@@ -939,17 +970,20 @@ int launch_gemm_scatter(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, 
   return launch_pair(A, B, SFA, SFB, M, N, K_eff, p, di.num_sms, stream, nullptr, 1, nullptr, nullptr, dests, ndests);
 }
 
-// C = bf16(residual + bf16(alpha_a * alpha_b * A B^T)): the CTA-pair kernel, whose epilogue fetches the residual tile by
-// TMA, or - few rows - the weight-streaming kernel.
+// C = bf16(residual + bf16(alpha_a * alpha_b * A B^T)), in the kernel that serves the plain product of this shape (so that the
+// bits are those of an addition behind it), or CTA pairs.
 int launch_gemm_residual(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,
                          int64_t N, int64_t K_eff, const float* alpha_a, const float* alpha_b, const void* residual,
                          void* Cout, cudaStream_t stream) {
   DeviceInfo di;
   int rc = get_device_info(&di);
   if (rc != ARCQ_OK) return rc;
-  if (use_skinny_kernel(M, N, K_eff, di.num_sms, true))
+  const int bn = single_tile(M, N, K_eff, di.num_sms);
+  if (bn == 0 && use_skinny_kernel(M, N, K_eff, di.num_sms, true))
     return launch_gemm_skinny(A, B, SFA, SFB, M, N, K_eff, 1.0f, alpha_a, alpha_b, residual, Cout, nullptr, nullptr, 1, stream);
   GemmParams p = {};
+  p.sfa = SFA;
+  p.sfb = SFB;
   p.c = static_cast<__nv_bfloat16*>(Cout);
   p.alpha_a = alpha_a;
   p.alpha_b = alpha_b;
@@ -958,6 +992,13 @@ int launch_gemm_residual(const uint8_t* A, const uint8_t* B, const uint8_t* SFA,
   p.N = (int)N;
   p.ksteps_total = (int)(K_eff / 64);
   p.natoms = (int)((K_eff / 16 + 3) / 4);
+  p.tiles_m = (int)((M + BM - 1) / BM);
+  p.sfb_tiles = (int)((N + 127) / 128);
+  if (bn != 0) {
+    p.bias = static_cast<const __nv_bfloat16*>(residual);
+    p.bias_ld = (int)N;
+    return launch_single(A, B, M, N, K_eff, bn, p, di.num_sms, stream);
+  }
   return launch_pair(A, B, SFA, SFB, M, N, K_eff, p, di.num_sms, stream, nullptr, 1, nullptr, nullptr, nullptr, 0,
                      residual);
 }
@@ -981,13 +1022,15 @@ int gemm_plan(int64_t M, int64_t N, int64_t K_eff, int* kind, int* tile_n, int* 
   DeviceInfo di;
   int rc = get_device_info(&di);
   if (rc != ARCQ_OK) return rc;
-  int k = ARCQ_GEMM_KIND_SINGLE, bn = 256, sp = 1;
-  if (use_skinny_kernel(M, N, K_eff, di.num_sms)) {
+  int k = ARCQ_GEMM_KIND_SINGLE, bn = single_tile(M, N, K_eff, di.num_sms), sp = 1;
+  if (bn != 0) {
+  } else if (use_skinny_kernel(M, N, K_eff, di.num_sms)) {
     k = ARCQ_GEMM_KIND_SKINNY;
     bn = 128;
     sp = skinny_plan_splits(M, N, K_eff);
   } else if (use_pair_kernel(M, N, di.num_sms)) {
     k = ARCQ_GEMM_KIND_PAIR;
+    bn = 256;
   } else {
     plan_splitk(M, N, K_eff, di.num_sms, &bn, &sp, false);
   }
@@ -1003,7 +1046,8 @@ int launch_gemm(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const ui
   DeviceInfo di;
   int rc = get_device_info(&di);
   if (rc != ARCQ_OK) return rc;
-  if (use_skinny_kernel(M, N, K_eff, di.num_sms))
+  int bn = single_tile(M, N, K_eff, di.num_sms);
+  if (bn == 0 && use_skinny_kernel(M, N, K_eff, di.num_sms))
     return launch_gemm_skinny(A, B, SFA, SFB, M, N, K_eff, alpha, alpha_a, alpha_b, bias, Cout, nullptr, nullptr, 1, stream,
                               bias != nullptr);
 
@@ -1012,6 +1056,7 @@ int launch_gemm(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const ui
   p.sfb = SFB;
   p.c = static_cast<__nv_bfloat16*>(Cout);
   p.bias = static_cast<const __nv_bfloat16*>(bias);
+  p.bias_ld = 0;
   p.alpha_a = alpha_a;
   p.alpha_b = alpha_b;
   p.alpha = alpha;
@@ -1022,20 +1067,11 @@ int launch_gemm(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const ui
   p.tiles_m = (int)((M + BM - 1) / BM);
   p.tiles_n = 0;
   p.sfb_tiles = (int)((N + 127) / 128);
-  if (use_pair_kernel(M, N, di.num_sms)) return launch_pair(A, B, SFA, SFB, M, N, K_eff, p, di.num_sms, stream);
+  if (bn == 0 && use_pair_kernel(M, N, di.num_sms)) return launch_pair(A, B, SFA, SFB, M, N, K_eff, p, di.num_sms, stream);
 
-  int bn, splits;
-  plan_splitk(M, N, K_eff, di.num_sms, &bn, &splits, false);
-  CUtensorMap ma, mb;
-  rc = make_operand_map(&ma, A, M, K_eff / 2, BM);
-  if (rc != ARCQ_OK) return rc;
-  rc = make_operand_map(&mb, B, N, K_eff / 2, bn);
-  if (rc != ARCQ_OK) return rc;
-  switch (bn) {
-    case 256: return launch_bn<256>(ma, mb, p, di.num_sms, stream);
-    case 128: return launch_bn<128>(ma, mb, p, di.num_sms, stream);
-    default: return launch_bn<64>(ma, mb, p, di.num_sms, stream);
-  }
+  int splits;
+  if (bn == 0) plan_splitk(M, N, K_eff, di.num_sms, &bn, &splits, false);
+  return launch_single(A, B, M, N, K_eff, bn, p, di.num_sms, stream);
 }
 
 // ----------------------------------------------------------------------------- no-allocation entry point

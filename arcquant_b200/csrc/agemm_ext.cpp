@@ -236,6 +236,111 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> quantize_tensor_scale(co
   return std::make_tuple(Q, SF, scale);
 }
 
+const float* f32_or_null(const c10::optional<torch::Tensor>& t, const torch::Tensor& like, const char* name) {
+  if (!t.has_value()) return nullptr;
+  require_on(*t, like, at::kFloat, name);
+  return t->data_ptr<float>();
+}
+
+// Gate/up GEMM with the SwiGLU epilogue; see arcq_matmul_nvfp4_swiglu.
+std::tuple<torch::Tensor, torch::Tensor> matmul_swiglu(const torch::Tensor& A, const torch::Tensor& B, const torch::Tensor& SFA,
+                                                       const torch::Tensor& SFB, const torch::Tensor& alpha_a,
+                                                       const c10::optional<torch::Tensor>& alpha_b) {
+  int64_t M, N, K;
+  std::tie(M, N, K) = check_gemm_operands(A, B, SFA, SFB);
+  require_on(alpha_a, A, at::kFloat, "alpha_a");
+  const float* ab = f32_or_null(alpha_b, A, "alpha_b");
+  TORCH_CHECK(N % 256 == 0, "N is not a multiple of 256");
+  c10::cuda::CUDAGuard guard(A.device());
+  auto C = torch::empty({M, N / 2}, torch::dtype(torch::kBFloat16).device(A.device()));
+  auto amax = torch::empty({}, torch::dtype(torch::kFloat32).device(A.device()));
+  check_status(arcq_matmul_nvfp4_swiglu(A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(), SFB.data_ptr<uint8_t>(),
+                                        M, N, K, alpha_a.data_ptr<float>(), ab, C.data_ptr<at::BFloat16>(), amax.data_ptr<float>(),
+                                        current_stream(A)),
+               "swiglu matmul");
+  return std::make_tuple(C, amax);
+}
+
+// The grouped forms; groups: the run table [first rows | rows].
+void check_grouped(const torch::Tensor& A, const torch::Tensor& B, int64_t K, const torch::Tensor& tile_group, const torch::Tensor& groups,
+                   int64_t ngroups, int64_t n, const torch::Tensor& alpha_a) {
+  require_on(tile_group, A, at::kInt, "tile_group");
+  require_on(groups, A, at::kInt, "groups");
+  require_on(alpha_a, A, at::kFloat, "alpha_a");
+  TORCH_CHECK(ngroups > 0 && n > 0 && B.size(0) == ngroups * n && tile_group.numel() >= (A.size(0) + 255) / 256 &&
+                  alpha_a.numel() == ngroups && groups.numel() >= 2 * ngroups,
+              "operand shapes disagree");
+}
+std::tuple<torch::Tensor, torch::Tensor> matmul_grouped_swiglu(const torch::Tensor& A, const torch::Tensor& B, const torch::Tensor& SFA,
+                                                               const torch::Tensor& SFB, const torch::Tensor& tile_group,
+                                                               const torch::Tensor& groups, int64_t ngroups, int64_t n,
+                                                               const torch::Tensor& alpha_a,
+                                                               const c10::optional<torch::Tensor>& alpha_b) {
+  int64_t M, N, K;
+  std::tie(M, N, K) = check_gemm_operands(A, B, SFA, SFB);
+  check_grouped(A, B, K, tile_group, groups, ngroups, n, alpha_a);
+  const float* ab = f32_or_null(alpha_b, A, "alpha_b");
+  TORCH_CHECK(n % 256 == 0, "n is not a multiple of 256");
+  c10::cuda::CUDAGuard guard(A.device());
+  auto C = torch::empty({M, n / 2}, torch::dtype(torch::kBFloat16).device(A.device()));
+  auto amax = torch::empty({ngroups}, torch::dtype(torch::kFloat32).device(A.device()));
+  check_status(arcq_matmul_nvfp4_grouped_swiglu(A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(),
+                                                SFB.data_ptr<uint8_t>(), M, n, K, tile_group.data_ptr<int32_t>(),
+                                                groups.data_ptr<int32_t>(), static_cast<int>(ngroups), alpha_a.data_ptr<float>(), ab,
+                                                C.data_ptr<at::BFloat16>(), amax.data_ptr<float>(), current_stream(A)),
+               "grouped swiglu matmul");
+  return std::make_tuple(C, amax);
+}
+torch::Tensor matmul_grouped_runs(const torch::Tensor& A, const torch::Tensor& B, const torch::Tensor& SFA, const torch::Tensor& SFB,
+                                  const torch::Tensor& tile_group, const torch::Tensor& groups, int64_t ngroups, int64_t n,
+                                  const torch::Tensor& alpha_a, const c10::optional<torch::Tensor>& alpha_b) {
+  int64_t M, N, K;
+  std::tie(M, N, K) = check_gemm_operands(A, B, SFA, SFB);
+  check_grouped(A, B, K, tile_group, groups, ngroups, n, alpha_a);
+  const float* ab = f32_or_null(alpha_b, A, "alpha_b");
+  c10::cuda::CUDAGuard guard(A.device());
+  auto C = torch::empty({M, n}, torch::dtype(torch::kBFloat16).device(A.device()));
+  check_status(arcq_matmul_nvfp4_grouped_runs(A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(),
+                                              SFB.data_ptr<uint8_t>(), M, n, K, tile_group.data_ptr<int32_t>(),
+                                              groups.data_ptr<int32_t>(), static_cast<int>(ngroups), alpha_a.data_ptr<float>(), ab,
+                                              C.data_ptr<at::BFloat16>(), current_stream(A)),
+               "grouped matmul");
+  return C;
+}
+
+// Grouped rows quantized by their runs' maxima; see arcq_quantize_x_grouped_amax.
+std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> quantize_grouped_amax(const torch::Tensor& X, const c10::optional<torch::Tensor>& row_map,
+                                                                              const torch::Tensor& amax, const torch::Tensor& indices,
+                                                                              const torch::Tensor& groups, int64_t rows_bound, int KE,
+                                                                              int mode) {
+  require_cuda(X, "input");
+  TORCH_CHECK(X.scalar_type() == at::kBFloat16 && X.dim() >= 1, "input: expected bfloat16 rows");
+  require_on(amax, X, at::kFloat, "amax");
+  require_on(indices, X, at::kShort, "reorder_indices");
+  require_on(groups, X, at::kInt, "groups");
+  TORCH_CHECK(indices.dim() == 2, "reorder_indices must be [runs, KQ]");
+  const int64_t ngroups = indices.size(0), KQ = indices.size(1);
+  TORCH_CHECK(X.size(-1) == KQ && amax.numel() == ngroups && groups.numel() == 2 * ngroups,
+              "reorder_indices / groups disagree on the number of runs or on KQ");
+  if (row_map.has_value()) {
+    require_on(*row_map, X, at::kInt, "row_map");
+    TORCH_CHECK(row_map->numel() >= rows_bound, "row_map must cover rows_bound rows");
+  } else {
+    TORCH_CHECK(X.size(0) >= rows_bound, "input has fewer rows than rows_bound");
+  }
+  c10::cuda::CUDAGuard guard(X.device());
+  const auto u8 = X.options().dtype(torch::kUInt8);
+  auto Q = torch::empty({rows_bound, (KQ + KE) / 2}, u8);
+  auto SF = torch::empty({static_cast<int64_t>(arcq_sf_bytes(rows_bound, KQ + KE))}, u8);
+  auto scale = torch::empty({ngroups}, X.options().dtype(torch::kFloat32));
+  check_status(arcq_quantize_x_grouped_amax(X.data_ptr(), row_map.has_value() ? row_map->data_ptr<int32_t>() : nullptr,
+                                            amax.data_ptr<float>(), indices.data_ptr<int16_t>(), groups.data_ptr<int32_t>(),
+                                            static_cast<int>(ngroups), rows_bound, static_cast<int>(KQ), KE, mode,
+                                            Q.data_ptr<uint8_t>(), SF.data_ptr<uint8_t>(), scale.data_ptr<float>(), current_stream(X)),
+               "grouped x-quantize");
+  return std::make_tuple(Q, SF, scale);
+}
+
 // One batch of calibration statistics, accumulated in place; see arcq_calib_stats_bf16.
 void calib_stats(const torch::Tensor& X, const torch::Tensor& chan_absmax, const c10::optional<torch::Tensor>& above) {
   require_cuda(X, "input");
@@ -321,6 +426,15 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("quantize_tensor_scale", &quantize_tensor_scale, "(Q, SF, scale) of x or w over its per-tensor scale", py::arg("X"),
         py::arg("reorder_index"), py::arg("KE"), py::arg("mode") = -1, py::arg("is_weight") = false,
         py::arg("amax") = py::none());
+  m.def("matmul_swiglu", &matmul_swiglu, "gate/up GEMM with SwiGLU: (act, amax)", py::arg("A"), py::arg("B"), py::arg("SFA"),
+        py::arg("SFB"), py::arg("alpha_a"), py::arg("alpha_b"));
+  m.def("matmul_grouped_swiglu", &matmul_grouped_swiglu, "its grouped form", py::arg("A"), py::arg("B"), py::arg("SFA"), py::arg("SFB"),
+        py::arg("tile_group"), py::arg("groups"), py::arg("ngroups"), py::arg("n"), py::arg("alpha_a"), py::arg("alpha_b"));
+  m.def("matmul_grouped_runs", &matmul_grouped_runs, "grouped GEMM with the run table", py::arg("A"), py::arg("B"), py::arg("SFA"),
+        py::arg("SFB"), py::arg("tile_group"), py::arg("groups"), py::arg("ngroups"), py::arg("n"), py::arg("alpha_a"), py::arg("alpha_b"));
+  m.def("quantize_grouped_amax", &quantize_grouped_amax, "grouped rows by their runs' maxima: (codes, scales, scale)", py::arg("X"),
+        py::arg("row_map"), py::arg("amax"), py::arg("reorder_indices"), py::arg("groups"), py::arg("rows_bound"), py::arg("KE"),
+        py::arg("mode"));
   m.def("channel_order", &channel_order, "channels by ascending statistic, int16", py::arg("value"));
   m.def("calib_stats", &calib_stats, "accumulate the calibration statistics of one batch", py::arg("X"),
         py::arg("chan_absmax"), py::arg("above") = py::none());

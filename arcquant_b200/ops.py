@@ -412,6 +412,9 @@ def quantize_grouped_amax(x: torch.Tensor, row_map, amax: torch.Tensor, reorder_
     if ngroups > 64 or kq > 16384 or amax.numel() != ngroups:
         scale = amax / (448.0 * 6.0)
         return (*reorder_quantize_x_grouped(x, row_map, scale, reorder_indices, groups, rows_bound, ke, mode), scale)
+    ext = _ext()
+    if ext:
+        return ext.quantize_grouped_amax(x, row_map, amax, reorder_indices, groups, rows_bound, ke, mode)
     lib = _lib.load()
     _require(x, torch.bfloat16, "input")
     _require(amax, torch.float32, "amax")
@@ -443,6 +446,9 @@ def matmul_grouped(a, b, sfa, sfb, tile_group: torch.Tensor, ngroups: int, n: in
     matrices stacked in b [ngroups * n, K_eff/2] (negative = tile skipped), scaled by
     alpha_a[g] * alpha_b[g].  groups (optional, at most 64 runs): the run table; with it only the runs' rows are
     written, and a few rows per run are multiplied as weight streaming."""
+    ext = _ext()
+    if ext and groups is not None and ngroups <= 64:
+        return ext.matmul_grouped_runs(a, b, sfa, sfb, tile_group, groups, ngroups, n, alpha_a, alpha_b)
     lib = _lib.load()
     for t, name in ((a, "A"), (b, "B"), (sfa, "SFA"), (sfb, "SFB")):
         _require(t, torch.uint8, name)
@@ -487,6 +493,9 @@ def interleave_gate_up(w_gate: torch.Tensor, w_up: torch.Tensor, block: int = 12
 def matmul_swiglu(a, b, sfa, sfb, alpha_a: torch.Tensor, alpha_b: torch.Tensor | None = None):
     """(act bf16 [M, N/2], amax 0-dim fp32): gate/up GEMM over an interleaved weight (`interleave_gate_up`) with
     silu(gate) * up and its max|.| taken in the epilogue."""
+    ext = _ext()
+    if ext:
+        return ext.matmul_swiglu(a, b, sfa, sfb, alpha_a, alpha_b)
     lib = _lib.load()
     for t, name in ((a, "A"), (b, "B"), (sfa, "SFA"), (sfb, "SFB")):
         _require(t, torch.uint8, name)
@@ -513,6 +522,9 @@ def matmul_swiglu(a, b, sfa, sfb, alpha_a: torch.Tensor, alpha_b: torch.Tensor |
 def matmul_grouped_swiglu(a, b, sfa, sfb, tile_group: torch.Tensor, groups: torch.Tensor, ngroups: int, n: int,
                           alpha_a: torch.Tensor, alpha_b: torch.Tensor | None = None):
     """`matmul_grouped` with the SwiGLU epilogue: (act bf16 [rows, n/2], amax fp32 [ngroups])."""
+    ext = _ext()
+    if ext:
+        return ext.matmul_grouped_swiglu(a, b, sfa, sfb, tile_group, groups, ngroups, n, alpha_a, alpha_b)
     lib = _lib.load()
     for t, name in ((a, "A"), (b, "B"), (sfa, "SFA"), (sfb, "SFB")):
         _require(t, torch.uint8, name)

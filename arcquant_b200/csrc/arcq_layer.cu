@@ -643,6 +643,16 @@ arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, u
   for (int j = 0; j < CPT; ++j) cmax[j][0] = cmax[j][1] = cmax[j][2] = cmax[j][3] = 0;
   unsigned long long count = 0;
   int buf = 0;
+  // The running maxima that this thread's first word will meet are asked for now, so that their latency is not behind the
+  // cluster's meeting (a value that is stale by then only costs an atomic): 2000 x 4096 10.0 -> 9.1 us, 300 x 4096 6.5 -> 5.5.  With
+  // two chunks per thread the registers are not there (1500 x 5120 11.6 -> 12.3).
+  constexpr bool EARLY = CLUSTER && CPT == 1;
+  uint32_t run0 = 0, run1 = 0;
+  const int w_early = EARLY ? (int)cluster.block_rank() * CALIB_THREADS + tid : 0;
+  if (EARLY && w_early < (K >> 1)) {
+    run0 = __ldcg(chan_absmax + 2 * w_early);
+    run1 = __ldcg(chan_absmax + 2 * w_early + 1);
+  }
   for (long long r0 = (long long)blockIdx.x * RB; r0 < rows; r0 += (long long)gridDim.x * RB, buf ^= 1) {
     uint4 v[RB][CPT];
 #pragma unroll
@@ -718,17 +728,20 @@ arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, u
       if (c < nchunks) *reinterpret_cast<uint4*>(s_col + 4 * c) = make_uint4(cmax[j][0], cmax[j][1], cmax[j][2], cmax[j][3]);
     }
     cluster.sync();
-    const int rank = (int)cluster.block_rank();
     const uint32_t* peers[CALIB_CLUSTER];
 #pragma unroll
     for (int q = 0; q < CALIB_CLUSTER; ++q) peers[q] = cluster.map_shared_rank(s_col, q);
-    for (int w = rank * CALIB_THREADS + tid; w < (K >> 1); w += CALIB_CLUSTER * CALIB_THREADS) {
+    for (int w = (int)cluster.block_rank() * CALIB_THREADS + tid; w < (K >> 1); w += CALIB_CLUSTER * CALIB_THREADS) {
       uint32_t m = 0;
 #pragma unroll
       for (int q = 0; q < CALIB_CLUSTER; ++q) asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(peers[q][w]));
       // (non-negative floats order like their bit patterns; a stale value read here only costs an atomic)
-      if ((m << 16) > __ldcg(chan_absmax + 2 * w)) atomicMax(chan_absmax + 2 * w, m << 16);
-      if ((m & 0xffff0000u) > __ldcg(chan_absmax + 2 * w + 1)) atomicMax(chan_absmax + 2 * w + 1, m & 0xffff0000u);
+      if (!EARLY || w != w_early) {
+        run0 = __ldcg(chan_absmax + 2 * w);
+        run1 = __ldcg(chan_absmax + 2 * w + 1);
+      }
+      if ((m << 16) > run0) atomicMax(chan_absmax + 2 * w, m << 16);
+      if ((m & 0xffff0000u) > run1) atomicMax(chan_absmax + 2 * w + 1, m & 0xffff0000u);
     }
   }
   if (above != nullptr) {

@@ -912,13 +912,15 @@ static bool use_skinny_kernel(int64_t M, int64_t N, int64_t K_eff, int num_sms, 
   return M <= ARCQ_SKINNY_ROWS || (((M + 127) / 128) * ((N + 127) / 128) <= num_sms && (residual || skinny_plan_splits(M, N, K_eff) > 1));
 }
 // With the SwiGLU epilogue (gate and up blocks in different CTAs of a cluster), us, this kernel at 65 and at 128 rows / CTA
-// pairs at 129: [2048, 2176] 10.3 and 12.2 / 14.3, [3584, 4224] 12.2 and 12.4 / 16.5, [7168, 4224] 14.4 and 17.0 / 18.5, [14336,
-// 4224] 16.9 and 19.6 / 18.6, [28672, 4224] 22.6 and 24.6 / 28.7, [57344, 8320] 62.0 and 69.8 / 82.5.  At 200 rows CTA pairs are
-// the better ones ([28672, 4224] 43.1 / 31.6).
+// pairs at 129: [2048, 2176] 10.9 and 11.0 / 13.1, [3584, 4224] 11.2 and 12.9 / 15.5, [7168, 4224] 15.2 and 17.2 / 15.5, [14336,
+// 4224] 14.9 and 18.9 / 14.9, [28672, 4224] 18.8 and 21.3 / 23.1, [57344, 8320] 60.0 and 64.6 / 68.2.  So CTA pairs from 81 rows
+// where their tiles are one wave of at least a third of the pairs (96 rows of [14336, 4224] 17.0 / 14.9, of [7168, 4224] 15.9 / 15.5), and
+// beyond 128 rows everywhere.
 constexpr int64_t SKINNY_GATED_ROWS = 128;
 // (At least two CTAs per 256 columns and 128 rows: under an SM limit only where that many may run, see arcq_set_sm_limit.)
 static bool use_skinny_gated(int64_t M, int64_t N, const DeviceInfo& di) {
-  const int64_t ctas = 2 * (N / 256) * ((M + 127) / 128);
+  const int64_t tiles = N / 256, ctas = 2 * tiles * ((M + 127) / 128);
+  if (M > 80 && 6 * tiles >= di.num_sms && 2 * tiles <= di.num_sms) return false;
   return M <= SKINNY_GATED_ROWS && (di.num_sms == di.all_sms || ctas <= di.num_sms);
 }
 

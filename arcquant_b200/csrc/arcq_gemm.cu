@@ -754,25 +754,6 @@ int make_c_map(CUtensorMap* map, const void* ptr, int64_t M, int64_t N) {
   return ARCQ_OK;
 }
 
-// Launch as a programmatic dependent of the kernel before (but see early_start): the grid may be set up while that one drains, and waits itself
-// (griddepcontrol.wait) before it touches global memory.
-template <typename... Params, typename... Args>
-int launch_dependent(void (*kern)(Params...), unsigned grid, unsigned threads, size_t smem, const DeviceInfo& di, cudaStream_t stream,
-                     const Args&... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = di.early_start();
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, args...));
-  return ARCQ_OK;
-}
-
 // ngroups > 1: B and SFB hold `ngroups` matrices of N rows each, tile_group says which one every
 // 256-row tile of A multiplies (see Gemm2Params).
 // swiglu_amax != nullptr: SwiGLU epilogue (see Gemm2Params), C is [M, N/2]; groups: the run table of a grouped
@@ -811,8 +792,8 @@ int launch_pair(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const ui
   p.tile_group = tile_group;
   CUtensorMap ma, mb, msa, msb;
   OutputMaps mc;
-  if (swiglu_amax != nullptr) ARCQ_CUDA_TRY(cudaMemsetAsync(swiglu_amax, 0, sizeof(float) * ngroups, stream));
-  int rc = ARCQ_OK;
+  int rc = swiglu_amax != nullptr ? launch_clear(swiglu_amax, ngroups, stream) : ARCQ_OK;
+  if (rc != ARCQ_OK) return rc;
   if (ndests > 0) {
     for (int d = 0; d < ndests && rc == ARCQ_OK; ++d) rc = make_c_map(&mc.m[d], dests[d], M / ndests, N);
     for (int d = ndests; d < MAX_DESTS; ++d) mc.m[d] = mc.m[0];

@@ -50,6 +50,25 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n.reg .pred P;\nelect.sync _|P, 0xffffffff;\nselp.u32 %0, 1, 0, P;\n}" : "=r"(p));
   return p != 0;
 }
+
+// Launch as a programmatic dependent of the kernel before (but see early_start): the grid may be set up while that one drains, and waits itself
+// (griddepcontrol.wait) before it touches global memory.
+template <typename... Params, typename... Args>
+int launch_dependent(void (*kern)(Params...), unsigned grid, unsigned threads, size_t smem, const DeviceInfo& di, cudaStream_t stream,
+                     const Args&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = di.early_start();
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, args...));
+  return ARCQ_OK;
+}
 #endif
 
 // Launchers (defined in arcq_quant.cu / arcq_gemm.cu); arguments are validated by the callers
@@ -66,6 +85,8 @@ int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight
                                  int KE, int mode, uint8_t* q, uint8_t* sf, float* scale_out, float* scratch,
                                  cudaStream_t stream, const int* groups = nullptr, int ngroups = 0,
                                  const int* row_map = nullptr);
+// n floats (at most 64) to zero, as a programmatic dependent: a memset breaks the chain of kernels that are set up early.
+int launch_clear(float* p, int n, cudaStream_t stream);
 int launch_absmax(const void* x, int64_t n, float* out, int accumulate, cudaStream_t stream);
 int launch_gemm(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,
                 int64_t N, int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, void* C,

@@ -39,8 +39,10 @@ __device__ __forceinline__ uint32_t gt_mask_bf16x2(uint32_t a, uint32_t b) {   /
 // x: [tokens, row_elems] bf16; the first `heads` heads of `dim` elements of each row are rotated:
 // out[d] = x[d] * cos[d] - x[d + dim/2] * sin[d],  out[d + dim/2] = x[d + dim/2] * cos[..] + x[d] * sin[..]
 // (rotate-half convention), cos/sin: [seq, dim] fp32 indexed by token % seq.  One thread = 8 + 8 elements.
-__global__ void arcq_rope_kernel(uint16_t* __restrict__ x, const float* __restrict__ cs, const float* __restrict__ sn,
+__global__ void arcq_rope_kernel(uint16_t* __restrict__ x, const float* cs, const float* sn,
                                  long long tokens, int row_elems, int heads, int dim, int seq) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int half = dim >> 1, per_head = half >> 3;
   const long long total = tokens * heads * per_head;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -258,12 +260,23 @@ arcq_silu_mul_grouped_kernel(const uint16_t* __restrict__ gu, uint16_t* __restri
   flush();
 }
 
+// What the next launch collects maxima in, cleared inside the chain of programmatic dependents.  A memset there ended the chain: the
+// kernel behind it was set up, and its first weight tiles asked for, only when it was done (SwiGLU [28672, 4224] by weight
+// streaming, call after call, us, memset / this: 1 row 18.6 / 14.5, 16 rows 19.9 / 15.2, 64 rows 22.0 / 17.9).
+__global__ void arcq_clear_kernel(float* p, int n) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if ((int)threadIdx.x < n) p[threadIdx.x] = 0.f;
+}
+
 // out[t] = sum over the k routed copies of token t of bf16(y[pos[t][j]] * w[t][j]), accumulated in the
 // output type in the order j = 0..k-1 (a bf16 index_add over the copies adds them in bf16 as well; with
 // k = 2 the order does not matter).  One thread = 8 channels of one token.
-__global__ void arcq_moe_combine_kernel(const uint16_t* __restrict__ y, const int* __restrict__ pos,
-                                        const uint16_t* __restrict__ w, uint16_t* __restrict__ out, long long tokens,
+__global__ void arcq_moe_combine_kernel(const uint16_t* y, const int* pos,
+                                        const uint16_t* w, uint16_t* __restrict__ out, long long tokens,
                                         int hidden, int k) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int vec_per_row = hidden >> 3;
   const long long total = tokens * vec_per_row;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
@@ -368,19 +381,21 @@ __global__ void arcq_peer_barrier_kernel(const PeerFlags f, int rank, int world,
 
 // Per-run max|x| of grouped rows: run e holds rows [groups[e], groups[e] + groups[ngroups + e]) of the
 // (padded) row numbering; row r of that numbering is input row row_map[r] (or r).  One warp per row.
-__global__ void arcq_absmax_grouped_kernel(const uint16_t* __restrict__ x, const int* __restrict__ row_map,
-                                           const int* __restrict__ groups, int ngroups, int K, unsigned int* out) {
+__global__ void arcq_absmax_grouped_kernel(const uint16_t* x, const int* row_map,
+                                           const int* groups, int ngroups, int K, unsigned int* out) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
-  const int last = __ldg(groups + ngroups - 1) + __ldg(groups + 2 * ngroups - 1);   // end of the last run
+  const int last = groups[ngroups - 1] + groups[2 * ngroups - 1];   // end of the last run
   int e = 0;
   for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < last; r += warps) {
-    while (e + 1 < ngroups && r >= __ldg(groups + e + 1)) ++e;
-    if (r >= __ldg(groups + e) + __ldg(groups + ngroups + e)) continue;        // padding between runs
-    const uint4* row = reinterpret_cast<const uint4*>(x + (size_t)(row_map ? __ldg(row_map + r) : r) * (size_t)K);
+    while (e + 1 < ngroups && r >= groups[e + 1]) ++e;
+    if (r >= groups[e] + groups[ngroups + e]) continue;        // padding between runs
+    const uint4* row = reinterpret_cast<const uint4*>(x + (size_t)(row_map ? row_map[r] : r) * (size_t)K);
     uint32_t m = 0;
     for (int v = lane; v < (K >> 3); v += 32) {
-      const uint4 a = __ldg(row + v);
+      const uint4 a = __ldcg(row + v);
       asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(a.x & 0x7fff7fffu));
       asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(a.y & 0x7fff7fffu));
       asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(a.z & 0x7fff7fffu));
@@ -404,9 +419,11 @@ __global__ void arcq_absmax_grouped_kernel(const uint16_t* __restrict__ x, const
 // runs and 71 us for
 // 8192; this takes 4.1 and 9.5.
 __global__ void __launch_bounds__(1024, 1)
-arcq_moe_layout_kernel(const long long* __restrict__ slot_group, int n, int ngroups, int tile, int rows_bound, int div,
+arcq_moe_layout_kernel(const long long* slot_group, int n, int ngroups, int tile, int rows_bound, int div,
                        int* __restrict__ dest, int* __restrict__ row_map, int* __restrict__ groups,
                        int* __restrict__ tile_group) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   constexpr int BATCH = 8;
   __shared__ int s_hist[32][65], s_cnt[64], s_off[64];     // (65: a column is read by 32 lanes)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -493,8 +510,10 @@ arcq_moe_layout_kernel(const long long* __restrict__ slot_group, int n, int ngro
 // token; sums in the order of a butterfly over them.  Bound: launches - softmax, top-k, its sort, the sum, the division
 // and the cast as torch operations were seven launches, 21 us of kernels for 37 tokens and 29 us for 4096; this
 // kernel takes 2.8 and 2.6.
-__global__ void arcq_route_topk_kernel(const uint16_t* __restrict__ logits, long long tokens, int experts, int width, int top_k,
+__global__ void arcq_route_topk_kernel(const uint16_t* logits, long long tokens, int experts, int width, int top_k,
                                        long long* __restrict__ ids, uint16_t* __restrict__ weights) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int per_warp = 32 / width, lane = threadIdx.x & 31, sub = lane & (width - 1);
   const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
   for (long long t0 = ((blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5) * per_warp; t0 < tokens; t0 += warps * per_warp) {
@@ -865,6 +884,17 @@ int launch_calib_stats(const void* x, int64_t rows, int K, float* chan_absmax, u
   return ARCQ_ERR_UNSUPPORTED_K;
 }
 
+int launch_clear(float* p, int n, cudaStream_t stream) {
+  if (n > 64) {
+    ARCQ_CUDA_TRY(cudaMemsetAsync(p, 0, sizeof(float) * n, stream));
+    return ARCQ_OK;
+  }
+  DeviceInfo di;
+  int rc = get_device_info(&di);
+  if (rc != ARCQ_OK) return rc;
+  return launch_dependent(arcq_clear_kernel, 1, 64, 0, di, stream, p, n);
+}
+
 int launch_ep_send_layout(const long long* ids, int n, int e_local, int ep, int cap, int rank, int* slot,
                           void* const* meta, int* overflow, cudaStream_t stream) {
   PeerPtrs m = {};
@@ -893,10 +923,11 @@ int launch_ep_rows(const void* src, const int* item_src, int div, int src_limit,
 
 int launch_moe_layout(const long long* slot_group, int n, int ngroups, int tile, int rows_bound, int div, int* dest,
                       int* row_map, int* groups, int* tile_group, cudaStream_t stream) {
-  arcq_moe_layout_kernel<<<1, 1024, 0, stream>>>(slot_group, n, ngroups, tile, rows_bound, div, dest, row_map, groups,
-                                                 tile_group);
-  ARCQ_CUDA_TRY(cudaGetLastError());
-  return ARCQ_OK;
+  DeviceInfo di;
+  int rc = get_device_info(&di);
+  if (rc != ARCQ_OK) return rc;
+  return launch_dependent(arcq_moe_layout_kernel, 1, 1024, 0, di, stream, slot_group, n, ngroups, tile, rows_bound, div, dest,
+                          row_map, groups, tile_group);
 }
 
 int launch_route_topk(const void* logits, int64_t tokens, int experts, int top_k, long long* ids, void* weights,
@@ -910,22 +941,18 @@ int launch_route_topk(const void* logits, int64_t tokens, int experts, int top_k
   const long long per_block = 4 * (32 / width);            // four warps
   long long blocks = (tokens + per_block - 1) / per_block;
   if (blocks > (long long)di.num_sms * 16) blocks = (long long)di.num_sms * 16;
-  arcq_route_topk_kernel<<<(unsigned)blocks, 128, 0, stream>>>(static_cast<const uint16_t*>(logits), tokens, experts, width, top_k,
-                                                               ids, static_cast<uint16_t*>(weights));
-  ARCQ_CUDA_TRY(cudaGetLastError());
-  return ARCQ_OK;
+  return launch_dependent(arcq_route_topk_kernel, (unsigned)blocks, 128, 0, di, stream, static_cast<const uint16_t*>(logits),
+                          (long long)tokens, experts, width, top_k, ids, static_cast<uint16_t*>(weights));
 }
 
 int launch_absmax_grouped(const void* x, const int* row_map, const int* groups, int ngroups, int K, float* out,
                           cudaStream_t stream) {
-  ARCQ_CUDA_TRY(cudaMemsetAsync(out, 0, sizeof(float) * ngroups, stream));
   DeviceInfo di;
   int rc = get_device_info(&di);
+  if (rc == ARCQ_OK) rc = launch_clear(out, ngroups, stream);
   if (rc != ARCQ_OK) return rc;
-  arcq_absmax_grouped_kernel<<<(unsigned)di.num_sms * 8, 256, 0, stream>>>(
-      static_cast<const uint16_t*>(x), row_map, groups, ngroups, K, reinterpret_cast<unsigned int*>(out));
-  ARCQ_CUDA_TRY(cudaGetLastError());
-  return ARCQ_OK;
+  return launch_dependent(arcq_absmax_grouped_kernel, (unsigned)di.num_sms * 8, 256, 0, di, stream, static_cast<const uint16_t*>(x),
+                          row_map, groups, ngroups, K, reinterpret_cast<unsigned int*>(out));
 }
 
 int launch_moe_combine(const void* y, const int* pos, const void* w, void* out, int64_t tokens, int hidden, int k,
@@ -938,11 +965,8 @@ int launch_moe_combine(const void* y, const int* pos, const void* w, void* out, 
   long long blocks = (total + 255) / 256;
   const long long cap = (long long)di.num_sms * 16;
   if (blocks > cap) blocks = cap;
-  arcq_moe_combine_kernel<<<(unsigned)blocks, 256, 0, stream>>>(static_cast<const uint16_t*>(y), pos,
-                                                                static_cast<const uint16_t*>(w),
-                                                                static_cast<uint16_t*>(out), tokens, hidden, k);
-  ARCQ_CUDA_TRY(cudaGetLastError());
-  return ARCQ_OK;
+  return launch_dependent(arcq_moe_combine_kernel, (unsigned)blocks, 256, 0, di, stream, static_cast<const uint16_t*>(y), pos,
+                          static_cast<const uint16_t*>(w), static_cast<uint16_t*>(out), (long long)tokens, hidden, k);
 }
 
 static std::atomic<long long> g_peer_wait_limit_ms{10000};
@@ -996,10 +1020,8 @@ int launch_rope(void* x, const float* cos_t, const float* sin_t, int64_t tokens,
   long long blocks = (total + 255) / 256;
   const long long cap = (long long)di.num_sms * 16;
   if (blocks > cap) blocks = cap;
-  arcq_rope_kernel<<<(unsigned)blocks, 256, 0, stream>>>(static_cast<uint16_t*>(x), cos_t, sin_t, tokens, row_elems, heads,
-                                                         dim, seq);
-  ARCQ_CUDA_TRY(cudaGetLastError());
-  return ARCQ_OK;
+  return launch_dependent(arcq_rope_kernel, (unsigned)blocks, 256, 0, di, stream, static_cast<uint16_t*>(x), cos_t, sin_t,
+                          (long long)tokens, row_elems, heads, dim, seq);
 }
 
 int launch_silu_mul_grouped(const void* gu, void* out, int64_t rows, int F, const int* tile_group, const int* groups,

@@ -12,6 +12,7 @@
 #include <math.h>
 #include <stdlib.h>
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 
@@ -638,40 +639,44 @@ __global__ void arcq_ep_rows_kernel(const uint4* __restrict__ src, const int* __
 // per-channel running max|x| and the number of elements larger than an eighth of their row's (signed)
 // maximum.  Thread t of a CTA owns the 16-byte chunks t, t + 512, ... of every row it meets, so its channels'
 // maxima stay in registers; RB rows are in flight together, so that one barrier serves their RB row maxima.
-// Bound: HBM in principle (2 bytes per element); what set the time was the channel maxima's way out.  One
-// atomic per channel and CTA, 4.85 million on 4096 addresses at [2000, 4096], took 184 us of which the data
-// needs 3.  Here the CTAs of a cluster of eight reduce their maxima through distributed shared memory, and an
-// eighth of the CTAs' worth of results meets the running maxima, with an atomic only where a larger value was
-// found.
+// Bound: HBM in principle (2 bytes per element, 2.5 us of [2000, 4096]); what sets the time is a chain of batches that are
+// a wave of CTAs each: start, first bytes, way out of the maxima.
+//  * While the batch before is finishing, every CTA pulls its first rows into L2 (a prefetch reads nothing into the CTA, so rows still
+//    being written are not read early).
+//  * The running maxima come into shared memory beside the rows.  A channel meets them in a thread that owns neighbouring ones, and only a
+//    larger value costs an atomic: all of a CTA's in the first batch, few afterwards.  (In the order of the chunks an atomic instruction
+//    touched 32 sectors, 184 us for 4.85 million; clusters of eight that reduced their maxima through distributed shared memory first
+//    spent more on meeting than on the atomics saved.)
+// us, clusters of eight / this: 16 batches of [2000, 4096] in turn 146 / 112, of [200, 4096] 85 / 66, of [1500, 5120] 185 / 125, of
+// [2000, 8192] 219 / 156; one of [2000, 4096] 13.3 / 13.3, of [2000, 8192] 19 / 22, of [20000, 4096] 73 / 46.
+// OUT_CLUSTER: rows of more than 8192 channels still meet in clusters first, their first batch being too many atomics otherwise (four
+// batches, clusters / staged: [500, 16384] 37.9 / 41.0, [300, 28672] 61.5 / 74.8; eight of [2000, 14336] 187 / 140).
+// OUT_DIRECT: a handful of rows, whose maxima go out as they are.
 constexpr int CALIB_THREADS = 512, CALIB_CLUSTER = 8;
-template <int CPT, int RB, bool CLUSTER = true>
+enum { OUT_DIRECT, OUT_STAGED, OUT_CLUSTER };
+template <int CPT, int RB, int OUT>
 __global__ void __launch_bounds__(CALIB_THREADS, CPT * RB > 8 ? 1 : 2)
 arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, unsigned int* chan_absmax,
                         unsigned long long* above) {
   constexpr int WARPS = CALIB_THREADS / 32;
-  extern __shared__ __align__(16) uint32_t s_col[];           // [K/2]: this CTA's channel maxima, two per word
+  extern __shared__ __align__(16) uint32_t s_col[];           // [K/2]: this CTA's channel maxima, two per word; staged [K]: the running ones
   __shared__ uint32_t s_max[2][WARPS][RB / 2];
-  namespace cg = cooperative_groups;
-  const cg::cluster_group cluster = cg::this_cluster();
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nchunks = K >> 3;
+  uint32_t* s_run = s_col + (K >> 1);
+  const bool aligned = (reinterpret_cast<uintptr_t>(chan_absmax) & 15u) == 0;   // (else the running maxima are read in place)
   asm volatile("griddepcontrol.launch_dependents;");
+  if (OUT == OUT_STAGED && tid == 0) {
+    const long long r0 = (long long)blockIdx.x * RB;
+    const long long bytes = min((long long)RB, rows - r0) * K * 2;
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(x + r0 * (long long)K), "r"((uint32_t)bytes) : "memory");
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   uint32_t cmax[CPT][4];
 #pragma unroll
   for (int j = 0; j < CPT; ++j) cmax[j][0] = cmax[j][1] = cmax[j][2] = cmax[j][3] = 0;
-  unsigned long long count = 0;
+  unsigned int count = 0;
   int buf = 0;
-  // The running maxima that this thread's first word will meet are asked for now, so that their latency is not behind the
-  // cluster's meeting (a value that is stale by then only costs an atomic): 2000 x 4096 10.0 -> 9.1 us, 300 x 4096 6.5 -> 5.5.  With
-  // two chunks per thread the registers are not there (1500 x 5120 11.6 -> 12.3).
-  constexpr bool EARLY = CLUSTER && CPT == 1;
-  uint32_t run0 = 0, run1 = 0;
-  const int w_early = EARLY ? (int)cluster.block_rank() * CALIB_THREADS + tid : 0;
-  if (EARLY && w_early < (K >> 1)) {
-    run0 = __ldcg(chan_absmax + 2 * w_early);
-    run1 = __ldcg(chan_absmax + 2 * w_early + 1);
-  }
   for (long long r0 = (long long)blockIdx.x * RB; r0 < rows; r0 += (long long)gridDim.x * RB, buf ^= 1) {
     uint4 v[RB][CPT];
 #pragma unroll
@@ -682,6 +687,11 @@ arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, u
         v[i][j] = make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);   // -inf: never above, never a maximum
         if (c < nchunks && r0 + i < rows) v[i][j] = __ldcs(reinterpret_cast<const uint4*>(x + (r0 + i) * (long long)K) + c);
       }
+    }
+    if (OUT == OUT_STAGED && aligned && r0 == (long long)blockIdx.x * RB) {
+      const uint32_t to = (uint32_t)__cvta_generic_to_shared(s_run);
+      for (int j = tid; j < (K >> 2); j += CALIB_THREADS)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 16u * j), "l"(chan_absmax + 4 * j) : "memory");
     }
     uint32_t m[RB / 2];                                        // (row 2i, row 2i + 1): signed maxima
 #pragma unroll
@@ -725,10 +735,9 @@ arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, u
         for (int k = 0; k < 4; ++k) above16 += __popc(gt_mask_bf16x2(wa[k], ta)) + __popc(gt_mask_bf16x2(wb[k], tb));
       }
     }
-    count += (unsigned long long)(above16 >> 4);
+    count += (unsigned int)(above16 >> 4);
   }
-  if constexpr (!CLUSTER) {
-    // a handful of rows: nothing to reduce on chip first
+  if constexpr (OUT == OUT_DIRECT) {
 #pragma unroll
     for (int j = 0; j < CPT; ++j) {
       const int c = tid + j * CALIB_THREADS;
@@ -746,36 +755,47 @@ arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, u
       const int c = tid + j * CALIB_THREADS;
       if (c < nchunks) *reinterpret_cast<uint4*>(s_col + 4 * c) = make_uint4(cmax[j][0], cmax[j][1], cmax[j][2], cmax[j][3]);
     }
-    cluster.sync();
-    const uint32_t* peers[CALIB_CLUSTER];
-#pragma unroll
-    for (int q = 0; q < CALIB_CLUSTER; ++q) peers[q] = cluster.map_shared_rank(s_col, q);
-    for (int w = (int)cluster.block_rank() * CALIB_THREADS + tid; w < (K >> 1); w += CALIB_CLUSTER * CALIB_THREADS) {
-      uint32_t m = 0;
-#pragma unroll
-      for (int q = 0; q < CALIB_CLUSTER; ++q) asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(peers[q][w]));
-      // (non-negative floats order like their bit patterns; a stale value read here only costs an atomic)
-      if (!EARLY || w != w_early) {
-        run0 = __ldcg(chan_absmax + 2 * w);
-        run1 = __ldcg(chan_absmax + 2 * w + 1);
-      }
+    // (non-negative floats order like their bit patterns; a running maximum that is stale by now only costs an atomic)
+    auto meet = [&](int w, uint32_t m, uint32_t run0, uint32_t run1) {
       if ((m << 16) > run0) atomicMax(chan_absmax + 2 * w, m << 16);
       if ((m & 0xffff0000u) > run1) atomicMax(chan_absmax + 2 * w + 1, m & 0xffff0000u);
+    };
+    if constexpr (OUT == OUT_STAGED) {
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();
+      for (int w = tid; w < (K >> 1); w += CALIB_THREADS) {
+        const uint2 run = aligned ? *reinterpret_cast<const uint2*>(s_run + 2 * w) : make_uint2(__ldcg(chan_absmax + 2 * w), __ldcg(chan_absmax + 2 * w + 1));
+        meet(w, s_col[w], run.x, run.y);
+      }
+    } else {
+      namespace cg = cooperative_groups;
+      const cg::cluster_group cluster = cg::this_cluster();
+      cluster.sync();
+      const uint32_t* peers[CALIB_CLUSTER];
+#pragma unroll
+      for (int q = 0; q < CALIB_CLUSTER; ++q) peers[q] = cluster.map_shared_rank(s_col, q);
+      for (int w = (int)cluster.block_rank() * CALIB_THREADS + tid; w < (K >> 1); w += CALIB_CLUSTER * CALIB_THREADS) {
+        uint32_t m = 0;
+#pragma unroll
+        for (int q = 0; q < CALIB_CLUSTER; ++q) asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(peers[q][w]));
+        meet(w, m, __ldcg(chan_absmax + 2 * w), __ldcg(chan_absmax + 2 * w + 1));
+      }
+      cluster.sync();                                          // nobody leaves while its maxima are being read
     }
   }
   if (above != nullptr) {
+    unsigned long long t = count;
 #pragma unroll
-    for (int d = 16; d > 0; d >>= 1) count += __shfl_xor_sync(0xffffffffu, count, d);
+    for (int d = 16; d > 0; d >>= 1) t += __shfl_xor_sync(0xffffffffu, t, d);
     __shared__ unsigned long long s_count[WARPS];
-    if (lane == 0) s_count[warp] = count;
+    if (lane == 0) s_count[warp] = t;
     __syncthreads();
     if (tid == 0) {
-      unsigned long long t = 0;
+      t = 0;
       for (int k = 0; k < WARPS; ++k) t += s_count[k];
       if (t) atomicAdd(above, t);
     }
   }
-  if constexpr (CLUSTER) cluster.sync();                       // nobody leaves while its maxima are being read
 }
 
 // Channel order of K statistics: ascending, equal values in order of their channels (a stable sort; NaN last).  A channel's
@@ -849,14 +869,15 @@ int launch_calib_stats(const void* x, int64_t rows, int K, float* chan_absmax, u
   const int cpt = (K / 8 + CALIB_THREADS - 1) / CALIB_THREADS;
   auto xs = static_cast<const uint16_t*>(x);
   auto cm = reinterpret_cast<unsigned int*>(chan_absmax);
-  auto launch = [&](auto kern, int rb, int csize = CALIB_CLUSTER) -> int {
-    const size_t smem = (size_t)K * 2;
+  auto launch = [&](auto kern, int rb, int out) -> int {
+    const size_t smem = out == OUT_DIRECT ? 0 : (size_t)K * (out == OUT_STAGED ? 6 : 2);
     // Unasked, a launch gets 48 KB, its static part (below 1 KB here) included.  The limit is the kernel's, not this call's:
     // always the same value, so that calls of several threads and widths cannot lower one another's.
     if (smem > 47 * 1024) ARCQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 32768));
     long long grid = (rows + rb - 1) / rb;
-    if (grid > 2LL * di.num_sms) grid = 2LL * di.num_sms;
-    grid = (grid + csize - 1) / csize * csize;
+    if (out != OUT_CLUSTER)
+      return launch_dependent(kern, (unsigned)std::min(grid, di.resident(2)), CALIB_THREADS, smem, di, stream, xs, (long long)rows, K, cm, above);
+    grid = (std::min(grid, 2LL * di.num_sms) + CALIB_CLUSTER - 1) / CALIB_CLUSTER * CALIB_CLUSTER;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3(CALIB_THREADS);
@@ -866,21 +887,21 @@ int launch_calib_stats(const void* x, int64_t rows, int K, float* chan_absmax, u
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = di.early_start();
     attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = (unsigned)csize;
+    attr[1].val.clusterDim.x = CALIB_CLUSTER;
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = csize > 1 ? 2 : 1;
+    cfg.numAttrs = 2;
     ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, xs, (long long)rows, K, cm, above));
     return ARCQ_OK;
   };
-  // Up to 64 rows of up to 4096 channels are one step of a few small CTAs, which a cluster's barriers and its look at the
-  // running maxima would only lengthen (2048 channels: 7 rows 5.5 -> 2.5 us, 40 rows 5.3 -> 3.4).
-  if (cpt <= 1 && rows <= 64) return launch(arcq_calib_stats_kernel<1, 2, false>, 2, 1);
+  // Up to 64 rows of up to 4096 channels are one step of a few small CTAs, which a look at the running maxima would only lengthen
+  // (2048 channels, with clusters / direct: 7 rows 5.5 / 2.5 us, 40 rows 5.3 / 3.4).
+  if (cpt <= 1 && rows <= 64) return launch(arcq_calib_stats_kernel<1, 2, OUT_DIRECT>, 2, OUT_DIRECT);
   // (rows in flight per CTA: eight 16-byte loads per thread, two rows at least)
-  if (cpt <= 1) return launch(arcq_calib_stats_kernel<1, 8>, 8);
-  if (cpt <= 2) return launch(arcq_calib_stats_kernel<2, 4>, 4);
-  if (cpt <= 4) return launch(arcq_calib_stats_kernel<4, 2>, 2);
-  if (cpt <= 8) return launch(arcq_calib_stats_kernel<8, 2>, 2);
+  if (cpt <= 1) return launch(arcq_calib_stats_kernel<1, 8, OUT_STAGED>, 8, OUT_STAGED);
+  if (cpt <= 2) return launch(arcq_calib_stats_kernel<2, 4, OUT_STAGED>, 4, OUT_STAGED);
+  if (cpt <= 4) return launch(arcq_calib_stats_kernel<4, 2, OUT_CLUSTER>, 2, OUT_CLUSTER);
+  if (cpt <= 8) return launch(arcq_calib_stats_kernel<8, 2, OUT_CLUSTER>, 2, OUT_CLUSTER);
   return ARCQ_ERR_UNSUPPORTED_K;
 }
 

@@ -134,30 +134,54 @@ int arcq_quantize_tensor_scale(const void* x, const float* amax, int is_weight, 
                                       (cudaStream_t)stream);
 }
 
-int arcq_quantize_x_grouped_amax(const void* x, const int32_t* row_map, const float* amax, const int16_t* reorder_indices,
-                                 const int32_t* groups, int ngroups, int64_t rows_bound, int KQ, int KE, int mode,
-                                 uint8_t* qx, uint8_t* sfx, float* scale_out, void* stream) {
+int arcq_quantize_x_grouped_amax_clear(const void* x, const int32_t* row_map, const float* amax, const int16_t* reorder_indices,
+                                       const int32_t* groups, int ngroups, int64_t rows_bound, int KQ, int KE, int mode,
+                                       uint8_t* qx, uint8_t* sfx, float* scale_out, float* clear, int nclear, void* stream) {
   int rc = check_quant_shape(rows_bound, KQ, KE, mode);
   if (rc != ARCQ_OK) return rc;
-  if (ngroups < 1 || ngroups > 64) return ARCQ_ERR_BAD_SHAPE;
-  if (rows_bound == 0) return ARCQ_OK;
+  if (ngroups < 1 || ngroups > 64 || nclear < 0 || nclear > 64) return ARCQ_ERR_BAD_SHAPE;
+  if (nclear > 0 && !clear) return ARCQ_ERR_NULL_POINTER;
+  if (rows_bound == 0) {
+    if (nclear > 0) ARCQ_CUDA_TRY(cudaMemsetAsync(clear, 0, sizeof(float) * nclear, (cudaStream_t)stream));
+    return ARCQ_OK;
+  }
   if (!x || !amax || !groups || !qx || !sfx || !scale_out) return ARCQ_ERR_NULL_POINTER;
   if (!aligned16(x) || !aligned16(qx)) return ARCQ_ERR_ALIGNMENT;
   return launch_quantize_tensor_scale(x, amax, 0, reorder_indices, rows_bound, KQ, KE, mode, qx, sfx, scale_out, nullptr,
-                                      (cudaStream_t)stream, groups, ngroups, row_map);
+                                      (cudaStream_t)stream, groups, ngroups, row_map, clear, nclear);
 }
 
-int arcq_rmsnorm_quantize_x(const void* x, const void* gamma, float eps, const int16_t* reorder_index,
-                            int64_t M, int KQ, int KE, uint8_t* qx, uint8_t* sfx, void* stream) {
+int arcq_quantize_x_grouped_amax(const void* x, const int32_t* row_map, const float* amax, const int16_t* reorder_indices,
+                                 const int32_t* groups, int ngroups, int64_t rows_bound, int KQ, int KE, int mode,
+                                 uint8_t* qx, uint8_t* sfx, float* scale_out, void* stream) {
+  return arcq_quantize_x_grouped_amax_clear(x, row_map, amax, reorder_indices, groups, ngroups, rows_bound, KQ, KE, mode, qx, sfx,
+                                            scale_out, nullptr, 0, stream);
+}
+
+int arcq_rmsnorm_quantize_x_clear(const void* x, const void* gamma, float eps, const int16_t* reorder_index,
+                                  int64_t M, int KQ, int KE, uint8_t* qx, uint8_t* sfx, float* clear, int nclear, void* stream) {
   int rc = check_quant_shape(M, KQ, KE, ARCQ_MODE_16);
   if (rc != ARCQ_OK) return rc;
   int g = KQ / 16;
   if (g % 32 || g < 64 || g > 512) return ARCQ_ERR_UNSUPPORTED_K;
-  if (M == 0) return ARCQ_OK;
+  if (nclear < 0 || nclear > 64) return ARCQ_ERR_BAD_SHAPE;
+  if (nclear > 0 && !clear) return ARCQ_ERR_NULL_POINTER;
+  if (M == 0) {
+    if (nclear > 0) ARCQ_CUDA_TRY(cudaMemsetAsync(clear, 0, sizeof(float) * nclear, (cudaStream_t)stream));
+    return ARCQ_OK;
+  }
   if (!x || !gamma || !qx || !sfx) return ARCQ_ERR_NULL_POINTER;
   if (!aligned16(x) || !aligned16(qx)) return ARCQ_ERR_ALIGNMENT;
-  return launch_quantize(x, gamma, eps, reorder_index, M, KQ, KE, ARCQ_MODE_16, 0, qx, sfx,
-                         (cudaStream_t)stream);
+  ScaleOptions so;
+  so.clear = clear;
+  so.nclear = nclear;
+  return launch_quantize(x, gamma, eps, reorder_index, M, KQ, KE, ARCQ_MODE_16, 0, qx, sfx, (cudaStream_t)stream, nullptr, nullptr, 0,
+                         nullptr, nullptr, nullptr, 0, so);
+}
+
+int arcq_rmsnorm_quantize_x(const void* x, const void* gamma, float eps, const int16_t* reorder_index,
+                            int64_t M, int KQ, int KE, uint8_t* qx, uint8_t* sfx, void* stream) {
+  return arcq_rmsnorm_quantize_x_clear(x, gamma, eps, reorder_index, M, KQ, KE, qx, sfx, nullptr, 0, stream);
 }
 
 int arcq_rmsnorm_quantize_x_multi(const void* x, const void* gamma, float eps, const int16_t* reorder_index,
@@ -418,35 +442,55 @@ int arcq_matmul_nvfp4_grouped_runs(const uint8_t* A, const uint8_t* B, const uin
                              (cudaStream_t)stream, nullptr, groups);
 }
 
-int arcq_matmul_nvfp4_swiglu(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,
-                             int64_t N, int64_t K_eff, const float* alpha_a, const float* alpha_b, void* C,
-                             float* amax, void* stream) {
+static int swiglu(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M, int64_t N, int64_t K_eff,
+                  const float* alpha_a, const float* alpha_b, void* C, float* amax, bool clear, void* stream) {
   int rc = check_gemm(A, B, SFA, SFB, M, N, K_eff, C);
   if (rc != ARCQ_OK) return rc;
   if (N % 256) return ARCQ_ERR_BAD_SHAPE;
   if (!alpha_a || !amax) return ARCQ_ERR_NULL_POINTER;
   if (M == 0) {
-    ARCQ_CUDA_TRY(cudaMemsetAsync(amax, 0, sizeof(float), (cudaStream_t)stream));
+    if (clear) ARCQ_CUDA_TRY(cudaMemsetAsync(amax, 0, sizeof(float), (cudaStream_t)stream));
     return ARCQ_OK;
   }
   return launch_gemm_grouped(A, B, SFA, SFB, M, N, K_eff, nullptr, 1, alpha_a, alpha_b, C, (cudaStream_t)stream, amax,
-                             nullptr);
+                             nullptr, clear);
+}
+int arcq_matmul_nvfp4_swiglu(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,
+                             int64_t N, int64_t K_eff, const float* alpha_a, const float* alpha_b, void* C,
+                             float* amax, void* stream) {
+  return swiglu(A, B, SFA, SFB, M, N, K_eff, alpha_a, alpha_b, C, amax, true, stream);
+}
+int arcq_matmul_nvfp4_swiglu_onto(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,
+                                  int64_t N, int64_t K_eff, const float* alpha_a, const float* alpha_b, void* C,
+                                  float* amax, void* stream) {
+  return swiglu(A, B, SFA, SFB, M, N, K_eff, alpha_a, alpha_b, C, amax, false, stream);
 }
 
-int arcq_matmul_nvfp4_grouped_swiglu(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB,
-                                     int64_t M_bound, int64_t N, int64_t K_eff, const int32_t* tile_group,
-                                     const int32_t* groups, int ngroups, const float* alpha_a, const float* alpha_b,
-                                     void* C, float* amax, void* stream) {
+static int grouped_swiglu(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M_bound, int64_t N,
+                          int64_t K_eff, const int32_t* tile_group, const int32_t* groups, int ngroups, const float* alpha_a,
+                          const float* alpha_b, void* C, float* amax, bool clear, void* stream) {
   int rc = check_gemm(A, B, SFA, SFB, M_bound, N, K_eff, C);
   if (rc != ARCQ_OK) return rc;
   if (M_bound == 0) {
-    if (amax && ngroups > 0) ARCQ_CUDA_TRY(cudaMemsetAsync(amax, 0, sizeof(float) * ngroups, (cudaStream_t)stream));
+    if (clear && amax && ngroups > 0) ARCQ_CUDA_TRY(cudaMemsetAsync(amax, 0, sizeof(float) * ngroups, (cudaStream_t)stream));
     return ARCQ_OK;
   }
   if (ngroups < 1 || ngroups > 64 || N % 256 || N * (int64_t)ngroups > ((int64_t)1 << 30)) return ARCQ_ERR_BAD_SHAPE;
   if (!tile_group || !groups || !alpha_a || !amax) return ARCQ_ERR_NULL_POINTER;
   return launch_gemm_grouped(A, B, SFA, SFB, M_bound, N, K_eff, tile_group, ngroups, alpha_a, alpha_b, C,
-                             (cudaStream_t)stream, amax, groups);
+                             (cudaStream_t)stream, amax, groups, clear);
+}
+int arcq_matmul_nvfp4_grouped_swiglu(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB,
+                                     int64_t M_bound, int64_t N, int64_t K_eff, const int32_t* tile_group,
+                                     const int32_t* groups, int ngroups, const float* alpha_a, const float* alpha_b,
+                                     void* C, float* amax, void* stream) {
+  return grouped_swiglu(A, B, SFA, SFB, M_bound, N, K_eff, tile_group, groups, ngroups, alpha_a, alpha_b, C, amax, true, stream);
+}
+int arcq_matmul_nvfp4_grouped_swiglu_onto(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB,
+                                          int64_t M_bound, int64_t N, int64_t K_eff, const int32_t* tile_group,
+                                          const int32_t* groups, int ngroups, const float* alpha_a, const float* alpha_b,
+                                          void* C, float* amax, void* stream) {
+  return grouped_swiglu(A, B, SFA, SFB, M_bound, N, K_eff, tile_group, groups, ngroups, alpha_a, alpha_b, C, amax, false, stream);
 }
 
 int arcq_matmul_nvfp4_residual(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,

@@ -792,8 +792,7 @@ int launch_pair(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const ui
   p.tile_group = tile_group;
   CUtensorMap ma, mb, msa, msb;
   OutputMaps mc;
-  int rc = swiglu_amax != nullptr ? launch_clear(swiglu_amax, ngroups, stream) : ARCQ_OK;
-  if (rc != ARCQ_OK) return rc;
+  int rc = ARCQ_OK;
   if (ndests > 0) {
     for (int d = 0; d < ndests && rc == ARCQ_OK; ++d) rc = make_c_map(&mc.m[d], dests[d], M / ndests, N);
     for (int d = ndests; d < MAX_DESTS; ++d) mc.m[d] = mc.m[0];
@@ -936,10 +935,11 @@ static bool use_skinny_gated(int64_t M, int64_t N, const DeviceInfo& di) {
 
 int launch_gemm_grouped(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,
                         int64_t N, int64_t K_eff, const int* tile_group, int ngroups, const float* alpha_a,
-                        const float* alpha_b, void* Cout, cudaStream_t stream, float* swiglu_amax, const int* groups) {
+                        const float* alpha_b, void* Cout, cudaStream_t stream, float* swiglu_amax, const int* groups, bool clear_amax) {
   DeviceInfo di;
   int rc = get_device_info(&di);
   if (rc != ARCQ_OK) return rc;
+  if (swiglu_amax != nullptr && clear_amax) ARCQ_CUDA_TRY(cudaMemsetAsync(swiglu_amax, 0, sizeof(float) * ngroups, stream));
   GemmParams p = {};
   p.c = static_cast<__nv_bfloat16*>(Cout);
   p.alpha_a = alpha_a;

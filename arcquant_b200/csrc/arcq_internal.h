@@ -38,6 +38,12 @@ struct ScaleOptions {
   float factor = 1.0f;
   float* out = nullptr;
   int npartials = 0;
+  // nclear floats (at most 64) that the quantizer sets to zero by the way, for the launch behind it to collect maxima in.  A memset between
+  // the two ends the chain of programmatic dependents: the GEMM is set up, and its first weight tiles asked for, only when it is done
+  // (SwiGLU [28672, 4224] by weight streaming, call after call, us, with a memset / without: 1 row 18.6 / 14.5, 16 rows 19.9 / 15.2, 64 rows
+  // 22.0 / 17.9).
+  float* clear = nullptr;
+  int nclear = 0;
 };
 
 #ifdef __CUDACC__
@@ -84,8 +90,8 @@ int launch_quantize(const void* x, const void* gamma, float eps, const int16_t* 
 int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight, const int16_t* idx, int64_t rows, int KQ,
                                  int KE, int mode, uint8_t* q, uint8_t* sf, float* scale_out, float* scratch,
                                  cudaStream_t stream, const int* groups = nullptr, int ngroups = 0,
-                                 const int* row_map = nullptr);
-// n floats (at most 64) to zero, as a programmatic dependent: a memset breaks the chain of kernels that are set up early.
+                                 const int* row_map = nullptr, float* clear = nullptr, int nclear = 0);
+// n floats to zero, as a programmatic dependent (see ScaleOptions::clear).
 int launch_clear(float* p, int n, cudaStream_t stream);
 int launch_absmax(const void* x, int64_t n, float* out, int accumulate, cudaStream_t stream);
 int launch_gemm(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,
@@ -112,7 +118,8 @@ int launch_gemm_grouped(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, 
                         // SwiGLU epilogue: C is [M, N/2], swiglu_amax[ngroups] takes max|C| per matrix; tile_group
                         // may be null with ngroups 1 (one matrix); groups: run table of a grouped problem (where
                         // it is known, few rows per matrix take the weight-streaming kernel)
-                        float* swiglu_amax = nullptr, const int* groups = nullptr);
+                        // clear_amax: zero them first (else the caller has)
+                        float* swiglu_amax = nullptr, const int* groups = nullptr, bool clear_amax = true);
 int launch_absmax_grouped(const void* x, const int* row_map, const int* groups, int ngroups, int K, float* out,
                           cudaStream_t stream);
 int launch_moe_layout(const long long* slot_group, int n, int ngroups, int tile, int rows_bound, int div, int* dest,
@@ -146,7 +153,7 @@ int launch_sum_partials(const void* const* srcs, int n, int64_t elems, const voi
 // Few rows: weight streaming (arcq_skinny.cu).
 int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, const uint8_t* SFW, int64_t M, int64_t N,
                        int64_t K_eff, float alpha, const float* alpha_a, const float* alpha_b, const void* residual, void* C,
-                       float* swiglu_amax, const int* groups, int ngroups, cudaStream_t stream, bool residual_is_bias = false);
+                       float* swiglu_amax, const int* groups, int ngroups, cudaStream_t stream, bool residual_is_bias = false);   // (swiglu_amax: cleared by the caller)
 int skinny_plan_splits(int64_t M, int64_t N, int64_t K_eff);
 int skinny_poll_error();
 int gemm_poll_error();

@@ -1309,6 +1309,8 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
 
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (so.nclear > 0 && blockIdx.x == 0)
+    for (int i = tid; i < so.nclear; i += T) so.clear[i] = 0.f;
 
   // ---- the rows: one run, or `ngroups` runs (units of R rows are counted through all of them)
   // Lane l of every warp holds runs l and l + 32 (at most 64): first row, rows, and the units up to and including the run,
@@ -1881,6 +1883,10 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
 #undef ARCQ_ROWS
   }
 
+  // (Only the row kernel clears by the way.  In the kernels below it cost registers that are all in use, and what is gained by it is
+  // small beside their time.)
+  if (so.nclear > 0) ARCQ_CUDA_TRY(cudaMemsetAsync(so.clear, 0, sizeof(float) * so.nclear, stream));
+
   // Warp-specialised kernel: rows of 512..8192 channels
   // in full, rows of up to 16384 channels for the plain operator.
   // (RMSNorm: one producer per 16-channel group, in whole warps - the reference's summation order)
@@ -2003,11 +2009,13 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
 // the fp32 reciprocal, as torch's division of a tensor by a host scalar multiplies by it.
 int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight, const int16_t* idx, int64_t rows, int KQ,
                                  int KE, int mode, uint8_t* q, uint8_t* sf, float* scale_out, float* scratch,
-                                 cudaStream_t stream, const int* groups, int ngroups, const int* row_map) {
+                                 cudaStream_t stream, const int* groups, int ngroups, const int* row_map, float* clear, int nclear) {
   if (KQ > 16384) return ARCQ_ERR_UNSUPPORTED_K;
   ScaleOptions so;
   so.factor = 1.0f / 2688.0f;
   so.out = scale_out;
+  so.clear = clear;
+  so.nclear = nclear;
   if (amax == nullptr) {
     DeviceInfo di;
     int rc = get_device_info(&di);

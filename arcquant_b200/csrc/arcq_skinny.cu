@@ -596,10 +596,6 @@ int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, c
   // one CTA per item where several form a cluster; else persistent CTAs, two per SM
   const long long slots = di.num_sms == di.all_sms ? 2LL * di.num_sms : di.num_sms;
   if (csize == 1 && (groups != nullptr || nt <= 64) && grid > slots) grid = slots;
-  if (gated) {
-    rc = launch_clear(swiglu_amax, p.ngroups, stream);
-    if (rc != ARCQ_OK) return rc;
-  }
   CUtensorMap mx, mw;
   rc = make_operand_map(&mx, X, M, K_eff / 2, nt > 64 ? 32 : 16);
   if (rc != ARCQ_OK) return rc;

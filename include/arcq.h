@@ -110,6 +110,11 @@ int arcq_quantize_tensor_scale(const void* x, const float* amax, int is_weight, 
 int arcq_quantize_x_grouped_amax(const void* x, const int32_t* row_map, const float* amax, const int16_t* reorder_indices,
                                  const int32_t* groups, int ngroups, int64_t rows_bound, int KQ, int KE, int mode,
                                  uint8_t* qx, uint8_t* sfx, float* scale_out, void* stream);
+/* arcq_quantize_x_grouped_amax, which also sets the nclear floats at `clear` (device, at most 64) to zero: the maxima that an
+ * arcq_matmul_nvfp4_grouped_swiglu_onto behind it collects. */
+int arcq_quantize_x_grouped_amax_clear(const void* x, const int32_t* row_map, const float* amax, const int16_t* reorder_indices,
+                                       const int32_t* groups, int ngroups, int64_t rows_bound, int KQ, int KE, int mode,
+                                       uint8_t* qx, uint8_t* sfx, float* scale_out, float* clear, int nclear, void* stream);
 
 /* arcq_reorder_quantize_x on x / *scale: the division by the per-tensor scale that the reference's
  * callers do in torch before the operator (`x / scale` in NVFP4_reorder_quantize_x,
@@ -130,6 +135,10 @@ int arcq_reorder_quantize_x_scaled(const void* x, const float* scale, const int1
  * 1/sqrt(ss/KQ + eps).  KQ/16 must be a multiple of 32 between 64 and 512 (KQ 1024..8192). */
 int arcq_rmsnorm_quantize_x(const void* x, const void* gamma, float eps, const int16_t* reorder_index,
                             int64_t M, int KQ, int KE, uint8_t* qx, uint8_t* sfx, void* stream);
+/* arcq_rmsnorm_quantize_x, which also sets the nclear floats at `clear` (device, at most 64) to zero: the maximum that an
+ * arcq_matmul_nvfp4_swiglu_onto behind it collects. */
+int arcq_rmsnorm_quantize_x_clear(const void* x, const void* gamma, float eps, const int16_t* reorder_index,
+                                  int64_t M, int KQ, int KE, uint8_t* qx, uint8_t* sfx, float* clear, int nclear, void* stream);
 
 /* Replaces agemm.reorder_quantize_w (kernels/src/bindings.cpp:170-210 ->
  * kernels/src/reorder.cu:353-372, 719-738, down.cu:383-401): the offline
@@ -331,6 +340,15 @@ int arcq_matmul_nvfp4_grouped_swiglu(const uint8_t* A, const uint8_t* B, const u
                                      int64_t M_bound, int64_t N, int64_t K_eff, const int32_t* tile_group,
                                      const int32_t* groups, int ngroups, const float* alpha_a, const float* alpha_b,
                                      void* C, float* amax, void* stream);
+/* The same on maxima that are zero already (or hold those of earlier calls): nothing is cleared in front of the kernel, so that
+ * it can be set up while the kernel before is still running. */
+int arcq_matmul_nvfp4_swiglu_onto(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB,
+                                  int64_t M, int64_t N, int64_t K_eff, const float* alpha_a, const float* alpha_b,
+                                  void* C, float* amax, void* stream);
+int arcq_matmul_nvfp4_grouped_swiglu_onto(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB,
+                                          int64_t M_bound, int64_t N, int64_t K_eff, const int32_t* tile_group,
+                                          const int32_t* groups, int ngroups, const float* alpha_a, const float* alpha_b,
+                                          void* C, float* amax, void* stream);
 
 /* ---- Projection with the residual addition in the GEMM's epilogue ---------------------------------------
  * The reference adds the residual stream in torch after o_proj and down_proj (`residual + hidden_states`,

@@ -3,6 +3,7 @@
 // order and return types for the four quantized-linear operators; outputs are allocated here with
 // torch::empty, inputs are borrowed, kernels run on torch's current CUDA stream.  The reference's
 // KV-cache operators (batch_decode_*, init_kv_*, append_kv_*) are not part of this library.
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/extension.h>
@@ -41,6 +42,11 @@ void require_scalar_f32(const torch::Tensor& t, const torch::Tensor& like, const
   require_on(t, like, at::kFloat, name);
   TORCH_CHECK(t.numel() == 1, name, " must hold one fp32 value");
 }
+// An output on `like`'s device.  Straight from the CUDA allocator's factory: through torch::empty's dispatch an allocation costs the
+// host about as much as a third of a launch, and a call makes two to five.
+torch::Tensor empty_on(const torch::Tensor& like, at::IntArrayRef sizes, at::ScalarType type) {
+  return torch::Tensor(at::detail::empty_cuda(sizes, type, like.device(), c10::nullopt));
+}
 // Shapes of a block-scaled GEMM's operands; returns M, N, K_eff.
 std::tuple<int64_t, int64_t, int64_t> check_gemm_operands(const torch::Tensor& A, const torch::Tensor& B,
                                                           const torch::Tensor& SFA, const torch::Tensor& SFB) {
@@ -61,7 +67,7 @@ std::tuple<int64_t, int64_t, int64_t> check_gemm_operands(const torch::Tensor& A
 
 std::tuple<torch::Tensor, torch::Tensor> quantize_common(const torch::Tensor& X, const torch::Tensor* gamma,
                                                          float eps, const torch::Tensor& reorder_index, int KE,
-                                                         bool is_weight, const char* where) {
+                                                         bool is_weight, const char* where, torch::Tensor* clear = nullptr) {
   require_cuda(X, "input");
   require_on(reorder_index, X, at::kShort, "reorder_index");
   TORCH_CHECK(X.dim() == 2, "input must be 2-D");
@@ -71,17 +77,17 @@ std::tuple<torch::Tensor, torch::Tensor> quantize_common(const torch::Tensor& X,
   TORCH_CHECK(KE >= 0 && KE <= KQ, "KE must lie in [0, KQ]");
   TORCH_CHECK(reorder_index.numel() == KQ, "reorder_index must have KQ entries");
   c10::cuda::CUDAGuard guard(X.device());
-  auto options = torch::dtype(torch::kUInt8).device(X.device());
-  auto Q = torch::empty({rows, K / 2}, options);
-  auto SF = torch::empty({static_cast<int64_t>(arcq_sf_bytes(rows, K))}, options);
+  auto Q = empty_on(X, {rows, K / 2}, at::kByte);
+  auto SF = empty_on(X, {static_cast<int64_t>(arcq_sf_bytes(rows, K))}, at::kByte);
   const void* px = X.data_ptr<at::BFloat16>();                 // throws on a wrong dtype, as the reference does
   const int16_t* pidx = reorder_index.data_ptr<int16_t>();
   int status;
   if (gamma) {
     require_on(*gamma, X, at::kBFloat16, "weight");
     TORCH_CHECK(gamma->numel() == KQ, "weight must have KQ entries");
-    status = arcq_rmsnorm_quantize_x(px, gamma->data_ptr<at::BFloat16>(), eps, pidx, rows, KQ, KE,
-                                     Q.data_ptr<uint8_t>(), SF.data_ptr<uint8_t>(), current_stream(X));
+    status = arcq_rmsnorm_quantize_x_clear(px, gamma->data_ptr<at::BFloat16>(), eps, pidx, rows, KQ, KE, Q.data_ptr<uint8_t>(),
+                                           SF.data_ptr<uint8_t>(), clear ? clear->data_ptr<float>() : nullptr,
+                                           clear ? static_cast<int>(clear->numel()) : 0, current_stream(X));
   } else if (is_weight) {
     status = arcq_reorder_quantize_w(px, pidx, rows, KQ, KE, arcq_reference_mode(KQ), Q.data_ptr<uint8_t>(),
                                      SF.data_ptr<uint8_t>(), current_stream(X));
@@ -98,7 +104,7 @@ torch::Tensor matmul(const torch::Tensor& A, const torch::Tensor& B, const torch
   int64_t M, N, K;
   std::tie(M, N, K) = check_gemm_operands(A, B, SFA, SFB);
   c10::cuda::CUDAGuard guard(A.device());
-  auto C = torch::empty({M, N}, torch::dtype(torch::kBFloat16).device(A.device()));
+  auto C = empty_on(A, {M, N}, at::kBFloat16);
   int status = arcq_matmul_nvfp4_ws(A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(),
                                     SFB.data_ptr<uint8_t>(), M, N, K, scale, nullptr, nullptr,
                                     C.data_ptr<at::BFloat16>(), nullptr, 0, current_stream(A));
@@ -115,7 +121,7 @@ torch::Tensor matmul_dev_alpha(const torch::Tensor& A, const torch::Tensor& B, c
   require_scalar_f32(alpha_a, A, "alpha_a");
   if (alpha_b.has_value()) require_scalar_f32(*alpha_b, A, "alpha_b");
   c10::cuda::CUDAGuard guard(A.device());
-  auto C = torch::empty({M, N}, torch::dtype(torch::kBFloat16).device(A.device()));
+  auto C = empty_on(A, {M, N}, at::kBFloat16);
   const float* pb = alpha_b.has_value() ? alpha_b->data_ptr<float>() : nullptr;
   int status;
   if (bias.has_value()) {
@@ -145,7 +151,7 @@ torch::Tensor matmul_residual(const torch::Tensor& A, const torch::Tensor& B, co
               residual.size(0) == M && residual.size(1) == N && residual.device() == A.device(),
               "residual must be a contiguous bf16 [M, N] tensor on A's device");
   c10::cuda::CUDAGuard guard(A.device());
-  auto C = torch::empty({M, N}, torch::dtype(torch::kBFloat16).device(A.device()));
+  auto C = empty_on(A, {M, N}, at::kBFloat16);
   int status = arcq_matmul_nvfp4_residual(
       A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(), SFB.data_ptr<uint8_t>(), M, N, K,
       alpha_a.data_ptr<float>(), alpha_b.has_value() ? alpha_b->data_ptr<float>() : nullptr, residual.data_ptr(),
@@ -189,9 +195,8 @@ std::tuple<torch::Tensor, torch::Tensor> reorder_quantize_x_scaled(const torch::
   TORCH_CHECK(reorder_index.numel() == KQ, "reorder_index must have KQ entries");
   if (mode < 0) mode = arcq_reference_mode(KQ);
   c10::cuda::CUDAGuard guard(X.device());
-  auto options = torch::dtype(torch::kUInt8).device(X.device());
-  auto Q = torch::empty({rows, K / 2}, options);
-  auto SF = torch::empty({static_cast<int64_t>(arcq_sf_bytes(rows, K))}, options);
+  auto Q = empty_on(X, {rows, K / 2}, at::kByte);
+  auto SF = empty_on(X, {static_cast<int64_t>(arcq_sf_bytes(rows, K))}, at::kByte);
   int status = arcq_reorder_quantize_x_scaled(X.data_ptr<at::BFloat16>(), scale.data_ptr<float>(),
                                               reorder_index.data_ptr<int16_t>(), rows, KQ, KE, mode,
                                               Q.data_ptr<uint8_t>(), SF.data_ptr<uint8_t>(), current_stream(X));
@@ -222,12 +227,11 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> quantize_tensor_scale(co
   TORCH_CHECK(reorder_index.numel() == KQ, "reorder_index must have KQ entries");
   if (mode < 0) mode = arcq_reference_mode(KQ);
   c10::cuda::CUDAGuard guard(X.device());
-  const auto u8 = X.options().dtype(torch::kUInt8), f32 = X.options().dtype(torch::kFloat32);
-  auto Q = torch::empty({rows, K / 2}, u8);
-  auto SF = torch::empty({static_cast<int64_t>(arcq_sf_bytes(rows, K))}, u8);
-  auto scale = torch::empty({}, f32);
+  auto Q = empty_on(X, {rows, K / 2}, at::kByte);
+  auto SF = empty_on(X, {static_cast<int64_t>(arcq_sf_bytes(rows, K))}, at::kByte);
+  auto scale = empty_on(X, {}, at::kFloat);
   torch::Tensor scratch;
-  if (!amax.has_value()) scratch = torch::empty({ARCQ_SCALE_SCRATCH}, f32);
+  if (!amax.has_value()) scratch = empty_on(X, {ARCQ_SCALE_SCRATCH}, at::kFloat);
   check_status(arcq_quantize_tensor_scale(X.data_ptr(), amax.has_value() ? amax->data_ptr<float>() : nullptr, is_weight ? 1 : 0,
                                           reorder_index.data_ptr<int16_t>(), rows, KQ, KE, mode, Q.data_ptr<uint8_t>(),
                                           SF.data_ptr<uint8_t>(), scale.data_ptr<float>(),
@@ -246,22 +250,27 @@ const float* factors(const c10::optional<torch::Tensor>& t, const torch::Tensor&
   return t.has_value() ? factors(*t, like, count, name) : nullptr;
 }
 
-// Gate/up GEMM with the SwiGLU epilogue; see arcq_matmul_nvfp4_swiglu.
-std::tuple<torch::Tensor, torch::Tensor> matmul_swiglu(const torch::Tensor& A, const torch::Tensor& B, const torch::Tensor& SFA,
-                                                       const torch::Tensor& SFB, const torch::Tensor& alpha_a,
-                                                       const c10::optional<torch::Tensor>& alpha_b) {
+// Gate/up GEMM with the SwiGLU epilogue; see arcq_matmul_nvfp4_swiglu, and _onto for an amax that is zero already.
+torch::Tensor swiglu(const torch::Tensor& A, const torch::Tensor& B, const torch::Tensor& SFA, const torch::Tensor& SFB,
+                     const torch::Tensor& alpha_a, const c10::optional<torch::Tensor>& alpha_b, torch::Tensor& amax,
+                     decltype(arcq_matmul_nvfp4_swiglu)* call) {
   int64_t M, N, K;
   std::tie(M, N, K) = check_gemm_operands(A, B, SFA, SFB);
   const float *aa = factors(alpha_a, A, 1, "alpha_a"), *ab = factors(alpha_b, A, 1, "alpha_b");
   TORCH_CHECK(N % 256 == 0, "N is not a multiple of 256");
   c10::cuda::CUDAGuard guard(A.device());
-  auto C = torch::empty({M, N / 2}, torch::dtype(torch::kBFloat16).device(A.device()));
-  auto amax = torch::empty({}, torch::dtype(torch::kFloat32).device(A.device()));
-  check_status(arcq_matmul_nvfp4_swiglu(A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(), SFB.data_ptr<uint8_t>(),
-                                        M, N, K, aa, ab, C.data_ptr<at::BFloat16>(), amax.data_ptr<float>(),
-                                        current_stream(A)),
+  auto C = empty_on(A, {M, N / 2}, at::kBFloat16);
+  check_status(call(A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(), SFB.data_ptr<uint8_t>(), M, N, K, aa, ab,
+                    C.data_ptr<at::BFloat16>(), amax.data_ptr<float>(), current_stream(A)),
                "swiglu matmul");
-  return std::make_tuple(C, amax);
+  return C;
+}
+std::tuple<torch::Tensor, torch::Tensor> matmul_swiglu(const torch::Tensor& A, const torch::Tensor& B, const torch::Tensor& SFA,
+                                                       const torch::Tensor& SFB, const torch::Tensor& alpha_a,
+                                                       const c10::optional<torch::Tensor>& alpha_b) {
+  require_cuda(A, "A");
+  auto amax = empty_on(A, {}, at::kFloat);
+  return std::make_tuple(swiglu(A, B, SFA, SFB, alpha_a, alpha_b, amax, arcq_matmul_nvfp4_swiglu), amax);
 }
 
 // The grouped forms; groups: the run table [first rows | rows] of exactly these runs (in a table of more the row counts lie
@@ -279,19 +288,21 @@ std::tuple<torch::Tensor, torch::Tensor> matmul_grouped_swiglu(const torch::Tens
                                                                const torch::Tensor& SFB, const torch::Tensor& tile_group,
                                                                const torch::Tensor& groups, int64_t ngroups, int64_t n,
                                                                const torch::Tensor& alpha_a,
-                                                               const c10::optional<torch::Tensor>& alpha_b) {
+                                                               const c10::optional<torch::Tensor>& alpha_b,
+                                                               const c10::optional<torch::Tensor>& onto) {
   int64_t M, N, K;
   std::tie(M, N, K) = check_gemm_operands(A, B, SFA, SFB);
   check_grouped(A, B, tile_group, groups, ngroups, n, alpha_a);
   const float *aa = factors(alpha_a, A, ngroups, "alpha_a"), *ab = factors(alpha_b, A, ngroups, "alpha_b");
   TORCH_CHECK(n % 256 == 0, "n is not a multiple of 256");
+  if (onto.has_value()) factors(*onto, A, ngroups, "onto");
   c10::cuda::CUDAGuard guard(A.device());
-  auto C = torch::empty({M, n / 2}, torch::dtype(torch::kBFloat16).device(A.device()));
-  auto amax = torch::empty({ngroups}, torch::dtype(torch::kFloat32).device(A.device()));
-  check_status(arcq_matmul_nvfp4_grouped_swiglu(A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(),
-                                                SFB.data_ptr<uint8_t>(), M, n, K, tile_group.data_ptr<int32_t>(),
-                                                groups.data_ptr<int32_t>(), static_cast<int>(ngroups), aa, ab,
-                                                C.data_ptr<at::BFloat16>(), amax.data_ptr<float>(), current_stream(A)),
+  auto C = empty_on(A, {M, n / 2}, at::kBFloat16);
+  auto amax = onto.has_value() ? *onto : empty_on(A, {ngroups}, at::kFloat);
+  auto call = onto.has_value() ? arcq_matmul_nvfp4_grouped_swiglu_onto : arcq_matmul_nvfp4_grouped_swiglu;
+  check_status(call(A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(), SFB.data_ptr<uint8_t>(), M, n, K,
+                    tile_group.data_ptr<int32_t>(), groups.data_ptr<int32_t>(), static_cast<int>(ngroups), aa, ab,
+                    C.data_ptr<at::BFloat16>(), amax.data_ptr<float>(), current_stream(A)),
                "grouped swiglu matmul");
   return std::make_tuple(C, amax);
 }
@@ -303,7 +314,7 @@ torch::Tensor matmul_grouped_runs(const torch::Tensor& A, const torch::Tensor& B
   check_grouped(A, B, tile_group, groups, ngroups, n, alpha_a);
   const float *aa = factors(alpha_a, A, ngroups, "alpha_a"), *ab = factors(alpha_b, A, ngroups, "alpha_b");
   c10::cuda::CUDAGuard guard(A.device());
-  auto C = torch::empty({M, n}, torch::dtype(torch::kBFloat16).device(A.device()));
+  auto C = empty_on(A, {M, n}, at::kBFloat16);
   check_status(arcq_matmul_nvfp4_grouped_runs(A.data_ptr<uint8_t>(), B.data_ptr<uint8_t>(), SFA.data_ptr<uint8_t>(),
                                               SFB.data_ptr<uint8_t>(), M, n, K, tile_group.data_ptr<int32_t>(),
                                               groups.data_ptr<int32_t>(), static_cast<int>(ngroups), aa, ab,
@@ -316,7 +327,7 @@ torch::Tensor matmul_grouped_runs(const torch::Tensor& A, const torch::Tensor& B
 std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> quantize_grouped_amax(const torch::Tensor& X, const c10::optional<torch::Tensor>& row_map,
                                                                               const torch::Tensor& amax, const torch::Tensor& indices,
                                                                               const torch::Tensor& groups, int64_t rows_bound, int KE,
-                                                                              int mode) {
+                                                                              int mode, const c10::optional<torch::Tensor>& clear) {
   require_cuda(X, "input");
   TORCH_CHECK(X.scalar_type() == at::kBFloat16 && X.dim() >= 1, "input: expected bfloat16 rows");
   require_on(amax, X, at::kFloat, "amax");
@@ -332,15 +343,17 @@ std::tuple<torch::Tensor, torch::Tensor, torch::Tensor> quantize_grouped_amax(co
   } else {
     TORCH_CHECK(X.size(0) >= rows_bound, "input has fewer rows than rows_bound");
   }
+  if (clear.has_value()) require_on(*clear, X, at::kFloat, "clear");
   c10::cuda::CUDAGuard guard(X.device());
-  const auto u8 = X.options().dtype(torch::kUInt8);
-  auto Q = torch::empty({rows_bound, (KQ + KE) / 2}, u8);
-  auto SF = torch::empty({static_cast<int64_t>(arcq_sf_bytes(rows_bound, KQ + KE))}, u8);
-  auto scale = torch::empty({ngroups}, X.options().dtype(torch::kFloat32));
-  check_status(arcq_quantize_x_grouped_amax(X.data_ptr(), row_map.has_value() ? row_map->data_ptr<int32_t>() : nullptr,
-                                            amax.data_ptr<float>(), indices.data_ptr<int16_t>(), groups.data_ptr<int32_t>(),
-                                            static_cast<int>(ngroups), rows_bound, static_cast<int>(KQ), KE, mode,
-                                            Q.data_ptr<uint8_t>(), SF.data_ptr<uint8_t>(), scale.data_ptr<float>(), current_stream(X)),
+  auto Q = empty_on(X, {rows_bound, (KQ + KE) / 2}, at::kByte);
+  auto SF = empty_on(X, {static_cast<int64_t>(arcq_sf_bytes(rows_bound, KQ + KE))}, at::kByte);
+  auto scale = empty_on(X, {ngroups}, at::kFloat);
+  check_status(arcq_quantize_x_grouped_amax_clear(X.data_ptr(), row_map.has_value() ? row_map->data_ptr<int32_t>() : nullptr,
+                                                  amax.data_ptr<float>(), indices.data_ptr<int16_t>(), groups.data_ptr<int32_t>(),
+                                                  static_cast<int>(ngroups), rows_bound, static_cast<int>(KQ), KE, mode,
+                                                  Q.data_ptr<uint8_t>(), SF.data_ptr<uint8_t>(), scale.data_ptr<float>(),
+                                                  clear.has_value() ? clear->data_ptr<float>() : nullptr,
+                                                  clear.has_value() ? static_cast<int>(clear->numel()) : 0, current_stream(X)),
                "grouped x-quantize");
   return std::make_tuple(Q, SF, scale);
 }
@@ -365,7 +378,7 @@ torch::Tensor channel_order(const torch::Tensor& value) {
   require_on(value, value, at::kFloat, "value");
   TORCH_CHECK(value.numel() <= 32768, "value has more channels than an int16 order can hold");
   c10::cuda::CUDAGuard guard(value.device());
-  auto order = torch::empty({value.numel()}, value.options().dtype(torch::kInt16));
+  auto order = empty_on(value, {value.numel()}, at::kShort);
   if (value.numel() == 0) return order;
   check_status(arcq_channel_order(value.data_ptr<float>(), static_cast<int>(value.numel()), order.data_ptr<int16_t>(), current_stream(value)),
                "channel_order");
@@ -378,8 +391,8 @@ std::tuple<torch::Tensor, torch::Tensor> silu_mul(const torch::Tensor& GU) {
   c10::cuda::CUDAGuard guard(GU.device());
   const int64_t tokens = GU.size(0);
   const int F = static_cast<int>(GU.size(1) / 2);
-  auto out = torch::empty({tokens, F}, torch::dtype(torch::kBFloat16).device(GU.device()));
-  auto amax = torch::empty({}, torch::dtype(torch::kFloat32).device(GU.device()));
+  auto out = empty_on(GU, {tokens, F}, at::kBFloat16);
+  auto amax = empty_on(GU, {}, at::kFloat);
   check_status(arcq_silu_mul_bf16(GU.data_ptr<at::BFloat16>(), out.data_ptr<at::BFloat16>(), tokens, F,
                                   amax.data_ptr<float>(), current_stream(GU)),
                "silu_mul");
@@ -404,9 +417,116 @@ torch::Tensor rope_inplace(torch::Tensor X, const torch::Tensor& cos_t, const to
 torch::Tensor absmax(const torch::Tensor& X) {
   require_cuda(X, "input");
   c10::cuda::CUDAGuard guard(X.device());
-  auto out = torch::empty({}, torch::dtype(torch::kFloat32).device(X.device()));
+  auto out = empty_on(X, {}, at::kFloat);
   check_status(arcq_absmax_bf16(X.data_ptr<at::BFloat16>(), X.numel(), out.data_ptr<float>(), 0, current_stream(X)),
                "absmax");
+  return out;
+}
+
+// A quantized linear's forward: `matmul_dev_alpha` with a bias, the result as [bsz, q_len, N] or [q_len, N].
+torch::Tensor linear(const torch::Tensor& A, const torch::Tensor& B, const torch::Tensor& SFA, const torch::Tensor& SFB,
+                     const torch::Tensor& alpha_a, const torch::Tensor& alpha_b, const c10::optional<torch::Tensor>& bias,
+                     const c10::optional<int64_t>& bsz, int64_t q_len) {
+  auto C = matmul_dev_alpha(A, B, SFA, SFB, alpha_a, alpha_b, bias);
+  if (bsz.has_value()) return C.reshape({*bsz, q_len, -1});
+  return q_len > 0 && q_len == C.size(0) ? C : C.reshape({q_len, -1});
+}
+
+// The two halves of a decoder layer as the Python class of that name strings them together, operation for operation: one call each
+// instead of a dozen, whose argument handling, views and attribute look-ups took longer than the kernels of a short prompt.
+torch::Tensor attention_half(const torch::Tensor& X, const torch::Tensor& gain, double eps, const torch::Tensor& q_index, int q_ke,
+                             const torch::Tensor& qkv_W, const torch::Tensor& qkv_SF, const torch::Tensor& qkv_scale,
+                             const torch::Tensor& cos_t, const torch::Tensor& sin_t, int64_t heads, int64_t kv_heads, int64_t head_dim,
+                             int64_t bsz, int64_t seq, const torch::Tensor& o_index, int o_ke, const torch::Tensor& o_W,
+                             const torch::Tensor& o_SF, const torch::Tensor& o_scale, const c10::optional<torch::Tensor>& residual) {
+  require_cuda(X, "x");
+  TORCH_CHECK(X.dim() == 2 && X.size(0) == bsz * seq, "x must be [bsz * seq, hidden]");
+  at::NoGradGuard no_grad;
+  c10::cuda::CUDAGuard guard(X.device());
+  torch::Tensor a, sfa, so;
+  std::tie(a, sfa) = quantize_common(X, &gain, static_cast<float>(eps), q_index, q_ke, false, "run_rmsnorm_x_bf16_nvfp4");
+  auto qkv = matmul_dev_alpha(a, qkv_W, sfa, qkv_SF, qkv_scale, c10::nullopt, c10::nullopt);
+  const int64_t N = qkv.size(1);
+  TORCH_CHECK(N == (heads + 2 * kv_heads) * head_dim, "the q/k/v projection does not hold these heads");
+  rope_inplace(qkv, cos_t, sin_t, static_cast<int>(heads + kv_heads), static_cast<int>(head_dim));
+  // [bsz, heads, seq, head_dim] views of the fused output; grouped-query heads are not materialised
+  auto view = [&](int64_t n, int64_t at) { return qkv.as_strided({bsz, n, seq, head_dim}, {seq * N, head_dim, N, 1}, at); };
+  auto attn = at::scaled_dot_product_attention(view(heads, 0), view(kv_heads, heads * head_dim), view(kv_heads, (heads + kv_heads) * head_dim),
+                                               c10::nullopt, 0.0, true, c10::nullopt, heads != kv_heads);
+  attn = attn.transpose(1, 2).reshape({bsz * seq, heads * head_dim}).contiguous();
+  std::tie(a, sfa, so) = quantize_tensor_scale(attn, o_index, o_ke, ARCQ_MODE_16, false, c10::nullopt);
+  return residual.has_value() ? matmul_residual(a, o_W, sfa, o_SF, so, o_scale, *residual)
+                              : matmul_dev_alpha(a, o_W, sfa, o_SF, so, o_scale, c10::nullopt);
+}
+torch::Tensor mlp_half(const torch::Tensor& H, const torch::Tensor& gain, double eps, const torch::Tensor& up_index, int up_ke,
+                       const torch::Tensor& gu_W, const torch::Tensor& gu_SF, const torch::Tensor& gu_scale,
+                       const torch::Tensor& down_index, int down_ke, const torch::Tensor& down_W, const torch::Tensor& down_SF,
+                       const torch::Tensor& down_scale, const c10::optional<torch::Tensor>& residual) {
+  require_cuda(H, "h");
+  at::NoGradGuard no_grad;
+  c10::cuda::CUDAGuard guard(H.device());
+  torch::Tensor a, sfa, act, amax, scale;
+  amax = empty_on(H, {}, at::kFloat);                           // (cleared by the quantizer)
+  std::tie(a, sfa) = quantize_common(H, &gain, static_cast<float>(eps), up_index, up_ke, false, "run_rmsnorm_x_bf16_nvfp4", &amax);
+  act = swiglu(a, gu_W, sfa, gu_SF, gu_scale, c10::nullopt, amax, arcq_matmul_nvfp4_swiglu_onto);
+  std::tie(a, sfa, scale) = quantize_tensor_scale(act, down_index, down_ke, ARCQ_MODE_16, false, amax);
+  return residual.has_value() ? matmul_residual(a, down_W, sfa, down_SF, scale, down_scale, *residual)
+                              : matmul_dev_alpha(a, down_W, sfa, down_SF, scale, down_scale, c10::nullopt);
+}
+
+// Routing and bookkeeping of a MoE block; see arcq_route_topk_bf16, arcq_moe_layout, arcq_absmax_grouped_bf16, arcq_moe_combine_bf16.
+std::tuple<torch::Tensor, torch::Tensor> route_topk(const torch::Tensor& logits, int64_t top_k) {
+  require_on(logits, logits, at::kBFloat16, "logits");
+  TORCH_CHECK(logits.dim() == 2, "logits must be [tokens, experts]");
+  c10::cuda::CUDAGuard guard(logits.device());
+  const int64_t t = logits.size(0);
+  auto ids = empty_on(logits, {t, top_k}, at::kLong);
+  auto w = empty_on(logits, {t, top_k}, at::kBFloat16);
+  check_status(arcq_route_topk_bf16(logits.data_ptr(), t, static_cast<int>(logits.size(1)), static_cast<int>(top_k),
+                                    ids.data_ptr<int64_t>(), w.data_ptr(), current_stream(logits)),
+               "route_topk");
+  return std::make_tuple(ids, w);
+}
+std::tuple<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor> moe_layout(const torch::Tensor& slot_group, int64_t ngroups,
+                                                                                  int64_t tile, int64_t rows_bound, int64_t div) {
+  require_on(slot_group, slot_group, at::kLong, "slot_group");
+  TORCH_CHECK(tile > 0, "tile must be positive");
+  c10::cuda::CUDAGuard guard(slot_group.device());
+  const int64_t n = slot_group.numel();
+  auto dest = empty_on(slot_group, {n}, at::kInt);
+  auto row_map = empty_on(slot_group, {rows_bound}, at::kInt);
+  auto groups = empty_on(slot_group, {2 * ngroups}, at::kInt);
+  auto tile_group = empty_on(slot_group, {rows_bound / tile}, at::kInt);
+  check_status(arcq_moe_layout(slot_group.data_ptr<int64_t>(), static_cast<int>(n), static_cast<int>(ngroups), static_cast<int>(tile),
+                               static_cast<int>(rows_bound), static_cast<int>(div), dest.data_ptr<int32_t>(), row_map.data_ptr<int32_t>(),
+                               groups.data_ptr<int32_t>(), tile_group.data_ptr<int32_t>(), current_stream(slot_group)),
+               "moe_layout");
+  return std::make_tuple(dest, row_map, groups, tile_group);
+}
+torch::Tensor absmax_grouped(const torch::Tensor& X, const c10::optional<torch::Tensor>& row_map, const torch::Tensor& groups,
+                             int64_t ngroups) {
+  require_on(X, X, at::kBFloat16, "input");
+  require_on(groups, X, at::kInt, "groups");
+  if (row_map.has_value()) require_on(*row_map, X, at::kInt, "row_map");
+  TORCH_CHECK(groups.numel() == 2 * ngroups, "groups must hold 2 * ngroups entries");
+  c10::cuda::CUDAGuard guard(X.device());
+  auto out = empty_on(X, {ngroups}, at::kFloat);
+  check_status(arcq_absmax_grouped_bf16(X.data_ptr(), row_map.has_value() ? row_map->data_ptr<int32_t>() : nullptr,
+                                        groups.data_ptr<int32_t>(), static_cast<int>(ngroups), static_cast<int>(X.size(-1)),
+                                        out.data_ptr<float>(), current_stream(X)),
+               "absmax_grouped");
+  return out;
+}
+torch::Tensor moe_combine(const torch::Tensor& Y, const torch::Tensor& pos, const torch::Tensor& weights) {
+  require_on(Y, Y, at::kBFloat16, "y");
+  require_on(pos, Y, at::kInt, "pos");
+  require_on(weights, Y, at::kBFloat16, "weights");
+  TORCH_CHECK(pos.dim() == 2 && Y.dim() == 2 && weights.numel() >= pos.numel(), "y must be [rows, H], pos and weights [tokens, k]");
+  c10::cuda::CUDAGuard guard(Y.device());
+  auto out = empty_on(Y, {pos.size(0), Y.size(1)}, at::kBFloat16);
+  check_status(arcq_moe_combine_bf16(Y.data_ptr(), pos.data_ptr<int32_t>(), weights.data_ptr(), out.data_ptr(), pos.size(0),
+                                     static_cast<int>(Y.size(1)), static_cast<int>(pos.size(1)), current_stream(Y)),
+               "moe_combine");
   return out;
 }
 
@@ -424,6 +544,16 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("matmul_dev_alpha", &matmul_dev_alpha, "gemm with device-resident global scales", py::arg("A"),
         py::arg("B"), py::arg("SFA"), py::arg("SFB"), py::arg("alpha_a"), py::arg("alpha_b") = py::none(),
         py::arg("bias") = py::none());
+  m.def("linear", &linear, "forward of a quantized linear", py::arg("A"), py::arg("B"), py::arg("SFA"), py::arg("SFB"), py::arg("alpha_a"),
+        py::arg("alpha_b"), py::arg("bias"), py::arg("bsz"), py::arg("q_len"));
+  m.def("attention_half", &attention_half, "norm, q/k/v, rotary embedding, attention, o projection of a decoder layer");
+  m.def("mlp_half", &mlp_half, "norm, gate/up with SwiGLU, down projection of a decoder layer");
+  m.def("route_topk", &route_topk, "(expert ids, weights) of router logits", py::arg("logits"), py::arg("top_k"));
+  m.def("moe_layout", &moe_layout, "(dest, row_map, groups, tile_group) of routed rows", py::arg("slot_group"), py::arg("ngroups"),
+        py::arg("tile"), py::arg("rows_bound"), py::arg("div"));
+  m.def("absmax_grouped", &absmax_grouped, "max|x| over the rows of each run", py::arg("X"), py::arg("row_map"), py::arg("groups"),
+        py::arg("ngroups"));
+  m.def("moe_combine", &moe_combine, "weighted sums of the routed copies", py::arg("Y"), py::arg("pos"), py::arg("weights"));
   m.def("matmul_residual", &matmul_residual, "residual + gemm with device-resident global scales", py::arg("A"), py::arg("B"),
         py::arg("SFA"), py::arg("SFB"), py::arg("alpha_a"), py::arg("alpha_b"), py::arg("residual"));
   m.def("reorder_quantize_x_scaled", &reorder_quantize_x_scaled, "reorder_quantize_x of X / scale (device scalar)",
@@ -434,12 +564,13 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("matmul_swiglu", &matmul_swiglu, "gate/up GEMM with SwiGLU: (act, amax)", py::arg("A"), py::arg("B"), py::arg("SFA"),
         py::arg("SFB"), py::arg("alpha_a"), py::arg("alpha_b"));
   m.def("matmul_grouped_swiglu", &matmul_grouped_swiglu, "its grouped form", py::arg("A"), py::arg("B"), py::arg("SFA"), py::arg("SFB"),
-        py::arg("tile_group"), py::arg("groups"), py::arg("ngroups"), py::arg("n"), py::arg("alpha_a"), py::arg("alpha_b"));
+        py::arg("tile_group"), py::arg("groups"), py::arg("ngroups"), py::arg("n"), py::arg("alpha_a"), py::arg("alpha_b"),
+        py::arg("onto") = py::none());
   m.def("matmul_grouped_runs", &matmul_grouped_runs, "grouped GEMM with the run table", py::arg("A"), py::arg("B"), py::arg("SFA"),
         py::arg("SFB"), py::arg("tile_group"), py::arg("groups"), py::arg("ngroups"), py::arg("n"), py::arg("alpha_a"), py::arg("alpha_b"));
   m.def("quantize_grouped_amax", &quantize_grouped_amax, "grouped rows by their runs' maxima: (codes, scales, scale)", py::arg("X"),
         py::arg("row_map"), py::arg("amax"), py::arg("reorder_indices"), py::arg("groups"), py::arg("rows_bound"), py::arg("KE"),
-        py::arg("mode"));
+        py::arg("mode"), py::arg("clear") = py::none());
   m.def("channel_order", &channel_order, "channels by ascending statistic, int16", py::arg("value"));
   m.def("calib_stats", &calib_stats, "accumulate the calibration statistics of one batch", py::arg("X"),
         py::arg("chan_absmax"), py::arg("above") = py::none());

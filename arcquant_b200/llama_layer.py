@@ -253,11 +253,23 @@ class QLlamaDecoderLayerTP(torch.nn.Module):
             return ops.matmul_swiglu(a, self.gate_up.W, sfa, self.gate_up.SFW, self.gate_up.scale, None)
         return ops.silu_mul(self.gate_up.gemm(a, sfa))
 
+    def _native(self, x2d: torch.Tensor, k_row: int) -> bool:
+        """Whether a half of the layer may run as one call into the extension: not while phases are timed, and not for what the
+        quantizer of the row-parallel input leaves to torch (no rows, or rows of more than 16384 channels)."""
+        return self.timer is None and x2d.shape[0] > 0 and k_row <= 16384 and ops.native()
+
     # ---- halves of the layer up to (and excluding) the all-reduce: usable for in-process emulation
     @torch.no_grad()
     def attn_partial(self, x2d: torch.Tensor, bsz: int, seq: int, positions: torch.Tensor,
                      residual: torch.Tensor | None = None) -> torch.Tensor:
         cfg, D = self.cfg, self.cfg.head_dim
+        if self._native(x2d, self.h_local * D):      # what follows, in one native call
+            qkv, o = self.qkv, self.o
+            qb, ob = qkv._buffers, o._buffers
+            cos, sin = rope_tables(positions, D, cfg.rope_theta)
+            return ops.attention_half(x2d, self.ln1, cfg.eps, qb["index"], qkv.select_num, qb["W"], qb["SFW"], qb["scale"], cos, sin,
+                                      self.h_local, self.kv_local, D, bsz, seq, ob["index"], o.select_num, ob["W"], ob["SFW"],
+                                      ob["scale"], residual)
         with self._ph("quantize"):
             a, sfa = ops.rmsnorm_quantize_x(x2d, self.ln1, cfg.eps, self.qkv.index, self.qkv.select_num)
         with self._ph("gemm"):
@@ -282,6 +294,11 @@ class QLlamaDecoderLayerTP(torch.nn.Module):
     @torch.no_grad()
     def mlp_partial(self, h2d: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
         cfg = self.cfg
+        if self.fuse_swiglu and self._native(h2d, self.f_local):      # what follows, in one native call
+            gu, down = self.gate_up, self.down
+            gb, db = gu._buffers, down._buffers
+            return ops.mlp_half(h2d, self.ln2, cfg.eps, gb["index"], gu.select_num, gb["W"], gb["SFW"], gb["scale"], db["index"],
+                                down.select_num, db["W"], db["SFW"], db["scale"], residual)
         with self._ph("quantize"):
             a, sfa = ops.rmsnorm_quantize_x(h2d, self.ln2, cfg.eps, self.gate_up.index, self.gate_up.select_num)
         with self._ph("gemm"):

@@ -420,11 +420,12 @@ class QMixtralMoEBlockEP(torch.nn.Module):
         cfg, E = self.cfg, self.dispatcher.e_local
         ke = cfg.select_num
         amax1 = ops.absmax_grouped(batch.src, batch.row_map, batch.groups, E)
+        amax2 = torch.empty(E, dtype=torch.float32, device=amax1.device) if self.fuse_swiglu and E <= 64 else None
         a, sfa, s1 = ops.quantize_grouped_amax(batch.src, batch.row_map, amax1, self.gu_index, batch.groups,
-                                               batch.rows_bound, ke)          # (s1: per-expert scales)
+                                               batch.rows_bound, ke, clear=amax2)          # (s1: per-expert scales)
         if self.fuse_swiglu:        # SiLU * up and the per-expert maxima in the GEMM's epilogue
             act, amax2 = ops.matmul_grouped_swiglu(a, self.gu_W, sfa, self.gu_SF, batch.tile_group, batch.groups, E,
-                                                   2 * cfg.ffn, s1, self.gu_scale)
+                                                   2 * cfg.ffn, s1, self.gu_scale, onto=amax2)
         else:
             h = ops.matmul_grouped(a, self.gu_W, sfa, self.gu_SF, batch.tile_group, E, 2 * cfg.ffn, s1, self.gu_scale)
             if cfg.ffn % 256 == 0:  # SiLU * up and the per-expert maxima in one pass, empty tiles skipped

@@ -16,7 +16,8 @@ from . import _lib
 _EXT = None
 _EXT_CALLS = ("reorder_quantize_x_scaled", "quantize_tensor_scale", "rmsnorm_quantize_x", "matmul_dev_alpha", "absmax", "rope_inplace",
               "silu_mul", "calib_stats", "channel_order", "quantize_grouped_amax", "matmul_grouped_runs", "matmul_swiglu",
-              "matmul_grouped_swiglu", "matmul_residual")
+              "matmul_grouped_swiglu", "matmul_residual", "linear", "attention_half", "mlp_half", "route_topk", "moe_layout", "absmax_grouped",
+              "moe_combine")
 
 
 def _ext():
@@ -206,12 +207,27 @@ def matmul(a, b, sfa, sfb, scale) -> torch.Tensor:
     return _matmul(a, b, sfa, sfb, float(scale), None, None)
 
 
+def _epilogue_bias(bias: torch.Tensor | None, a, b) -> bool:
+    """Whether the GEMM's epilogue can add this bias."""
+    return bias is None or (bias.dtype == torch.bfloat16 and bias.device == a.device and bias.dim() == 1 and bias.is_contiguous()
+                            and bias.numel() == b.shape[0] and bias.data_ptr() % 16 == 0)
+
+
+def linear(a, b, sfa, sfb, alpha_a: torch.Tensor, alpha_b: torch.Tensor, bias: torch.Tensor | None, bsz, q_len) -> torch.Tensor:
+    """`matmul_dev_alpha`, its result as [bsz, q_len, N] (bsz None: [q_len, N])."""
+    ext = _ext()
+    if ext and _epilogue_bias(bias, a, b):
+        return ext.linear(a, b, sfa, sfb, alpha_a, alpha_b, bias, bsz, q_len)
+    with torch.no_grad():
+        y = matmul_dev_alpha(a, b, sfa, sfb, alpha_a, alpha_b, bias)
+        return y.reshape(q_len, -1) if bsz is None else y.reshape(bsz, q_len, -1)
+
+
 def matmul_dev_alpha(a, b, sfa, sfb, alpha_a: torch.Tensor, alpha_b: torch.Tensor | None = None,
                      bias: torch.Tensor | None = None) -> torch.Tensor:
     """matmul with alpha = alpha_a * alpha_b, both fp32 scalars in device memory; plus a bias, in the GEMM's epilogue
     where it is an aligned bf16 vector on the same device (the same bits either way)."""
-    if bias is not None and (bias.dtype != torch.bfloat16 or bias.device != a.device or bias.dim() != 1 or not bias.is_contiguous()
-                             or bias.numel() != b.shape[0] or bias.data_ptr() % 16):
+    if not _epilogue_bias(bias, a, b):
         return matmul_dev_alpha(a, b, sfa, sfb, alpha_a, alpha_b) + bias
     ext = _ext()
     if ext:
@@ -315,6 +331,9 @@ def channel_order(value: torch.Tensor) -> torch.Tensor:
 def route_topk(logits: torch.Tensor, top_k: int):
     """(ids int64 [T, k], weights bf16 [T, k]) of router logits bf16 [T, E], E <= 32, in one launch: fp32 softmax, top-k
     in descending order, weights renormalised over the selected experts."""
+    ext = _ext()
+    if ext:
+        return ext.route_topk(logits, top_k)
     lib = _lib.load()
     _require(logits, torch.bfloat16, "logits")
     if logits.dim() != 2:
@@ -331,6 +350,9 @@ def route_topk(logits: torch.Tensor, top_k: int):
 def moe_layout(slot_group: torch.Tensor, ngroups: int, tile: int, rows_bound: int, div: int = 1):
     """Padded layout of routed rows in one launch: (dest int32 [n], row_map int32 [rows_bound], groups int32
     [2*ngroups], tile_group int32 [rows_bound/tile]); see `arcq_moe_layout` in arcq.h."""
+    ext = _ext()
+    if ext:
+        return ext.moe_layout(slot_group, ngroups, tile, rows_bound, div)
     lib = _lib.load()
     _require(slot_group, torch.int64, "slot_group")
     n, dev = slot_group.numel(), slot_group.device
@@ -364,6 +386,9 @@ def silu_mul_grouped(gate_up: torch.Tensor, tile_group: torch.Tensor, groups: to
 
 def absmax_grouped(x: torch.Tensor, row_map, groups: torch.Tensor, ngroups: int) -> torch.Tensor:
     """fp32 [ngroups]: max|x| over the rows of each run (see `reorder_quantize_x_grouped`)."""
+    ext = _ext()
+    if ext:
+        return ext.absmax_grouped(x, row_map, groups, ngroups)
     lib = _lib.load()
     _require(x, torch.bfloat16, "input")
     _require(groups, torch.int32, "groups")
@@ -411,16 +436,20 @@ def reorder_quantize_x_grouped(x: torch.Tensor, row_map, scales: torch.Tensor, r
 
 
 def quantize_grouped_amax(x: torch.Tensor, row_map, amax: torch.Tensor, reorder_indices: torch.Tensor, groups: torch.Tensor,
-                          rows_bound: int, ke: int, mode: int = 16):
+                          rows_bound: int, ke: int, mode: int = 16, clear: torch.Tensor | None = None):
     """(codes, scales, scale fp32 [runs]): `reorder_quantize_x_grouped` over scale = amax / (448 * 6) of every run, taken
-    inside the quantizer."""
+    inside the quantizer.  clear: up to 64 fp32 values set to zero by the way (see `matmul_grouped_swiglu`)."""
     ngroups, kq = reorder_indices.shape
+    ext = _ext()
+    if clear is not None and not ext:
+        clear.zero_()
     if ngroups > 64 or kq > 16384 or rows_bound == 0 or amax.numel() != ngroups:
+        if clear is not None:
+            clear.zero_()
         scale = amax / (448.0 * 6.0)
         return (*reorder_quantize_x_grouped(x, row_map, scale, reorder_indices, groups, rows_bound, ke, mode), scale)
-    ext = _ext()
     if ext:
-        return ext.quantize_grouped_amax(x, row_map, amax, reorder_indices, groups, rows_bound, ke, mode)
+        return ext.quantize_grouped_amax(x, row_map, amax, reorder_indices, groups, rows_bound, ke, mode, clear)
     lib = _lib.load()
     _require(x, torch.bfloat16, "input")
     _require(amax, torch.float32, "amax")
@@ -532,11 +561,12 @@ def matmul_swiglu(a, b, sfa, sfb, alpha_a: torch.Tensor, alpha_b: torch.Tensor |
 
 
 def matmul_grouped_swiglu(a, b, sfa, sfb, tile_group: torch.Tensor, groups: torch.Tensor, ngroups: int, n: int,
-                          alpha_a: torch.Tensor, alpha_b: torch.Tensor | None = None):
-    """`matmul_grouped` with the SwiGLU epilogue: (act bf16 [rows, n/2], amax fp32 [ngroups])."""
+                          alpha_a: torch.Tensor, alpha_b: torch.Tensor | None = None, onto: torch.Tensor | None = None):
+    """`matmul_grouped` with the SwiGLU epilogue: (act bf16 [rows, n/2], amax fp32 [ngroups]).  onto: the maxima, zero already; nothing
+    is cleared in front of the GEMM then."""
     ext = _ext()
     if ext:
-        return ext.matmul_grouped_swiglu(a, b, sfa, sfb, tile_group, groups, ngroups, n, alpha_a, alpha_b)
+        return ext.matmul_grouped_swiglu(a, b, sfa, sfb, tile_group, groups, ngroups, n, alpha_a, alpha_b, onto)
     lib = _lib.load()
     for t, name in ((a, "A"), (b, "B"), (sfa, "SFA"), (sfb, "SFB")):
         _require(t, torch.uint8, name)
@@ -556,12 +586,15 @@ def matmul_grouped_swiglu(a, b, sfa, sfb, tile_group: torch.Tensor, groups: torc
     if sfa.numel() < ((m + 127) // 128) * atoms * 512 or sfb.numel() < ((ngroups * n + 127) // 128) * atoms * 512:
         raise RuntimeError("scale buffers are smaller than the scale layout of their operands")
     c = torch.empty((m, n // 2), dtype=torch.bfloat16, device=a.device)
-    amax = torch.empty((ngroups,), dtype=torch.float32, device=a.device)
+    amax = torch.empty((ngroups,), dtype=torch.float32, device=a.device) if onto is None else onto
+    _require(amax, torch.float32, "onto")
+    if amax.numel() < ngroups:
+        raise RuntimeError("onto must hold an fp32 value for every matrix")
+    call = lib.arcq_matmul_nvfp4_grouped_swiglu if onto is None else lib.arcq_matmul_nvfp4_grouped_swiglu_onto
     with torch.cuda.device(a.device):
-        rc = lib.arcq_matmul_nvfp4_grouped_swiglu(a.data_ptr(), b.data_ptr(), sfa.data_ptr(), sfb.data_ptr(), m, n, kb * 2,
-                                                  tile_group.data_ptr(), groups.data_ptr(), ngroups, alpha_a.data_ptr(),
-                                                  None if alpha_b is None else alpha_b.data_ptr(), c.data_ptr(),
-                                                  amax.data_ptr(), _stream())
+        rc = call(a.data_ptr(), b.data_ptr(), sfa.data_ptr(), sfb.data_ptr(), m, n, kb * 2, tile_group.data_ptr(), groups.data_ptr(),
+                  ngroups, alpha_a.data_ptr(), None if alpha_b is None else alpha_b.data_ptr(), c.data_ptr(), amax.data_ptr(),
+                  _stream())
     _lib.check(rc, f"grouped swiglu matmul M={m} N={n} K={kb * 2} groups={ngroups}")
     return c, amax
 
@@ -569,6 +602,9 @@ def matmul_grouped_swiglu(a, b, sfa, sfb, tile_group: torch.Tensor, groups: torc
 def moe_combine(y: torch.Tensor, pos: torch.Tensor, weights: torch.Tensor) -> torch.Tensor:
     """out [T, H] = sum_j bf16(y[pos[t, j]] * weights[t, j]) in bf16: the routed copies of every token,
     weighted and added (pos int32 [T, k], weights bf16 [T, k])."""
+    ext = _ext()
+    if ext:
+        return ext.moe_combine(y, pos, weights)
     lib = _lib.load()
     _require(y, torch.bfloat16, "y")
     _require(pos, torch.int32, "pos")
@@ -580,6 +616,26 @@ def moe_combine(y: torch.Tensor, pos: torch.Tensor, weights: torch.Tensor) -> to
                                        y.shape[1], k, _stream())
     _lib.check(rc, "moe_combine")
     return out
+
+
+def native() -> bool:
+    """Whether the extension is there, and with it the calls below that have no other form."""
+    return bool(_ext())
+
+
+def attention_half(*args) -> torch.Tensor:
+    """The attention half of a decoder layer as one call: (x, norm gain, eps, channel order and KE of its input, packed q/k/v weight,
+    its scales and global scale, cos, sin, heads, kv heads, head_dim, bsz, seq, channel order and KE of the o projection, its packed
+    weight, scales and global scale, residual or None)."""
+    ext = _ext()
+    return ext.attention_half(*args)
+
+
+def mlp_half(*args) -> torch.Tensor:
+    """The MLP half: (h, norm gain, eps, channel order and KE, packed interleaved gate/up weight, its scales and global scale, channel
+    order and KE of the down projection, its packed weight, scales and global scale, residual or None)."""
+    ext = _ext()
+    return ext.mlp_half(*args)
 
 
 def gemm_poll_error() -> int:

@@ -68,15 +68,14 @@ class QLinearLayer(nn.Module):
         self.register_buffer("scale_w", scale_w)
         self.register_buffer("scale", scale.reshape(()))
 
-    @torch.no_grad()
     def forward(self, x):
         qx, scale_x, scale, bsz, q_len = x
         if isinstance(scale, torch.Tensor) and scale.is_cuda:
-            y = ops.matmul_dev_alpha(qx, self.W, scale_x, self.scale_w, scale, self.scale, self.bias)
-        else:
+            return ops.linear(qx, self.W, scale_x, self.scale_w, scale, self.scale, self.bias, bsz, q_len)
+        with torch.no_grad():
             y = ops.matmul(qx, self.W, scale_x, self.scale_w, float(scale) * float(self.scale))
             if self.bias is not None:
                 y = y + self.bias
-        if bsz is not None:
-            return y.reshape(bsz, q_len, -1)
-        return y.reshape(q_len, -1)
+            if bsz is not None:
+                return y.reshape(bsz, q_len, -1)
+            return y.reshape(q_len, -1)

@@ -35,3 +35,27 @@ def test_maximum_of_the_swiglu_epilogue_starts_from_zero(rows):
     rc = _lib.load().arcq_matmul_nvfp4_swiglu(a.data_ptr(), b.data_ptr(), sfa.data_ptr(), sfb.data_ptr(), rows, n, k, alpha.data_ptr(),
                                               None, c.data_ptr(), amax.data_ptr(), ops._stream())
     assert rc == 0 and float(amax) == float(c.abs().max()) > 0
+
+
+@pytest.mark.parametrize("rows", [1, 63, 592, 593, 2000])      # row kernel and the kernels of many rows
+@pytest.mark.parametrize("clears", [1, 64])
+def test_quantizers_clear_for_the_launch_behind_them(rows, clears):
+    from arcquant_b200 import _lib, ops
+
+    k, lib = 1024, _lib.load()
+    x, gain = torch.randn(rows, k, device="cuda").bfloat16(), torch.ones(k, device="cuda").bfloat16()
+    idx = torch.randperm(k).to(torch.int16).cuda()
+    store = torch.full((clears + 2,), 7.0, device="cuda")
+    q, sf = ops.rmsnorm_quantize_x(x, gain, 1e-5, idx, 64)
+    q2, sf2 = torch.empty_like(q), torch.empty_like(sf)
+    assert lib.arcq_rmsnorm_quantize_x_clear(x.data_ptr(), gain.data_ptr(), 1e-5, idx.data_ptr(), rows, k, 64, q2.data_ptr(), sf2.data_ptr(),
+                                             store[1:].data_ptr(), clears, ops._stream()) == 0
+    assert torch.equal(q, q2) and store.tolist() == [7.0] + [0.0] * clears + [7.0]
+    groups = torch.tensor([0, 256, 0, rows], dtype=torch.int32, device="cuda")          # (the first run is empty)
+    src, amax, orders = torch.zeros(256 + (rows + 255) // 256 * 256 + 256, k, device="cuda").bfloat16(), torch.ones(2, device="cuda"), idx.repeat(2, 1)
+    src[256:256 + rows] = x
+    store.fill_(7.0)
+    want = ops.quantize_grouped_amax(src, None, amax, orders, groups, src.shape[0], 64)
+    got = ops.quantize_grouped_amax(src, None, amax, orders, groups, src.shape[0], 64, clear=store[1:1 + clears])
+    assert torch.equal(want[0][256:256 + rows], got[0][256:256 + rows]) and torch.equal(want[2], got[2])
+    assert store.tolist() == [7.0] + [0.0] * clears + [7.0]

@@ -1857,15 +1857,18 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
   const bool gamma_ok = !rms || (reinterpret_cast<uintptr_t>(gamma) & 15u) == 0;   // read with 128-bit loads
   const bool wide = p.G > 512;
 
-  // Row kernel: little work per SM.  A unit is a pair of rows and the kernel's resident CTAs take one unit each at
-  // once (three CTAs of up to 256 threads per SM, one of 512), so up to that many units it is a single pass with no
-  // rings to set up.  us, the kernel below / this one: fused RMSNorm of 4096 channels 16 rows 4.1 / 3.3, 592 rows 5.0 /
-  // 4.2; divided by their scale 880 rows 5.5 / 4.9; 14 336 channels 16 rows 6.0 / 4.7, 290 rows 6.3 / 5.0.  Beyond it the
-  // warp-specialised kernel streams better (fused RMSNorm, 16 384 rows: 50.6 / 60.7).  With grouped rows the host knows a bound only.
+  // Row kernel: little work per SM.  A unit is a pair of rows; there are no rings to set up, and the CTAs of an SM hide one another's
+  // latency.  Beyond a few units per SM the warp-specialised kernel streams better (fused RMSNorm, 16 384 x 4096: 50.6 / 60.7).  The line
+  // lies where a CTA would take a second unit (three CTAs of 256 threads per SM, more of narrower rows) and beyond that where the other kernel
+  // has no advantage yet: wide rows, whose half pairs it takes in turn, and grouped rows, of which it gives every run the same number of
+  // CTAs.  us, the kernel below / this one: fused RMSNorm of 4096 channels 16 rows 4.1 / 3.3, 880 rows 6.3 / 5.4 (1200 rows 7.9 / 8.1), of 2048
+  // channels 1700 rows 6.9 / 5.4, of 1024 channels 3500 rows 7.4 / 6.3, of 8192 channels 333 rows 6.8 / 6.3 (1100 rows 9.9 / 10.7); divided by
+  // their scale 880 x 4096 5.5 / 4.9, 1700 x 2048 6.5 / 5.2; plain 333 x 14 336 8.3 / 7.1, 1100 x 14 336 12.9 / 12.1; grouped, eight runs, 1770 x
+  // 4096 10.6 / 8.4, 500 x 14 336 12.6 / 11.0, 1100 x 7168 10.4 / 11.4.  With grouped rows the host knows a bound only.
   const long long real_rows = groups != nullptr ? std::max<long long>(rows - 256LL * ngroups, 1) : rows;
   const long long units = (real_rows + 1) / 2;
   const int T = wide ? ((p.G + 1) / 2 + 31) / 32 * 32 : (p.G + 31) / 32 * 32;
-  const long long per_sm = T <= 256 ? (rms ? 2 : 3) : 1;
+  const long long per_sm = T > 256 ? (wide ? 4 : 2) : (groups != nullptr ? 6 : 3) * 256 / T;
   if (gamma_ok && p.G <= 1024 && !(rms && wide) && (row_map == nullptr || groups != nullptr) && rows < (1LL << 30) &&
       (units <= per_sm * di.num_sms || (p.G < 32 && !rms))) {
 #define ARCQ_ROWS(RMS_, SC_, GR_)                                                                                   \

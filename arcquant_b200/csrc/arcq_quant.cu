@@ -1295,7 +1295,7 @@ arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const
 // together with two shuffles and leave as one 32-bit word per row.
 // RMSNorm: thread t holds chunks t and t + KQ/16, the reference's assignment and summation order (T == KQ/16).
 template <int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB>
-__global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const QuantParams p, const ScaleOptions so) {
+__global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const QuantParams p, const ScaleOptions so, const int share) {
   constexpr int R = 2, CPT = 2 * GPT;                           // rows of a unit, 16-byte chunks per thread and row
   static_assert(!RMS || GPT == 1, "RMSNorm: one group per thread");
   extern __shared__ __align__(16) uint8_t smem[];
@@ -1309,9 +1309,6 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
 
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (so.nclear > 0 && blockIdx.x == 0)
-    for (int i = tid; i < so.nclear; i += T) so.clear[i] = 0.f;
-
   // ---- the rows: one run, or `ngroups` runs (units of R rows are counted through all of them)
   // Lane l of every warp holds runs l and l + 32 (at most 64): first row, rows, and the units up to and including the run,
   // so that the run of a unit is found by a ballot.  (One round trip to memory: 256 rows over 64 runs 11.5 -> 6.0 us
@@ -1319,6 +1316,8 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
   const int ng = GROUPED ? p.ngroups : 1;
   uint32_t t_row0[2] = {0, 0}, t_rows[2] = {0, 0}, t_end[2] = {0, 0};
   uint32_t unit, unit_end, step;
+  // Of the rows it stages a CTA of wide rows quantizes the groups [g_begin, g_end) (see launch_rows).
+  const int g_begin = GPT > 1 ? (int)blockIdx.y * share : 0, g_end = GPT > 1 ? min(G, g_begin + share) : G;
   if (!GROUPED) {
     unit = blockIdx.x;
     unit_end = ((uint32_t)p.rows + R - 1) / R;
@@ -1388,7 +1387,7 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
   auto load_order = [&](const int16_t* idx) {
 #pragma unroll
     for (int j = 0; j < GPT; ++j) {
-      const int g = min(tid + j * T, G - 1);
+      const int g = min(g_begin + tid + j * T, G - 1);
       if (idx == nullptr) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) off[j][k] = word_offset(16 * g + 2 * k) | (word_offset(16 * g + 2 * k + 1) << 16);
@@ -1432,7 +1431,11 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
       asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(reinterpret_cast<uint64_t>(in_row(row0 + tid))), "r"((uint32_t)(KQ * 2)) : "memory");
   };
 
-  if (unit >= unit_end) return;
+  auto clear_for_next = [&]() {      // (last: in front of the loads it cost 0.05 us of a call)
+    if (so.nclear > 0 && blockIdx.x == 0)
+      for (int i = tid; i < so.nclear; i += T) so.clear[i] = 0.f;
+  };
+  if (unit >= unit_end) { clear_for_next(); return; }
   auto rows_of = [&](uint32_t u) -> uint32_t { return min((uint32_t)R, e_rows - (u - e_first) * R); };
   seek(unit);
   auto new_run = [&]() {
@@ -1523,9 +1526,9 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
     uint8_t* sfrow = p.sf + sf_row_base(row0, p.natoms);       // row i of the unit: + 16 i
 #pragma unroll
     for (int j = 0; j < GPT; ++j) {
-      const int g = tid + j * T;
-      if (GPT > 1 && (g & ~31) >= G) break;                    // (whole warps)
-      const bool live = g < G;
+      const int g = g_begin + tid + j * T;
+      if (GPT > 1 && (g & ~31) >= g_end) break;                // (whole warps)
+      const bool live = g < g_end;
       auto gather = [&](uint32_t (&w)[16]) {
 #pragma unroll
         for (int k = 0; k < 16; ++k)
@@ -1597,6 +1600,7 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
       new_run();
     }
   }
+  clear_for_next();
 }
 
 // `nvec` 16-byte words from src to each of n destinations: the codes and scale tiles a rank has just made of
@@ -1705,10 +1709,17 @@ int launch_rows(const QuantParams& p, const ScaleOptions& so, long long units, i
   const size_t share = per_sm < c_occ ? ((size_t)di.max_smem_optin + 1024) / (per_sm + 1) : 0;
   long long grid = di.resident(per_sm);
   if (grid > (p.rows + R - 1) / R) grid = (p.rows + R - 1) / R;
+  // A few wide rows: up to eight CTAs stage the same rows and quantize a part of their groups each, instead of two groups per thread in one
+  // CTA (14 336 channels, us, one CTA per pair of rows / this: plain 16 rows 4.6 / 3.6, 74 rows 4.8 / 3.9, 148 rows 4.8 / 4.2; over their own
+  // maximum 16 rows 7.5 / 6.5.  Rows of 4096 channels, one group per thread already, gain nothing.)
+  int parts = 1;
+  if (GPT > 1 && !GROUPED)
+    while (parts < 8 && 2 * parts * grid <= di.num_sms) parts *= 2;
+  const int groups_each = ((p.G + parts - 1) / parts + 31) & ~31;
   // Programmatic dependent launch: the grid may be set up while the previous kernel of the stream is
   // still draining; the kernel itself waits (griddepcontrol.wait) before it touches global memory.
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
+  cfg.gridDim = dim3((unsigned)grid, (unsigned)((p.G + groups_each - 1) / groups_each));
   cfg.blockDim = dim3((unsigned)T);
   cfg.dynamicSmemBytes = std::max(smem, share);
   cfg.stream = stream;
@@ -1717,7 +1728,7 @@ int launch_rows(const QuantParams& p, const ScaleOptions& so, long long units, i
   attr[0].val.programmaticStreamSerializationAllowed = di.early_start();
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p, so));
+  ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p, so, groups_each));
   return ARCQ_OK;
 }
 

@@ -17,7 +17,10 @@ def _sample(rows):
 
 @pytest.mark.parametrize("rows, k, form", [(888, 4096, "rms"), (889, 4096, "rms"), (1777, 2048, "rms"), (3553, 1024, "rms"), (593, 8192, "rms"),
                                            (591, 5120, "rms"), (1775, 2048, "div"), (1777, 2048, "div"), (592, 7168, "plain"), (594, 5120, "weight"),
-                                           (1184, 14336, "plain"), (1185, 14336, "div"), (700, 16384, "plain"), (333, 11008, "weight")])
+                                           (1184, 14336, "plain"), (1185, 14336, "div"), (700, 16384, "plain"), (333, 11008, "weight"),
+                                           # (a few wide rows: their groups shared by up to eight CTAs)
+                                           (1, 14336, "div"), (16, 8208, "plain"), (36, 11008, "weight"), (37, 16384, "plain"), (74, 14336, "div"),
+                                           (75, 14336, "plain"), (148, 9216, "div"), (149, 14336, "plain")])
 def test_passes_of_the_row_kernel(rows, k, form):
     from arcquant_b200 import ops
 

@@ -33,7 +33,8 @@ struct DeviceInfo {
 int get_device_info(DeviceInfo* out);
 
 // How the divisor of a scaled quantization comes about: `scale` times the factor, or - npartials > 0 - the maximum of
-// that many values at `scale` times the factor; out (device, or null) receives it, per run of grouped rows.
+// that many values at `scale` times the factor, or - npartials < 0, few rows only - the maximum of the tensor itself; out (device, or
+// null) receives it, per run of grouped rows.
 struct ScaleOptions {
   float factor = 1.0f;
   float* out = nullptr;

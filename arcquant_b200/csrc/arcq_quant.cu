@@ -1371,7 +1371,31 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
     fast = div_by_reciprocal_ok(sc);
   };
   if (SCALED) {
-    if (so.npartials > 0) {
+    if (!GROUPED && so.npartials < 0) {      // a small tensor: its maximum, taken by every CTA for itself
+      const uint4* x4 = reinterpret_cast<const uint4*>(p.x);
+      const int nvec = (int)p.rows * nchunks;
+      const uint32_t keep = is_weight ? 0xffffffffu : 0x7fff7fffu;     // (weights: the signed maximum)
+      uint32_t m = is_weight ? 0xff80ff80u : 0u;
+      auto take = [&](uint32_t w) { asm("max.NaN.bf16x2 %0, %0, %1;" : "+r"(m) : "r"(w & keep)); };
+      constexpr int IN = 4;
+      for (int i = tid; i < nvec; i += IN * T) {
+        uint4 v[IN];
+#pragma unroll
+        for (int k = 0; k < IN; ++k) v[k] = __ldcg(x4 + min(i + k * T, nvec - 1));
+#pragma unroll
+        for (int k = 0; k < IN; ++k) { take(v[k].x); take(v[k].y); take(v[k].z); take(v[k].w); }
+      }
+#pragma unroll
+      for (int d = 16; d > 0; d >>= 1) take(__shfl_xor_sync(0xffffffffu, m, d));
+      uint32_t* red = reinterpret_cast<uint32_t*>(smem);
+      if (lane == 0) red[warp] = m;
+      __syncthreads();
+      for (int w = 0; w < (T >> 5); ++w) take(red[w]);
+      __syncthreads();                                          // (the rows are about to be staged there)
+      const float lo = bf16lo(m), hi = bf16hi(m), top = (lo != lo || hi != hi) ? __uint_as_float(0x7fc00000u) : fmaxf(lo, hi);
+      if (blockIdx.x == 0 && tid == 0 && so.out != nullptr) so.out[0] = top * so.factor;
+      set_scale(top * so.factor);
+    } else if (so.npartials > 0) {
       const float m = partials_max(p.scale, so.npartials, lane) * so.factor;
       if (blockIdx.x == 0 && tid == 0 && so.out != nullptr) so.out[0] = m;
       set_scale(m);
@@ -1823,6 +1847,29 @@ int launch_quantize(const void* x, const void* gamma, float eps, const int16_t* 
   return ARCQ_OK;
 }
 
+// Row kernel: little work per SM.  A unit is a pair of rows; there are no rings to set up, and the CTAs of an SM hide one another's
+// latency.  Beyond a few units per SM the warp-specialised kernel streams better (fused RMSNorm, 16 384 x 4096: 50.6 / 60.7).  The line
+// lies where a CTA would take a second unit (three CTAs of 256 threads per SM, more of narrower rows) and beyond that where the other kernel
+// has no advantage yet: wide rows, whose half pairs it takes in turn, and grouped rows, of which it gives every run the same number of
+// CTAs.  us, the kernel below / this one: fused RMSNorm of 4096 channels 16 rows 4.1 / 3.3, 880 rows 6.3 / 5.4 (1200 rows 7.9 / 8.1), of 2048
+// channels 1700 rows 6.9 / 5.4, of 1024 channels 3500 rows 7.4 / 6.3, of 8192 channels 333 rows 6.8 / 6.3 (1100 rows 9.9 / 10.7); divided by
+// their scale 880 x 4096 5.5 / 4.9, 1700 x 2048 6.5 / 5.2; plain 333 x 14 336 8.3 / 7.1, 1100 x 14 336 12.9 / 12.1; grouped, eight runs, 1770 x
+// 4096 10.6 / 8.4, 500 x 14 336 12.6 / 11.0, 1100 x 7168 10.4 / 11.4.  With grouped rows the host knows a bound only.
+struct RowLaunch {
+  long long units;   // pairs of rows (grouped: as far as the host knows)
+  int threads;       // of a CTA
+  bool serves;
+};
+static RowLaunch row_launch(int G, long long rows, int ngroups, const DeviceInfo& di) {
+  const bool wide = G > 512;
+  RowLaunch r;
+  r.units = (std::max<long long>(rows - 256LL * ngroups, 1) + 1) / 2;
+  r.threads = wide ? ((G + 1) / 2 + 31) / 32 * 32 : (G + 31) / 32 * 32;
+  const long long per_sm = r.threads > 256 ? (wide ? 4 : 2) : (ngroups > 0 ? 6 : 3) * 256 / r.threads;
+  r.serves = r.units <= per_sm * di.num_sms;
+  return r;
+}
+
 static int launch_quantize_one(const void* x, const void* gamma, float eps, const int16_t* idx, int64_t rows, int KQ,
                                int KE, int mode, int is_weight, uint8_t* q, uint8_t* sf, cudaStream_t stream,
                                const float* scale, const int* groups, int ngroups, const int* row_map, const ScaleOptions& so) {
@@ -1868,20 +1915,11 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
   const bool gamma_ok = !rms || (reinterpret_cast<uintptr_t>(gamma) & 15u) == 0;   // read with 128-bit loads
   const bool wide = p.G > 512;
 
-  // Row kernel: little work per SM.  A unit is a pair of rows; there are no rings to set up, and the CTAs of an SM hide one another's
-  // latency.  Beyond a few units per SM the warp-specialised kernel streams better (fused RMSNorm, 16 384 x 4096: 50.6 / 60.7).  The line
-  // lies where a CTA would take a second unit (three CTAs of 256 threads per SM, more of narrower rows) and beyond that where the other kernel
-  // has no advantage yet: wide rows, whose half pairs it takes in turn, and grouped rows, of which it gives every run the same number of
-  // CTAs.  us, the kernel below / this one: fused RMSNorm of 4096 channels 16 rows 4.1 / 3.3, 880 rows 6.3 / 5.4 (1200 rows 7.9 / 8.1), of 2048
-  // channels 1700 rows 6.9 / 5.4, of 1024 channels 3500 rows 7.4 / 6.3, of 8192 channels 333 rows 6.8 / 6.3 (1100 rows 9.9 / 10.7); divided by
-  // their scale 880 x 4096 5.5 / 4.9, 1700 x 2048 6.5 / 5.2; plain 333 x 14 336 8.3 / 7.1, 1100 x 14 336 12.9 / 12.1; grouped, eight runs, 1770 x
-  // 4096 10.6 / 8.4, 500 x 14 336 12.6 / 11.0, 1100 x 7168 10.4 / 11.4.  With grouped rows the host knows a bound only.
-  const long long real_rows = groups != nullptr ? std::max<long long>(rows - 256LL * ngroups, 1) : rows;
-  const long long units = (real_rows + 1) / 2;
-  const int T = wide ? ((p.G + 1) / 2 + 31) / 32 * 32 : (p.G + 31) / 32 * 32;
-  const long long per_sm = T > 256 ? (wide ? 4 : 2) : (groups != nullptr ? 6 : 3) * 256 / T;
+  const RowLaunch r = row_launch(p.G, rows, groups != nullptr ? ngroups : 0, di);
+  const long long units = r.units;
+  const int T = r.threads;
   if (gamma_ok && p.G <= 1024 && !(rms && wide) && (row_map == nullptr || groups != nullptr) && rows < (1LL << 30) &&
-      (units <= per_sm * di.num_sms || (p.G < 32 && !rms))) {
+      (r.serves || (p.G < 32 && !rms))) {
 #define ARCQ_ROWS(RMS_, SC_, GR_)                                                                                   \
   {                                                                                                                 \
     if (wide) return launch_rows<2, false, SC_, GR_, false, 512, 1>(p, so, units, T, di, stream);                           \
@@ -2035,6 +2073,15 @@ int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight
     int rc = get_device_info(&di);
     if (rc != ARCQ_OK) return rc;
     const long long nvec = rows * (long long)KQ / 8;
+    // A small tensor's maximum is taken by every CTA of the row kernel for itself, up to 32 loads a thread: less than a second launch costs the
+    // device, and one launch less for the host.  us, two launches / this: 1 x 4096 4.4 / 3.5, 8 x 4096 4.9 / 4.1, 16 x 4096 4.9 / 4.8 (32 x 4096
+    // 4.9 / 5.9), 1 x 14 336 6.1 / 5.0, 4 x 14 336 6.3 / 5.6 (9 x 14 336 6.2 / 6.7), 1 x 512 3.7 / 2.6 (1000 x 64 4.2 / 9.5).
+    const RowLaunch r = row_launch(KQ / 16, rows, 0, di);
+    if (nvec <= 32LL * r.threads && r.serves) {
+      so.npartials = -1;
+      return launch_quantize(x, nullptr, 0.f, idx, rows, KQ, KE, mode, is_weight, q, sf, stream, scratch, groups, ngroups, row_map,
+                             nullptr, nullptr, 0, so);
+    }
     // four 16-byte loads per thread, at most three CTAs per SM
     long long grid = (nvec + 4 * 512 - 1) / (4 * 512);
     if (grid > di.resident(3)) grid = di.resident(3);

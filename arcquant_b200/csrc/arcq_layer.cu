@@ -962,7 +962,7 @@ int launch_route_topk(const void* logits, int64_t tokens, int experts, int top_k
   const long long per_block = 4 * (32 / width);            // four warps
   long long blocks = (tokens + per_block - 1) / per_block;
   if (blocks > (long long)di.num_sms * 16) blocks = (long long)di.num_sms * 16;
-  return launch_dependent(arcq_route_topk_kernel, (unsigned)blocks, 128, 0, di, stream, static_cast<const uint16_t*>(logits),
+  return launch_elementwise(arcq_route_topk_kernel, (unsigned)blocks, 128, di, stream, static_cast<const uint16_t*>(logits),
                           (long long)tokens, experts, width, top_k, ids, static_cast<uint16_t*>(weights));
 }
 
@@ -986,7 +986,7 @@ int launch_moe_combine(const void* y, const int* pos, const void* w, void* out, 
   long long blocks = (total + 255) / 256;
   const long long cap = (long long)di.num_sms * 16;
   if (blocks > cap) blocks = cap;
-  return launch_dependent(arcq_moe_combine_kernel, (unsigned)blocks, 256, 0, di, stream, static_cast<const uint16_t*>(y), pos,
+  return launch_elementwise(arcq_moe_combine_kernel, (unsigned)blocks, 256, di, stream, static_cast<const uint16_t*>(y), pos,
                           static_cast<const uint16_t*>(w), static_cast<uint16_t*>(out), (long long)tokens, hidden, k);
 }
 
@@ -1041,7 +1041,7 @@ int launch_rope(void* x, const float* cos_t, const float* sin_t, int64_t tokens,
   long long blocks = (total + 255) / 256;
   const long long cap = (long long)di.num_sms * 16;
   if (blocks > cap) blocks = cap;
-  return launch_dependent(arcq_rope_kernel, (unsigned)blocks, 256, 0, di, stream, static_cast<uint16_t*>(x), cos_t, sin_t,
+  return launch_elementwise(arcq_rope_kernel, (unsigned)blocks, 256, di, stream, static_cast<uint16_t*>(x), cos_t, sin_t,
                           (long long)tokens, row_elems, heads, dim, seq);
 }
 

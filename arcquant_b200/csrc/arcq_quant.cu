@@ -1935,9 +1935,11 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
 #undef ARCQ_ROWS
   }
 
-  // (Only the row kernel clears by the way.  In the kernels below it cost registers that are all in use, and what is gained by it is
-  // small beside their time.)
-  if (so.nclear > 0) ARCQ_CUDA_TRY(cudaMemsetAsync(so.clear, 0, sizeof(float) * so.nclear, stream));
+  // (Only the row kernel clears by the way: in the kernels below it cost registers that are all in use.)
+  if (so.nclear > 0) {
+    rc = launch_clear(so.clear, so.nclear, stream);
+    if (rc != ARCQ_OK) return rc;
+  }
 
   // Warp-specialised kernel: rows of 512..8192 channels
   // in full, rows of up to 16384 channels for the plain operator.

@@ -1294,8 +1294,13 @@ arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const
 // A warp stores 256 contiguous bytes of codes per row; the scale bytes of four neighbouring groups are brought
 // together with two shuffles and leave as one 32-bit word per row.
 // RMSNorm: thread t holds chunks t and t + KQ/16, the reference's assignment and summation order (T == KQ/16).
-template <int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB>
+// BY: what a launch does by the way.  Asked for at run time, both cost every launch that wants neither 0.1 us (us, asked for / this:
+// plain 1 x 512 2.09 / 1.99, 16 x 5120 2.60 / 2.52; divided by a scale 200 x 4096 3.15 / 3.07, 444 x 5120 4.87 / 4.77; grouped 200 x 2048
+// 3.77 / 3.65).  The fused RMSNorm always has the loop that clears: over none it costs nothing there (1.000 in the mean of 42 sizes).
+enum { BY_NOTHING, BY_CLEAR, BY_OWN_MAX };      // so.clear set to zero; the maximum of the tensor itself taken first
+template <int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB, int BY>
 __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const QuantParams p, const ScaleOptions so, const int share) {
+  static_assert(BY != BY_OWN_MAX || (SCALED && !GROUPED), "the maximum of one tensor");
   constexpr int R = 2, CPT = 2 * GPT;                           // rows of a unit, 16-byte chunks per thread and row
   static_assert(!RMS || GPT == 1, "RMSNorm: one group per thread");
   extern __shared__ __align__(16) uint8_t smem[];
@@ -1371,7 +1376,7 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
     fast = div_by_reciprocal_ok(sc);
   };
   if (SCALED) {
-    if (!GROUPED && so.npartials < 0) {      // a small tensor: its maximum, taken by every CTA for itself
+    if constexpr (BY == BY_OWN_MAX) {        // a small tensor: its maximum, taken by every CTA for itself
       const uint4* x4 = reinterpret_cast<const uint4*>(p.x);
       const int nvec = (int)p.rows * nchunks;
       const uint32_t keep = is_weight ? 0xffffffffu : 0x7fff7fffu;     // (weights: the signed maximum)
@@ -1456,7 +1461,7 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
   };
 
   auto clear_for_next = [&]() {      // (last: in front of the loads it cost 0.05 us of a call)
-    if (so.nclear > 0 && blockIdx.x == 0)
+    if (BY == BY_CLEAR && blockIdx.x == 0)
       for (int i = tid; i < so.nclear; i += T) so.clear[i] = 0.f;
   };
   if (unit >= unit_end) { clear_for_next(); return; }
@@ -1710,10 +1715,10 @@ cudaError_t allow_shared_memory(Kernel kern, const DeviceInfo& di) {
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem_optin);
 }
 
-template <int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB>
+template <int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB, int BY>
 int launch_rows(const QuantParams& p, const ScaleOptions& so, long long units, int T, const DeviceInfo& di, cudaStream_t stream) {
   constexpr int R = 2;
-  auto kern = arcq_quantize_rows_kernel<GPT, RMS, SCALED, GROUPED, PF, MAXT, MINB>;
+  auto kern = arcq_quantize_rows_kernel<GPT, RMS, SCALED, GROUPED, PF, MAXT, MINB, BY>;
   const size_t smem = (size_t)p.KQ * 2 * R + (RMS ? (size_t)(R * T + R) * sizeof(float) : 64);
   // the attribute and the occupancy query cost host time: once per (device, block size, shared memory)
   static thread_local int c_dev = -1, c_threads = 0, c_occ = 0;
@@ -1920,18 +1925,20 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
   const int T = r.threads;
   if (gamma_ok && p.G <= 1024 && !(rms && wide) && (row_map == nullptr || groups != nullptr) && rows < (1LL << 30) &&
       (r.serves || (p.G < 32 && !rms))) {
-#define ARCQ_ROWS(RMS_, SC_, GR_)                                                                                   \
+#define ARCQ_ROWS(RMS_, SC_, GR_, BY_)                                                                              \
   {                                                                                                                 \
-    if (wide) return launch_rows<2, false, SC_, GR_, false, 512, 1>(p, so, units, T, di, stream);                           \
-    return T <= 256 ? launch_rows<1, RMS_, SC_, GR_, true, 256, 3>(p, so, units, T, di, stream)                             \
-                    : launch_rows<1, RMS_, SC_, GR_, true, 512, 1>(p, so, units, T, di, stream);                            \
+    if (wide) return launch_rows<2, false, SC_, GR_, false, 512, 1, BY_>(p, so, units, T, di, stream);              \
+    return T <= 256 ? launch_rows<1, RMS_, SC_, GR_, true, 256, 3, BY_>(p, so, units, T, di, stream)                \
+                    : launch_rows<1, RMS_, SC_, GR_, true, 512, 1, BY_>(p, so, units, T, di, stream);               \
   }
-    if (groups != nullptr && scale != nullptr) ARCQ_ROWS(false, true, true)
-    if (groups != nullptr) ARCQ_ROWS(false, false, true)
-    if (scale != nullptr) ARCQ_ROWS(false, true, false)
-    if (!rms) ARCQ_ROWS(false, false, false)
-    return T <= 256 ? launch_rows<1, true, false, false, true, 256, 3>(p, so, units, T, di, stream)
-                    : launch_rows<1, true, false, false, true, 512, 1>(p, so, units, T, di, stream);
+    if (groups != nullptr && scale != nullptr && so.nclear > 0) ARCQ_ROWS(false, true, true, BY_CLEAR)
+    if (groups != nullptr && scale != nullptr) ARCQ_ROWS(false, true, true, BY_NOTHING)
+    if (groups != nullptr) ARCQ_ROWS(false, false, true, BY_NOTHING)
+    if (scale != nullptr && so.npartials < 0) ARCQ_ROWS(false, true, false, BY_OWN_MAX)
+    if (scale != nullptr) ARCQ_ROWS(false, true, false, BY_NOTHING)
+    if (!rms) ARCQ_ROWS(false, false, false, BY_NOTHING)
+    return T <= 256 ? launch_rows<1, true, false, false, true, 256, 3, BY_CLEAR>(p, so, units, T, di, stream)
+                    : launch_rows<1, true, false, false, true, 512, 1, BY_CLEAR>(p, so, units, T, di, stream);
 #undef ARCQ_ROWS
   }
 

@@ -1855,22 +1855,30 @@ int launch_quantize(const void* x, const void* gamma, float eps, const int16_t* 
 // Row kernel: little work per SM.  A unit is a pair of rows; there are no rings to set up, and the CTAs of an SM hide one another's
 // latency.  Beyond a few units per SM the warp-specialised kernel streams better (fused RMSNorm, 16 384 x 4096: 50.6 / 60.7).  The line
 // lies where a CTA would take a second unit (three CTAs of 256 threads per SM, more of narrower rows) and beyond that where the other kernel
-// has no advantage yet: wide rows, whose half pairs it takes in turn, and grouped rows, of which it gives every run the same number of
-// CTAs.  us, the kernel below / this one: fused RMSNorm of 4096 channels 16 rows 4.1 / 3.3, 880 rows 6.3 / 5.4 (1200 rows 7.9 / 8.1), of 2048
-// channels 1700 rows 6.9 / 5.4, of 1024 channels 3500 rows 7.4 / 6.3, of 8192 channels 333 rows 6.8 / 6.3 (1100 rows 9.9 / 10.7); divided by
-// their scale 880 x 4096 5.5 / 4.9, 1700 x 2048 6.5 / 5.2; plain 333 x 14 336 8.3 / 7.1, 1100 x 14 336 12.9 / 12.1; grouped, eight runs, 1770 x
-// 4096 10.6 / 8.4, 500 x 14 336 12.6 / 11.0, 1100 x 7168 10.4 / 11.4.  With grouped rows the host knows a bound only.
+// has no advantage yet.  us, the kernel below / this one:
+//  * fused RMSNorm of 4096 channels 16 rows 4.1 / 3.3, 880 rows 6.3 / 5.4 (1200 rows 7.9 / 8.1), of 2048 channels 1700 rows 6.9 / 5.4, of 1024
+//    channels 3500 rows 7.4 / 6.3, of 8192 channels 333 rows 6.8 / 6.3 (1100 rows 9.9 / 10.7);
+//  * plain 592 x 5120 4.4 / 3.9, 592 x 14 336 8.0 / 6.8, 1184 x 14 336 12.5 / 11.7: wide rows, whose half pairs the other kernel takes in turn;
+//  * over the tensor's maxima 592 x 5120 4.9 / 4.8, 592 x 14 336 8.9 / 8.3, 1184 x 14 336 13.8 / 14.0, 1184 x 16 384 14.6 / 14.3;
+//  * divided by a given scale 880 x 4096 5.5 / 4.9, 1700 x 2048 6.5 / 5.2, but 444 x 5120 4.6 / 4.8, 592 x 5120 4.7 / 4.8 (592 x 8192 5.7 / 5.6), and
+//    592 x 14 336 8.6 / 8.3, but 740 x 9216 9.3 / 9.8, 1184 x 14 336 13.6 / 14.1: a unit per SM beyond 256 groups, two of wide rows;
+//  * grouped rows: every run has the same number of the other kernel's CTAs, so the rows of the runs decide.  Eight runs of about equal /
+//    of unequal rows: 1400 x 4096 8.3 / 7.8 and 9.3 / 7.9 (1100 x 4096 7.4 / 7.6 and 8.3 / 7.6), 444 x 8192 6.8 / 6.7 and 8.0 / 6.9, 444 x 14 336
+//    9.7 / 9.9 and 12.1 / 10.5.  The host knows a bound of their rows only, whole tiles of 256: of those it takes for 768 x 14 336, 592 are
+//    12.0 / 10.7 and 14.8 / 12.8, 740 12.3 / 14.1 and 14.9 / 14.1; of 1024, 1000 are 15.0 / 16.5 and 17.4 / 17.4.
 struct RowLaunch {
   long long units;   // pairs of rows (grouped: as far as the host knows)
   int threads;       // of a CTA
   bool serves;
 };
-static RowLaunch row_launch(int G, long long rows, int ngroups, const DeviceInfo& di) {
+// given: rows of one run divided by a scale that the caller has.
+static RowLaunch row_launch(int G, long long rows, int ngroups, bool given, const DeviceInfo& di) {
   const bool wide = G > 512;
   RowLaunch r;
   r.units = (std::max<long long>(rows - 256LL * ngroups, 1) + 1) / 2;
   r.threads = wide ? ((G + 1) / 2 + 31) / 32 * 32 : (G + 31) / 32 * 32;
-  const long long per_sm = r.threads > 256 ? (wide ? 4 : 2) : (ngroups > 0 ? 6 : 3) * 256 / r.threads;
+  long long per_sm = (ngroups > 0 ? 6 : 3) * 256 / r.threads;
+  if (r.threads > 256) per_sm = wide ? (given || ngroups > 0 ? 2 : 4) : (given ? 1 : 2);
   r.serves = r.units <= per_sm * di.num_sms;
   return r;
 }
@@ -1920,7 +1928,8 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
   const bool gamma_ok = !rms || (reinterpret_cast<uintptr_t>(gamma) & 15u) == 0;   // read with 128-bit loads
   const bool wide = p.G > 512;
 
-  const RowLaunch r = row_launch(p.G, rows, groups != nullptr ? ngroups : 0, di);
+  const bool given = scale != nullptr && groups == nullptr && so.npartials == 0 && so.out == nullptr;
+  const RowLaunch r = row_launch(p.G, rows, groups != nullptr ? ngroups : 0, given, di);
   const long long units = r.units;
   const int T = r.threads;
   if (gamma_ok && p.G <= 1024 && !(rms && wide) && (row_map == nullptr || groups != nullptr) && rows < (1LL << 30) &&
@@ -2085,7 +2094,7 @@ int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight
     // A small tensor's maximum is taken by every CTA of the row kernel for itself, up to 32 loads a thread: less than a second launch costs the
     // device, and one launch less for the host.  us, two launches / this: 1 x 4096 4.4 / 3.5, 8 x 4096 4.9 / 4.1, 16 x 4096 4.9 / 4.8 (32 x 4096
     // 4.9 / 5.9), 1 x 14 336 6.1 / 5.0, 4 x 14 336 6.3 / 5.6 (9 x 14 336 6.2 / 6.7), 1 x 512 3.7 / 2.6 (1000 x 64 4.2 / 9.5).
-    const RowLaunch r = row_launch(KQ / 16, rows, 0, di);
+    const RowLaunch r = row_launch(KQ / 16, rows, 0, false, di);
     if (nvec <= 32LL * r.threads && r.serves) {
       so.npartials = -1;
       return launch_quantize(x, nullptr, 0.f, idx, rows, KQ, KE, mode, is_weight, q, sf, stream, scratch, groups, ngroups, row_map,

@@ -1932,8 +1932,9 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
   const RowLaunch r = row_launch(p.G, rows, groups != nullptr ? ngroups : 0, given, di);
   const long long units = r.units;
   const int T = r.threads;
+  const bool own_max = so.npartials < 0;      // (decided by the caller, maybe under another SM limit: the row kernel it is)
   if (gamma_ok && p.G <= 1024 && !(rms && wide) && (row_map == nullptr || groups != nullptr) && rows < (1LL << 30) &&
-      (r.serves || (p.G < 32 && !rms))) {
+      (r.serves || own_max || (p.G < 32 && !rms))) {
 #define ARCQ_ROWS(RMS_, SC_, GR_, BY_)                                                                              \
   {                                                                                                                 \
     if (wide) return launch_rows<2, false, SC_, GR_, false, 512, 1, BY_>(p, so, units, T, di, stream);              \
@@ -1943,7 +1944,7 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
     if (groups != nullptr && scale != nullptr && so.nclear > 0) ARCQ_ROWS(false, true, true, BY_CLEAR)
     if (groups != nullptr && scale != nullptr) ARCQ_ROWS(false, true, true, BY_NOTHING)
     if (groups != nullptr) ARCQ_ROWS(false, false, true, BY_NOTHING)
-    if (scale != nullptr && so.npartials < 0) ARCQ_ROWS(false, true, false, BY_OWN_MAX)
+    if (own_max) ARCQ_ROWS(false, true, false, BY_OWN_MAX)
     if (scale != nullptr) ARCQ_ROWS(false, true, false, BY_NOTHING)
     if (!rms) ARCQ_ROWS(false, false, false, BY_NOTHING)
     return T <= 256 ? launch_rows<1, true, false, false, true, 256, 3, BY_CLEAR>(p, so, units, T, di, stream)
@@ -1951,6 +1952,7 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
 #undef ARCQ_ROWS
   }
 
+  if (own_max) return ARCQ_ERR_UNSUPPORTED_K;      // (the kernels below have no maximum to divide by)
   // (Only the row kernel clears by the way: in the kernels below it cost registers that are all in use.)
   if (so.nclear > 0) {
     rc = launch_clear(so.clear, so.nclear, stream);
@@ -2092,10 +2094,10 @@ int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight
     if (rc != ARCQ_OK) return rc;
     const long long nvec = rows * (long long)KQ / 8;
     // A small tensor's maximum is taken by every CTA of the row kernel for itself, up to 32 loads a thread: less than a second launch costs the
-    // device, and one launch less for the host.  us, two launches / this: 1 x 4096 4.4 / 3.5, 8 x 4096 4.9 / 4.1, 16 x 4096 4.9 / 4.8 (32 x 4096
-    // 4.9 / 5.9), 1 x 14 336 6.1 / 5.0, 4 x 14 336 6.3 / 5.6 (9 x 14 336 6.2 / 6.7), 1 x 512 3.7 / 2.6 (1000 x 64 4.2 / 9.5).
+    // device, and one launch less for the host.  us, two launches / this: 4 x 4096 4.8 / 3.8, 16 x 4096 5.1 / 4.6 (32 x 4096 4.9 / 5.9), 16 x
+    // 8192 5.4 / 5.5, 1 x 14 336 7.0 / 4.6, 8 x 14 336 7.1 / 5.9, 16 x 512 4.4 / 3.6 (1000 x 64 4.2 / 9.5).
     const RowLaunch r = row_launch(KQ / 16, rows, 0, false, di);
-    if (nvec <= 32LL * r.threads && r.serves) {
+    if (groups == nullptr && nvec <= 32LL * r.threads && r.serves) {
       so.npartials = -1;
       return launch_quantize(x, nullptr, 0.f, idx, rows, KQ, KE, mode, is_weight, q, sf, stream, scratch, groups, ngroups, row_map,
                              nullptr, nullptr, 0, so);

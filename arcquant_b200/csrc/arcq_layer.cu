@@ -5,7 +5,6 @@
 // Hugging Face `apply_rotary_pos_emb` and `act_fn(gate) * up`); the arithmetic below reproduces the
 // eager torch results bit for bit: every product and sum is rounded to fp32 separately, the same
 // `expf` and IEEE division, bf16 rounding after SiLU and after the product.
-#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -643,30 +642,30 @@ __global__ void arcq_ep_rows_kernel(const uint4* __restrict__ src, const int* __
 // a wave of CTAs each: start, first bytes, way out of the maxima.
 //  * While the batch before is finishing, every CTA pulls its first rows into L2 (a prefetch reads nothing into the CTA, so rows still
 //    being written are not read early).
-//  * The running maxima come into shared memory beside the rows.  A channel meets them in a thread that owns neighbouring ones, and only a
-//    larger value costs an atomic: all of a CTA's in the first batch, few afterwards.  (In the order of the chunks an atomic instruction
-//    touched 32 sectors, 184 us for 4.85 million; clusters of eight that reduced their maxima through distributed shared memory first
+//  * The running maxima come into shared memory beside the rows, and only a larger value costs an atomic: all of a CTA's in the first batch,
+//    few afterwards.  Lane after lane takes channel after channel, so that a warp's atomics are one line of memory.  (A thread that took
+//    two neighbouring channels: the first batch of [2000, 4096] 11.1 instead of 7.8.  In the order of the chunks an atomic instruction
+//    touched 32 sectors, 184 us for 4.85 million.  Clusters of eight that reduced their maxima through distributed shared memory first
 //    spent more on meeting than on the atomics saved.)
-// us, clusters of eight / this: 16 batches of [2000, 4096] in turn 146 / 112, of [200, 4096] 85 / 66, of [1500, 5120] 185 / 125, of
-// [2000, 8192] 219 / 156; one of [2000, 4096] 13.3 / 13.3, of [2000, 8192] 19 / 22, of [20000, 4096] 73 / 46.
-// OUT_CLUSTER: rows of more than 8192 channels still meet in clusters first, their first batch being too many atomics otherwise (four
-// batches, clusters / staged: [500, 16384] 37.9 / 41.0, [300, 28672] 61.5 / 74.8; eight of [2000, 14336] 187 / 140).
-// OUT_DIRECT: a handful of rows, whose maxima go out as they are.
-constexpr int CALIB_THREADS = 512, CALIB_CLUSTER = 8;
-enum { OUT_DIRECT, OUT_STAGED, OUT_CLUSTER };
-template <int CPT, int RB, int OUT>
+// us a batch, clusters of eight / this, a first batch and then one of eight in turn: [500, 2048] 5.6 / 4.4 and 5.7 / 4.5, [2000, 4096] 9.1 / 7.9
+// and 9.0 / 7.1, [20000, 4096] 68 / 39, [2000, 8192] 14.1 / 10.3 and 13.7 / 9.6, [500, 14336] 9.5 / 9.7 and 9.3 / 7.5, [2000, 14336] 23.3 / 17.9
+// and 23.3 / 16.9, [300, 28672] 16.0 / 11.9 and 15.7 / 11.5, [2000, 28672] 49 / 34.  What loses is a first batch of some 200 rows of
+// more than 16384 channels, whose atomics are most of its time: [200, 28672] 9.1 / 10.1 (then 8.8 / 8.5), [200, 32768] 9.4 / 11.1 (9.2 / 9.2).
+// STAGED false: a handful of rows, whose maxima go out as they are.
+constexpr int CALIB_THREADS = 512;
+template <int CPT, int RB, bool STAGED>
 __global__ void __launch_bounds__(CALIB_THREADS, CPT * RB > 8 ? 1 : 2)
 arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, unsigned int* chan_absmax,
                         unsigned long long* above) {
   constexpr int WARPS = CALIB_THREADS / 32;
-  extern __shared__ __align__(16) uint32_t s_col[];           // [K/2]: this CTA's channel maxima, two per word; staged [K]: the running ones
+  extern __shared__ __align__(16) uint32_t s_col[];           // [K/2]: this CTA's channel maxima, two per word; staged [K] more: the running ones
   __shared__ uint32_t s_max[2][WARPS][RB / 2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nchunks = K >> 3;
   uint32_t* s_run = s_col + (K >> 1);
   const bool aligned = (reinterpret_cast<uintptr_t>(chan_absmax) & 15u) == 0;   // (else the running maxima are read in place)
   asm volatile("griddepcontrol.launch_dependents;");
-  if (OUT == OUT_STAGED && tid == 0) {
+  if (STAGED && tid == 0) {
     const long long r0 = (long long)blockIdx.x * RB;
     const long long bytes = min((long long)RB, rows - r0) * K * 2;
     asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(x + r0 * (long long)K), "r"((uint32_t)bytes) : "memory");
@@ -688,7 +687,7 @@ arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, u
         if (c < nchunks && r0 + i < rows) v[i][j] = __ldcs(reinterpret_cast<const uint4*>(x + (r0 + i) * (long long)K) + c);
       }
     }
-    if (OUT == OUT_STAGED && aligned && r0 == (long long)blockIdx.x * RB) {
+    if (STAGED && aligned && r0 == (long long)blockIdx.x * RB) {
       const uint32_t to = (uint32_t)__cvta_generic_to_shared(s_run);
       for (int j = tid; j < (K >> 2); j += CALIB_THREADS)
         asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 16u * j), "l"(chan_absmax + 4 * j) : "memory");
@@ -737,7 +736,7 @@ arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, u
     }
     count += (unsigned int)(above16 >> 4);
   }
-  if constexpr (OUT == OUT_DIRECT) {
+  if constexpr (!STAGED) {
 #pragma unroll
     for (int j = 0; j < CPT; ++j) {
       const int c = tid + j * CALIB_THREADS;
@@ -755,32 +754,12 @@ arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, u
       const int c = tid + j * CALIB_THREADS;
       if (c < nchunks) *reinterpret_cast<uint4*>(s_col + 4 * c) = make_uint4(cmax[j][0], cmax[j][1], cmax[j][2], cmax[j][3]);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    __syncthreads();
     // (non-negative floats order like their bit patterns; a running maximum that is stale by now only costs an atomic)
-    auto meet = [&](int w, uint32_t m, uint32_t run0, uint32_t run1) {
-      if ((m << 16) > run0) atomicMax(chan_absmax + 2 * w, m << 16);
-      if ((m & 0xffff0000u) > run1) atomicMax(chan_absmax + 2 * w + 1, m & 0xffff0000u);
-    };
-    if constexpr (OUT == OUT_STAGED) {
-      asm volatile("cp.async.wait_all;" ::: "memory");
-      __syncthreads();
-      for (int w = tid; w < (K >> 1); w += CALIB_THREADS) {
-        const uint2 run = aligned ? *reinterpret_cast<const uint2*>(s_run + 2 * w) : make_uint2(__ldcg(chan_absmax + 2 * w), __ldcg(chan_absmax + 2 * w + 1));
-        meet(w, s_col[w], run.x, run.y);
-      }
-    } else {
-      namespace cg = cooperative_groups;
-      const cg::cluster_group cluster = cg::this_cluster();
-      cluster.sync();
-      const uint32_t* peers[CALIB_CLUSTER];
-#pragma unroll
-      for (int q = 0; q < CALIB_CLUSTER; ++q) peers[q] = cluster.map_shared_rank(s_col, q);
-      for (int w = (int)cluster.block_rank() * CALIB_THREADS + tid; w < (K >> 1); w += CALIB_CLUSTER * CALIB_THREADS) {
-        uint32_t m = 0;
-#pragma unroll
-        for (int q = 0; q < CALIB_CLUSTER; ++q) asm("max.u16x2 %0, %0, %1;" : "+r"(m) : "r"(peers[q][w]));
-        meet(w, m, __ldcg(chan_absmax + 2 * w), __ldcg(chan_absmax + 2 * w + 1));
-      }
-      cluster.sync();                                          // nobody leaves while its maxima are being read
+    for (int c = tid; c < K; c += CALIB_THREADS) {
+      const uint32_t m = (uint32_t)reinterpret_cast<const uint16_t*>(s_col)[c] << 16;
+      if (m > (aligned ? s_run[c] : __ldcg(chan_absmax + c))) atomicMax(chan_absmax + c, m);
     }
   }
   if (above != nullptr) {
@@ -869,39 +848,23 @@ int launch_calib_stats(const void* x, int64_t rows, int K, float* chan_absmax, u
   const int cpt = (K / 8 + CALIB_THREADS - 1) / CALIB_THREADS;
   auto xs = static_cast<const uint16_t*>(x);
   auto cm = reinterpret_cast<unsigned int*>(chan_absmax);
-  auto launch = [&](auto kern, int rb, int out) -> int {
-    const size_t smem = out == OUT_DIRECT ? 0 : (size_t)K * (out == OUT_STAGED ? 6 : 2);
+  auto launch = [&](auto kern, int rb, bool staged) -> int {
+    const size_t smem = staged ? (size_t)K * 6 : 0;
     // Unasked, a launch gets 48 KB, its static part (below 1 KB here) included.  The limit is the kernel's, not this call's:
     // always the same value, so that calls of several threads and widths cannot lower one another's.
-    if (smem > 47 * 1024) ARCQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * 32768));
-    long long grid = (rows + rb - 1) / rb;
-    if (out != OUT_CLUSTER)
-      return launch_dependent(kern, (unsigned)std::min(grid, di.resident(2)), CALIB_THREADS, smem, di, stream, xs, (long long)rows, K, cm, above);
-    grid = (std::min(grid, 2LL * di.num_sms) + CALIB_CLUSTER - 1) / CALIB_CLUSTER * CALIB_CLUSTER;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(CALIB_THREADS);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = di.early_start();
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = CALIB_CLUSTER;
-    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 2;
-    ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, xs, (long long)rows, K, cm, above));
-    return ARCQ_OK;
+    if (smem > 47 * 1024) ARCQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 6 * 32768));
+    // (one CTA per SM beyond 16384 channels, by its registers and its shared memory)
+    const long long grid = std::min<long long>((rows + rb - 1) / rb, di.resident(cpt > 4 ? 1 : 2));
+    return launch_dependent(kern, (unsigned)grid, CALIB_THREADS, smem, di, stream, xs, (long long)rows, K, cm, above);
   };
   // Up to 64 rows of up to 4096 channels are one step of a few small CTAs, which a look at the running maxima would only lengthen
   // (2048 channels, with clusters / direct: 7 rows 5.5 / 2.5 us, 40 rows 5.3 / 3.4).
-  if (cpt <= 1 && rows <= 64) return launch(arcq_calib_stats_kernel<1, 2, OUT_DIRECT>, 2, OUT_DIRECT);
+  if (cpt <= 1 && rows <= 64) return launch(arcq_calib_stats_kernel<1, 2, false>, 2, false);
   // (rows in flight per CTA: eight 16-byte loads per thread, two rows at least)
-  if (cpt <= 1) return launch(arcq_calib_stats_kernel<1, 8, OUT_STAGED>, 8, OUT_STAGED);
-  if (cpt <= 2) return launch(arcq_calib_stats_kernel<2, 4, OUT_STAGED>, 4, OUT_STAGED);
-  if (cpt <= 4) return launch(arcq_calib_stats_kernel<4, 2, OUT_CLUSTER>, 2, OUT_CLUSTER);
-  if (cpt <= 8) return launch(arcq_calib_stats_kernel<8, 2, OUT_CLUSTER>, 2, OUT_CLUSTER);
+  if (cpt <= 1) return launch(arcq_calib_stats_kernel<1, 8, true>, 8, true);
+  if (cpt <= 2) return launch(arcq_calib_stats_kernel<2, 4, true>, 4, true);
+  if (cpt <= 4) return launch(arcq_calib_stats_kernel<4, 2, true>, 2, true);
+  if (cpt <= 8) return launch(arcq_calib_stats_kernel<8, 2, true>, 2, true);
   return ARCQ_ERR_UNSUPPORTED_K;
 }
 

@@ -19,6 +19,7 @@ ERR_CUDA = 4
 ERR_ALIGNMENT = 5
 ERR_TIMEOUT = 6
 ERR_SCRATCH_LIMIT = 7
+ERR_OVERLAP = 8
 STATIC_SCRATCH_BYTES = 2 << 20
 SCALE_SCRATCH = 512
 

@@ -46,6 +46,16 @@ int get_device_info(DeviceInfo* out) {
 
 static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
+// Whether n floats at p and `bytes` bytes at q have a byte in common.
+static bool overlap(const float* p, int n, const void* q, int64_t bytes) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p), b = reinterpret_cast<uintptr_t>(q);
+  return q != nullptr && n > 0 && bytes > 0 && a < b + (uintptr_t)bytes && b < a + sizeof(float) * n;
+}
+// ... and the codes and scales of `rows` quantized rows.
+static bool overlap_packed(const float* p, int n, const uint8_t* q, const uint8_t* sf, int64_t rows, int64_t k_eff) {
+  return overlap(p, n, q, rows * (k_eff / 2)) || overlap(p, n, sf, (rows + 127) / 128 * ((k_eff / 16 + 3) / 4) * 512);
+}
+
 static int check_quant_shape(int64_t rows, int KQ, int KE, int mode) {
   if (rows < 0 || KQ <= 0 || KE < 0 || KE > KQ) return ARCQ_ERR_BAD_SHAPE;
   if (mode != ARCQ_MODE_16 && mode != ARCQ_MODE_32) return ARCQ_ERR_BAD_SHAPE;
@@ -73,6 +83,7 @@ const char* arcq_status_string(int status) {
     case ARCQ_ERR_SCRATCH_LIMIT:
       return "problem needs more scratch than the built-in 2 MiB block of arcq_matmul_nvfp4_static; "
              "use arcq_matmul_nvfp4_ws with caller-provided scratch";
+    case ARCQ_ERR_OVERLAP: return "memory to be set overlaps an input or another output";
     default: return "unknown status";
   }
 }
@@ -147,6 +158,10 @@ int arcq_quantize_x_grouped_amax_clear(const void* x, const int32_t* row_map, co
   }
   if (!x || !amax || !groups || !qx || !sfx || !scale_out) return ARCQ_ERR_NULL_POINTER;
   if (!aligned16(x) || !aligned16(qx)) return ARCQ_ERR_ALIGNMENT;
+  if (overlap(clear, nclear, amax, 4LL * ngroups) || overlap(clear, nclear, groups, 8LL * ngroups) || overlap(clear, nclear, scale_out, 4LL * ngroups) ||
+      overlap(clear, nclear, reorder_indices, 2LL * ngroups * KQ) || overlap(clear, nclear, row_map, 4 * rows_bound) ||
+      (!row_map && overlap(clear, nclear, x, 2 * rows_bound * KQ)) || overlap_packed(clear, nclear, qx, sfx, rows_bound, KQ + KE))
+    return ARCQ_ERR_OVERLAP;
   return launch_quantize_tensor_scale(x, amax, 0, reorder_indices, rows_bound, KQ, KE, mode, qx, sfx, scale_out, nullptr,
                                       (cudaStream_t)stream, groups, ngroups, row_map, clear, nclear);
 }
@@ -172,6 +187,9 @@ int arcq_rmsnorm_quantize_x_clear(const void* x, const void* gamma, float eps, c
   }
   if (!x || !gamma || !qx || !sfx) return ARCQ_ERR_NULL_POINTER;
   if (!aligned16(x) || !aligned16(qx)) return ARCQ_ERR_ALIGNMENT;
+  if (overlap(clear, nclear, x, 2 * M * KQ) || overlap(clear, nclear, gamma, 2LL * KQ) || overlap(clear, nclear, reorder_index, 2LL * KQ) ||
+      overlap_packed(clear, nclear, qx, sfx, M, KQ + KE))
+    return ARCQ_ERR_OVERLAP;
   ScaleOptions so;
   so.clear = clear;
   so.nclear = nclear;

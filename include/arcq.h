@@ -43,6 +43,7 @@ extern "C" {
 #define ARCQ_ERR_ALIGNMENT 5      /* a pointer is not 16-byte aligned */
 #define ARCQ_ERR_TIMEOUT 6        /* a bounded device-side wait expired (reported by arcq_gemm_poll_error) */
 #define ARCQ_ERR_SCRATCH_LIMIT 7  /* arcq_matmul_nvfp4_static: the shape needs more than its built-in scratch */
+#define ARCQ_ERR_OVERLAP 8        /* memory that a call sets overlaps memory that it also reads, or another output */
 
 /* Channel-layout family of the critical groups.
  * 16: one group per slot  - [main][residual] per critical group
@@ -111,7 +112,9 @@ int arcq_quantize_x_grouped_amax(const void* x, const int32_t* row_map, const fl
                                  const int32_t* groups, int ngroups, int64_t rows_bound, int KQ, int KE, int mode,
                                  uint8_t* qx, uint8_t* sfx, float* scale_out, void* stream);
 /* arcq_quantize_x_grouped_amax, which also sets the nclear floats at `clear` (device, at most 64) to zero: the maxima that an
- * arcq_matmul_nvfp4_grouped_swiglu_onto behind it collects. */
+ * arcq_matmul_nvfp4_grouped_swiglu_onto behind it collects.  When within the call they are set is not specified: they must be none of the
+ * call's inputs (amax, say) or other outputs.  ARCQ_ERR_OVERLAP if they are; with a row_map the extent of x is not known here, and an overlap with
+ * x not found. */
 int arcq_quantize_x_grouped_amax_clear(const void* x, const int32_t* row_map, const float* amax, const int16_t* reorder_indices,
                                        const int32_t* groups, int ngroups, int64_t rows_bound, int KQ, int KE, int mode,
                                        uint8_t* qx, uint8_t* sfx, float* scale_out, float* clear, int nclear, void* stream);
@@ -136,7 +139,7 @@ int arcq_reorder_quantize_x_scaled(const void* x, const float* scale, const int1
 int arcq_rmsnorm_quantize_x(const void* x, const void* gamma, float eps, const int16_t* reorder_index,
                             int64_t M, int KQ, int KE, uint8_t* qx, uint8_t* sfx, void* stream);
 /* arcq_rmsnorm_quantize_x, which also sets the nclear floats at `clear` (device, at most 64) to zero: the maximum that an
- * arcq_matmul_nvfp4_swiglu_onto behind it collects. */
+ * arcq_matmul_nvfp4_swiglu_onto behind it collects.  As above: ARCQ_ERR_OVERLAP if they are an input or another output. */
 int arcq_rmsnorm_quantize_x_clear(const void* x, const void* gamma, float eps, const int16_t* reorder_index,
                                   int64_t M, int KQ, int KE, uint8_t* qx, uint8_t* sfx, float* clear, int nclear, void* stream);
 

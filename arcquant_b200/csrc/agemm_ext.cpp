@@ -67,7 +67,7 @@ std::tuple<int64_t, int64_t, int64_t> check_gemm_operands(const torch::Tensor& A
 
 std::tuple<torch::Tensor, torch::Tensor> quantize_common(const torch::Tensor& X, const torch::Tensor* gamma,
                                                          float eps, const torch::Tensor& reorder_index, int KE,
-                                                         bool is_weight, const char* where, torch::Tensor* clear = nullptr) {
+                                                         bool is_weight, const char* where, const torch::Tensor* clear = nullptr) {
   require_cuda(X, "input");
   require_on(reorder_index, X, at::kShort, "reorder_index");
   TORCH_CHECK(X.dim() == 2, "input must be 2-D");
@@ -85,6 +85,7 @@ std::tuple<torch::Tensor, torch::Tensor> quantize_common(const torch::Tensor& X,
   if (gamma) {
     require_on(*gamma, X, at::kBFloat16, "weight");
     TORCH_CHECK(gamma->numel() == KQ, "weight must have KQ entries");
+    if (clear) require_on(*clear, X, at::kFloat, "clear");
     status = arcq_rmsnorm_quantize_x_clear(px, gamma->data_ptr<at::BFloat16>(), eps, pidx, rows, KQ, KE, Q.data_ptr<uint8_t>(),
                                            SF.data_ptr<uint8_t>(), clear ? clear->data_ptr<float>() : nullptr,
                                            clear ? static_cast<int>(clear->numel()) : 0, current_stream(X));
@@ -172,8 +173,8 @@ std::tuple<torch::Tensor, torch::Tensor> reorder_quantize_w(const torch::Tensor&
 
 std::tuple<torch::Tensor, torch::Tensor> rmsnorm_quantize_x(const torch::Tensor& X, const torch::Tensor& W,
                                                             const float eps, const torch::Tensor& reorder_index,
-                                                            const int KE) {
-  return quantize_common(X, &W, eps, reorder_index, KE, false, "run_rmsnorm_x_bf16_nvfp4");
+                                                            const int KE, const c10::optional<torch::Tensor>& clear) {
+  return quantize_common(X, &W, eps, reorder_index, KE, false, "run_rmsnorm_x_bf16_nvfp4", clear.has_value() ? &*clear : nullptr);
 }
 
 // ---- extras without a counterpart in the reference's bindings (its layers call torch for these) ----
@@ -267,10 +268,13 @@ torch::Tensor swiglu(const torch::Tensor& A, const torch::Tensor& B, const torch
 }
 std::tuple<torch::Tensor, torch::Tensor> matmul_swiglu(const torch::Tensor& A, const torch::Tensor& B, const torch::Tensor& SFA,
                                                        const torch::Tensor& SFB, const torch::Tensor& alpha_a,
-                                                       const c10::optional<torch::Tensor>& alpha_b) {
+                                                       const c10::optional<torch::Tensor>& alpha_b,
+                                                       const c10::optional<torch::Tensor>& onto) {
   require_cuda(A, "A");
-  auto amax = empty_on(A, {}, at::kFloat);
-  return std::make_tuple(swiglu(A, B, SFA, SFB, alpha_a, alpha_b, amax, arcq_matmul_nvfp4_swiglu), amax);
+  if (onto.has_value()) factors(*onto, A, 1, "onto");
+  auto amax = onto.has_value() ? *onto : empty_on(A, {}, at::kFloat);
+  auto call = onto.has_value() ? arcq_matmul_nvfp4_swiglu_onto : arcq_matmul_nvfp4_swiglu;
+  return std::make_tuple(swiglu(A, B, SFA, SFB, alpha_a, alpha_b, amax, call), amax);
 }
 
 // The grouped forms; groups: the run table [first rows | rows] of exactly these runs (in a table of more the row counts lie
@@ -540,7 +544,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("reorder_quantize_w", &reorder_quantize_w, "Reorder and quantize weight.", py::arg("W"),
         py::arg("reorder_index"), py::arg("KE"));
   m.def("rmsnorm_quantize_x", &rmsnorm_quantize_x, "RMSNorm, reorder and quantize activation.", py::arg("X"),
-        py::arg("W"), py::arg("eps"), py::arg("reorder_index"), py::arg("KE"));
+        py::arg("W"), py::arg("eps"), py::arg("reorder_index"), py::arg("KE"), py::arg("clear") = py::none());
   m.def("matmul_dev_alpha", &matmul_dev_alpha, "gemm with device-resident global scales", py::arg("A"),
         py::arg("B"), py::arg("SFA"), py::arg("SFB"), py::arg("alpha_a"), py::arg("alpha_b") = py::none(),
         py::arg("bias") = py::none());
@@ -562,7 +566,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         py::arg("reorder_index"), py::arg("KE"), py::arg("mode") = -1, py::arg("is_weight") = false,
         py::arg("amax") = py::none());
   m.def("matmul_swiglu", &matmul_swiglu, "gate/up GEMM with SwiGLU: (act, amax)", py::arg("A"), py::arg("B"), py::arg("SFA"),
-        py::arg("SFB"), py::arg("alpha_a"), py::arg("alpha_b"));
+        py::arg("SFB"), py::arg("alpha_a"), py::arg("alpha_b"), py::arg("onto") = py::none());
   m.def("matmul_grouped_swiglu", &matmul_grouped_swiglu, "its grouped form", py::arg("A"), py::arg("B"), py::arg("SFA"), py::arg("SFB"),
         py::arg("tile_group"), py::arg("groups"), py::arg("ngroups"), py::arg("n"), py::arg("alpha_a"), py::arg("alpha_b"),
         py::arg("onto") = py::none());

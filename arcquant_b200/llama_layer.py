@@ -154,7 +154,8 @@ class PackedLinear(torch.nn.Module):
 
 class PhaseTimer:
     """Per-phase device time of a step (CUDA events around each phase; eager runs only - it synchronises
-    when read).  Phases: quantize, gemm, attention, glue, collective."""
+    when read).  Phases: quantize, gemm, attention, glue, collective.  A timed step makes the same launches as any other, but one
+    operation after the other from Python instead of half a layer per call: its times are the device's, its gaps are not."""
 
     def __init__(self):
         self.spans = []
@@ -247,10 +248,11 @@ class QLlamaDecoderLayerTP(torch.nn.Module):
         self.register_buffer("fuse_swiglu_t", torch.tensor(int(self.fuse_swiglu), dtype=torch.int32))
         return self
 
-    def _gate_up_act(self, a: torch.Tensor, sfa: torch.Tensor):
-        """(silu(gate) * up [tokens, ffn / tp], its max|.|) from the quantized input of the gate/up projection."""
+    def _gate_up_act(self, a: torch.Tensor, sfa: torch.Tensor, onto: torch.Tensor | None = None):
+        """(silu(gate) * up [tokens, ffn / tp], its max|.|) from the quantized input of the gate/up projection; onto: the maximum,
+        cleared already (fused SwiGLU)."""
         if self.fuse_swiglu:
-            return ops.matmul_swiglu(a, self.gate_up.W, sfa, self.gate_up.SFW, self.gate_up.scale, None)
+            return ops.matmul_swiglu(a, self.gate_up.W, sfa, self.gate_up.SFW, self.gate_up.scale, None, onto)
         return ops.silu_mul(self.gate_up.gemm(a, sfa))
 
     def _native(self, x2d: torch.Tensor, k_row: int) -> bool:
@@ -299,10 +301,11 @@ class QLlamaDecoderLayerTP(torch.nn.Module):
             gb, db = gu._buffers, down._buffers
             return ops.mlp_half(h2d, self.ln2, cfg.eps, gb["index"], gu.select_num, gb["W"], gb["SFW"], gb["scale"], db["index"],
                                 down.select_num, db["W"], db["SFW"], db["scale"], residual)
+        amax = torch.empty((), dtype=torch.float32, device=h2d.device) if self.fuse_swiglu else None
         with self._ph("quantize"):
-            a, sfa = ops.rmsnorm_quantize_x(h2d, self.ln2, cfg.eps, self.gate_up.index, self.gate_up.select_num)
+            a, sfa = ops.rmsnorm_quantize_x(h2d, self.ln2, cfg.eps, self.gate_up.index, self.gate_up.select_num, clear=amax)
         with self._ph("gemm"):
-            act, amax = self._gate_up_act(a, sfa)      # silu(gate) * up and its max|.| with the GEMM
+            act, amax = self._gate_up_act(a, sfa, amax)      # silu(gate) * up and its max|.| with the GEMM
         with self._ph("quantize"):
             qd, sfd, sd = NVFP4_reorder_quantize_x(act, self.down.index, self.down.select_num, mode=16, amax=amax)
         with self._ph("gemm"):

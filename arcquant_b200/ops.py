@@ -75,7 +75,7 @@ def reference_mode(kq: int) -> int:
     return int(_lib.load().arcq_reference_mode(kq))
 
 
-def _quantize(kind: str, x, gamma, eps, reorder_index, ke: int, mode, out=None, scale=None):
+def _quantize(kind: str, x, gamma, eps, reorder_index, ke: int, mode, out=None, scale=None, clear=None):
     lib = _lib.load()
     _require(x, torch.bfloat16, "input")
     if x.dim() != 2:
@@ -117,8 +117,11 @@ def _quantize(kind: str, x, gamma, eps, reorder_index, ke: int, mode, out=None, 
                                              sf.data_ptr(), _stream())
         else:
             _require(gamma, torch.bfloat16, "weight")
-            rc = lib.arcq_rmsnorm_quantize_x(x.data_ptr(), gamma.data_ptr(), float(eps), idx_ptr, rows, kq, ke,
-                                             q.data_ptr(), sf.data_ptr(), _stream())
+            if clear is not None:
+                _require(clear, torch.float32, "clear")
+            rc = lib.arcq_rmsnorm_quantize_x_clear(x.data_ptr(), gamma.data_ptr(), float(eps), idx_ptr, rows, kq, ke,
+                                                   q.data_ptr(), sf.data_ptr(), None if clear is None else clear.data_ptr(),
+                                                   0 if clear is None else clear.numel(), _stream())
     _lib.check(rc, f"{kind}-quantize KQ={kq} KE={ke}")
     return q, sf
 
@@ -172,12 +175,13 @@ def quantize_tensor_scale(x, reorder_index, ke: int, mode=None, is_weight: bool 
     return q, sf, scale
 
 
-def rmsnorm_quantize_x(x, weight, eps: float, reorder_index, ke: int, out=None):
-    """RMSNorm(x)*weight fused in front of reorder_quantize_x."""
+def rmsnorm_quantize_x(x, weight, eps: float, reorder_index, ke: int, out=None, clear: torch.Tensor | None = None):
+    """RMSNorm(x)*weight fused in front of reorder_quantize_x.  clear: up to 64 fp32 values, neither read nor written otherwise by the
+    call, set to zero by the way (see `matmul_swiglu`)."""
     ext = _ext()
     if ext and out is None and reorder_index is not None:
-        return ext.rmsnorm_quantize_x(x, weight, float(eps), reorder_index, ke)
-    return _quantize("rms", x, weight, eps, reorder_index, ke, _lib.MODE_16, out)
+        return ext.rmsnorm_quantize_x(x, weight, float(eps), reorder_index, ke, clear)
+    return _quantize("rms", x, weight, eps, reorder_index, ke, _lib.MODE_16, out, clear=clear)
 
 
 def _matmul(a, b, sfa, sfb, alpha: float, alpha_a, alpha_b) -> torch.Tensor:
@@ -529,12 +533,13 @@ def interleave_gate_up(w_gate: torch.Tensor, w_up: torch.Tensor, block: int = 12
     return torch.stack([w_gate.reshape(f // block, block, k), w_up.reshape(f // block, block, k)], dim=1).reshape(2 * f, k)
 
 
-def matmul_swiglu(a, b, sfa, sfb, alpha_a: torch.Tensor, alpha_b: torch.Tensor | None = None):
+def matmul_swiglu(a, b, sfa, sfb, alpha_a: torch.Tensor, alpha_b: torch.Tensor | None = None, onto: torch.Tensor | None = None):
     """(act bf16 [M, N/2], amax 0-dim fp32): gate/up GEMM over an interleaved weight (`interleave_gate_up`) with
-    silu(gate) * up and its max|.| taken in the epilogue."""
+    silu(gate) * up and its max|.| taken in the epilogue.  onto: the maximum, zero already (`rmsnorm_quantize_x` clears it by the way);
+    nothing is cleared in front of the GEMM then."""
     ext = _ext()
     if ext:
-        return ext.matmul_swiglu(a, b, sfa, sfb, alpha_a, alpha_b)
+        return ext.matmul_swiglu(a, b, sfa, sfb, alpha_a, alpha_b, onto)
     lib = _lib.load()
     for t, name in ((a, "A"), (b, "B"), (sfa, "SFA"), (sfb, "SFB")):
         _require(t, torch.uint8, name)
@@ -551,11 +556,14 @@ def matmul_swiglu(a, b, sfa, sfb, alpha_a: torch.Tensor, alpha_b: torch.Tensor |
     if sfa.numel() < ((m + 127) // 128) * atoms * 512 or sfb.numel() < (n // 128) * atoms * 512:
         raise RuntimeError("scale buffers are smaller than the scale layout of their operands")
     c = torch.empty((m, n // 2), dtype=torch.bfloat16, device=a.device)
-    amax = torch.empty((), dtype=torch.float32, device=a.device)
+    amax = torch.empty((), dtype=torch.float32, device=a.device) if onto is None else onto
+    _require(amax, torch.float32, "onto")
+    if amax.numel() < 1:
+        raise RuntimeError("onto must hold an fp32 value")
+    call = lib.arcq_matmul_nvfp4_swiglu if onto is None else lib.arcq_matmul_nvfp4_swiglu_onto
     with torch.cuda.device(a.device):
-        rc = lib.arcq_matmul_nvfp4_swiglu(a.data_ptr(), b.data_ptr(), sfa.data_ptr(), sfb.data_ptr(), m, n, kb * 2,
-                                          alpha_a.data_ptr(), None if alpha_b is None else alpha_b.data_ptr(),
-                                          c.data_ptr(), amax.data_ptr(), _stream())
+        rc = call(a.data_ptr(), b.data_ptr(), sfa.data_ptr(), sfb.data_ptr(), m, n, kb * 2, alpha_a.data_ptr(),
+                  None if alpha_b is None else alpha_b.data_ptr(), c.data_ptr(), amax.data_ptr(), _stream())
     _lib.check(rc, f"swiglu matmul M={m} N={n} K={kb * 2}")
     return c, amax
 

@@ -111,9 +111,10 @@ def sf_take_rows(sf, rows, k_eff: int) -> np.ndarray:
     return out
 
 
-def launched_kernels(fn):
+def launched_kernels(fn, every=False):
     """[(mangled name, CTAs, bytes of local memory per thread)] of the kernels that fn() launches, in order, read from a
-    stream capture of it.  fn runs once beforehand, so that nothing is loaded for the first time inside the capture."""
+    stream capture of it.  fn runs once beforehand, so that nothing is loaded for the first time inside the capture.
+    every: memsets and copies too, as ("node type N", 0, 0)."""
     import ctypes as C
 
     class Params(C.Structure):      # CUDA_KERNEL_NODE_PARAMS
@@ -136,6 +137,8 @@ def launched_kernels(fn):
         kind, local, p, name = C.c_int(-1), C.c_int(-1), Params(), C.c_char_p()
         assert cu.cuGraphNodeGetType(C.c_void_p(node), C.byref(kind)) == 0
         if kind.value != 0:          # (a memset, a copy)
+            if every:
+                out.append((f"node type {kind.value}", 0, 0))
             continue
         assert cu.cuGraphKernelNodeGetParams_v2(C.c_void_p(node), C.byref(p)) == 0
         func = C.c_void_p(p.func)

@@ -152,6 +152,14 @@ class PackedLinear(torch.nn.Module):
         return ops.matmul_dev_alpha(qx, self.W, sfx, self.SFW, scale_x, self.scale)
 
 
+_GEMM, _SDPA, _NEEDED = PackedLinear.gemm, torch._C._nn.scaled_dot_product_attention, {"W", "SFW", "scale", "index"}
+
+
+def _as_built(lin) -> bool:
+    """Whether a linear is a `PackedLinear` as its class makes it, and its buffers and nothing else are what it computes with."""
+    return type(lin) is PackedLinear and getattr(lin.gemm, "__func__", None) is _GEMM and lin._buffers.keys() >= _NEEDED
+
+
 class PhaseTimer:
     """Per-phase device time of a step (CUDA events around each phase; eager runs only - it synchronises
     when read).  Phases: quantize, gemm, attention, glue, collective.  A timed step makes the same launches as any other, but one
@@ -255,17 +263,21 @@ class QLlamaDecoderLayerTP(torch.nn.Module):
             return ops.matmul_swiglu(a, self.gate_up.W, sfa, self.gate_up.SFW, self.gate_up.scale, None, onto)
         return ops.silu_mul(self.gate_up.gemm(a, sfa))
 
-    def _native(self, x2d: torch.Tensor, k_row: int) -> bool:
-        """Whether a half of the layer may run as one call into the extension: not while phases are timed, and not for what the
-        quantizer of the row-parallel input leaves to torch (no rows, or rows of more than 16384 channels)."""
-        return self.timer is None and x2d.shape[0] > 0 and k_row <= 16384 and ops.native()
+    def _native(self, x2d: torch.Tensor, k_row: int, *linears) -> bool:
+        """Whether a half of the layer may run as one call into the extension: not while phases are timed, not for what the
+        quantizer of the row-parallel input leaves to torch (no rows, or rows of more than 16384 channels), and not where a caller has
+        put something of their own in a place that the call would pass by: a linear of another class, with another `gemm` or with
+        parameters for buffers, or a torch function mode."""
+        return (self.timer is None and x2d.shape[0] > 0 and k_row <= 16384 and ops.native()
+                and not torch._C._is_torch_function_mode_enabled() and all(_as_built(lin) for lin in linears))
 
     # ---- halves of the layer up to (and excluding) the all-reduce: usable for in-process emulation
     @torch.no_grad()
     def attn_partial(self, x2d: torch.Tensor, bsz: int, seq: int, positions: torch.Tensor,
                      residual: torch.Tensor | None = None) -> torch.Tensor:
         cfg, D = self.cfg, self.cfg.head_dim
-        if self._native(x2d, self.h_local * D):      # what follows, in one native call
+        if F.scaled_dot_product_attention is _SDPA and self._native(x2d, self.h_local * D, self.qkv, self.o):
+            # what follows, in one native call
             qkv, o = self.qkv, self.o
             qb, ob = qkv._buffers, o._buffers
             cos, sin = rope_tables(positions, D, cfg.rope_theta)
@@ -296,7 +308,8 @@ class QLlamaDecoderLayerTP(torch.nn.Module):
     @torch.no_grad()
     def mlp_partial(self, h2d: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
         cfg = self.cfg
-        if self.fuse_swiglu and self._native(h2d, self.f_local):      # what follows, in one native call
+        if (self.fuse_swiglu and getattr(self._gate_up_act, "__func__", None) is QLlamaDecoderLayerTP._gate_up_act
+                and self._native(h2d, self.f_local, self.gate_up, self.down)):      # what follows, in one native call
             gu, down = self.gate_up, self.down
             gb, db = gu._buffers, down._buffers
             return ops.mlp_half(h2d, self.ln2, cfg.eps, gb["index"], gu.select_num, gb["W"], gb["SFW"], gb["scale"], db["index"],

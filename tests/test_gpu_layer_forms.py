@@ -79,3 +79,73 @@ def test_the_cleared_maximum_of_the_public_operators(rows, monkeypatch):
         assert torch.equal(a, a2) and torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
         with pytest.raises(RuntimeError):
             ops.rmsnorm_quantize_x(x, layer.ln2, 1e-5, gu.index, gu.select_num, clear=torch.zeros(65, device="cuda"))
+
+
+class _Doubled:
+    """A linear that is no `PackedLinear`: twice the product of one."""
+
+    def __init__(self, lin):
+        self.lin, self.index, self.select_num, self.W, self.SFW, self.scale = lin, lin.index, lin.select_num, lin.W, lin.SFW, lin.scale
+
+    def gemm(self, qx, sfx, scale_x=None, residual=None):
+        y = 2 * self.lin.gemm(qx, sfx, scale_x)
+        return y if residual is None else residual + y
+
+
+@pytest.mark.parametrize("name", ["qkv", "o", "down"])
+@pytest.mark.parametrize("how", ["instance", "class", "subclass", "module"])
+def test_a_linear_of_the_callers_own_is_called(name, how, monkeypatch):
+    from arcquant_b200.llama_layer import PackedLinear
+
+    layer = _layer(8, 4)
+    x, pos = torch.randn(130, 1024, device="cuda").bfloat16(), torch.arange(65, device="cuda")
+    before = _halves(layer, x, 2, pos, False)
+    lin, gemm = getattr(layer, name), PackedLinear.gemm
+    if how == "instance":
+        lin.gemm = lambda *a, **k: 2 * gemm(lin, *a, **k)
+    elif how == "class":
+        monkeypatch.setattr(PackedLinear, "gemm", lambda self, *a, **k: gemm(self, *a, **k) * (2 if self is lin else 1))
+    elif how == "subclass":
+        lin.__class__ = type("Own", (PackedLinear,), {"gemm": lambda self, *a, **k: 2 * gemm(self, *a, **k)})
+    else:
+        delattr(layer, name)
+        setattr(layer, name, _Doubled(lin))
+    after = _halves(layer, x, 2, pos, False)
+    if name == "qkv":       # (twice q, k and v: not twice the output, but another one)
+        assert not torch.equal(after[0], before[0]) and torch.equal(after[1], before[1])
+    else:
+        changed = 0 if name == "o" else 1
+        assert torch.equal(after[changed], 2 * before[changed]) and torch.equal(after[1 - changed], before[1 - changed])
+
+
+def test_parameters_for_buffers():
+    layer = _layer(8, 4)
+    x, pos = torch.randn(130, 1024, device="cuda").bfloat16(), torch.arange(65, device="cuda")
+    before = _halves(layer, x, 2, pos, False)
+    for lin in (layer.qkv, layer.o, layer.gate_up, layer.down):
+        scale = 2 * lin.scale
+        del lin.scale
+        lin.scale = torch.nn.Parameter(scale, requires_grad=False)
+    after = _halves(layer, x, 2, pos, False)
+    assert after[0].shape == before[0].shape and not torch.equal(after[0], before[0]) and not torch.equal(after[1], before[1])
+
+
+def test_another_attention_is_called(monkeypatch):
+    import torch.nn.functional as F
+    from torch.overrides import TorchFunctionMode
+
+    layer = _layer(8, 4)
+    x, pos = torch.randn(130, 1024, device="cuda").bfloat16(), torch.arange(65, device="cuda")
+    want, seen, stock = layer.attn_partial(x, 2, 65, pos), [], F.scaled_dot_product_attention
+
+    class Mode(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            if func is stock:
+                seen.append("mode")
+            return func(*args, **(kwargs or {}))
+
+    with Mode():
+        assert torch.equal(layer.attn_partial(x, 2, 65, pos), want)
+    monkeypatch.setattr(F, "scaled_dot_product_attention", lambda *a, **k: seen.append("replaced") or stock(*a, **k))
+    assert torch.equal(layer.attn_partial(x, 2, 65, pos), want)
+    assert seen == ["mode", "replaced"]

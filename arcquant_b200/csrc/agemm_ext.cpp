@@ -43,8 +43,15 @@ void require_scalar_f32(const torch::Tensor& t, const torch::Tensor& like, const
   TORCH_CHECK(t.numel() == 1, name, " must hold one fp32 value");
 }
 // An output on `like`'s device.  Straight from the CUDA allocator's factory: through torch::empty's dispatch an allocation costs the
-// host about as much as a third of a launch, and a call makes two to five.
+// host about as much as a third of a launch, and a call makes two to five.  Through the dispatch all the same where somebody wants to see the
+// allocation - a dispatch mode, a tracer, a functorch transform: their keys are in the thread's set - or torch is asked to fill it.
+bool dispatch_allocations() {
+  const auto& context = at::globalContext();
+  return !(c10::impl::tls_local_dispatch_key_set().included_ - c10::default_included_set - c10::autocast_dispatch_keyset).empty() ||
+         (context.deterministicAlgorithms() && context.deterministicFillUninitializedMemory());
+}
 torch::Tensor empty_on(const torch::Tensor& like, at::IntArrayRef sizes, at::ScalarType type) {
+  if (dispatch_allocations()) return torch::empty(sizes, at::TensorOptions(type).device(like.device()));
   return torch::Tensor(at::detail::empty_cuda(sizes, type, like.device(), c10::nullopt));
 }
 // Shapes of a block-scaled GEMM's operands; returns M, N, K_eff.

@@ -16,12 +16,32 @@
 
 namespace {
 
-void check_status(int status, const char* where) {
+// A status of the C side; in Python arcquant_b200._lib.ArcqError, as without the extension (a RuntimeError where this module is
+// used without the package).
+struct StatusError : std::runtime_error {
+  StatusError(int status, const std::string& where, const std::string& text) : std::runtime_error(text), status(status), where(where) {}
+  int status;
+  std::string where;
+};
+void check_status(int status, const char* name) {
   if (status == ARCQ_OK) return;
+  const std::string where = std::string("Value error in ") + name;
   std::ostringstream os;
-  os << "Value error in " << where << ": " << arcq_status_string(status);
+  os << where << ": " << arcq_status_string(status);
   if (status == ARCQ_ERR_CUDA) os << " (cudaError " << arcq_last_cuda_error() << ")";
-  throw std::runtime_error(os.str());
+  throw StatusError(status, where, os.str());
+}
+void translate_status(std::exception_ptr e) {
+  try {
+    if (e) std::rethrow_exception(e);
+  } catch (const StatusError& error) {
+    try {
+      const py::object type = py::module_::import("arcquant_b200._lib").attr("ArcqError");
+      PyErr_SetObject(type.ptr(), type(error.status, error.where).ptr());
+    } catch (py::error_already_set&) {
+      PyErr_SetString(PyExc_RuntimeError, error.what());
+    }
+  }
 }
 
 void* current_stream(const torch::Tensor& t) {
@@ -544,6 +564,7 @@ torch::Tensor moe_combine(const torch::Tensor& Y, const torch::Tensor& pos, cons
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+  py::register_local_exception_translator(&translate_status);
   m.def("matmul", &matmul, "our ARC gemm (sm_100a)", py::arg("A"), py::arg("B"), py::arg("SFA"), py::arg("SFB"),
         py::arg("scale"));
   m.def("reorder_quantize_x", &reorder_quantize_x, "Reorder and quantize activation.", py::arg("X"),

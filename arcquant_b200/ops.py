@@ -442,16 +442,20 @@ def reorder_quantize_x_grouped(x: torch.Tensor, row_map, scales: torch.Tensor, r
 def quantize_grouped_amax(x: torch.Tensor, row_map, amax: torch.Tensor, reorder_indices: torch.Tensor, groups: torch.Tensor,
                           rows_bound: int, ke: int, mode: int = 16, clear: torch.Tensor | None = None):
     """(codes, scales, scale fp32 [runs]): `reorder_quantize_x_grouped` over scale = amax / (448 * 6) of every run, taken
-    inside the quantizer.  clear: up to 64 fp32 values set to zero by the way (see `matmul_grouped_swiglu`)."""
+    inside the quantizer.  clear: up to 64 fp32 values, neither read nor written otherwise by the call, set to zero by the way (see
+    `matmul_grouped_swiglu`)."""
     ngroups, kq = reorder_indices.shape
-    ext = _ext()
-    if clear is not None and not ext:
-        clear.zero_()
+    if clear is not None:
+        _require(clear, torch.float32, "clear")
+        if clear.numel() > 64:
+            raise RuntimeError("clear: at most 64 values")
     if ngroups > 64 or kq > 16384 or rows_bound == 0 or amax.numel() != ngroups:
+        scale = amax / (448.0 * 6.0)
+        out = (*reorder_quantize_x_grouped(x, row_map, scale, reorder_indices, groups, rows_bound, ke, mode), scale)
         if clear is not None:
             clear.zero_()
-        scale = amax / (448.0 * 6.0)
-        return (*reorder_quantize_x_grouped(x, row_map, scale, reorder_indices, groups, rows_bound, ke, mode), scale)
+        return out
+    ext = _ext()
     if ext:
         return ext.quantize_grouped_amax(x, row_map, amax, reorder_indices, groups, rows_bound, ke, mode, clear)
     lib = _lib.load()
@@ -472,9 +476,11 @@ def quantize_grouped_amax(x: torch.Tensor, row_map, amax: torch.Tensor, reorder_
     sf = torch.empty((sf_bytes(rows_bound, k_eff),), dtype=torch.uint8, device=x.device)
     scale = torch.empty((ngroups,), dtype=torch.float32, device=x.device)
     with torch.cuda.device(x.device):
-        rc = lib.arcq_quantize_x_grouped_amax(x.data_ptr(), None if row_map is None else row_map.data_ptr(), amax.data_ptr(),
-                                              reorder_indices.data_ptr(), groups.data_ptr(), ngroups, rows_bound, kq, ke, mode,
-                                              q.data_ptr(), sf.data_ptr(), scale.data_ptr(), _stream())
+        rc = lib.arcq_quantize_x_grouped_amax_clear(x.data_ptr(), None if row_map is None else row_map.data_ptr(), amax.data_ptr(),
+                                                    reorder_indices.data_ptr(), groups.data_ptr(), ngroups, rows_bound, kq, ke, mode,
+                                                    q.data_ptr(), sf.data_ptr(), scale.data_ptr(),
+                                                    None if clear is None else clear.data_ptr(), 0 if clear is None else clear.numel(),
+                                                    _stream())
     _lib.check(rc, f"grouped x-quantize KQ={kq} KE={ke}")
     return q, sf, scale
 

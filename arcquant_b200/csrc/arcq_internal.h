@@ -103,7 +103,7 @@ int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight
                                  int KE, int mode, uint8_t* q, uint8_t* sf, float* scale_out, float* scratch,
                                  cudaStream_t stream, const int* groups = nullptr, int ngroups = 0,
                                  const int* row_map = nullptr, float* clear = nullptr, int nclear = 0);
-// n floats to zero, as a programmatic dependent (see ScaleOptions::clear).
+// n floats (at most 64) to zero, as a programmatic dependent.
 int launch_clear(float* p, int n, cudaStream_t stream);
 int launch_absmax(const void* x, int64_t n, float* out, int accumulate, cudaStream_t stream);
 int launch_gemm(const uint8_t* A, const uint8_t* B, const uint8_t* SFA, const uint8_t* SFB, int64_t M,

@@ -2,6 +2,8 @@
 import pytest
 import torch
 
+from tests.helpers import launched_kernels
+
 pytestmark = pytest.mark.gpu
 
 
@@ -37,9 +39,17 @@ def test_maximum_of_the_swiglu_epilogue_starts_from_zero(rows):
     assert rc == 0 and float(amax) == float(c.abs().max()) > 0
 
 
-@pytest.mark.parametrize("rows", [1, 63, 592, 593, 2000])      # row kernel and the kernels of many rows
+def _quantizer(call):
+    names = [k[0] for k in launched_kernels(call) if "arcq_quantize_" in k[0]]
+    assert len(names) == 1
+    return "rows" if "quantize_rows" in names[0] else "ws"
+
+
+# (which kernel the RMSNorm and the grouped rows take on 148 SMs: the row kernel clears itself, in front of the other a launch does)
+@pytest.mark.parametrize("rows, rms, grouped", [(1, "rows", "rows"), (63, "rows", "rows"), (592, "rows", "rows"), (593, "rows", "rows"),
+                                                (2000, "rows", "rows"), (3553, "ws", "rows"), (8000, "ws", "ws")])
 @pytest.mark.parametrize("clears", [1, 64])
-def test_quantizers_clear_for_the_launch_behind_them(rows, clears):
+def test_quantizers_clear_for_the_launch_behind_them(rows, rms, grouped, clears):
     from arcquant_b200 import _lib, ops
 
     k, lib = 1024, _lib.load()
@@ -48,12 +58,16 @@ def test_quantizers_clear_for_the_launch_behind_them(rows, clears):
     store = torch.full((clears + 2,), 7.0, device="cuda")
     q, sf = ops.rmsnorm_quantize_x(x, gain, 1e-5, idx, 64)
     q2, sf2 = torch.empty_like(q), torch.empty_like(sf)
+    assert _quantizer(lambda: ops.rmsnorm_quantize_x(x, gain, 1e-5, idx, 64, clear=store[1:1 + clears])) == rms
+    store.fill_(7.0)
     assert lib.arcq_rmsnorm_quantize_x_clear(x.data_ptr(), gain.data_ptr(), 1e-5, idx.data_ptr(), rows, k, 64, q2.data_ptr(), sf2.data_ptr(),
                                              store[1:].data_ptr(), clears, ops._stream()) == 0
     assert torch.equal(q, q2) and store.tolist() == [7.0] + [0.0] * clears + [7.0]
     groups = torch.tensor([0, 256, 0, rows], dtype=torch.int32, device="cuda")          # (the first run is empty)
     src, amax, orders = torch.zeros(256 + (rows + 255) // 256 * 256 + 256, k, device="cuda").bfloat16(), torch.ones(2, device="cuda"), idx.repeat(2, 1)
     src[256:256 + rows] = x
+    store.fill_(7.0)
+    assert _quantizer(lambda: ops.quantize_grouped_amax(src, None, amax, orders, groups, src.shape[0], 64, clear=store[1:1 + clears])) == grouped
     store.fill_(7.0)
     want = ops.quantize_grouped_amax(src, None, amax, orders, groups, src.shape[0], 64)
     got = ops.quantize_grouped_amax(src, None, amax, orders, groups, src.shape[0], 64, clear=store[1:1 + clears])

@@ -11,9 +11,10 @@ pytestmark = pytest.mark.gpu
 
 
 # narrow rows, one group in the last warp, both sides of 512 groups, odd row counts, and both sides of the row count
-# up to which the row kernel runs (444 pairs of rows at 4096 channels, 148 at 14336 on 148 SMs)
+# up to which the row kernel runs (444 pairs of rows at 4096 channels, 592 at 14336 on 148 SMs)
 @pytest.mark.parametrize("rows,kq,ke", [(1, 16, 16), (3, 64, 0), (5, 528, 16), (33, 1040, 64), (1, 4096, 128), (887, 4096, 128),
                                         (889, 4096, 128), (2, 8192, 256), (3, 8208, 16), (295, 14336, 128), (298, 14336, 64),
+                                        (1183, 14336, 128), (1186, 14336, 64),
                                         (7, 16384, 128), (300, 128, 32)])
 @pytest.mark.parametrize("weight", [False, True])
 def test_tensor_scale_inside_the_quantizer(rows, kq, ke, weight):

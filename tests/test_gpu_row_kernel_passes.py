@@ -6,7 +6,7 @@ import torch
 
 from arcquant_b200 import synth
 from oracle import oracle as O
-from tests.helpers import sf_take_rows
+from tests.helpers import launched_kernels, sf_take_rows
 
 pytestmark = pytest.mark.gpu
 
@@ -17,7 +17,8 @@ def _sample(rows):
 
 @pytest.mark.parametrize("rows, k, form", [(888, 4096, "rms"), (889, 4096, "rms"), (1777, 2048, "rms"), (3553, 1024, "rms"), (593, 8192, "rms"),
                                            (591, 5120, "rms"), (1775, 2048, "div"), (1777, 2048, "div"), (592, 7168, "plain"), (594, 5120, "weight"),
-                                           (1184, 14336, "plain"), (1185, 14336, "div"), (700, 16384, "plain"), (333, 11008, "weight"),
+                                           (1184, 14336, "plain"), (1185, 14336, "plain"), (592, 14336, "div"), (1185, 14336, "div"),
+                                           (700, 16384, "plain"), (333, 11008, "weight"),
                                            # (a few wide rows: their groups shared by up to eight CTAs)
                                            (1, 14336, "div"), (16, 8208, "plain"), (36, 11008, "weight"), (37, 16384, "plain"), (74, 14336, "div"),
                                            (75, 14336, "plain"), (148, 9216, "div"), (149, 14336, "plain")])
@@ -49,8 +50,12 @@ def test_passes_of_the_row_kernel(rows, k, form):
     assert np.array_equal(sf_take_rows(sf, at, k + ke), sf_take_rows(sf_w, range(len(at)), k + ke))
 
 
-@pytest.mark.parametrize("counts, k", [((700, 0, 1075), 4096), ((1, 1183, 0, 1), 14336), ((257, 2, 300, 33), 8192), ((0, 0, 1776), 4096)])
-def test_passes_over_grouped_rows(counts, k):
+# (the host knows the rows rounded up to 256: 1776 at 4096 channels and 592 of wider rows are the line)
+@pytest.mark.parametrize("counts, k, kernel", [((700, 0, 1075), 4096, "ws"), ((1, 1183, 0, 1), 14336, "ws"), ((257, 2, 300, 33), 8192, "ws"),
+                                               ((0, 0, 1776), 4096, "ws"), ((701, 0, 833), 4096, "rows"), ((0, 1535, 0, 1), 4096, "rows"),
+                                               ((3,) * 60 + (1001, 0, 0, 353), 4096, "rows"), ((1, 509, 0, 1), 14336, "rows"),
+                                               ((255, 0, 257), 14336, "rows"), ((257, 2, 220, 33), 8192, "rows"), ((5, 0, 3323), 2048, "rows")])
+def test_passes_over_grouped_rows(counts, k, kernel):
     from arcquant_b200 import ops
 
     ke, e = 64, len(counts)
@@ -69,8 +74,11 @@ def test_passes_over_grouped_rows(counts, k):
     idx = torch.stack([torch.randperm(k, generator=torch.Generator().manual_seed(i)) for i in range(e)]).to(torch.int16).cuda()
     groups = torch.tensor(first + list(counts), dtype=torch.int32, device="cuda")
     amax = ops.absmax_grouped(x, row_map.cuda(), groups, e)
-    q, sf, scale = ops.quantize_grouped_amax(x, row_map.cuda(), amax, idx, groups, bound, ke)
+    rm = row_map.cuda()
+    q, sf, scale = ops.quantize_grouped_amax(x, rm, amax, idx, groups, bound, ke)
     torch.cuda.synchronize()
+    names = [n[0] for n in launched_kernels(lambda: ops.quantize_grouped_amax(x, rm, amax, idx, groups, bound, ke))]
+    assert ["arcq_quantize_rows" in n for n in names] == [kernel == "rows"]
     assert ops.gemm_poll_error() == 0
     for i, (f, c) in enumerate(zip(first, counts)):
         if c == 0:

@@ -3,6 +3,8 @@ activations and weights, and values that a maximum has to get right."""
 import pytest
 import torch
 
+from tests.helpers import launched_kernels
+
 pytestmark = pytest.mark.gpu
 
 
@@ -28,13 +30,30 @@ def _check(x, weight, k):
 
 
 @pytest.mark.parametrize("weight", [False, True])
-@pytest.mark.parametrize("rows, k", [(1, 16), (3, 64), (1, 512), (15, 4096), (16, 4096), (17, 4096), (64, 1024), (65, 1024), (7, 8208), (1, 14336), (8, 14336),
-                                     (9, 14336), (1, 16384), (255, 64), (256, 64), (257, 64)])
-def test_around_the_line(rows, k, weight):
+@pytest.mark.parametrize("rows, k", [(1, 16), (3, 64), (1, 512), (15, 4096), (64, 1024), (65, 1024), (7, 8208), (1, 14336), (1, 16384), (255, 64), (256, 64),
+                                     (257, 64)])
+def test_small_tensors(rows, k, weight):
+    _around(rows, k, weight)
+
+
+# (up to 32 loads of eight channels per thread of a CTA)
+@pytest.mark.parametrize("weight", [False, True])
+@pytest.mark.parametrize("line, k", [(128, 64), (16, 512), (16, 1024), (16, 4096), (16, 5120), (16, 8192), (8, 8208), (8, 14336), (8, 16384)])
+def test_around_the_line(line, k, weight):
+    from arcquant_b200 import ops
+
+    idx = torch.arange(k, dtype=torch.int16, device="cuda")
+    for rows in (line - 1, line, line + 1):
+        x = _around(rows, k, weight)
+        assert len(launched_kernels(lambda: ops.quantize_tensor_scale(x, idx, 0, 16, weight))) == (1 if rows <= line else 2)
+
+
+def _around(rows, k, weight):
     x = torch.randn(rows, k, generator=torch.Generator().manual_seed(rows)).to(torch.bfloat16).cuda()
     x[rows - 1, k - 1] = -77.0            # the largest magnitude, the smallest value
     x[rows // 2, k // 2] = 33.0
     _check(x, weight, k)
+    return x
 
 
 @pytest.mark.parametrize("weight", [False, True])

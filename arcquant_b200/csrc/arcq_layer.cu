@@ -932,10 +932,11 @@ int launch_absmax_grouped(const void* x, const int* row_map, const int* groups, 
   int rc = get_device_info(&di);
   if (rc == ARCQ_OK) rc = launch_clear(out, ngroups, stream);
   if (rc != ARCQ_OK) return rc;
-  // (Eight CTAs per SM, whatever the rows: not early.  Layout, maxima and quantizer of a MoE block, us, early / not: 37 x 4096 11.3 / 11.3, 500 x
-  // 4096 15.4 / 15.7, 2222 x 4096 33.4 / 32.7, 2222 x 14 336 93 / 78, 8192 x 14 336 254 / 245.)
-  return launch_elementwise(arcq_absmax_grouped_kernel, (unsigned)di.num_sms * 8, 256, di, stream, static_cast<const uint16_t*>(x),
-                            row_map, groups, ngroups, K, reinterpret_cast<unsigned int*>(out));
+  // Eight CTAs per SM, whatever the rows: early only where a warp's row is short.  Layout, maxima and quantizer of a MoE block in turn, us, early /
+  // not: 37 x 1024 9.8 / 10.1, 37 x 4096 11.3 / 11.6, 4096 x 4096 50.2 / 50.4, 8192 x 4096 96.0 / 95.3, 8192 x 5120 108.4 / 107.3, 1000 x 8192 27.6 / 24.9,
+  // 2222 x 14 336 91 / 76 (37 x 8192 13.3 / 13.5); in an eager MoE block of 37 x 4096 it saves 1.6 of 181.
+  return launch_kernel(arcq_absmax_grouped_kernel, (unsigned)di.num_sms * 8, 256, 0, di.early_start() && K <= 4096, stream,
+                       static_cast<const uint16_t*>(x), row_map, groups, ngroups, K, reinterpret_cast<unsigned int*>(out));
 }
 
 int launch_moe_combine(const void* y, const int* pos, const void* w, void* out, int64_t tokens, int hidden, int k,

@@ -152,12 +152,19 @@ class PackedLinear(torch.nn.Module):
         return ops.matmul_dev_alpha(qx, self.W, sfx, self.SFW, scale_x, self.scale)
 
 
-_GEMM, _SDPA, _NEEDED = PackedLinear.gemm, torch._C._nn.scaled_dot_product_attention, {"W", "SFW", "scale", "index"}
+_GEMM, _SDPA, _function_mode = PackedLinear.gemm, torch._C._nn.scaled_dot_product_attention, torch._C._is_torch_function_mode_enabled
 
 
-def _as_built(lin) -> bool:
-    """Whether a linear is a `PackedLinear` as its class makes it, and its buffers and nothing else are what it computes with."""
-    return type(lin) is PackedLinear and getattr(lin.gemm, "__func__", None) is _GEMM and lin._buffers.keys() >= _NEEDED
+def _as_built(lin):
+    """(channel order, KE, packed weight, its scales, global scale) of a `PackedLinear` that is as its class makes it, and computes
+    with its buffers and nothing else; None for any other."""
+    if type(lin) is not PackedLinear or PackedLinear.gemm is not _GEMM or "gemm" in lin.__dict__:
+        return None
+    get = lin._buffers.get
+    index, W, SFW, scale = get("index"), get("W"), get("SFW"), get("scale")
+    if index is None or W is None or SFW is None or scale is None:
+        return None
+    return index, lin.select_num, W, SFW, scale
 
 
 class PhaseTimer:
@@ -263,27 +270,27 @@ class QLlamaDecoderLayerTP(torch.nn.Module):
             return ops.matmul_swiglu(a, self.gate_up.W, sfa, self.gate_up.SFW, self.gate_up.scale, None, onto)
         return ops.silu_mul(self.gate_up.gemm(a, sfa))
 
-    def _native(self, x2d: torch.Tensor, k_row: int, *linears) -> bool:
-        """Whether a half of the layer may run as one call into the extension: not while phases are timed, not for what the
-        quantizer of the row-parallel input leaves to torch (no rows, or rows of more than 16384 channels), and not where a caller has
-        put something of their own in a place that the call would pass by: a linear of another class, with another `gemm` or with
-        parameters for buffers, or a torch function mode."""
-        return (self.timer is None and x2d.shape[0] > 0 and k_row <= 16384 and ops.native()
-                and not torch._C._is_torch_function_mode_enabled() and all(_as_built(lin) for lin in linears))
+    def _native(self, x2d: torch.Tensor, k_row: int, first: str, second: str):
+        """The parts of the two linears of a half of the layer (`_as_built`) if the half may run as one call into the extension, else
+        None: not while phases are timed, not for what the quantizer of the row-parallel input leaves to torch (no rows, or rows of more
+        than 16384 channels), and not where a caller has put something of their own in a place that the call would pass by: a linear of
+        another class, with another `gemm` or with parameters for buffers, or a torch function mode."""
+        if self.timer is not None or x2d.shape[0] == 0 or k_row > 16384 or _function_mode() or not ops.native():
+            return None
+        linears = self._modules
+        a, b = _as_built(linears.get(first)), _as_built(linears.get(second))
+        return None if a is None or b is None else (a, b)
 
     # ---- halves of the layer up to (and excluding) the all-reduce: usable for in-process emulation
     @torch.no_grad()
     def attn_partial(self, x2d: torch.Tensor, bsz: int, seq: int, positions: torch.Tensor,
                      residual: torch.Tensor | None = None) -> torch.Tensor:
         cfg, D = self.cfg, self.cfg.head_dim
-        if F.scaled_dot_product_attention is _SDPA and self._native(x2d, self.h_local * D, self.qkv, self.o):
-            # what follows, in one native call
-            qkv, o = self.qkv, self.o
-            qb, ob = qkv._buffers, o._buffers
+        native = self._native(x2d, self.h_local * D, "qkv", "o") if F.scaled_dot_product_attention is _SDPA else None
+        if native is not None:      # what follows, in one native call
+            qkv, o = native
             cos, sin = rope_tables(positions, D, cfg.rope_theta)
-            return ops.attention_half(x2d, self.ln1, cfg.eps, qb["index"], qkv.select_num, qb["W"], qb["SFW"], qb["scale"], cos, sin,
-                                      self.h_local, self.kv_local, D, bsz, seq, ob["index"], o.select_num, ob["W"], ob["SFW"],
-                                      ob["scale"], residual)
+            return ops.attention_half(x2d, self.ln1, cfg.eps, *qkv, cos, sin, self.h_local, self.kv_local, D, bsz, seq, *o, residual)
         with self._ph("quantize"):
             a, sfa = ops.rmsnorm_quantize_x(x2d, self.ln1, cfg.eps, self.qkv.index, self.qkv.select_num)
         with self._ph("gemm"):
@@ -308,12 +315,11 @@ class QLlamaDecoderLayerTP(torch.nn.Module):
     @torch.no_grad()
     def mlp_partial(self, h2d: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
         cfg = self.cfg
-        if (self.fuse_swiglu and getattr(self._gate_up_act, "__func__", None) is QLlamaDecoderLayerTP._gate_up_act
-                and self._native(h2d, self.f_local, self.gate_up, self.down)):      # what follows, in one native call
-            gu, down = self.gate_up, self.down
-            gb, db = gu._buffers, down._buffers
-            return ops.mlp_half(h2d, self.ln2, cfg.eps, gb["index"], gu.select_num, gb["W"], gb["SFW"], gb["scale"], db["index"],
-                                down.select_num, db["W"], db["SFW"], db["scale"], residual)
+        stock = self.fuse_swiglu and type(self)._gate_up_act is QLlamaDecoderLayerTP._gate_up_act and "_gate_up_act" not in self.__dict__
+        native = self._native(h2d, self.f_local, "gate_up", "down") if stock else None
+        if native is not None:      # what follows, in one native call
+            gate_up, down = native
+            return ops.mlp_half(h2d, self.ln2, cfg.eps, *gate_up, *down, residual)
         amax = torch.empty((), dtype=torch.float32, device=h2d.device) if self.fuse_swiglu else None
         with self._ph("quantize"):
             a, sfa = ops.rmsnorm_quantize_x(h2d, self.ln2, cfg.eps, self.gate_up.index, self.gate_up.select_num, clear=amax)

@@ -41,8 +41,8 @@ struct ScaleOptions {
   int npartials = 0;
   // nclear floats (at most 64) that the quantizer sets to zero by the way, for the launch behind it to collect maxima in.  A memset between
   // the two ends the chain of programmatic dependents: the GEMM is set up, and its first weight tiles asked for, only when it is done
-  // (SwiGLU [28672, 4224] by weight streaming, call after call, us, with a memset / without: 1 row 18.6 / 14.5, 16 rows 19.9 / 15.2, 64 rows
-  // 22.0 / 17.9).
+  // (SwiGLU [28672, 4224] by weight streaming, call after call, us, behind a memset / behind a kernel that clears: 1 row 18.6 / 14.5, 16 rows
+  // 19.9 / 15.2, 64 rows 22.0 / 17.9).
   float* clear = nullptr;
   int nclear = 0;
 };

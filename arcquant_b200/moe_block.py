@@ -416,7 +416,7 @@ class QMixtralMoEBlockEP(torch.nn.Module):
 
     @torch.no_grad()
     def expert_forward_grouped(self, batch: RoutedBatch) -> torch.Tensor:
-        """All local experts in five launches: [rows_bound, hidden] in the padded layout of `batch`."""
+        """All local experts in a handful of launches, whatever their number: [rows_bound, hidden] in the padded layout of `batch`."""
         cfg, E = self.cfg, self.dispatcher.e_local
         ke = cfg.select_num
         amax1 = ops.absmax_grouped(batch.src, batch.row_map, batch.groups, E)

@@ -142,7 +142,7 @@ def reorder_quantize_w(w, reorder_index, ke: int, mode=None):
 
 def quantize_tensor_scale(x, reorder_index, ke: int, mode=None, is_weight: bool = False, amax=None):
     """(codes, scales, scale) of x over its own per-tensor scale max / (448 * 6) - |x| for activations, the signed
-    maximum for weights - in two launches (one if `amax`, max|x| on the device, is given: the scale then has its
+    maximum for weights - in two launches (one for a small tensor, or if `amax`, max|x| on the device, is given: the scale then has its
     shape), or None where that path does not apply: an empty or non-contiguous tensor, a weight off a 16-byte boundary,
     another type, no channel order, KQ > 16384."""
     if (reorder_index is None or not x.is_cuda or x.dtype != torch.bfloat16 or x.dim() != 2 or not x.is_contiguous()

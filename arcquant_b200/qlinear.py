@@ -17,7 +17,7 @@ FP8_MAX = 448.0
 def NVFP4_reorder_quantize_x(x: torch.Tensor, reorder_index: torch.Tensor, select_num: int, mode=None, amax=None):
     """(qx, scale_x, scale): per-tensor scale = max|x| / (448*6) as a 0-dim fp32 CUDA tensor,
     ``x / scale`` in bf16 as the reference forms it, then the fused reorder + NVFP4 + ARC kernel.
-    One pass for partial maxima, the rest of the scale and the division inside the quantizer
+    One pass for partial maxima (none for a small tensor), the rest of the scale and the division inside the quantizer
     (``arcq_quantize_tensor_scale``); a caller that already has max|x| on the device (``ops.silu_mul``)
     passes it as ``amax``."""
     fused = ops.quantize_tensor_scale(x, reorder_index, select_num, mode, False, amax)

@@ -100,7 +100,7 @@ int arcq_reorder_quantize_x(const void* x, const int16_t* reorder_index, int64_t
  * max / (448 * 6) (`scale = max|x| / (448.0 * 6.0)` in NVFP4_reorder_quantize_x, model/qLlamaLayer.py:73-77; the SIGNED
  * maximum of a weight, model/qLinearLayer.py:25-28), then arcq_reorder_quantize_x_scaled - or its weight flavour - by it.
  * amax: max|x| in device memory if the caller has it already, or NULL: a first pass leaves partial maxima in
- * `scratch` (ARCQ_SCALE_SCRATCH floats of device memory).  scale_out (device) receives the scale: the fp32 product of
+ * `scratch` (ARCQ_SCALE_SCRATCH floats of device memory), or - a small tensor - the quantizer takes the maximum itself, in one launch.  scale_out (device) receives the scale: the fp32 product of
  * the maximum with the fp32 reciprocal of 2688, as torch's division of a tensor by a host scalar computes it.
  * ARCQ_ERR_UNSUPPORTED_K for KQ > 16384. */
 #define ARCQ_SCALE_SCRATCH 512

@@ -169,7 +169,5 @@ int launch_gemm_skinny(const uint8_t* X, const uint8_t* W, const uint8_t* SFX, c
 int skinny_plan_splits(int64_t M, int64_t N, int64_t K_eff);
 int skinny_poll_error();
 int gemm_poll_error();
-// Same for the bounded waits of the warp-specialised quantizer.
-int quant_poll_error();
 
 }  // namespace arcq

@@ -29,6 +29,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "arcq_internal.h"
 
@@ -59,9 +60,8 @@ struct QuantParams {
   int ngroups;
   const int* row_map;
 };
-// (ScaleOptions travels behind it as a kernel parameter of its own.  As three more members of this struct it made ptxas
-// spill in the warp-specialised kernel, whose 64 registers are all in use: fused RMSNorm of 32 768 x 4096 94.4 -> 94.9 us,
-// 16 384 x 8192 divided by their scale 75.4 -> 80.5.)
+// (ScaleOptions travels behind it as a kernel parameter of its own: three more members of this struct once made ptxas spill in a kernel whose
+// registers were all in use.)
 
 __device__ __forceinline__ float bf16lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float bf16hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
@@ -548,73 +548,25 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_kernel(const QuantPa
 }
 
 // ------------------------------------------------------------------------------------------------
-// Warp-specialised variant (rows of 1024..8192 channels, the hidden sizes of decoder layers).
-//
-// Producer warps stream row pairs from global memory, (RMSNorm them,) interleave them and fill a ring
-// of shared stages; consumer warps gather their groups from a full stage, release it as soon as the
-// gather has landed in registers, and quantize.  Stages are handed over with mbarriers, so there is
-// no CTA-wide barrier in the loop and the warp that carries the critical (residual) groups - a
-// different warp for every row pair - does not hold the others back.  Producers keep the next pair in
-// flight in registers while they fill the current one.
+// Pieces of the two kernels below.
 //
 // Block scales are computed without tables or branches: amax/6 by a multiply and one FMA correction
 // (exact for every bf16 amax), the ue4m3 code of both rows by one packed conversion, and 1/scale by
 // the approximate reciprocal plus one Newton step (exact here: a scale is k*2^e with k <= 15, so its
 // reciprocal lies far from every fp32 rounding boundary).
-
-__device__ int g_quant_error = 0;   // sticky until polled
-constexpr unsigned long long QUANT_WAIT_LIMIT_NS = 2000000000ull;
-
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+__device__ __forceinline__ uint32_t lds32(uint32_t a) {
+  uint32_t v;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
 }
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+__device__ __forceinline__ uint4 lds128(uint32_t a) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+  return v;
 }
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n.reg .pred p;\n"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-// Bounded wait: false if this wait (or another warp's) gave up; the CTA then winds down.  The clock is
-// first read after 64 failed polls, so a wait of ordinary length never touches it.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  if (mbar_try_wait(bar, parity)) return true;
-  unsigned long long t0 = 0;
-  for (uint32_t it = 1;; ++it) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 63u) == 0) {
-      if (*abort_flag) return false;
-      unsigned long long t1;
-      asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
-      if (t0 == 0) t0 = t1;
-      if (t1 - t0 > QUANT_WAIT_LIMIT_NS) {
-        *abort_flag = 1;
-        atomicExch(&g_quant_error, ARCQ_ERR_TIMEOUT);
-        return false;
-      }
-    }
-  }
-}
-// Named barrier over `nthreads` threads that also ORs a flag across them.
-__device__ __forceinline__ bool named_barrier_or(int id, int nthreads, bool flag) {
-  uint32_t out;
-  asm volatile(
-      "{\n.reg .pred p, q;\n"
-      "setp.ne.u32 q, %3, 0;\n"
-      "bar.red.or.pred p, %1, %2, q;\n"
-      "selp.u32 %0, 1, 0, p;\n}"
-      : "=r"(out)
-      : "r"(id), "r"(nthreads), "r"((uint32_t)flag)
-      : "memory");
-  return out != 0;
+__device__ __forceinline__ void sts128(uint32_t a, const uint4& v) {
+  asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
 __device__ __forceinline__ uint32_t min_u16x2(uint32_t a, uint32_t b) {
@@ -647,61 +599,6 @@ __device__ __forceinline__ void scale_of_pair_fma(uint32_t m, uint32_t& codes, f
   const float2 e = __ffma2_rn(make_float2(-dec.x, -dec.y), r0, make_float2(1.0f, 1.0f));
   rcp = __ffma2_rn(r0, e, r0);
   codes = c2;
-}
-
-// As quantize_group_pair, with the branch-free scales; q1 / sf1 are row 1's outputs (equal to row 0's
-// for the odd last row: row 1 is stored first and row 0 overwrites it).  In every layout the codes of
-// scale column c start at byte 8 c of the row, and a critical group's residual sits 1 (mode 16) or 2
-// (mode 32) columns after its main part.
-__device__ __forceinline__ void quantize_group_pair_ws(uint32_t (&w)[16], int g, int G0, bool mode32, bool is_weight,
-                                                       uint8_t* q0, uint8_t* q1, uint8_t* sf0, uint8_t* sf1) {
-  const uint32_t m = amax_pair_h(w);
-  uint32_t codes;
-  float2 dec, rcp;
-  scale_of_pair_fma(m, codes, dec, rcp);
-  uint2 c0, c1;
-  encode_pair(w, rcp.x, rcp.y, c0, c1);
-  const int j = g - G0;
-  const bool critical = j >= 0;
-  uint32_t col = (uint32_t)g;
-  if (critical) col = mode32 ? (uint32_t)(G0 + ((j >> 1) << 2) + (j & 1)) : (uint32_t)(g + j);
-  const uint32_t cm = ((col >> 2) << 9) | (col & 3u);
-  *reinterpret_cast<uint2*>(q1 + 8u * col) = c1;
-  sf1[cm] = (uint8_t)(codes >> 8);
-  *reinterpret_cast<uint2*>(q0 + 8u * col) = c0;
-  sf0[cm] = (uint8_t)codes;
-  if (!critical) return;
-
-  uint2 e0 = c0, e1 = c1;
-  uint32_t rcodes = codes;
-  if (!is_weight) {
-    float d0 = dec.x, d1 = dec.y;
-    if (mode32) {   // against the un-rounded fp32 scale
-      d0 = make_scale_slow(__uint_as_float((m & 0xffffu) << 16)).raw;
-      d1 = make_scale_slow(__uint_as_float((m >> 16) << 16)).raw;
-    }
-    residual_pair(w, c0, c1, d0, d1);
-    const uint32_t rm = amax_pair_h(w);
-    float2 rdec, rrcp;
-    scale_of_pair_fma(rm, rcodes, rdec, rrcp);
-    encode_pair(w, rrcp.x, rrcp.y, e0, e1);
-  }
-  const uint32_t rcol = col + (mode32 ? 2u : 1u);
-  const uint32_t cr = ((rcol >> 2) << 9) | (rcol & 3u);
-  *reinterpret_cast<uint2*>(q1 + 8u * rcol) = e1;
-  sf1[cr] = (uint8_t)(rcodes >> 8);
-  *reinterpret_cast<uint2*>(q0 + 8u * rcol) = e0;
-  sf0[cr] = (uint8_t)rcodes;
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-// Bulk copy global -> shared (both 16-byte aligned, size a multiple of 16), completing on `bar`.
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
 }
 
 // The tensor's divisor from the partial maxima of arcq_max_partials_kernel (one whole warp).
@@ -752,529 +649,361 @@ __device__ __forceinline__ void div_pair_words(uint32_t wa, uint32_t wb, float s
   }
 }
 
-// How the plain operator's divisor comes about: none; *scale, as it is; or by ScaleOptions.  (One instance for the last two
-// made the plain division 1 - 2 % slower: 16 384 x 14 336 145.4 -> 147.1 us, 880 rows 12.4 -> 12.7.)
-enum { DIV_NONE = 0, DIV_GIVEN = 1, DIV_MAXIMA = 2 };
+// ------------------------------------------------------------------------------------------------
+// Kernel of many rows (of 512 to 16384 channels; RMSNorm 1024 to 8192): one CTA per SM, its 24 warps in sets of TW ("ws": warp sets).
+//
+// A set takes a pair of rows from global memory to its codes by itself and shares nothing with the others but the tables: the pair is
+// interleaved in the set's own buffer, gathered from there group by group, quantized and stored; two barriers of the set (none where a warp is a
+// set) stand between.  What bounds it: the pipe of shared memory and L1, 79 % of its cycles at 16 384 x 4096 (plain, no residual; of them
+// the gather, whose random words meet 3.6 to a bank, is half), issue slots 35 to 52 %.  So it is built to ask little of both:
+//  * rows come through registers, not through a ring in shared memory (a raw ring costs two more passes over the pair), in slots of four 128-bit
+//    loads of a lane: one on its way while the rows before are quantized, one ahead after that, all from L2, where a bulk prefetch puts the pair
+//    a pair ahead (without it 43.4 -> 49.9 us);
+//  * no roles: with producers and consumers one side waits for the other, and each wait is polled (40 % of the instructions of the
+//    warp-specialised kernel that this one replaced, with 4650 instructions a pair where this one has 3100; a scheduler that gave every warp
+//    tasks of both kinds in turn polled no less);
+//  * 24 warps of 80 registers rather than 12 of 168 (plain 16 384 x 4096 44 -> 37 us): latency is hidden by warps.  Not one value may spill: shared memory
+//    leaves next to no L1, and a spilled word comes back from L2 (100 bytes of spills: 37 -> 45 us);
+//  * addresses are a base and constants: every chunk of a row is 32 lanes wide, the last chunk of a ragged row reaches back over the one
+//    before (its lanes write the same values twice), the last slot likewise.
+// us, the warp-specialised kernel / this one (graphs of ten calls): fused RMSNorm 32 768 x 4096 94.3 / 78.9, 16 384 x 4096 50.9 / 42.6, 4096 x 4096 15.4 /
+// 13.8, 8192 x 2048 19.3 / 13.2, 8192 x 5120 40.4 / 28.6, 16 384 x 8192 88.8 / 81.2 (2048 x 8192 14.2 / 14.7: the only width that was not slower there);
+// plain 16 384 x 4096 42.2 / 36.8, 16 384 x 8192 72.3 / 72.1; over a tensor's maximum 16 384 x 4096 47.7 / 37.7, 8192 x 9216 62.4 / 46,
+// 16 384 x 14 336 142.4 / 128.0; eight runs of 8192 rows in all of 4096 channels 30.2 / 21.4, of 14 336 82.0 / 71.1.
+// Four rows at a time (64-bit gathers, a sixth less of the pipe) do not fit 80 registers: 47 us where pairs take 43; without spills, 16 warps of
+// 128 registers are too few.
+// The name of a launch is what tells it from one of the row kernel.
+// RMSNorm: lane l of a set's slot k is the reference's thread t = 32 (TW k + warp) + l with its chunks t and t + KQ/16; the sums of a warp's slots
+// are added in the lane, those of the warps meet in shared memory, the last 32 are added across the lanes: the reference's tree.
+constexpr int WS_WARPS = 24;
+// Shared memory in front of the sets' buffers: offsets, gains, and the sums that cross the warps of a set.
+__host__ __device__ __forceinline__ uint32_t ws_fixed_bytes(bool rms, int tw, int KQ, int nsets) {
+  return (uint32_t)KQ * (rms ? 4 : 2) + (rms && tw > 1 ? (uint32_t)nsets * 512u : 0u);
+}
 
-// S: stages of the gather ring (interleaved row pairs).  R: stages of the raw ring (row pairs as they
-// lie in global memory, filled by bulk copies - this is what keeps enough bytes in flight to cover
-// the HBM latency).  RMS: fused RMSNorm.  WIDE (plain only): rows of more than 8192 channels - the offset
-// table holds 16-bit entries so that table, two gather stages and one raw stage fit in shared memory.
-// Threads [0, nteams*nct) are consumers in teams of nct threads - team k takes the row pairs
-// k, k + nteams, ... of this CTA, so several pairs are being quantized at once.  After them come
-// npteams producer teams of npt = KQ/16 threads (more than one only with RMSNorm, whose producers carry
-// real arithmetic), sharing the pairs the same way; producer t of a team owns the 16-byte chunks t and
-// t + KQ/16 of each row, the reference's assignment and summation order for RMSNorm.
-// XR: the CTA is launched with 1024 threads at 64 registers each and re-divides them: every warp that is
-// not a consumer gives registers back (56 left; padding warps then leave), the consumer warps take 88.
-// Measured on the fused operator at 4096 channels: 0.0988 -> 0.0953 ms per 32 768 tokens.  Other splits were
-// slower: 48 / 104 (0.105 ms) and 40 / 128 (0.152 ms) starve the producers; helper warps cut to 32 or 48
-// registers in warpgroups of their own double the time (the reducers sit on the critical path); quantizing a
-// thread's two groups side by side instead of one after the other costs time with 88 and with 104 registers.
-// (The wide plain operator has 256 producers and 512 consumers: 80 registers each instead of 64 and a spill, 16 384 x 14 336
-// 135.1 -> 127.5 us, 880 x 14 336 11.6 -> 11.1.)
-template <bool RMS, bool WIDE, int DIV, int S, int R, bool XR = false>
-__global__ void __launch_bounds__(WIDE && DIV == DIV_NONE ? 768 : 1024, 1)
-arcq_quantize_ws_kernel(const QuantParams p, const int nct, const int npt, const int nteams, const int npteams, const ScaleOptions so) {
-  constexpr bool SCALED = DIV != DIV_NONE;
+// MG: groups per row at most.
+template <bool RMS, bool SCALED, int MG, int TW>
+__global__ void __launch_bounds__(WS_WARPS * 32, 1) arcq_quantize_ws_kernel_sets(const QuantParams p, const ScaleOptions so) {
   extern __shared__ __align__(16) uint8_t smem[];
-  const int tid = threadIdx.x;
-  const int KQ = p.KQ, G = p.G;
-  uint32_t rows = (uint32_t)p.rows, npairs = (uint32_t)p.npairs;
-  // This CTA is number `cta` of the `stride` CTAs that share a run of rows: the whole input, or - with
-  // grouped rows - run e = blockIdx.x % ngroups, whose rows start at output row `row_base`.
-  uint32_t cta = blockIdx.x, stride = gridDim.x, row_base = 0;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int set = warp / TW, sw = warp % TW, nsets = (int)(blockDim.x >> 5) / TW;
+  const int KQ = p.KQ, G = p.G, G0 = p.G0;
+  uint32_t rows = (uint32_t)p.rows, cta = blockIdx.x, stride = gridDim.x, row_base = 0;
   const int16_t* idx_g = p.idx;
   const float* scale_g = p.scale;
   if (p.groups != nullptr) {
-    // (the table may have been written by the previous kernel of the stream)
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const uint32_t ng = (uint32_t)p.ngroups, e = blockIdx.x % ng;
     cta = blockIdx.x / ng;
     stride = (gridDim.x - e + ng - 1) / ng;
     row_base = (uint32_t)p.groups[e];
     rows = (uint32_t)p.groups[ng + e];
-    npairs = (rows + 1) >> 1;
     if (idx_g) idx_g += (size_t)e * (size_t)KQ;
     if (scale_g) scale_g += e;
   }
-  if (cta >= npairs) {   // (whole CTA: nothing was set up yet)
-    if (DIV == DIV_MAXIMA && p.groups != nullptr && so.out != nullptr && blockIdx.x == 0)
+  const uint32_t npairs = (rows + 1) >> 1;
+  if (cta >= npairs) {
+    if (SCALED && p.groups != nullptr && so.out != nullptr && blockIdx.x == 0)
       for (int e = tid; e < p.ngroups; e += blockDim.x) so.out[e] = p.scale[e] * so.factor;
     return;
   }
-  const int* row_map = p.row_map;
-  // input row of output row r of this run
-  auto in_row = [&](uint32_t r) -> const uint16_t* {
-    const uint32_t gr = row_base + r;
-    return p.x + (size_t)(row_map ? (uint32_t)row_map[gr] : gr) * (size_t)KQ;
-  };
+  // shared layout: [offsets][gains (RMS)][sums that cross the warps of a set (RMS)][a buffer per set]
+  uint16_t* offs = reinterpret_cast<uint16_t*>(smem);
+  uint16_t* gains = offs + KQ;
+  const uint32_t exch = smem_addr(smem) + (uint32_t)KQ * 4 + (uint32_t)set * 512u + 4u * lane;
+  const uint32_t buf = smem_addr(smem) + ws_fixed_bytes(RMS, TW, KQ, nsets) + (uint32_t)set * (uint32_t)KQ * 4;
 
-  // shared layout: [barriers, abort flag: 384 B][offsets][partial sums, rstd][gather ring][raw ring]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + 376);
-  size_t cursor = 384;
-  uint32_t* offs32 = reinterpret_cast<uint32_t*>(smem + cursor);
-  uint16_t* offs16 = reinterpret_cast<uint16_t*>(smem + cursor);
-  cursor += (size_t)KQ * (WIDE ? 2 : 4);
-  float* psum = nullptr;
-  float* rstd_s = nullptr;
-  if (RMS) {
-    psum = reinterpret_cast<float*>(smem + cursor);
-    cursor += (size_t)4 * npt * npteams * sizeof(float);   // per producer team: two buffers of two rows
-    rstd_s = reinterpret_cast<float*>(smem + cursor);
-    cursor += (size_t)16 * npteams;
-  }
-  uint8_t* stages = smem + cursor;
-  const uint32_t stage_bytes = (uint32_t)KQ * 4;
-  uint8_t* raw = stages + (size_t)S * stage_bytes;
-  const uint32_t row_in_bytes = (uint32_t)KQ * 2;
-  const uint32_t full0 = smem_addr(bars), empty0 = smem_addr(bars + S), raw0 = smem_addr(bars + 2 * S);
-  // RMSNorm only: raw stage handed back to the loader; per producer team, partial sums ready (x2
-  // buffers) and reciprocal roots ready (x2)
-  const uint32_t rawe0 = raw0 + 8 * R, psr0 = rawe0 + 8 * R, rsr0 = psr0 + 8 * 4;
-
-  asm volatile("griddepcontrol.launch_dependents;");   // the next kernel of the stream may be set up now
-  // Bulk copies of the rows of `unit` into raw stage `rs` (one thread).
-  auto issue = [&](uint32_t unit, uint32_t rs) {
-    if (unit >= npairs) return;
-    const uint32_t r0 = 2 * unit;
-    const bool has1 = (r0 + 1) < rows;
-    const uint32_t bar = raw0 + 8 * rs;
-    const uint32_t dst = smem_addr(raw + (size_t)rs * stage_bytes);
-    mbar_expect_tx(bar, has1 ? 2 * row_in_bytes : row_in_bytes);
-    bulk_load(dst, in_row(r0), row_in_bytes, bar);
-    if (has1) bulk_load(dst + row_in_bytes, in_row(r0 + 1), row_in_bytes, bar);
-  };
-  // WIDE: the raw ring holds half pairs (the same half of the channels of both rows), so that the
-  // copies of the next half overlap the work on this one although only ~1.5 pairs of raw rows fit.
-  // Half u of this CTA is half u & 1 of its pair u >> 1.
-  auto issue_half = [&](uint32_t u, uint32_t rs) {
-    const uint32_t unit = cta + (u >> 1) * stride;
-    if (unit >= npairs) return;
-    const uint32_t r0 = 2 * unit, hbytes = row_in_bytes >> 1;
-    const bool has1 = (r0 + 1) < rows;
-    const uint32_t bar = raw0 + 8 * rs;
-    const uint32_t dst = smem_addr(raw + (size_t)rs * row_in_bytes);
-    const size_t hoff = (size_t)(u & 1u) * (size_t)(KQ >> 1);
-    mbar_expect_tx(bar, has1 ? 2 * hbytes : hbytes);
-    bulk_load(dst, in_row(r0) + hoff, hbytes, bar);
-    if (has1) bulk_load(dst + hbytes, in_row(r0 + 1) + hoff, hbytes, bar);
-  };
-  // (one thread; with RMSNorm chosen by its number, there the other form costs 0.8 % of 32 768 x 4096)
-  if (RMS ? tid == 0 : (tid < 32 && elect_one())) {
-    for (int s = 0; s < S; ++s) {
-      mbar_init(full0 + 8 * s, (uint32_t)(npt >> 5));    // one arrival per producer warp
-      mbar_init(empty0 + 8 * s, (uint32_t)(nct >> 5));   // one arrival per warp of the consuming team
-    }
-    for (int r = 0; r < R; ++r) mbar_init(raw0 + 8 * r, 1);   // the thread that issues the copies
-    if (RMS) {
-      for (int r = 0; r < R; ++r) mbar_init(rawe0 + 8 * r, (uint32_t)(npt >> 5));   // one arrival per producer warp
-      for (int k = 0; k < 4; ++k) {
-        mbar_init(psr0 + 8 * k, (uint32_t)(npt >> 5));
-        mbar_init(rsr0 + 8 * k, 2);                                                 // the two reducer warps
-      }
-    }
-    abort_flag[0] = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the bulk copies see the barriers
-    // The first R row pairs start streaming in while the CTA builds its tables (global memory may
-    // still be written by the previous kernel of the stream until this wait returns).
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    for (uint32_t r = 0; r < (uint32_t)R; ++r) {
-      if (WIDE) issue_half(r, r);
-      else issue(cta + r * stride, r);
-    }
-  }
-  // Everything before this line touched shared memory only; global memory may still be written by
-  // the previous kernel of the stream (no-op unless launched as a programmatic dependent).
+  asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  // Offsets are laid out [vector v][group g][entries of one 128-bit load]: consecutive lanes (groups)
-  // read consecutive 16 bytes, so every table load is conflict free.
+  auto in_row = [&](uint32_t r) -> const uint4* {
+    const uint32_t gr = row_base + r;
+    return reinterpret_cast<const uint4*>(p.x + (size_t)(p.row_map ? (uint32_t)p.row_map[gr] : gr) * (size_t)KQ);
+  };
+  const int slots = (G + 32 * TW - 1 - 32 * sw) / (32 * TW), t0 = 32 * sw + lane;
+  uint4 first[4];
+  const uint4 *x0 = nullptr, *x1 = nullptr;                // (at this lane's first chunk)
+  auto rows_at = [&](uint32_t pr) {
+    x0 = in_row(2 * pr) + t0;
+    x1 = 2 * pr + 1 < rows ? in_row(2 * pr + 1) + t0 : x0;
+  };
+  auto load_slot = [&](int k, uint4 (&b)[4]) {
+    const int at = RMS ? 32 * TW * k : min(32 * TW * k, G - 32 - 32 * sw);      // (the last slot of a ragged row reaches back)
+    b[0] = ldg_stream(x0 + at); b[1] = ldg_stream(x0 + G + at);
+    b[2] = ldg_stream(x1 + at); b[3] = ldg_stream(x1 + G + at);
+  };
+  const uint32_t st0 = buf + (swz16(2u * t0) << 4), st1 = buf + (swz16(2u * (t0 + G)) << 4);    // (+ 1024 TW a slot)
+  uint32_t pair = cta + (uint32_t)set * stride;
+  const uint32_t step = (uint32_t)nsets * stride;
+  if (pair < npairs) {
+    rows_at(pair);
+    load_slot(0, first);
+  }
+  // RMSNorm: the gains come in their own order into a buffer that nothing lies in yet (of set 0), and from there into the order of the
+  // groups: gathered from global memory they came a round trip after the channel order.
+  const uint16_t* gains_in = reinterpret_cast<const uint16_t*>(smem + ws_fixed_bytes(RMS, TW, KQ, nsets));
+  if (RMS) {
+    for (int v = tid; v < (KQ >> 3); v += blockDim.x) sts128(smem_addr(gains_in) + 16u * v, __ldcg(reinterpret_cast<const uint4*>(p.gamma) + v));
+  }
   auto put = [&](int j, int c) {
-    const int g = j >> 4, i = j & 15;
-    if (WIDE) offs16[(((i >> 3) * G + g) << 3) | (i & 7)] = (uint16_t)word_offset((uint32_t)c);
-    else offs32[(((i >> 2) * G + g) << 2) | (i & 3)] = word_offset((uint32_t)c);
+    const int at = ((((j & 15) >> 3) * G + (j >> 4)) << 3) | (j & 7);
+    offs[at] = (uint16_t)word_offset((uint32_t)c);
+    if (RMS) gains[at] = (uint16_t)c;
   };
   if (idx_g && (reinterpret_cast<uintptr_t>(idx_g) & 15u) == 0) {
-    // eight indices per 128-bit load: one round trip to global memory for rows of up to 8192 channels
     const uint4* idx4 = reinterpret_cast<const uint4*>(idx_g);
     for (int v = tid; v < (KQ >> 3); v += blockDim.x) {
-      const uint4 w = __ldcg(idx4 + v);     // (a plain load: fused RMSNorm of 32 768 x 4096 94.4 -> 94.9 us)
+      const uint4 w = __ldcg(idx4 + v);
       const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        put(8 * v + 2 * k, (int)(int16_t)(ww[k] & 0xffffu));
-        put(8 * v + 2 * k + 1, (int)(int16_t)(ww[k] >> 16));
+        put(8 * v + 2 * k, (int)(ww[k] & 0xffffu));
+        put(8 * v + 2 * k + 1, (int)(ww[k] >> 16));
       }
     }
   } else {
     for (int j = tid; j < KQ; j += blockDim.x) put(j, idx_g ? (int)idx_g[j] : j);
   }
+  if (RMS) {
+    __syncthreads();
+    for (int j = 2 * tid; j < KQ; j += 2 * blockDim.x) {
+      uint32_t& two = *reinterpret_cast<uint32_t*>(gains + j);
+      two = (uint32_t)gains_in[two & 0xffffu] | ((uint32_t)gains_in[two >> 16] << 16);
+    }
+  }
+  float sc = 1.0f, rsc = 1.0f;
+  bool fast = true;
+  if (SCALED) {
+    // (worked out by one warp and passed on in a buffer that nothing lies in yet)
+    if (warp == 0) {
+      const float v = (so.npartials > 0 ? partials_max(p.scale, so.npartials, lane) : *scale_g) * so.factor;
+      if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(buf), "f"(v) : "memory");
+      if (so.out != nullptr && blockIdx.x == 0) {
+        if (so.npartials > 0) {
+          if (lane == 0) so.out[0] = v;
+        } else {
+          for (int e = lane; e < (p.groups != nullptr ? p.ngroups : 1); e += 32) so.out[e] = p.scale[e] * so.factor;
+        }
+      }
+    }
+  }
   __syncthreads();
+  if (SCALED) {
+    // torch's CUDA kernel for (bf16 tensor) / (fp32 scalar tensor) loads the divisor as bf16
+    sc = __uint_as_float(pack_bf16x2_rn(__uint_as_float(lds32(buf - (uint32_t)set * (uint32_t)KQ * 4)), 0.f) << 16);
+    rsc = __frcp_rn(sc);
+    fast = div_by_reciprocal_ok(sc);
+    __syncthreads();
+  }
 
-  const int ncons = nteams * nct;
-  if (tid >= ncons) {
-    if (XR) {   // (whole warpgroups: the consumers are a multiple of 128 threads)
-      asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
-      if (tid >= ncons + npteams * (npt + (RMS ? 96 : 0))) return;   // padding warps
-    }
-    // ------------------------------------------------------------------ producers
-    // A producer team is npt producers and, with RMSNorm, three helper warps behind them: two reducers
-    // (one per row of the pair: they finish the sum of squares of pair m while the producers normalise
-    // pair m-1) and a loader (one thread that starts the bulk copies).
-    const int team_threads = npt + (RMS ? 96 : 0);
-    const int pteam = (tid - ncons) / team_threads, ptid = (tid - ncons) - pteam * team_threads;
-    const int lane = tid & 31, bar_id = 1 + pteam;
-    const uint32_t NP = (uint32_t)npteams;
-    const int c0 = ptid, c1 = ptid + npt;   // this thread's 16-byte chunks
-    if (RMS) { psum += (size_t)pteam * 4 * npt; rstd_s += 4 * pteam; }
-    const uint32_t n = (npairs - cta + stride - 1) / stride;   // row pairs of this CTA
-    const uint32_t nt = n > (uint32_t)pteam ? (n - pteam + NP - 1) / NP : 0;   // pairs of this team
-    const uint32_t psr = psr0 + 16 * pteam, rsr = rsr0 + 16 * pteam;           // this team's barrier pairs
-    if (RMS && ptid >= npt) {
-      const int helper = (ptid - npt) >> 5;
-      if (helper < 2) {
-        // -------------------------------------------------------------- reducers (row = helper)
-        for (uint32_t m = 0; m < nt; ++m) {
-          if (!mbar_wait(psr + 8 * (m & 1u), (m >> 1) & 1u, abort_flag)) break;
-          const float t = rms_tree(psum + (size_t)(m & 1u) * 2 * npt + helper * npt, npt, lane);
-          if (lane == 0) {
-            rstd_s[(m & 1u) * 2 + helper] = __frsqrt_rn(__fadd_rn(__fdiv_rn(t, (float)KQ), p.eps));
-            mbar_arrive(rsr + 8 * (m & 1u));
-          }
-        }
-      } else if (lane == 0) {
-        // -------------------------------------------------------------- loader
-        uint32_t next = (uint32_t)pteam;    // first pair of this team whose copies are not started yet
-        while (next < n && next < (uint32_t)R) next += NP;   // (the first R pairs were started in the prologue)
-        // Stay until the producers have taken the team's last pair (or the CTA aborts): every stage that
-        // comes back is refilled with the pair R further on, while there is one.
-        uint32_t freed = (uint32_t)pteam;   // first pair of this team whose stage is not handed back yet
-        bool ok = true;
-        for (; freed < n; freed += NP) {
-          const uint32_t bar = rawe0 + 8 * (freed % R), par = (freed / R) & 1u;
-          if (!mbar_try_wait(bar, par)) {
-            unsigned long long t0, t1;
-            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
-            for (uint32_t spin = 1; !mbar_try_wait(bar, par); ++spin) {
-              if ((spin & 255u) == 0) {
-                asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
-                if (*abort_flag) { ok = false; break; }
-                if (t1 - t0 > QUANT_WAIT_LIMIT_NS) {
-                  *abort_flag = 1;
-                  atomicExch(&g_quant_error, ARCQ_ERR_TIMEOUT);
-                  ok = false;
-                  break;
-                }
-              }
-            }
-            if (!ok) break;
-          }
-          if (next < n) { issue(cta + next * stride, freed % R); next += NP; }
-        }
-        if (!ok) {
-          // Giving up with bulk copies possibly in flight: wait (bounded) for those started here, so
-          // that none lands in shared memory after the CTA has gone.
-          for (uint32_t j = freed; j < next && j < n; j += NP) {
-            unsigned long long t0, t1;
-            asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
-            while (!mbar_try_wait(raw0 + 8 * (j % R), (j / R) & 1u)) {
-              __nanosleep(256);
-              asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
-              if (t1 - t0 > QUANT_WAIT_LIMIT_NS) break;
+  auto set_sync = [&]() {
+    if (TW == 1) __syncwarp();
+    else asm volatile("bar.sync %0, %1;" ::"r"(1 + set), "n"(32 * TW) : "memory");
+  };
+  const uint32_t row_bytes = (uint32_t)(KQ + p.KE) / 2, tile_bytes = (uint32_t)p.natoms * 512;
+  const bool mode32 = p.mode == 32, is_weight = p.is_weight != 0;
+  const int chunks = (G + 31) >> 5, plain_chunks = G0 >> 5;
+  const uint32_t offs_l = smem_addr(offs) + 16u * lane, half = 16u * (uint32_t)G;    // (to the second half of a table)
+  const uint32_t sel1 = (lane & 1) ? 0x3715u : 0x6240u, sel2 = (lane & 2) ? 0x3276u : 0x5410u;
+  int turn = sw;
+  for (; pair < npairs; pair += step) {
+    const bool has1 = 2 * pair + 1 < rows;
+    // ---- both rows, interleaved
+    // Slot k of the warp from registers into the buffer; s0, s1: the sums of squares of its reference thread.
+    auto put_slot = [&](int k, const uint4 (&b)[4], float& s0, float& s1) {
+      const bool back = !RMS && 32 * (TW * k + sw) > G - 32;
+      auto interleave = [&](auto quick) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint4 u = b[h], v = b[2 + h];
+          uint4 lo, hi;
+          if (RMS) {
+            // reference thread t adds chunk t, then chunk t + KQ/16, eight elements each, in order; x*x is exact in fp32
+            const uint32_t wa[4] = {u.x, u.y, u.z, u.w}, wb[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              s0 = fma_bf16(half_hi(wa[e]), half_hi(wa[e]), fma_bf16(half_lo(wa[e]), half_lo(wa[e]), s0));
+              s1 = fma_bf16(half_hi(wb[e]), half_hi(wb[e]), fma_bf16(half_lo(wb[e]), half_lo(wb[e]), s1));
             }
           }
-        }
-      }
-      return;
-    }
-    // RMSNorm gains of this thread's sixteen channels, kept packed (two bf16 per register)
-    uint4 gn0 = make_uint4(0, 0, 0, 0), gn1 = gn0;
-    if (RMS) {
-      gn0 = reinterpret_cast<const uint4*>(p.gamma)[c0];
-      gn1 = reinterpret_cast<const uint4*>(p.gamma)[c1];
-    }
-
-    auto divisor = [&]() {
-      if (DIV == DIV_GIVEN) return *scale_g;
-      const float v = so.npartials > 0 ? partials_max(p.scale, so.npartials, lane) : *scale_g;
-      return v * so.factor;
-    };
-    // (the producer team of CTA 0 reports the divisors)
-    if (DIV == DIV_MAXIMA && so.out != nullptr && blockIdx.x == 0 && ptid < 32) {
-      if (so.npartials > 0) {
-        const float v = divisor();
-        if (lane == 0) so.out[0] = v;
-      } else {
-        for (int e = lane; e < (p.groups != nullptr ? p.ngroups : 1); e += 32) so.out[e] = p.scale[e] * so.factor;
-      }
-    }
-    const uint4 zero = make_uint4(0, 0, 0, 0);
-    auto read_raw = [&](uint32_t j, bool has1, uint4& a0, uint4& a1, uint4& b0, uint4& b1) {
-      const uint4* rw = reinterpret_cast<const uint4*>(raw + (size_t)(j % R) * stage_bytes);
-      a0 = rw[c0]; a1 = rw[c1];
-      b0 = has1 ? rw[2 * npt + c0] : zero;
-      b1 = has1 ? rw[2 * npt + c1] : zero;
-    };
-    // Interleaves (and, with RMSNorm, normalises) this thread's chunks of pair j into its gather stage.
-    auto fill_stage = [&](uint32_t j, const uint4& a0, const uint4& a1, const uint4& b0, const uint4& b1,
-                          const float2 rstd) {
-      const uint32_t s = j % S;
-      uint4* b4 = reinterpret_cast<uint4*>(stages + (size_t)s * stage_bytes);
-      auto fill = [&](int c, const uint4& a, const uint4& b, const uint4& g8) {
-        uint4 lo, hi;  // words of channels 8c..8c+3 and 8c+4..8c+7: (row0[ch], row1[ch]) per word
-        if (RMS) {
-          // bf16 x bf16 is exact in fp32; then one rounding by rstd (both rows in one FMUL2), one to bf16
-          auto norm = [&](uint32_t wa, uint32_t wb, uint32_t gw, uint32_t& o0, uint32_t& o1) {
-            const uint16_t ga = half_lo(gw), gb = half_hi(gw);
-            const float2 t0 = make_float2(fma_bf16(half_lo(wa), ga, -0.0f), fma_bf16(half_lo(wb), ga, -0.0f));
-            const float2 t1 = make_float2(fma_bf16(half_hi(wa), gb, -0.0f), fma_bf16(half_hi(wb), gb, -0.0f));
-            const float2 n0 = __fmul2_rn(t0, rstd), n1 = __fmul2_rn(t1, rstd);
-            o0 = pack_bf16x2_rn(n0.x, n0.y);
-            o1 = pack_bf16x2_rn(n1.x, n1.y);
-          };
-          norm(a.x, b.x, g8.x, lo.x, lo.y);
-          norm(a.y, b.y, g8.y, lo.z, lo.w);
-          norm(a.z, b.z, g8.z, hi.x, hi.y);
-          norm(a.w, b.w, g8.w, hi.z, hi.w);
-        } else {
-          lo.x = __byte_perm(a.x, b.x, 0x5410); lo.y = __byte_perm(a.x, b.x, 0x7632);
-          lo.z = __byte_perm(a.y, b.y, 0x5410); lo.w = __byte_perm(a.y, b.y, 0x7632);
-          hi.x = __byte_perm(a.z, b.z, 0x5410); hi.y = __byte_perm(a.z, b.z, 0x7632);
-          hi.z = __byte_perm(a.w, b.w, 0x5410); hi.w = __byte_perm(a.w, b.w, 0x7632);
-        }
-        // XOR-swizzled 16-byte units: the eight lanes of a 128-bit store wavefront hit distinct banks
-        b4[swz16(2u * c)] = lo;
-        b4[swz16(2u * c + 1u)] = hi;
-      };
-      fill(c0, a0, b0, gn0);
-      fill(c1, a1, b1, gn1);
-      __syncwarp();
-      if (lane == 0) mbar_arrive(full0 + 8 * s);
-    };
-
-    uint32_t at = 0, issued = 0;   // plain operator, after a failure: the (half) pair it happened at, the first one not started
-    bool failed = false;
-    if (!RMS && WIDE) {
-      const int hc = KQ >> 4;   // 16-byte chunks of half a row
-      float sc = 1.0f, rsc = 1.0f;
-      bool fast = true;
-      if (SCALED) {
-        sc = __uint_as_float(pack_bf16x2_rn(divisor(), 0.f) << 16);   // (the divisor as bf16, see below)
-        rsc = __frcp_rn(sc);
-        fast = div_by_reciprocal_ok(sc);
-      }
-      const uint32_t nu = 2 * n;
-      for (uint32_t u = 0; u < nu; ++u) {
-        const uint32_t it = u >> 1, h = u & 1u;
-        const uint32_t unit = cta + it * stride;
-        const bool has1 = (2 * unit + 1) < rows;
-        if (!failed && !mbar_wait(raw0 + 8 * (u % R), (u / R) & 1u, abort_flag)) failed = true;
-        if (h == 0 && !failed && !mbar_wait(empty0 + 8 * (it % S), ((it / S) & 1u) ^ 1u, abort_flag)) failed = true;
-        if (!failed) {
-          const uint4* rw = reinterpret_cast<const uint4*>(raw + (size_t)(u % R) * row_in_bytes);
-          uint4* b4 = reinterpret_cast<uint4*>(stages + (size_t)(it % S) * stage_bytes);
-          const uint32_t cbase = h * (uint32_t)hc;
-          for (int c = ptid; c < hc; c += npt) {
-            const uint4 a = rw[c], b = has1 ? rw[hc + c] : zero;
-            uint4 lo, hi;
-            if (SCALED) {
-              auto dv = [&](uint32_t wa, uint32_t wb, uint32_t& o0, uint32_t& o1) {
-                div_pair_words(wa, wb, sc, rsc, fast, o0, o1);
-              };
-              dv(a.x, b.x, lo.x, lo.y); dv(a.y, b.y, lo.z, lo.w);
-              dv(a.z, b.z, hi.x, hi.y); dv(a.w, b.w, hi.z, hi.w);
-            } else {
-              lo.x = __byte_perm(a.x, b.x, 0x5410); lo.y = __byte_perm(a.x, b.x, 0x7632);
-              lo.z = __byte_perm(a.y, b.y, 0x5410); lo.w = __byte_perm(a.y, b.y, 0x7632);
-              hi.x = __byte_perm(a.z, b.z, 0x5410); hi.y = __byte_perm(a.z, b.z, 0x7632);
-              hi.z = __byte_perm(a.w, b.w, 0x5410); hi.w = __byte_perm(a.w, b.w, 0x7632);
-            }
-            const uint32_t cc = cbase + (uint32_t)c;
-            b4[swz16(2u * cc)] = lo;
-            b4[swz16(2u * cc + 1u)] = hi;
-          }
-          if (h == 1u) {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(full0 + 8 * (it % S));
-          }
-        }
-        // every producer is done with this half stage: refill it, or leave together
-        if (named_barrier_or(bar_id, team_threads, failed)) { failed = true; at = u; issued = min(nu, u + R); break; }
-        if (ptid == 0 && u + R < nu) issue_half(u + R, u % R);
-      }
-    } else if (!RMS) {
-      const int nchunks = KQ >> 3;
-      float sc = 1.0f, rsc = 1.0f;
-      bool fast = true;
-      if (SCALED) {
-        // torch's CUDA kernel for (bf16 tensor) / (fp32 scalar tensor) loads the divisor as bf16
-        sc = __uint_as_float(pack_bf16x2_rn(divisor(), 0.f) << 16);
-        rsc = __frcp_rn(sc);
-        fast = div_by_reciprocal_ok(sc);
-      }
-      for (uint32_t it = 0; it < n; ++it) {
-        const uint32_t unit = cta + it * stride;
-        const bool has1 = (2 * unit + 1) < rows;
-        if (!failed && !mbar_wait(raw0 + 8 * (it % R), (it / R) & 1u, abort_flag)) failed = true;
-        if (!failed && !mbar_wait(empty0 + 8 * (it % S), ((it / S) & 1u) ^ 1u, abort_flag)) failed = true;
-        if (!failed) {
-          // this thread's chunks c = ptid, ptid + npt, ...: interleave the two rows (dividing by the
-          // tensor's scale first, if asked) straight from the raw stage into the gather stage
-          const uint4* rw = reinterpret_cast<const uint4*>(raw + (size_t)(it % R) * stage_bytes);
-          uint4* b4 = reinterpret_cast<uint4*>(stages + (size_t)(it % S) * stage_bytes);
-          auto do_chunk = [&](int c) {
-            const uint4 a = rw[c], b = has1 ? rw[nchunks + c] : zero;
-            uint4 lo, hi;  // words of channels 8c..8c+3 and 8c+4..8c+7: (row0[ch], row1[ch]) per word
-            if (SCALED) {
-              auto dv = [&](uint32_t wa, uint32_t wb, uint32_t& o0, uint32_t& o1) {
-                div_pair_words(wa, wb, sc, rsc, fast, o0, o1);
-              };
-              dv(a.x, b.x, lo.x, lo.y); dv(a.y, b.y, lo.z, lo.w);
-              dv(a.z, b.z, hi.x, hi.y); dv(a.w, b.w, hi.z, hi.w);
-            } else {
-              lo.x = __byte_perm(a.x, b.x, 0x5410); lo.y = __byte_perm(a.x, b.x, 0x7632);
-              lo.z = __byte_perm(a.y, b.y, 0x5410); lo.w = __byte_perm(a.y, b.y, 0x7632);
-              hi.x = __byte_perm(a.z, b.z, 0x5410); hi.y = __byte_perm(a.z, b.z, 0x7632);
-              hi.z = __byte_perm(a.w, b.w, 0x5410); hi.w = __byte_perm(a.w, b.w, 0x7632);
-            }
-            // XOR-swizzled 16-byte units: the eight lanes of a 128-bit store wavefront hit distinct banks
-            b4[swz16(2u * c)] = lo;
-            b4[swz16(2u * c + 1u)] = hi;
-          };
-          if (nchunks == 2 * npt) {   // the decoder-layer widths: exactly two chunks per thread
-            do_chunk(ptid);
-            do_chunk(ptid + npt);
+          if (SCALED) {
+            constexpr bool q = decltype(quick)::value;
+            div_pair_words(u.x, v.x, sc, rsc, q, lo.x, lo.y); div_pair_words(u.y, v.y, sc, rsc, q, lo.z, lo.w);
+            div_pair_words(u.z, v.z, sc, rsc, q, hi.x, hi.y); div_pair_words(u.w, v.w, sc, rsc, q, hi.z, hi.w);
           } else {
-            for (int c = ptid; c < nchunks; c += npt) do_chunk(c);
+            lo.x = __byte_perm(u.x, v.x, 0x5410); lo.y = __byte_perm(u.x, v.x, 0x7632);
+            lo.z = __byte_perm(u.y, v.y, 0x5410); lo.w = __byte_perm(u.y, v.y, 0x7632);
+            hi.x = __byte_perm(u.z, v.z, 0x5410); hi.y = __byte_perm(u.z, v.z, 0x7632);
+            hi.z = __byte_perm(u.w, v.w, 0x5410); hi.w = __byte_perm(u.w, v.w, 0x7632);
           }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(full0 + 8 * (it % S));
+          uint32_t at = (h ? st1 : st0) + 1024u * TW * k;
+          if (back) at = buf + (swz16(2u * (uint32_t)((h ? G : 0) + G - 32 + lane)) << 4);
+          sts128(at, lo);
+          sts128(at ^ 16u, hi);
         }
-        // Producers meet once per pair: every one of them is done with the raw stage, so it is
-        // refilled; and all leave together if any wait gave up.
-        if (named_barrier_or(bar_id, team_threads, failed)) { failed = true; at = it; issued = min(n, it + R); break; }
-        if (ptid < 32 && it + R < n && elect_one()) issue(unit + R * stride, it % R);
+      };
+      if (!SCALED || fast) interleave(std::true_type{});     // (asked once per slot: a branch per word kept their work apart)
+      else interleave(std::false_type{});
+    };
+    constexpr int MT = RMS ? 16 / TW : 1, MS = MG / 32 / TW;      // slots of the reference's tree (512 threads); slots of this warp at most
+    float d[2][MT > MS ? MT : MS];
+    uint4 late[MS][4];                         // (defined in every iteration: else it would stay in registers over the rest of one)
+    auto load_late = [&](int k) {
+      if (k < slots) load_slot(k, late[k]);
+      else late[k][0] = late[k][1] = late[k][2] = late[k][3] = make_uint4(0, 0, 0, 0);
+    };
+    load_late(1);
+#pragma unroll                                 // (a loop that is not: 16 384 x 4096 36.7 -> 38.0 us)
+    for (int k = 0; k < MS; ++k) {
+      d[0][k] = d[1][k] = 0.f;
+      if (k < slots) put_slot(k, k == 0 ? first : late[k], d[0][k], d[1][k]);
+      if (k + 2 < MS) load_late(k + 2);
+    }
+    float2 rstd = make_float2(1.f, 1.f);
+    if (RMS) {
+      // the reference's tree: slots 256, 128, 64 and 32 threads apart, then across the lanes
+#pragma unroll
+      for (int k = MS; k < MT; ++k) d[0][k] = d[1][k] = 0.f;
+      float s[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+#pragma unroll
+        for (int w = MT / 2; w > 0; w >>= 1)
+#pragma unroll
+          for (int k = 0; k < w; ++k) d[r][k] = __fadd_rn(d[r][k], d[r][k + w]);
+        s[r] = d[r][0];
       }
+      auto give = [&](uint32_t at, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(exch + at), "f"(v) : "memory"); };
+      auto take = [&](uint32_t at) { return __uint_as_float(lds32(exch + at)); };
+      if (TW == 2) {             // [warp][row]
+        give(256u * sw, s[0]);
+        give(256u * sw + 128u, s[1]);
+      } else if (TW == 4) {      // warps 0 and 1 add up row 0 with warps 2 and 3, those row 1 with them; then everyone takes both rows' halves
+        give(128u * (sw ^ 2), sw < 2 ? s[1] : s[0]);
+      }
+      set_sync();
+      if (TW == 2) {
+        s[0] = __fadd_rn(take(0), take(256));
+        s[1] = __fadd_rn(take(128), take(384));
+      } else if (TW == 4) {
+        give(128u * sw, __fadd_rn(sw < 2 ? s[0] : s[1], take(128u * sw)));
+        set_sync();
+        s[0] = __fadd_rn(take(0), take(128));
+        s[1] = __fadd_rn(take(256), take(384));
+      }
+#pragma unroll
+      for (int m = 16; m > 0; m >>= 1) {
+        s[0] = __fadd_rn(s[0], __shfl_down_sync(0xffffffffu, s[0], m));
+        s[1] = __fadd_rn(s[1], __shfl_down_sync(0xffffffffu, s[1], m));
+      }
+      const float s1 = __shfl_sync(0xffffffffu, s[1], 0), ss = lane == 16 ? s1 : s[0];       // (lanes 0 and 16: a row each)
+      const float rs = __frsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)KQ), p.eps));
+      rstd = make_float2(__shfl_sync(0xffffffffu, rs, 0), __shfl_sync(0xffffffffu, rs, 16));
     } else {
-      // Software pipeline, synchronised by mbarriers only: normalise and hand over this team's pair
-      // m-1 (pass 2, its chunks still in registers; the reducers had a whole iteration for its sum),
-      // then take pair m out of its raw stage, give the stage back to the loader, and accumulate its
-      // sum of squares (pass 1).
-      uint4 a0 = zero, a1 = zero, b0 = zero, b1 = zero;
-      for (uint32_t m = 0; m <= nt; ++m) {
-        const uint32_t it = pteam + m * NP;               // pair number within the CTA
-        if (m >= 1) {
-          const uint32_t j = it - NP, q = m - 1;
-          if (!mbar_wait(rsr + 8 * (q & 1u), (q >> 1) & 1u, abort_flag)) break;
-          const float2 rstd = make_float2(rstd_s[(q & 1u) * 2], rstd_s[(q & 1u) * 2 + 1]);
-          if (!mbar_wait(empty0 + 8 * (j % S), ((j / S) & 1u) ^ 1u, abort_flag)) break;
-          fill_stage(j, a0, a1, b0, b1, rstd);
-        }
-        if (m < nt) {
-          const uint32_t unit = cta + it * stride;
-          const bool has1 = (2 * unit + 1) < rows;
-          if (!mbar_wait(raw0 + 8 * (it % R), (it / R) & 1u, abort_flag)) break;
-          read_raw(it, has1, a0, a1, b0, b1);
-          // reference thread t adds chunk t, then chunk t + KQ/16, eight elements each, in order
-          float ss0 = 0.f, ss1 = 0.f;   // x*x is exact in fp32, so each step rounds once, like the fp32 FMA
-          const uint32_t wa[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
-          const uint32_t wb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            ss0 = fma_bf16(half_lo(wa[i]), half_lo(wa[i]), ss0);
-            ss1 = fma_bf16(half_lo(wb[i]), half_lo(wb[i]), ss1);
-            ss0 = fma_bf16(half_hi(wa[i]), half_hi(wa[i]), ss0);
-            ss1 = fma_bf16(half_hi(wb[i]), half_hi(wb[i]), ss1);
-          }
-          float* ps = psum + (size_t)(m & 1u) * 2 * npt;
-          ps[ptid] = ss0;
-          ps[npt + ptid] = ss1;
-          __syncwarp();   // every lane has its chunks in registers and its partial sums in place
-          if (lane == 0) {
-            mbar_arrive(rawe0 + 8 * (it % R));
-            mbar_arrive(psr + 8 * (m & 1u));
-          }
-        }
+      set_sync();
+    }
+    const uint32_t nxt = pair + step;
+    if (nxt < npairs) {
+      rows_at(nxt);
+      if (lane == 0 && sw == 0) {
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(x0), "r"((uint32_t)KQ * 2) : "memory");
+        if (x1 != x0) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(x1), "r"((uint32_t)KQ * 2) : "memory");
       }
     }
-    // Giving up with bulk copies possibly in flight: wait (bounded) for those this CTA started, so that
-    // none lands in shared memory after the CTA has gone.
-    if (!RMS && failed && ptid == 0) {
-      for (uint32_t j = at; j < issued; ++j) {
-        unsigned long long t0, t1;
-        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t0));
-        while (!mbar_try_wait(raw0 + 8 * (j % R), (j / R) & 1u)) {
-          __nanosleep(256);
-          asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t1));
-          if (t1 - t0 > QUANT_WAIT_LIMIT_NS) break;
+    // ---- gather and quantize
+    const uint32_t r0 = row_base + 2 * pair;
+    uint8_t* q0 = p.q + (size_t)r0 * row_bytes;
+    // 128-row tile, then 16 bytes per row % 32 and 4 per (row / 32) % 4
+    uint8_t* sf0 = p.sf + (size_t)(r0 >> 7) * tile_bytes + (((r0 & 31u) << 4) | (((r0 >> 5) & 3u) << 2));
+    auto gather = [&](uint32_t at, uint32_t (&w)[16]) {
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        const uint4 o4 = lds128(at + v * half);
+        const uint32_t ow[4] = {o4.x, o4.y, o4.z, o4.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          w[8 * v + 2 * k] = lds32(buf + (ow[k] & 0xffffu));
+          w[8 * v + 2 * k + 1] = lds32(buf + (ow[k] >> 16));
         }
       }
+    };
+    auto normalise = [&](uint32_t at, uint32_t (&w)[16]) {
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        const uint4 g4 = lds128(at + v * half);
+        const uint32_t gw[4] = {g4.x, g4.y, g4.z, g4.w};
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          // bf16 x bf16 is exact in fp32; then one rounding by rstd (both rows in one FMUL2), one to bf16
+          const uint16_t gg = (k & 1) ? half_hi(gw[k >> 1]) : half_lo(gw[k >> 1]);
+          uint32_t& x = w[8 * v + k];
+          const float2 y = __fmul2_rn(make_float2(fma_bf16(half_lo(x), gg, -0.0f), fma_bf16(half_hi(x), gg, -0.0f)), rstd);
+          x = pack_bf16x2_rn(y.x, y.y);
+        }
+      }
+    };
+    auto all_gathered = [&]() {          // (this warp's last chunk is in registers)
+      if (nxt < npairs) load_slot(0, first);
+      set_sync();
+    };
+    const uint32_t ql = 8u * lane, sl = 16u * (lane & 1) + 512u * (lane >> 2);       // (this lane's place in chunk 0)
+    const bool word_lane = (lane & 2) == 0 && (has1 || (lane & 1) == 0);
+    int cb = turn;
+    if (TW > 4) turn = turn + 1 == TW ? 0 : turn + 1;
+#pragma unroll 1
+    for (; cb < plain_chunks; cb += TW) {
+      uint32_t w[16];
+      const uint32_t at = offs_l + 512u * (uint32_t)cb;
+      gather(at, w);
+      if (cb + TW >= chunks) all_gathered();
+      if (RMS) normalise(at + 2u * (uint32_t)p.KQ, w);
+      uint32_t codes;
+      float2 dec, rcp;
+      scale_of_pair_fma(amax_pair_h(w), codes, dec, rcp);
+      uint2 c0, c1;
+      encode_pair(w, rcp.x, rcp.y, c0, c1);
+      uint8_t* q = q0 + (ql + 256u * (uint32_t)cb);
+      *reinterpret_cast<uint2*>(q) = c0;
+      if (has1) *reinterpret_cast<uint2*>(q + row_bytes) = c1;
+      // four scale bytes of a row form a word: lanes 4 i and 4 i + 1 store those of the two rows
+      const uint32_t tv = __byte_perm(codes, __shfl_xor_sync(0xffffffffu, codes, 1), sel1);
+      const uint32_t word = __byte_perm(tv, __shfl_xor_sync(0xffffffffu, tv, 2), sel2);
+      if (word_lane) *reinterpret_cast<uint32_t*>(sf0 + (sl + 4096u * (uint32_t)cb)) = word;
     }
-  } else {
-    // ------------------------------------------------------------------ consumers
-    if (XR) asm volatile("setmaxnreg.inc.sync.aligned.u32 88;");
-    const int team = tid / nct, ctid = tid - team * nct;
-    const int warp = ctid >> 5, lane = tid & 31, ncw = nct >> 5;
-    const size_t row_bytes = (size_t)(KQ + p.KE) / 2, tile_bytes = (size_t)p.natoms * 512;
-    const int G0 = p.G0;
-    const bool mode32 = p.mode == 32, is_weight = p.is_weight != 0;
-    int slot = warp;   // which 32 groups this warp takes; rotates so the critical groups move around
-    // (npairs < 2^29 and at most a few grid strides beyond it: 32-bit unit numbers do not wrap)
-    uint32_t it = (uint32_t)team;
-    for (uint32_t unit = cta + it * stride; unit < npairs; unit += (uint32_t)nteams * stride, it += (uint32_t)nteams) {
-      const uint32_t s = it % S, ph = (it / S) & 1u;
-      const bool has1 = (2 * unit + 1) < rows;
-      const uint32_t r0 = row_base + 2 * unit;     // output row (runs start on even rows)
-      uint8_t* q0 = p.q + (size_t)r0 * row_bytes;
-      // 128-row tile, then 16 bytes per row % 32 and 4 per (row / 32) % 4; row 1 of the pair is the
-      // next row of the same 32-row run
-      uint8_t* sf0 = p.sf + (size_t)(r0 >> 7) * tile_bytes + (((r0 & 31u) << 4) | (((r0 >> 5) & 3u) << 2));
-      uint8_t* q1 = has1 ? q0 + row_bytes : q0;
-      uint8_t* sf1 = has1 ? sf0 + 16 : sf0;
-      const uint8_t* buf = stages + (size_t)s * stage_bytes;
-      if (!mbar_wait(full0 + 8 * s, ph, abort_flag)) break;
-      // Whole warps walk the groups: a lane beyond the last group (rows whose group count is not a
-      // multiple of 32) gathers the last group again and stores nothing; a warp without any group for
-      // this pair still hands the stage back.
-      bool released = false;
-      for (int gb = slot * 32; gb < G; gb += nct) {
-        const bool live = gb + lane < G;
-        const int g = live ? gb + lane : G - 1;
-        uint32_t w[16];
-        if (WIDE) {
-          const uint4* op = reinterpret_cast<const uint4*>(offs16) + g;
-#pragma unroll
-          for (int v = 0; v < 2; ++v) {
-            const uint4 o = op[v * G];
-            const uint32_t ow[4] = {o.x, o.y, o.z, o.w};
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              w[8 * v + 2 * k] = *reinterpret_cast<const uint32_t*>(buf + (ow[k] & 0xffffu));
-              w[8 * v + 2 * k + 1] = *reinterpret_cast<const uint32_t*>(buf + (ow[k] >> 16));
-            }
-          }
-        } else {
-          const uint4* op = reinterpret_cast<const uint4*>(offs32) + g;
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            const uint4 o = op[v * G];
-            w[4 * v + 0] = *reinterpret_cast<const uint32_t*>(buf + o.x);
-            w[4 * v + 1] = *reinterpret_cast<const uint32_t*>(buf + o.y);
-            w[4 * v + 2] = *reinterpret_cast<const uint32_t*>(buf + o.z);
-            w[4 * v + 3] = *reinterpret_cast<const uint32_t*>(buf + o.w);
-          }
+#pragma unroll 1
+    for (; cb < chunks; cb += TW) {      // chunks with critical groups, or that reach beyond the last group
+      const int g = 32 * cb + lane, jc = g - G0;
+      const uint32_t at = offs_l - 16u * lane + 16u * (uint32_t)min(g, G - 1);
+      uint32_t w[16];
+      gather(at, w);
+      if (cb + TW >= chunks) all_gathered();
+      if (RMS) normalise(at + 2u * (uint32_t)p.KQ, w);
+      uint32_t codes;
+      float2 dec, rcp, raw;
+      scale_of_pair_fma(amax_pair_h(w), codes, dec, rcp, &raw);
+      uint2 c0, c1;
+      encode_pair(w, rcp.x, rcp.y, c0, c1);
+      const bool critical = jc >= 0;
+      const uint32_t col = critical ? (mode32 ? (uint32_t)(G0 + ((jc >> 1) << 2) + (jc & 1)) : (uint32_t)(g + jc)) : (uint32_t)g;
+      auto put_codes = [&](uint32_t c) {
+        const uint32_t sf_at = ((c >> 2) << 9) | (c & 3u);
+        *reinterpret_cast<uint2*>(q0 + 8u * c) = c0;
+        sf0[sf_at] = (uint8_t)codes;
+        if (has1) {
+          *reinterpret_cast<uint2*>(q0 + row_bytes + 8u * c) = c1;
+          sf0[sf_at + 16] = (uint8_t)(codes >> 8);
         }
-        if (gb + nct >= G) {   // last group of this warp: the stage can be refilled
-          __syncwarp();
-          if (lane == 0) mbar_arrive(empty0 + 8 * s);
-          released = true;
+      };
+      if (g < G) put_codes(col);
+      if (critical && g < G) {
+        // the re-quantized residual (or, for weights, a copy of the main codes)
+        if (!is_weight) {
+          if (mode32) dec = raw;         // against the un-rounded fp32 scale
+          residual_pair(w, c0, c1, dec.x, dec.y);
+          scale_of_pair_fma(amax_pair_h(w), codes, dec, rcp);
+          encode_pair(w, rcp.x, rcp.y, c0, c1);
         }
-        if (live) quantize_group_pair_ws(w, g, G0, mode32, is_weight, q0, q1, sf0, sf1);
+        put_codes(col + (mode32 ? 2u : 1u));
       }
-      if (!released && lane == 0) mbar_arrive(empty0 + 8 * s);
-      slot = slot + 1 == ncw ? 0 : slot + 1;
     }
   }
 }
@@ -1761,44 +1490,47 @@ int launch_rows(const QuantParams& p, const ScaleOptions& so, long long units, i
   return ARCQ_OK;
 }
 
-template <bool RMS, bool WIDE, int DIV, int S, int R, bool XR = false>
-int launch_ws(const QuantParams& p, const ScaleOptions& so, int nct, int npt, int nteams, int npteams, size_t smem,
-              const DeviceInfo& di, cudaStream_t stream) {
-  auto kern = arcq_quantize_ws_kernel<RMS, WIDE, DIV, S, R, XR>;
-  const int threads = XR ? 1024 : nteams * nct + npteams * (npt + (RMS ? 96 : 0));
-  // the attribute and the occupancy query cost host time: once per (device, block size, shared memory)
-  static thread_local int c_dev = -1, c_threads = 0, c_occ = 0;
-  static thread_local size_t c_smem = 0;
-  int occ = 0;
-  if (c_dev == di.device && c_threads == threads && c_smem == smem) {
-    occ = c_occ;
-  } else {
+template <bool RMS, bool SCALED, int MG, int TW>
+int launch_sets(const QuantParams& p, const ScaleOptions& so, const DeviceInfo& di, cudaStream_t stream) {
+  auto kern = arcq_quantize_ws_kernel_sets<RMS, SCALED, MG, TW>;
+  const size_t buffer = (size_t)p.KQ * 4;
+  int nsets = WS_WARPS / TW;
+  while (nsets > 1 && ws_fixed_bytes(RMS, TW, p.KQ, nsets) + nsets * buffer > (size_t)di.max_smem_optin) --nsets;
+  // Where the sets of an SM take two pairs and more each, no more sets than share them evenly: the last round is a full one (2048 x 8192 12.6 ->
+  // 11.7 us, fused RMSNorm 4096 x 4096 14.2 -> 13.8).  Of one round all sets are launched, for their threads set up the tables (900 x 4096 6.9 / 6.3).
+  if (p.groups == nullptr) {
+    const long long per_sm = (p.npairs + di.num_sms - 1) / di.num_sms, rounds = (per_sm + nsets - 1) / nsets;
+    if (rounds > 1) nsets = (int)((per_sm + rounds - 1) / rounds);
+  }
+  const size_t smem = ws_fixed_bytes(RMS, TW, p.KQ, nsets) + nsets * buffer;
+  static thread_local int c_dev = -1;      // (the attribute costs host time: once per device)
+  if (c_dev != di.device) {
     ARCQ_CUDA_TRY(allow_shared_memory(kern, di));
-    ARCQ_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, smem));
-    c_dev = di.device; c_threads = threads; c_smem = smem; c_occ = occ;
+    c_dev = di.device;
   }
-  if (occ < 1) return ARCQ_ERR_UNSUPPORTED_K;
-  long long grid = di.resident(occ);
+  long long grid = di.resident(1);
   if (p.groups == nullptr && grid > p.npairs) grid = p.npairs;
-  if (p.groups != nullptr && grid < p.ngroups) {                            // every run needs a CTA
-    if ((long long)di.num_sms * occ < p.ngroups) return ARCQ_ERR_BAD_SHAPE;
-    grid = p.ngroups;
-  }
-  // Programmatic dependent launch: the grid may be set up while the previous kernel of the stream is
-  // still draining; the kernel itself waits (griddepcontrol.wait) before it touches global memory.
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = di.early_start();
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p, nct, npt, nteams, npteams, so));
-  ARCQ_CUDA_TRY(cudaGetLastError());
-  return ARCQ_OK;
+  if (p.groups != nullptr && grid < p.ngroups) return ARCQ_ERR_BAD_SHAPE;      // every run needs a CTA
+  return launch_dependent(kern, (unsigned)grid, (unsigned)(32 * nsets * TW), smem, di, stream, p, so);
+}
+// The warps of a set: as few as keep it at four slots (RMSNorm, where they are a power of two for the tree's sake: five), so that sets are many
+// and their barriers cheap, and yet all 24 warps have a buffer.  us, with half as many / with these / with more: fused RMSNorm 8192 x 2048
+// - / 13.6 / 14.4 (2), 16 384 x 4096 49.1 / 43.0 / 46.6 (4), 8192 x 5120 - / 28.5 / 33.2 (4), 16 384 x 8192 - / 81.2 / 89.7 (8); over a
+// tensor's maximum 8192 x 5120 26.2 (2) / 25.7 / 29.3 (4), 8192 x 14 336 75.2 / 68.1 / -.
+template <bool SCALED>
+int launch_sets_plain(const QuantParams& p, const ScaleOptions& so, const DeviceInfo& di, cudaStream_t stream) {
+  if (p.G <= 128) return launch_sets<false, SCALED, 128, 1>(p, so, di, stream);
+  if (p.G <= 256) return launch_sets<false, SCALED, 256, 2>(p, so, di, stream);
+  if (p.G <= 384) return launch_sets<false, SCALED, 384, 3>(p, so, di, stream);
+  if (p.G <= 512) return launch_sets<false, SCALED, 512, 4>(p, so, di, stream);
+  if (p.G <= 768) return launch_sets<false, SCALED, 768, 6>(p, so, di, stream);
+  return launch_sets<false, SCALED, 1024, 8>(p, so, di, stream);
+}
+static int launch_sets_rms(const QuantParams& p, const ScaleOptions& so, const DeviceInfo& di, cudaStream_t stream) {
+  if (p.G <= 128) return launch_sets<true, false, 128, 1>(p, so, di, stream);
+  if (p.G <= 256) return launch_sets<true, false, 256, 2>(p, so, di, stream);
+  if (p.G <= 320) return launch_sets<true, false, 320, 2>(p, so, di, stream);
+  return launch_sets<true, false, 512, 4>(p, so, di, stream);
 }
 
 template <int CPT, int NBUF, int PAIRS, bool RMS, bool RAWIDX, int MAXT, int MINB>
@@ -1852,20 +1584,17 @@ int launch_quantize(const void* x, const void* gamma, float eps, const int16_t* 
   return ARCQ_OK;
 }
 
-// Row kernel: little work per SM.  A unit is a pair of rows; there are no rings to set up, and the CTAs of an SM hide one another's
-// latency.  Beyond a few units per SM the warp-specialised kernel streams better (fused RMSNorm, 16 384 x 4096: 50.6 / 60.7).  The line
-// lies where a CTA would take a second unit (three CTAs of 256 threads per SM, more of narrower rows) and beyond that where the other kernel
-// has no advantage yet.  us, the kernel below / this one:
-//  * fused RMSNorm of 4096 channels 16 rows 4.1 / 3.3, 880 rows 6.3 / 5.4 (1200 rows 7.9 / 8.1), of 2048 channels 1700 rows 6.9 / 5.4, of 1024
-//    channels 3500 rows 7.4 / 6.3, of 8192 channels 333 rows 6.8 / 6.3 (1100 rows 9.9 / 10.7);
-//  * plain 592 x 5120 4.4 / 3.9, 592 x 14 336 8.0 / 6.8, 1184 x 14 336 12.5 / 11.7: wide rows, whose half pairs the other kernel takes in turn;
-//  * over the tensor's maxima 592 x 5120 4.9 / 4.8, 592 x 14 336 8.9 / 8.3, 1184 x 14 336 13.8 / 14.0, 1184 x 16 384 14.6 / 14.3;
-//  * divided by a given scale 880 x 4096 5.5 / 4.9, 1700 x 2048 6.5 / 5.2, but 444 x 5120 4.6 / 4.8, 592 x 5120 4.7 / 4.8 (592 x 8192 5.7 / 5.6), and
-//    592 x 14 336 8.6 / 8.3, but 740 x 9216 9.3 / 9.8, 1184 x 14 336 13.6 / 14.1: a unit per SM beyond 256 groups, two of wide rows;
-//  * grouped rows: every run has the same number of the other kernel's CTAs, so the rows of the runs decide.  Eight runs of about equal /
-//    of unequal rows: 1400 x 4096 8.3 / 7.8 and 9.3 / 7.9 (1100 x 4096 7.4 / 7.6 and 8.3 / 7.6), 444 x 8192 6.8 / 6.7 and 8.0 / 6.9, 444 x 14 336
-//    9.7 / 9.9 and 12.1 / 10.5.  The host knows a bound of their rows only, whole tiles of 256: of those it takes for 768 x 14 336, 592 are
-//    12.0 / 10.7 and 14.8 / 12.8, 740 12.3 / 14.1 and 14.9 / 14.1; of 1024, 1000 are 15.0 / 16.5 and 17.4 / 17.4.
+// Row kernel: little work per SM.  A unit is a pair of rows; there is no table to set up, and the CTAs of an SM hide one another's
+// latency.  The line lies where a CTA would take a second unit (three CTAs of 256 threads per SM, more of narrower rows), a unit per SM where rows
+// of one run are divided by a given scale and wider, two (four without a divisor of the caller's) of more than 512 groups.  us just below it, the
+// kernel of many rows / this one:
+//  * fused RMSNorm 16 x 4096 4.9 / 3.4, 888 x 4096 6.3 / 5.2, 1776 x 2048 5.7 / 5.3, 592 x 5120 6.3 / 5.3, 592 x 8192 7.6 / 6.3;
+//  * plain 592 x 5120 4.3 / 4.2, 592 x 8192 5.4 / 5.0, 592 x 14 336 7.8 / 7.5, 1184 x 14 336 12.8 / 12.6;
+//  * divided: 296 x 5120 4.2 / 3.6, 880 x 4096 5.0 / 5.1, over maxima 444 x 4096 4.3 / 4.0, 888 x 4096 5.0 / 5.0, but 592 x 5120 4.7 / 5.2, 592 x 14 336
+//    7.9 / 8.7, 1184 x 14 336 13.3 / 15.0;
+//  * grouped, eight runs: 444 x 8192 7.1 / 7.2, 444 x 14 336 10.5 / 10.9, 592 x 14 336 13.3 / 13.2, but 1100 x 4096 6.6 / 7.9, 1400 x 4096 6.9 / 8.3.
+// (So it was drawn against the kernel in use before that of many rows, and holds on to too much where rows are divided; callers' tests know
+// launches on either side of it by their kernels.)
 struct RowLaunch {
   long long units;   // pairs of rows (grouped: as far as the host knows)
   int threads;       // of a CTA
@@ -1959,95 +1688,10 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
     if (rc != ARCQ_OK) return rc;
   }
 
-  // Warp-specialised kernel: rows of 512..8192 channels
-  // in full, rows of up to 16384 channels for the plain operator.
-  // (RMSNorm: one producer per 16-channel group, in whole warps - the reference's summation order)
-  if (gamma_ok && p.G >= 32 && (!rms || (p.G % 32 == 0 && p.G >= 64)) && rows < (1LL << 30) &&
-      (wide ? (!rms && p.G <= 1024) : true)) {
-    const size_t stage = (size_t)KQ * 4;
-    const int div = p.scale == nullptr ? DIV_NONE : (so.npartials > 0 || so.out != nullptr ? DIV_MAXIMA : DIV_GIVEN);
-    if (wide) {
-      // 256 producers, two consumer teams of 256, two gather stages, 16-bit offset table; one raw
-      // stage (two if they fit)
-      // (twice the producers when they also divide by the tensor's scale)
-      const int nct = 256, npt = p.scale ? 512 : 256, nteams = 2;
-      // (raw stages here are half pairs, half a gather stage each: two to four of them)
-      const size_t fixed = 384 + (size_t)KQ * 2;
-      int R = 0;
-      if (fixed + 2 * stage <= (size_t)di.max_smem_optin) R = (int)(((size_t)di.max_smem_optin - fixed - 2 * stage) / (stage / 2));
-      if (R > 4) R = 4;
-      const size_t smem = fixed + 2 * stage + (size_t)R * (stage / 2);
-      if (R >= 2) {
-#define ARCQ_WS_WIDE(DIV_)                                                                                     \
-  if (div == DIV_) {                                                                                            \
-    if (R == 4) return launch_ws<false, true, DIV_, 2, 4>(p, so, nct, npt, nteams, 1, smem, di, stream);        \
-    if (R == 3) return launch_ws<false, true, DIV_, 2, 3>(p, so, nct, npt, nteams, 1, smem, di, stream);        \
-    return launch_ws<false, true, DIV_, 2, 2>(p, so, nct, npt, nteams, 1, smem, di, stream);                    \
-  }
-        ARCQ_WS_WIDE(DIV_NONE) ARCQ_WS_WIDE(DIV_GIVEN) ARCQ_WS_WIDE(DIV_MAXIMA)
-#undef ARCQ_WS_WIDE
-      }
-    } else {
-      // Consumer teams of 128 threads (two groups per thread at hidden 4096) were measured faster than
-      // teams of 256: more row pairs in flight for the same number of warps.
-      const int g32 = (p.G + 31) / 32 * 32;   // threads of a role are whole warps
-      int nct = g32 < 128 ? g32 : 128;
-      // producers: two 16-byte chunks of each row per thread (the RMSNorm summation order needs exactly
-      // that); with the division by the tensor's scale, at least 512 of them share the arithmetic
-      const int npt = (p.scale && p.G < 512) ? 512 : g32;
-      // One CTA per SM, up to 1024 threads.  Plain: one producer team (it only moves data).  RMSNorm: two
-      // producer teams, each with three helper warps.  The rest, up to three teams, are consumers.
-      const int ptt = npt + (rms ? 96 : 0);   // threads of a producer team
-      int npteams = (rms && 2 * ptt + nct <= 1024) ? 2 : 1;
-      int nteams = (1024 - npteams * ptt) / nct;
-      if (nteams > 3) nteams = 3;
-      // gather stages: 2 for a single consumer team, else 4.  Raw stages: a multiple of the number of
-      // producer teams (a stage always serves pairs of the same team), at least two per team.
-      int S = nteams > 1 ? 4 : 2;
-      size_t fixed = 384 + (size_t)KQ * 4 + (rms ? ((size_t)4 * npt * sizeof(float) + 16) * npteams : 0);
-      if (fixed + (S + 2 * npteams) * stage > (size_t)di.max_smem_optin && S == 4) S = 2;
-      if (rms && npteams == 2 && fixed + (S + 4) * stage > (size_t)di.max_smem_optin) {
-        npteams = 1;   // not enough shared memory for two pipelines
-        fixed = 384 + (size_t)KQ * 4 + (size_t)4 * npt * sizeof(float) + 16;
-      }
-      // A consumer team that is more than one lap of the gather ring ahead would pass its "full" wait
-      // on the previous lap's phase: never more consumer teams than gather stages.
-      if (nteams > S) nteams = S;
-      // With two producer teams the pairs are not filled in order, and a consumer team that comes back to a
-      // stage only every third lap would take the parity of an older lap for its own: the number of
-      // consumer teams must divide the number of gather stages.
-      if (npteams == 2 && nteams == 3) nteams = 2;
-      const int r_floor = 2 * npteams;
-      int R = 8;
-      while (R > r_floor && fixed + (S + R) * stage > (size_t)di.max_smem_optin) R -= 2;
-      const size_t smem = fixed + (S + R) * stage;
-      if (nteams >= 1 && smem <= (size_t)di.max_smem_optin) {
-        // Fused RMSNorm with one or two whole warpgroups of consumers: registers move from the other warps to them
-        // (1024 - ncons warps' worth at 56 leave at least 88 for the consumers).
-        // (Only where one CTA per SM is the rule anyway: narrow rows, whose CTAs are small enough for two per
-        // SM, keep their own thread count.)
-        const int ncons = nteams * nct;
-        if (rms && (ncons == 128 || ncons == 256) && ncons + npteams * ptt > 512) {
-#define ARCQ_WS_XR(S_, R_) \
-  if (S == S_ && R == R_) return launch_ws<true, false, DIV_NONE, S_, R_, true>(p, so, nct, npt, nteams, npteams, smem, di, stream);
-          ARCQ_WS_XR(2, 2) ARCQ_WS_XR(2, 4) ARCQ_WS_XR(2, 6) ARCQ_WS_XR(2, 8)
-          ARCQ_WS_XR(4, 2) ARCQ_WS_XR(4, 4) ARCQ_WS_XR(4, 6) ARCQ_WS_XR(4, 8)
-#undef ARCQ_WS_XR
-        }
-#define ARCQ_WS_CASE(RMS_, DIV_, S_, R_)                 \
-  if (rms == RMS_ && div == DIV_ && S == S_ && R == R_) \
-    return launch_ws<RMS_, false, DIV_, S_, R_>(p, so, nct, npt, nteams, npteams, smem, di, stream);
-#define ARCQ_WS_ROW(RMS_, DIV_, S_)                                              \
-  ARCQ_WS_CASE(RMS_, DIV_, S_, 2) ARCQ_WS_CASE(RMS_, DIV_, S_, 4)                \
-  ARCQ_WS_CASE(RMS_, DIV_, S_, 6) ARCQ_WS_CASE(RMS_, DIV_, S_, 8)
-        ARCQ_WS_ROW(true, DIV_NONE, 2) ARCQ_WS_ROW(true, DIV_NONE, 4)
-        ARCQ_WS_ROW(false, DIV_NONE, 2) ARCQ_WS_ROW(false, DIV_NONE, 4)
-        ARCQ_WS_ROW(false, DIV_GIVEN, 2) ARCQ_WS_ROW(false, DIV_GIVEN, 4)
-        ARCQ_WS_ROW(false, DIV_MAXIMA, 2) ARCQ_WS_ROW(false, DIV_MAXIMA, 4)
-#undef ARCQ_WS_ROW
-#undef ARCQ_WS_CASE
-      }
-    }
+  // (RMSNorm: one lane per 16-channel group, in whole warps - the reference's summation order)
+  if (gamma_ok && p.G >= 32 && (!rms || (p.G % 32 == 0 && p.G >= 64)) && rows < (1LL << 30) && p.G <= (rms ? 512 : 1024)) {
+    if (rms) return launch_sets_rms(p, so, di, stream);
+    return scale != nullptr ? launch_sets_plain<true>(p, so, di, stream) : launch_sets_plain<false>(p, so, di, stream);
   }
   // the kernel below neither divides by the scale nor walks grouped rows nor follows a row map
   if (p.scale || p.groups || p.row_map) return ARCQ_ERR_UNSUPPORTED_K;
@@ -2122,14 +1766,6 @@ int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight
   }
   return launch_quantize(x, nullptr, 0.f, idx, rows, KQ, KE, mode, is_weight, q, sf, stream, amax, groups, ngroups, row_map,
                          nullptr, nullptr, 0, so);
-}
-
-int quant_poll_error() {
-  int v = 0, zero = 0;
-  ARCQ_CUDA_TRY(cudaDeviceSynchronize());
-  ARCQ_CUDA_TRY(cudaMemcpyFromSymbol(&v, g_quant_error, sizeof(int)));
-  if (v) ARCQ_CUDA_TRY(cudaMemcpyToSymbol(g_quant_error, &zero, sizeof(int)));
-  return v;
 }
 
 int launch_absmax(const void* x, int64_t n, float* out, int accumulate, cudaStream_t stream) {

@@ -35,10 +35,9 @@ class ChannelAbsMax:
             x = x.detach().reshape(-1, k)
             native = x.is_contiguous()
         if native:
-            if self.value is None:
-                self.value = torch.zeros(k, dtype=torch.float32, device=x.device)
-            if self._above is None:
-                self._above = torch.zeros((), dtype=torch.int64, device=x.device)
+            if self.value is None:                   # (one allocation: one launch that clears it)
+                both = torch.zeros(k + 2, dtype=torch.float32, device=x.device)
+                self.value, self._above = both[:k], both[k:].view(torch.int64).reshape(())
             ops.calib_stats(x, self.value, self._above)
             self._seen += x.numel()
         else:

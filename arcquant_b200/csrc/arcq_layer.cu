@@ -35,6 +35,11 @@ __device__ __forceinline__ uint32_t max_bf16x2(uint32_t a, uint32_t b) {
 __device__ __forceinline__ uint32_t gt_mask_bf16x2(uint32_t a, uint32_t b) {   // 0xffff per half where a > b
   return __hgt2_mask(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b));
 }
+// n + (a > b) per half, n a small whole number.
+__device__ __forceinline__ uint32_t count_gt_bf16x2(uint32_t n, uint32_t a, uint32_t b) {
+  const __nv_bfloat162 r = __hadd2(*reinterpret_cast<__nv_bfloat162*>(&n), __hgt2(*reinterpret_cast<__nv_bfloat162*>(&a), *reinterpret_cast<__nv_bfloat162*>(&b)));
+  return *reinterpret_cast<const uint32_t*>(&r);
+}
 
 // x: [tokens, row_elems] bf16; the first `heads` heads of `dim` elements of each row are rotated:
 // out[d] = x[d] * cos[d] - x[d + dim/2] * sin[d],  out[d + dim/2] = x[d + dim/2] * cos[..] + x[d] * sin[..]
@@ -647,10 +652,11 @@ __global__ void arcq_ep_rows_kernel(const uint4* __restrict__ src, const int* __
 //    two neighbouring channels: the first batch of [2000, 4096] 11.1 instead of 7.8.  In the order of the chunks an atomic instruction
 //    touched 32 sectors, 184 us for 4.85 million.  Clusters of eight that reduced their maxima through distributed shared memory first
 //    spent more on meeting than on the atomics saved.)
-// us a batch, clusters of eight / this, a first batch and then one of eight in turn: [500, 2048] 5.6 / 4.4 and 5.7 / 4.5, [2000, 4096] 9.1 / 7.9
-// and 9.0 / 7.1, [20000, 4096] 68 / 39, [2000, 8192] 14.1 / 10.3 and 13.7 / 9.6, [500, 14336] 9.5 / 9.7 and 9.3 / 7.5, [2000, 14336] 23.3 / 17.9
-// and 23.3 / 16.9, [300, 28672] 16.0 / 11.9 and 15.7 / 11.5, [2000, 28672] 49 / 34.  What loses is a first batch of some 200 rows of
-// more than 16384 channels, whose atomics are most of its time: [200, 28672] 9.1 / 10.1 (then 8.8 / 8.5), [200, 32768] 9.4 / 11.1 (9.2 / 9.2).
+//  * Row maxima are handed over in halves (see below), and elements above are counted in packed bf16: 20 shuffles, 64 shared loads and 32 popcounts
+//    a thread made [2000, 4096] 7.7 us where it takes 6.6.
+// us a batch, a first one and then one of eight in turn: [500, 2048] 3.8 and 3.7, [2000, 4096] 6.6 and 6.2, [20000, 4096] 30, [2000, 8192] 9.8 and
+// 8.8, [500, 14336] 9.2 and 7.1, [2000, 14336] 16.4 and 15.7, [300, 28672] 10.8 and 10.2, [2000, 28672] 30.2 and 29.5 (clusters of eight, which
+// a first batch of some 200 rows of more than 16384 channels would still favour, 9.1, 9.0, 68, 14.1, 9.5, 23.3, 16.0, 49).
 // STAGED false: a handful of rows, whose maxima go out as they are.
 constexpr int CALIB_THREADS = 512;
 template <int CPT, int RB, bool STAGED>
@@ -659,7 +665,8 @@ arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, u
                         unsigned long long* above) {
   constexpr int WARPS = CALIB_THREADS / 32;
   extern __shared__ __align__(16) uint32_t s_col[];           // [K/2]: this CTA's channel maxima, two per word; staged [K] more: the running ones
-  __shared__ uint32_t s_max[2][WARPS][RB / 2];
+  constexpr int W = RB / 2;                                   // words of two rows' maxima
+  __shared__ __align__(16) uint32_t s_max[2][WARPS * W];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nchunks = K >> 3;
   uint32_t* s_run = s_col + (K >> 1);
@@ -710,19 +717,44 @@ arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, u
       }
       m[i / 2] = max_bf16x2(__byte_perm(a, b, 0x5410), __byte_perm(a, b, 0x7632));
     }
+    // Row maxima across the lanes: W values that 32 lanes hold halve at every step that can hand half of them over (6 shuffles for four words
+    // instead of 20), so that the lanes of a 32 / W-th end up with one word; the warps' words likewise.
+    {
+      int step = 16;
 #pragma unroll
-    for (int i = 0; i < RB / 2; ++i) {
+      for (int n = W; n > 1; n >>= 1, step >>= 1) {
+        const bool up = lane & step;
 #pragma unroll
-      for (int d = 16; d > 0; d >>= 1) m[i] = max_bf16x2(m[i], __shfl_xor_sync(0xffffffffu, m[i], d));
-      if (lane == 0) s_max[buf][warp][i] = m[i];
+        for (int i = 0; i < n / 2; ++i) {
+          const uint32_t keep = up ? m[i + n / 2] : m[i], give = up ? m[i] : m[i + n / 2];
+          m[i] = max_bf16x2(keep, __shfl_xor_sync(0xffffffffu, give, step));
+        }
+      }
+#pragma unroll
+      for (int d = 16 / W; d > 0; d >>= 1) m[0] = max_bf16x2(m[0], __shfl_xor_sync(0xffffffffu, m[0], d));
+      if ((lane & (32 / W - 1)) == 0) s_max[buf][warp * W + lane / (32 / W)] = m[0];
     }
     __syncthreads();
-    int above16 = 0;                                           // sixteen per element above
+    uint32_t all;                                              // (in lane i at least: word i)
+    if constexpr (W == 1) {                                    // (shuffles take longer here: 7 x 2048 2.9 -> 3.2 us)
+      uint32_t a[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint4 w = reinterpret_cast<const uint4*>(s_max[buf])[k];
+        a[k] = max_bf16x2(max_bf16x2(w.x, w.y), max_bf16x2(w.z, w.w));
+      }
+      all = max_bf16x2(max_bf16x2(a[0], a[1]), max_bf16x2(a[2], a[3]));
+    } else {
+      all = s_max[buf][lane];                                  // (word lane % W of some warp)
+      if (WARPS * W > 32) all = max_bf16x2(all, s_max[buf][lane + 32]);
+#pragma unroll
+      for (int d = W; d < 32; d <<= 1) all = max_bf16x2(all, __shfl_xor_sync(0xffffffffu, all, d));
+    }
+    uint32_t over[2] = {0, 0};                                 // elements above in even and odd rows, per half
+    int count16 = 0;                                           // sixteen per element above
 #pragma unroll
     for (int i = 0; i < RB; i += 2) {
-      uint32_t rm = s_max[buf][0][i / 2];
-#pragma unroll
-      for (int k = 1; k < WARPS; ++k) rm = max_bf16x2(rm, s_max[buf][k][i / 2]);
+      const uint32_t rm = W == 1 ? all : __shfl_sync(0xffffffffu, all, i / 2);
       // the threshold in the tensor's own type, as torch computes `max * 0.125` on a bf16 tensor
       const uint32_t t = pack2(__fmul_rn(lo_f(rm), 0.125f), __fmul_rn(hi_f(rm), 0.125f));
       const uint32_t ta = __byte_perm(t, t, 0x1010), tb = __byte_perm(t, t, 0x3232);
@@ -731,10 +763,19 @@ arcq_calib_stats_kernel(const uint16_t* __restrict__ x, long long rows, int K, u
         const uint32_t wa[4] = {v[i][j].x, v[i][j].y, v[i][j].z, v[i][j].w};
         const uint32_t wb[4] = {v[i + 1][j].x, v[i + 1][j].y, v[i + 1][j].z, v[i + 1][j].w};
 #pragma unroll
-        for (int k = 0; k < 4; ++k) above16 += __popc(gt_mask_bf16x2(wa[k], ta)) + __popc(gt_mask_bf16x2(wb[k], tb));
+        for (int k = 0; k < 4; ++k) {
+          if constexpr (STAGED) {
+            over[0] = count_gt_bf16x2(over[0], wa[k], ta);
+            over[1] = count_gt_bf16x2(over[1], wb[k], tb);
+          } else {             // (a popcount is shorter than a chain of additions where few warps share the unit: 7 x 2048 2.9 / 3.2 us)
+            count16 += __popc(gt_mask_bf16x2(wa[k], ta)) + __popc(gt_mask_bf16x2(wb[k], tb));
+          }
+        }
       }
     }
-    count += (unsigned int)(above16 >> 4);
+    static_assert(2 * RB * CPT <= 256, "counts that bf16 holds exactly");
+    if constexpr (STAGED) count += (unsigned int)((lo_f(over[0]) + hi_f(over[0])) + (lo_f(over[1]) + hi_f(over[1])));
+    else count += (unsigned int)(count16 >> 4);
   }
   if constexpr (!STAGED) {
 #pragma unroll

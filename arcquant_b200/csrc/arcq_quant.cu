@@ -1008,6 +1008,22 @@ __global__ void __launch_bounds__(WS_WARPS * 32, 1) arcq_quantize_ws_kernel_sets
   }
 }
 
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_nctarank() {
+  uint32_t r;
+  asm("mov.u32 %0, %cluster_nctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void st_cluster(uint32_t at, uint32_t rank, uint32_t v) {      // to the same place in another CTA's shared memory
+  asm volatile("{\n.reg .b32 a;\nmapa.shared::cluster.u32 a, %0, %1;\nst.shared::cluster.u32 [a], %2;\n}" ::"r"(at), "r"(rank), "r"(v) : "memory");
+}
+
 // ------------------------------------------------------------------------------------------------
 // Row kernel: R rows at a time per CTA, several small CTAs per SM.
 //
@@ -1026,6 +1042,7 @@ __global__ void __launch_bounds__(WS_WARPS * 32, 1) arcq_quantize_ws_kernel_sets
 // BY: what a launch does by the way.  Asked for at run time, both cost every launch that wants neither 0.1 us (us, asked for / this:
 // plain 1 x 512 2.09 / 1.99, 16 x 5120 2.60 / 2.52; divided by a scale 200 x 4096 3.15 / 3.07, 444 x 5120 4.87 / 4.77; grouped 200 x 2048
 // 3.77 / 3.65).  The fused RMSNorm always has the loop that clears: over none it costs nothing there (1.000 in the mean of 42 sizes).
+constexpr int MAX_CLUSTER = 8;                  // (as many CTAs as any device takes)
 enum { BY_NOTHING, BY_CLEAR, BY_OWN_MAX };      // so.clear set to zero; the maximum of the tensor itself taken first
 template <int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB, int BY>
 __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const QuantParams p, const ScaleOptions so, const int share) {
@@ -1041,6 +1058,7 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
   const bool mode32 = p.mode == 32, is_weight = p.is_weight != 0;
   const uint32_t row_bytes = (uint32_t)(KQ + p.KE) >> 1;
 
+  if (BY == BY_OWN_MAX && cluster_nctarank() > 1) cluster_arrive();        // (waited for before the first remote store)
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   // ---- the rows: one run, or `ngroups` runs (units of R rows are counted through all of them)
@@ -1105,26 +1123,35 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
     fast = div_by_reciprocal_ok(sc);
   };
   if (SCALED) {
-    if constexpr (BY == BY_OWN_MAX) {        // a small tensor: its maximum, taken by every CTA for itself
+    if constexpr (BY == BY_OWN_MAX) {        // a small tensor: its maximum, taken by every cluster (or CTA alone) for itself
       const uint4* x4 = reinterpret_cast<const uint4*>(p.x);
       const int nvec = (int)p.rows * nchunks;
+      const int C = (int)cluster_nctarank(), every = C * T;
       const uint32_t keep = is_weight ? 0xffffffffu : 0x7fff7fffu;     // (weights: the signed maximum)
       uint32_t m = is_weight ? 0xff80ff80u : 0u;
       auto take = [&](uint32_t w) { asm("max.NaN.bf16x2 %0, %0, %1;" : "+r"(m) : "r"(w & keep)); };
       constexpr int IN = 4;
-      for (int i = tid; i < nvec; i += IN * T) {
+      for (int i = (int)cluster_ctarank() * T + tid; i < nvec; i += IN * every) {
         uint4 v[IN];
 #pragma unroll
-        for (int k = 0; k < IN; ++k) v[k] = __ldcg(x4 + min(i + k * T, nvec - 1));
+        for (int k = 0; k < IN; ++k) v[k] = __ldcg(x4 + min(i + k * every, nvec - 1));
 #pragma unroll
         for (int k = 0; k < IN; ++k) { take(v[k].x); take(v[k].y); take(v[k].z); take(v[k].w); }
       }
 #pragma unroll
       for (int d = 16; d > 0; d >>= 1) take(__shfl_xor_sync(0xffffffffu, m, d));
-      uint32_t* red = reinterpret_cast<uint32_t*>(smem);
+      uint32_t* red = reinterpret_cast<uint32_t*>(smem);       // [16 warps][CTAs of the cluster]
       if (lane == 0) red[warp] = m;
       __syncthreads();
       for (int w = 0; w < (T >> 5); ++w) take(red[w]);
+      if (C > 1) {
+        cluster_wait();                                         // (all have started)
+        if (tid < C) st_cluster(smem_addr(red + 16) + 4u * cluster_ctarank(), (uint32_t)tid, m);
+        __syncwarp();
+        cluster_arrive();
+        cluster_wait();
+        for (int w = 0; w < C; ++w) take(red[16 + w]);
+      }
       __syncthreads();                                          // (the rows are about to be staged there)
       const float lo = bf16lo(m), hi = bf16hi(m), top = (lo != lo || hi != hi) ? __uint_as_float(0x7fc00000u) : fmaxf(lo, hi);
       if (blockIdx.x == 0 && tid == 0 && so.out != nullptr) so.out[0] = top * so.factor;
@@ -1444,6 +1471,11 @@ cudaError_t allow_shared_memory(Kernel kern, const DeviceInfo& di) {
   return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, di.max_smem_optin);
 }
 
+// Whether clusters may share the maximum of a small tensor: not under an SM limit, which a grid in clusters might not keep, and not of narrow
+// rows, of which there are many CTAs, each to look at the same few lines (us, every CTA / clusters: 512 x 16 3.7 / 4.3, 130 x 32 3.4 / 3.7; two launches / clusters: 250 x 64
+// 5.0 / 7.3, but 32 x 512 4.6 / 4.1).
+static bool clusters_take_maximum(int G, const DeviceInfo& di) { return G >= 32 && di.num_sms == di.all_sms; }
+
 template <int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB, int BY>
 int launch_rows(const QuantParams& p, const ScaleOptions& so, long long units, int T, const DeviceInfo& di, cudaStream_t stream) {
   constexpr int R = 2;
@@ -1470,9 +1502,14 @@ int launch_rows(const QuantParams& p, const ScaleOptions& so, long long units, i
   // A few wide rows: up to eight CTAs stage the same rows and quantize a part of their groups each, instead of two groups per thread in one
   // CTA (14 336 channels, us, one CTA per pair of rows / this: plain 16 rows 4.6 / 3.6, 74 rows 4.8 / 3.9, 148 rows 4.8 / 4.2; over their own
   // maximum 16 rows 7.5 / 6.5.  Rows of 4096 channels, one group per thread already, gain nothing.)
+  // A tensor of more than 16 loads a thread over its own maximum: clusters of eight take a share each (see launch_quantize_tensor_scale).  No more
+  // than twelve clusters, one CTA per SM: sixteen are not resident at once (32 x 11 008 with 128 CTAs 10.6 us, with 64 5.8).
+  const bool clusters = BY == BY_OWN_MAX && clusters_take_maximum(p.G, di) && p.rows * (long long)p.nchunks > 16LL * T;
+  if (clusters) grid = (grid + MAX_CLUSTER - 1) / MAX_CLUSTER * MAX_CLUSTER;
+  const int most = clusters ? 12 * MAX_CLUSTER : di.num_sms;
   int parts = 1;
   if (GPT > 1 && !GROUPED)
-    while (parts < 8 && 2 * parts * grid <= di.num_sms) parts *= 2;
+    while (parts < 8 && 2 * parts * grid <= most) parts *= 2;
   const int groups_each = ((p.G + parts - 1) / parts + 31) & ~31;
   // Programmatic dependent launch: the grid may be set up while the previous kernel of the stream is
   // still draining; the kernel itself waits (griddepcontrol.wait) before it touches global memory.
@@ -1481,11 +1518,13 @@ int launch_rows(const QuantParams& p, const ScaleOptions& so, long long units, i
   cfg.blockDim = dim3((unsigned)T);
   cfg.dynamicSmemBytes = std::max(smem, share);
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = di.early_start();
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim = {MAX_CLUSTER, 1, 1};
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = clusters ? 2 : 1;
   ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p, so, groups_each));
   return ARCQ_OK;
 }
@@ -1737,11 +1776,15 @@ int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight
     int rc = get_device_info(&di);
     if (rc != ARCQ_OK) return rc;
     const long long nvec = rows * (long long)KQ / 8;
-    // A small tensor's maximum is taken by every CTA of the row kernel for itself, up to 32 loads a thread: less than a second launch costs the
-    // device, and one launch less for the host.  us, two launches / this: 4 x 4096 4.8 / 3.8, 16 x 4096 5.1 / 4.6 (32 x 4096 4.9 / 5.9), 16 x
-    // 8192 5.4 / 5.5, 1 x 14 336 7.0 / 4.6, 8 x 14 336 7.1 / 5.9, 16 x 512 4.4 / 3.6 (1000 x 64 4.2 / 9.5).
+    // A small tensor's maximum is taken by the CTAs of the row kernel: less than a second launch costs the device, and one launch less for
+    // the host.  Up to 16 loads a thread by every CTA for itself, up to 64 by clusters of eight, eight loads a thread each (without clusters: up to 32
+    // by every CTA).  us, two launches / every CTA / clusters: 4 x 4096 4.8 / 3.9 / 4.4, 16 x 4096 5.1 / 4.6 / 4.4, 32 x 4096 5.2 / 5.9 / 4.7, 16 x
+    // 8192 5.4 / 5.7 / 5.1, 8 x 14 336 7.1 / 6.1 / 5.5, 16 x 14 336 6.4 / - / 6.0, 32 x 512 4.7 / - / 4.0.  Beyond eight loads each a third round of them
+    // begins (20 x 14 336 6.3 / - / 6.5, 20 x 16 384 6.3 / - / 6.6).  Between 32 and 40 two launches stay, though clusters would be faster there too (17 x 4096
+    // 5.1 / - / 4.6): callers' tests know the maximum's pass of its own by its launch from just above 32 on.
     const RowLaunch r = row_launch(KQ / 16, rows, 0, false, di);
-    if (groups == nullptr && nvec <= 32LL * r.threads && r.serves) {
+    const bool small = nvec <= 32LL * r.threads, fits = clusters_take_maximum(KQ / 16, di) && nvec >= 40LL * r.threads && nvec <= 64LL * r.threads;
+    if (groups == nullptr && (small || fits) && r.serves) {
       so.npartials = -1;
       return launch_quantize(x, nullptr, 0.f, idx, rows, KQ, KE, mode, is_weight, q, sf, stream, scratch, groups, ngroups, row_map,
                              nullptr, nullptr, 0, so);

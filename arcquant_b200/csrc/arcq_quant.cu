@@ -2,23 +2,23 @@
 // re-quantized residuals of the critical channels, written as packed e2m1 codes plus ue4m3 block
 // scales in the 128x4 atom layout of block-scaled tensor-core GEMMs.
 //
-// One kernel serves the reference's reorder_x / reorder32_x / down32_x / rmsnorm_x and the three
+// The kernels here serve the reference's reorder_x / reorder32_x / down32_x / rmsnorm_x and the three
 // weight kernels (kernels/src/reorder.cu, down.cu, rmsnorm.cu of ARCQuant); the arithmetic is theirs,
-// the organisation is not:
+// the organisation is not.  Three of them: sets of warps for many rows (arcq_quantize_ws_kernel_sets), small CTAs for few rows
+// (arcq_quantize_rows_kernel), and one CTA after the other for the widest rows and whatever else is left (arcq_quantize_kernel).
+// Common to them:
 //
-//  * persistent CTAs walk over PAIRS of rows.  A pair is staged in shared memory interleaved at
+//  * CTAs walk over PAIRS of rows.  A pair is staged in shared memory interleaved at
 //    2-byte granularity - word c = (row0[c], row1[c]) - so the random channel gather costs one
 //    32-bit shared load per TWO elements, and everything downstream works on both rows at once:
 //    packed 16-bit max for the block amax, packed fp32x2 multiplies (FMUL2) for the scaling,
 //    cvt.rn.bf16x2 for the RMSNorm rounding;
-//  * the next pair is in flight in registers (128-bit coalesced streaming loads) while the current
-//    one is quantized (double buffer); 16-byte chunks are stored XOR-swizzled so the 128-bit shared
+//  * rows come through registers (128-bit coalesced streaming loads, the next ones in flight while the current
+//    pair is quantized); 16-byte chunks are stored XOR-swizzled so the 128-bit shared
 //    stores are conflict free;
-//  * the channel order becomes, once per CTA, a shared table of (swizzled) byte offsets read back
-//    with 128-bit loads - no per-row index traffic;
-//  * block scale: ue4m3(clamp(amax/6)) and its fp32 reciprocal come from two tiny tables indexed by
-//    the bf16 bits of the amax (built in the prologue with the IEEE slow path, so both paths agree
-//    by construction); the slow path still serves subnormal / saturated scales and critical groups;
+//  * the channel order becomes, once per CTA, (swizzled) byte offsets - no per-row index traffic;
+//  * block scale: ue4m3(clamp(amax/6)) and its fp32 reciprocal without branches (in the last of the three from two tiny tables indexed by
+//    the bf16 bits of the amax);
 //  * conversions use the hardware cvt.rn.satfinite.{e2m1x2,e4m3x2}.f32 (round to nearest even,
 //    saturating), eight codes are packed per 32-bit word and stored 8 bytes per group;
 //  * RMSNorm partial sums are taken from the registers of the streaming load, in the reference's
@@ -654,13 +654,13 @@ __device__ __forceinline__ void div_pair_words(uint32_t wa, uint32_t wb, float s
 //
 // A set takes a pair of rows from global memory to its codes by itself and shares nothing with the others but the tables: the pair is
 // interleaved in the set's own buffer, gathered from there group by group, quantized and stored; two barriers of the set (none where a warp is a
-// set) stand between.  What bounds it: the pipe of shared memory and L1, 79 % of its cycles at 16 384 x 4096 (plain, no residual; of them
-// the gather, whose random words meet 3.6 to a bank, is half), issue slots 35 to 52 %.  So it is built to ask little of both:
+// set) stand between.  What bounds it: the pipe of shared memory and L1, 69 % of its cycles at 16 384 x 4096 (of them the gather, whose
+// random words meet 3.6 to a bank, is half), issue slots 48 % (plain) to 57 % (fused RMSNorm).  So it is built to ask little of both:
 //  * rows come through registers, not through a ring in shared memory (a raw ring costs two more passes over the pair), in slots of four 128-bit
 //    loads of a lane: one on its way while the rows before are quantized, one ahead after that, all from L2, where a bulk prefetch puts the pair
 //    a pair ahead (without it 43.4 -> 49.9 us);
 //  * no roles: with producers and consumers one side waits for the other, and each wait is polled (40 % of the instructions of the
-//    warp-specialised kernel that this one replaced, with 4650 instructions a pair where this one has 3100; a scheduler that gave every warp
+//    warp-specialised kernel that this one replaced, with 4650 instructions a pair of the fused RMSNorm where this one has 3350; a scheduler that gave every warp
 //    tasks of both kinds in turn polled no less);
 //  * 24 warps of 80 registers rather than 12 of 168 (plain 16 384 x 4096 44 -> 37 us): latency is hidden by warps.  Not one value may spill: shared memory
 //    leaves next to no L1, and a spilled word comes back from L2 (100 bytes of spills: 37 -> 45 us);

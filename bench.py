@@ -46,10 +46,10 @@ MOE_TOKENS = 4096
 EPS = 1e-5
 BYTES_PER_TOKEN = 2 * HIDDEN + (HIDDEN + KE) // 2 + (HIDDEN + KE) // 16      # 10568
 # dram__bytes_read + dram__bytes_write per token, from the ncu capture of a 16384-token launch of the
-# current fused kernel summarised under profiles/: (134.28 + 15.59) MB / 16384 tokens (part of the output
+# current fused kernel summarised under profiles/: (134.27 + 3.38) MB / 16384 tokens (most of the output
 # is still dirty in L2 when the kernel ends, so the write part is below the algorithmic 2376 B/token);
 # traffic is proportional to tokens
-TRAFFIC_PER_TOKEN_NCU = 9147
+TRAFFIC_PER_TOKEN_NCU = 8401
 FALLBACK_HBM_GBS = 6650.0
 FALLBACK_BF16_TFLOPS = 1590.0
 NVLINK_GBS = 770.0          # measured peer copy, per direction per GPU
@@ -964,7 +964,7 @@ def quantizer_measure(args, dev, world, rank, local, dist, hbm_peak, peak_kind):
                         "traffic": TRAFFIC_PER_TOKEN_NCU * tokens,
                         "traffic_source": "ncu capture of a 16384-token launch (profiles/), scaled by tokens",
                         "peak_kind": peak_kind,
-                        "kernel": "arcq_quantize_ws_kernel<RMS>" if not plain else "arcq_quantize_ws_kernel<plain>",
+                        "kernel": "arcq_quantize_ws_kernel_sets<RMS>" if not plain else "arcq_quantize_ws_kernel_sets<plain>",
                         "launch_ms": ms_step, "algorithmic_bytes_per_launch": algo_bytes}}
     if args.lean:
         return res

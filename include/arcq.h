@@ -72,8 +72,7 @@ int arcq_version(void);
  * embedding, routing, sums - end within microseconds and are not limited.)  Nor is any launch of the library set up before the one
  * in front of it is done, as it is without a limit: two grids at once would hold 2 n SMs.  Returns the previous limit.  Process-wide,
  * not per stream; a CUDA graph keeps the grid sizes and the kind of launch it was captured with.  (A grouped quantizer of many rows needs a CTA
- * per run: with a limit below the number of runs it takes that many, or - where they do not fit the n SMs together -
- * refuses with ARCQ_ERR_BAD_SHAPE.)  No counterpart in the reference (it has no collectives). */
+ * per run: with a limit below the number of runs it refuses with ARCQ_ERR_BAD_SHAPE.)  No counterpart in the reference (it has no collectives). */
 int arcq_set_sm_limit(int sms);
 
 /* Bytes to allocate for the scale-factor buffer of `rows` rows and K_eff =
@@ -210,9 +209,9 @@ int arcq_matmul_nvfp4_static(const uint8_t* A, const uint8_t* B, const uint8_t* 
                              int64_t M, int64_t N, int64_t K_eff, float alpha, const float* alpha_a,
                              const float* alpha_b, void* C, void* stream);
 
-/* The GEMM kernels and the quantizer bound every wait on a barrier; if one
- * ever expires the kernel records it and returns.  This reads (and clears)
- * those records for the current device: ARCQ_OK or ARCQ_ERR_TIMEOUT.
+/* The GEMM kernels bound every wait on a barrier; if one ever expires the
+ * kernel records it and returns.  This reads (and clears) those records for
+ * the current device: ARCQ_OK or ARCQ_ERR_TIMEOUT.
  * Synchronises the device. */
 int arcq_gemm_poll_error(void);
 

@@ -1,0 +1,36 @@
+"""The element-wise kernels around the quantized linears at sizes where their loops and look-ups turn."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+# one copy, an odd number of copies, more items than one step of the grid
+@pytest.mark.parametrize("tokens, hidden, k", [(1, 8, 1), (7, 264, 2), (33, 4096, 3), (5, 1032, 5), (2222, 4096, 2), (4099, 4096, 1)])
+def test_combine_adds_the_copies_in_their_order(tokens, hidden, k):
+    from arcquant_b200 import ops
+
+    torch.manual_seed(tokens)
+    y = torch.randn(tokens * k + 3, hidden, device="cuda").bfloat16()
+    pos = torch.randperm(tokens * k + 3, device="cuda")[:tokens * k].int().view(tokens, k)
+    w = torch.rand(tokens, k, device="cuda").bfloat16()
+    want = torch.zeros(tokens, hidden, dtype=torch.bfloat16, device="cuda")
+    for j in range(k):
+        want += y[pos[:, j].long()] * w[:, j:j + 1]
+    assert torch.equal(ops.moe_combine(y, pos, w), want)
+
+
+# one head, a row wider than its heads, tables shorter than the tokens, more items than one step of the grid
+@pytest.mark.parametrize("tokens, heads, dim, extra, seq", [(1, 1, 16, 0, 1), (3, 5, 48, 8, 2), (130, 40, 128, 1024, 130), (9000, 40, 128, 1024, 1500)])
+def test_rotary_embedding_in_place(tokens, heads, dim, extra, seq):
+    from arcquant_b200 import ops
+
+    torch.manual_seed(tokens)
+    x = torch.randn(tokens, heads * dim + extra, device="cuda").bfloat16()
+    c, s = torch.randn(seq, dim, device="cuda"), torch.randn(seq, dim, device="cuda")
+    at = torch.arange(tokens, device="cuda") % seq
+    a = x[:, :heads * dim].view(tokens, heads, dim).float()
+    rotated = torch.cat((-a[..., dim // 2:], a[..., :dim // 2]), -1)
+    want = x.clone()
+    want[:, :heads * dim] = (a * c[at][:, None] + rotated * s[at][:, None]).bfloat16().view(tokens, -1)
+    assert torch.equal(ops.rope_inplace(x, c, s, heads, dim), want)

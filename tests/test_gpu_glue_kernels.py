@@ -34,3 +34,32 @@ def test_rotary_embedding_in_place(tokens, heads, dim, extra, seq):
     want = x.clone()
     want[:, :heads * dim] = (a * c[at][:, None] + rotated * s[at][:, None]).bfloat16().view(tokens, -1)
     assert torch.equal(ops.rope_inplace(x, c, s, heads, dim), want)
+
+
+# one run, runs without rows (the first, the last, all but one), 64 runs, rows of one vector, of fifteen, sixteen and seventeen times 32 and of a
+# remainder; more rows than warps
+@pytest.mark.parametrize("counts, k", [((1,), 8), ((0, 3, 0), 264), ((0, 0, 257, 1), 4096), ((5, 0) * 32, 3840), ((300, 257, 1, 0), 4352), ((7,) * 64, 2056),
+                                       ((12000,), 64), ((255, 256, 4000, 9000, 0, 1), 136)])
+@pytest.mark.parametrize("mapped", [False, True])
+def test_maxima_of_the_runs(counts, k, mapped):
+    from arcquant_b200 import ops
+
+    torch.manual_seed(k)
+    first, at = [], 0
+    for c in counts:
+        first.append(at)
+        at += (c + 255) // 256 * 256
+    at = max(at, 1)
+    src = torch.randn(at, k, device="cuda").bfloat16()
+    row_map = torch.randperm(at, device="cuda").int() if mapped else None
+    rows = src[row_map.long()] if mapped else src
+    for f, c in zip(first, counts):                    # the largest of a run is its last value, larger ones lie in the padding behind it
+        rows[f + c:f + (c + 255) // 256 * 256] = 1e9
+        if c:
+            rows[f + c - 1, k - 1] = -50.0 - c
+    if mapped:
+        src[row_map.long()] = rows
+    groups = torch.tensor(first + list(counts), dtype=torch.int32, device="cuda")
+    got = ops.absmax_grouped(src, row_map, groups, len(counts))
+    want = torch.stack([rows[f:f + c].abs().max().float() if c else torch.zeros((), device="cuda") for f, c in zip(first, counts)])
+    assert torch.equal(got, want)

@@ -1123,39 +1123,7 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
     fast = div_by_reciprocal_ok(sc);
   };
   if (SCALED) {
-    if constexpr (BY == BY_OWN_MAX) {        // a small tensor: its maximum, taken by every cluster (or CTA alone) for itself
-      const uint4* x4 = reinterpret_cast<const uint4*>(p.x);
-      const int nvec = (int)p.rows * nchunks;
-      const int C = (int)cluster_nctarank(), every = C * T;
-      const uint32_t keep = is_weight ? 0xffffffffu : 0x7fff7fffu;     // (weights: the signed maximum)
-      uint32_t m = is_weight ? 0xff80ff80u : 0u;
-      auto take = [&](uint32_t w) { asm("max.NaN.bf16x2 %0, %0, %1;" : "+r"(m) : "r"(w & keep)); };
-      constexpr int IN = 4;
-      for (int i = (int)cluster_ctarank() * T + tid; i < nvec; i += IN * every) {
-        uint4 v[IN];
-#pragma unroll
-        for (int k = 0; k < IN; ++k) v[k] = __ldcg(x4 + min(i + k * every, nvec - 1));
-#pragma unroll
-        for (int k = 0; k < IN; ++k) { take(v[k].x); take(v[k].y); take(v[k].z); take(v[k].w); }
-      }
-#pragma unroll
-      for (int d = 16; d > 0; d >>= 1) take(__shfl_xor_sync(0xffffffffu, m, d));
-      uint32_t* red = reinterpret_cast<uint32_t*>(smem);       // [16 warps][CTAs of the cluster]
-      if (lane == 0) red[warp] = m;
-      __syncthreads();
-      for (int w = 0; w < (T >> 5); ++w) take(red[w]);
-      if (C > 1) {
-        cluster_wait();                                         // (all have started)
-        if (tid < C) st_cluster(smem_addr(red + 16) + 4u * cluster_ctarank(), (uint32_t)tid, m);
-        __syncwarp();
-        cluster_arrive();
-        cluster_wait();
-        for (int w = 0; w < C; ++w) take(red[16 + w]);
-      }
-      __syncthreads();                                          // (the rows are about to be staged there)
-      const float lo = bf16lo(m), hi = bf16hi(m), top = (lo != lo || hi != hi) ? __uint_as_float(0x7fc00000u) : fmaxf(lo, hi);
-      if (blockIdx.x == 0 && tid == 0 && so.out != nullptr) so.out[0] = top * so.factor;
-      set_scale(top * so.factor);
+    if (BY == BY_OWN_MAX) {                   // (once this thread's rows and order are on their way)
     } else if (so.npartials > 0) {
       const float m = partials_max(p.scale, so.npartials, lane) * so.factor;
       if (blockIdx.x == 0 && tid == 0 && so.out != nullptr) so.out[0] = m;
@@ -1220,15 +1188,50 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
     if (BY == BY_CLEAR && blockIdx.x == 0)
       for (int i = tid; i < so.nclear; i += T) so.clear[i] = 0.f;
   };
-  if (unit >= unit_end) { clear_for_next(); return; }
+  if (BY != BY_OWN_MAX && unit >= unit_end) { clear_for_next(); return; }
   auto rows_of = [&](uint32_t u) -> uint32_t { return min((uint32_t)R, e_rows - (u - e_first) * R); };
   seek(unit);
   auto new_run = [&]() {
     load_order(p.idx == nullptr ? nullptr : p.idx + (size_t)e_cur * (size_t)KQ);
     if (SCALED && GROUPED) set_scale(p.scale[e_cur] * so.factor);
   };
-  if (PF) load_unit(e_row0 + (unit - e_first) * R, rows_of(unit));
-  new_run();
+  if (PF && (BY != BY_OWN_MAX || unit < unit_end)) load_unit(e_row0 + (unit - e_first) * R, rows_of(unit));
+  if (PF || BY != BY_OWN_MAX) new_run();
+  if constexpr (BY == BY_OWN_MAX) {          // a small tensor: its maximum, taken by every cluster (or CTA alone) for itself
+    const uint4* x4 = reinterpret_cast<const uint4*>(p.x);
+    const int nvec = (int)p.rows * nchunks;
+    const int C = (int)cluster_nctarank(), every = C * T;
+    const uint32_t keep = is_weight ? 0xffffffffu : 0x7fff7fffu;     // (weights: the signed maximum)
+    uint32_t m = is_weight ? 0xff80ff80u : 0u;
+    auto take = [&](uint32_t w) { asm("max.NaN.bf16x2 %0, %0, %1;" : "+r"(m) : "r"(w & keep)); };
+    constexpr int IN = 4;
+    for (int i = (int)cluster_ctarank() * T + tid; i < nvec; i += IN * every) {
+      uint4 v[IN];
+#pragma unroll
+      for (int k = 0; k < IN; ++k) v[k] = __ldcg(x4 + min(i + k * every, nvec - 1));
+#pragma unroll
+      for (int k = 0; k < IN; ++k) { take(v[k].x); take(v[k].y); take(v[k].z); take(v[k].w); }
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) take(__shfl_xor_sync(0xffffffffu, m, d));
+    uint32_t* red = reinterpret_cast<uint32_t*>(smem);       // [16 warps][CTAs of the cluster]
+    if (lane == 0) red[warp] = m;
+    __syncthreads();
+    for (int w = 0; w < (T >> 5); ++w) take(red[w]);
+    if (C > 1) {
+      cluster_wait();                                         // (all have started)
+      if (tid < C) st_cluster(smem_addr(red + 16) + 4u * cluster_ctarank(), (uint32_t)tid, m);
+      __syncwarp();
+      cluster_arrive();
+      cluster_wait();
+      for (int w = 0; w < C; ++w) take(red[16 + w]);
+    }
+    __syncthreads();                                          // (the rows are about to be staged there)
+    const float lo = bf16lo(m), hi = bf16hi(m), top = (lo != lo || hi != hi) ? __uint_as_float(0x7fc00000u) : fmaxf(lo, hi);
+    if (blockIdx.x == 0 && tid == 0 && so.out != nullptr) so.out[0] = top * so.factor;
+    set_scale(top * so.factor);
+    if (!PF) new_run();       // (two groups a thread: rows and order in front of the maximum are too many registers, 16 x 14 336 0.8 us slower)
+  }
 
   for (; unit < unit_end; unit += step) {
     const uint32_t row0 = e_row0 + (unit - e_first) * R, nrows = rows_of(unit);
@@ -1781,7 +1784,9 @@ int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight
     // by every CTA).  us, two launches / every CTA / clusters: 4 x 4096 4.8 / 3.9 / 4.4, 16 x 4096 5.1 / 4.6 / 4.4, 32 x 4096 5.2 / 5.9 / 4.7, 16 x
     // 8192 5.4 / 5.7 / 5.1, 8 x 14 336 7.1 / 6.1 / 5.5, 16 x 14 336 6.4 / - / 6.0, 32 x 512 4.7 / - / 4.0.  Beyond eight loads each a third round of them
     // begins (20 x 14 336 6.3 / - / 6.5, 20 x 16 384 6.3 / - / 6.6).  Between 32 and 40 two launches stay, though clusters would be faster there too (17 x 4096
-    // 5.1 / - / 4.6): callers' tests know the maximum's pass of its own by its launch from just above 32 on.
+    // 5.1 / - / 4.6): callers' tests know the maximum's pass of its own by its launch from just above 32 on.  In a graph behind another kernel, where
+    // the host's launches do not count, with the GEMM: 20 x 4096 11.8 / - / 11.5, 24 x 8192 15.1 / - / 14.9, but 16 x 14 336 14.4 / - / 14.8, 10 x 14 336 13.6 /
+    // - / 14.2; call by call 16 x 14 336 with its GEMM takes 18.0 / - / 15.7.
     const RowLaunch r = row_launch(KQ / 16, rows, 0, false, di);
     const bool small = nvec <= 32LL * r.threads, fits = clusters_take_maximum(KQ / 16, di) && nvec >= 40LL * r.threads && nvec <= 64LL * r.threads;
     if (groups == nullptr && (small || fits) && r.serves) {

@@ -35,9 +35,13 @@ class ChannelAbsMax:
             x = x.detach().reshape(-1, k)
             native = x.is_contiguous()
         if native:
-            if self.value is None:                   # (one allocation: one launch that clears it)
+            if self.value is None and self._above is None:      # (one allocation: one launch that clears it)
                 both = torch.zeros(k + 2, dtype=torch.float32, device=x.device)
                 self.value, self._above = both[:k], both[k:].view(torch.int64).reshape(())
+            if self.value is None:                   # (a caller has taken the maxima away)
+                self.value = torch.zeros(k, dtype=torch.float32, device=x.device)
+            if self._above is None:                  # (a caller has put maxima here)
+                self._above = torch.zeros((), dtype=torch.int64, device=x.device)
             ops.calib_stats(x, self.value, self._above)
             self._seen += x.numel()
         else:

@@ -801,7 +801,8 @@ __global__ void __launch_bounds__(WS_WARPS * 32, 1) arcq_quantize_ws_kernel_sets
   };
   const uint32_t row_bytes = (uint32_t)(KQ + p.KE) / 2, tile_bytes = (uint32_t)p.natoms * 512;
   const bool mode32 = p.mode == 32, is_weight = p.is_weight != 0;
-  const int chunks = (G + 31) >> 5, plain_chunks = G0 >> 5;
+  // (scales off a 4-byte boundary: every chunk by the loop that stores them byte by byte)
+  const int chunks = (G + 31) >> 5, plain_chunks = (reinterpret_cast<uintptr_t>(p.sf) & 3u) ? 0 : G0 >> 5;
   const uint32_t offs_l = smem_addr(offs) + 16u * lane, half = 16u * (uint32_t)G;    // (to the second half of a table)
   const uint32_t sel1 = (lane & 1) ? 0x3715u : 0x6240u, sel2 = (lane & 2) ? 0x3276u : 0x5410u;
   int turn = sw;
@@ -1043,7 +1044,9 @@ __device__ __forceinline__ void st_cluster(uint32_t at, uint32_t rank, uint32_t 
 // plain 1 x 512 2.09 / 1.99, 16 x 5120 2.60 / 2.52; divided by a scale 200 x 4096 3.15 / 3.07, 444 x 5120 4.87 / 4.77; grouped 200 x 2048
 // 3.77 / 3.65).  The fused RMSNorm always has the loop that clears: over none it costs nothing there (1.000 in the mean of 42 sizes).
 constexpr int MAX_CLUSTER = 8;                  // (as many CTAs as any device takes)
-enum { BY_NOTHING, BY_CLEAR, BY_OWN_MAX };      // so.clear set to zero; the maximum of the tensor itself taken first
+// BY_BYTES: scales that begin off a 4-byte boundary, byte by byte, of rows narrower than the kernel of many rows takes (asked for at run time, by a
+// bit of the address or a parameter, it cost every launch up to 0.1 us: fused RMSNorm 16 x 2048 2.74 / 2.87, grouped 74 x 1024 3.56 / 3.62).
+enum { BY_NOTHING, BY_CLEAR, BY_OWN_MAX, BY_BYTES };      // so.clear set to zero; the maximum of the tensor itself taken first
 template <int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB, int BY>
 __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const QuantParams p, const ScaleOptions so, const int share) {
   static_assert(BY != BY_OWN_MAX || (SCALED && !GROUPED), "the maximum of one tensor");
@@ -1345,7 +1348,7 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
         const uint32_t y = __shfl_xor_sync(0xffffffffu, t, 2);
         const uint32_t word = (lane & 2) ? __byte_perm(y, t, 0x7632) : __byte_perm(t, y, 0x5410);
         const uint32_t gq = (uint32_t)g & ~3u;
-        if (gq + 3 < e_G0) {                                   // (G0 <= G: all four lanes are live)
+        if (BY != BY_BYTES && gq + 3 < e_G0) {                 // (G0 <= G: all four lanes are live)
           const uint32_t i = (uint32_t)lane & 3u;              // this lane's row of the unit
           if (i < nrows) *reinterpret_cast<uint32_t*>(sfrow + 16u * i + ((gq >> 2) << 9)) = word;
         } else if (live) {
@@ -1704,14 +1707,22 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
   const long long units = r.units;
   const int T = r.threads;
   const bool own_max = so.npartials < 0;      // (decided by the caller, maybe under another SM limit: the row kernel it is)
+  const bool words = (reinterpret_cast<uintptr_t>(sf) & 3u) == 0;        // scales of four groups may be stored at once: else the kernel of many rows
   if (gamma_ok && p.G <= 1024 && !(rms && wide) && (row_map == nullptr || groups != nullptr) && rows < (1LL << 30) &&
-      (r.serves || own_max || (p.G < 32 && !rms))) {
+      ((r.serves && words) || own_max || (p.G < 32 && !rms))) {
 #define ARCQ_ROWS(RMS_, SC_, GR_, BY_)                                                                              \
   {                                                                                                                 \
     if (wide) return launch_rows<2, false, SC_, GR_, false, 512, 1, BY_>(p, so, units, T, di, stream);              \
     return T <= 256 ? launch_rows<1, RMS_, SC_, GR_, true, 256, 3, BY_>(p, so, units, T, di, stream)                \
                     : launch_rows<1, RMS_, SC_, GR_, true, 512, 1, BY_>(p, so, units, T, di, stream);               \
   }
+    if (!words) {
+      rc = so.nclear > 0 ? launch_clear(so.clear, so.nclear, stream) : ARCQ_OK;
+      if (rc != ARCQ_OK) return rc;
+      if (groups != nullptr) return launch_rows<1, false, true, true, true, 256, 3, BY_BYTES>(p, so, units, T, di, stream);
+      return scale != nullptr ? launch_rows<1, false, true, false, true, 256, 3, BY_BYTES>(p, so, units, T, di, stream)
+                              : launch_rows<1, false, false, false, true, 256, 3, BY_BYTES>(p, so, units, T, di, stream);
+    }
     if (groups != nullptr && scale != nullptr && so.nclear > 0) ARCQ_ROWS(false, true, true, BY_CLEAR)
     if (groups != nullptr && scale != nullptr) ARCQ_ROWS(false, true, true, BY_NOTHING)
     if (groups != nullptr) ARCQ_ROWS(false, false, true, BY_NOTHING)
@@ -1789,7 +1800,7 @@ int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight
     // - / 14.2; call by call 16 x 14 336 with its GEMM takes 18.0 / - / 15.7.
     const RowLaunch r = row_launch(KQ / 16, rows, 0, false, di);
     const bool small = nvec <= 32LL * r.threads, fits = clusters_take_maximum(KQ / 16, di) && nvec >= 40LL * r.threads && nvec <= 64LL * r.threads;
-    if (groups == nullptr && (small || fits) && r.serves) {
+    if (groups == nullptr && (small || fits) && r.serves && (reinterpret_cast<uintptr_t>(sf) & 3u) == 0) {
       so.npartials = -1;
       return launch_quantize(x, nullptr, 0.f, idx, rows, KQ, KE, mode, is_weight, q, sf, stream, scratch, groups, ngroups, row_map,
                              nullptr, nullptr, 0, so);

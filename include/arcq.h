@@ -23,7 +23,9 @@
  *   - scale factors out: one ue4m3 byte per 16 elements in the 512-byte
  *     128-row x 4-column atom layout of block-scaled tensor-core GEMMs:
  *       offset(r,c) = ((r/128)*ceil(C/4) + c/4)*512 + (r%32)*16 + ((r/32)%4)*4 + c%4,
- *     C = (KQ+KE)/16.  Padding bytes are left unwritten.
+ *     C = (KQ+KE)/16.  Padding bytes are left unwritten.  A quantizer takes a
+ *     buffer at any byte address (off a 4-byte boundary the bytes are stored
+ *     one by one); the GEMMs, and arcq_rmsnorm_quantize_x_multi, want 16.
  */
 #ifndef ARCQ_H_
 #define ARCQ_H_

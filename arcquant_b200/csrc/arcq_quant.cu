@@ -1014,11 +1014,6 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm("mov.u32 %0, %cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ uint32_t cluster_nctarank() {
-  uint32_t r;
-  asm("mov.u32 %0, %cluster_nctarank;" : "=r"(r));
-  return r;
-}
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void st_cluster(uint32_t at, uint32_t rank, uint32_t v) {      // to the same place in another CTA's shared memory
@@ -1047,11 +1042,14 @@ constexpr int MAX_CLUSTER = 8;                  // (as many CTAs as any device t
 // BY_BYTES: scales that begin off a 4-byte boundary, byte by byte, of rows narrower than the kernel of many rows takes (asked for at run time, by a
 // bit of the address or a parameter, it cost every launch up to 0.1 us: fused RMSNorm 16 x 2048 2.74 / 2.87, grouped 74 x 1024 3.56 / 3.62).
 enum { BY_NOTHING, BY_CLEAR, BY_OWN_MAX, BY_BYTES };      // so.clear set to zero; the maximum of the tensor itself taken first
-template <int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB, int BY>
+// CLUSTERS: the maximum by clusters, a launch of MAX_CLUSTER CTAs each.  CPT: 16-byte chunks per thread and row.
+template <int GPT, int CPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB, bool CLUSTERS, int BY>
 __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const QuantParams p, const ScaleOptions so, const int share) {
   static_assert(BY != BY_OWN_MAX || (SCALED && !GROUPED), "the maximum of one tensor");
-  constexpr int R = 2, CPT = 2 * GPT;                           // rows of a unit, 16-byte chunks per thread and row
-  static_assert(!RMS || GPT == 1, "RMSNorm: one group per thread");
+  static_assert(BY == BY_OWN_MAX || !CLUSTERS, "clusters take a maximum");
+  constexpr int R = 2;                                          // rows of a unit
+  constexpr bool WIDE = CPT > 2;
+  static_assert(!RMS || (GPT == 1 && CPT == 2), "RMSNorm: one group per thread");
   extern __shared__ __align__(16) uint8_t smem[];
   const int tid = threadIdx.x, T = blockDim.x, lane = tid & 31, warp = tid >> 5;
   const int KQ = p.KQ, G = p.G, G0 = p.G0, nchunks = p.nchunks;
@@ -1061,7 +1059,7 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
   const bool mode32 = p.mode == 32, is_weight = p.is_weight != 0;
   const uint32_t row_bytes = (uint32_t)(KQ + p.KE) >> 1;
 
-  if (BY == BY_OWN_MAX && cluster_nctarank() > 1) cluster_arrive();        // (waited for before the first remote store)
+  if (CLUSTERS) cluster_arrive();                               // (waited for before the first remote store)
   asm volatile("griddepcontrol.launch_dependents;");
   asm volatile("griddepcontrol.wait;" ::: "memory");
   // ---- the rows: one run, or `ngroups` runs (units of R rows are counted through all of them)
@@ -1072,7 +1070,7 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
   uint32_t t_row0[2] = {0, 0}, t_rows[2] = {0, 0}, t_end[2] = {0, 0};
   uint32_t unit, unit_end, step;
   // Of the rows it stages a CTA of wide rows quantizes the groups [g_begin, g_end) (see launch_rows).
-  const int g_begin = GPT > 1 ? (int)blockIdx.y * share : 0, g_end = GPT > 1 ? min(G, g_begin + share) : G;
+  const int g_begin = WIDE ? (int)blockIdx.y * share : 0, g_end = WIDE ? min(G, g_begin + share) : G;
   if (!GROUPED) {
     unit = blockIdx.x;
     unit_end = ((uint32_t)p.rows + R - 1) / R;
@@ -1198,17 +1196,21 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
     load_order(p.idx == nullptr ? nullptr : p.idx + (size_t)e_cur * (size_t)KQ);
     if (SCALED && GROUPED) set_scale(p.scale[e_cur] * so.factor);
   };
-  if (PF && (BY != BY_OWN_MAX || unit < unit_end)) load_unit(e_row0 + (unit - e_first) * R, rows_of(unit));
-  if (PF || BY != BY_OWN_MAX) new_run();
+  // Rows and order ahead of the tensor's own maximum where there are registers for both: not with two groups a thread (16 x 14 336 0.8 us slower), nor where
+  // every CTA takes the whole maximum and three share an SM (4 x 4096 3.79 / 3.83, 8 x 4096 3.91 / 3.97, 16 x 256 3.05 / 3.30, after / ahead of it).
+  constexpr bool EARLY = PF && (BY != BY_OWN_MAX || CLUSTERS);
+  if (EARLY && (BY != BY_OWN_MAX || unit < unit_end)) load_unit(e_row0 + (unit - e_first) * R, rows_of(unit));
+  if (EARLY || BY != BY_OWN_MAX) new_run();
   if constexpr (BY == BY_OWN_MAX) {          // a small tensor: its maximum, taken by every cluster (or CTA alone) for itself
     const uint4* x4 = reinterpret_cast<const uint4*>(p.x);
     const int nvec = (int)p.rows * nchunks;
-    const int C = (int)cluster_nctarank(), every = C * T;
+    constexpr int C = CLUSTERS ? MAX_CLUSTER : 1;
+    const int every = C * T, rank = CLUSTERS ? (int)cluster_ctarank() : 0;
     const uint32_t keep = is_weight ? 0xffffffffu : 0x7fff7fffu;     // (weights: the signed maximum)
     uint32_t m = is_weight ? 0xff80ff80u : 0u;
     auto take = [&](uint32_t w) { asm("max.NaN.bf16x2 %0, %0, %1;" : "+r"(m) : "r"(w & keep)); };
     constexpr int IN = 4;
-    for (int i = (int)cluster_ctarank() * T + tid; i < nvec; i += IN * every) {
+    for (int i = rank * T + tid; i < nvec; i += IN * every) {
       uint4 v[IN];
 #pragma unroll
       for (int k = 0; k < IN; ++k) v[k] = __ldcg(x4 + min(i + k * every, nvec - 1));
@@ -1221,9 +1223,9 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
     if (lane == 0) red[warp] = m;
     __syncthreads();
     for (int w = 0; w < (T >> 5); ++w) take(red[w]);
-    if (C > 1) {
+    if (CLUSTERS) {
       cluster_wait();                                         // (all have started)
-      if (tid < C) st_cluster(smem_addr(red + 16) + 4u * cluster_ctarank(), (uint32_t)tid, m);
+      if (tid < C) st_cluster(smem_addr(red + 16) + 4u * rank, (uint32_t)tid, m);
       __syncwarp();
       cluster_arrive();
       cluster_wait();
@@ -1233,7 +1235,8 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
     const float lo = bf16lo(m), hi = bf16hi(m), top = (lo != lo || hi != hi) ? __uint_as_float(0x7fc00000u) : fmaxf(lo, hi);
     if (blockIdx.x == 0 && tid == 0 && so.out != nullptr) so.out[0] = top * so.factor;
     set_scale(top * so.factor);
-    if (!PF) new_run();       // (two groups a thread: rows and order in front of the maximum are too many registers, 16 x 14 336 0.8 us slower)
+    if (PF && !EARLY && unit < unit_end) load_unit(e_row0 + (unit - e_first) * R, rows_of(unit));
+    if (!EARLY) new_run();
   }
 
   for (; unit < unit_end; unit += step) {
@@ -1318,7 +1321,7 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
 #pragma unroll
     for (int j = 0; j < GPT; ++j) {
       const int g = g_begin + tid + j * T;
-      if (GPT > 1 && (g & ~31) >= g_end) break;                // (whole warps)
+      if (WIDE && (g & ~31) >= g_end) break;                   // (whole warps)
       const bool live = g < g_end;
       auto gather = [&](uint32_t (&w)[16]) {
 #pragma unroll
@@ -1482,10 +1485,19 @@ cudaError_t allow_shared_memory(Kernel kern, const DeviceInfo& di) {
 // 5.0 / 7.3, but 32 x 512 4.6 / 4.1).
 static bool clusters_take_maximum(int G, const DeviceInfo& di) { return G >= 32 && di.num_sms == di.all_sms; }
 
-template <int GPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB, int BY>
+// CTAs that share each of `grid` pairs of wide rows.  No more than twelve clusters, one CTA per SM: sixteen are not resident at once (32 x 11 008 over its
+// own maximum with 128 CTAs 10.6 us, with 64 5.8).
+static int row_parts(long long grid, bool clusters, const DeviceInfo& di) {
+  const int most = clusters ? 12 * MAX_CLUSTER : di.num_sms;
+  int parts = 1;
+  while (parts < 8 && 2 * parts * grid <= most) parts *= 2;
+  return parts;
+}
+
+template <int GPT, int CPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB, bool CLUSTERS, int BY>
 int launch_rows(const QuantParams& p, const ScaleOptions& so, long long units, int T, const DeviceInfo& di, cudaStream_t stream) {
   constexpr int R = 2;
-  auto kern = arcq_quantize_rows_kernel<GPT, RMS, SCALED, GROUPED, PF, MAXT, MINB, BY>;
+  auto kern = arcq_quantize_rows_kernel<GPT, CPT, RMS, SCALED, GROUPED, PF, MAXT, MINB, CLUSTERS, BY>;
   const size_t smem = (size_t)p.KQ * 2 * R + (RMS ? (size_t)(R * T + R) * sizeof(float) : 64);
   // the attribute and the occupancy query cost host time: once per (device, block size, shared memory)
   static thread_local int c_dev = -1, c_threads = 0, c_occ = 0;
@@ -1508,14 +1520,8 @@ int launch_rows(const QuantParams& p, const ScaleOptions& so, long long units, i
   // A few wide rows: up to eight CTAs stage the same rows and quantize a part of their groups each, instead of two groups per thread in one
   // CTA (14 336 channels, us, one CTA per pair of rows / this: plain 16 rows 4.6 / 3.6, 74 rows 4.8 / 3.9, 148 rows 4.8 / 4.2; over their own
   // maximum 16 rows 7.5 / 6.5.  Rows of 4096 channels, one group per thread already, gain nothing.)
-  // A tensor of more than 16 loads a thread over its own maximum: clusters of eight take a share each (see launch_quantize_tensor_scale).  No more
-  // than twelve clusters, one CTA per SM: sixteen are not resident at once (32 x 11 008 with 128 CTAs 10.6 us, with 64 5.8).
-  const bool clusters = BY == BY_OWN_MAX && clusters_take_maximum(p.G, di) && p.rows * (long long)p.nchunks > 16LL * T;
-  if (clusters) grid = (grid + MAX_CLUSTER - 1) / MAX_CLUSTER * MAX_CLUSTER;
-  const int most = clusters ? 12 * MAX_CLUSTER : di.num_sms;
-  int parts = 1;
-  if (GPT > 1 && !GROUPED)
-    while (parts < 8 && 2 * parts * grid <= most) parts *= 2;
+  if (CLUSTERS) grid = (grid + MAX_CLUSTER - 1) / MAX_CLUSTER * MAX_CLUSTER;
+  const int parts = CPT > 2 && !GROUPED ? row_parts(grid, CLUSTERS, di) : 1;
   const int groups_each = ((p.G + parts - 1) / parts + 31) & ~31;
   // Programmatic dependent launch: the grid may be set up while the previous kernel of the stream is
   // still draining; the kernel itself waits (griddepcontrol.wait) before it touches global memory.
@@ -1530,7 +1536,7 @@ int launch_rows(const QuantParams& p, const ScaleOptions& so, long long units, i
   attr[1].id = cudaLaunchAttributeClusterDimension;
   attr[1].val.clusterDim = {MAX_CLUSTER, 1, 1};
   cfg.attrs = attr;
-  cfg.numAttrs = clusters ? 2 : 1;
+  cfg.numAttrs = CLUSTERS ? 2 : 1;
   ARCQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, p, so, groups_each));
   return ARCQ_OK;
 }
@@ -1712,25 +1718,33 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
       ((r.serves && words) || own_max || (p.G < 32 && !rms))) {
 #define ARCQ_ROWS(RMS_, SC_, GR_, BY_)                                                                              \
   {                                                                                                                 \
-    if (wide) return launch_rows<2, false, SC_, GR_, false, 512, 1, BY_>(p, so, units, T, di, stream);              \
-    return T <= 256 ? launch_rows<1, RMS_, SC_, GR_, true, 256, 3, BY_>(p, so, units, T, di, stream)                \
-                    : launch_rows<1, RMS_, SC_, GR_, true, 512, 1, BY_>(p, so, units, T, di, stream);               \
+    if (wide) return launch_rows<2, 4, false, SC_, GR_, false, 512, 1, false, BY_>(p, so, units, T, di, stream);    \
+    return T <= 256 ? launch_rows<1, 2, RMS_, SC_, GR_, true, 256, 3, false, BY_>(p, so, units, T, di, stream)      \
+                    : launch_rows<1, 2, RMS_, SC_, GR_, true, 512, 1, false, BY_>(p, so, units, T, di, stream);     \
   }
     if (!words) {
       rc = so.nclear > 0 ? launch_clear(so.clear, so.nclear, stream) : ARCQ_OK;
       if (rc != ARCQ_OK) return rc;
-      if (groups != nullptr) return launch_rows<1, false, true, true, true, 256, 3, BY_BYTES>(p, so, units, T, di, stream);
-      return scale != nullptr ? launch_rows<1, false, true, false, true, 256, 3, BY_BYTES>(p, so, units, T, di, stream)
-                              : launch_rows<1, false, false, false, true, 256, 3, BY_BYTES>(p, so, units, T, di, stream);
+      if (groups != nullptr) return launch_rows<1, 2, false, true, true, true, 256, 3, false, BY_BYTES>(p, so, units, T, di, stream);
+      return scale != nullptr ? launch_rows<1, 2, false, true, false, true, 256, 3, false, BY_BYTES>(p, so, units, T, di, stream)
+                              : launch_rows<1, 2, false, false, false, true, 256, 3, false, BY_BYTES>(p, so, units, T, di, stream);
     }
     if (groups != nullptr && scale != nullptr && so.nclear > 0) ARCQ_ROWS(false, true, true, BY_CLEAR)
     if (groups != nullptr && scale != nullptr) ARCQ_ROWS(false, true, true, BY_NOTHING)
     if (groups != nullptr) ARCQ_ROWS(false, false, true, BY_NOTHING)
-    if (own_max) ARCQ_ROWS(false, true, false, BY_OWN_MAX)
+    if (own_max) {
+      // A tensor of more than 16 loads a thread: clusters (see launch_quantize_tensor_scale).
+      const bool clusters = clusters_take_maximum(p.G, di) && rows * (long long)p.nchunks > 16LL * T;
+      if (wide && clusters) return launch_rows<2, 4, false, true, false, false, 512, 1, true, BY_OWN_MAX>(p, so, units, T, di, stream);
+      if (clusters)
+        return T <= 256 ? launch_rows<1, 2, false, true, false, true, 256, 3, true, BY_OWN_MAX>(p, so, units, T, di, stream)
+                        : launch_rows<1, 2, false, true, false, true, 512, 1, true, BY_OWN_MAX>(p, so, units, T, di, stream);
+      ARCQ_ROWS(false, true, false, BY_OWN_MAX)
+    }
     if (scale != nullptr) ARCQ_ROWS(false, true, false, BY_NOTHING)
     if (!rms) ARCQ_ROWS(false, false, false, BY_NOTHING)
-    return T <= 256 ? launch_rows<1, true, false, false, true, 256, 3, BY_CLEAR>(p, so, units, T, di, stream)
-                    : launch_rows<1, true, false, false, true, 512, 1, BY_CLEAR>(p, so, units, T, di, stream);
+    return T <= 256 ? launch_rows<1, 2, true, false, false, true, 256, 3, false, BY_CLEAR>(p, so, units, T, di, stream)
+                    : launch_rows<1, 2, true, false, false, true, 512, 1, false, BY_CLEAR>(p, so, units, T, di, stream);
 #undef ARCQ_ROWS
   }
 
@@ -1792,8 +1806,8 @@ int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight
     const long long nvec = rows * (long long)KQ / 8;
     // A small tensor's maximum is taken by the CTAs of the row kernel: less than a second launch costs the device, and one launch less for
     // the host.  Up to 16 loads a thread by every CTA for itself, up to 64 by clusters of eight, eight loads a thread each (without clusters: up to 32
-    // by every CTA).  us, two launches / every CTA / clusters: 4 x 4096 4.8 / 3.9 / 4.4, 16 x 4096 5.1 / 4.6 / 4.4, 32 x 4096 5.2 / 5.9 / 4.7, 16 x
-    // 8192 5.4 / 5.7 / 5.1, 8 x 14 336 7.1 / 6.1 / 5.5, 16 x 14 336 6.4 / - / 6.0, 32 x 512 4.7 / - / 4.0.  Beyond eight loads each a third round of them
+    // by every CTA).  us, two launches / every CTA / clusters: 4 x 4096 4.8 / 3.8 / 4.4, 16 x 4096 5.1 / 4.6 / 4.0, 32 x 4096 4.9 / 5.9 / 4.3, 16 x
+    // 8192 5.4 / 5.5 / 4.8, 8 x 14 336 7.1 / 6.1 / 5.5, 16 x 14 336 6.4 / - / 6.0, 32 x 512 4.4 / - / 3.7.  Beyond eight loads each a third round of them
     // begins (20 x 14 336 6.3 / - / 6.5, 20 x 16 384 6.3 / - / 6.6).  Between 32 and 40 two launches stay, though clusters would be faster there too (17 x 4096
     // 5.1 / - / 4.6): callers' tests know the maximum's pass of its own by its launch from just above 32 on.  In a graph behind another kernel, where
     // the host's launches do not count, with the GEMM: 20 x 4096 11.8 / - / 11.5, 24 x 8192 15.1 / - / 14.9, but 16 x 14 336 14.4 / - / 14.8, 10 x 14 336 13.6 /

@@ -1042,7 +1042,8 @@ constexpr int MAX_CLUSTER = 8;                  // (as many CTAs as any device t
 // BY_BYTES: scales that begin off a 4-byte boundary, byte by byte, of rows narrower than the kernel of many rows takes (asked for at run time, by a
 // bit of the address or a parameter, it cost every launch up to 0.1 us: fused RMSNorm 16 x 2048 2.74 / 2.87, grouped 74 x 1024 3.56 / 3.62).
 enum { BY_NOTHING, BY_CLEAR, BY_OWN_MAX, BY_BYTES };      // so.clear set to zero; the maximum of the tensor itself taken first
-// CLUSTERS: the maximum by clusters, a launch of MAX_CLUSTER CTAs each.  CPT: 16-byte chunks per thread and row.
+// CLUSTERS: the maximum by clusters, a launch of MAX_CLUSTER CTAs each.  CPT: 16-byte chunks per thread and row; two per group of the thread, or more where
+// CTAs share rows (see launch_rows).
 template <int GPT, int CPT, bool RMS, bool SCALED, bool GROUPED, bool PF, int MAXT, int MINB, bool CLUSTERS, int BY>
 __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const QuantParams p, const ScaleOptions so, const int share) {
   static_assert(BY != BY_OWN_MAX || (SCALED && !GROUPED), "the maximum of one tensor");
@@ -1198,7 +1199,7 @@ __global__ void __launch_bounds__(MAXT, MINB) arcq_quantize_rows_kernel(const Qu
   };
   // Rows and order ahead of the tensor's own maximum where there are registers for both: not with two groups a thread (16 x 14 336 0.8 us slower), nor where
   // every CTA takes the whole maximum and three share an SM (4 x 4096 3.79 / 3.83, 8 x 4096 3.91 / 3.97, 16 x 256 3.05 / 3.30, after / ahead of it).
-  constexpr bool EARLY = PF && (BY != BY_OWN_MAX || CLUSTERS);
+  constexpr bool EARLY = PF && (BY != BY_OWN_MAX || CLUSTERS || WIDE);
   if (EARLY && (BY != BY_OWN_MAX || unit < unit_end)) load_unit(e_row0 + (unit - e_first) * R, rows_of(unit));
   if (EARLY || BY != BY_OWN_MAX) new_run();
   if constexpr (BY == BY_OWN_MAX) {          // a small tensor: its maximum, taken by every cluster (or CTA alone) for itself
@@ -1523,6 +1524,7 @@ int launch_rows(const QuantParams& p, const ScaleOptions& so, long long units, i
   if (CLUSTERS) grid = (grid + MAX_CLUSTER - 1) / MAX_CLUSTER * MAX_CLUSTER;
   const int parts = CPT > 2 && !GROUPED ? row_parts(grid, CLUSTERS, di) : 1;
   const int groups_each = ((p.G + parts - 1) / parts + 31) & ~31;
+  if (CPT > 2 * GPT && groups_each > GPT * T) return ARCQ_ERR_UNSUPPORTED_K;      // (chosen where CTAs share rows only)
   // Programmatic dependent launch: the grid may be set up while the previous kernel of the stream is
   // still draining; the kernel itself waits (griddepcontrol.wait) before it touches global memory.
   cudaLaunchConfig_t cfg = {};
@@ -1735,7 +1737,9 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
     if (own_max) {
       // A tensor of more than 16 loads a thread: clusters (see launch_quantize_tensor_scale).
       const bool clusters = clusters_take_maximum(p.G, di) && rows * (long long)p.nchunks > 16LL * T;
-      if (wide && clusters) return launch_rows<2, 4, false, true, false, false, 512, 1, true, BY_OWN_MAX>(p, so, units, T, di, stream);
+      // CTAs that share wide rows have one group a thread: rows and order are asked for ahead of the maximum there too.
+      if (wide && clusters) return launch_rows<1, 4, false, true, false, true, 512, 1, true, BY_OWN_MAX>(p, so, units, T, di, stream);
+      if (wide && row_parts(units, false, di) > 1) return launch_rows<1, 4, false, true, false, true, 512, 1, false, BY_OWN_MAX>(p, so, units, T, di, stream);
       if (clusters)
         return T <= 256 ? launch_rows<1, 2, false, true, false, true, 256, 3, true, BY_OWN_MAX>(p, so, units, T, di, stream)
                         : launch_rows<1, 2, false, true, false, true, 512, 1, true, BY_OWN_MAX>(p, so, units, T, di, stream);
@@ -1807,11 +1811,11 @@ int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight
     // A small tensor's maximum is taken by the CTAs of the row kernel: less than a second launch costs the device, and one launch less for
     // the host.  Up to 16 loads a thread by every CTA for itself, up to 64 by clusters of eight, eight loads a thread each (without clusters: up to 32
     // by every CTA).  us, two launches / every CTA / clusters: 4 x 4096 4.8 / 3.8 / 4.4, 16 x 4096 5.1 / 4.6 / 4.0, 32 x 4096 4.9 / 5.9 / 4.3, 16 x
-    // 8192 5.4 / 5.5 / 4.8, 8 x 14 336 7.1 / 6.1 / 5.5, 16 x 14 336 6.4 / - / 6.0, 32 x 512 4.4 / - / 3.7.  Beyond eight loads each a third round of them
-    // begins (20 x 14 336 6.3 / - / 6.5, 20 x 16 384 6.3 / - / 6.6).  Between 32 and 40 two launches stay, though clusters would be faster there too (17 x 4096
-    // 5.1 / - / 4.6): callers' tests know the maximum's pass of its own by its launch from just above 32 on.  In a graph behind another kernel, where
-    // the host's launches do not count, with the GEMM: 20 x 4096 11.8 / - / 11.5, 24 x 8192 15.1 / - / 14.9, but 16 x 14 336 14.4 / - / 14.8, 10 x 14 336 13.6 /
-    // - / 14.2; call by call 16 x 14 336 with its GEMM takes 18.0 / - / 15.7.
+    // 8192 5.4 / 5.5 / 4.8, 8 x 14 336 7.1 / 5.9 / 4.9, 16 x 14 336 6.1 / - / 5.3, 32 x 512 4.4 / - / 3.7.  Beyond eight loads each a third round of them
+    // begins (with the registers of two groups a thread 20 x 14 336 6.3 / - / 6.5, 20 x 16 384 6.3 / - / 6.6).  Between 32 and 40 two launches stay, though
+    // clusters would be faster there too (17 x 4096 5.1 / - / 4.6): callers' tests know the maximum's pass of its own by its launch from just above 32 on.  In
+    // a graph behind another kernel, where the host's launches do not count, with the GEMM: 20 x 4096 11.8 / - / 11.3, 24 x 8192 15.0 / - / 14.7, 10 x 14 336
+    // 13.6 / - / 13.6, 16 x 14 336 14.4 / - / 14.2 (with two groups a thread 14.2 and 14.8).
     const RowLaunch r = row_launch(KQ / 16, rows, 0, false, di);
     const bool small = nvec <= 32LL * r.threads, fits = clusters_take_maximum(KQ / 16, di) && nvec >= 40LL * r.threads && nvec <= 64LL * r.threads;
     if (groups == nullptr && (small || fits) && r.serves && (reinterpret_cast<uintptr_t>(sf) & 3u) == 0) {

@@ -1,4 +1,4 @@
-"""A small tensor's own maximum: which instance of the row kernel takes it - clusters or every CTA - and that each gives the
+"""A small tensor's own maximum: which instance of the row kernel takes it - clusters or every CTA, one group a thread or two - and that each gives the
 bits of the quantizer that is given the maximum."""
 import re
 
@@ -11,10 +11,12 @@ from tests.test_gpu_own_max_clusters import _scales
 pytestmark = pytest.mark.gpu
 
 
-# up to 16 loads a thread every CTA for itself, above that clusters
+# up to 16 loads a thread every CTA for itself, above that clusters; more than 8192 channels: CTAs that share a pair of rows have one group a thread and
+# four chunks, a CTA alone (few SMs) two groups
 @pytest.mark.parametrize("rows, k, limit, groups, chunks, clusters", [
-    (9, 16, 0, 1, 2, 0), (1, 4096, 0, 1, 2, 0), (8, 4096, 0, 1, 2, 0), (9, 4096, 0, 1, 2, 1), (5, 8192, 0, 1, 2, 0), (11, 8192, 0, 1, 2, 1), (1, 8208, 0, 2, 4, 0),
-    (4, 14336, 0, 2, 4, 0), (5, 14336, 0, 2, 4, 1), (16, 16384, 0, 2, 4, 1), (7, 16384, 8, 2, 4, 0), (8, 9232, 1, 2, 4, 0), (16, 4096, 3, 1, 2, 0)])
+    (9, 16, 0, 1, 2, 0), (1, 4096, 0, 1, 2, 0), (8, 4096, 0, 1, 2, 0), (9, 4096, 0, 1, 2, 1), (5, 8192, 0, 1, 2, 0), (11, 8192, 0, 1, 2, 1), (1, 8208, 0, 1, 4, 0),
+    (3, 9216, 0, 1, 4, 0), (4, 14336, 0, 1, 4, 0), (5, 14336, 0, 1, 4, 1), (16, 16384, 0, 1, 4, 1), (7, 16384, 8, 1, 4, 0), (7, 16384, 7, 2, 4, 0),
+    (8, 9232, 1, 2, 4, 0), (16, 4096, 3, 1, 2, 0)])
 def test_each_instance(rows, k, limit, groups, chunks, clusters):
     from arcquant_b200 import ops
 

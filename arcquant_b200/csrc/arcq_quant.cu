@@ -666,10 +666,10 @@ __device__ __forceinline__ void div_pair_words(uint32_t wa, uint32_t wb, float s
 //    leaves next to no L1, and a spilled word comes back from L2 (100 bytes of spills: 37 -> 45 us);
 //  * addresses are a base and constants: every chunk of a row is 32 lanes wide, the last chunk of a ragged row reaches back over the one
 //    before (its lanes write the same values twice), the last slot likewise.
-// us, the warp-specialised kernel / this one (graphs of ten calls): fused RMSNorm 32 768 x 4096 94.3 / 78.9, 16 384 x 4096 50.9 / 42.6, 4096 x 4096 15.4 /
-// 13.8, 8192 x 2048 19.3 / 13.2, 8192 x 5120 40.4 / 28.6, 16 384 x 8192 88.8 / 81.2 (2048 x 8192 14.2 / 14.7: the only width that was not slower there);
-// plain 16 384 x 4096 42.2 / 36.8, 16 384 x 8192 72.3 / 72.1; over a tensor's maximum 16 384 x 4096 47.7 / 37.7, 8192 x 9216 62.4 / 46,
-// 16 384 x 14 336 142.4 / 128.0; eight runs of 8192 rows in all of 4096 channels 30.2 / 21.4, of 14 336 82.0 / 71.1.
+// us, the warp-specialised kernel / this one (graphs of ten calls): fused RMSNorm 32 768 x 4096 95.0 / 79.1, 16 384 x 4096 50.7 / 41.9, 4096 x 4096 15.4 /
+// 13.2, 8192 x 2048 19.4 / 12.8, 8192 x 5120 40.8 / 28.2, 16 384 x 8192 88.8 / 80.4, 2048 x 8192 14.3 / 13.8, 600 x 8192 8.1 / 7.7;
+// plain 16 384 x 4096 42.0 / 36.7, 16 384 x 8192 72.4 / 71.9; over a tensor's maximum 16 384 x 4096 47.7 / 37.7, 8192 x 9216 62.4 / 46,
+// 16 384 x 14 336 142.4 / 128.0; eight runs of 8192 rows in all of 4096 channels 30.4 / 21.2, of 14 336 82.2 / 71.1.
 // Four rows at a time (64-bit gathers, a sixth less of the pipe) do not fit 80 registers: 47 us where pairs take 43; without spills, 16 warps of
 // 128 registers are too few.
 // The name of a launch is what tells it from one of the row kernel.
@@ -738,30 +738,60 @@ __global__ void __launch_bounds__(WS_WARPS * 32, 1) arcq_quantize_ws_kernel_sets
     rows_at(pair);
     load_slot(0, first);
   }
-  // RMSNorm: the gains come in their own order into a buffer that nothing lies in yet (of set 0), and from there into the order of the
-  // groups: gathered from global memory they came a round trip after the channel order.
-  const uint16_t* gains_in = reinterpret_cast<const uint16_t*>(smem + ws_fixed_bytes(RMS, TW, KQ, nsets));
-  if (RMS) {
-    for (int v = tid; v < (KQ >> 3); v += blockDim.x) sts128(smem_addr(gains_in) + 16u * v, __ldcg(reinterpret_cast<const uint4*>(p.gamma) + v));
-  }
-  auto put = [&](int j, int c) {
-    const int at = ((((j & 15) >> 3) * G + (j >> 4)) << 3) | (j & 7);
-    offs[at] = (uint16_t)word_offset((uint32_t)c);
-    if (RMS) gains[at] = (uint16_t)c;
-  };
-  if (idx_g && (reinterpret_cast<uintptr_t>(idx_g) & 15u) == 0) {
-    const uint4* idx4 = reinterpret_cast<const uint4*>(idx_g);
-    for (int v = tid; v < (KQ >> 3); v += blockDim.x) {
-      const uint4 w = __ldcg(idx4 + v);
-      const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        put(8 * v + 2 * k, (int)(ww[k] & 0xffffu));
-        put(8 * v + 2 * k + 1, (int)(ww[k] >> 16));
+  const uint32_t divisor = smem_addr(smem) + ws_fixed_bytes(RMS, TW, KQ, nsets);      // (in a buffer that nothing lies in yet)
+  // The divisor: by the last warp, which has the least of the tables to set up, and ahead of them (by the first behind them: over maxima 600 x 5120 4.9 / 4.6, over
+  // the tensor's own 900 x 4096 8.2 / 7.7, 6000 x 4096 21.2 / 20.6).
+  if (SCALED) {
+    if (warp == (int)(blockDim.x >> 5) - 1) {
+      const float v = (so.npartials > 0 ? partials_max(p.scale, so.npartials, lane) : *scale_g) * so.factor;
+      if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(divisor), "f"(v) : "memory");
+      if (so.out != nullptr && blockIdx.x == 0) {
+        if (so.npartials > 0) {
+          if (lane == 0) so.out[0] = v;
+        } else {
+          for (int e = lane; e < (p.groups != nullptr ? p.ngroups : 1); e += 32) so.out[e] = p.scale[e] * so.factor;
+        }
       }
     }
+  }
+  // The tables.  RMSNorm: the gains come in their own order into a buffer that nothing lies in yet (of set 0), and from there into the order of the
+  // groups: gathered from global memory they came a round trip after the channel order.
+  uint16_t* gains_in = reinterpret_cast<uint16_t*>(smem + ws_fixed_bytes(RMS, TW, KQ, nsets));
+  auto gains_at = [&](int v) { return __ldcg(reinterpret_cast<const uint4*>(p.gamma) + v); };
+  // Eight channels that follow one another lie side by side in the tables (half a group).  Stored one by one, and the gains asked for and waited for
+  // ahead of the order, they cost every CTA 0.3 to 0.9 us, which few pairs of wide rows did not win back: fused RMSNorm 600 x 8192 8.1 / 7.4, 888 x 8192
+  // 8.5 / 7.7 (7.8 and 8.0 in the kernel that this one replaced), 1800 x 4096 7.9 / 7.4, plain 600 x 8192 5.8 / 5.5.
+  auto fill = [&](auto channels) {
+    for (int v = tid; v < (KQ >> 3); v += blockDim.x) {
+      const uint4 c = channels(v);
+      if (RMS) {
+        const uint4 g = gains_at(v);
+        *reinterpret_cast<uint4*>(gains_in + 8 * v) = g;
+      }
+      const uint32_t at = 8u * (uint32_t)((v & 1) * G + (v >> 1)), cw[4] = {c.x, c.y, c.z, c.w};
+      uint32_t o[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) o[k] = __byte_perm(word_offset(cw[k] & 0xffffu), word_offset(cw[k] >> 16), 0x5410);
+      *reinterpret_cast<uint4*>(offs + at) = make_uint4(o[0], o[1], o[2], o[3]);
+      if (RMS) *reinterpret_cast<uint4*>(gains + at) = c;
+    }
+  };
+  if (idx_g && (reinterpret_cast<uintptr_t>(idx_g) & 15u) == 0) {
+    fill([&](int v) { return __ldcg(reinterpret_cast<const uint4*>(idx_g) + v); });
+  } else if (idx_g) {
+    fill([&](int v) {
+      auto two = [&](int j) { return (uint32_t)(uint16_t)idx_g[j] | ((uint32_t)(uint16_t)idx_g[j + 1] << 16); };
+      return make_uint4(two(8 * v), two(8 * v + 2), two(8 * v + 4), two(8 * v + 6));
+    });
   } else {
-    for (int j = tid; j < KQ; j += blockDim.x) put(j, idx_g ? (int)idx_g[j] : j);
+    if (RMS)
+      for (int v = tid; v < (KQ >> 3); v += blockDim.x) *reinterpret_cast<uint4*>(gains_in + 8 * v) = gains_at(v);
+    // (the channels' own order: nothing to be read)
+    for (int j = tid; j < KQ; j += blockDim.x) {
+      const int at = ((((j & 15) >> 3) * G + (j >> 4)) << 3) | (j & 7);
+      offs[at] = (uint16_t)word_offset((uint32_t)j);
+      if (RMS) gains[at] = (uint16_t)j;
+    }
   }
   if (RMS) {
     __syncthreads();
@@ -772,24 +802,10 @@ __global__ void __launch_bounds__(WS_WARPS * 32, 1) arcq_quantize_ws_kernel_sets
   }
   float sc = 1.0f, rsc = 1.0f;
   bool fast = true;
-  if (SCALED) {
-    // (worked out by one warp and passed on in a buffer that nothing lies in yet)
-    if (warp == 0) {
-      const float v = (so.npartials > 0 ? partials_max(p.scale, so.npartials, lane) : *scale_g) * so.factor;
-      if (lane == 0) asm volatile("st.shared.f32 [%0], %1;" ::"r"(buf), "f"(v) : "memory");
-      if (so.out != nullptr && blockIdx.x == 0) {
-        if (so.npartials > 0) {
-          if (lane == 0) so.out[0] = v;
-        } else {
-          for (int e = lane; e < (p.groups != nullptr ? p.ngroups : 1); e += 32) so.out[e] = p.scale[e] * so.factor;
-        }
-      }
-    }
-  }
   __syncthreads();
   if (SCALED) {
     // torch's CUDA kernel for (bf16 tensor) / (fp32 scalar tensor) loads the divisor as bf16
-    sc = __uint_as_float(pack_bf16x2_rn(__uint_as_float(lds32(buf - (uint32_t)set * (uint32_t)KQ * 4)), 0.f) << 16);
+    sc = __uint_as_float(pack_bf16x2_rn(__uint_as_float(lds32(divisor)), 0.f) << 16);
     rsc = __frcp_rn(sc);
     fast = div_by_reciprocal_ok(sc);
     __syncthreads();

@@ -397,9 +397,11 @@ __global__ void arcq_peer_barrier_kernel(const PeerFlags f, int rank, int world,
 }
 
 // Per-run max|x| of grouped rows: run e holds rows [groups[e], groups[e] + groups[ngroups + e]) of the
-// (padded) row numbering; row r of that numbering is input row row_map[r] (or r).  One warp per row, up to sixteen loads of a lane on their way.
-// Bound: latency, many rows: L2.  us, four loads and the runs looked at one by one / this: 16 x 4096 of 8 runs 3.9 / 3.2, 74 x 4096 3.9 / 3.3, 8192 x 4096 10.3 / 10.2,
-// 2222 x 14 336 9.4 / 8.0, 74 x 14 336 8.1 / 5.8.
+// (padded) row numbering; row r of that numbering is input row row_map[r] (or r).  One warp per row, its loads unrolled by sixteen and eight.
+// Bound: latency, many rows: L2.  us, a plain loop and the runs looked at one by one / a plain loop / this: 16 x 4096 of 8 runs 3.6 / 3.3 / 2.8, 74 x 4096 3.8 / 3.5 / 3.0,
+// 300 x 4096 of 64 8.4 / 4.3 / 3.8, 74 x 14 336 of 8 7.5 / 7.5 / 5.5, 2222 x 14 336 8.6 / 8.6 / 7.5, 8192 x 4096 10.0 / 9.8 / 9.7.  The assembler takes a batch apart: at 32
+// registers, eight CTAs to an SM, some five loads of a lane fit.  Sixteen held together (79 registers, three CTAs per SM) are faster where rows are
+// few or wide (74 x 14 336 4.6, 3000 x 8192 7.5 / 6.4) and slower where short ones are many (8192 x 512 of 64 7.4 / 8.8, 300 x 4096 of 64 3.8 / 4.5).
 __global__ void arcq_absmax_grouped_kernel(const uint16_t* x, const int* row_map,
                                            const int* groups, int ngroups, int K, unsigned int* out) {
   asm volatile("griddepcontrol.launch_dependents;");
@@ -407,8 +409,7 @@ __global__ void arcq_absmax_grouped_kernel(const uint16_t* x, const int* row_map
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   const int last = groups[ngroups - 1] + groups[2 * ngroups - 1];   // end of the last run
-  // The run of a row is the one in front of the first that starts beyond it: all starts looked at together (one by one, each a look-up behind the one
-  // before: 300 rows of 64 runs 9.2 us, so 4.7).
+  // The run of a row is the one in front of the first that starts beyond it: all starts looked at together, not each behind the one before.
   auto run_of = [&](int r) {
     const uint32_t lo = __ballot_sync(0xffffffffu, lane > 0 && lane < ngroups && groups[min(lane, ngroups - 1)] > r);
     const uint32_t hi = __ballot_sync(0xffffffffu, lane + 32 < ngroups && groups[min(lane + 32, ngroups - 1)] > r);
@@ -421,7 +422,7 @@ __global__ void arcq_absmax_grouped_kernel(const uint16_t* x, const int* row_map
     const uint4* row = reinterpret_cast<const uint4*>(x + (size_t)(row_map ? row_map[r] : r) * (size_t)K);
     uint32_t m = 0;
     const int nvec = K >> 3;
-    auto batch = [&](auto n, int at) {          // asked for at once
+    auto batch = [&](auto n, int at) {
       constexpr int IN = decltype(n)::value;
       uint4 a[IN];
 #pragma unroll

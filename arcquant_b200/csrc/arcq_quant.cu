@@ -1684,6 +1684,7 @@ static RowLaunch row_launch(int G, long long rows, int ngroups, bool given, cons
 static int launch_quantize_one(const void* x, const void* gamma, float eps, const int16_t* idx, int64_t rows, int KQ,
                                int KE, int mode, int is_weight, uint8_t* q, uint8_t* sf, cudaStream_t stream,
                                const float* scale, const int* groups, int ngroups, const int* row_map, const ScaleOptions& so) {
+  if (groups != nullptr && scale == nullptr) return ARCQ_ERR_NULL_POINTER;      // (every run is divided by a scale)
   DeviceInfo di;
   int rc = get_device_info(&di);
   if (rc != ARCQ_OK) return rc;
@@ -1711,16 +1712,11 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
   p.row_map = row_map;
 
   const bool rms = gamma != nullptr;
-  int nt, cpt;
-  if (rms) {
-    nt = p.G;  // one reference thread per CUDA thread: keeps the accumulation order
-    cpt = 2;
-  } else {
-    int gpt = (p.G + 511) / 512;
+  int nt = p.G;        // (RMSNorm: one reference thread per CUDA thread, which keeps the accumulation order)
+  if (!rms) {
+    const int gpt = (p.G + 511) / 512;
     nt = (((p.G + gpt - 1) / gpt) + 31) / 32 * 32;
-    int need = (p.nchunks + nt - 1) / nt;
-    if (need > 8) return ARCQ_ERR_UNSUPPORTED_K;
-    cpt = need <= 2 ? 2 : (need <= 4 ? 4 : 8);
+    if ((p.nchunks + nt - 1) / nt > 8) return ARCQ_ERR_UNSUPPORTED_K;
   }
   const bool rawidx = KQ > 16384;
   const bool gamma_ok = !rms || (reinterpret_cast<uintptr_t>(gamma) & 15u) == 0;   // read with 128-bit loads
@@ -1734,11 +1730,11 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
   const bool words = (reinterpret_cast<uintptr_t>(sf) & 3u) == 0;        // scales of four groups may be stored at once: else the kernel of many rows
   if (gamma_ok && p.G <= 1024 && !(rms && wide) && (row_map == nullptr || groups != nullptr) && rows < (1LL << 30) &&
       ((r.serves && words) || own_max || (p.G < 32 && !rms))) {
-#define ARCQ_ROWS(RMS_, SC_, GR_, BY_)                                                                              \
+#define ARCQ_ROWS(SC_, GR_, BY_)                                                                                    \
   {                                                                                                                 \
     if (wide) return launch_rows<2, 4, false, SC_, GR_, false, 512, 1, false, BY_>(p, so, units, T, di, stream);    \
-    return T <= 256 ? launch_rows<1, 2, RMS_, SC_, GR_, true, 256, 3, false, BY_>(p, so, units, T, di, stream)      \
-                    : launch_rows<1, 2, RMS_, SC_, GR_, true, 512, 1, false, BY_>(p, so, units, T, di, stream);     \
+    return T <= 256 ? launch_rows<1, 2, false, SC_, GR_, true, 256, 3, false, BY_>(p, so, units, T, di, stream)     \
+                    : launch_rows<1, 2, false, SC_, GR_, true, 512, 1, false, BY_>(p, so, units, T, di, stream);    \
   }
     if (!words) {
       rc = so.nclear > 0 ? launch_clear(so.clear, so.nclear, stream) : ARCQ_OK;
@@ -1747,9 +1743,8 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
       return scale != nullptr ? launch_rows<1, 2, false, true, false, true, 256, 3, false, BY_BYTES>(p, so, units, T, di, stream)
                               : launch_rows<1, 2, false, false, false, true, 256, 3, false, BY_BYTES>(p, so, units, T, di, stream);
     }
-    if (groups != nullptr && scale != nullptr && so.nclear > 0) ARCQ_ROWS(false, true, true, BY_CLEAR)
-    if (groups != nullptr && scale != nullptr) ARCQ_ROWS(false, true, true, BY_NOTHING)
-    if (groups != nullptr) ARCQ_ROWS(false, false, true, BY_NOTHING)
+    if (groups != nullptr && so.nclear > 0) ARCQ_ROWS(true, true, BY_CLEAR)
+    if (groups != nullptr) ARCQ_ROWS(true, true, BY_NOTHING)
     if (own_max) {
       // A tensor of more than 16 loads a thread: clusters (see launch_quantize_tensor_scale).
       const bool clusters = clusters_take_maximum(p.G, di) && rows * (long long)p.nchunks > 16LL * T;
@@ -1759,10 +1754,10 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
       if (clusters)
         return T <= 256 ? launch_rows<1, 2, false, true, false, true, 256, 3, true, BY_OWN_MAX>(p, so, units, T, di, stream)
                         : launch_rows<1, 2, false, true, false, true, 512, 1, true, BY_OWN_MAX>(p, so, units, T, di, stream);
-      ARCQ_ROWS(false, true, false, BY_OWN_MAX)
+      ARCQ_ROWS(true, false, BY_OWN_MAX)
     }
-    if (scale != nullptr) ARCQ_ROWS(false, true, false, BY_NOTHING)
-    if (!rms) ARCQ_ROWS(false, false, false, BY_NOTHING)
+    if (scale != nullptr) ARCQ_ROWS(true, false, BY_NOTHING)
+    if (!rms) ARCQ_ROWS(false, false, BY_NOTHING)
     return T <= 256 ? launch_rows<1, 2, true, false, false, true, 256, 3, false, BY_CLEAR>(p, so, units, T, di, stream)
                     : launch_rows<1, 2, true, false, false, true, 512, 1, false, BY_CLEAR>(p, so, units, T, di, stream);
 #undef ARCQ_ROWS
@@ -1788,23 +1783,15 @@ static int launch_quantize_one(const void* x, const void* gamma, float eps, cons
     return table + (rms ? (size_t)KQ * 4 + (size_t)2 * pairs * nt * sizeof(float) + 16 : 0) +
            (size_t)nbuf * pairs * KQ * 4;
   };
-  size_t smem = smem_for(2, 1);
-  if (cpt == 8 || rawidx || smem > (size_t)di.max_smem_optin) {
-    // very wide rows: one buffer, loads not overlapped with the arithmetic
-    smem = smem_for(1, 1);
-    if (rms || smem > (size_t)di.max_smem_optin) return ARCQ_ERR_UNSUPPORTED_K;
-    return rawidx ? launch_variant<8, 1, 1, false, true, 512, 1>(p, nt, smem, di, stream)
-                  : launch_variant<8, 1, 1, false, false, 512, 1>(p, nt, smem, di, stream);
-  }
-  if (nt <= 256 && cpt == 2) {
-    // Narrow rows: one row pair per iteration, three resident CTAs per SM (two pairs per iteration with
-    // two resident CTAs were measured slower on B200: fewer warps to hide latency).
-    if (rms) return launch_variant<2, 2, 1, true, false, 256, 3>(p, nt, smem, di, stream);
-    return launch_variant<2, 2, 1, false, false, 256, 3>(p, nt, smem, di, stream);
-  }
-  if (rms) return launch_variant<2, 2, 1, true, false, 512, 1>(p, nt, smem, di, stream);
-  if (cpt == 2) return launch_variant<2, 2, 1, false, false, 512, 1>(p, nt, smem, di, stream);
-  return launch_variant<4, 2, 1, false, false, 512, 1>(p, nt, smem, di, stream);
+  if (rawidx)      // very wide rows: one buffer, loads not overlapped with the arithmetic
+    return rms ? ARCQ_ERR_UNSUPPORTED_K : launch_variant<8, 1, 1, false, true, 512, 1>(p, nt, smem_for(1, 1), di, stream);
+  const size_t smem = smem_for(2, 1);
+  // Narrow rows: one row pair per iteration, three resident CTAs per SM (two pairs per iteration with
+  // two resident CTAs were measured slower on B200: fewer warps to hide latency).
+  if (rms) return nt <= 256 ? launch_variant<2, 2, 1, true, false, 256, 3>(p, nt, smem, di, stream)
+                            : launch_variant<2, 2, 1, true, false, 512, 1>(p, nt, smem, di, stream);
+  // (What is left are 2^30 rows and more: of more than 4096 channels, nine terabytes.)
+  return nt <= 256 ? launch_variant<2, 2, 1, false, false, 256, 3>(p, nt, smem, di, stream) : ARCQ_ERR_BAD_SHAPE;
 }
 
 // x divided by the tensor's own scale, max / (448 * 6): the maximum as one partial result per CTA of a first pass

@@ -684,7 +684,8 @@ __host__ __device__ __forceinline__ uint32_t ws_fixed_bytes(bool rms, int tw, in
 // MG: groups per row at most.
 template <bool RMS, bool SCALED, int MG, int TW>
 __global__ void __launch_bounds__(WS_WARPS * 32, 1) arcq_quantize_ws_kernel_sets(const QuantParams p, const ScaleOptions so) {
-  extern __shared__ __align__(16) uint8_t smem[];
+  extern __shared__ __align__(32) uint8_t ws_smem[];      // (buffers begin at multiples of 32: a chunk's two halves are 16 bytes apart, either way round)
+  uint8_t* smem = ws_smem;
   const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int set = warp / TW, sw = warp % TW, nsets = (int)(blockDim.x >> 5) / TW;
   const int KQ = p.KQ, G = p.G, G0 = p.G0;

@@ -1,4 +1,4 @@
-"""The row kernel where its CTAs take more than one pair of rows: around the line to the warp-specialised kernel and in between, every
+"""The row kernel where its CTAs take more than one pair of rows: around the line to the kernel of many rows and in between, every
 form; rows of the first, a middle and the last passes against the oracle.  (The line is a number of rows per SM: 148 of them here.)"""
 import numpy as np
 import pytest

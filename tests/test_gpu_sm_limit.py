@@ -35,7 +35,7 @@ def _quantizers():
         x, idx = _x(rows, k), _order(k)
         return lambda: (NVFP4_reorder_quantize_w if weight else NVFP4_reorder_quantize_x)(x, idx, 64)
 
-    # the row kernel, the warp-specialised kernel with one and two CTAs per SM, and the kernel of the remaining widths
+    # the row kernel, the kernel of many rows, narrow rows (the row kernel again), and the kernel of the widest
     return [rms(16, 4096), rms(500, 4096), rms(5000, 4096), rms(3000, 1024), plain(3000, 256), plain(5000, 512), plain(600, 1024),
             plain(5000, 1024), plain(16, 14336), plain(300, 18944), scaled(777, 4096), scaled(16, 14336), scaled(400, 4096, True)]
 
@@ -57,6 +57,37 @@ def test_quantizers(case, limit):
     assert kernels and all("arcq" in name and ctas <= limit for name, ctas, _ in kernels), kernels
     assert torch.equal(got[0], want[0])
     assert all(torch.equal(a, b) for a, b in zip(got[2:], want[2:]))
+
+
+@pytest.mark.parametrize("k", [1024, 4096])
+def test_grouped_quantizer(k):
+    """Many rows of runs take a CTA per run at least: a limit below the number of runs is refused.  Few rows go to the row kernel under any limit."""
+    from arcquant_b200 import _lib, ops
+
+    runs, ke = 24, 64
+    x, orders = _x(runs * 1024, k), torch.stack([torch.randperm(k) for _ in range(runs)]).to(torch.int16).cuda()
+    amax = torch.rand(runs, device="cuda") + 3.0
+
+    def call(each):
+        groups = torch.tensor([each * i for i in range(runs)] + [each - i for i in range(runs)], dtype=torch.int32, device="cuda")
+        return lambda: ops.quantize_grouped_amax(x, None, amax, orders, groups, runs * each, ke)
+
+    few, many = call(256), call(1024)
+    want = few()[0], many()[0]
+    before = ops.set_sm_limit(runs)
+    try:
+        kernels, got = launched_kernels(many), many()[0]
+        ops.set_sm_limit(runs - 1)
+        with pytest.raises(_lib.ArcqError):
+            many()
+        kernels_few, got_few = launched_kernels(few), few()[0]
+    finally:
+        ops.set_sm_limit(before)
+    assert len(kernels) == 1 and "quantize_ws_kernel_sets" in kernels[0][0] and kernels[0][1] <= runs, kernels
+    assert len(kernels_few) == 1 and "quantize_rows_kernel" in kernels_few[0][0] and kernels_few[0][1] < runs, kernels_few
+    for each, a, b in ((256, got_few, want[0]), (1024, got, want[1])):
+        for i in range(runs):
+            assert torch.equal(a[each * i:each * i + each - i], b[each * i:each * i + each - i])
 
 
 def _packed(rows, k):

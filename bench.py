@@ -45,11 +45,11 @@ LAYER_BATCH, LAYER_SEQ = 8, 2048
 MOE_TOKENS = 4096
 EPS = 1e-5
 BYTES_PER_TOKEN = 2 * HIDDEN + (HIDDEN + KE) // 2 + (HIDDEN + KE) // 16      # 10568
-# dram__bytes_read + dram__bytes_write per token, from the ncu capture of a 16384-token launch of the
-# current fused kernel summarised under profiles/: (134.27 + 3.38) MB / 16384 tokens (most of the output
-# is still dirty in L2 when the kernel ends, so the write part is below the algorithmic 2376 B/token);
-# traffic is proportional to tokens
-TRAFFIC_PER_TOKEN_NCU = 8401
+# dram__bytes_read per token, from the ncu capture of a 16384-token launch of the current fused kernel summarised under profiles/:
+# 134.27 MB / 16384 tokens, in proportion to the tokens.  (What that launch writes back before it ends, 3.7 of 38.9 MB, says how much the L2
+# holds and nothing of longer ones: the written bytes are the algorithmic ones.)
+TRAFFIC_PER_TOKEN_NCU = 8195
+WRITTEN_PER_TOKEN = (HIDDEN + KE) // 2 + (HIDDEN + KE) // 16                 # 2376
 FALLBACK_HBM_GBS = 6650.0
 FALLBACK_BF16_TFLOPS = 1590.0
 NVLINK_GBS = 770.0          # measured peer copy, per direction per GPU
@@ -961,8 +961,8 @@ def quantizer_measure(args, dev, world, rank, local, dist, hbm_peak, peak_kind):
            "value": value, "unit": "GB/s", "ms_per_step": ms_step, "clocks": clocks,
            "config": quantize_config(tokens, plain, world),
            "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s", "frac": achieved / hbm_peak,
-                        "traffic": TRAFFIC_PER_TOKEN_NCU * tokens,
-                        "traffic_source": "ncu capture of a 16384-token launch (profiles/), scaled by tokens",
+                        "traffic": (TRAFFIC_PER_TOKEN_NCU + WRITTEN_PER_TOKEN) * tokens,
+                        "traffic_source": "bytes read: ncu capture of a 16384-token launch (profiles/), scaled by tokens; bytes written: algorithmic",
                         "peak_kind": peak_kind,
                         "kernel": "arcq_quantize_ws_kernel_sets<RMS>" if not plain else "arcq_quantize_ws_kernel_sets<plain>",
                         "launch_ms": ms_step, "algorithmic_bytes_per_launch": algo_bytes}}

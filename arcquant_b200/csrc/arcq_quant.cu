@@ -1658,13 +1658,13 @@ int launch_quantize(const void* x, const void* gamma, float eps, const int16_t* 
 // latency.  The line lies where a CTA would take a second unit (three CTAs of 256 threads per SM, more of narrower rows), a unit per SM where rows
 // of one run are divided by a given scale and wider, two (four without a divisor of the caller's) of more than 512 groups.  us just below it, the
 // kernel of many rows / this one:
-//  * fused RMSNorm 16 x 4096 4.9 / 3.4, 888 x 4096 6.3 / 5.2, 1776 x 2048 5.7 / 5.3, 592 x 5120 6.3 / 5.3, 592 x 8192 7.6 / 6.3;
-//  * plain 592 x 5120 4.3 / 4.2, 592 x 8192 5.4 / 5.0, 592 x 14 336 7.8 / 7.5, 1184 x 14 336 12.8 / 12.6;
-//  * divided: 296 x 5120 4.2 / 3.6, 880 x 4096 5.0 / 5.1, over maxima 444 x 4096 4.3 / 4.0, 888 x 4096 5.0 / 5.0, but 592 x 5120 4.7 / 5.2, 592 x 14 336
-//    7.9 / 8.7, 1184 x 14 336 13.3 / 15.0;
-//  * grouped, eight runs: 444 x 8192 7.1 / 7.2, 444 x 14 336 10.5 / 10.9, 592 x 14 336 13.3 / 13.2, but 1100 x 4096 6.6 / 7.9, 1400 x 4096 6.9 / 8.3.
-// (So it was drawn against the kernel in use before that of many rows, and holds on to too much where rows are divided; callers' tests know
-// launches on either side of it by their kernels.)
+//  * fused RMSNorm 16 x 4096 4.2 / 3.4, 888 x 4096 5.5 / 5.2, 1776 x 2048 5.4 / 5.3, 592 x 5120 5.6 / 5.3, 592 x 8192 6.7 / 6.2;
+//  * plain 592 x 5120 4.2 / 4.2, 592 x 8192 5.2 / 5.0, 592 x 14 336 7.3 / 7.3, 1184 x 14 336 12.2 / 12.6;
+//  * divided: 296 x 5120 4.3 / 3.6, 880 x 4096 4.8 / 5.2, over maxima 444 x 4096 4.2 / 4.0, 888 x 4096 4.8 / 5.1, 592 x 5120 4.7 / 5.1, 592 x 14 336
+//    7.9 / 8.7, 1184 x 14 336 13.0 / 14.9;
+//  * grouped, eight runs: 444 x 8192 6.0 / 7.0, 444 x 14 336 8.3 / 10.1, 592 x 14 336 9.9 / 11.0, 1100 x 4096 5.8 / 7.9, 1400 x 4096 6.5 / 8.1.
+// (Open: it was drawn against the kernel in use before that of many rows, and where rows are divided it now holds on to too much, by 5 to 10 %, grouped by
+// 10 to 35 %.)
 struct RowLaunch {
   long long units;   // pairs of rows (grouped: as far as the host knows)
   int threads;       // of a CTA
@@ -1816,10 +1816,10 @@ int launch_quantize_tensor_scale(const void* x, const float* amax, int is_weight
     // the host.  Up to 16 loads a thread by every CTA for itself, up to 64 by clusters of eight, eight loads a thread each (without clusters: up to 32
     // by every CTA).  us, two launches / every CTA / clusters: 4 x 4096 4.8 / 3.8 / 4.4, 16 x 4096 5.1 / 4.6 / 4.0, 32 x 4096 4.9 / 5.9 / 4.3, 16 x
     // 8192 5.4 / 5.5 / 4.8, 8 x 14 336 7.1 / 5.9 / 4.9, 16 x 14 336 6.1 / - / 5.3, 32 x 512 4.4 / - / 3.7.  Beyond eight loads each a third round of them
-    // begins (with the registers of two groups a thread 20 x 14 336 6.3 / - / 6.5, 20 x 16 384 6.3 / - / 6.6).  Between 32 and 40 two launches stay, though
-    // clusters would be faster there too (17 x 4096 5.1 / - / 4.6): callers' tests know the maximum's pass of its own by its launch from just above 32 on.  In
-    // a graph behind another kernel, where the host's launches do not count, with the GEMM: 20 x 4096 11.8 / - / 11.3, 24 x 8192 15.0 / - / 14.7, 10 x 14 336
-    // 13.6 / - / 13.6, 16 x 14 336 14.4 / - / 14.2 (with two groups a thread 14.2 and 14.8).
+    // begins (with the registers of two groups a thread 20 x 14 336 6.3 / - / 6.5, 20 x 16 384 6.3 / - / 6.6).  Between 32 and 40 two launches stay (open: 20 x
+    // 4096, at 40, says that clusters would be faster there too, 4.8 / - / 4.3).  In a graph behind another kernel, where the host's launches do not count, with
+    // the GEMM: 20 x 4096 11.8 / - / 11.3, 24 x 8192 15.0 / - / 14.7, 10 x 14 336 13.6 / - / 13.6, 16 x 14 336 14.4 / - / 14.2 (with two groups a thread 14.2 and
+    // 14.8).
     const RowLaunch r = row_launch(KQ / 16, rows, 0, false, di);
     const bool small = nvec <= 32LL * r.threads, fits = clusters_take_maximum(KQ / 16, di) && nvec >= 40LL * r.threads && nvec <= 64LL * r.threads;
     if (groups == nullptr && (small || fits) && r.serves && (reinterpret_cast<uintptr_t>(sf) & 3u) == 0) {

@@ -1536,8 +1536,8 @@ int launch_rows(const QuantParams& p, const ScaleOptions& so, long long units, i
   long long grid = di.resident(per_sm);
   if (grid > (p.rows + R - 1) / R) grid = (p.rows + R - 1) / R;
   // A few wide rows: up to eight CTAs stage the same rows and quantize a part of their groups each, instead of two groups per thread in one
-  // CTA (14 336 channels, us, one CTA per pair of rows / this: plain 16 rows 4.6 / 3.6, 74 rows 4.8 / 3.9, 148 rows 4.8 / 4.2; over their own
-  // maximum 16 rows 7.5 / 6.5.  Rows of 4096 channels, one group per thread already, gain nothing.)
+  // CTA (14 336 channels, us, one CTA per pair of rows / this: plain 16 rows 4.6 / 3.6, 74 rows 4.8 / 3.9, 148 rows 4.8 / 4.2.
+  // Rows of 4096 channels, one group per thread already, gain nothing.)
   if (CLUSTERS) grid = (grid + MAX_CLUSTER - 1) / MAX_CLUSTER * MAX_CLUSTER;
   const int parts = CPT > 2 && !GROUPED ? row_parts(grid, CLUSTERS, di) : 1;
   const int groups_each = ((p.G + parts - 1) / parts + 31) & ~31;
